@@ -323,6 +323,11 @@ int ks_model_forward(ks_model* m, int first_slot, int n_slots, const int* tokens
  * enqueues only, apart from the wait for the pinned staging words between chunks. */
 int ks_model_prefill(ks_model* m, int slot, const int* tokens, int n_tokens);
 int ks_model_decode_token(ks_model* m, int first_slot, int n_slots, const int* tokens, int* next);    /* GP:1616 decode_token, blocking */
+/* One blocking step of slots first..first+n-1 whose tokens are sampled (GP:1622 decode_token_sampled + sample.rs:9-81 per slot):
+ * ks_model_forward with logits, then ks_sample_softcap_min_p over each slot's row, with only the logits that can survive
+ * the min-p filter leaving the device. */
+int ks_model_sample_step(ks_model* m, int first_slot, int n_slots, const int* tokens, const float* temperature, const float* min_p,
+                         const uint32_t* seed, int* next);
 int ks_model_generate(ks_model* m, int slot, const int* prompt, int n_prompt, int n_new, int max_inflight,
                       int* out, ks_generate_stats* stats);                   /* GP:1658 generate_timed */
 const void* ks_model_debug_ptr(const ks_model* m, int which, int slot);      /* test hook: 0 residual x, 1 logits, 2 phase stamps (first, last block), 3 every block's stamps */

@@ -1,0 +1,16 @@
+// Between ks_gemm.cu (images, epilogues, dispatch) and ks_gemm_q4k.cu (the Q4_K kernel).
+#pragma once
+#include "ks_gemm_common.cuh"
+
+struct ks_gemm_job {
+  int n_seg;
+  const uint8_t* W[3];
+  size_t rows[3];
+  float* y[3];               // partial `slot` of matrix i: y[i] + slot * part_stride[i], [token][row] with row stride ldy[i]
+  size_t ldy[3], part_stride[3];
+  unsigned cols, n_tok, np;
+  const __half* xt;
+  ks_gemm_map map;
+};
+ks_gemm_map ks_gemm_q4k_map(const ks_ctx* ctx, unsigned tiles, unsigned cols, unsigned np);
+int ks_launch_gemm_q4k(ks_ctx* ctx, const ks_gemm_job& job);

@@ -1,0 +1,573 @@
+// Q4_K weights x a batch of token rows on the tensor cores (tcgen05), weights dequantised into TENSOR memory.
+//
+// The reference's op is mul_mm (crates/ksearch_codegen/src/render.rs:1073-1291, reached from
+// crates/ksearch_kernels/src/lib.rs:1414).  A Q4_K weight is  d sc q - dmin m  with an 11-bit d, 6-bit sc and m and a 4-bit q
+// (crates/ksearch_gguf/src/gguf_impl.rs:690-721).  What goes to the tensor core is the integer  sc q  (at most 945: exact
+// in ONE f16), so a super-block of 256 k costs two products (x_hi, x_lo) where a split weight would cost three, and the
+// f32 result of each super-block is multiplied by its d on the way out of tensor memory:
+//   y[row, t] = sum over super-blocks of  s ( sum_k (sc q p) x[t, k]  -  sum_sub (mu m) S[t, sub] ),   s = d 2^j, p = 2^-j
+// with S the sub-block sums of x (2^-5 scaled, in the B image) and mu = 32 dmin / s as two f16 terms: the minima ride along as
+// 32 more k.  j = 0 unless dmin > 32 d, where it keeps mu m inside f16; sc q 2^-j stays exact.
+//
+// Per unit (128 rows x one super-block):
+//   * the packed rows come by ONE 2-D TMA box (128 rows x 144 bytes; 144-byte row pitch: 16-byte reads of 8 rows hit 8
+//     different bank groups) into a ring; the token rows by bulk copies of 32, 96 or 288 k into another;
+//   * 16 warps: warp w owns the 32 rows of tensor-memory lane quadrant w % 4 and the 64 weights g = w / 4 of each: one
+//     LOP3 and one HFMA2 make two weights out of packed nibbles ((1024 + q) sc - 1024 sc, exact), tcgen05.st puts them where
+//     the MMA reads A.  Shared memory then carries only packed weights and B: A never passes through it;
+//   * one elected lane issues the MMAs; after a super-block tcgen05.commit hands the accumulator to the 16 warps, which
+//     fold it into registers (s times) while the next super-block's MMAs run in the other accumulator.
+// Tensor memory (512 columns): A ring of three half super-blocks (3 x 64) and two blocks of minima (2 x 16) below 224, two
+// accumulators of up to 128 columns above: up to 64 token rows x_hi and x_lo are ONE MMA of 2 NP columns, up to 128 rows two
+// MMAs of NP; more rows have one accumulator of up to 256 columns.
+// One CTA per SM walks its units (ks_gemm_map) without a gap between tiles: the copies of the next tile are in flight while
+// the last one is written out.
+//
+// Bound by: few token rows, the packed weights from memory and the issue slots of the dequantisation (about 1.7 instructions
+// per weight and lane of 16 warps); 256 rows, the tensor core (34 MMAs of 128x256x16 per unit, 4350 cycles) and B through
+// shared memory (64 B per cycle in, 64 B per cycle out).
+// Every wait is bounded; on expiry the CTA raises the context's status word, waits (bounded) for what it has in flight, frees
+// its tensor memory and returns.
+#include <cuda.h>
+
+#include <cstdlib>
+#include <cstring>
+
+#include "ks_gemm_common.cuh"
+#include "ks_gemm.h"
+
+namespace {
+
+constexpr unsigned Q_WARPS = 16, Q_THREADS = (Q_WARPS + 3) * 32;  // workers, MMA, packed rows, token rows
+constexpr unsigned Q_RAW = GM_ROWS * KS_Q4K_BLOCK_BYTES;          // bytes of a unit's packed rows
+constexpr unsigned Q_EXT = 192, Q_D = 224;                        // tensor-memory columns: minima, first accumulator
+constexpr unsigned Q_WAIT = 1u << 20;
+constexpr unsigned Q_MAX_RAW = 6, Q_MAX_B = 6;
+
+struct __align__(64) Q4Args {
+  CUtensorMap w[3];        // matrix i: rows[i] rows of row_bytes bytes
+  float* y[3];             // y[i] + slot * part_stride[i] + token * ldy[i] + row
+  size_t ldy[3], part_stride[3];
+  unsigned rows[3], tile0[4];
+  ks_gemm_map map;
+  const __half* xt;        // the q4k form of the B image
+  unsigned cols, n_tok, np;
+  unsigned n_raw, n_b;     // ring depths
+  unsigned wait_limit, test_stall;
+  unsigned* err;
+};
+
+// barriers (8 bytes each) at the start of shared memory
+enum { QB_RAW_FULL = 0, QB_RAW_FREE = QB_RAW_FULL + Q_MAX_RAW, QB_B_FULL = QB_RAW_FREE + Q_MAX_RAW, QB_B_FREE = QB_B_FULL + Q_MAX_B,
+       QB_A_FULL = QB_B_FREE + Q_MAX_B, QB_A_FREE = QB_A_FULL + 3, QB_D_FULL = QB_A_FREE + 3, QB_D_FREE = QB_D_FULL + 2, QB_DONE = QB_D_FREE + 2,
+       QB_COUNT };
+constexpr unsigned Q_HEAD = 2048;  // barriers, then from 512 the token rows' scale factors
+static_assert(QB_COUNT * 8 + 16 <= 512, "barriers fit the head of shared memory");
+
+__device__ __forceinline__ void mb_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ uint32_t and_or(uint32_t w, uint32_t mask, uint32_t bits) { return (w & mask) | bits; }
+
+// What a thread needs of its row's super-block header: the two sub-blocks 2 g and 2 g + 1 (g uniform in a warp).
+struct Q4Hdr {
+  __half2 sc[2], cc[2];     // sub-block 2 g: sc p, -1024 sc p;  2 g + 1: sc p / 16, -64 sc p
+  uint32_t mhi, mlo;        // -(mu m) of both, two f16 terms
+  float s;
+};
+__device__ __forceinline__ __half2 small_int_h2(unsigned v) {  // v < 1024 in both halves: 1024 + v by its bits, then an exact subtract
+  return __hsub2(as_h2(v * 0x00010001u | 0x64006400u), __float2half2_rn(1024.0f));
+}
+__device__ __forceinline__ void q4_header(const uint4 h, unsigned g, Q4Hdr& o) {
+  const __half2 dd = *reinterpret_cast<const __half2*>(&h.x);
+  const float d = __low2float(dd), dm = __high2float(dd);
+  // bytes 2 g', 2 g' + 1 (g' = g & 1) of the three groups of four scale bytes; g < 2: sc and m lie in the low six bits of the
+  // first two, else nibbles of the third and the top bits of the first two
+  const unsigned sh = 16u * (g & 1u);
+  const unsigned y = h.y >> sh, z = h.z >> sh, w = h.w >> sh;
+  unsigned sc0, sc1, m0, m1;
+  if (g < 2u) {
+    sc0 = y & 63u;
+    sc1 = (y >> 8) & 63u;
+    m0 = z & 63u;
+    m1 = (z >> 8) & 63u;
+  } else {
+    sc0 = (w & 15u) | ((y >> 2) & 48u);
+    sc1 = ((w >> 8) & 15u) | ((y >> 10) & 48u);
+    m0 = ((w >> 4) & 15u) | ((z >> 2) & 48u);
+    m1 = ((w >> 12) & 15u) | ((z >> 10) & 48u);
+  }
+  const float ad = fabsf(d), am = fabsf(dm);
+  __half2 s0 = small_int_h2(sc0), s1 = small_int_h2(sc1);
+  float s = d, mu = ad > 0.0f ? __fdividef(32.0f * dm, d) : 0.0f;
+  if (am > 32.0f * ad) {
+    // j: the smallest power of two with dmin <= 32 d 2^j; beyond 2^20 (or d = 0) the d part is below the last bit of the minima
+    float p = 0.0f;
+    if (am <= 32.0f * 1048576.0f * ad) {
+      const unsigned e = (__float_as_uint(__fdividef(am, 32.0f * ad)) >> 23) - 127u + 1u;  // 1..21
+      p = __uint_as_float((127u - e) << 23);
+      s = d * __uint_as_float((127u + e) << 23);
+      mu *= p;
+    } else {
+      s = dm * 0.03125f;
+      mu = 1024.0f;
+    }
+    s0 = __hmul2(s0, __float2half2_rn(p));
+    s1 = __hmul2(s1, __float2half2_rn(p));
+  }
+  o.sc[0] = s0;
+  o.cc[0] = __hmul2(s0, __float2half2_rn(-1024.0f));
+  o.sc[1] = __hmul2(s1, __float2half2_rn(0.0625f));
+  o.cc[1] = __hmul2(s1, __float2half2_rn(-64.0f));
+  const float v0 = -mu * (float)m0, v1 = -mu * (float)m1;
+  const __half2 mh = __floats2half2_rn(v0, v1);
+  const float2 mf = __half22float2(mh);
+  o.mhi = pack_h2(mh);
+  o.mlo = pack_h2(__floats2half2_rn(v0 - mf.x, v1 - mf.y));
+  o.s = s;
+}
+// 16 packed bytes (16 weights of sub-block 2 g in the low nibbles, 16 of 2 g + 1 in the high ones) -> 8 + 8 words of A.
+__device__ __forceinline__ void q4_words(const uint4 q, const Q4Hdr& h, uint32_t (&lo)[8], uint32_t (&hi)[8]) {
+  const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const uint32_t v = w[i] >> 8;
+    lo[2 * i] = pack_h2(__hfma2(as_h2(and_or(w[i], 0x000F000Fu, 0x64006400u)), h.sc[0], h.cc[0]));
+    lo[2 * i + 1] = pack_h2(__hfma2(as_h2(and_or(v, 0x000F000Fu, 0x64006400u)), h.sc[0], h.cc[0]));
+    hi[2 * i] = pack_h2(__hfma2(as_h2(and_or(w[i], 0x00F000F0u, 0x64006400u)), h.sc[1], h.cc[1]));
+    hi[2 * i + 1] = pack_h2(__hfma2(as_h2(and_or(v, 0x00F000F0u, 0x64006400u)), h.sc[1], h.cc[1]));
+  }
+}
+
+struct Seg {  // one matrix of the launch, picked without dynamic indexing of the parameters
+  unsigned rows, tile0;
+  float* y;
+  size_t ldy, part;
+};
+__device__ __forceinline__ Seg pick_seg(const Q4Args& a, unsigned tile) {
+  const int i = (tile >= a.tile0[1]) + (tile >= a.tile0[2]);
+  Seg s;
+  s.rows = i == 0 ? a.rows[0] : i == 1 ? a.rows[1] : a.rows[2];
+  s.tile0 = i == 0 ? a.tile0[0] : i == 1 ? a.tile0[1] : a.tile0[2];
+  s.y = i == 0 ? a.y[0] : i == 1 ? a.y[1] : a.y[2];
+  s.ldy = i == 0 ? a.ldy[0] : i == 1 ? a.ldy[1] : a.ldy[2];
+  s.part = i == 0 ? a.part_stride[0] : i == 1 ? a.part_stride[1] : a.part_stride[2];
+  return s;
+}
+
+// Groups of 32 k (a super-block has 9, the minima's among them) per B stage: as many as let two or more stages fit.
+__host__ __device__ constexpr unsigned q4_kb(int tq) { return tq <= 16 ? 9u : tq == 32 ? 3u : 1u; }
+
+// TQ: token rows per worker thread at most (NP / 4: the four warps of a lane quadrant share the accumulator's columns).
+template <int TQ>
+__global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_constant__ Q4Args a) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  const uint32_t bars = sm32(smem);
+  auto bar = [&](unsigned i) { return bars + 8u * i; };
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + QB_COUNT * 8);
+  volatile unsigned* fail = reinterpret_cast<volatile unsigned*>(smem + QB_COUNT * 8 + 8);
+  const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  constexpr bool CONCAT = TQ <= 16;               // x_hi and x_lo side by side in one MMA
+  constexpr unsigned KB = q4_kb(TQ), NACC = TQ == 64 ? 1 : 2;   // groups of 32 k per B stage, accumulators
+  const unsigned b_group = 4u * 2u * a.np * 16u, b_stage = KB * b_group;
+  float* up_s = reinterpret_cast<float*>(smem + 512);   // 2^e of every token row
+  const uint32_t raw0 = bars + Q_HEAD, b0 = raw0 + a.n_raw * Q_RAW;
+  const unsigned u0 = ks_gemm_first(a.map, blockIdx.x), n_units = a.map.base + (blockIdx.x < a.map.rem ? 1u : 0u);
+
+  if (threadIdx.x == 0) {
+    for (unsigned i = 0; i < a.n_raw; i++) {
+      mb_init(bar(QB_RAW_FULL + i), 1);
+      mb_init(bar(QB_RAW_FREE + i), Q_WARPS);
+    }
+    for (unsigned i = 0; i < a.n_b; i++) {
+      mb_init(bar(QB_B_FULL + i), 1);
+      mb_init(bar(QB_B_FREE + i), 1);
+    }
+    for (unsigned i = 0; i < 3; i++) {
+      mb_init(bar(QB_A_FULL + i), Q_WARPS / 2);
+      mb_init(bar(QB_A_FREE + i), 1);
+    }
+    for (unsigned i = 0; i < 2; i++) {
+      mb_init(bar(QB_D_FULL + i), 1);
+      mb_init(bar(QB_D_FREE + i), Q_WARPS);
+    }
+    mb_init(bar(QB_DONE), 1);
+    *fail = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 0) tc_alloc(sm32(tslot), 512);
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (*tslot != 0u && threadIdx.x == 0) *fail = 1;  // all 512 columns were asked for: they start at 0
+  constexpr uint32_t tmem = 0;
+
+  if (warp < Q_WARPS) {
+    // ---- workers
+    const unsigned quad = warp & 3u, g = warp >> 2, half = g >> 1;
+    const uint32_t tlane = tmem + ((quad * 32u) << 16);
+    const unsigned row = quad * 32u + lane;
+    const unsigned tq = a.np >> 2;               // tokens of this thread: [g * tq, + tq)
+    const unsigned acc_cols = CONCAT ? 2u * a.np : a.np;
+    float acc[TQ];
+#pragma unroll
+    for (int i = 0; i < TQ; i++) acc[i] = 0.0f;
+    float s_prev = 0.0f;
+    bool ok = true;
+    unsigned tile = u0 / a.map.S, sb = u0 - tile * a.map.S, prev_tile = 0;
+    unsigned rs = 0, rph = 0;  // ring stage of the packed rows and its phase
+    uint4 hraw = {}, qa = {}, qb = {};
+    // the packed bytes of this thread, read one unit ahead: the reads overlap the accumulator's way out
+    auto fetch = [&]() {
+      const bool got = __all_sync(0xffffffffu, mb_wait(bar(QB_RAW_FULL + rs), rph, a.wait_limit));
+      if (got) {
+        const uint32_t blk = raw0 + rs * Q_RAW + row * KS_Q4K_BLOCK_BYTES;
+        hraw = lds128(blk);
+        qa = lds128(blk + 16u + 32u * g);
+        qb = lds128(blk + 32u + 32u * g);
+        __syncwarp();
+        if (lane == 0) mb_arrive(bar(QB_RAW_FREE + rs));
+        if (++rs == a.n_raw) {
+          rs = 0;
+          rph ^= 1u;
+        }
+      }
+      return got;
+    };
+    // (with 64 sums per thread there are no registers for that)
+    constexpr bool AHEAD = TQ < 64;
+    if (AHEAD && n_units) ok = fetch();
+    for (unsigned i = 0; i <= n_units && ok; i++) {
+      float s_cur = 0.0f;
+      bool last = i == n_units;   // the unit before this one ends a tile, or this CTA's share of one
+      // the first unit's weights need nothing of the kernels before this one; the waits below depend on the image, and what is
+      // written at the end may still be read by them
+      if (i == 1) asm volatile("griddepcontrol.wait;" ::: "memory");
+      if (i < n_units) {
+        if (!AHEAD && !fetch()) { ok = false; break; }
+        Q4Hdr h;
+        q4_header(hraw, g, h);
+        s_cur = h.s;
+        const unsigned n = 2u * i + half, slot = n % 3u;
+        if (n >= 3u && !__all_sync(0xffffffffu, mb_wait(bar(QB_A_FREE + slot), (n / 3u - 1u) & 1u, a.wait_limit))) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t at = tlane + slot * 64u + (g & 1u) * 32u;
+        uint32_t lo[8], hi[8];
+        q4_words(qa, h, lo, hi);
+        tc_st8(at, lo);
+        tc_st8(at + 16u, hi);
+        q4_words(qb, h, lo, hi);
+        tc_st8(at + 8u, lo);
+        tc_st8(at + 24u, hi);
+        tc_st4(tlane + Q_EXT + (i & 1u) * 16u + 4u * g, h.mhi, h.mhi, h.mlo, 0u);
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mb_arrive(bar(QB_A_FULL + slot));
+        if (AHEAD && i + 1u < n_units && !fetch()) { ok = false; break; }
+        if (i > 0 && sb == 0) last = true;
+        if (++sb == a.map.S) {
+          sb = 0;
+          tile++;
+        }
+      }
+      if (i > 0) {  // fold the previous super-block's accumulators
+        const unsigned j = i - 1u, buf = j % NACC;
+        if (!__all_sync(0xffffffffu, mb_wait(bar(QB_D_FULL + buf), (j / NACC) & 1u, a.wait_limit))) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t dcol = tlane + Q_D + buf * acc_cols + g * tq;
+#pragma unroll
+        for (int c = 0; c < TQ; c += 16) {
+          if ((unsigned)c < tq) {
+            uint32_t d0[16], d1[16];
+            if (TQ >= 16 && (unsigned)c + 16u <= tq) {
+              tc_ld16(dcol + c, d0);
+              if (CONCAT) tc_ld16(dcol + a.np + c, d1);
+            } else {
+#pragma unroll
+              for (int k = 0; k < 16; k += 4)
+                if (c + k < TQ && (unsigned)(c + k) < tq) {
+                  tc_ld4(dcol + c + k, d0 + k);
+                  if (CONCAT) tc_ld4(dcol + a.np + c + k, d1 + k);
+                }
+            }
+            tc_wait_ld16(d0);
+            if (CONCAT) tc_wait_ld16(d1);
+#pragma unroll
+            for (int k = 0; k < 16; k++)
+              if (c + k < TQ && (unsigned)(c + (k & ~3)) < tq) {
+                float t = __uint_as_float(d0[k]);
+                if (CONCAT) t += __uint_as_float(d1[k]);
+                acc[c + k] = fmaf(s_prev, t, acc[c + k]);
+              }
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mb_arrive(bar(QB_D_FREE + buf));
+        if (last) {
+          const Seg sg = pick_seg(a, prev_tile);
+          const unsigned out_row = (prev_tile - sg.tile0) * GM_ROWS + row;
+          const unsigned pslot = blockIdx.x - ks_gemm_owner(a.map, prev_tile * a.map.S);
+          float* y = sg.y + (size_t)pslot * sg.part + out_row;
+          const bool live = out_row < sg.rows;
+#pragma unroll
+          for (int k = 0; k < TQ; k++) {
+            const unsigned t = g * tq + k;
+            if ((unsigned)k < tq && t < a.n_tok && live) y[(size_t)t * sg.ldy] = acc[k] * up_s[t];
+            acc[k] = 0.0f;
+          }
+        }
+      }
+      s_prev = s_cur;
+      prev_tile = sb == 0 ? tile - 1u : tile;  // tile and sb already point one unit on
+    }
+    if (!ok && lane == 0) *fail = 1;
+  } else if (warp == Q_WARPS) {
+    // ---- MMAs: the whole warp runs the loop, converged, and one elected lane issues (loop state and descriptors then stay in
+    // uniform registers)
+    const unsigned leader = elect_one();
+    const unsigned ncol = CONCAT ? 2u * a.np : a.np;
+    const uint32_t idesc = (1u << 4) | ((ncol >> 3) << 17) | ((unsigned)(GM_ROWS >> 4) << 24);  // f32 accumulate, f16 x f16, K-major both
+    const uint64_t bdesc0 = tc_desc(b0, 2u * a.np * 16u, 128u);
+    const unsigned chunk2 = 4u * a.np, lo_rows = a.np;   // in descriptor units of 16 bytes: two chunks of 8 k, the hi rows
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // What an MMA takes has to be in uniform registers when it issues.  It gets there by itself only while the compiler can see
+    // that the warp stays together: loop bounds from launch parameters and blockIdx, no value out of memory (hence the
+    // constant tensor-memory base), one way out.  Otherwise every MMA waits for five register moves, about 200 cycles.
+    bool ok = false;
+    unsigned bs = 0, bph = 0;                   // B stage and its phase
+    unsigned s0 = 0, ph0 = 0, s1 = 1, ph1 = 0;  // A slots of the unit's two halves and their phases
+    for (unsigned i = 0; i < n_units; i++) {
+      const unsigned buf = i % NACC;
+      const uint32_t d = tmem + Q_D + buf * ncol;
+      if (i >= NACC && !__all_sync(0xffffffffu, mb_wait(bar(QB_D_FREE + buf), (i / NACC - 1u) & 1u, a.wait_limit))) goto out;
+      uint64_t bd = 0;
+#pragma unroll
+      for (unsigned kg = 0; kg < 9; kg++) {  // groups of 32 k: four of each half, the minima
+        bool got = true, waited = false;
+        if (kg == 0 || kg == 4u) {
+          got = mb_wait(bar(QB_A_FULL + (kg ? s1 : s0)), kg ? ph1 : ph0, a.wait_limit);
+          waited = true;
+        }
+        if (kg % KB == 0) {
+          got = got && mb_wait(bar(QB_B_FULL + bs), bph, a.wait_limit);
+          waited = true;
+          bd = bdesc0 + (uint64_t)(bs * (b_stage >> 4));
+        }
+        if (waited) {
+          if (!__all_sync(0xffffffffu, got)) goto out;
+          tc_fence_after();
+        }
+        if (leader) {
+          const uint32_t at = kg == 8u ? tmem + Q_EXT + (i & 1u) * 16u : tmem + (kg < 4u ? s0 : s1) * 64u + (kg & 3u) * 16u;
+          const uint64_t b = bd + (uint64_t)((kg % KB) * (b_group >> 4));
+          tc_mma_f16_ta(d, at, b, idesc, kg ? 1u : 0u);
+          if (!CONCAT && kg < 8u) tc_mma_f16_ta(d, at, b + lo_rows, idesc, 1u);
+          tc_mma_f16_ta(d, at + 8u, b + chunk2, idesc, 1u);
+          if (!CONCAT && kg < 8u) tc_mma_f16_ta(d, at + 8u, b + chunk2 + lo_rows, idesc, 1u);
+          if (kg % KB == KB - 1u) tc_commit(bar(QB_B_FREE + bs));
+          if (kg == 3u) tc_commit(bar(QB_A_FREE + s0));
+          if (kg == 8u) {
+            tc_commit(bar(QB_A_FREE + s1));
+            tc_commit(bar(QB_D_FULL + buf));
+          }
+        }
+        if (kg % KB == KB - 1u && ++bs == a.n_b) {
+          bs = 0;
+          bph ^= 1u;
+        }
+      }
+      __syncwarp();
+      // the next unit's halves: two slots further round the ring of three
+      s0 += 2u;
+      if (s0 >= 3u) {
+        s0 -= 3u;
+        ph0 ^= 1u;
+      }
+      s1 += 2u;
+      if (s1 >= 3u) {
+        s1 -= 3u;
+        ph1 ^= 1u;
+      }
+    }
+    ok = true;
+  out:
+    // every MMA issued must finish before shared and tensor memory go away (bounded): a last commit tracks them all
+    if (leader) {
+      if (!ok) *fail = 1;
+      tc_commit(bar(QB_DONE));
+    }
+    __syncwarp();
+    mb_wait(bar(QB_DONE), 0u, Q_WAIT);
+  } else if (warp == Q_WARPS + 1) {
+    // ---- packed rows: they depend on no kernel before this one
+    const unsigned leader = elect_one();
+    unsigned issued = 0, st = 0, ph = 1, tile = u0 / a.map.S, sb = u0 - tile * a.map.S;
+    for (unsigned i = 0; i < n_units; i++) {
+      const bool got = i < a.n_raw || mb_wait(bar(QB_RAW_FREE + st), ph, a.wait_limit);
+      if (!__all_sync(0xffffffffu, got)) {
+        if (leader) *fail = 1;
+        break;
+      }
+      if (leader) {
+        const int k = (tile >= a.tile0[1]) + (tile >= a.tile0[2]);
+        const unsigned t0 = k == 0 ? a.tile0[0] : k == 1 ? a.tile0[1] : a.tile0[2];
+        mb_expect(bar(QB_RAW_FULL + st), Q_RAW);  // rows past the matrix come as zeros and count
+        tma_in_2d(raw0 + st * Q_RAW, k == 0 ? &a.w[0] : k == 1 ? &a.w[1] : &a.w[2], sb * KS_Q4K_BLOCK_BYTES, (tile - t0) * GM_ROWS, bar(QB_RAW_FULL + st));
+      }
+      issued++;
+      if (++st == a.n_raw) {
+        st = 0;
+        ph ^= 1u;
+      }
+      if (++sb == a.map.S) {
+        sb = 0;
+        tile++;
+      }
+      __syncwarp();
+    }
+    for (unsigned j = issued > a.n_raw ? issued - a.n_raw : 0u; j < issued; j++) mb_wait(bar(QB_RAW_FULL + j % a.n_raw), (j / a.n_raw) & 1u, a.wait_limit);
+  } else {
+    // ---- token rows
+    const unsigned leader = elect_one();
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the image comes from the kernel before this one
+    const float* up = reinterpret_cast<const float*>(a.xt + xt_scale_off(a.cols, a.np));
+    for (unsigned t = lane; t < a.np; t += 32u) up_s[t] = up[t];  // read behind the first accumulator, which waits for the copies below
+    __syncwarp();
+    constexpr unsigned PER = 9u / KB;
+    const unsigned total = n_units * PER;
+    unsigned issued = 0, sb = u0 % a.map.S, k = 0, st = 0, ph = 1;
+    for (unsigned j = 0; j < total; j++) {
+      const bool got = j < a.n_b || mb_wait(bar(QB_B_FREE + st), ph, a.wait_limit);
+      if (!__all_sync(0xffffffffu, got)) {
+        if (leader) *fail = 1;
+        break;
+      }
+      if (a.test_stall && j / PER + 1u == a.test_stall) break;  // test hook: this unit's token rows never arrive
+      if (leader) {
+        mb_expect(bar(QB_B_FULL + st), b_stage);
+        const size_t at = ((size_t)sb * 9u + (size_t)k * KB) * b_group;
+        bulk_in(b0 + st * b_stage, reinterpret_cast<const unsigned char*>(a.xt) + at, b_stage, bar(QB_B_FULL + st));
+      }
+      issued++;
+      if (++st == a.n_b) {
+        st = 0;
+        ph ^= 1u;
+      }
+      if (++k == PER) {
+        k = 0;
+        if (++sb == a.map.S) sb = 0;
+      }
+      __syncwarp();
+    }
+    for (unsigned j = issued > a.n_b ? issued - a.n_b : 0u; j < issued; j++) mb_wait(bar(QB_B_FULL + j % a.n_b), (j / a.n_b) & 1u, a.wait_limit);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (threadIdx.x == 0 && *fail) atomicOr(a.err, 8u);
+  if (warp == 0) tc_dealloc(tmem, 512);
+}
+
+typedef CUresult (*encode_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                              const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+encode_fn tensor_map_encoder() {
+  static encode_fn fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) p = nullptr;
+    return reinterpret_cast<encode_fn>(p);
+  }();
+  return fn;
+}
+
+// Ring depths: two B stages at least, then packed rows up to the four units that cover the latency of memory, then whatever
+// of either still fits.
+size_t q4_rings(const ks_ctx* ctx, unsigned np, unsigned kb, unsigned* n_raw, unsigned* n_b) {
+  const size_t room = ctx->smem_optin - Q_HEAD, stage = (size_t)kb * np * 128u;
+  *n_raw = 2;
+  *n_b = kb == 1 ? 4 : kb == 3 ? 3 : 2;
+  auto fits = [&](unsigned r, unsigned b) { return r <= Q_MAX_RAW && b <= Q_MAX_B && b * stage + r * Q_RAW <= room; };
+  while (*n_raw < 4 && fits(*n_raw + 1, *n_b)) ++*n_raw;
+  while (fits(*n_raw, *n_b + 1)) ++*n_b;
+  while (fits(*n_raw + 1, *n_b)) ++*n_raw;
+  return Q_HEAD + *n_b * stage + *n_raw * Q_RAW;
+}
+}  // namespace
+
+// How many CTAs a launch of `tiles` tiles takes.  A CTA's time is its units (t_u each) plus writing its shares of tiles; the
+// partials are then read once more.  More CTAs mean fewer units each and more partials.
+ks_gemm_map ks_gemm_q4k_map(const ks_ctx* ctx, unsigned tiles, unsigned cols, unsigned np) {
+  ks_gemm_map m{};
+  m.S = cols / 256u;
+  const unsigned U = tiles * m.S, most = (unsigned)ctx->sm_count < U ? (unsigned)ctx->sm_count : U;
+  const double t_u = 0.45 + np * 0.0085, t_w = 0.1 + np * 0.005;
+  double best = 1e30;
+  for (unsigned G = 1; G <= most; G++) {
+    if (G < most && tiles % G && G * 4u < most * 3u) continue;
+    const unsigned per = (U + G - 1) / G, shares = (per + m.S - 2) / m.S + 1;
+    const double slots = (double)G / tiles + 1.0;
+    const double cost = per * t_u + shares * t_w + slots * tiles * np * (GM_ROWS * 4e-6 / 5.0);
+    if (cost < best) {
+      best = cost;
+      m.G = G;
+    }
+  }
+  m.base = U / m.G;
+  m.rem = U % m.G;
+  return m;
+}
+
+int ks_launch_gemm_q4k(ks_ctx* ctx, const ks_gemm_job& job) {
+  encode_fn enc = tensor_map_encoder();
+  if (!enc) return ks_fail(ctx, KS_ERR_CUDA, "gemm: cuTensorMapEncodeTiled is not available");
+  Q4Args a;
+  memset(&a, 0, sizeof a);
+  const cuuint64_t row_bytes = (cuuint64_t)job.cols / 256 * KS_Q4K_BLOCK_BYTES;
+  unsigned tiles = 0;
+  for (int i = 0; i < 3; i++) {
+    a.tile0[i] = i < job.n_seg ? tiles : 0xFFFFFFFFu;  // no tile reaches an absent matrix
+    if (i >= job.n_seg) continue;
+    a.rows[i] = (unsigned)job.rows[i];
+    a.y[i] = job.y[i];
+    a.ldy[i] = job.ldy[i];
+    a.part_stride[i] = job.part_stride[i];
+    tiles += (unsigned)((job.rows[i] + GM_ROWS - 1) / GM_ROWS);
+    const cuuint64_t dims[2] = {row_bytes, (cuuint64_t)job.rows[i]}, strides[1] = {row_bytes};
+    const cuuint32_t box[2] = {KS_Q4K_BLOCK_BYTES, GM_ROWS}, es[2] = {1, 1};
+    if (enc(&a.w[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(job.W[i]), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return ks_fail(ctx, KS_ERR_INVALID, "gemm: the packed rows cannot be described to TMA (base must be 16-byte aligned)");
+  }
+  a.tile0[3] = tiles;
+  a.map = job.map;
+  a.xt = job.xt;
+  a.cols = job.cols;
+  a.n_tok = job.n_tok;
+  a.np = job.np;
+  const int c = job.np <= 16 ? 0 : job.np <= 32 ? 1 : job.np <= 64 ? 2 : job.np <= 128 ? 3 : 4;
+  const size_t smem = q4_rings(ctx, job.np, q4_kb(4 << c), &a.n_raw, &a.n_b);
+  a.err = (unsigned*)ctx->ws + KS_WS_ERR_WORD;
+  a.wait_limit = Q_WAIT;
+  if (const char* t = getenv("KSEARCH_GEMM_TEST_STALL")) {  // exercises the give-up path: short waits, one operand withheld
+    a.test_stall = (unsigned)atoi(t);
+    if (a.test_stall) a.wait_limit = 4000;
+  }
+  void (*kern)(Q4Args) = c == 0 ? gemm_q4k_tc_kernel<4> : c == 1 ? gemm_q4k_tc_kernel<8> : c == 2 ? gemm_q4k_tc_kernel<16>
+                       : c == 3 ? gemm_q4k_tc_kernel<32> : gemm_q4k_tc_kernel<64>;
+  static size_t set[5][16] = {{0}};
+  size_t& have = set[c][ctx->device & 15];
+  if (smem > have) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return ks_fail(ctx, KS_ERR_CUDA, "gemm: cannot set %zu B shared memory: %s", smem, cudaGetErrorString(e));
+    have = smem;
+  }
+  KS_LAUNCH(ctx, kern, dim3(job.map.G), Q_THREADS, smem, a);
+  return ks_after_launch(ctx, "gemm_q4k_tc");
+}

@@ -146,6 +146,26 @@ int ks_launch_copy_scale_indexed(ks_ctx* ctx, size_t n, size_t batch, float scal
                                  const void* src, const float* idx, ks_dtype act, void* dst);
 int ks_launch_softcap_argmax(ks_ctx* ctx, size_t n, float cap, ks_dtype act, const void* logits, float* out_idx);
 
+// ---- sampling candidates (ks_sample_gpu.cu, ks_sample.cpp) -------------------------------------------
+constexpr unsigned KS_CAND_MAX = 2048;  // pairs kept per slot; more and the host takes the whole row
+struct ks_cand {
+  unsigned index;
+  float logit;
+};
+struct ks_cand_head {
+  unsigned count, odd;  // odd: the row holds an infinity or NaN
+  int max_ordered;
+  int pad;
+};
+struct ks_cand_cut {
+  float below[64];      // per slot: temperature * ln(1 / min_p)
+};
+// Logit rows [n_slots][n] -> head[n_slots], list[n_slots][KS_CAND_MAX] (in no order).
+int ks_launch_candidates(ks_ctx* ctx, ks_dtype act, const void* logits, size_t n, int n_slots, float cap, const ks_cand_cut& cuts, ks_cand_head* head,
+                         ks_cand* list);
+// The draw over candidates in index order; the others' probabilities fall under the min-p threshold.
+uint32_t ks_sample_candidates(const ks_cand* c, size_t n, float cap, float temperature, float min_p, uint32_t seed);
+
 // ---- tensor-core GEMM for batches of more than 8 token rows (ks_gemm.cu) ---------------------------
 // nelem (a multiple of 256) elements of src (Q6K, Q4K, F16, F32) -> Q4_K blocks, as the reference's load-time quantizer.
 int ks_launch_quantize_q4k(ks_ctx* ctx, ks_dtype src_dtype, const void* src, size_t nelem, void* dst);
@@ -153,8 +173,8 @@ size_t ks_gemm_xt_bytes(size_t cols, int n_tok);  // bytes of the split image of
 size_t ks_gemm_part_floats(const ks_ctx* ctx, size_t total_rows, size_t cols, int n_tok);  // k-split partials, at most
 // The context's scratch, grown to `bytes` (fails inside a stream capture when it would have to grow).
 int ks_ctx_gemm_scratch(ks_ctx* ctx, size_t bytes, void** out);
-// x[t * ldx + k] (f32) -> the image the GEMM reads its token rows from.
-int ks_launch_gemm_split(ks_ctx* ctx, const float* x, size_t ldx, int n_tok, size_t cols, void* xt);
+// x[t * ldx + k] (f32) -> the image the GEMM over weights of that dtype reads its token rows from.
+int ks_launch_gemm_split(ks_ctx* ctx, ks_dtype wdtype, const float* x, size_t ldx, int n_tok, size_t cols, void* xt);
 // Up to three matrices over the same columns and token rows (q, k, v; gate, up) in one launch.  What becomes of
 // the sums: PLAIN y[i] = W[i] x; GELU (two matrices) y[0] = gelu(W[0] x) * (W[1] x); NORM_SPLIT (one matrix)
 // out_x = res + rms(W x) * w_post and the image of rms(out_x) * w_norm for the next GEMM in xt_out; GELU_SPLIT
@@ -165,6 +185,7 @@ struct ks_gemm_epi {
   float eps;
   float* out_x;                        // NORM_SPLIT: the updated residual rows
   void* xt_out;                        // the image written for the next GEMM (may be the image this GEMM read)
+  ks_dtype next_dtype;                 // NORM_SPLIT: weights of that next GEMM
 };
 int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* const* W, const size_t* rows, size_t cols, const void* xt,
                         int n_tok, float* const* y, const size_t* ldy, float* P, int mode, const ks_gemm_epi* epi);

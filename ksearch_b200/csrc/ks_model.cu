@@ -13,6 +13,7 @@
 //     run as one launch (the same two-output kernel as after attention).
 // Per-layer embeddings, sliding windows and shared-KV layers of real Gemma-4
 // checkpoints are not part of this driver.
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <utility>
@@ -137,6 +138,9 @@ struct ks_model {
   unsigned req_id = 0;        // the last request word handed to collect_kernel
   int solo_max = 2;           // up to this many slots step as one persistent-kernel pass each
   size_t host_tok_n = 0;
+  // sampled steps (built on first use): candidates of every slot on the device and in pinned memory
+  ks_cand_head* cand_head = nullptr;  // [n_slots] heads, then [n_slots][KS_CAND_MAX] pairs
+  void* host_cand = nullptr;
   // graphs keyed by (first slot, n slots, src parity, want_logits)
   std::map<uint64_t, cudaGraphExec_t> graphs;
   std::map<uint64_t, size_t> graph_nodes;
@@ -163,8 +167,8 @@ struct ks_model {
   float* cmeta_swa = nullptr;
   float* cattn_tmp = nullptr;
   int chunk = 1;  // tokens per prompt chunk: as many as the matvec kernels can stage side by side (<= KS_PREFILL_CHUNK)
-  // rows per pass through the tensor-core GEMM (0: not available, activations are not f32); its scratch inside the
-  // context's GEMM workspace: the split operand image, two sets of k-split partials
+  // rows per pass through the tensor-core GEMM (0: not available, activations are not f32) and its scratch: the split
+  // operand image, the k-split partials
   int gemm_chunk = 0;
   void* gemm_xt = nullptr;
   float* gemm_p0 = nullptr;
@@ -348,7 +352,7 @@ int enqueue_forward_gemm(ks_model* m, const Lane& L_, int n, bool want_logits) {
   if ((rc = lane_begin(m, L_, n))) return rc;
   if ((rc = ks_launch_copy_scale_indexed(c, H, n, sqrtf((float)H), (ks_dtype)g.embd_dtype, m->token_embd.dptr, L_.tok_in, act, x))) return rc;
   if ((rc = ks_launch_rmsnorm(c, H, n, g.eps, act, x, m->layers[0].attn_norm.dptr, nullptr, 0, 0.f, x2))) return rc;
-  if ((rc = ks_launch_gemm_split(c, (const float*)x2, H, n, H, m->gemm_xt))) return rc;
+  if ((rc = ks_launch_gemm_split(c, KS_Q4K, (const float*)x2, H, n, H, m->gemm_xt))) return rc;
   // From here on the normed rows exist only as the image the next GEMM reads: the sums of the o-proj and
   // down-proj partials go straight through the residual update and the next norm into that image.
   ks_gemm_epi epi{};
@@ -371,10 +375,11 @@ int enqueue_forward_gemm(ks_model* m, const Lane& L_, int n, bool want_logits) {
       return rc;
     if ((rc = ks_launch_sdpa(c, n, nq, nkv, hd, g.attn_scale, act, q, kk, kv, L_.kv_stride, layer_meta(m, L_, l), L_.attn_tmp, o, att_splits)))
       return rc;
-    if ((rc = ks_launch_gemm_split(c, (const float*)o, qn, n, qn, m->gemm_xt))) return rc;
+    if ((rc = ks_launch_gemm_split(c, KS_Q4K, (const float*)o, qn, n, qn, m->gemm_xt))) return rc;
     {  // o-proj, x += rms(.) * w_post_attn, image of rms(x) * w_ffn_norm (lib.rs:539)
       const uint8_t* Ws[1] = {(const uint8_t*)L.wo.dptr};
       float* ys[1] = {nullptr};
+      epi.next_dtype = KS_Q4K;
       epi.w_post = (const float*)L.post_attn_norm.dptr;
       epi.w_norm = (const float*)L.ffn_norm.dptr;
       if ((rc = ks_launch_gemm_segs(c, KS_Q4K, 1, Ws, &H, qn, m->gemm_xt, n, ys, &H, m->gemm_p0, KS_GEMM_NORM_SPLIT, &epi))) return rc;
@@ -388,6 +393,7 @@ int enqueue_forward_gemm(ks_model* m, const Lane& L_, int n, bool want_logits) {
     {  // down-proj, x += rms(.) * w_post_ffw, image of the NEXT norm (next layer's attn norm, or the output norm)
       const uint8_t* Ws[1] = {(const uint8_t*)L.wdown.dptr};
       float* ys[1] = {nullptr};
+      epi.next_dtype = l + 1 < g.n_layers ? KS_Q4K : (ks_dtype)g.embd_dtype;
       epi.w_post = (const float*)L.post_ffw_norm.dptr;
       epi.w_norm = (const float*)((l + 1 < g.n_layers) ? m->layers[l + 1].attn_norm.dptr : m->output_norm.dptr);
       if ((rc = ks_launch_gemm_segs(c, KS_Q4K, 1, Ws, &H, F, m->gemm_xt, n, ys, &H, m->gemm_p0, KS_GEMM_NORM_SPLIT, &epi))) return rc;
@@ -752,13 +758,18 @@ ks_model* ks_model_create(ks_ctx* ctx, const ks_model_config* cfg) {
       const size_t rows_of[5] = {qn + 2 * kvn, H, 2 * F, H, (size_t)g.vocab}, cols_of[5] = {H, qn, H, F, H};
       size_t xt = 0, part = 0;
       for (int i = 0; i < 5; i++) {
-        const size_t a = ks_gemm_xt_bytes(cols_of[i], G), b = 4 * ks_gemm_part_floats(ctx, rows_of[i], cols_of[i], G);
+        const int most = i < 4 ? G : g.n_slots;  // only decode steps reach the head
+        const size_t a = ks_gemm_xt_bytes(cols_of[i], most);
         xt = a > xt ? a : xt;
-        part = b > part ? b : part;
+        for (int n = 1; n <= most; n += n < 16 ? 15 : 16) {  // fewer rows are split finer
+          const int rows = n + 15 < most ? n + 15 : most;
+          const size_t b = 4 * ks_gemm_part_floats(ctx, rows_of[i], cols_of[i], rows);
+          part = b > part ? b : part;
+        }
       }
       xt = (xt + 255) & ~(size_t)255;
       void* ws = nullptr;
-      if (ks_ctx_gemm_scratch(ctx, xt + part, &ws) != KS_OK) {
+      if (dev_alloc(m, &ws, xt + part) != KS_OK) {
         ok = false;
       } else {
         m->gemm_xt = ws;
@@ -862,6 +873,7 @@ void ks_model_destroy(ks_model* m) {
   if (m->host_tok) cudaFreeHost(m->host_tok);
   if (m->host_ret) cudaFreeHost(m->host_ret);
   if (m->host_ids) cudaFreeHost(m->host_ids);
+  if (m->host_cand) cudaFreeHost(m->host_cand);
   delete m;
 }
 
@@ -1205,6 +1217,60 @@ int ks_model_decode_token(ks_model* m, int first, int n, const int* tokens, int*
     if ((rc = check_device_status(m, &flag, first, n, 1))) return rc;
   }
   for (int s = 0; s < n; s++) next[s] = (int)back[s];
+  return KS_OK;
+}
+
+// One step of slots first..first+n-1 and the tokens sampled from its logits (decode_token_sampled, gemma_prim.rs:1622-1634;
+// the draw of sample.rs:9-81).  The device lists the logits that can survive the min-p filter; a slot without such a filter
+// (min_p = 0), or whose row holds more than KS_CAND_MAX of them or a value that is not finite, is sampled from the whole row.
+int ks_model_sample_step(ks_model* m, int first, int n, const int* tokens, const float* temperature, const float* min_p, const uint32_t* seed,
+                         int* next) {
+  if (!m) return KS_ERR_INVALID;
+  ks_ctx* c = m->ctx;
+  KS_REQUIRE(c, tokens && temperature && min_p && seed && next, "sample_step: null argument");
+  const ks_model_config& g = m->cfg;
+  const size_t S = g.n_slots, head_b = S * sizeof(ks_cand_head), list_b = S * KS_CAND_MAX * sizeof(ks_cand);
+  int rc;
+  if (!m->cand_head && (rc = dev_alloc(m, (void**)&m->cand_head, head_b + list_b))) return rc;
+  if (!m->host_cand && cudaMallocHost(&m->host_cand, head_b + list_b) != cudaSuccess) {
+    m->host_cand = nullptr;
+    return ks_fail(c, KS_ERR_OOM, "sample_step: pinned allocation failed");
+  }
+  if ((rc = ks_model_forward(m, first, n, tokens, 1))) return rc;
+  const size_t ab = act_b(m), V = g.vocab;
+  ks_cand_cut cuts{};
+  bool listed[64];
+  for (int s = 0; s < n; s++) {
+    const bool greedy = temperature[s] < 1e-6f;
+    listed[s] = greedy || min_p[s] > 1e-6f;
+    cuts.below[s] = greedy || !listed[s] || min_p[s] >= 1.0f ? 0.0f : -temperature[s] * logf(min_p[s]) * 1.0001f;
+  }
+  char* dev = (char*)m->cand_head;
+  char* host = (char*)m->host_cand;
+  const ks_cand* dlist = (const ks_cand*)(dev + head_b);
+  ks_cand* hlist = (ks_cand*)(host + head_b);
+  constexpr size_t FEW = 64;  // pairs of a slot that come along with the counts
+  if ((rc = ks_launch_candidates(c, (ks_dtype)g.act, (const char*)m->logits + (size_t)first * V * ab, V, n, g.softcap, cuts, m->cand_head, (ks_cand*)dlist)))
+    return rc;
+  KS_CUDA(c, cudaMemcpyAsync(host, dev, n * sizeof(ks_cand_head), cudaMemcpyDeviceToHost, c->stream));
+  KS_CUDA(c, cudaMemcpy2DAsync(hlist, KS_CAND_MAX * sizeof(ks_cand), dlist, KS_CAND_MAX * sizeof(ks_cand), FEW * sizeof(ks_cand), n, cudaMemcpyDeviceToHost,
+                               c->stream));
+  if ((rc = ks_synchronize(c))) return rc;
+  const ks_cand_head* hh = (const ks_cand_head*)host;
+  for (int s = 0; s < n; s++) {
+    ks_cand* l = hlist + (size_t)s * KS_CAND_MAX;
+    const size_t count = hh[s].count;
+    if (listed[s] && !hh[s].odd && count >= 1 && count <= KS_CAND_MAX) {
+      if (count > FEW) KS_CUDA(c, cudaMemcpy(l, dlist + (size_t)s * KS_CAND_MAX, count * sizeof(ks_cand), cudaMemcpyDeviceToHost));
+      std::sort(l, l + count, [](const ks_cand& a, const ks_cand& b) { return a.index < b.index; });
+      next[s] = (int)ks_sample_candidates(l, count, g.softcap, temperature[s], min_p[s], seed[s]);
+      continue;
+    }
+    std::vector<unsigned char> row(V * ab);
+    KS_CUDA(c, cudaMemcpy(row.data(), (const char*)m->logits + (size_t)(first + s) * V * ab, V * ab, cudaMemcpyDeviceToHost));
+    next[s] = (int)(g.act == KS_F32 ? ks_sample_softcap_min_p_f32((const float*)row.data(), V, g.softcap, temperature[s], min_p[s], seed[s])
+                                    : ks_sample_softcap_min_p((const uint16_t*)row.data(), V, g.softcap, temperature[s], min_p[s], seed[s]));
+  }
   return KS_OK;
 }
 

@@ -86,6 +86,41 @@ uint32_t sample_impl(size_t n, Get get, float cap, float temperature, float min_
 
 }  // namespace
 
+// sample.rs:9-81 over the tokens that can survive its min-p filter (a superset, in index order).  A dropped token adds to
+// nothing but the softmax's normaliser, which scales the probabilities, their threshold and the drawn number alike, so it is
+// left out on both sides.
+uint32_t ks_sample_candidates(const ks_cand* c, size_t n, float cap, float temperature, float min_p, uint32_t seed) {
+  size_t best = 0;
+  float best_v = -INFINITY;
+  std::vector<float> xs(n);
+  for (size_t i = 0; i < n; i++) {
+    const float x = c[i].logit;
+    xs[i] = cap > 0.0f ? cap * tanhf(x / cap) : x;
+    if (xs[i] > best_v) {
+      best_v = xs[i];
+      best = i;
+    }
+  }
+  if (temperature < 1e-6f) return c[best].index;
+  const float threshold = fmaxf(min_p, 0.0f);
+  float filtered = 0.0f;
+  for (float& x : xs) {
+    x = expf((x - best_v) / temperature);
+    if (x < threshold) x = 0.0f;
+    else filtered += x;
+  }
+  uint32_t rng = seed | 1u;
+  const float r = ((float)splitmix32(&rng) / 4294967296.0f) * filtered;
+  float cdf = 0.0f;
+  size_t last = best;
+  for (size_t i = 0; i < n; i++) {
+    cdf += xs[i];
+    if (xs[i] > 0.0f) last = i;
+    if (r < cdf) return c[i].index;
+  }
+  return c[last].index;
+}
+
 extern "C" {
 
 // sample_softcap_min_p over f16 logit bits, as the reference takes them.  n >= 1; returns the token id.

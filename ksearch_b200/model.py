@@ -197,6 +197,14 @@ class GemmaCudaModel:
         self.ctx.check(self.lib.ks_model_decode_token(self.h, first, n, (C.c_int * n)(*toks), out))
         return list(out)
 
+    def sample_step(self, tokens, first: int, temperature, min_p, seed):
+        """decode_token_sampled (gemma_prim.rs:1622-1634) for neighbouring slots: one step, one sampled token each."""
+        n = len(tokens)
+        out = (C.c_int * n)()
+        self.ctx.check(self.lib.ks_model_sample_step(self.h, first, n, (C.c_int * n)(*[int(t) for t in tokens]), (C.c_float * n)(*temperature),
+                                                     (C.c_float * n)(*min_p), (C.c_uint32 * n)(*seed), out))
+        return list(out)
+
     def generate_timed(self, prompt, n_new: int, slot: int = 0, max_inflight: int = 1):
         p = (C.c_int * len(prompt))(*[int(t) for t in prompt])
         out = (C.c_int * max(1, n_new))()

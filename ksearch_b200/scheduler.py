@@ -11,7 +11,7 @@ whole budget otherwise (scheduler.rs:233-304) — then frees the slots of finish
 One deliberate difference: the reference decodes its active requests one after the other (one `decode_token_sampled`
 each, scheduler.rs:163-231); here the requests of a decode round that sit in neighbouring slots advance in ONE
 model step (the backend's multi-slot path).  Greedy requests (temperature < 1e-6) take the device arg-max; the others
-read their logits back and are sampled on the host with the reference's sampler (sample.rs:9-81)."""
+are sampled with the reference's sampler (sample.rs:9-81) from the logits the step left behind."""
 from __future__ import annotations
 
 from collections import deque
@@ -145,6 +145,8 @@ class Scheduler:
         try:
             if all(a.req.temperature < 1e-6 for a in run):
                 nxt = self.model.decode_token(ids, first)          # device arg-max after the softcap
+            elif hasattr(self.model, "sample_step"):               # one native call: the step, then each slot's draw
+                nxt = self.model.sample_step(ids, first, [a.req.temperature for a in run], [a.req.min_p for a in run], [a.rng for a in run])
             else:
                 self.model.forward(first, len(run), ids, True)
                 self.model.ctx.synchronize()

@@ -1,0 +1,32 @@
+"""ks_model_sample_step: the device lists the logits that can survive the min-p filter, the host draws.  Every token has to be
+the one the CPU sampler (sample.rs:9-81) takes from the whole row, on the paths of one, two and several slots, with the
+filter off, with more survivors than the list holds, and greedy."""
+import numpy as np
+import pytest
+
+from ksearch_b200 import F16, F32, CudaContext, synth
+from ksearch_b200 import model as ksm
+from ksearch_b200.sample import sample_softcap_min_p
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("act", [F32, F16])
+@pytest.mark.parametrize("n", [1, 2, 5])
+def test_sample_step_takes_the_cpu_samplers_tokens(n, act):
+    c = CudaContext(0, flags=1)
+    cfg = ksm.tiny_config(max_seq=64, n_slots=n, act=act)
+    cfg.vocab = 8193                      # not a multiple of anything the kernels use
+    cfg.sigma_embd = 2e-5                 # flat logits: many survivors
+    model = ksm.GemmaCudaModel.synthetic(c, cfg, seed=31)
+    slots = [model.slot_alloc() for _ in range(n)]
+    ids = [int(t) for t in synth.token_ids(31, "ids", n, cfg.vocab)]
+    for step, (temp, min_p) in enumerate([(0.8, 0.05), (1.5, 0.3), (0.7, 1e-4), (4.0, 1e-3), (1.0, 0.0), (0.0, 0.05), (1.0, 1.0), (0.9, 2.0)]):
+        seeds = [1000 * step + 7 * s for s in slots]
+        got = model.sample_step(ids, 0, [temp] * n, [min_p] * n, seeds)
+        want = [sample_softcap_min_p(model.read_debug(1, s), cfg.softcap, temp, min_p, seeds[s]) for s in slots]
+        assert got == want, (temp, min_p)
+        ids = got
+    assert [model.seq_len(s) for s in slots] == [8] * n
+    model.close()
+    c.close()
