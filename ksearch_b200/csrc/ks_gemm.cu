@@ -589,6 +589,8 @@ bool gemm_covers(ks_dtype wdtype, size_t cols, int n_tok) {
 }
 }  // namespace
 
+unsigned ks_gemm_np(int n_tok) { return gemm_np(n_tok); }
+
 // Bytes of the B image of n_tok rows of `cols` values (hi + lo halves, token count padded to 16).
 size_t ks_gemm_xt_bytes(size_t cols, int n_tok) { return cols / 256 * 288 * gemm_np(n_tok) * 4 + (size_t)gemm_np(n_tok) * 4; }  // image + one factor per row
 

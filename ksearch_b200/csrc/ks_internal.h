@@ -142,6 +142,14 @@ int ks_launch_per_head_qkv_q40(ks_ctx* ctx, size_t n_q, size_t n_kv, size_t hd, 
 int ks_launch_sdpa(ks_ctx* ctx, size_t n_slots, size_t n_q, size_t n_kv, size_t hd, float scale, ks_dtype act,
                    const void* q, const uint8_t* K, const uint8_t* V, size_t slot_stride_bytes, const float* meta,
                    float* tmp, void* out, int n_splits);
+// A prompt chunk's rows against one slot's cache on the tensor cores (ks_sdpa_chunk.cu), and the merge of its records into
+// the operand image of the output projection.
+int ks_sdpa_chunk_splits(const ks_ctx* ctx, int n_tok, size_t n_q, size_t n_kv, size_t ctx_len, int most);
+bool ks_sdpa_chunk_covers(size_t n_q, size_t n_kv, size_t hd, const void* K, const void* V);
+int ks_launch_sdpa_chunk(ks_ctx* ctx, int n_tok, size_t n_q, size_t n_kv, size_t hd, float scale, const float* q, const uint8_t* K,
+                         const uint8_t* V, const float* meta, float* tmp, int n_splits);
+int ks_launch_sdpa_merge_split(ks_ctx* ctx, int n_tok, unsigned np, size_t n_q, size_t hd, const float* tmp, int n_splits, void* xt);
+unsigned ks_gemm_np(int n_tok);  // token rows of an operand image: n_tok padded
 int ks_launch_copy_scale_indexed(ks_ctx* ctx, size_t n, size_t batch, float scale, ks_dtype src_dtype,
                                  const void* src, const float* idx, ks_dtype act, void* dst);
 int ks_launch_softcap_argmax(ks_ctx* ctx, size_t n, float cap, ks_dtype act, const void* logits, float* out_idx);

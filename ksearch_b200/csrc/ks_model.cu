@@ -188,6 +188,7 @@ int dev_alloc(ks_model* m, void** p, size_t bytes) {
 
 constexpr int KS_PREFILL_CHUNK = 8;  // tokens per pass over the weights (the matvec kernels take up to 8)
 constexpr int KS_GEMM_CHUNK = 256;   // rows per pass when the tensor-core GEMM takes the matrices (f32 activations)
+constexpr int KS_CHUNK_ATT_MIN = 4;  // prompt rows from which they share one pass over their context (a block takes 64 rows x heads)
 constexpr size_t KS_STAGE_IDS = 256; // pinned words that stage host token ids
 
 // Where a forward pass reads and writes: n rows of activations, their positions, and the KV caches
@@ -348,7 +349,7 @@ int enqueue_forward_gemm(ks_model* m, const Lane& L_, int n, bool want_logits) {
   char *x = L_.x, *x2 = L_.x2, *q = L_.q, *k = L_.k, *v = L_.v, *o = L_.o, *logits = L_.logits;
   float* tok_out = L_.tok_out;
   int rc;
-  const int att_splits = att_splits_for(m, n);
+  const int att_splits = att_splits_for(m, n), chunk_splits = ks_sdpa_chunk_splits(c, n, nq, nkv, (size_t)g.max_seq, m->n_splits);
   if ((rc = lane_begin(m, L_, n))) return rc;
   if ((rc = ks_launch_copy_scale_indexed(c, H, n, sqrtf((float)H), (ks_dtype)g.embd_dtype, m->token_embd.dptr, L_.tok_in, act, x))) return rc;
   if ((rc = ks_launch_rmsnorm(c, H, n, g.eps, act, x, m->layers[0].attn_norm.dptr, nullptr, 0, 0.f, x2))) return rc;
@@ -373,9 +374,15 @@ int enqueue_forward_gemm(ks_model* m, const Lane& L_, int n, bool want_logits) {
     if ((rc = ks_launch_per_head_qkv_q40(c, nq, nkv, hd, n, g.eps, act, q, L.q_norm.dptr, m->rope, k, L.k_norm.dptr, v, q,
                                          kk, kv, L_.pos, L_.kv_stride)))
       return rc;
-    if ((rc = ks_launch_sdpa(c, n, nq, nkv, hd, g.attn_scale, act, q, kk, kv, L_.kv_stride, layer_meta(m, L_, l), L_.attn_tmp, o, att_splits)))
-      return rc;
-    if ((rc = ks_launch_gemm_split(c, KS_Q4K, (const float*)o, qn, n, qn, m->gemm_xt))) return rc;
+    if (L_.chunk_base && n >= KS_CHUNK_ATT_MIN && ks_sdpa_chunk_covers(nq, nkv, hd, kk, kv)) {  // the rows of a chunk share their context
+      if ((rc = ks_launch_sdpa_chunk(c, n, nq, nkv, hd, g.attn_scale, (const float*)q, kk, kv, layer_meta(m, L_, l), L_.attn_tmp, chunk_splits)) ||
+          (rc = ks_launch_sdpa_merge_split(c, n, ks_gemm_np(n), nq, hd, L_.attn_tmp, chunk_splits, m->gemm_xt)))
+        return rc;
+    } else {
+      if ((rc = ks_launch_sdpa(c, n, nq, nkv, hd, g.attn_scale, act, q, kk, kv, L_.kv_stride, layer_meta(m, L_, l), L_.attn_tmp, o, att_splits)))
+        return rc;
+      if ((rc = ks_launch_gemm_split(c, KS_Q4K, (const float*)o, qn, n, qn, m->gemm_xt))) return rc;
+    }
     {  // o-proj, x += rms(.) * w_post_attn, image of rms(x) * w_ffn_norm (lib.rs:539)
       const uint8_t* Ws[1] = {(const uint8_t*)L.wo.dptr};
       float* ys[1] = {nullptr};
