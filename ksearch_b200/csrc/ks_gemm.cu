@@ -361,26 +361,33 @@ struct FinishArgs {
   ks_gemm_map map;
   int mode;
 };
-// One block per row tile and eight token rows (the tile's partial count is the block's); a thread sums four neighbouring rows.
-constexpr unsigned FIN_TOKENS = 8;
-__device__ __forceinline__ float4 sum_slots(const float* P, size_t stride, unsigned n, size_t at, bool vec, unsigned valid) {
-  float4 g = make_float4(0.f, 0.f, 0.f, 0.f);
+// One block per row tile and a few token rows (the tile's partial count is the block's); a thread sums four neighbouring rows
+// where row counts and addresses allow 16-byte accesses, else one.
+template <int V>
+struct FinVec {
+  float v[V];
+};
+template <int V>
+__device__ __forceinline__ FinVec<V> sum_slots(const float* P, size_t stride, unsigned n, size_t at) {
+  FinVec<V> g;
+#pragma unroll
+  for (int k = 0; k < V; k++) g.v[k] = 0.0f;
+#pragma unroll 4
   for (unsigned s = 0; s < n; s++) {
     const float* p = P + (size_t)s * stride + at;
-    if (vec) {
+    if constexpr (V == 4) {
       const float4 a = *reinterpret_cast<const float4*>(p);
-      g.x += a.x; g.y += a.y; g.z += a.z; g.w += a.w;
+      g.v[0] += a.x; g.v[1] += a.y; g.v[2] += a.z; g.v[3] += a.w;
     } else {
-      g.x += p[0];
-      if (valid > 1u) g.y += p[1];
-      if (valid > 2u) g.z += p[2];
-      if (valid > 3u) g.w += p[3];
+      g.v[0] += *p;
     }
   }
   return g;
 }
+template <int V>
 __global__ void __launch_bounds__(256) gemm_finish_kernel(const FinishArgs f) {
   ks_pdl_entry();
+  constexpr unsigned PER = GM_ROWS / V, TOK = 256u / PER;  // threads per token row, token rows per block
   const unsigned bx = blockIdx.x, seg = f.mode == 1 ? 0u : (bx >= f.tile0[1]) + (bx >= f.tile0[2]);
   const unsigned rows = seg == 0 ? f.rows[0] : seg == 1 ? f.rows[1] : f.rows[2];
   const unsigned tile0 = seg == 0 ? f.tile0[0] : seg == 1 ? f.tile0[1] : f.tile0[2];
@@ -388,25 +395,18 @@ __global__ void __launch_bounds__(256) gemm_finish_kernel(const FinishArgs f) {
   const size_t ps = seg == 0 ? f.part_stride[0] : seg == 1 ? f.part_stride[1] : f.part_stride[2];
   const size_t ldy = seg == 0 ? f.ldy[0] : seg == 1 ? f.ldy[1] : f.ldy[2];
   float* y = seg == 0 ? f.y[0] : seg == 1 ? f.y[1] : f.y[2];
-  const unsigned t = blockIdx.y * FIN_TOKENS + (threadIdx.x >> 5), r = (bx - tile0) * GM_ROWS + (threadIdx.x & 31u) * 4u;
+  const unsigned t = blockIdx.y * TOK + threadIdx.x / PER, r = (bx - tile0) * GM_ROWS + (threadIdx.x % PER) * V;
   if (t >= f.n_tok || r >= rows) return;
-  const unsigned valid = rows - r < 4u ? rows - r : 4u;
-  const bool vec = valid == 4u && rows % 4u == 0;
   const size_t at = (size_t)t * rows + r;  // partials are dense [split][token][row]
-  float4 g = sum_slots(P, ps, ks_gemm_slots(f.map, bx), at, vec, valid);
+  FinVec<V> g = sum_slots<V>(P, ps, ks_gemm_slots(f.map, bx), at);
   if (f.mode == 1) {
-    const float4 u = sum_slots(f.P[1], f.part_stride[1], ks_gemm_slots(f.map, f.tile0[1] + bx), at, vec, valid);
-    g = make_float4(gelu_mul(g.x, u.x), gelu_mul(g.y, u.y), gelu_mul(g.z, u.z), gelu_mul(g.w, u.w));
+    const FinVec<V> u = sum_slots<V>(f.P[1], f.part_stride[1], ks_gemm_slots(f.map, f.tile0[1] + bx), at);
+#pragma unroll
+    for (int k = 0; k < V; k++) g.v[k] = gelu_mul(g.v[k], u.v[k]);
   }
   float* o = y + (size_t)t * ldy + r;
-  if (vec && ((uintptr_t)o & 15u) == 0) {
-    *reinterpret_cast<float4*>(o) = g;
-  } else {
-    o[0] = g.x;
-    if (valid > 1u) o[1] = g.y;
-    if (valid > 2u) o[2] = g.z;
-    if (valid > 3u) o[3] = g.w;
-  }
+  if constexpr (V == 4) *reinterpret_cast<float4*>(o) = make_float4(g.v[0], g.v[1], g.v[2], g.v[3]);
+  else *o = g.v[0];
 }
 
 }  // namespace
@@ -736,7 +736,15 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
   f.n_tok = (unsigned)n_tok;
   f.mode = mode;
   const unsigned out_tiles = mode == KS_GEMM_GELU ? tile0[1] : tiles;
-  KS_LAUNCH(ctx, (gemm_finish_kernel), dim3(out_tiles, ((unsigned)n_tok + FIN_TOKENS - 1) / FIN_TOKENS), 256, 0, f);
+  bool vec = true;
+  for (int i = 0; i < n_seg; i++) {
+    vec = vec && rows[i] % 4 == 0 && ((uintptr_t)out[i] & 15) == 0;
+    if (mode == KS_GEMM_PLAIN || i == 0) vec = vec && ((uintptr_t)f.y[i] & 15) == 0 && f.ldy[i] % 4 == 0;
+  }
+  const unsigned tok = vec ? 8u : 2u;
+  const dim3 grid(out_tiles, ((unsigned)n_tok + tok - 1) / tok);
+  if (vec) KS_LAUNCH(ctx, (gemm_finish_kernel<4>), grid, 256, 0, f);
+  else KS_LAUNCH(ctx, (gemm_finish_kernel<1>), grid, 256, 0, f);
   return ks_after_launch(ctx, "gemm_finish");
 }
 

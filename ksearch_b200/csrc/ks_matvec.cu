@@ -308,6 +308,36 @@ int launch_q6k_nt(ks_ctx* ctx, const MvArgs& a, int grid, int threads, size_t sm
 
 }  // namespace
 
+// What one token takes without a plan, measured over rows 512..262144 and cols 1536..10240 (rotating copies beyond L2, both
+// activation dtypes).  Q6_K: the ring kernel (262144x1536 91 -> 66 us, 8192x4096 27 -> 14 us against variant 2); two row sets
+// per tile while four tiles of them are within 40 KB (up to 2048 columns), and as many warps as keep the last round of a short
+// launch full.  Q4_K: the fixed-point kernel where its shorter inner loop pays for staging x (rows of 4096 columns on:
+// 1536x6144 11.4 -> 6.5 us; or many rows of at most 2048: 12288x1536 7.8 -> 6.7 us), else the streamed kernel with eight warps
+// and two blocks per SM (20480x2560 16.5 -> 14.6 us).
+static ks_plan single_token_default(const ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_t cols, bool one_matrix) {
+  ks_plan p{};
+  if (wdtype == KS_Q4K) {
+    p.variant = one_matrix && (cols >= 4096 || (rows >= 8192 && cols <= 2048)) ? 3 : 0;
+    p.nr = p.variant == 3 ? 0 : 1;
+    p.nwarps = 8;
+    p.ctas_per_sm = 2;
+    return p;
+  }
+  p.nr = cols <= 2048 ? 2 : 1;
+  p.variant = 4 | (2 << 8);
+  p.ctas_per_sm = 1;
+  const size_t tiles = rows / (4 * (size_t)p.nr), sms = (size_t)ctx->sm_count;
+  size_t best = 0;
+  for (int nw = 12; nw >= 8; nw--) {
+    const size_t rounds = (tiles + sms * nw - 1) / (sms * nw);
+    if (!best || (rounds * nw < best && rounds <= 12)) {
+      best = rounds * nw;
+      p.nwarps = nw;
+    }
+  }
+  return p;
+}
+
 bool ks_matvec_can_fuse_pro(ks_dtype wdtype, size_t cols) { return wdtype == KS_Q4K && cols % 256 == 0 && cols <= 4096; }
 
 int ks_launch_matvec(ks_ctx* ctx, ks_dtype wdtype, const ks_mv_seg* segs, int n_seg, ks_mv_epilogue epi,
@@ -335,6 +365,11 @@ int ks_launch_matvec(ks_ctx* ctx, ks_dtype wdtype, const ks_mv_seg* segs, int n_
                                                                   : (wdtype == KS_Q4K ? "mv_q4k" : "mv_q6k");
     plan = ks_plan_lookup(ctx, op, epi == KS_EPI_GATE_UP ? segs[0].rows : total, cols, n_tok);
   }
+  ks_plan dflt;
+  if (!plan && n_tok == 1 && !(pro && pro->mode != KS_PRO_NONE)) {
+    dflt = single_token_default(ctx, wdtype, segs[0].rows, cols, n_seg == 1);
+    plan = &dflt;
+  }
   if (pro && pro->mode != KS_PRO_NONE) {
     KS_REQUIRE(ctx, ks_matvec_can_fuse_pro(wdtype, cols), "matvec: no fused norm prologue for dtype %d, cols=%zu", (int)wdtype, cols);
     return ks_launch_matvec_stream_q4k(ctx, segs, n_seg, epi, cols, act, x, n_tok, plan, pro);
@@ -350,9 +385,10 @@ int ks_launch_matvec(ks_ctx* ctx, ks_dtype wdtype, const ks_mv_seg* segs, int n_
     if (rc != 1) return rc;
   }
   if (wdtype == KS_Q6K && (!plan || (plan->variant & 0xFF) == 2 || (plan->variant & 0xFF) == 4)) {  // also the default: single-token calls take it, others fall through
-    const int rc = ks_launch_matvec_q6k_fx(ctx, segs, n_seg, cols, act, x, n_tok, plan);
+    const int rc = ks_launch_matvec_q6k_fx(ctx, segs, n_seg, cols, act, x, n_tok, plan == &dflt ? nullptr : plan);
     if (rc != 1) return rc;
   }
+  if (plan == &dflt) plan = nullptr;  // the shape takes neither: every further kernel has its own defaults
   if (wdtype == KS_Q6K && (!plan || (plan->variant & 0xFF) == 0)) {
     const int rc = ks_launch_matvec_stream_q6k(ctx, segs, n_seg, cols, act, x, n_tok, plan);
     if (rc != 1) return rc;

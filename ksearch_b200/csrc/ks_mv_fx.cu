@@ -1,4 +1,5 @@
-// Q4_K matvec, one token, f32 x and y: the planner's variant 3.
+// Q4_K matvec, one token, x and y in the activation dtype: the planner's variant 3, and what single matrices of long rows
+// or many rows take without a plan (ks_matvec.cu).
 //
 // y = W x (crates/ksearch_kernels/src/lib.rs:137 matvec_wd; the G1 kernel of
 // crates/ksearch_codegen/src/lower.rs:1763-2082) for matrices of a few megabytes, where a launch lasts
@@ -24,8 +25,8 @@ constexpr int FXM_MAXSLOTS = 16;
 
 struct FxmArgs {
   const uint8_t* W;
-  const float* x;
-  float* y;
+  const void* x;
+  void* y;
   unsigned rows, cols, row_bytes;
   unsigned n_seg, seg_units;   // column segments of <= 32 units
   unsigned piece_rows;         // rows per ring slot (multiple of 4)
@@ -46,6 +47,7 @@ __host__ __device__ inline FxmSmem fxm_smem(unsigned x_bytes, unsigned slot_byte
   return L;
 }
 
+template <typename XT>
 __global__ void __launch_bounds__(FXM_THREADS, 2) mv_q4k_fx_kernel(const FxmArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -82,7 +84,7 @@ __global__ void __launch_bounds__(FXM_THREADS, 2) mv_q4k_fx_kernel(const FxmArgs
 #pragma unroll
     for (int k = 0; k < 4; k++) {
       const unsigned c = base + threadIdx.x + k * FXM_THREADS;
-      if (c < nchunk) v[k] = reinterpret_cast<const float4*>(a.x)[c];
+      if (c < nchunk) v[k] = ld_chunk<XT>(reinterpret_cast<const XT*>(a.x), c);
     }
 #pragma unroll
     for (int k = 0; k < 4; k++) {
@@ -166,7 +168,7 @@ __global__ void __launch_bounds__(FXM_THREADS, 2) mv_q4k_fx_kernel(const FxmArgs
       const unsigned r = wr0 + threadIdx.x;
       float v = 0.0f;
       for (unsigned sg2 = 0; sg2 < a.n_seg; sg2++) v += psum[r * a.n_seg + sg2];
-      a.y[lo + r] = v;
+      act_store<XT>(reinterpret_cast<XT*>(a.y), lo + r, v);
     }
   }
 }
@@ -176,12 +178,12 @@ __global__ void __launch_bounds__(FXM_THREADS, 2) mv_q4k_fx_kernel(const FxmArgs
 // Returns 1 when the call is outside what this kernel takes (the caller picks another variant).
 int ks_launch_matvec_q4k_fx(ks_ctx* ctx, const ks_mv_seg* segs, int n_seg, ks_mv_epilogue epi, size_t cols, ks_dtype act,
                             const void* x, int n_tok, const ks_plan* plan) {
-  if (n_seg != 1 || epi != KS_EPI_PLAIN || act != KS_F32 || n_tok != 1) return 1;
+  if (n_seg != 1 || epi != KS_EPI_PLAIN || n_tok != 1) return 1;
   const unsigned U = (unsigned)(cols / 64);
   const unsigned S = (U + 31u) / 32u;
   if (S > (unsigned)FXM_MAXSEG || U % S) return 1;
   const unsigned rows = segs[0].rows, row_bytes = (unsigned)(cols / 256 * KS_Q4K_BLOCK_BYTES);
-  if (rows < 2 || ((uintptr_t)x & 15u)) return 1;
+  if (rows < 2 || ((uintptr_t)x & (act == KS_F32 ? 15u : 7u))) return 1;
   // grid: one or two blocks per SM, as long as every block keeps a few rows
   const int cps = (plan && plan->ctas_per_sm > 0) ? (plan->ctas_per_sm > 2 ? 2 : plan->ctas_per_sm) : 1;
   unsigned grid = (unsigned)(ctx->sm_count * cps);
@@ -205,8 +207,8 @@ int ks_launch_matvec_q4k_fx(ks_ctx* ctx, const ks_mv_seg* segs, int n_seg, ks_mv
   if (n_slots > (unsigned)FXM_MAXSLOTS) n_slots = FXM_MAXSLOTS;
   FxmArgs a{};
   a.W = segs[0].W;
-  a.x = (const float*)x;
-  a.y = (float*)segs[0].y;
+  a.x = x;
+  a.y = segs[0].y;
   a.rows = rows;
   a.cols = (unsigned)cols;
   a.row_bytes = row_bytes;
@@ -218,12 +220,14 @@ int ks_launch_matvec_q4k_fx(ks_ctx* ctx, const ks_mv_seg* segs, int n_seg, ks_mv
   a.x_bytes = x_bytes;
   a.err = (unsigned*)ctx->ws + KS_WS_ERR_WORD;
   const size_t smem = fxm_smem(x_bytes, slot_bytes, n_slots).total;
-  static size_t smem_set[16] = {0};
-  if (smem > smem_set[ctx->device & 15]) {
-    cudaError_t e = cudaFuncSetAttribute(mv_q4k_fx_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  void (*kern)(FxmArgs) = act == KS_F32 ? mv_q4k_fx_kernel<float> : mv_q4k_fx_kernel<__half>;
+  static size_t smem_set[2][16] = {{0}};
+  size_t& set = smem_set[act == KS_F32 ? 0 : 1][ctx->device & 15];
+  if (smem > set) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return ks_fail(ctx, KS_ERR_CUDA, "matvec (fixed point): cannot set %zu B shared memory: %s", smem, cudaGetErrorString(e));
-    smem_set[ctx->device & 15] = smem;
+    set = smem;
   }
-  KS_LAUNCH(ctx, (mv_q4k_fx_kernel), grid, FXM_THREADS, smem, a);
+  KS_LAUNCH(ctx, kern, grid, FXM_THREADS, smem, a);
   return ks_after_launch(ctx, "matvec_q4k_fx");
 }
