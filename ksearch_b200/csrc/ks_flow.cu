@@ -1183,6 +1183,8 @@ void ks_flow_destroy(ks_flow* mg) {
 // the launch-per-op path), a negative code on a CUDA failure.
 int ks_flow_create(ks_ctx* ctx, const ks_mega_desc* d, const ks_mega_layer* layers, ks_flow** out) {
   *out = nullptr;
+  for (int l = 0; l < d->n_layers; l++)
+    if (layers[l].window) return KS_OK;
   const unsigned H = d->hidden, F = d->ffn, hd = d->hd, nq = d->n_q, nkv = d->n_kv;
   const unsigned qn = nq * hd, kvn = nkv * hd;
   if (H % 256u || F % 256u || qn % 256u) return KS_OK;

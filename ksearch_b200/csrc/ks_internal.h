@@ -207,6 +207,7 @@ struct ks_mega_layer {
   const void *wq, *wk, *wv, *wo, *wgate, *wup, *wdown;  // Q4_K
   const void *attn_norm, *q_norm, *k_norm, *post_attn_norm, *ffn_norm, *post_ffw_norm;  // f32
   uint8_t *kv_k, *kv_v;  // this slot's cache rows [max_seq, n_kv, hd] Q4_0
+  int window;            // positions the layer attends to, 0: all
 };
 struct ks_mega_desc {
   int n_layers;

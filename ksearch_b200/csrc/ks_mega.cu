@@ -1,4 +1,4 @@
-// One persistent kernel for all layers of a decode token (single slot, f32 activations).
+// One persistent kernel for all layers of a decode token (single slot; f32 inside whatever the model's activation dtype).
 //
 // The op order is forward_token's (crates/ksearch_gemma/src/gemma_prim.rs:923-1197) for dense,
 // KV-owning layers; what changes is WHERE the boundaries between ops are.  On B200 a token is a
@@ -45,6 +45,7 @@ struct MegaLayer {          // per-layer pointers, copied to shared memory when 
   const uint8_t* W[7];      // wq, wk, wv, wo, wgate, wup, wdown (Q4_K)
   const float* norm[6];     // attn_norm, q_norm, k_norm, post_attn_norm, ffn_norm, post_ffw_norm
   uint8_t *kv_k, *kv_v;     // this slot's cache rows [max_seq, n_kv, hd] Q4_0
+  size_t window;            // positions the layer attends to (0: all), gemma_prim.rs:1009-1016
 };
 
 struct MegaArgs {
@@ -753,11 +754,11 @@ __device__ __forceinline__ void mg_attention(const MegaArgs& a, const MegaLayer&
   if (blockIdx.x >= a.n_q * NSMAX) return;
   const unsigned head = blockIdx.x / NSMAX, split = blockIdx.x % NSMAX;
   const unsigned G = a.n_q / a.n_kv, kvh = head / G;
-  const unsigned pos = (unsigned)a.pos[0], tlen = pos + 1;
+  const unsigned pos = (unsigned)a.pos[0], win = (unsigned)L.window, first = win && pos + 1u > win ? pos + 1u - win : 0u, tlen = pos + 1u - first;
   const unsigned NS = mg_active_splits(tlen, NSMAX);
   if (split >= NS) return;
   const unsigned chunk = (tlen + NS - 1) / NS;
-  const unsigned p0 = split * chunk, p1 = min(p0 + chunk, tlen);
+  const unsigned p0 = first + split * chunk, p1 = min(p0 + chunk, pos + 1u);
   const bool owner = pos >= p0 && pos < p1;  // the split that holds the newest position
   float* part = reinterpret_cast<float*>(sm);     // [8][HD + 2]
   uint8_t* skrow = reinterpret_cast<uint8_t*>(part + 8 * (HD + 2));
@@ -1445,6 +1446,7 @@ int ks_mega_create(ks_ctx* ctx, const ks_mega_desc* d, const ks_mega_layer* laye
     o.W[4] = (const uint8_t*)L.wgate; o.W[5] = (const uint8_t*)L.wup; o.W[6] = (const uint8_t*)L.wdown;
     o.norm[0] = (const float*)L.attn_norm; o.norm[1] = (const float*)L.q_norm; o.norm[2] = (const float*)L.k_norm;
     o.norm[3] = (const float*)L.post_attn_norm; o.norm[4] = (const float*)L.ffn_norm; o.norm[5] = (const float*)L.post_ffw_norm;
+    o.window = (size_t)L.window;
     o.kv_k = L.kv_k; o.kv_v = L.kv_v;
   }
 

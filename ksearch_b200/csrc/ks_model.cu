@@ -103,6 +103,9 @@ struct Tensor {
 struct Layer {
   Tensor wq, wk, wv, wo, wgate, wup, wdown;
   Tensor attn_norm, q_norm, k_norm, post_attn_norm, ffn_norm, post_ffw_norm;
+  // the norm weights in f32, for the paths that compute in f32 whatever the activation dtype: the tensors themselves, or
+  // (f16 models) copies that every upload refreshes
+  float *attn32, *q32, *k32, *post_attn32, *ffn32, *post_ffw32;
 };
 
 }  // namespace
@@ -112,6 +115,9 @@ struct ks_model {
   ks_model_config cfg{};
   std::vector<Layer> layers;
   Tensor token_embd, output_norm;
+  float* output32 = nullptr;
+  std::map<const Tensor*, float*> norm32;  // f16 models: where a norm tensor's f32 copy lives
+  float* step32 = nullptr;                 // f16 models: [n_slots][3][hidden] f32 vectors of the persistent decode kernel
   std::map<std::string, Tensor*> by_name;
   void* arena = nullptr;  // all weights, one allocation
   size_t arena_bytes = 0;
@@ -167,9 +173,10 @@ struct ks_model {
   float* cmeta_swa = nullptr;
   float* cattn_tmp = nullptr;
   int chunk = 1;  // tokens per prompt chunk: as many as the matvec kernels can stage side by side (<= KS_PREFILL_CHUNK)
-  // rows per pass through the tensor-core GEMM (0: not available, activations are not f32) and its scratch: the split
+  // rows per pass through the tensor-core GEMM (0: not available) and its scratch: the split
   // operand image, the k-split partials
   int gemm_chunk = 0;
+  int prompt_chunk = 1;  // prompt rows up to which the batch matvec takes them although the GEMM could
   void* gemm_xt = nullptr;
   float* gemm_p0 = nullptr;
 };
@@ -352,7 +359,7 @@ int enqueue_forward_gemm(ks_model* m, const Lane& L_, int n, bool want_logits) {
   const int att_splits = att_splits_for(m, n), chunk_splits = ks_sdpa_chunk_splits(c, n, nq, nkv, (size_t)g.max_seq, m->n_splits);
   if ((rc = lane_begin(m, L_, n))) return rc;
   if ((rc = ks_launch_copy_scale_indexed(c, H, n, sqrtf((float)H), (ks_dtype)g.embd_dtype, m->token_embd.dptr, L_.tok_in, act, x))) return rc;
-  if ((rc = ks_launch_rmsnorm(c, H, n, g.eps, act, x, m->layers[0].attn_norm.dptr, nullptr, 0, 0.f, x2))) return rc;
+  if ((rc = ks_launch_rmsnorm(c, H, n, g.eps, act, x, m->layers[0].attn32, nullptr, 0, 0.f, x2))) return rc;
   if ((rc = ks_launch_gemm_split(c, KS_Q4K, (const float*)x2, H, n, H, m->gemm_xt))) return rc;
   // From here on the normed rows exist only as the image the next GEMM reads: the sums of the o-proj and
   // down-proj partials go straight through the residual update and the next norm into that image.
@@ -371,7 +378,7 @@ int enqueue_forward_gemm(ks_model* m, const Lane& L_, int n, bool want_logits) {
     }
     uint8_t* kk = m->kv_k[l] + L_.kv_off;
     uint8_t* kv = m->kv_v[l] + L_.kv_off;
-    if ((rc = ks_launch_per_head_qkv_q40(c, nq, nkv, hd, n, g.eps, act, q, L.q_norm.dptr, m->rope, k, L.k_norm.dptr, v, q,
+    if ((rc = ks_launch_per_head_qkv_q40(c, nq, nkv, hd, n, g.eps, act, q, L.q32, m->rope, k, L.k32, v, q,
                                          kk, kv, L_.pos, L_.kv_stride)))
       return rc;
     if (L_.chunk_base && n >= KS_CHUNK_ATT_MIN && ks_sdpa_chunk_covers(nq, nkv, hd, kk, kv)) {  // the rows of a chunk share their context
@@ -387,8 +394,8 @@ int enqueue_forward_gemm(ks_model* m, const Lane& L_, int n, bool want_logits) {
       const uint8_t* Ws[1] = {(const uint8_t*)L.wo.dptr};
       float* ys[1] = {nullptr};
       epi.next_dtype = KS_Q4K;
-      epi.w_post = (const float*)L.post_attn_norm.dptr;
-      epi.w_norm = (const float*)L.ffn_norm.dptr;
+      epi.w_post = L.post_attn32;
+      epi.w_norm = L.ffn32;
       if ((rc = ks_launch_gemm_segs(c, KS_Q4K, 1, Ws, &H, qn, m->gemm_xt, n, ys, &H, m->gemm_p0, KS_GEMM_NORM_SPLIT, &epi))) return rc;
     }
     {  // gate and up share the operand image; their partials meet in the GeGLU epilogue (lib.rs:953)
@@ -401,8 +408,8 @@ int enqueue_forward_gemm(ks_model* m, const Lane& L_, int n, bool want_logits) {
       const uint8_t* Ws[1] = {(const uint8_t*)L.wdown.dptr};
       float* ys[1] = {nullptr};
       epi.next_dtype = l + 1 < g.n_layers ? KS_Q4K : (ks_dtype)g.embd_dtype;
-      epi.w_post = (const float*)L.post_ffw_norm.dptr;
-      epi.w_norm = (const float*)((l + 1 < g.n_layers) ? m->layers[l + 1].attn_norm.dptr : m->output_norm.dptr);
+      epi.w_post = L.post_ffw32;
+      epi.w_norm = l + 1 < g.n_layers ? m->layers[l + 1].attn32 : m->output32;
       if ((rc = ks_launch_gemm_segs(c, KS_Q4K, 1, Ws, &H, F, m->gemm_xt, n, ys, &H, m->gemm_p0, KS_GEMM_NORM_SPLIT, &epi))) return rc;
     }
   }
@@ -496,37 +503,60 @@ int enqueue_forward_fused(ks_model* m, const Lane& L_, int n, bool want_logits) 
 
 int mega_reset(ks_ctx* c, const ks_model::Mega& mg) { return mg.bar ? ks_mega_reset(c, mg.bar) : ks_flow_reset(c, mg.flow); }
 
-// Rows that share one pass over the weights when `left` rows are waiting: what the batch matvec stages side by
-// side, or, for more rows than that, a tensor-core GEMM chunk.
-int pass_rows(const ks_model* m, int left) { return left > m->chunk && m->gemm_chunk ? m->gemm_chunk : m->chunk; }
+// Rows of a decode step that share one pass over the weights when `left` rows are waiting: what the batch matvec stages side
+// by side, or, for more rows than that, a tensor-core GEMM chunk (f32 models: its logits are f32).
+int pass_rows(const ks_model* m, int left) { return left > m->chunk && m->gemm_chunk && m->cfg.act == KS_F32 ? m->gemm_chunk : m->chunk; }
+// The same for prompt rows, which leave no logits: both activation dtypes.
+bool prompt_gemm(const ks_model* m, int left) { return m->gemm_chunk && left > m->prompt_chunk; }
+int prompt_rows(const ks_model* m, int left) {
+  const int most = prompt_gemm(m, left) ? m->gemm_chunk : m->chunk;
+  return left < most ? left : most;
+}
+
+__global__ void widen_kernel(const __half* src, float* dst, unsigned n) {
+  ks_pdl_entry();
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) dst[i] = __half2float(src[i]);
+}
+__global__ void narrow_kernel(const float* a, const float* b, __half* oa, __half* ob, unsigned n) {
+  ks_pdl_entry();
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) {
+    oa[i] = __float2half_rn(a[i]);
+    ob[i] = __float2half_rn(b[i]);
+  }
+}
 
 // One slot's token with every layer inside one persistent kernel; embedding before, head after.
 int enqueue_forward_mega(ks_model* m, const ks_model::Mega& mg, int first, int src, bool want_logits) {
   ks_ctx* c = m->ctx;
   const ks_model_config& g = m->cfg;
+  const ks_dtype act = (ks_dtype)g.act;
   const size_t H = g.hidden;
-  float* cur = (float*)m->x + (size_t)first * H;
-  float* yb = (float*)m->x2 + (size_t)first * H;
-  float* xn = (float*)m->xn + (size_t)first * H;
-  float* logits = (float*)m->logits + (size_t)first * g.vocab;
-  const float* tok_in = src == 2 ? m->host_ids + first : m->tok + (size_t)src * g.n_slots + first;
-  float* tok_out = m->tok + (size_t)(src == 2 ? 1 : src ^ 1) * g.n_slots + first;
-  int* pos = m->pos + first;
+  const Lane L = slot_lane(m, first, src);
   int rc;
-  if ((rc = ks_launch_copy_scale_indexed(c, H, 1, sqrtf((float)H), (ks_dtype)g.embd_dtype, m->token_embd.dptr, tok_in, KS_F32, cur))) return rc;
+  float* x32 = m->step32 ? m->step32 + (size_t)first * 3 * H : (float*)L.x;
+  if ((rc = ks_launch_copy_scale_indexed(c, H, 1, sqrtf((float)H), (ks_dtype)g.embd_dtype, m->token_embd.dptr, L.tok_in, KS_F32, x32))) return rc;
   if ((rc = mg.bar ? ks_mega_launch(c, mg.bar) : ks_flow_launch(c, mg.flow))) return rc;
-  KS_LAUNCH(c, (end_token_kernel), 1, 32, 0, 1, pos);
+  KS_LAUNCH(c, (end_token_kernel), 1, 32, 0, 1, L.pos);
   if ((rc = ks_after_launch(c, "end_token"))) return rc;
   if (!want_logits) return KS_OK;
-  float* res = mg.bar ? ks_mega_residual(mg.bar) : ks_flow_residual(mg.flow);
-  if ((rc = ks_launch_rmsnorm_add_then_rmsnorm(c, H, 1, g.eps, KS_F32, yb, m->layers[g.n_layers - 1].post_ffw_norm.dptr, res,
-                                               m->output_norm.dptr, res, xn)))
+  void* res = mg.bar ? ks_mega_residual(mg.bar) : ks_flow_residual(mg.flow);
+  void* yb = m->step32 ? (void*)(x32 + 2 * H) : (void*)L.x2;
+  if (act == KS_F16) {  // the head runs in the model's activation dtype
+    KS_LAUNCH(c, (narrow_kernel), (unsigned)((H + 255) / 256), 256, 0, (const float*)res, (const float*)yb, (__half*)L.x, (__half*)L.x2, (unsigned)H);
+    if ((rc = ks_after_launch(c, "narrow"))) return rc;
+    res = L.x;
+    yb = L.x2;
+  }
+  if ((rc = ks_launch_rmsnorm_add_then_rmsnorm(c, H, 1, g.eps, act, yb, m->layers[g.n_layers - 1].post_ffw_norm.dptr, res,
+                                               m->output_norm.dptr, res, L.xn)))
     return rc;
-  ks_mv_seg sh{(const uint8_t*)m->token_embd.dptr, logits, (unsigned)g.vocab};
-  if ((rc = ks_launch_matvec(c, (ks_dtype)g.embd_dtype, &sh, 1, KS_EPI_PLAIN, H, KS_F32, xn, 1, nullptr))) return rc;
-  if ((rc = ks_launch_softcap_argmax(c, g.vocab, g.softcap, KS_F32, logits, tok_out))) return rc;
-  KS_LAUNCH(c, (collect_kernel), 1, 32, 0, 1, (const float*)tok_out, (const unsigned*)c->ws + KS_WS_ERR_WORD,
-            m->ret + (size_t)first * (g.n_slots + 1), (float*)m->host_ret, (int)g.n_slots);
+  ks_mv_seg sh{(const uint8_t*)m->token_embd.dptr, L.logits, (unsigned)g.vocab};
+  if ((rc = ks_launch_matvec(c, (ks_dtype)g.embd_dtype, &sh, 1, KS_EPI_PLAIN, H, act, L.xn, 1, nullptr))) return rc;
+  if ((rc = ks_launch_softcap_argmax(c, g.vocab, g.softcap, act, L.logits, L.tok_out))) return rc;
+  KS_LAUNCH(c, (collect_kernel), 1, 32, 0, 1, (const float*)L.tok_out, (const unsigned*)c->ws + KS_WS_ERR_WORD, L.ret, (float*)m->host_ret,
+            (int)g.n_slots);
   return ks_after_launch(c, "collect");
 }
 
@@ -547,9 +577,9 @@ int get_mega(ks_model* m, int first, ks_model::Mega* out) {
   d.eps = g.eps; d.attn_scale = g.attn_scale;
   d.rope = m->rope;
   d.pos = m->pos + first;
-  d.x_a = (float*)m->x + (size_t)first * H;
-  d.x_b = (float*)m->xb + (size_t)first * H;
-  d.yb = (float*)m->x2 + (size_t)first * H;
+  d.x_a = m->step32 ? m->step32 + (size_t)first * 3 * H : (float*)m->x + (size_t)first * H;
+  d.x_b = m->step32 ? d.x_a + H : (float*)m->xb + (size_t)first * H;
+  d.yb = m->step32 ? d.x_a + 2 * H : (float*)m->x2 + (size_t)first * H;
   d.q = (float*)m->q + (size_t)first * qn;
   d.k = (float*)m->k + (size_t)first * kvn;
   d.v = (float*)m->v + (size_t)first * kvn;
@@ -563,10 +593,11 @@ int get_mega(ks_model* m, int first, ks_model::Mega* out) {
     ks_mega_layer& o = ls[l];
     o.wq = L.wq.dptr; o.wk = L.wk.dptr; o.wv = L.wv.dptr; o.wo = L.wo.dptr;
     o.wgate = L.wgate.dptr; o.wup = L.wup.dptr; o.wdown = L.wdown.dptr;
-    o.attn_norm = L.attn_norm.dptr; o.q_norm = L.q_norm.dptr; o.k_norm = L.k_norm.dptr;
-    o.post_attn_norm = L.post_attn_norm.dptr; o.ffn_norm = L.ffn_norm.dptr; o.post_ffw_norm = L.post_ffw_norm.dptr;
+    o.attn_norm = L.attn32; o.q_norm = L.q32; o.k_norm = L.k32;
+    o.post_attn_norm = L.post_attn32; o.ffn_norm = L.ffn32; o.post_ffw_norm = L.post_ffw32;
     o.kv_k = m->kv_k[l] + (size_t)first * m->slot_stride;
     o.kv_v = m->kv_v[l] + (size_t)first * m->slot_stride;
+    o.window = has_window(g) && ((g.swa_layers >> l) & 1ull) ? g.sliding_window : 0;
   }
   ks_model::Mega mg;
   int rc = m->decode_kernel == 2 ? ks_flow_create(m->ctx, &d, ls.data(), &mg.flow) : ks_mega_create(m->ctx, &d, ls.data(), &mg.bar);
@@ -583,7 +614,7 @@ int run_forward(ks_model* m, int first, int n, int src, bool want_logits) {
   auto it = m->graphs.find(key);
   if (it == m->graphs.end()) {
     ks_model::Mega mg;
-    if (n == 1) {  // (with sliding-window layers get_mega leaves mg empty: the launch-per-op path runs)
+    if (n == 1) {
       int rcm = get_mega(m, first, &mg);
       if (rcm) return rcm;
     }
@@ -618,7 +649,7 @@ int run_forward(ks_model* m, int first, int n, int src, bool want_logits) {
 }
 
 // A chunk of n prompt tokens of one slot (ids already in m->ctok) through every layer, no head.
-int run_prefill_chunk(ks_model* m, int slot, int n) {
+int run_prefill_chunk(ks_model* m, int slot, int n, bool gemm) {
   ks_ctx* c = m->ctx;
   const uint64_t key = (1ull << 63) | ((uint64_t)slot << 32) | ((uint64_t)n << 8);
   auto it = m->graphs.find(key);
@@ -627,9 +658,9 @@ int run_prefill_chunk(ks_model* m, int slot, int n) {
     KS_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     const uint64_t before = c->launches;
     const Lane lane = chunk_lane(m, slot);
-    int rc = n > m->chunk ? enqueue_forward_gemm(m, lane, n, false)
-             : m->fused   ? enqueue_forward_fused(m, lane, n, false)
-                          : enqueue_forward(m, lane, n, false);
+    int rc = gemm       ? enqueue_forward_gemm(m, lane, n, false)
+             : m->fused ? enqueue_forward_fused(m, lane, n, false)
+                        : enqueue_forward(m, lane, n, false);
     cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
     c->launches = before;
     if (rc) {
@@ -716,6 +747,28 @@ ks_model* ks_model_create(ks_ctx* ctx, const ks_model_config* cfg) {
   if (ok)
     for (auto& kv : m->by_name) kv.second->dptr = (char*)m->arena + (size_t)kv.second->dptr;
 
+  if (ok) {
+    const size_t per_layer = 4 * H + 2 * (size_t)g.hd;
+    float* at = nullptr;
+    if (g.act != KS_F32) ok = dev_alloc(m, (void**)&at, ((size_t)g.n_layers * per_layer + H) * sizeof(float)) == KS_OK &&
+                              dev_alloc(m, (void**)&m->step32, (size_t)g.n_slots * 3 * H * sizeof(float)) == KS_OK;
+    auto f32 = [&](const Tensor& t, size_t n) {
+      if (!at) return (float*)t.dptr;
+      float* p = at;
+      m->norm32[&t] = p;
+      at += n;
+      return p;
+    };
+    for (Layer& L : m->layers) {
+      L.attn32 = f32(L.attn_norm, H);
+      L.q32 = f32(L.q_norm, g.hd);
+      L.k32 = f32(L.k_norm, g.hd);
+      L.post_attn32 = f32(L.post_attn_norm, H);
+      L.ffn32 = f32(L.ffn_norm, H);
+      L.post_ffw32 = f32(L.post_ffw_norm, H);
+    }
+    m->output32 = f32(m->output_norm, H);
+  }
   const size_t rowb = (size_t)g.hd / 32 * KS_Q40_BLOCK_BYTES;
   m->slot_stride = (size_t)g.max_seq * g.n_kv * rowb;
   m->kv_k.resize(g.n_layers);
@@ -733,8 +786,7 @@ ks_model* ks_model_create(ks_ctx* ctx, const ks_model_config* cfg) {
   // launch per op (the path every multi-slot step takes anyway), 1 = the kernel whose phases meet at grid
   // barriers (default), 2 = the kernel whose blocks exchange tagged words instead of meeting.
   const char* dk = getenv("KSEARCH_DECODE_KERNEL");
-  // (the persistent kernels attend to the whole context: a model with sliding-window layers takes one launch per op)
-  m->use_mega = m->fused && g.act == KS_F32 && !(dk && dk[0] == '0') && !has_window(g);
+  m->use_mega = m->fused && !(dk && dk[0] == '0');
   m->decode_kernel = dk && dk[0] == '2' ? 2 : 1;
   // Two slots step faster as two persistent-kernel passes than side by side through one launch per op (same
   // measurement: E2B 938 against 1074 us, E4B 1157 against 1378); from three slots on the GEMM path wins.
@@ -757,8 +809,9 @@ ks_model* ks_model_create(ks_ctx* ctx, const ks_model_config* cfg) {
     if (qn > maxcols) maxcols = qn;
     m->chunk = KS_PREFILL_CHUNK;
     while (m->chunk > 1 && (size_t)m->chunk * (maxcols / 64) * 280 + (64u << 10) > ctx->smem_optin) m->chunk--;
-    // f32 activations and block-aligned columns: larger batches go through the tensor-core GEMM
-    if (g.act == KS_F32 && H % 256 == 0 && F % 256 == 0 && qn % 256 == 0 && !getenv("KSEARCH_NO_GEMM")) {
+    // block-aligned columns: larger batches go through the tensor-core GEMM, which computes in f32 (a chunk of an f16 model
+    // too: its rows meet f16 vectors nowhere)
+    if (H % 256 == 0 && F % 256 == 0 && qn % 256 == 0 && !getenv("KSEARCH_NO_GEMM")) {
       const int G = KS_GEMM_CHUNK;
       m->gemm_chunk = G;
       // one launch each: q|k|v, o, gate|up, down, head
@@ -787,14 +840,16 @@ ks_model* ks_model_create(ks_ctx* ctx, const ks_model_config* cfg) {
         // KSEARCH_BATCH_ROWS moves the limit (measurement).
         int limit = 2;
         if (const char* br = getenv("KSEARCH_BATCH_ROWS")) limit = atoi(br) < 1 ? 1 : atoi(br);
-        if (limit < m->chunk) m->chunk = limit;
+        m->prompt_chunk = limit < m->chunk ? limit : m->chunk;
+        if (g.act == KS_F32) m->chunk = m->prompt_chunk;
       }
     }
     const size_t C = m->gemm_chunk > KS_PREFILL_CHUNK ? m->gemm_chunk : KS_PREFILL_CHUNK;
-    ok = ok && dev_alloc(m, &m->cx, C * H * ab) == KS_OK && dev_alloc(m, &m->cxb, C * H * ab) == KS_OK &&
-         dev_alloc(m, &m->cx2, C * H * ab) == KS_OK && dev_alloc(m, &m->cq, C * qn * ab) == KS_OK &&
-         dev_alloc(m, &m->ck, C * kvn * ab) == KS_OK && dev_alloc(m, &m->cv, C * kvn * ab) == KS_OK &&
-         dev_alloc(m, &m->co, C * qn * ab) == KS_OK && dev_alloc(m, &m->cff, C * F * ab) == KS_OK &&
+    const size_t cb = m->gemm_chunk ? sizeof(float) : ab;  // the batch matvec's rows fit as well
+    ok = ok && dev_alloc(m, &m->cx, C * H * cb) == KS_OK && dev_alloc(m, &m->cxb, C * H * cb) == KS_OK &&
+         dev_alloc(m, &m->cx2, C * H * cb) == KS_OK && dev_alloc(m, &m->cq, C * qn * cb) == KS_OK &&
+         dev_alloc(m, &m->ck, C * kvn * cb) == KS_OK && dev_alloc(m, &m->cv, C * kvn * cb) == KS_OK &&
+         dev_alloc(m, &m->co, C * qn * cb) == KS_OK && dev_alloc(m, &m->cff, C * F * cb) == KS_OK &&
          dev_alloc(m, (void**)&m->ctok, C * sizeof(float)) == KS_OK && dev_alloc(m, (void**)&m->cpos, C * sizeof(int)) == KS_OK &&
          dev_alloc(m, (void**)&m->cmeta, C * 4 * sizeof(float)) == KS_OK &&
          (!has_window(g) || dev_alloc(m, (void**)&m->cmeta_swa, C * 4 * sizeof(float)) == KS_OK);
@@ -898,6 +953,13 @@ int ks_model_upload_tensor(ks_model* m, const char* name, const void* host, size
   KS_REQUIRE(c, it != m->by_name.end(), "missing tensor %s", name);
   KS_REQUIRE(c, bytes == it->second->bytes, "tensor %s: got %zu bytes, expected %zu", name, bytes, it->second->bytes);
   KS_CUDA(c, cudaMemcpyAsync(it->second->dptr, host, bytes, cudaMemcpyHostToDevice, c->stream));
+  const auto wide = m->norm32.find(it->second);
+  if (wide != m->norm32.end()) {
+    const unsigned n = (unsigned)(bytes / sizeof(__half));
+    KS_LAUNCH(c, (widen_kernel), (n + 255u) / 256u, 256, 0, (const __half*)it->second->dptr, wide->second, n);
+    const int rc = ks_after_launch(c, "widen");
+    if (rc) return rc;
+  }
   KS_CUDA(c, cudaStreamSynchronize(c->stream));
   it->second->set = true;
   return KS_OK;
@@ -1158,15 +1220,14 @@ int ks_model_prefill(ks_model* m, int slot, const int* tokens, int n_tokens) {
   if (m->seq_len[slot] + n_tokens > m->cfg.max_seq) return ks_fail(c, KS_ERR_STATE, "max_seq exceeded");
   float* stage = m->host_tok + m->host_tok_n - 16 - KS_STAGE_IDS;
   for (int t0 = 0; t0 < n_tokens;) {
-    const int per_pass = pass_rows(m, n_tokens - t0);
-    const int n = n_tokens - t0 < per_pass ? n_tokens - t0 : per_pass;
+    const int n = prompt_rows(m, n_tokens - t0);
     KS_CUDA(c, cudaStreamSynchronize(c->stream));  // the staging words may still be in flight
     for (int t = 0; t < n; t++) {
       KS_REQUIRE(c, tokens[t0 + t] >= 0 && tokens[t0 + t] < m->cfg.vocab, "token id %d outside the vocabulary", tokens[t0 + t]);
       stage[t] = (float)tokens[t0 + t];
     }
     KS_CUDA(c, cudaMemcpyAsync(m->ctok, stage, n * sizeof(float), cudaMemcpyHostToDevice, c->stream));
-    if ((rc = run_prefill_chunk(m, slot, n))) return rc;
+    if ((rc = run_prefill_chunk(m, slot, n, prompt_gemm(m, n)))) return rc;
     m->seq_len[slot] += n;
     t0 += n;
   }
@@ -1352,6 +1413,7 @@ const void* ks_model_debug_ptr(const ks_model* m, int which, int slot) {
   const size_t ab = ks_act_bytes((ks_dtype)m->cfg.act);
   if (which == 0) return (const char*)m->x + (size_t)slot * m->cfg.hidden * ab;
   if (which == 1) return (const char*)m->logits + (size_t)slot * m->cfg.vocab * ab;
+  if (which == 2 && has_window(m->cfg)) return nullptr;  // stamps are read per full-attention layer; windowed models hand out none
   if (which == 2) {  // phase stamps of the persistent decode kernel, first and last block: [2][n_layers][5][8] int64
     auto it = m->mega.find(slot);  // (clock64 ticks from the barrier kernel, globaltimer ns from the dataflow one)
     if (it == m->mega.end() || !it->second) return nullptr;

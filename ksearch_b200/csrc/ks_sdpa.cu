@@ -320,255 +320,324 @@ __global__ void __launch_bounds__(1024) sdpa_reduce_kernel(unsigned hd, const fl
   }
 }
 
-// ---- the tiled form: positions across lanes for q.k, dims across lanes for p.v ------------------------------
-// One block of 256 threads per (split, KV head, slot) serves the query heads of the KV head (up to four; a group of
-// eight is two blocks).  The split's rows come
-// into shared memory 256 positions at a time (cp.async, 4 bytes per request, row stride ROWB + 4 bytes so that 32
-// lanes reading 32 different rows hit 32 different banks).
-//   scores   thread t owns position t of the tile: it walks its K row two Q4_0 blocks (nine words) at a time and
-//            multiplies the 64 nibbles against q of every head (q and the per-block 8 * sum(q) sit in shared memory,
-//            read as broadcasts) -- no shuffle, and the row is decoded once for all heads;
-//   softmax  warp g owns head g: tile maximum, rescale factor of what was gathered before, probabilities in place;
-//   values   lane L owns the dims of its nibbles (as in the per-row kernel above), the eight warps take positions
-//            round-robin, the probabilities are shared-memory broadcasts.
-// Per position and head this costs ~25 warp instructions where the per-row kernel needs ~70 (it pays five shuffles
-// and an exp chain per row and head).  Records and the merge kernel are the same.
-constexpr int kTP = 256;
-constexpr int kMinChunk = 128;
+// ---- the tensor-core form ------------------------------------------------------------------------------------
+// One block of eight warps per (split, group of up to four query heads of a KV head, slot).  Warps take tiles of 16 positions
+// round-robin and never wait for one another before the end; a warp's next tile is on its way (cp.async) meanwhile.  Per tile:
+//   scores   mma m16n8k16 with positions as rows and heads as columns.  A cached value is d (n - 8): the integers n - 8 come out
+//            of the packed words by one LOP3 and one HADD2 / HFMA2 per two values, in the order the words hold them (the dims of
+//            a k step are permuted alike in q); each query is split into two f16 terms, columns 0..3 and 4..7, so one
+//            instruction takes both; the integer product of a 32-dim block is multiplied by its d in f32.  q is scaled by a
+//            power of two per head, so nothing leaves the f16 range;
+//   values   dims as rows, positions as k, and p d(position, block) as columns, again as two f16 terms.  2^k brings the largest
+//            p d of the warp so far below 2^15; a tile with a larger d lowers k and rescales like a new maximum does.
+// What is dropped is below 2^-21 of the largest product.  No shuffle per position: six per tile for the running maximum.
+// About 700 warp instructions per 16 positions and four heads; the kernel this replaced (positions across threads, f32 FMAs)
+// took about 2900.  Bound by latency: a few tiles per warp, then two dependent launches.
+constexpr int kMmaWarps = 8;
+constexpr int kMmaTile = 16;
+constexpr int kMmaRing = 2;
+constexpr int kMinChunk = kMmaWarps * kMmaTile;  // positions of a split at least: one tile per warp
 
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-}
-
-template <int G, int HD>
-struct TileSmem {
-  static constexpr unsigned ROWB = (HD / 32) * KS_Q40_BLOCK_BYTES, RP = ROWB + 4, NW = ROWB / 4, NB = HD / 32;
-  static constexpr unsigned q_off = 0;                         // G * HD floats
-  static constexpr unsigned st_off = q_off + G * HD * 4;       // m[G], l[G], alpha[G]
-  static constexpr unsigned s_off = st_off + 3 * 8 * 4;        // G * kTP floats: scores, then probabilities
-  static constexpr unsigned k_off = s_off + G * kTP * 4;       // kTP rows of K, then of V
-  static constexpr unsigned v_off = k_off + kTP * RP;
-  static constexpr unsigned tiles = 2 * kTP * RP, merge = 8 * G * HD * 4;  // the warps' partial O reuse the tiles
-  static constexpr unsigned total = k_off + (tiles > merge ? tiles : merge);
+template <int HD>
+struct MmaSmem {
+  static constexpr unsigned NB = HD / 32, ROWB = NB * KS_Q40_BLOCK_BYTES, TILE = 2 * kMmaTile * ROWB;
+  static constexpr unsigned q_off = 0, p_off = q_off + NB * 32 * 16, st_off = p_off + kMmaWarps * kMmaTile * 16,
+                            ring_off = (st_off + kMmaWarps * 4 * 8 + 32 + 127) & ~127u;
+  static constexpr unsigned ring = kMmaWarps * kMmaRing * TILE, merge = kMmaWarps * 4 * HD * 4;
+  static constexpr unsigned total = ring_off + (ring > merge ? ring : merge);
 };
+__device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
+__device__ __forceinline__ __half2 bits_h2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
+__device__ __forceinline__ uint32_t low_nibbles(uint32_t w) {   // nibbles 0 of bytes 0 and 2 -> n - 8
+  return h2_bits(__hadd2(bits_h2((w & 0x000F000Fu) | 0x64006400u), __float2half2_rn(-1032.0f)));
+}
+__device__ __forceinline__ uint32_t high_nibbles(uint32_t w) {  // nibbles 1 of bytes 0 and 2 (1024 + 16 n) -> n - 8
+  return h2_bits(__hfma2(bits_h2((w & 0x00F000F0u) | 0x64006400u), __float2half2_rn(0.0625f), __float2half2_rn(-72.0f)));
+}
+__device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ float half_at(const unsigned char* p) { return __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short*>(p))); }
 
-template <int G, int HD, typename T>
-__global__ void __launch_bounds__(kTP, 2)
-sdpa_tile_kernel(unsigned n_q, unsigned n_kv, float scale, const T* q, const uint8_t* K, const uint8_t* V, size_t slot_stride,
-                 const float* meta, float* tmp, T* out, int n_splits) {
+template <int HD, typename T>
+__global__ void __launch_bounds__(kMmaWarps * 32, 2)
+sdpa_mma_kernel(unsigned n_q, unsigned n_kv, unsigned gb, float scale, const T* q, const uint8_t* K, const uint8_t* V, size_t slot_stride,
+                const float* meta, float* tmp, T* out, int n_splits) {
   ks_pdl_entry();
-  using S = TileSmem<G, HD>;
-  constexpr int DPL = HD / 32;
-  constexpr unsigned ROWB = S::ROWB, RP = S::RP, NW = S::NW, NB = S::NB;
-  extern __shared__ __align__(16) unsigned char smem[];
-  float* sq = reinterpret_cast<float*>(smem + S::q_off);
-  float* sst = reinterpret_cast<float*>(smem + S::st_off);
-  float* ss = reinterpret_cast<float*>(smem + S::s_off);
-  unsigned char* kt = smem + S::k_off;
-  unsigned char* vt = smem + S::v_off;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const unsigned hpk = n_q / n_kv, gpk = hpk / G;  // heads and blocks per KV head
-  const int split = blockIdx.x, kvh = blockIdx.y / gpk, slot = blockIdx.z;
-  const unsigned head0 = (unsigned)kvh * hpk + (blockIdx.y % gpk) * G;
+  using S = MmaSmem<HD>;
+  constexpr unsigned NB = S::NB, ROWB = S::ROWB;
+  extern __shared__ __align__(128) unsigned char smem[];
+  const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, g = lane >> 2, t = lane & 3u;
+  const unsigned hpk = n_q / n_kv, gpk = hpk / gb;  // heads and blocks per KV head
+  const unsigned split = blockIdx.x, kvh = blockIdx.y / gpk, slot = blockIdx.z;
+  const unsigned head0 = kvh * hpk + (blockIdx.y % gpk) * gb;
   const unsigned tlen = (unsigned)meta[slot * 4 + 0], start = (unsigned)meta[slot * 4 + 1];
   // a split never holds fewer than kMinChunk positions: on a short context the later splits are empty and their
   // blocks leave after writing an empty record, so a split count sized for the longest context costs little
   const unsigned chunk = max((tlen + n_splits - 1) / n_splits, (unsigned)kMinChunk);
   const unsigned p0 = split * chunk, p1 = min(p0 + chunk, tlen);
-  const uint8_t* Ks = K + (size_t)slot * slot_stride;
-  const uint8_t* Vs = V + (size_t)slot * slot_stride;
-
   if (p0 >= p1 && n_splits > 1) {  // nothing to do: the empty record (m = -1e30, l = 0) is all the merge needs
-    if (tid < G) {
+    if (tid < gb) {
       float* rec = tmp + (((size_t)slot * n_q + head0 + tid) * n_splits + split) * (HD + 2);
       rec[0] = kNegInit;
       rec[1] = 0.0f;
     }
     return;
   }
-  for (int i = tid; i < G * HD; i += kTP) sq[i] = ld_act<T>(q, ((size_t)slot * n_q + head0) * HD + i) * scale;
-  if (tid < 3 * 8) sst[tid] = tid < 8 ? kNegInit : 0.0f;
-  __syncthreads();
-  float o[G][DPL], c[G];
-#pragma unroll
-  for (int g = 0; g < G; g++) {
-    c[g] = 0.0f;
-#pragma unroll
-    for (int j = 0; j < DPL; j++) o[g][j] = 0.0f;
-  }
-  const uint32_t kt_s = (uint32_t)__cvta_generic_to_shared(kt), vt_s = (uint32_t)__cvta_generic_to_shared(vt);
+  const uint8_t* Ks = K + (size_t)slot * slot_stride + ((size_t)start * n_kv + kvh) * ROWB;
+  const uint8_t* Vs = V + (size_t)slot * slot_stride + ((size_t)start * n_kv + kvh) * ROWB;
+  const size_t rowstride = (size_t)n_kv * ROWB;
+  unsigned char* ring = smem + S::ring_off + warp * (kMmaRing * S::TILE);
+  const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring);
+  const unsigned n_tiles = p1 > p0 ? (p1 - p0 + kMmaTile - 1) / kMmaTile : 0u;
 
-  for (unsigned t0 = p0; t0 < p1; t0 += kTP) {
-    const unsigned n = min((unsigned)kTP, p1 - t0);
-    __syncthreads();  // the previous tile is used up
-    for (unsigned r = warp; r < n; r += kTP / 32) {  // a warp per row: lane = word, the first lanes take the tail
-      const size_t src = ((size_t)(start + t0 + r) * n_kv + kvh) * ROWB + 4u * lane;
-      const uint32_t dst = r * RP + 4u * lane;
-      if ((unsigned)lane < NW) {
-        cp_async4(kt_s + dst, Ks + src);
-        cp_async4(vt_s + dst, Vs + src);
-      }
-      if (NW > 32 && (unsigned)lane + 32u < NW) {
-        cp_async4(kt_s + dst + 128u, Ks + src + 128u);
-        cp_async4(vt_s + dst + 128u, Vs + src + 128u);
+  auto fetch = [&](unsigned i, unsigned stage) {  // this warp's i-th tile (an empty group past the end; rows past the split repeat its last)
+    const unsigned tile = warp + i * kMmaWarps;
+    if (tile < n_tiles) {
+      constexpr unsigned CH = HD == 256 ? 16u : 8u, PER = ROWB / CH;  // rows of 144 (72) bytes
+      for (unsigned c = lane; c < kMmaTile * PER; c += 32u) {
+        const unsigned r = c / PER, o = (c - r * PER) * CH;
+        const size_t src = (size_t)min(p0 + tile * kMmaTile + r, p1 - 1u) * rowstride + o;
+        const uint32_t dst = ring_s + stage * S::TILE + r * ROWB + o;
+        if (CH == 16u) {
+          cp_async16(dst, Ks + src);
+          cp_async16(dst + kMmaTile * ROWB, Vs + src);
+        } else {
+          cp_async8(dst, Ks + src);
+          cp_async8(dst + kMmaTile * ROWB, Vs + src);
+        }
       }
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
-    // ---- scores: thread = position; a short tile spreads the block pairs of a row over 2 or 4 neighbouring lanes
-    const unsigned wshift = (n * 4u <= (unsigned)kTP && NB >= 8u) ? 2u : (n * 2u <= (unsigned)kTP && NB >= 4u) ? 1u : 0u;
-    const unsigned pos_t = (unsigned)tid >> wshift, part = (unsigned)tid & ((1u << wshift) - 1u);
-    {
-      const uint32_t* kr = reinterpret_cast<const uint32_t*>(kt + (size_t)(pos_t < n ? pos_t : 0u) * RP);
-      float sc[G];
+  };
+  fetch(0, 0);
+
+  // ---- q: per head a power-of-two scale, then the B fragments of every block in the order the lanes read them
+  float* qscale = reinterpret_cast<float*>(smem + S::st_off + kMmaWarps * 4 * 8);  // [0..4) down, [4..8) up
+  if (warp < gb) {
+    float m = 0.0f;
+    for (unsigned i = lane; i < HD; i += 32u) m = fmaxf(m, fabsf(ld_act<T>(q, ((size_t)slot * n_q + head0 + warp) * HD + i)));
 #pragma unroll
-      for (int g = 0; g < G; g++) sc[g] = 0.0f;
-#pragma unroll 1
-      for (unsigned pb = part; pb < NB / 2; pb += 1u << wshift) {
-        uint32_t w[9];
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane == 0) {
+      int e = 0;
+      if (m > 0.0f && m < 3.0e38f) {
+        e = (int)((__float_as_uint(m) >> 23) & 0xFFu) - 127 - 14;
+        e = e < -100 ? -100 : e;
+      }
+      qscale[warp] = __uint_as_float((unsigned)(127 - e) << 23);
+      qscale[4 + warp] = __uint_as_float((unsigned)(127 + e) << 23);
+    }
+  } else if (warp < 4) {
+    if (lane == 0) qscale[warp] = qscale[4 + warp] = 0.0f;
+  }
+  __syncthreads();
+  for (unsigned i = tid; i < NB * 32u; i += kMmaWarps * 32) {
+    const unsigned b = i >> 5, l = i & 31u, n = l >> 2, lt = l & 3u, h = n & 3u;
+    uint32_t w[4] = {0u, 0u, 0u, 0u};
+    if (h < gb) {
+      const size_t at = ((size_t)slot * n_q + head0 + h) * HD + 32u * b + 4u * lt;
+      const float dn = qscale[h];
 #pragma unroll
-        for (int i = 0; i < 9; i++) w[i] = kr[9 * pb + i];
-        // two blocks of 18 bytes: [d0 | 16 nibble bytes][d1 | 16 nibble bytes]; the first one's bytes straddle the words
-        uint32_t qw[2][4];
+      for (int half = 0; half < 2; half++)
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-          qw[0][i] = __funnelshift_r(w[i], w[i + 1], 16);
-          qw[1][i] = w[5 + i];
+        for (int k = 0; k < 2; k++) {
+          const float x0 = ld_act<T>(q, at + 16u * half + k) * dn, x1 = ld_act<T>(q, at + 16u * half + k + 2u) * dn;
+          const __half2 hh = __floats2half2_rn(x0, x1);
+          const float2 hf = __half22float2(hh);
+          w[2 * half + k] = n < 4u ? h2_bits(hh) : h2_bits(__floats2half2_rn(x0 - hf.x, x1 - hf.y));
         }
-        const float d01[2] = {__half2float(__ushort_as_half((unsigned short)(w[0] & 0xFFFFu))),
-                              __half2float(__ushort_as_half((unsigned short)(w[4] >> 16)))};
+    }
+    reinterpret_cast<uint4*>(smem + S::q_off)[i] = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+  __syncthreads();
+  const uint4* qf = reinterpret_cast<const uint4*>(smem + S::q_off) + lane;
+  float* pw = reinterpret_cast<float*>(smem + S::p_off) + warp * (kMmaTile * 4);
+  const unsigned ha = 2u * (t & 1u);                       // this lane's two heads (columns 2t, 2t + 1 and their other halves)
+  const float sa = qscale[4 + ha] * scale, sb = qscale[5 + ha] * scale;
+  const bool is_lo = g >= 4u;
+
+  float o[HD / 16][4];
 #pragma unroll
-        for (int b = 0; b < 2; b++) {
-          float lo[16], hi[16];  // dims 0..15 and 16..31 of the block
+  for (int i = 0; i < HD / 16; i++)
 #pragma unroll
-          for (int i = 0; i < 4; i++)
+    for (int e = 0; e < 4; e++) o[i][e] = 0.0f;
+  float m0 = kNegInit, m1 = kNegInit, l0 = 0.0f, l1 = 0.0f;
+  int kx = 29;  // values carry 2^kx
+  unsigned stage = 0;
+  for (unsigned i = 0; warp + i * kMmaWarps < n_tiles; i++) {
+    fetch(i + 1, stage ^ 1u);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();
+    const unsigned char* kt = ring + stage * S::TILE;
+    const unsigned char* vt = kt + kMmaTile * ROWB;
+    // ---- scores: rows g and g + 8 of the tile, columns 2t, 2t + 1
+    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    const unsigned char* ra = kt + g * ROWB;
+    const unsigned char* rb = ra + 8u * ROWB;
+#pragma unroll 2
+    for (unsigned pr = 0; pr < NB / 2; pr++) {  // two blocks, 36 bytes: [d0 | 16 bytes][d1 | 16 bytes]; the first one's bytes straddle words
+      const uint32_t* wa = reinterpret_cast<const uint32_t*>(ra + 36u * pr) + t;
+      const uint32_t* wb = reinterpret_cast<const uint32_t*>(rb + 36u * pr) + t;
+      const uint32_t a[2] = {__funnelshift_r(wa[0], wa[1], 16), wa[5]}, b[2] = {__funnelshift_r(wb[0], wb[1], 16), wb[5]};
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-              // 2^23 + n as a float, minus (2^23 + 8): the signed nibble without an int-to-float conversion
-              lo[4 * i + k] = __uint_as_float(((qw[b][i] >> (8 * k)) & 0xFu) | 0x4B000000u) - 8388616.0f;
-              hi[4 * i + k] = __uint_as_float(((qw[b][i] >> (8 * k + 4)) & 0xFu) | 0x4B000000u) - 8388616.0f;
-            }
-          const unsigned blk = 2 * pb + b;
-#pragma unroll
-          for (int g = 0; g < G; g++) {
-            const float4* q4 = reinterpret_cast<const float4*>(sq + (size_t)g * HD + blk * 32);
-            float a = 0.0f;
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-              const float4 ql = q4[i], qh = q4[4 + i];
-              a = fmaf(ql.x, lo[4 * i], a); a = fmaf(ql.y, lo[4 * i + 1], a); a = fmaf(ql.z, lo[4 * i + 2], a); a = fmaf(ql.w, lo[4 * i + 3], a);
-              a = fmaf(qh.x, hi[4 * i], a); a = fmaf(qh.y, hi[4 * i + 1], a); a = fmaf(qh.z, hi[4 * i + 2], a); a = fmaf(qh.w, hi[4 * i + 3], a);
-            }
-            sc[g] = fmaf(a, d01[b], sc[g]);
-          }
-        }
-      }
-      for (unsigned off = (1u << wshift) >> 1; off > 0; off >>= 1)
-#pragma unroll
-        for (int g = 0; g < G; g++) sc[g] += __shfl_xor_sync(0xffffffffu, sc[g], off);
-      if (pos_t < n && part == 0) {
-#pragma unroll
-        for (int g = 0; g < G; g++) ss[g * kTP + pos_t] = sc[g];
+      for (int k = 0; k < 2; k++) {
+        const uint4 f = qf[(2u * pr + k) * 32u];
+        float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        mma16816(c, low_nibbles(a[k]), low_nibbles(b[k]), low_nibbles(a[k] >> 8), low_nibbles(b[k] >> 8), f.x, f.y);
+        mma16816(c, high_nibbles(a[k]), high_nibbles(b[k]), high_nibbles(a[k] >> 8), high_nibbles(b[k] >> 8), f.z, f.w);
+        const float da = half_at(ra + 36u * pr + 18u * k), db = half_at(rb + 36u * pr + 18u * k);
+        s[0] = fmaf(c[0], da, s[0]);
+        s[1] = fmaf(c[1], da, s[1]);
+        s[2] = fmaf(c[2], db, s[2]);
+        s[3] = fmaf(c[3], db, s[3]);
       }
     }
-    __syncthreads();
-    // ---- softmax of the tile: warp = head
-    if (warp < G) {
-      float* sg = ss + warp * kTP;
-      float mx = kNegInit;
-      for (unsigned i = lane; i < n; i += 32) mx = fmaxf(mx, sg[i]);
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-      const float m_old = sst[warp], m_new = fmaxf(m_old, mx);
-      float sum = 0.0f;
-      for (unsigned i = lane; i < n; i += 32) {
-        const float e = __expf(sg[i] - m_new);
-        sg[i] = e;
-        sum += e;
-      }
+    for (int e = 0; e < 4; e++) s[e] += __shfl_xor_sync(0xffffffffu, s[e], 2);  // the two f16 terms of q
+    const unsigned pos = p0 + (warp + i * kMmaWarps) * kMmaTile + g;
+    s[0] = pos < p1 ? s[0] * sa : -INFINITY;
+    s[1] = pos < p1 ? s[1] * sb : -INFINITY;
+    s[2] = pos + 8u < p1 ? s[2] * sa : -INFINITY;
+    s[3] = pos + 8u < p1 ? s[3] * sb : -INFINITY;
+    float x0 = fmaxf(s[0], s[2]), x1 = fmaxf(s[1], s[3]);
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-      if (lane == 0) {
-        const float alpha = __expf(m_old - m_new);
-        sst[warp] = m_new;
-        sst[8 + warp] = sst[8 + warp] * alpha + sum;
-        sst[16 + warp] = alpha;
+    for (int off = 4; off <= 16; off <<= 1) {
+      x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, off));
+      x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, off));
+    }
+    // ---- the tile's largest |d| of V: its exponent bounds 2^kx
+    unsigned dmax = 0;
+    for (unsigned c = lane; c < kMmaTile * NB; c += 32u)
+      dmax = max(dmax, (unsigned)*reinterpret_cast<const unsigned short*>(vt + (c / NB) * ROWB + (c % NB) * KS_Q40_BLOCK_BYTES) & 0x7FFFu);
+    dmax = __reduce_max_sync(0xffffffffu, dmax);
+    const int k2 = min(kx, 29 - (int)(dmax >> 10));
+    const float n0 = fmaxf(m0, x0), n1 = fmaxf(m1, x1);
+    const float f0 = __expf(m0 - n0), f1 = __expf(m1 - n1);
+    l0 *= f0;
+    l1 *= f1;
+    if (__any_sync(0xffffffffu, f0 != 1.0f || f1 != 1.0f) || k2 != kx) {
+      const float r = __uint_as_float((unsigned)(127 + k2 - kx) << 23), a0 = f0 * r, a1 = f1 * r;
+#pragma unroll
+      for (int j = 0; j < HD / 16; j++) {
+        o[j][0] *= a0;
+        o[j][1] *= a1;
+        o[j][2] *= a0;
+        o[j][3] *= a1;
       }
     }
-    __syncthreads();
-    // ---- values: lane = dims, warps take positions round-robin
-#pragma unroll
-    for (int g = 0; g < G; g++) {
-      const float alpha = sst[16 + g];
-      c[g] *= alpha;
-#pragma unroll
-      for (int j = 0; j < DPL; j++) o[g][j] *= alpha;
+    m0 = n0;
+    m1 = n1;
+    kx = k2;
+    const float e0 = __expf(s[0] - m0), e1 = __expf(s[1] - m1), e2 = __expf(s[2] - m0), e3 = __expf(s[3] - m1);
+    l0 += e0 + e2;
+    l1 += e1 + e3;
+    if (t < 2u) {
+      *reinterpret_cast<float2*>(pw + g * 4u + ha) = make_float2(e0, e1);
+      *reinterpret_cast<float2*>(pw + (g + 8u) * 4u + ha) = make_float2(e2, e3);
     }
-    for (unsigned pos = warp; pos < n; pos += kTP / 32) {
-      float vv[DPL];
-      const float dv = load_row_raw<DPL>(vt + (size_t)pos * RP, lane, vv);
+    __syncwarp();
+    // ---- values: k = positions 2t, 2t + 1, 2t + 8, 2t + 9; column g = head g & 3, its first or second f16 term
+    const float up = __uint_as_float((unsigned)(127 + kx) << 23);
+    const float* pr = pw + 2u * t * 4u + (g & 3u);
+    const float p[4] = {pr[0] * up, pr[4] * up, pr[32] * up, pr[36] * up};
+    const unsigned char* v0 = vt + 2u * t * ROWB;
 #pragma unroll
-      for (int g = 0; g < G; g++) {
-        const float ed = ss[g * kTP + pos] * dv;
-        c[g] += ed;
-#pragma unroll
-        for (int j = 0; j < DPL; j++) o[g][j] = fmaf(ed, vv[j], o[g][j]);
+    for (unsigned b = 0; b < NB; b++) {
+      const unsigned char* vb = v0 + b * KS_Q40_BLOCK_BYTES;
+      const float y0 = p[0] * half_at(vb), y1 = p[1] * half_at(vb + ROWB), y2 = p[2] * half_at(vb + 8u * ROWB), y3 = p[3] * half_at(vb + 9u * ROWB);
+      __half2 h01 = __floats2half2_rn(y0, y1), h23 = __floats2half2_rn(y2, y3);
+      if (is_lo) {
+        const float2 q01 = __half22float2(h01), q23 = __half22float2(h23);
+        h01 = __floats2half2_rn(y0 - q01.x, y1 - q01.y);
+        h23 = __floats2half2_rn(y2 - q23.x, y3 - q23.y);
       }
+      // bytes 2g, 2g + 1 of the block (rows g and g + 8 of the product are dims 2g, 2g + 1; 16 more for the high nibbles)
+      const unsigned char* by = vb + 2u + 2u * g;
+      const uint32_t w0 = __byte_perm(*reinterpret_cast<const unsigned short*>(by), *reinterpret_cast<const unsigned short*>(by + ROWB), 0x5410);
+      const uint32_t w8 = __byte_perm(*reinterpret_cast<const unsigned short*>(by + 8u * ROWB), *reinterpret_cast<const unsigned short*>(by + 9u * ROWB), 0x5410);
+      mma16816(o[2 * b], low_nibbles(w0), low_nibbles(w0 >> 8), low_nibbles(w8), low_nibbles(w8 >> 8), h2_bits(h01), h2_bits(h23));
+      mma16816(o[2 * b + 1], high_nibbles(w0), high_nibbles(w0 >> 8), high_nibbles(w8), high_nibbles(w8 >> 8), h2_bits(h01), h2_bits(h23));
+    }
+    __syncwarp();  // every lane is done with the stage and the probabilities
+    stage ^= 1u;
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+#pragma unroll
+  for (int off = 4; off <= 16; off <<= 1) {
+    l0 += __shfl_xor_sync(0xffffffffu, l0, off);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, off);
+  }
+  // ---- the warps' (m, l, O) meet in shared memory (the rings are free), threads fold one dim each in warp order
+  __syncthreads();
+  float* ml = reinterpret_cast<float*>(smem + S::st_off);           // [warp][head](m, l)
+  float* mo = reinterpret_cast<float*>(smem + S::ring_off);         // [warp][head][HD]
+  const float down = __uint_as_float((unsigned)(127 - kx) << 23);
+#pragma unroll
+  for (int j = 0; j < HD / 16; j++) {
+#pragma unroll
+    for (int e = 0; e < 4; e++) o[j][e] = (o[j][e] + __shfl_xor_sync(0xffffffffu, o[j][e], 2)) * down;
+    if (t < 2u) {
+      const unsigned d = 32u * (j >> 1) + 16u * (j & 1) + 2u * g;
+      *reinterpret_cast<float2*>(mo + (warp * 4u + ha) * HD + d) = make_float2(o[j][0], o[j][2]);
+      *reinterpret_cast<float2*>(mo + (warp * 4u + ha + 1u) * HD + d) = make_float2(o[j][1], o[j][3]);
     }
   }
-  __syncthreads();  // tiles are free: the warps' partial O meet there
-  float* mo = reinterpret_cast<float*>(kt);  // [warp][g][dim]
-#pragma unroll
-  for (int g = 0; g < G; g++)
-#pragma unroll
-    for (int j = 0; j < DPL; j++) mo[((size_t)warp * G + g) * HD + lane_dim<DPL>(lane, j)] = fmaf(-8.0f, c[g], o[g][j]);
+  if (g == 0 && t < 2u) {
+    ml[(warp * 4u + ha) * 2u] = m0;
+    ml[(warp * 4u + ha) * 2u + 1u] = l0;
+    ml[(warp * 4u + ha + 1u) * 2u] = m1;
+    ml[(warp * 4u + ha + 1u) * 2u + 1u] = l1;
+  }
   __syncthreads();
-  for (int i = tid; i < G * HD; i += kTP) {
-    const int g = i / HD, d = i - g * HD;
-    float a = 0.0f;
+  for (unsigned i = tid; i < gb * HD; i += kMmaWarps * 32) {
+    const unsigned h = i / HD, d = i - h * HD;
+    float M = kNegInit;
 #pragma unroll
-    for (int w = 0; w < kTP / 32; w++) a += mo[((size_t)w * G + g) * HD + d];
-    const unsigned head = head0 + g;
+    for (unsigned w = 0; w < kMmaWarps; w++) M = fmaxf(M, ml[(w * 4u + h) * 2u]);
+    float a = 0.0f, L = 0.0f;
+#pragma unroll
+    for (unsigned w = 0; w < kMmaWarps; w++) {
+      const float f = __expf(ml[(w * 4u + h) * 2u] - M);
+      L = fmaf(ml[(w * 4u + h) * 2u + 1u], f, L);
+      a = fmaf(mo[(w * 4u + h) * HD + d], f, a);
+    }
+    const unsigned head = head0 + h;
     if (n_splits == 1) {
-      st_act<T>(out, ((size_t)slot * n_q + head) * HD + d, a / sst[8 + g]);
+      st_act<T>(out, ((size_t)slot * n_q + head) * HD + d, a / L);
     } else {
       float* rec = tmp + (((size_t)slot * n_q + head) * n_splits + split) * (HD + 2);
       if (d == 0) {
-        rec[0] = sst[g];
-        rec[1] = sst[8 + g];
+        rec[0] = M;
+        rec[1] = L;
       }
       rec[2 + d] = a;
     }
   }
 }
 
-template <int G, int HD, typename T>
-int launch_tile(ks_ctx* ctx, dim3 grid, unsigned n_q, unsigned n_kv, float scale, const void* q, const uint8_t* K, const uint8_t* V,
-                size_t slot_stride, const float* meta, float* tmp, void* out, int n_splits) {
-  auto kern = sdpa_tile_kernel<G, HD, T>;
-  constexpr size_t smem = TileSmem<G, HD>::total;
+// Returns 1 when the call is outside what the kernel takes.
+template <int HD, typename T>
+int launch_mma(ks_ctx* ctx, unsigned hpk, dim3 grid, unsigned n_q, unsigned n_kv, float scale, const void* q, const uint8_t* K, const uint8_t* V,
+               size_t slot_stride, const float* meta, float* tmp, void* out, int n_splits) {
+  const unsigned gb = hpk % 4 == 0 ? 4u : hpk % 2 == 0 ? 2u : 1u;
+  if (((uintptr_t)K | (uintptr_t)V | (uintptr_t)slot_stride) & (HD == 256 ? 15u : 7u)) return 1;
+  auto kern = sdpa_mma_kernel<HD, T>;
+  constexpr size_t smem = MmaSmem<HD>::total;
   static bool set[16] = {false};
   if (!set[ctx->device & 15]) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return ks_fail(ctx, KS_ERR_CUDA, "sdpa: cannot set %zu B shared memory: %s", smem, cudaGetErrorString(e));
     set[ctx->device & 15] = true;
   }
-  KS_LAUNCH(ctx, kern, grid, kTP, smem, n_q, n_kv, scale, (const T*)q, K, V, slot_stride, meta, tmp, (T*)out, n_splits);
-  return ks_after_launch(ctx, "sdpa_tile");
-}
-template <int HD, typename T>
-int launch_tile_g(ks_ctx* ctx, int G, dim3 grid, unsigned n_q, unsigned n_kv, float scale, const void* q, const uint8_t* K,
-                  const uint8_t* V, size_t slot_stride, const float* meta, float* tmp, void* out, int n_splits) {
-  switch (G) {
-    case 1: return launch_tile<1, HD, T>(ctx, grid, n_q, n_kv, scale, q, K, V, slot_stride, meta, tmp, out, n_splits);
-    case 2: return launch_tile<2, HD, T>(ctx, grid, n_q, n_kv, scale, q, K, V, slot_stride, meta, tmp, out, n_splits);
-    case 4: return launch_tile<4, HD, T>(ctx, grid, n_q, n_kv, scale, q, K, V, slot_stride, meta, tmp, out, n_splits);
-    case 8:  // four heads per block, two blocks per KV head: no register spills, and twice the blocks
-      grid.y *= 2;
-      return launch_tile<4, HD, T>(ctx, grid, n_q, n_kv, scale, q, K, V, slot_stride, meta, tmp, out, n_splits);
-  }
-  return 1;
+  grid.y *= hpk / gb;
+  KS_LAUNCH(ctx, kern, grid, kMmaWarps * 32, smem, n_q, n_kv, gb, scale, (const T*)q, K, V, slot_stride, meta, tmp, (T*)out, n_splits);
+  return ks_after_launch(ctx, "sdpa_mma");
 }
 
 template <int G, int DPL, typename T>
@@ -608,17 +677,14 @@ int ks_launch_sdpa(ks_ctx* ctx, size_t n_slots, size_t n_q, size_t n_kv, size_t 
   dim3 grid((unsigned)n_splits, (unsigned)n_kv, (unsigned)n_slots);
   int rc = 1;
   static const bool per_row = getenv("KSEARCH_SDPA_PER_ROW") != nullptr;  // keep the per-row kernel (comparison runs)
-  const bool aligned4 = (((uintptr_t)K | (uintptr_t)V | (uintptr_t)slot_stride_bytes) & 3u) == 0;
-  if (!per_row && aligned4 && G <= 8 && (hd == 256 || hd == 128)) {
-    if (hd == 256)
-      rc = act == KS_F32 ? launch_tile_g<256, float>(ctx, G, grid, (unsigned)n_q, (unsigned)n_kv, scale, q, K, V, slot_stride_bytes, meta, tmp, out, n_splits)
-                         : launch_tile_g<256, __half>(ctx, G, grid, (unsigned)n_q, (unsigned)n_kv, scale, q, K, V, slot_stride_bytes, meta, tmp, out, n_splits);
-    else
-      rc = act == KS_F32 ? launch_tile_g<128, float>(ctx, G, grid, (unsigned)n_q, (unsigned)n_kv, scale, q, K, V, slot_stride_bytes, meta, tmp, out, n_splits)
-                         : launch_tile_g<128, __half>(ctx, G, grid, (unsigned)n_q, (unsigned)n_kv, scale, q, K, V, slot_stride_bytes, meta, tmp, out, n_splits);
+  if (!per_row && (hd == 256 || hd == 128)) {
+#define KS_MMA(HD_, T_) launch_mma<HD_, T_>(ctx, (unsigned)G, grid, (unsigned)n_q, (unsigned)n_kv, scale, q, K, V, slot_stride_bytes, meta, tmp, out, n_splits)
+    if (hd == 256) rc = act == KS_F32 ? KS_MMA(256, float) : KS_MMA(256, __half);
+    else rc = act == KS_F32 ? KS_MMA(128, float) : KS_MMA(128, __half);
+#undef KS_MMA
   }
   if (rc != 1) {
-    // the tiled kernel took it
+    // the tensor-core kernel took it
   } else if (hd == 256) {
     rc = act == KS_F32 ? launch_part_g<8, float>(ctx, G, grid, (unsigned)n_q, (unsigned)n_kv, scale, q, K, V, slot_stride_bytes, meta, tmp, out, n_splits)
                        : launch_part_g<8, __half>(ctx, G, grid, (unsigned)n_q, (unsigned)n_kv, scale, q, K, V, slot_stride_bytes, meta, tmp, out, n_splits);
@@ -645,8 +711,8 @@ size_t ks_sdpa_tmp_floats(size_t n_slots, size_t n_q, size_t hd, int n_splits) {
 }
 
 int ks_sdpa_pick_splits(const ks_ctx* ctx, size_t n_slots, size_t n_kv, size_t max_t) {
-  // about 256 blocks in all (a block serves up to four query heads, so a slot has at least two per split), at least
-  // 128 positions per split: measured best over 1..8 slots x 1024..16384 positions on B200
+  // about 256 blocks in all (two fit an SM; a block serves up to four query heads, so a slot has at least two per split), at
+  // least 128 positions per split: measured best over 1..8 slots x 1024..16384 positions on B200
   (void)ctx;
   const size_t per_split = (n_slots ? n_slots : 1) * (n_kv > 2 ? n_kv : 2);
   size_t want = 256 / per_split;
