@@ -274,49 +274,67 @@ sdpa_part_kernel(unsigned n_q, unsigned n_kv, float scale, const T* q, const uin
   }
 }
 
-// Merge the per-split records of one (slot, head): lower.rs:5897-6088.  The (m, l) pairs go through shared
-// memory; 1024 / hd groups of threads share the splits, thread (group, d) adds O[d] of its splits eight loads at a
-// time, and the groups' sums meet in shared memory in a fixed order.
+// Merge the per-split records of one (slot, head): lower.rs:5897-6088.  A block takes 64 dims; four threads share a dim's splits
+// (p = part, part + 4, ...) and their sums meet in a fixed order.  The O values are requested before the (m, l) pairs are looked
+// at, so the two trips to memory are one.  Bound by that trip and the launch.
+constexpr int kRedDims = 64, kRedParts = 4, kRedFly = 8;
 template <typename T>
-__global__ void __launch_bounds__(1024) sdpa_reduce_kernel(unsigned hd, const float* tmp, T* out, int n_splits) {
+__global__ void __launch_bounds__(kRedDims * kRedParts) sdpa_reduce_kernel(unsigned hd, const float* tmp, T* out, int n_splits) {
   ks_pdl_entry();
-  __shared__ float sm[2 * KS_SDPA_MAX_SPLITS];
-  __shared__ float part[1024];
+  __shared__ float fac[KS_SDPA_MAX_SPLITS];
+  __shared__ float part_sum[kRedDims * kRedParts];
   const size_t sh = blockIdx.x;  // slot * n_q + head
   const float* rec0 = tmp + sh * n_splits * (hd + 2);
-  for (int p = threadIdx.x; p < n_splits; p += blockDim.x) {
-    sm[2 * p] = rec0[(size_t)p * (hd + 2)];
-    sm[2 * p + 1] = rec0[(size_t)p * (hd + 2) + 1];
-  }
-  __syncthreads();
-  float M = kNegInit;
-  for (int p = 0; p < n_splits; p++) M = fmaxf(M, sm[2 * p]);
-  float L = 0.0f;
-  for (int p = 0; p < n_splits; p++) L = fmaf(sm[2 * p + 1], __expf(sm[2 * p] - M), L);
-  // thread (group, d): the splits p = group, group + groups, ... of dimension d, eight loads in flight at a time
-  const unsigned groups = blockDim.x / hd, grp = threadIdx.x / hd, d = threadIdx.x % hd;
-  float o = 0.0f;
-  if (grp < groups) {
-    for (int pb = (int)grp; pb < n_splits; pb += 8 * (int)groups) {
-      float v[8];
+  const int part = threadIdx.x / kRedDims, lane = threadIdx.x & 31;
+  const unsigned d = blockIdx.y * kRedDims + threadIdx.x % kRedDims;
+  float v[kRedFly];
+  auto request = [&](int p0) {
 #pragma unroll
-      for (int k = 0; k < 8; k++) {  // an empty split (l = 0) left no O behind
-        const int p = pb + k * (int)groups;
-        v[k] = (p < n_splits && sm[2 * p + 1] != 0.0f) ? rec0[(size_t)p * (hd + 2) + 2 + d] : 0.0f;
-      }
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const int p = pb + k * (int)groups;
-        if (p < n_splits) o = fmaf(v[k], __expf(sm[2 * p] - M), o);
-      }
+    for (int k = 0; k < kRedFly; k++) {
+      const int p = p0 + k * kRedParts;
+      v[k] = p < n_splits ? rec0[(size_t)p * (hd + 2) + 2 + d] : 0.0f;
     }
-    part[threadIdx.x] = o;
+  };
+  request(part);
+  if (threadIdx.x < 32) {  // exp(m - M) / L of every split; an empty one (l = 0) has no O and counts for nothing
+    float m[KS_SDPA_MAX_SPLITS / 32], l[KS_SDPA_MAX_SPLITS / 32], M = kNegInit, L = 0.0f;
+#pragma unroll
+    for (int k = 0; k < KS_SDPA_MAX_SPLITS / 32; k++) {
+      const int p = lane + 32 * k;
+      m[k] = p < n_splits ? rec0[(size_t)p * (hd + 2)] : kNegInit;
+      l[k] = p < n_splits ? rec0[(size_t)p * (hd + 2) + 1] : 0.0f;
+      M = fmaxf(M, m[k]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+#pragma unroll
+    for (int k = 0; k < KS_SDPA_MAX_SPLITS / 32; k++) {
+      m[k] = l[k] != 0.0f ? __expf(m[k] - M) : 0.0f;
+      L = fmaf(l[k], m[k], L);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+#pragma unroll
+    for (int k = 0; k < KS_SDPA_MAX_SPLITS / 32; k++)
+      if (lane + 32 * k < n_splits) fac[lane + 32 * k] = m[k] / L;
   }
   __syncthreads();
-  if (threadIdx.x < hd) {
-    float a = 0.0f;
-    for (unsigned g2 = 0; g2 < groups; g2++) a += part[g2 * hd + threadIdx.x];  // fixed order
-    st_act<T>(out, sh * hd + threadIdx.x, a / L);
+  float o = 0.0f;
+  for (int p0 = part; p0 < n_splits; p0 += kRedFly * kRedParts) {
+    if (p0 != part) request(p0);
+#pragma unroll
+    for (int k = 0; k < kRedFly; k++) {
+      const int p = p0 + k * kRedParts;
+      const float f = p < n_splits ? fac[p] : 0.0f;
+      if (f != 0.0f) o = fmaf(v[k], f, o);
+    }
+  }
+  part_sum[threadIdx.x] = o;
+  __syncthreads();
+  if (threadIdx.x < kRedDims) {
+#pragma unroll
+    for (int k = 1; k < kRedParts; k++) o += part_sum[k * kRedDims + threadIdx.x];
+    st_act<T>(out, sh * hd + d, o);
   }
 }
 
@@ -400,9 +418,12 @@ sdpa_mma_kernel(unsigned n_q, unsigned n_kv, unsigned gb, float scale, const T* 
     const unsigned tile = warp + i * kMmaWarps;
     if (tile < n_tiles) {
       constexpr unsigned CH = HD == 256 ? 16u : 8u, PER = ROWB / CH;  // rows of 144 (72) bytes
-      for (unsigned c = lane; c < kMmaTile * PER; c += 32u) {
-        const unsigned r = c / PER, o = (c - r * PER) * CH;
-        const size_t src = (size_t)min(p0 + tile * kMmaTile + r, p1 - 1u) * rowstride + o;
+      const unsigned first = p0 + tile * kMmaTile, last = p1 - 1u - first;
+#pragma unroll
+      for (unsigned k = 0; k < (kMmaTile * PER + 31u) / 32u; k++) {
+        const unsigned c = lane + 32u * k, r = c / PER, o = (c - r * PER) * CH;
+        if (c >= kMmaTile * PER) break;
+        const size_t src = (size_t)(first + min(r, last)) * rowstride + o;
         const uint32_t dst = ring_s + stage * S::TILE + r * ROWB + o;
         if (CH == 16u) {
           cp_async16(dst, Ks + src);
@@ -595,26 +616,37 @@ sdpa_mma_kernel(unsigned n_q, unsigned n_kv, unsigned gb, float scale, const T* 
     ml[(warp * 4u + ha + 1u) * 2u + 1u] = l1;
   }
   __syncthreads();
+  float* fac = reinterpret_cast<float*>(smem + S::p_off);  // [warp][head] exp(m - M); behind them per head (M, L)
+  if (warp == 0) {  // lane = (warp w, head h)
+    const unsigned w = lane >> 2, h = lane & 3u;
+    const float m = ml[(w * 4u + h) * 2u], l = ml[(w * 4u + h) * 2u + 1u];
+    float M = m;
+#pragma unroll
+    for (int off = 4; off <= 16; off <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
+    const float f = __expf(m - M);
+    float L = l * f;
+#pragma unroll
+    for (int off = 4; off <= 16; off <<= 1) L += __shfl_xor_sync(0xffffffffu, L, off);
+    fac[lane] = f;
+    if (w == 0) {
+      fac[32u + h] = M;
+      fac[36u + h] = L;
+    }
+  }
+  __syncthreads();
   for (unsigned i = tid; i < gb * HD; i += kMmaWarps * 32) {
     const unsigned h = i / HD, d = i - h * HD;
-    float M = kNegInit;
+    float a = 0.0f;
 #pragma unroll
-    for (unsigned w = 0; w < kMmaWarps; w++) M = fmaxf(M, ml[(w * 4u + h) * 2u]);
-    float a = 0.0f, L = 0.0f;
-#pragma unroll
-    for (unsigned w = 0; w < kMmaWarps; w++) {
-      const float f = __expf(ml[(w * 4u + h) * 2u] - M);
-      L = fmaf(ml[(w * 4u + h) * 2u + 1u], f, L);
-      a = fmaf(mo[(w * 4u + h) * HD + d], f, a);
-    }
+    for (unsigned w = 0; w < kMmaWarps; w++) a = fmaf(mo[(w * 4u + h) * HD + d], fac[w * 4u + h], a);
     const unsigned head = head0 + h;
     if (n_splits == 1) {
-      st_act<T>(out, ((size_t)slot * n_q + head) * HD + d, a / L);
+      st_act<T>(out, ((size_t)slot * n_q + head) * HD + d, a / fac[36u + h]);
     } else {
       float* rec = tmp + (((size_t)slot * n_q + head) * n_splits + split) * (HD + 2);
       if (d == 0) {
-        rec[0] = M;
-        rec[1] = L;
+        rec[0] = fac[32u + h];
+        rec[1] = fac[36u + h];
       }
       rec[2 + d] = a;
     }
@@ -695,11 +727,11 @@ int ks_launch_sdpa(ks_ctx* ctx, size_t n_slots, size_t n_q, size_t n_kv, size_t 
     return ks_fail(ctx, KS_ERR_UNSUPPORTED, "sdpa: head_dim %zu not supported (128, 256)", hd);
   }
   if (rc || n_splits == 1) return rc;
-  const unsigned blocks = (unsigned)(n_slots * n_q);
+  const dim3 blocks((unsigned)(n_slots * n_q), (unsigned)hd / kRedDims);
   if (act == KS_F32)
-    KS_LAUNCH(ctx, (sdpa_reduce_kernel<float>), blocks, 1024, 0, (unsigned)hd, tmp, (float*)out, n_splits);
+    KS_LAUNCH(ctx, (sdpa_reduce_kernel<float>), blocks, kRedDims * kRedParts, 0, (unsigned)hd, tmp, (float*)out, n_splits);
   else
-    KS_LAUNCH(ctx, (sdpa_reduce_kernel<__half>), blocks, 1024, 0, (unsigned)hd, tmp, (__half*)out, n_splits);
+    KS_LAUNCH(ctx, (sdpa_reduce_kernel<__half>), blocks, kRedDims * kRedParts, 0, (unsigned)hd, tmp, (__half*)out, n_splits);
   return ks_after_launch(ctx, "sdpa_reduce");
 }
 
