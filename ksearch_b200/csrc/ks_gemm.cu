@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(1024) x_split_kernel(const float* x, size_t ld
 #pragma unroll
       for (int e = 0; e < 8; e++) v[e] = 0.0f;
     }
-    put_split8(xt, np, t, ck, v, q4k != 0);
+    put_split8(xt, np, t, ck, chunks, v, q4k != 0);
   }
 }
 
@@ -357,7 +357,7 @@ struct FinishArgs {
   const float* P[3];
   float* y[3];
   size_t ldy[3], part_stride[3];
-  unsigned rows[3], tile0[3], n_seg, n_tok;
+  unsigned rows[3], tile0[3], group0[3], n_seg, n_tok;
   ks_gemm_map map;
   int mode;
 };
@@ -398,9 +398,10 @@ __global__ void __launch_bounds__(256) gemm_finish_kernel(const FinishArgs f) {
   const unsigned t = blockIdx.y * TOK + threadIdx.x / PER, r = (bx - tile0) * GM_ROWS + (threadIdx.x % PER) * V;
   if (t >= f.n_tok || r >= rows) return;
   const size_t at = (size_t)t * rows + r;  // partials are dense [split][token][row]
-  FinVec<V> g = sum_slots<V>(P, ps, ks_gemm_slots(f.map, bx), at);
+  const unsigned group0 = seg == 0 ? f.group0[0] : seg == 1 ? f.group0[1] : f.group0[2];
+  FinVec<V> g = sum_slots<V>(P, ps, ks_gemm_slots(f.map, group0, bx - tile0, t), at);
   if (f.mode == 1) {
-    const FinVec<V> u = sum_slots<V>(f.P[1], f.part_stride[1], ks_gemm_slots(f.map, f.tile0[1] + bx), at);
+    const FinVec<V> u = sum_slots<V>(f.P[1], f.part_stride[1], ks_gemm_slots(f.map, f.group0[1], bx, t), at);
 #pragma unroll
     for (int k = 0; k < V; k++) g.v[k] = gelu_mul(g.v[k], u.v[k]);
   }
@@ -437,7 +438,7 @@ __global__ void gemm_finish_norm_split_kernel(const EpiNormArgs e) {
   for (int i = 0; i < 8; i++) y[i] = 0.0f;
   const size_t at = (size_t)t * e.rows + 8u * ck;
   if (live) {
-    const unsigned n = ks_gemm_slots(e.map, 8u * ck / GM_ROWS);
+    const unsigned n = ks_gemm_slots(e.map, 0u, 8u * ck / GM_ROWS, t);
     for (unsigned s = 0; s < n; s++) {
       const float4 a = *reinterpret_cast<const float4*>(e.P + (size_t)s * e.part_stride + at);
       const float4 b = *reinterpret_cast<const float4*>(e.P + (size_t)s * e.part_stride + at + 4);
@@ -480,7 +481,7 @@ __global__ void gemm_finish_norm_split_kernel(const EpiNormArgs e) {
   if (ck < chunks) {
 #pragma unroll
     for (int i = 0; i < 8; i++) xn[i] *= down;
-    put_split8(e.xt, e.np, t, ck, xn, e.q4k != 0);
+    put_split8(e.xt, e.np, t, ck, chunks, xn, e.q4k != 0);
   }
 }
 
@@ -504,7 +505,8 @@ __global__ void __launch_bounds__(GM_ROW_THREADS) gemm_finish_gelu_split_kernel(
 #pragma unroll
       for (int k = 0; k < 8; k++) g[k] = u[k] = 0.0f;
       const size_t at = (size_t)t * rows + 8u * ck;
-      const unsigned tile = 8u * ck / GM_ROWS, ng = ks_gemm_slots(map, tile), nu = ks_gemm_slots(map, (rows + GM_ROWS - 1u) / GM_ROWS + tile);
+      const unsigned tile = 8u * ck / GM_ROWS, groups = map.G ? ((rows + GM_ROWS - 1u) / GM_ROWS + map.nt - 1u) / map.nt : 0u,
+                     ng = ks_gemm_slots(map, 0u, tile, t), nu = ks_gemm_slots(map, groups, tile, t);
       for (unsigned s = 0; s < ng; s++) {
         const float4 a = *reinterpret_cast<const float4*>(P0 + (size_t)s * part_stride + at);
         const float4 b = *reinterpret_cast<const float4*>(P0 + (size_t)s * part_stride + at + 4);
@@ -530,15 +532,15 @@ __global__ void __launch_bounds__(GM_ROW_THREADS) gemm_finish_gelu_split_kernel(
     if (ck < chunks) {
 #pragma unroll
       for (int k = 0; k < 8; k++) v[kk][k] *= down;
-      put_split8(xt, np, t, ck, v[kk], true);  // a down-projection is always Q4_K
+      put_split8(xt, np, t, ck, chunks, v[kk], true);  // a down-projection is always Q4_K
     }
   }
 }
 }  // namespace
 
 namespace {
-// Token rows padded to what the MMAs take (N a multiple of 16).
-unsigned gemm_np(int n_tok) { return ((unsigned)n_tok + 15u) / 16u * 16u; }
+// Token rows padded to what the MMAs take (N a multiple of 16; beyond 128 the Q4_K kernel takes them in two halves).
+unsigned gemm_np(int n_tok) { return n_tok > 128 ? ((unsigned)n_tok + 31u) / 32u * 32u : ((unsigned)n_tok + 15u) / 16u * 16u; }
 // Shared memory of one CTA and its stage count (A and B rings have the same depth): two stages when that lets two
 // CTAs share an SM (measured: a third stage that still lets them does not pay), else as many (up to four) as one CTA fits.
 size_t gemm_smem(const ks_ctx* ctx, unsigned np, unsigned* nb_out) {
@@ -577,9 +579,11 @@ unsigned gemm_splits(const ks_ctx* ctx, size_t rows, size_t cols, int n_tok) {
   }
   return best;
 }
-ks_gemm_map gemm_map(const ks_ctx* ctx, ks_dtype wdtype, size_t total_rows, unsigned tiles, size_t cols, int n_tok) {
-  if (wdtype == KS_Q4K) return ks_gemm_q4k_map(ctx, tiles, (unsigned)cols, gemm_np(n_tok));
+ks_gemm_map gemm_map(const ks_ctx* ctx, ks_dtype wdtype, const size_t* rows, int n_seg, size_t cols, int n_tok) {
+  if (wdtype == KS_Q4K) return ks_gemm_q4k_map(ctx, rows, n_seg, (unsigned)cols, gemm_np(n_tok));
   ks_gemm_map m{};
+  size_t total_rows = 0;
+  for (int i = 0; i < n_seg; i++) total_rows += rows[i];
   const unsigned ksteps = (unsigned)(cols / GM_KSTEP), s = gemm_splits(ctx, total_rows, cols, n_tok), per = (ksteps + s - 1) / s;
   m.splits = (ksteps + per - 1) / per;
   return m;
@@ -612,20 +616,23 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
   if ((mode == KS_GEMM_NORM_SPLIT && (n_seg != 1 || !epi || rows[0] % 8 || rows[0] > 8192)) ||
       (mode == KS_GEMM_GELU_SPLIT && (n_seg != 2 || !epi || rows[0] != rows[1] || rows[0] % 8 || rows[0] > 8u * GM_GELU_CHUNKS * GM_ROW_THREADS)))
     return ks_fail(ctx, KS_ERR_INVALID, "gemm: bad epilogue arguments");
-  unsigned tiles = 0, tile0[4];
+  const unsigned np = gemm_np(n_tok);
+  const ks_gemm_map map = gemm_map(ctx, wdtype, rows, n_seg, cols, n_tok);
+  unsigned tiles = 0, tile0[4], groups = 0, group0[3] = {0, 0, 0};
   size_t total_rows = 0;
   for (int i = 0; i < 3; i++) {
     tile0[i] = i < n_seg ? tiles : 0xFFFFFFFFu;  // no tile reaches an absent matrix
     if (i >= n_seg) continue;
-    tiles += (unsigned)((rows[i] + GM_ROWS - 1) / GM_ROWS);
+    const unsigned n = (unsigned)((rows[i] + GM_ROWS - 1) / GM_ROWS);
+    group0[i] = groups;
+    tiles += n;
+    groups += map.G ? (n + map.nt - 1) / map.nt : 0;
     total_rows += rows[i];
   }
   tile0[3] = tiles;
-  const unsigned np = gemm_np(n_tok);
-  const ks_gemm_map map = gemm_map(ctx, wdtype, total_rows, tiles, cols, n_tok);
-  unsigned slots = 0;
-  for (unsigned t = 0; t < tiles; t++) {
-    const unsigned n = ks_gemm_slots(map, t);
+  unsigned slots = map.G ? 0 : map.splits;
+  for (unsigned w = 0; map.G && w < groups * map.tb; w++) {
+    const unsigned n = ks_gemm_owner(map, w * map.S + map.S - 1u) - ks_gemm_owner(map, w * map.S) + 1u;
     slots = n > slots ? n : slots;
   }
   const bool direct = slots == 1 && mode == KS_GEMM_PLAIN;
@@ -732,7 +739,10 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
   }
   f.n_seg = (unsigned)n_seg;
   f.map = map;
-  for (int i = 0; i < 3; i++) f.tile0[i] = tile0[i];
+  for (int i = 0; i < 3; i++) {
+    f.tile0[i] = tile0[i];
+    f.group0[i] = group0[i];
+  }
   f.n_tok = (unsigned)n_tok;
   f.mode = mode;
   const unsigned out_tiles = mode == KS_GEMM_GELU ? tile0[1] : tiles;
@@ -750,11 +760,11 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
 
 // Floats of partials ks_launch_gemm_segs may write for up to three matrices of `total_rows` rows in all (either dtype).
 size_t ks_gemm_part_floats(const ks_ctx* ctx, size_t total_rows, size_t cols, int n_tok) {
-  const unsigned tiles = (unsigned)((total_rows + GM_ROWS - 1) / GM_ROWS);
-  unsigned slots = gemm_map(ctx, KS_Q6K, total_rows, tiles, cols, n_tok).splits;
-  for (unsigned t = tiles; t < tiles + 3; t++) {  // the matrices of a launch round their tiles up one by one
-    const ks_gemm_map m = gemm_map(ctx, KS_Q4K, total_rows, t, cols, n_tok);
-    const unsigned n = (m.S + m.base - 1) / m.base + 1;  // a CTA has at least `base` units, a tile may begin inside one
+  unsigned slots = gemm_map(ctx, KS_Q6K, &total_rows, 1, cols, n_tok).splits;
+  for (int extra = 0; extra < 3; extra++) {  // the matrices of a launch round their tiles up one by one
+    const size_t r = total_rows + (size_t)extra * 2 * GM_ROWS;
+    const ks_gemm_map m = gemm_map(ctx, KS_Q4K, &r, 1, cols, n_tok);
+    const unsigned n = (m.S + m.base - 1) / m.base + 1;  // a CTA has at least `base` units, a work tile may begin inside one
     slots = n > slots ? n : slots;
   }
   return (size_t)slots * (size_t)n_tok * total_rows;

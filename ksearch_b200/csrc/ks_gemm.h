@@ -12,5 +12,5 @@ struct ks_gemm_job {
   const __half* xt;
   ks_gemm_map map;
 };
-ks_gemm_map ks_gemm_q4k_map(const ks_ctx* ctx, unsigned tiles, unsigned cols, unsigned np);
+ks_gemm_map ks_gemm_q4k_map(const ks_ctx* ctx, const size_t* rows, int n_seg, unsigned cols, unsigned np);
 int ks_launch_gemm_q4k(ks_ctx* ctx, const ks_gemm_job& job);

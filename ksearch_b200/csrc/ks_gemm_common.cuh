@@ -8,13 +8,16 @@
 constexpr int GM_ROWS = 128;  // weight rows per tile (M of the MMA)
 
 // ---- work units ---------------------------------------------------------------------------------
-// The Q4_K kernel cuts a launch into units (row tile, 256-column super-block), numbered tile after tile, and gives every CTA
-// a run of them: the first `rem` CTAs base + 1, the others base.  So no CTA has more than one unit more than another whatever
-// the tile count, and a tile whose units several CTAs share leaves one partial per CTA, in CTA order.  (Plain multiplications
-// on purpose: what the MMA warp derives from them stays in uniform registers.)  G == 0: every tile has `splits` partials.
+// The Q4_K kernel cuts a launch into units: one super-block (256 columns) of `nt` neighbouring row tiles of a matrix against one
+// block of `tbn` token rows.  Units are numbered column after column inside a work tile (row tiles x token block), the token
+// blocks of the same row tiles next to each other, and every CTA gets a run of them: the first `rem` CTAs base + 1, the others
+// base.  So no CTA has more than one unit more than another whatever the tile count, and a work tile whose units several CTAs
+// share leaves one partial per CTA, in CTA order.  (Plain multiplications on purpose: what the MMA warp derives from them stays
+// in uniform registers.)  G == 0: every tile has `splits` partials.
 struct ks_gemm_map {
-  unsigned G, S;          // CTAs, units per tile
+  unsigned G, S;          // CTAs, units per work tile
   unsigned base, rem;
+  unsigned nt, tb, tbn;   // row tiles per unit, token blocks, token rows per block
   unsigned splits;
 };
 __host__ __device__ inline unsigned ks_gemm_first(const ks_gemm_map& m, unsigned cta) { return cta * m.base + (cta < m.rem ? cta : m.rem); }
@@ -22,8 +25,11 @@ __host__ __device__ inline unsigned ks_gemm_owner(const ks_gemm_map& m, unsigned
   const unsigned big = m.rem * (m.base + 1u);
   return u < big ? u / (m.base + 1u) : m.rem + (u - big) / m.base;
 }
-__host__ __device__ inline unsigned ks_gemm_slots(const ks_gemm_map& m, unsigned tile) {
-  return m.G == 0 ? m.splits : ks_gemm_owner(m, tile * m.S + m.S - 1u) - ks_gemm_owner(m, tile * m.S) + 1u;
+// Partials of row tile `tile` (counted inside its matrix, whose first row-tile group is `group0`) for token row `t`.
+__host__ __device__ inline unsigned ks_gemm_slots(const ks_gemm_map& m, unsigned group0, unsigned tile, unsigned t) {
+  if (m.G == 0) return m.splits;
+  const unsigned w = (group0 + tile / m.nt) * m.tb + t / m.tbn;
+  return ks_gemm_owner(m, w * m.S + m.S - 1u) - ks_gemm_owner(m, w * m.S) + 1u;
 }
 
 namespace {
@@ -56,10 +62,18 @@ __device__ __forceinline__ void split8(const float (&w)[8], uint4& hi, uint4& lo
 //                          order in which masking the packed nibbles in place leaves the weights.  Chunks 32..35 carry the
 //                          sub-block sums the minima multiply: chunk 32 + g holds, with S = 2^-5 (sum of a 32-value
 //                          sub-block), (S_hi, S_hi', S_lo, S_lo', S_hi, S_hi', 0, 0) of sub-blocks 2 g and 2 g + 1.
-__device__ __forceinline__ void put_split8(__half* xt, unsigned np, unsigned t, unsigned ck, const float (&v)[8], bool q4k) {
+//                          More than 128 token rows are two such images of half the rows, one behind the other.
+__device__ __host__ __forceinline__ unsigned q4k_block(unsigned np) { return np > 128u ? np / 2u : np; }  // token rows of one image
+__device__ __forceinline__ void put_split8(__half* xt, unsigned np, unsigned t, unsigned ck, unsigned chunks, const float (&v)[8], bool q4k) {
   unsigned at = ck;
   if (q4k) {
     at = (ck >> 5) * 36u + (ck & 31u);
+    const unsigned tbn = q4k_block(np);
+    if (t >= tbn) {
+      t -= tbn;
+      xt += (size_t)(chunks / 32u * 36u) * 2u * tbn * 8u;
+    }
+    np = tbn;
     const float w[8] = {v[0], v[2], v[1], v[3], v[4], v[6], v[5], v[7]};
     uint4 hi, lo;
     split8(w, hi, lo);

@@ -40,7 +40,7 @@ namespace {
 
 constexpr unsigned Q_WARPS = 16, Q_THREADS = (Q_WARPS + 3) * 32;  // workers, MMA, packed rows, token rows
 constexpr unsigned Q_RAW = GM_ROWS * KS_Q4K_BLOCK_BYTES;          // bytes of a unit's packed rows
-constexpr unsigned Q_EXT = 192, Q_D = 224;                        // tensor-memory columns: minima, first accumulator
+constexpr unsigned Q_EXT = 192;                                   // tensor-memory column of the first block of minima
 constexpr unsigned Q_WAIT = 1u << 20;
 constexpr unsigned Q_MAX_RAW = 6, Q_MAX_B = 6;
 
@@ -48,7 +48,7 @@ struct __align__(64) Q4Args {
   CUtensorMap w[3];        // matrix i: rows[i] rows of row_bytes bytes
   float* y[3];             // y[i] + slot * part_stride[i] + token * ldy[i] + row
   size_t ldy[3], part_stride[3];
-  unsigned rows[3], tile0[4];
+  unsigned rows[3], group0[3];
   ks_gemm_map map;
   const __half* xt;        // the q4k form of the B image
   unsigned cols, n_tok, np;
@@ -143,25 +143,23 @@ __device__ __forceinline__ void q4_words(const uint4 q, const Q4Hdr& h, uint32_t
 }
 
 struct Seg {  // one matrix of the launch, picked without dynamic indexing of the parameters
-  unsigned rows, tile0;
+  unsigned rows, group0;
   float* y;
   size_t ldy, part;
 };
-__device__ __forceinline__ Seg pick_seg(const Q4Args& a, unsigned tile) {
-  const int i = (tile >= a.tile0[1]) + (tile >= a.tile0[2]);
+__device__ __forceinline__ Seg pick_seg(const Q4Args& a, unsigned grp) {
+  const int i = (grp >= a.group0[1]) + (grp >= a.group0[2]);
   Seg s;
   s.rows = i == 0 ? a.rows[0] : i == 1 ? a.rows[1] : a.rows[2];
-  s.tile0 = i == 0 ? a.tile0[0] : i == 1 ? a.tile0[1] : a.tile0[2];
+  s.group0 = i == 0 ? a.group0[0] : i == 1 ? a.group0[1] : a.group0[2];
   s.y = i == 0 ? a.y[0] : i == 1 ? a.y[1] : a.y[2];
   s.ldy = i == 0 ? a.ldy[0] : i == 1 ? a.ldy[1] : a.ldy[2];
   s.part = i == 0 ? a.part_stride[0] : i == 1 ? a.part_stride[1] : a.part_stride[2];
   return s;
 }
 
-// Groups of 32 k (a super-block has 9, the minima's among them) per B stage: as many as let two or more stages fit.
-__host__ __device__ constexpr unsigned q4_kb(int tq) { return tq <= 16 ? 9u : tq == 32 ? 3u : 1u; }
-
-// TQ: token rows per worker thread at most (NP / 4: the four warps of a lane quadrant share the accumulator's columns).
+// Up to 64 token rows.  TQ: token rows per worker thread at most (tbn / 4: the four warps of a lane quadrant share the
+// accumulator's columns).
 template <int TQ>
 __global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_constant__ Q4Args a) {
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -170,9 +168,9 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + QB_COUNT * 8);
   volatile unsigned* fail = reinterpret_cast<volatile unsigned*>(smem + QB_COUNT * 8 + 8);
   const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-  constexpr bool CONCAT = TQ <= 16;               // x_hi and x_lo side by side in one MMA
-  constexpr unsigned KB = q4_kb(TQ), NACC = TQ == 64 ? 1 : 2;   // groups of 32 k per B stage, accumulators
-  const unsigned b_group = 4u * 2u * a.np * 16u, b_stage = KB * b_group;
+  constexpr unsigned Q_D = 224;                     // first accumulator
+  const unsigned tbn = a.map.tbn;                   // token rows of a unit
+  const unsigned b_group = 4u * 2u * tbn * 16u, b_stage = 9u * b_group;
   float* up_s = reinterpret_cast<float*>(smem + 512);   // 2^e of every token row
   const uint32_t raw0 = bars + Q_HEAD, b0 = raw0 + a.n_raw * Q_RAW;
   const unsigned u0 = ks_gemm_first(a.map, blockIdx.x), n_units = a.map.base + (blockIdx.x < a.map.rem ? 1u : 0u);
@@ -212,14 +210,12 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_
     const unsigned quad = warp & 3u, g = warp >> 2, half = g >> 1;
     const uint32_t tlane = tmem + ((quad * 32u) << 16);
     const unsigned row = quad * 32u + lane;
-    const unsigned tq = a.np >> 2;               // tokens of this thread: [g * tq, + tq)
-    const unsigned acc_cols = CONCAT ? 2u * a.np : a.np;
-    float acc[TQ];
+    const unsigned tq = tbn >> 2;                // tokens of this thread: [g * tq, + tq) of the unit's
+    float acc[TQ], s_prev = 0.0f;
 #pragma unroll
     for (int i = 0; i < TQ; i++) acc[i] = 0.0f;
-    float s_prev = 0.0f;
     bool ok = true;
-    unsigned tile = u0 / a.map.S, sb = u0 - tile * a.map.S, prev_tile = 0;
+    unsigned wt = u0 / a.map.S, sb = u0 - wt * a.map.S, prev_wt = 0;   // work tile and super-block of the unit
     unsigned rs = 0, rph = 0;  // ring stage of the packed rows and its phase
     uint4 hraw = {}, qa = {}, qb = {};
     // the packed bytes of this thread, read one unit ahead: the reads overlap the accumulator's way out
@@ -239,17 +235,15 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_
       }
       return got;
     };
-    // (with 64 sums per thread there are no registers for that)
-    constexpr bool AHEAD = TQ < 64;
-    if (AHEAD && n_units) ok = fetch();
+    if (n_units) ok = fetch();
     for (unsigned i = 0; i <= n_units && ok; i++) {
+      // does the unit before this one end a work tile, or this CTA's share of one?
+      const bool last = i == n_units || (i > 0 && sb == 0);
       float s_cur = 0.0f;
-      bool last = i == n_units;   // the unit before this one ends a tile, or this CTA's share of one
       // the first unit's weights need nothing of the kernels before this one; the waits below depend on the image, and what is
       // written at the end may still be read by them
       if (i == 1) asm volatile("griddepcontrol.wait;" ::: "memory");
       if (i < n_units) {
-        if (!AHEAD && !fetch()) { ok = false; break; }
         Q4Hdr h;
         q4_header(hraw, g, h);
         s_cur = h.s;
@@ -269,131 +263,105 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mb_arrive(bar(QB_A_FULL + slot));
-        if (AHEAD && i + 1u < n_units && !fetch()) { ok = false; break; }
-        if (i > 0 && sb == 0) last = true;
-        if (++sb == a.map.S) {
-          sb = 0;
-          tile++;
-        }
+        if (i + 1u < n_units && !fetch()) { ok = false; break; }
       }
-      if (i > 0) {  // fold the previous super-block's accumulators
-        const unsigned j = i - 1u, buf = j % NACC;
-        if (!__all_sync(0xffffffffu, mb_wait(bar(QB_D_FULL + buf), (j / NACC) & 1u, a.wait_limit))) { ok = false; break; }
+      if (i > 0) {  // fold the previous super-block's accumulator
+        const unsigned j = i - 1u, buf = j & 1u;
+        if (!__all_sync(0xffffffffu, mb_wait(bar(QB_D_FULL + buf), (j >> 1) & 1u, a.wait_limit))) { ok = false; break; }
         tc_fence_after();
-        const uint32_t dcol = tlane + Q_D + buf * acc_cols + g * tq;
+        const uint32_t dcol = tlane + Q_D + buf * 2u * tbn + g * tq;
+        uint32_t d0[16], d1[16];
+        if (TQ >= 16 && tq == 16u) {
+          tc_ld16(dcol, d0);
+          tc_ld16(dcol + tbn, d1);
+        } else {
 #pragma unroll
-        for (int c = 0; c < TQ; c += 16) {
-          if ((unsigned)c < tq) {
-            uint32_t d0[16], d1[16];
-            if (TQ >= 16 && (unsigned)c + 16u <= tq) {
-              tc_ld16(dcol + c, d0);
-              if (CONCAT) tc_ld16(dcol + a.np + c, d1);
-            } else {
-#pragma unroll
-              for (int k = 0; k < 16; k += 4)
-                if (c + k < TQ && (unsigned)(c + k) < tq) {
-                  tc_ld4(dcol + c + k, d0 + k);
-                  if (CONCAT) tc_ld4(dcol + a.np + c + k, d1 + k);
-                }
+          for (int k = 0; k < TQ; k += 4)
+            if ((unsigned)k < tq) {
+              tc_ld4(dcol + k, d0 + k);
+              tc_ld4(dcol + tbn + k, d1 + k);
             }
-            tc_wait_ld16(d0);
-            if (CONCAT) tc_wait_ld16(d1);
-#pragma unroll
-            for (int k = 0; k < 16; k++)
-              if (c + k < TQ && (unsigned)(c + (k & ~3)) < tq) {
-                float t = __uint_as_float(d0[k]);
-                if (CONCAT) t += __uint_as_float(d1[k]);
-                acc[c + k] = fmaf(s_prev, t, acc[c + k]);
-              }
-          }
         }
+        tc_wait_ld16(d0);
+        tc_wait_ld16(d1);
+#pragma unroll
+        for (int k = 0; k < TQ; k++)
+          if ((unsigned)(k & ~3) < tq) acc[k] = fmaf(s_prev, __uint_as_float(d0[k]) + __uint_as_float(d1[k]), acc[k]);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mb_arrive(bar(QB_D_FREE + buf));
         if (last) {
-          const Seg sg = pick_seg(a, prev_tile);
-          const unsigned out_row = (prev_tile - sg.tile0) * GM_ROWS + row;
-          const unsigned pslot = blockIdx.x - ks_gemm_owner(a.map, prev_tile * a.map.S);
+          const Seg sg = pick_seg(a, prev_wt);
+          const unsigned out_row = (prev_wt - sg.group0) * GM_ROWS + row;
+          const unsigned pslot = blockIdx.x - ks_gemm_owner(a.map, prev_wt * a.map.S);
           float* y = sg.y + (size_t)pslot * sg.part + out_row;
           const bool live = out_row < sg.rows;
 #pragma unroll
           for (int k = 0; k < TQ; k++) {
-            const unsigned t = g * tq + k;
-            if ((unsigned)k < tq && t < a.n_tok && live) y[(size_t)t * sg.ldy] = acc[k] * up_s[t];
+            const unsigned tok = g * tq + k;
+            if ((unsigned)k < tq && tok < a.n_tok && live) y[(size_t)tok * sg.ldy] = acc[k] * up_s[tok];
             acc[k] = 0.0f;
           }
         }
       }
       s_prev = s_cur;
-      prev_tile = sb == 0 ? tile - 1u : tile;  // tile and sb already point one unit on
+      prev_wt = wt;
+      if (++sb == a.map.S) {
+        sb = 0;
+        wt++;
+      }
     }
     if (!ok && lane == 0) *fail = 1;
   } else if (warp == Q_WARPS) {
     // ---- MMAs: the whole warp runs the loop, converged, and one elected lane issues (loop state and descriptors then stay in
     // uniform registers)
     const unsigned leader = elect_one();
-    const unsigned ncol = CONCAT ? 2u * a.np : a.np;
+    const unsigned ncol = 2u * tbn;   // x_hi and x_lo side by side
     const uint32_t idesc = (1u << 4) | ((ncol >> 3) << 17) | ((unsigned)(GM_ROWS >> 4) << 24);  // f32 accumulate, f16 x f16, K-major both
-    const uint64_t bdesc0 = tc_desc(b0, 2u * a.np * 16u, 128u);
-    const unsigned chunk2 = 4u * a.np, lo_rows = a.np;   // in descriptor units of 16 bytes: two chunks of 8 k, the hi rows
+    const uint64_t bdesc0 = tc_desc(b0, 2u * tbn * 16u, 128u);
+    const unsigned chunk2 = 4u * tbn;   // in descriptor units of 16 bytes: two chunks of 8 k
     asm volatile("griddepcontrol.wait;" ::: "memory");
     // What an MMA takes has to be in uniform registers when it issues.  It gets there by itself only while the compiler can see
     // that the warp stays together: loop bounds from launch parameters and blockIdx, no value out of memory (hence the
     // constant tensor-memory base), one way out.  Otherwise every MMA waits for five register moves, about 200 cycles.
     bool ok = false;
-    unsigned bs = 0, bph = 0;                   // B stage and its phase
-    unsigned s0 = 0, ph0 = 0, s1 = 1, ph1 = 0;  // A slots of the unit's two halves and their phases
+    unsigned bs = 0, bph = 0;   // B stage and its phase
+    unsigned sl = 0, sph = 0;   // A slot and its phase: the slots are taken in the order the MMAs go
     for (unsigned i = 0; i < n_units; i++) {
-      const unsigned buf = i % NACC;
+      const unsigned buf = i & 1u;
       const uint32_t d = tmem + Q_D + buf * ncol;
-      if (i >= NACC && !__all_sync(0xffffffffu, mb_wait(bar(QB_D_FREE + buf), (i / NACC - 1u) & 1u, a.wait_limit))) goto out;
-      uint64_t bd = 0;
 #pragma unroll
-      for (unsigned kg = 0; kg < 9; kg++) {  // groups of 32 k: four of each half, the minima
-        bool got = true, waited = false;
-        if (kg == 0 || kg == 4u) {
-          got = mb_wait(bar(QB_A_FULL + (kg ? s1 : s0)), kg ? ph1 : ph0, a.wait_limit);
-          waited = true;
-        }
-        if (kg % KB == 0) {
-          got = got && mb_wait(bar(QB_B_FULL + bs), bph, a.wait_limit);
-          waited = true;
-          bd = bdesc0 + (uint64_t)(bs * (b_stage >> 4));
-        }
-        if (waited) {
-          if (!__all_sync(0xffffffffu, got)) goto out;
-          tc_fence_after();
-        }
+      for (unsigned hf = 0; hf < 2; hf++) {
+        bool got = true;
+        if (hf == 0 && i >= 2u) got = mb_wait(bar(QB_D_FREE + buf), ((i >> 1) - 1u) & 1u, a.wait_limit);
+        got = got && mb_wait(bar(QB_A_FULL + sl), sph, a.wait_limit);
+        if (hf == 0) got = got && mb_wait(bar(QB_B_FULL + bs), bph, a.wait_limit);
+        if (!__all_sync(0xffffffffu, got)) goto out;
+        tc_fence_after();
         if (leader) {
-          const uint32_t at = kg == 8u ? tmem + Q_EXT + (i & 1u) * 16u : tmem + (kg < 4u ? s0 : s1) * 64u + (kg & 3u) * 16u;
-          const uint64_t b = bd + (uint64_t)((kg % KB) * (b_group >> 4));
-          tc_mma_f16_ta(d, at, b, idesc, kg ? 1u : 0u);
-          if (!CONCAT && kg < 8u) tc_mma_f16_ta(d, at, b + lo_rows, idesc, 1u);
-          tc_mma_f16_ta(d, at + 8u, b + chunk2, idesc, 1u);
-          if (!CONCAT && kg < 8u) tc_mma_f16_ta(d, at + 8u, b + chunk2 + lo_rows, idesc, 1u);
-          if (kg % KB == KB - 1u) tc_commit(bar(QB_B_FREE + bs));
-          if (kg == 3u) tc_commit(bar(QB_A_FREE + s0));
-          if (kg == 8u) {
-            tc_commit(bar(QB_A_FREE + s1));
+          const uint64_t bd = bdesc0 + (uint64_t)(bs * (b_stage >> 4)) + (uint64_t)((hf ? 4u : 0u) * (b_group >> 4));
+#pragma unroll
+          for (unsigned kg = 0; kg < 4u + hf; kg++) {  // groups of 32 k; the fifth: the minima
+            const uint32_t at = kg == 4u ? tmem + Q_EXT + (i & 1u) * 16u : tmem + sl * 64u + kg * 16u;
+            const uint64_t b = bd + (uint64_t)(kg * (b_group >> 4));
+            tc_mma_f16_ta(d, at, b, idesc, (hf | kg) ? 1u : 0u);
+            tc_mma_f16_ta(d, at + 8u, b + chunk2, idesc, 1u);
+          }
+          tc_commit(bar(QB_A_FREE + sl));
+          if (hf) {
+            tc_commit(bar(QB_B_FREE + bs));
             tc_commit(bar(QB_D_FULL + buf));
           }
         }
-        if (kg % KB == KB - 1u && ++bs == a.n_b) {
-          bs = 0;
-          bph ^= 1u;
+        __syncwarp();
+        if (++sl == 3u) {
+          sl = 0;
+          sph ^= 1u;
         }
       }
-      __syncwarp();
-      // the next unit's halves: two slots further round the ring of three
-      s0 += 2u;
-      if (s0 >= 3u) {
-        s0 -= 3u;
-        ph0 ^= 1u;
-      }
-      s1 += 2u;
-      if (s1 >= 3u) {
-        s1 -= 3u;
-        ph1 ^= 1u;
+      if (++bs == a.n_b) {
+        bs = 0;
+        bph ^= 1u;
       }
     }
     ok = true;
@@ -408,7 +376,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_
   } else if (warp == Q_WARPS + 1) {
     // ---- packed rows: they depend on no kernel before this one
     const unsigned leader = elect_one();
-    unsigned issued = 0, st = 0, ph = 1, tile = u0 / a.map.S, sb = u0 - tile * a.map.S;
+    unsigned issued = 0, st = 0, ph = 1, wt = u0 / a.map.S, sb = u0 - wt * a.map.S;
     for (unsigned i = 0; i < n_units; i++) {
       const bool got = i < a.n_raw || mb_wait(bar(QB_RAW_FREE + st), ph, a.wait_limit);
       if (!__all_sync(0xffffffffu, got)) {
@@ -416,10 +384,12 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_
         break;
       }
       if (leader) {
-        const int k = (tile >= a.tile0[1]) + (tile >= a.tile0[2]);
-        const unsigned t0 = k == 0 ? a.tile0[0] : k == 1 ? a.tile0[1] : a.tile0[2];
+        const unsigned grp = wt;
+        const int k = (grp >= a.group0[1]) + (grp >= a.group0[2]);
+        const unsigned g0 = k == 0 ? a.group0[0] : k == 1 ? a.group0[1] : a.group0[2];
         mb_expect(bar(QB_RAW_FULL + st), Q_RAW);  // rows past the matrix come as zeros and count
-        tma_in_2d(raw0 + st * Q_RAW, k == 0 ? &a.w[0] : k == 1 ? &a.w[1] : &a.w[2], sb * KS_Q4K_BLOCK_BYTES, (tile - t0) * GM_ROWS, bar(QB_RAW_FULL + st));
+        tma_in_2d(raw0 + st * Q_RAW, k == 0 ? &a.w[0] : k == 1 ? &a.w[1] : &a.w[2], sb * KS_Q4K_BLOCK_BYTES, (grp - g0) * GM_ROWS,
+                  bar(QB_RAW_FULL + st));
       }
       issued++;
       if (++st == a.n_raw) {
@@ -428,7 +398,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_
       }
       if (++sb == a.map.S) {
         sb = 0;
-        tile++;
+        wt++;
       }
       __syncwarp();
     }
@@ -440,33 +410,332 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_
     const float* up = reinterpret_cast<const float*>(a.xt + xt_scale_off(a.cols, a.np));
     for (unsigned t = lane; t < a.np; t += 32u) up_s[t] = up[t];  // read behind the first accumulator, which waits for the copies below
     __syncwarp();
-    constexpr unsigned PER = 9u / KB;
-    const unsigned total = n_units * PER;
-    unsigned issued = 0, sb = u0 % a.map.S, k = 0, st = 0, ph = 1;
-    for (unsigned j = 0; j < total; j++) {
+    unsigned issued = 0, sb = u0 % a.map.S, st = 0, ph = 1;
+    for (unsigned j = 0; j < n_units; j++) {  // a super-block each
       const bool got = j < a.n_b || mb_wait(bar(QB_B_FREE + st), ph, a.wait_limit);
       if (!__all_sync(0xffffffffu, got)) {
         if (leader) *fail = 1;
         break;
       }
-      if (a.test_stall && j / PER + 1u == a.test_stall) break;  // test hook: this unit's token rows never arrive
+      if (a.test_stall && j + 1u == a.test_stall) break;  // test hook: this unit's token rows never arrive
       if (leader) {
         mb_expect(bar(QB_B_FULL + st), b_stage);
-        const size_t at = ((size_t)sb * 9u + (size_t)k * KB) * b_group;
-        bulk_in(b0 + st * b_stage, reinterpret_cast<const unsigned char*>(a.xt) + at, b_stage, bar(QB_B_FULL + st));
+        bulk_in(b0 + st * b_stage, reinterpret_cast<const unsigned char*>(a.xt) + (size_t)sb * b_stage, b_stage, bar(QB_B_FULL + st));
       }
       issued++;
       if (++st == a.n_b) {
         st = 0;
         ph ^= 1u;
       }
-      if (++k == PER) {
-        k = 0;
-        if (++sb == a.map.S) sb = 0;
+      if (++sb == a.map.S) sb = 0;
+      __syncwarp();
+    }
+    for (unsigned j = issued > a.n_b ? issued - a.n_b : 0u; j < issued; j++) mb_wait(bar(QB_B_FULL + j % a.n_b), (j / a.n_b) & 1u, a.wait_limit);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (threadIdx.x == 0 && *fail) atomicOr(a.err, 8u);
+  if (warp == 0) tc_dealloc(tmem, 512);
+}
+
+// More than 64 token rows, in blocks of up to 128.  A unit is a super-block of TWO row tiles: the token rows of a half super-block
+// (4 groups of 32 k, or 5 with the minima's) are brought in once and the MMAs of the tiles alternate between two accumulators,
+//   (tile 0, half 0) (tile 1, half 0) (tile 0, half 1) (tile 1, half 1),
+// which halves the traffic of B from L2 (one tile against 256 rows at once read B at 8.9 TB/s and could not go faster).
+// Converting and folding are different warps: with the same 16 warps doing both, the MMAs waited 60 % of the time for an
+// accumulator whose folders stood before a slot of A (13.4k cycles per unit, MMAs 4.5k).  Eight warps convert (32 rows x 128 k
+// each), eight fold (32 rows x half the tokens of both tiles: 128 sums per thread, hence the register split 56 / 168 / 32 of the
+// 96 a thread is launched with).
+constexpr unsigned QW_THREADS = 640, QW_HEAD = 4096;  // 5 groups of 4 warps; barriers, from 512 the scale factors, from 1536 s
+constexpr unsigned QW_D = 256;
+__global__ void __launch_bounds__(QW_THREADS, 1) gemm_q4k_wide_kernel(const __grid_constant__ Q4Args a) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  const uint32_t bars = sm32(smem);
+  auto bar = [&](unsigned i) { return bars + 8u * i; };
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + QB_COUNT * 8);
+  volatile unsigned* fail = reinterpret_cast<volatile unsigned*>(smem + QB_COUNT * 8 + 8);
+  const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  const unsigned tbn = a.map.tbn;
+  const unsigned b_group = 4u * 2u * tbn * 16u, b_stage = 5u * b_group;
+  float* up_s = reinterpret_cast<float*>(smem + 512);    // 2^e of every token row
+  float* s_s = reinterpret_cast<float*>(smem + 1536);    // [4][128]: s of the rows of the last tiles, converters to folders
+  const uint32_t raw0 = bars + QW_HEAD, b0 = raw0 + a.n_raw * Q_RAW;
+  const unsigned u0 = ks_gemm_first(a.map, blockIdx.x), n_units = a.map.base + (blockIdx.x < a.map.rem ? 1u : 0u);
+
+  if (threadIdx.x == 0) {
+    for (unsigned i = 0; i < a.n_raw; i++) {
+      mb_init(bar(QB_RAW_FULL + i), 1);
+      mb_init(bar(QB_RAW_FREE + i), 8);
+    }
+    for (unsigned i = 0; i < a.n_b; i++) {
+      mb_init(bar(QB_B_FULL + i), 1);
+      mb_init(bar(QB_B_FREE + i), 1);
+    }
+    for (unsigned i = 0; i < 3; i++) {
+      mb_init(bar(QB_A_FULL + i), 4);
+      mb_init(bar(QB_A_FREE + i), 1);
+    }
+    for (unsigned i = 0; i < 2; i++) {
+      mb_init(bar(QB_D_FULL + i), 1);
+      mb_init(bar(QB_D_FREE + i), 8);
+    }
+    mb_init(bar(QB_DONE), 1);
+    *fail = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 0) tc_alloc(sm32(tslot), 512);
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (*tslot != 0u && threadIdx.x == 0) *fail = 1;  // all 512 columns were asked for: they start at 0
+  constexpr uint32_t tmem = 0;
+
+  if (warp < 8u) {
+    // ---- converters
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    const unsigned quad = warp & 3u, half = warp >> 2, row = quad * 32u + lane;
+    const uint32_t tlane = tmem + ((quad * 32u) << 16);
+    bool ok = true;
+    unsigned rs = 0, rph = 0;                        // ring stage of the packed rows and its phase
+    unsigned n = 2u * half, slot = n, sph = 1;       // A slot and the phase in which it is free
+    for (unsigned v = 0; v < 2u * n_units && ok; v++) {  // row tiles of units
+      if (!__all_sync(0xffffffffu, mb_wait(bar(QB_RAW_FULL + rs), rph, a.wait_limit))) { ok = false; break; }
+      const uint32_t blk = raw0 + rs * Q_RAW + row * KS_Q4K_BLOCK_BYTES;
+      const uint4 hraw = lds128(blk);
+      if (n >= 3u && !__all_sync(0xffffffffu, mb_wait(bar(QB_A_FREE + slot), sph, a.wait_limit))) { ok = false; break; }
+      tc_fence_after();
+#pragma unroll
+      for (unsigned gg = 0; gg < 2; gg++) {
+        const unsigned g = 2u * half + gg;
+        const uint4 qa = lds128(blk + 16u + 32u * g), qb = lds128(blk + 32u + 32u * g);
+        Q4Hdr h;
+        q4_header(hraw, g, h);
+        if (g == 0) s_s[(v & 3u) * 128u + row] = h.s;
+        const uint32_t at = tlane + slot * 64u + gg * 32u;
+        uint32_t lo[8], hi[8];
+        q4_words(qa, h, lo, hi);
+        tc_st8(at, lo);
+        tc_st8(at + 16u, hi);
+        q4_words(qb, h, lo, hi);
+        tc_st8(at + 8u, lo);
+        tc_st8(at + 24u, hi);
+        tc_st4(tlane + Q_EXT + (v & 3u) * 16u + 4u * g, h.mhi, h.mhi, h.mlo, 0u);
+      }
+      __syncwarp();
+      if (lane == 0) mb_arrive(bar(QB_RAW_FREE + rs));  // the packed bytes are in registers (and used)
+      if (++rs == a.n_raw) {
+        rs = 0;
+        rph ^= 1u;
+      }
+      tc_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mb_arrive(bar(QB_A_FULL + slot));
+      // slots go 4 i + t + 2 half: one on from tile 0 to tile 1, three (the same slot) to the next unit's tile 0
+      const unsigned step = (v & 1u) ? 3u : 1u;
+      n += step;
+      slot += step;
+      if (slot >= 3u) {
+        slot -= 3u;
+        sph ^= 1u;
+      }
+    }
+    if (!ok && lane == 0) *fail = 1;
+  } else if (warp < 16u) {
+    // ---- folders
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
+    const unsigned quad = warp & 3u, th = (warp >> 2) & 1u, row = quad * 32u + lane, tq = tbn >> 1;  // tokens [th * tq, + tq) of the unit's
+    const uint32_t tlane = tmem + ((quad * 32u) << 16);
+    float acc[2][64];
+#pragma unroll
+    for (int t = 0; t < 2; t++)
+#pragma unroll
+      for (int k = 0; k < 64; k++) acc[t][k] = 0.0f;
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the kernels before this one may still read what is written here
+    bool ok = true;
+    unsigned wt = u0 / a.map.S, sb = u0 - wt * a.map.S;
+    for (unsigned i = 0; i < n_units && ok; i++) {
+      const bool last = i + 1u == n_units || sb + 1u == a.map.S;  // the work tile, or this CTA's share of it, ends here
+#pragma unroll
+      for (unsigned t = 0; t < 2; t++) {
+        if (!__all_sync(0xffffffffu, mb_wait(bar(QB_D_FULL + t), i & 1u, a.wait_limit))) { ok = false; break; }
+        tc_fence_after();
+        const float s = s_s[((2u * i + t) & 3u) * 128u + row];
+        const uint32_t dcol = tlane + QW_D + t * tbn + th * tq;
+#pragma unroll
+        for (int c = 0; c < 64; c += 16) {
+          if ((unsigned)c < tq) {
+            uint32_t d0[16];
+            if ((unsigned)c + 16u <= tq) {
+              tc_ld16(dcol + c, d0);
+            } else {
+              tc_ld4(dcol + c, d0);
+              tc_ld4(dcol + c + 4, d0 + 4);
+            }
+            tc_wait_ld16(d0);
+#pragma unroll
+            for (int k = 0; k < 16; k++)
+              if (k < 8 || (unsigned)c + 16u <= tq) acc[t][c + k] = fmaf(s, __uint_as_float(d0[k]), acc[t][c + k]);
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mb_arrive(bar(QB_D_FREE + t));
+        if (last) {
+          const unsigned grp = wt / a.map.tb, tblk = wt - grp * a.map.tb;
+          const Seg sg = pick_seg(a, grp);
+          const unsigned out_row = ((grp - sg.group0) * 2u + t) * GM_ROWS + row, tok0 = tblk * tbn + th * tq;
+          const unsigned pslot = blockIdx.x - ks_gemm_owner(a.map, wt * a.map.S);
+          float* y = sg.y + (size_t)pslot * sg.part + (size_t)tok0 * sg.ldy + out_row;
+          const unsigned n_tok = out_row < sg.rows ? a.n_tok : 0u;
+#pragma unroll
+          for (int k = 0; k < 64; k++) {
+            if ((unsigned)k < tq && tok0 + k < n_tok) *y = acc[t][k] * up_s[tok0 + k];
+            y += sg.ldy;
+            acc[t][k] = 0.0f;
+          }
+        }
+      }
+      if (++sb == a.map.S) {
+        sb = 0;
+        wt++;
+      }
+    }
+    if (!ok && lane == 0) *fail = 1;
+  } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+    if (warp == 16u) {
+    // ---- MMAs: see above
+    const unsigned leader = elect_one();
+    const uint32_t idesc = (1u << 4) | ((tbn >> 3) << 17) | ((unsigned)(GM_ROWS >> 4) << 24);  // f32 accumulate, f16 x f16, K-major both
+    const uint64_t bdesc0 = tc_desc(b0, 2u * tbn * 16u, 128u);
+    const unsigned chunk2 = 4u * tbn, lo_rows = tbn;   // in descriptor units of 16 bytes: two chunks of 8 k, the hi rows
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    bool ok = false;
+    unsigned bs = 0, bph = 0;   // B stage and its phase
+    unsigned sl = 0, sph = 0;   // A slot and its phase: the slots are taken in the order the MMAs go
+    for (unsigned i = 0; i < n_units; i++) {
+#pragma unroll
+      for (unsigned hf = 0; hf < 2; hf++) {
+#pragma unroll
+        for (unsigned t = 0; t < 2; t++) {
+          const uint32_t d = tmem + QW_D + t * tbn;
+          bool got = true;
+          if (hf == 0 && i >= 1u) got = mb_wait(bar(QB_D_FREE + t), (i - 1u) & 1u, a.wait_limit);
+          got = got && mb_wait(bar(QB_A_FULL + sl), sph, a.wait_limit);
+          if (t == 0) got = got && mb_wait(bar(QB_B_FULL + bs), bph, a.wait_limit);
+          if (!__all_sync(0xffffffffu, got)) goto out;
+          tc_fence_after();
+          if (leader) {
+            const uint64_t bd = bdesc0 + (uint64_t)(bs * (b_stage >> 4));
+#pragma unroll
+            for (unsigned kg = 0; kg < 4u + hf; kg++) {  // groups of 32 k; the fifth: the minima
+              const bool ext = kg == 4u;
+              const uint32_t at = ext ? tmem + Q_EXT + ((2u * i + t) & 3u) * 16u : tmem + sl * 64u + kg * 16u;
+              const uint64_t b = bd + (uint64_t)(kg * (b_group >> 4));
+              tc_mma_f16_ta(d, at, b, idesc, (hf | kg) ? 1u : 0u);
+              if (!ext) tc_mma_f16_ta(d, at, b + lo_rows, idesc, 1u);
+              tc_mma_f16_ta(d, at + 8u, b + chunk2, idesc, 1u);
+              if (!ext) tc_mma_f16_ta(d, at + 8u, b + chunk2 + lo_rows, idesc, 1u);
+            }
+            tc_commit(bar(QB_A_FREE + sl));
+            if (t) tc_commit(bar(QB_B_FREE + bs));
+            if (hf) tc_commit(bar(QB_D_FULL + t));
+          }
+          __syncwarp();
+          if (++sl == 3u) {
+            sl = 0;
+            sph ^= 1u;
+          }
+        }
+        if (++bs == a.n_b) {
+          bs = 0;
+          bph ^= 1u;
+        }
+      }
+    }
+    ok = true;
+  out:
+    // every MMA issued must finish before shared and tensor memory go away (bounded): a last commit tracks them all
+    if (leader) {
+      if (!ok) *fail = 1;
+      tc_commit(bar(QB_DONE));
+    }
+    __syncwarp();
+    mb_wait(bar(QB_DONE), 0u, Q_WAIT);
+    } else if (warp == 17u) {
+    // ---- packed rows: they depend on no kernel before this one
+    const unsigned leader = elect_one();
+    unsigned issued = 0, st = 0, ph = 1, wt = u0 / a.map.S, sb = u0 - wt * a.map.S, t = 0;
+    for (unsigned i = 0; i < 2u * n_units; i++) {
+      const bool got = i < a.n_raw || mb_wait(bar(QB_RAW_FREE + st), ph, a.wait_limit);
+      if (!__all_sync(0xffffffffu, got)) {
+        if (leader) *fail = 1;
+        break;
+      }
+      if (leader) {
+        const unsigned grp = wt / a.map.tb;
+        const int k = (grp >= a.group0[1]) + (grp >= a.group0[2]);
+        const unsigned g0 = k == 0 ? a.group0[0] : k == 1 ? a.group0[1] : a.group0[2];
+        mb_expect(bar(QB_RAW_FULL + st), Q_RAW);  // rows past the matrix come as zeros and count
+        tma_in_2d(raw0 + st * Q_RAW, k == 0 ? &a.w[0] : k == 1 ? &a.w[1] : &a.w[2], sb * KS_Q4K_BLOCK_BYTES, ((grp - g0) * 2u + t) * GM_ROWS,
+                  bar(QB_RAW_FULL + st));
+      }
+      issued++;
+      if (++st == a.n_raw) {
+        st = 0;
+        ph ^= 1u;
+      }
+      if (++t == 2u) {
+        t = 0;
+        if (++sb == a.map.S) {
+          sb = 0;
+          wt++;
+        }
+      }
+      __syncwarp();
+    }
+    for (unsigned j = issued > a.n_raw ? issued - a.n_raw : 0u; j < issued; j++) mb_wait(bar(QB_RAW_FULL + j % a.n_raw), (j / a.n_raw) & 1u, a.wait_limit);
+    } else if (warp == 18u) {
+    // ---- token rows
+    const unsigned leader = elect_one();
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the image comes from the kernel before this one
+    const float* up = reinterpret_cast<const float*>(a.xt + xt_scale_off(a.cols, a.np));
+    for (unsigned t = lane; t < a.np; t += 32u) up_s[t] = up[t];  // read behind the first accumulator, which waits for the copies below
+    __syncwarp();
+    unsigned issued = 0, wt = u0 / a.map.S, sb = u0 - wt * a.map.S, hf = 0, st = 0, ph = 1;
+    for (unsigned j = 0; j < 2u * n_units; j++) {  // halves of a super-block: 4 and 5 groups
+      const bool got = j < a.n_b || mb_wait(bar(QB_B_FREE + st), ph, a.wait_limit);
+      if (!__all_sync(0xffffffffu, got)) {
+        if (leader) *fail = 1;
+        break;
+      }
+      if (a.test_stall && j / 2u + 1u == a.test_stall) break;  // test hook: this unit's token rows never arrive
+      if (leader) {
+        const unsigned tblk = wt % a.map.tb, bytes = (4u + hf) * b_group;
+        const size_t at = (((size_t)tblk * a.map.S + sb) * 9u + 4u * hf) * b_group;
+        mb_expect(bar(QB_B_FULL + st), bytes);
+        bulk_in(b0 + st * b_stage, reinterpret_cast<const unsigned char*>(a.xt) + at, bytes, bar(QB_B_FULL + st));
+      }
+      issued++;
+      if (++st == a.n_b) {
+        st = 0;
+        ph ^= 1u;
+      }
+      if (++hf == 2u) {
+        hf = 0;
+        if (++sb == a.map.S) {
+          sb = 0;
+          wt++;
+        }
       }
       __syncwarp();
     }
     for (unsigned j = issued > a.n_b ? issued - a.n_b : 0u; j < issued; j++) mb_wait(bar(QB_B_FULL + j % a.n_b), (j / a.n_b) & 1u, a.wait_limit);
+    }
   }
   tc_fence_before();
   __syncthreads();
@@ -489,31 +758,37 @@ encode_fn tensor_map_encoder() {
 
 // Ring depths: two B stages at least, then packed rows up to the four units that cover the latency of memory, then whatever
 // of either still fits.
-size_t q4_rings(const ks_ctx* ctx, unsigned np, unsigned kb, unsigned* n_raw, unsigned* n_b) {
-  const size_t room = ctx->smem_optin - Q_HEAD, stage = (size_t)kb * np * 128u;
+size_t q4_rings(const ks_ctx* ctx, unsigned tbn, unsigned nt, unsigned* n_raw, unsigned* n_b) {
+  const size_t head = nt == 1 ? Q_HEAD : QW_HEAD, room = ctx->smem_optin - head, stage = (size_t)(nt == 1 ? 9 : 5) * tbn * 128u;
   *n_raw = 2;
-  *n_b = kb == 1 ? 4 : kb == 3 ? 3 : 2;
+  *n_b = 2;
   auto fits = [&](unsigned r, unsigned b) { return r <= Q_MAX_RAW && b <= Q_MAX_B && b * stage + r * Q_RAW <= room; };
   while (*n_raw < 4 && fits(*n_raw + 1, *n_b)) ++*n_raw;
   while (fits(*n_raw, *n_b + 1)) ++*n_b;
   while (fits(*n_raw + 1, *n_b)) ++*n_raw;
-  return Q_HEAD + *n_b * stage + *n_raw * Q_RAW;
+  return head + *n_b * stage + *n_raw * Q_RAW;
 }
 }  // namespace
 
 // How many CTAs a launch of `tiles` tiles takes.  A CTA's time is its units (t_u each) plus writing its shares of tiles; the
 // partials are then read once more.  More CTAs mean fewer units each and more partials.
-ks_gemm_map ks_gemm_q4k_map(const ks_ctx* ctx, unsigned tiles, unsigned cols, unsigned np) {
+ks_gemm_map ks_gemm_q4k_map(const ks_ctx* ctx, const size_t* rows, int n_seg, unsigned cols, unsigned np) {
   ks_gemm_map m{};
   m.S = cols / 256u;
-  const unsigned U = tiles * m.S, most = (unsigned)ctx->sm_count < U ? (unsigned)ctx->sm_count : U;
-  const double t_u = 0.45 + np * 0.0085, t_w = 0.1 + np * 0.005;
+  m.tbn = q4k_block(np);
+  m.tb = np / m.tbn;
+  m.nt = np > 64u ? 2u : 1u;
+  unsigned wtiles = 0;
+  for (int i = 0; i < n_seg; i++) wtiles += (unsigned)(((rows[i] + GM_ROWS - 1) / GM_ROWS + m.nt - 1) / m.nt);
+  wtiles *= m.tb;
+  const unsigned U = wtiles * m.S, most = (unsigned)ctx->sm_count < U ? (unsigned)ctx->sm_count : U;
+  const double t_u = (0.45 + m.tbn * 0.0085) * m.nt, t_w = (0.1 + m.tbn * 0.005) * m.nt;
   double best = 1e30;
   for (unsigned G = 1; G <= most; G++) {
-    if (G < most && tiles % G && G * 4u < most * 3u) continue;
+    if (G < most && wtiles % G && G * 4u < most * 3u) continue;
     const unsigned per = (U + G - 1) / G, shares = (per + m.S - 2) / m.S + 1;
-    const double slots = (double)G / tiles + 1.0;
-    const double cost = per * t_u + shares * t_w + slots * tiles * np * (GM_ROWS * 4e-6 / 5.0);
+    const double slots = (double)G / wtiles + 1.0;
+    const double cost = per * t_u + shares * t_w + slots * wtiles * m.nt * m.tbn * (GM_ROWS * 4e-6 / 5.0);
     if (cost < best) {
       best = cost;
       m.G = G;
@@ -530,44 +805,42 @@ int ks_launch_gemm_q4k(ks_ctx* ctx, const ks_gemm_job& job) {
   Q4Args a;
   memset(&a, 0, sizeof a);
   const cuuint64_t row_bytes = (cuuint64_t)job.cols / 256 * KS_Q4K_BLOCK_BYTES;
-  unsigned tiles = 0;
+  unsigned groups = 0;
   for (int i = 0; i < 3; i++) {
-    a.tile0[i] = i < job.n_seg ? tiles : 0xFFFFFFFFu;  // no tile reaches an absent matrix
+    a.group0[i] = i < job.n_seg ? groups : 0xFFFFFFFFu;  // no unit reaches an absent matrix
     if (i >= job.n_seg) continue;
     a.rows[i] = (unsigned)job.rows[i];
     a.y[i] = job.y[i];
     a.ldy[i] = job.ldy[i];
     a.part_stride[i] = job.part_stride[i];
-    tiles += (unsigned)((job.rows[i] + GM_ROWS - 1) / GM_ROWS);
+    groups += (unsigned)(((job.rows[i] + GM_ROWS - 1) / GM_ROWS + job.map.nt - 1) / job.map.nt);
     const cuuint64_t dims[2] = {row_bytes, (cuuint64_t)job.rows[i]}, strides[1] = {row_bytes};
     const cuuint32_t box[2] = {KS_Q4K_BLOCK_BYTES, GM_ROWS}, es[2] = {1, 1};
     if (enc(&a.w[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t*>(job.W[i]), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return ks_fail(ctx, KS_ERR_INVALID, "gemm: the packed rows cannot be described to TMA (base must be 16-byte aligned)");
   }
-  a.tile0[3] = tiles;
   a.map = job.map;
   a.xt = job.xt;
   a.cols = job.cols;
   a.n_tok = job.n_tok;
   a.np = job.np;
-  const int c = job.np <= 16 ? 0 : job.np <= 32 ? 1 : job.np <= 64 ? 2 : job.np <= 128 ? 3 : 4;
-  const size_t smem = q4_rings(ctx, job.np, q4_kb(4 << c), &a.n_raw, &a.n_b);
+  const int c = job.np <= 16 ? 0 : job.np <= 32 ? 1 : job.np <= 64 ? 2 : 3;
+  const size_t smem = q4_rings(ctx, job.map.tbn, job.map.nt, &a.n_raw, &a.n_b);
   a.err = (unsigned*)ctx->ws + KS_WS_ERR_WORD;
   a.wait_limit = Q_WAIT;
   if (const char* t = getenv("KSEARCH_GEMM_TEST_STALL")) {  // exercises the give-up path: short waits, one operand withheld
     a.test_stall = (unsigned)atoi(t);
     if (a.test_stall) a.wait_limit = 4000;
   }
-  void (*kern)(Q4Args) = c == 0 ? gemm_q4k_tc_kernel<4> : c == 1 ? gemm_q4k_tc_kernel<8> : c == 2 ? gemm_q4k_tc_kernel<16>
-                       : c == 3 ? gemm_q4k_tc_kernel<32> : gemm_q4k_tc_kernel<64>;
-  static size_t set[5][16] = {{0}};
+  void (*kern)(Q4Args) = c == 0 ? gemm_q4k_tc_kernel<4> : c == 1 ? gemm_q4k_tc_kernel<8> : c == 2 ? gemm_q4k_tc_kernel<16> : gemm_q4k_wide_kernel;
+  static size_t set[4][16] = {{0}};
   size_t& have = set[c][ctx->device & 15];
   if (smem > have) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return ks_fail(ctx, KS_ERR_CUDA, "gemm: cannot set %zu B shared memory: %s", smem, cudaGetErrorString(e));
     have = smem;
   }
-  KS_LAUNCH(ctx, kern, dim3(job.map.G), Q_THREADS, smem, a);
+  KS_LAUNCH(ctx, kern, dim3(job.map.G), c == 3 ? QW_THREADS : Q_THREADS, smem, a);
   return ks_after_launch(ctx, "gemm_q4k_tc");
 }

@@ -821,8 +821,8 @@ ks_model* ks_model_create(ks_ctx* ctx, const ks_model_config* cfg) {
         const int most = i < 4 ? G : g.n_slots;  // only decode steps reach the head
         const size_t a = ks_gemm_xt_bytes(cols_of[i], most);
         xt = a > xt ? a : xt;
-        for (int n = 1; n <= most; n += n < 16 ? 15 : 16) {  // fewer rows are split finer
-          const int rows = n + 15 < most ? n + 15 : most;
+        for (int n = 16; n < most + 16; n += 16) {  // fewer rows are split finer
+          const int rows = n < most ? n : most;
           const size_t b = 4 * ks_gemm_part_floats(ctx, rows_of[i], cols_of[i], rows);
           part = b > part ? b : part;
         }

@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(512) sdpa_merge_split_kernel(unsigned n_tok, u
     if (ck < chunks) {
 #pragma unroll
       for (int e = 0; e < 8; e++) v[kk][e] *= down;
-      put_split8(xt, np, t, ck, v[kk], true);
+      put_split8(xt, np, t, ck, chunks, v[kk], true);
     }
   }
 }
