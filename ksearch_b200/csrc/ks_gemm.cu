@@ -26,6 +26,7 @@
 //     tcgen05.ld, scaled by 2^-6 and stored coalesced along the weight-row index.
 // Every wait is bounded; on expiry the CTA raises the context's status word, waits (bounded) for what it has in
 // flight, frees its tensor memory and returns.
+#include <cooperative_groups.h>
 #include <cuda_fp16.h>
 
 #include <cstdlib>
@@ -417,6 +418,28 @@ namespace {
 //   y = sum of partials;  x = res + rms(y) * w_post (lower.rs:3926-4077, the residual update of lib.rs:539);
 //   the image of rms(x) * w_norm for the next GEMM.
 // The f32 normed vector is not stored: on this path only a GEMM reads it.  Rows past n_tok become zeros.
+// Eight neighbouring rows of a token's partials, FLY partials in flight at a time: read one after the other, the partials of a
+// down-projection (12 row tiles over 148 CTAs: 13 each) cost 13 trips to L2, 9 us a launch instead of 5.
+template <unsigned FLY>
+__device__ __forceinline__ void sum8(const float* p, size_t stride, unsigned n, float (&y)[8]) {
+#pragma unroll
+  for (int i = 0; i < 8; i++) y[i] = 0.0f;
+  for (unsigned s = 0; s < n; s += FLY) {
+    float4 a[FLY], b[FLY];
+#pragma unroll
+    for (unsigned k = 0; k < FLY; k++)
+      if (s + k < n) {
+        a[k] = *reinterpret_cast<const float4*>(p + (size_t)(s + k) * stride);
+        b[k] = *reinterpret_cast<const float4*>(p + (size_t)(s + k) * stride + 4);
+      }
+#pragma unroll
+    for (unsigned k = 0; k < FLY; k++)
+      if (s + k < n) {
+        y[0] += a[k].x; y[1] += a[k].y; y[2] += a[k].z; y[3] += a[k].w;
+        y[4] += b[k].x; y[5] += b[k].y; y[6] += b[k].z; y[7] += b[k].w;
+      }
+  }
+}
 struct EpiNormArgs {
   const float* P;
   size_t part_stride;
@@ -434,17 +457,18 @@ __global__ void gemm_finish_norm_split_kernel(const EpiNormArgs e) {
   const unsigned t = blockIdx.x, ck = threadIdx.x, chunks = e.rows / 8u;
   const bool live = ck < chunks && t < e.n_tok;
   float y[8];
-#pragma unroll
-  for (int i = 0; i < 8; i++) y[i] = 0.0f;
   const size_t at = (size_t)t * e.rows + 8u * ck;
+  // everything that does not depend on the sums is requested first
+  float4 r0{}, r1{}, p0{}, p1{}, n0{}, n1{};
   if (live) {
-    const unsigned n = ks_gemm_slots(e.map, 0u, 8u * ck / GM_ROWS, t);
-    for (unsigned s = 0; s < n; s++) {
-      const float4 a = *reinterpret_cast<const float4*>(e.P + (size_t)s * e.part_stride + at);
-      const float4 b = *reinterpret_cast<const float4*>(e.P + (size_t)s * e.part_stride + at + 4);
-      y[0] += a.x; y[1] += a.y; y[2] += a.z; y[3] += a.w; y[4] += b.x; y[5] += b.y; y[6] += b.z; y[7] += b.w;
-    }
+    r0 = *reinterpret_cast<const float4*>(e.res + at);
+    r1 = *reinterpret_cast<const float4*>(e.res + at + 4);
+    p0 = *reinterpret_cast<const float4*>(e.w_post + 8u * ck);
+    p1 = *reinterpret_cast<const float4*>(e.w_post + 8u * ck + 4);
+    n0 = *reinterpret_cast<const float4*>(e.w_norm + 8u * ck);
+    n1 = *reinterpret_cast<const float4*>(e.w_norm + 8u * ck + 4);
   }
+  sum8<4>(e.P + at, e.part_stride, live ? ks_gemm_slots(e.map, 0u, 8u * ck / GM_ROWS, t) : 0u, y);
   float ss = 0.0f;
 #pragma unroll
   for (int i = 0; i < 8; i++) ss = fmaf(y[i], y[i], ss);
@@ -454,8 +478,6 @@ __global__ void gemm_finish_norm_split_kernel(const EpiNormArgs e) {
 #pragma unroll
   for (int i = 0; i < 8; i++) v[i] = 0.0f;
   if (live) {
-    const float4 r0 = *reinterpret_cast<const float4*>(e.res + at), r1 = *reinterpret_cast<const float4*>(e.res + at + 4);
-    const float4 p0 = *reinterpret_cast<const float4*>(e.w_post + 8u * ck), p1 = *reinterpret_cast<const float4*>(e.w_post + 8u * ck + 4);
     const float rr[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w}, pp[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
 #pragma unroll
     for (int i = 0; i < 8; i++) v[i] = __fadd_rn(rr[i], __fmul_rn(__fmul_rn(y[i], inv), pp[i]));
@@ -470,7 +492,6 @@ __global__ void gemm_finish_norm_split_kernel(const EpiNormArgs e) {
 #pragma unroll
   for (int i = 0; i < 8; i++) xn[i] = 0.0f;
   if (live) {
-    const float4 n0 = *reinterpret_cast<const float4*>(e.w_norm + 8u * ck), n1 = *reinterpret_cast<const float4*>(e.w_norm + 8u * ck + 4);
     const float nn[8] = {n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, n1.z, n1.w};
 #pragma unroll
     for (int i = 0; i < 8; i++) xn[i] = __fmul_rn(__fmul_rn(v[i], inv2), nn[i]);
@@ -485,55 +506,154 @@ __global__ void gemm_finish_norm_split_kernel(const EpiNormArgs e) {
   }
 }
 
-// gelu(sum of gate partials) * (sum of up partials) (lib.rs:953) straight into the image the down GEMM reads.
-constexpr int GM_GELU_CHUNKS = 2;     // 8-value chunks per thread
-constexpr int GM_ROW_THREADS = 1024;  // threads of a block that writes one token row of an image: rows up to 2 * 8 * 1024 = 16384
-__global__ void __launch_bounds__(GM_ROW_THREADS) gemm_finish_gelu_split_kernel(const float* P0, const float* P1, size_t part_stride, ks_gemm_map map,
-                                                                               unsigned n_tok, unsigned np, unsigned rows, __half* xt) {
+constexpr int GM_ROW_THREADS = 1024;  // threads of a block that writes one token row of an image
+// gelu(sum of gate partials) * (sum of up partials) (lib.rs:953) straight into the image the down GEMM reads.  A cluster of four
+// blocks per (padded) token row, 8 values per thread: the row maximum that scales the image meets in distributed shared memory,
+// and few token rows still make enough blocks (8 rows of 10240 values: 64 blocks instead of 16).
+constexpr unsigned GM_GELU_CL = 4, GM_GELU_THREADS = 512;
+__global__ void __cluster_dims__(GM_GELU_CL, 1, 1) __launch_bounds__(GM_GELU_THREADS)
+    gemm_finish_gelu_split_kernel(const float* P0, const float* P1, size_t part_stride, ks_gemm_map map, unsigned n_tok, unsigned np, unsigned rows,
+                                  __half* xt) {
   ks_pdl_entry();
-  __shared__ float red[32];
-  const unsigned t = blockIdx.x, chunks = rows / 8u;  // one block per (padded) token row
-  float v[GM_GELU_CHUNKS][8];
-  float m = 0.0f;
+  __shared__ float red[32], maxima[GM_GELU_CL];
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const unsigned rank = blockIdx.x % GM_GELU_CL, t = blockIdx.x / GM_GELU_CL, chunks = rows / 8u, ck = rank * blockDim.x + threadIdx.x;
+  float v[8];
 #pragma unroll
-  for (int kk = 0; kk < GM_GELU_CHUNKS; kk++) {
-    const unsigned ck = threadIdx.x + (unsigned)kk * blockDim.x;
+  for (int k = 0; k < 8; k++) v[k] = 0.0f;
+  if (t < n_tok && ck < chunks) {
+    float g[8], u[8];
+    const size_t at = (size_t)t * rows + 8u * ck;
+    const unsigned tile = 8u * ck / GM_ROWS, groups = map.G ? ((rows + GM_ROWS - 1u) / GM_ROWS + map.nt - 1u) / map.nt : 0u;
+    sum8<4>(P0 + at, part_stride, ks_gemm_slots(map, 0u, tile, t), g);
+    sum8<4>(P1 + at, part_stride, ks_gemm_slots(map, groups, tile, t), u);
 #pragma unroll
-    for (int k = 0; k < 8; k++) v[kk][k] = 0.0f;
-    if (t < n_tok && ck < chunks) {
-      float g[8], u[8];
-#pragma unroll
-      for (int k = 0; k < 8; k++) g[k] = u[k] = 0.0f;
-      const size_t at = (size_t)t * rows + 8u * ck;
-      const unsigned tile = 8u * ck / GM_ROWS, groups = map.G ? ((rows + GM_ROWS - 1u) / GM_ROWS + map.nt - 1u) / map.nt : 0u,
-                     ng = ks_gemm_slots(map, 0u, tile, t), nu = ks_gemm_slots(map, groups, tile, t);
-      for (unsigned s = 0; s < ng; s++) {
-        const float4 a = *reinterpret_cast<const float4*>(P0 + (size_t)s * part_stride + at);
-        const float4 b = *reinterpret_cast<const float4*>(P0 + (size_t)s * part_stride + at + 4);
-        g[0] += a.x; g[1] += a.y; g[2] += a.z; g[3] += a.w; g[4] += b.x; g[5] += b.y; g[6] += b.z; g[7] += b.w;
-      }
-      for (unsigned s = 0; s < nu; s++) {
-        const float4 c = *reinterpret_cast<const float4*>(P1 + (size_t)s * part_stride + at);
-        const float4 d = *reinterpret_cast<const float4*>(P1 + (size_t)s * part_stride + at + 4);
-        u[0] += c.x; u[1] += c.y; u[2] += c.z; u[3] += c.w; u[4] += d.x; u[5] += d.y; u[6] += d.z; u[7] += d.w;
-      }
-#pragma unroll
-      for (int k = 0; k < 8; k++) v[kk][k] = gelu_mul(g[k], u[k]);
-      m = fmaxf(m, absmax8(v[kk]));
-    }
+    for (int k = 0; k < 8; k++) v[k] = gelu_mul(g[k], u[k]);
   }
   // gelu(gate) * up is where a random-weight model leaves the f16 range
+  const float m = block_max_f(absmax8(v), red);
+  if (threadIdx.x < GM_GELU_CL) *cluster.map_shared_rank(&maxima[rank], threadIdx.x) = m;
+  cluster.sync();
+  float row_max = maxima[0];
+#pragma unroll
+  for (unsigned k = 1; k < GM_GELU_CL; k++) row_max = fmaxf(row_max, maxima[k]);
   float up;
-  const float down = row_scale_down(block_max_f(m, red), &up);
-  if (threadIdx.x == 0) reinterpret_cast<float*>(xt + xt_scale_off(rows, np))[t] = up;
+  const float down = row_scale_down(row_max, &up);
+  if (rank == 0 && threadIdx.x == 0) reinterpret_cast<float*>(xt + xt_scale_off(rows, np))[t] = up;
+  if (ck < chunks) {
 #pragma unroll
-  for (int kk = 0; kk < GM_GELU_CHUNKS; kk++) {
-    const unsigned ck = threadIdx.x + (unsigned)kk * blockDim.x;
-    if (ck < chunks) {
+    for (int k = 0; k < 8; k++) v[k] *= down;
+    put_split8(xt, np, t, ck, chunks, v, true);  // a down-projection is always Q4_K
+  }
+}
+
+// The q, k and v partials of a token through per-head RMS norm, RoPE and the Q4_0 pack of K and V (lower.rs:4231-4702), one warp
+// per (token, head).  A lane holds HD / 64 neighbouring dims of each half of the head, so RoPE partners sit in one lane and a
+// 32-value block in 8 (16) neighbouring lanes.
+struct EpiQkvArgs {
+  const float* P[3];
+  size_t part_stride[3];
+  unsigned rows[3], group0[3];
+  ks_gemm_map map;
+  unsigned n_tok, n_q, n_kv;
+  float eps;
+  const float *qw, *kw, *rope;
+  const int* pos;
+  float* q_out;
+  uint8_t *kv_k, *kv_v;
+  size_t slot_stride;
+};
+template <int HD>
+__global__ void __launch_bounds__(256) gemm_finish_qkv_kernel(const EpiQkvArgs e) {
+  constexpr int V = HD / 64, LPB = 32 / V;  // values per lane and half, lanes per 32-value block
+  constexpr unsigned ROWB = HD / 32 * KS_Q40_BLOCK_BYTES;
+  ks_pdl_entry();
+  const unsigned lane = threadIdx.x & 31u, jobs = e.n_q + 2u * e.n_kv, id = blockIdx.x * 8u + (threadIdx.x >> 5);
+  if (id >= e.n_tok * jobs) return;
+  const unsigned tok = id / jobs, job = id - tok * jobs;
+  const int seg = (job >= e.n_q) + (job >= e.n_q + e.n_kv);
+  const unsigned head = seg == 0 ? job : seg == 1 ? job - e.n_q : job - e.n_q - e.n_kv;
+  const float* P = seg == 0 ? e.P[0] : seg == 1 ? e.P[1] : e.P[2];
+  const size_t ps = seg == 0 ? e.part_stride[0] : seg == 1 ? e.part_stride[1] : e.part_stride[2];
+  const unsigned rows = seg == 0 ? e.rows[0] : seg == 1 ? e.rows[1] : e.rows[2], g0 = seg == 0 ? e.group0[0] : seg == 1 ? e.group0[1] : e.group0[2];
+  const size_t p = (size_t)e.pos[tok];
+  const float* cs = e.rope + p * HD;
+  float c[V], sn[V], w[2][V], x[2][V];
 #pragma unroll
-      for (int k = 0; k < 8; k++) v[kk][k] *= down;
-      put_split8(xt, np, t, ck, chunks, v[kk], true);  // a down-projection is always Q4_K
+  for (int k = 0; k < V; k++) {
+    const unsigned d = lane * V + k;
+    c[k] = cs[d];
+    sn[k] = cs[HD / 2 + d];
+    w[0][k] = seg == 0 ? e.qw[d] : seg == 1 ? e.kw[d] : 1.0f;
+    w[1][k] = seg == 0 ? e.qw[HD / 2 + d] : seg == 1 ? e.kw[HD / 2 + d] : 1.0f;
+  }
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const unsigned row = head * HD + (unsigned)h * (HD / 2) + lane * V;
+    const unsigned n = ks_gemm_slots(e.map, g0, row / GM_ROWS, tok);
+    const float* src = P + (size_t)tok * rows + row;
+#pragma unroll
+    for (int k = 0; k < V; k++) x[h][k] = 0.0f;
+#pragma unroll 4
+    for (unsigned s = 0; s < n; s++)
+      if constexpr (V == 4) {
+        const float4 a = *reinterpret_cast<const float4*>(src + (size_t)s * ps);
+        x[h][0] += a.x; x[h][1] += a.y; x[h][2] += a.z; x[h][3] += a.w;
+      } else {
+        const float2 a = *reinterpret_cast<const float2*>(src + (size_t)s * ps);
+        x[h][0] += a.x; x[h][1] += a.y;
+      }
+  }
+  float ss = 0.0f;
+#pragma unroll
+  for (int k = 0; k < V; k++) ss = fmaf(x[0][k], x[0][k], fmaf(x[1][k], x[1][k], ss));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  const float inv = 1.0f / sqrtf(ss / (float)HD + e.eps);
+  float y[2][V];
+#pragma unroll
+  for (int k = 0; k < V; k++) {
+    const float u = __fmul_rn(__fmul_rn(x[0][k], inv), w[0][k]), v = __fmul_rn(__fmul_rn(x[1][k], inv), w[1][k]);
+    y[0][k] = seg == 2 ? u : __fsub_rn(__fmul_rn(u, c[k]), __fmul_rn(v, sn[k]));
+    y[1][k] = seg == 2 ? v : __fadd_rn(__fmul_rn(u, sn[k]), __fmul_rn(v, c[k]));
+  }
+  if (seg == 0) {
+    float* o = e.q_out + (size_t)tok * e.rows[0] + head * HD + lane * V;
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+      if constexpr (V == 4) *reinterpret_cast<float4*>(o + h * (HD / 2)) = make_float4(y[h][0], y[h][1], y[h][2], y[h][3]);
+      else *reinterpret_cast<float2*>(o + h * (HD / 2)) = make_float2(y[h][0], y[h][1]);
+    return;
+  }
+  uint8_t* dst = (seg == 1 ? e.kv_k : e.kv_v) + (size_t)tok * e.slot_stride + (p * e.n_kv + head) * ROWB;
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    float amax = 0.0f, val[V];
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+      val[k] = __half2float(__float2half_rn(y[h][k]));  // values pass through f16 before packing (render.rs:1046)
+      amax = fmaxf(amax, fabsf(val[k]));
     }
+#pragma unroll
+    for (int o = LPB / 2; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    const float scale = amax > 0.0f ? amax / 7.0f : 1.0f, is = 1.0f / scale;
+    unsigned q = 0;
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+      int i = (int)roundf(__fmul_rn(val[k], is)) + 8;
+      i = i < 0 ? 0 : i > 15 ? 15 : i;
+      q |= (unsigned)i << (8 * k);
+    }
+    q |= __shfl_down_sync(0xffffffffu, q, LPB / 2) << 4;  // the block's second sixteen go to the high nibbles
+    const unsigned l = lane % LPB;
+    uint8_t* blk = dst + ((unsigned)h * (HD / 64) + lane / LPB) * KS_Q40_BLOCK_BYTES;
+    if (l < LPB / 2) {
+      unsigned short* o = reinterpret_cast<unsigned short*>(blk + 2 + l * V);
+      o[0] = (unsigned short)q;
+      if constexpr (V == 4) o[1] = (unsigned short)(q >> 16);
+    }
+    if (l == 0) *reinterpret_cast<__half*>(blk) = __float2half_rn(scale);
   }
 }
 }  // namespace
@@ -614,7 +734,9 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
                         int n_tok, float* const* y, const size_t* ldy, float* P, int mode, const ks_gemm_epi* epi) {
   if (!gemm_covers(wdtype, cols, n_tok) || n_seg < 1 || n_seg > 3) return ks_fail(ctx, KS_ERR_UNSUPPORTED, "gemm: shape not covered");
   if ((mode == KS_GEMM_NORM_SPLIT && (n_seg != 1 || !epi || rows[0] % 8 || rows[0] > 8192)) ||
-      (mode == KS_GEMM_GELU_SPLIT && (n_seg != 2 || !epi || rows[0] != rows[1] || rows[0] % 8 || rows[0] > 8u * GM_GELU_CHUNKS * GM_ROW_THREADS)))
+      (mode == KS_GEMM_QKV && (n_seg != 3 || !epi || (epi->hd != 128 && epi->hd != 256) || rows[0] != (size_t)epi->n_q * epi->hd ||
+                               rows[1] != (size_t)epi->n_kv * epi->hd || rows[2] != rows[1])) ||
+      (mode == KS_GEMM_GELU_SPLIT && (n_seg != 2 || !epi || rows[0] != rows[1] || rows[0] % 8 || rows[0] > 8u * GM_GELU_CL * GM_GELU_THREADS || rows[0] % 256)))
     return ks_fail(ctx, KS_ERR_INVALID, "gemm: bad epilogue arguments");
   const unsigned np = gemm_np(n_tok);
   const ks_gemm_map map = gemm_map(ctx, wdtype, rows, n_seg, cols, n_tok);
@@ -732,9 +854,37 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
     KS_LAUNCH(ctx, (gemm_finish_norm_split_kernel), np, (unsigned)((rows[0] / 8 + 31) / 32 * 32), 0, e);
     return ks_after_launch(ctx, "gemm_finish_norm_split");
   }
+  if (mode == KS_GEMM_QKV) {
+    EpiQkvArgs e{};
+    for (int i = 0; i < 3; i++) {
+      e.P[i] = out[i];
+      e.part_stride[i] = part_stride[i];
+      e.rows[i] = (unsigned)rows[i];
+      e.group0[i] = group0[i];
+    }
+    e.map = map;
+    e.n_tok = (unsigned)n_tok;
+    e.n_q = epi->n_q;
+    e.n_kv = epi->n_kv;
+    e.eps = epi->eps;
+    e.qw = epi->qw;
+    e.kw = epi->kw;
+    e.rope = epi->rope;
+    e.pos = epi->pos;
+    e.q_out = epi->out_x;
+    e.kv_k = epi->kv_k;
+    e.kv_v = epi->kv_v;
+    e.slot_stride = epi->slot_stride;
+    const unsigned grid = (e.n_tok * (e.n_q + 2 * e.n_kv) + 7) / 8;
+    if (epi->hd == 256) KS_LAUNCH(ctx, (gemm_finish_qkv_kernel<256>), grid, 256, 0, e);
+    else KS_LAUNCH(ctx, (gemm_finish_qkv_kernel<128>), grid, 256, 0, e);
+    return ks_after_launch(ctx, "gemm_finish_qkv");
+  }
   if (mode == KS_GEMM_GELU_SPLIT) {
-    KS_LAUNCH(ctx, (gemm_finish_gelu_split_kernel), np, GM_ROW_THREADS, 0, (const float*)out[0], (const float*)out[1],
-              part_stride[0], map, (unsigned)n_tok, np, (unsigned)rows[0], (__half*)epi->xt_out);
+    // whole warps per block: a 32-value sub-block of the image is four neighbouring lanes of one
+    const unsigned threads = ((unsigned)rows[0] / 8u / GM_GELU_CL + 31u) / 32u * 32u;
+    KS_LAUNCH(ctx, (gemm_finish_gelu_split_kernel), np * GM_GELU_CL, threads, 0, (const float*)out[0], (const float*)out[1], part_stride[0], map,
+              (unsigned)n_tok, np, (unsigned)rows[0], (__half*)epi->xt_out);
     return ks_after_launch(ctx, "gemm_finish_gelu_split");
   }
   f.n_seg = (unsigned)n_seg;

@@ -141,10 +141,11 @@ int ks_launch_per_head_qkv_q40(ks_ctx* ctx, size_t n_q, size_t n_kv, size_t hd, 
                                const int* pos_dev, size_t slot_stride_bytes);
 int ks_launch_sdpa(ks_ctx* ctx, size_t n_slots, size_t n_q, size_t n_kv, size_t hd, float scale, ks_dtype act,
                    const void* q, const uint8_t* K, const uint8_t* V, size_t slot_stride_bytes, const float* meta,
-                   float* tmp, void* out, int n_splits);
+                   float* tmp, void* out, int n_splits, bool records_only = false);  // records_only: the splits stay in tmp, unmerged
 // A prompt chunk's rows against one slot's cache on the tensor cores (ks_sdpa_chunk.cu), and the merge of its records into
 // the operand image of the output projection.
 int ks_sdpa_chunk_splits(const ks_ctx* ctx, int n_tok, size_t n_q, size_t n_kv, size_t ctx_len, int most);
+bool ks_sdpa_merge_split_covers(size_t n_q, size_t hd);
 bool ks_sdpa_chunk_covers(size_t n_q, size_t n_kv, size_t hd, const void* K, const void* V);
 int ks_launch_sdpa_chunk(ks_ctx* ctx, int n_tok, size_t n_q, size_t n_kv, size_t hd, float scale, const float* q, const uint8_t* K,
                          const uint8_t* V, const float* meta, float* tmp, int n_splits);
@@ -187,13 +188,19 @@ int ks_launch_gemm_split(ks_ctx* ctx, ks_dtype wdtype, const float* x, size_t ld
 // the sums: PLAIN y[i] = W[i] x; GELU (two matrices) y[0] = gelu(W[0] x) * (W[1] x); NORM_SPLIT (one matrix)
 // out_x = res + rms(W x) * w_post and the image of rms(out_x) * w_norm for the next GEMM in xt_out; GELU_SPLIT
 // (two matrices) the image of gelu(W[0] x) * (W[1] x) in xt_out.  P: ks_gemm_part_floats(sum of rows) floats.
-enum { KS_GEMM_PLAIN = 0, KS_GEMM_GELU = 1, KS_GEMM_NORM_SPLIT = 2, KS_GEMM_GELU_SPLIT = 3 };
+// QKV (three matrices): per-head norm and RoPE of q into out_x, of k and v into the cache rows (Q4_0).
+enum { KS_GEMM_PLAIN = 0, KS_GEMM_GELU = 1, KS_GEMM_NORM_SPLIT = 2, KS_GEMM_GELU_SPLIT = 3, KS_GEMM_QKV = 4 };
 struct ks_gemm_epi {
   const float *res, *w_post, *w_norm;  // NORM_SPLIT: residual rows [n_tok, rows], the two norm weights
   float eps;
   float* out_x;                        // NORM_SPLIT: the updated residual rows
   void* xt_out;                        // the image written for the next GEMM (may be the image this GEMM read)
   ks_dtype next_dtype;                 // NORM_SPLIT: weights of that next GEMM
+  unsigned n_q, n_kv, hd;              // QKV: heads; row t's cache entry: position pos[t] of the cache at t * slot_stride
+  const float *qw, *kw, *rope;
+  const int* pos;
+  uint8_t *kv_k, *kv_v;
+  size_t slot_stride;
 };
 int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* const* W, const size_t* rows, size_t cols, const void* xt,
                         int n_tok, float* const* y, const size_t* ldy, float* P, int mode, const ks_gemm_epi* epi);

@@ -370,20 +370,34 @@ int enqueue_forward_gemm(ks_model* m, const Lane& L_, int n, bool want_logits) {
   epi.xt_out = m->gemm_xt;
   for (int l = 0; l < g.n_layers; l++) {
     const Layer& L = m->layers[l];
-    {  // q, k and v rows in one launch (lib.rs:227)
-      const uint8_t* Ws[3] = {(const uint8_t*)L.wq.dptr, (const uint8_t*)L.wk.dptr, (const uint8_t*)L.wv.dptr};
-      float* ys[3] = {(float*)q, (float*)k, (float*)v};
-      const size_t rs[3] = {qn, kvn, kvn};
-      if ((rc = ks_launch_gemm_segs(c, KS_Q4K, 3, Ws, rs, H, m->gemm_xt, n, ys, rs, m->gemm_p0, KS_GEMM_PLAIN, nullptr))) return rc;
-    }
     uint8_t* kk = m->kv_k[l] + L_.kv_off;
     uint8_t* kv = m->kv_v[l] + L_.kv_off;
-    if ((rc = ks_launch_per_head_qkv_q40(c, nq, nkv, hd, n, g.eps, act, q, L.q32, m->rope, k, L.k32, v, q,
-                                         kk, kv, L_.pos, L_.kv_stride)))
-      return rc;
+    {  // q, k and v rows in one launch (lib.rs:227); their sums go through the per-head norms, RoPE and the pack (lib.rs:1257)
+      const uint8_t* Ws[3] = {(const uint8_t*)L.wq.dptr, (const uint8_t*)L.wk.dptr, (const uint8_t*)L.wv.dptr};
+      float* ys[3] = {nullptr, nullptr, nullptr};
+      const size_t rs[3] = {qn, kvn, kvn};
+      ks_gemm_epi head{};
+      head.eps = g.eps;
+      head.out_x = (float*)q;
+      head.n_q = (unsigned)nq;
+      head.n_kv = (unsigned)nkv;
+      head.hd = (unsigned)hd;
+      head.qw = L.q32;
+      head.kw = L.k32;
+      head.rope = m->rope;
+      head.pos = L_.pos;
+      head.kv_k = kk;
+      head.kv_v = kv;
+      head.slot_stride = L_.kv_stride;
+      if ((rc = ks_launch_gemm_segs(c, KS_Q4K, 3, Ws, rs, H, m->gemm_xt, n, ys, rs, m->gemm_p0, KS_GEMM_QKV, &head))) return rc;
+    }
     if (L_.chunk_base && n >= KS_CHUNK_ATT_MIN && ks_sdpa_chunk_covers(nq, nkv, hd, kk, kv)) {  // the rows of a chunk share their context
       if ((rc = ks_launch_sdpa_chunk(c, n, nq, nkv, hd, g.attn_scale, (const float*)q, kk, kv, layer_meta(m, L_, l), L_.attn_tmp, chunk_splits)) ||
           (rc = ks_launch_sdpa_merge_split(c, n, ks_gemm_np(n), nq, hd, L_.attn_tmp, chunk_splits, m->gemm_xt)))
+        return rc;
+    } else if (att_splits > 1 && ks_sdpa_merge_split_covers(nq, hd)) {
+      if ((rc = ks_launch_sdpa(c, n, nq, nkv, hd, g.attn_scale, act, q, kk, kv, L_.kv_stride, layer_meta(m, L_, l), L_.attn_tmp, o, att_splits, true)) ||
+          (rc = ks_launch_sdpa_merge_split(c, n, ks_gemm_np(n), nq, hd, L_.attn_tmp, att_splits, m->gemm_xt)))
         return rc;
     } else {
       if ((rc = ks_launch_sdpa(c, n, nq, nkv, hd, g.attn_scale, act, q, kk, kv, L_.kv_stride, layer_meta(m, L_, l), L_.attn_tmp, o, att_splits)))

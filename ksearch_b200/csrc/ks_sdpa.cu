@@ -704,7 +704,7 @@ int launch_part_g(ks_ctx* ctx, int G, dim3 grid, unsigned n_q, unsigned n_kv, fl
 
 int ks_launch_sdpa(ks_ctx* ctx, size_t n_slots, size_t n_q, size_t n_kv, size_t hd, float scale, ks_dtype act,
                    const void* q, const uint8_t* K, const uint8_t* V, size_t slot_stride_bytes, const float* meta,
-                   float* tmp, void* out, int n_splits) {
+                   float* tmp, void* out, int n_splits, bool records_only) {
   const int G = (int)(n_q / n_kv);
   dim3 grid((unsigned)n_splits, (unsigned)n_kv, (unsigned)n_slots);
   int rc = 1;
@@ -726,7 +726,7 @@ int ks_launch_sdpa(ks_ctx* ctx, size_t n_slots, size_t n_q, size_t n_kv, size_t 
   } else {
     return ks_fail(ctx, KS_ERR_UNSUPPORTED, "sdpa: head_dim %zu not supported (128, 256)", hd);
   }
-  if (rc || n_splits == 1) return rc;
+  if (rc || n_splits == 1 || records_only) return rc;
   const dim3 blocks((unsigned)(n_slots * n_q), (unsigned)hd / kRedDims);
   if (act == KS_F32)
     KS_LAUNCH(ctx, (sdpa_reduce_kernel<float>), blocks, kRedDims * kRedParts, 0, (unsigned)hd, tmp, (float*)out, n_splits);

@@ -344,14 +344,54 @@ sdpa_chunk_kernel(unsigned n_tok, unsigned n_q, unsigned n_kv, float scale, cons
 }
 
 // The (m, l, O) records of a token's heads -> the image the output projection reads its rows from (lower.rs:5897-6088 and
-// the operand split in one).  One block per (padded) token row, 8 neighbouring dims per thread and step.
+// the operand split in one).  One block per (padded) token row, 8 neighbouring dims per thread and step.  The first splits' O are
+// requested before the (m, l) pairs are looked at; a warp makes the factors of a head.
+constexpr unsigned MG_FLY = 4;
 __global__ void __launch_bounds__(512) sdpa_merge_split_kernel(unsigned n_tok, unsigned np, unsigned n_q, unsigned hd, const float* tmp, unsigned n_splits,
                                                                __half* xt) {
   ks_pdl_entry();
+  extern __shared__ float fac[];  // [n_q][n_splits]: exp(m - M) / L, 0 for an empty split (which may have left no O)
   __shared__ float red[32];
-  const unsigned t = blockIdx.x, chunks = n_q * hd / 8u;
+  const unsigned t = blockIdx.x, chunks = n_q * hd / 8u, lane = threadIdx.x & 31u;
+  const float* rec_t = tmp + (size_t)t * n_q * n_splits * (hd + 2u);
   constexpr int MOST = 2;
   float v[MOST][8];
+  float2 o[MG_FLY][4];
+  auto request = [&](const float* rec, unsigned d, unsigned s0) {
+#pragma unroll
+    for (unsigned k = 0; k < MG_FLY; k++)
+#pragma unroll
+      for (int e = 0; e < 4; e++)
+        o[k][e] = s0 + k < n_splits ? *reinterpret_cast<const float2*>(rec + (size_t)(s0 + k) * (hd + 2u) + 2 + d + 2 * e) : make_float2(0.f, 0.f);
+  };
+  auto place = [&](unsigned ck, const float*& rec, unsigned& head, unsigned& d) {
+    head = ck * 8u / hd;
+    d = ck * 8u - head * hd;
+    rec = rec_t + (size_t)head * n_splits * (hd + 2u);
+  };
+  const float* rec;
+  unsigned head, d;
+  if (t < n_tok && threadIdx.x < chunks) {
+    place(threadIdx.x, rec, head, d);
+    request(rec, d, 0);
+  }
+  if (t < n_tok)
+    for (unsigned h = threadIdx.x >> 5; h < n_q; h += blockDim.x >> 5) {
+      const float* r = rec_t + (size_t)h * n_splits * (hd + 2u);
+      float M = kNegInit, L = 0.0f;
+      for (unsigned s = lane; s < n_splits; s += 32u) M = fmaxf(M, r[(size_t)s * (hd + 2u)]);
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
+      for (unsigned s = lane; s < n_splits; s += 32u) {
+        const float l = r[(size_t)s * (hd + 2u) + 1], f = l != 0.0f ? __expf(r[(size_t)s * (hd + 2u)] - M) : 0.0f;
+        L = fmaf(l, f, L);
+        fac[h * n_splits + s] = f;
+      }
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) L += __shfl_xor_sync(0xffffffffu, L, off);
+      for (unsigned s = lane; s < n_splits; s += 32u) fac[h * n_splits + s] /= L;
+    }
+  __syncthreads();
   float m = 0.0f;
 #pragma unroll
   for (int kk = 0; kk < MOST; kk++) {
@@ -359,26 +399,20 @@ __global__ void __launch_bounds__(512) sdpa_merge_split_kernel(unsigned n_tok, u
 #pragma unroll
     for (int e = 0; e < 8; e++) v[kk][e] = 0.0f;
     if (t < n_tok && ck < chunks) {
-      const unsigned head = ck * 8u / hd, d = ck * 8u - head * hd;
-      const float* rec = tmp + ((size_t)t * n_q + head) * n_splits * (hd + 2u);
-      float M = kNegInit, L = 0.0f;
-      for (unsigned s = 0; s < n_splits; s++) M = fmaxf(M, rec[(size_t)s * (hd + 2u)]);
-      for (unsigned s = 0; s < n_splits; s++) {
-        const float* r = rec + (size_t)s * (hd + 2u);
-        const float l = r[1];
-        if (l == 0.0f) continue;  // an empty split may have left no O
-        const float f = __expf(r[0] - M);
-        L = fmaf(l, f, L);
+      place(ck, rec, head, d);
+      for (unsigned s0 = 0; s0 < n_splits; s0 += MG_FLY) {
+        if (kk || s0) request(rec, d, s0);
 #pragma unroll
-        for (int e = 0; e < 8; e += 2) {
-          const float2 x = *reinterpret_cast<const float2*>(r + 2 + d + e);
-          v[kk][e] = fmaf(x.x, f, v[kk][e]);
-          v[kk][e + 1] = fmaf(x.y, f, v[kk][e + 1]);
+        for (unsigned k = 0; k < MG_FLY; k++) {
+          const float f = s0 + k < n_splits ? fac[head * n_splits + s0 + k] : 0.0f;
+          if (f != 0.0f)
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+              v[kk][2 * e] = fmaf(o[k][e].x, f, v[kk][2 * e]);
+              v[kk][2 * e + 1] = fmaf(o[k][e].y, f, v[kk][2 * e + 1]);
+            }
         }
       }
-      const float inv = 1.0f / L;
-#pragma unroll
-      for (int e = 0; e < 8; e++) v[kk][e] *= inv;
       m = fmaxf(m, absmax8(v[kk]));
     }
   }
@@ -422,9 +456,10 @@ int ks_sdpa_chunk_splits(const ks_ctx* ctx, int n_tok, size_t n_q, size_t n_kv, 
   return s < 1 ? 1 : (int)s;
 }
 
+bool ks_sdpa_merge_split_covers(size_t n_q, size_t hd) { return n_q * hd <= 8192 && n_q * hd % 256 == 0 && n_q <= 64; }
 bool ks_sdpa_chunk_covers(size_t n_q, size_t n_kv, size_t hd, const void* K, const void* V) {
   const size_t G = n_q / n_kv;
-  return (hd == 256 || hd == 128) && G <= CH_BM && CH_BM % G == 0 && n_q * hd <= 8192 && n_q * hd % 256 == 0 && (((uintptr_t)K | (uintptr_t)V) & 3u) == 0;
+  return (hd == 256 || hd == 128) && G <= CH_BM && CH_BM % G == 0 && ks_sdpa_merge_split_covers(n_q, hd) && (((uintptr_t)K | (uintptr_t)V) & 3u) == 0;
 }
 
 // Rows of one slot: q [n_tok, n_q hd] f32, meta [n_tok][4] = (tlen, start, -, -) with both ends growing along the rows
@@ -439,6 +474,6 @@ int ks_launch_sdpa_chunk(ks_ctx* ctx, int n_tok, size_t n_q, size_t n_kv, size_t
 // Records of n_tok rows -> the Q4_K form of the operand image (rows past n_tok as zeros).
 int ks_launch_sdpa_merge_split(ks_ctx* ctx, int n_tok, unsigned np, size_t n_q, size_t hd, const float* tmp, int n_splits, void* xt) {
   const unsigned chunks = (unsigned)(n_q * hd / 8), threads = chunks < 512u ? (chunks + 31u) / 32u * 32u : 512u;
-  KS_LAUNCH(ctx, sdpa_merge_split_kernel, np, threads, 0, (unsigned)n_tok, np, (unsigned)n_q, (unsigned)hd, tmp, (unsigned)n_splits, (__half*)xt);
+  KS_LAUNCH(ctx, sdpa_merge_split_kernel, np, threads, (size_t)n_q * n_splits * sizeof(float), (unsigned)n_tok, np, (unsigned)n_q, (unsigned)hd, tmp, (unsigned)n_splits, (__half*)xt);
   return ks_after_launch(ctx, "sdpa_merge_split");
 }
