@@ -700,10 +700,11 @@ unsigned gemm_splits(const ks_ctx* ctx, size_t rows, size_t cols, int n_tok) {
   return best;
 }
 ks_gemm_map gemm_map(const ks_ctx* ctx, ks_dtype wdtype, const size_t* rows, int n_seg, size_t cols, int n_tok) {
-  if (wdtype == KS_Q4K) return ks_gemm_q4k_map(ctx, rows, n_seg, (unsigned)cols, gemm_np(n_tok));
   ks_gemm_map m{};
   size_t total_rows = 0;
   for (int i = 0; i < n_seg; i++) total_rows += rows[i];
+  if (wdtype == KS_Q4K && n_tok <= KS_GEMM_SKINNY && (m.splits = ks_gemm_skinny_splits(ctx, total_rows, (unsigned)cols)) != 0) return m;
+  if (wdtype == KS_Q4K) return ks_gemm_q4k_map(ctx, rows, n_seg, (unsigned)cols, gemm_np(n_tok));
   const unsigned ksteps = (unsigned)(cols / GM_KSTEP), s = gemm_splits(ctx, total_rows, cols, n_tok), per = (ksteps + s - 1) / s;
   m.splits = (ksteps + per - 1) / per;
   return m;
@@ -795,7 +796,7 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
     job.np = np;
     job.xt = (const __half*)xt;
     job.map = map;
-    rc = ks_launch_gemm_q4k(ctx, job);
+    rc = map.G ? ks_launch_gemm_q4k(ctx, job) : ks_launch_gemm_skinny(ctx, job);
   } else {
     GemmArgs a{};
     for (int i = 0; i < 3; i++) {
@@ -911,9 +912,13 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
 // Floats of partials ks_launch_gemm_segs may write for up to three matrices of `total_rows` rows in all (either dtype).
 size_t ks_gemm_part_floats(const ks_ctx* ctx, size_t total_rows, size_t cols, int n_tok) {
   unsigned slots = gemm_map(ctx, KS_Q6K, &total_rows, 1, cols, n_tok).splits;
+  if (n_tok <= KS_GEMM_SKINNY) {
+    const unsigned n = ks_gemm_skinny_splits(ctx, total_rows, (unsigned)cols);
+    slots = n > slots ? n : slots;
+  }
   for (int extra = 0; extra < 3; extra++) {  // the matrices of a launch round their tiles up one by one
     const size_t r = total_rows + (size_t)extra * 2 * GM_ROWS;
-    const ks_gemm_map m = gemm_map(ctx, KS_Q4K, &r, 1, cols, n_tok);
+    const ks_gemm_map m = ks_gemm_q4k_map(ctx, &r, 1, (unsigned)cols, gemm_np(n_tok));
     const unsigned n = (m.S + m.base - 1) / m.base + 1;  // a CTA has at least `base` units, a work tile may begin inside one
     slots = n > slots ? n : slots;
   }

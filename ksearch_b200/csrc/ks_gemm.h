@@ -1,6 +1,8 @@
-// Between ks_gemm.cu (images, epilogues, dispatch) and ks_gemm_q4k.cu (the Q4_K kernel).
+// Between ks_gemm.cu (images, epilogues, dispatch), ks_gemm_q4k.cu (the Q4_K kernel) and ks_gemm_skinny.cu (Q4_K, few rows).
 #pragma once
 #include "ks_gemm_common.cuh"
+
+constexpr int KS_GEMM_SKINNY = 8;  // token rows of the kernel in ks_gemm_skinny.cu (the columns of one mma)
 
 struct ks_gemm_job {
   int n_seg;
@@ -14,3 +16,5 @@ struct ks_gemm_job {
 };
 ks_gemm_map ks_gemm_q4k_map(const ks_ctx* ctx, const size_t* rows, int n_seg, unsigned cols, unsigned np);
 int ks_launch_gemm_q4k(ks_ctx* ctx, const ks_gemm_job& job);
+unsigned ks_gemm_skinny_splits(const ks_ctx* ctx, size_t rows, unsigned cols);  // column shares; 0: not covered
+int ks_launch_gemm_skinny(ks_ctx* ctx, const ks_gemm_job& job);

@@ -835,7 +835,7 @@ ks_model* ks_model_create(ks_ctx* ctx, const ks_model_config* cfg) {
         const int most = i < 4 ? G : g.n_slots;  // only decode steps reach the head
         const size_t a = ks_gemm_xt_bytes(cols_of[i], most);
         xt = a > xt ? a : xt;
-        for (int n = 16; n < most + 16; n += 16) {  // fewer rows are split finer
+        for (int n = 8; n < most + 16; n += n < 16 ? 8 : 16) {  // fewer rows are split finer, up to 8 take a kernel of their own
           const int rows = n < most ? n : most;
           const size_t b = 4 * ks_gemm_part_floats(ctx, rows_of[i], cols_of[i], rows);
           part = b > part ? b : part;
