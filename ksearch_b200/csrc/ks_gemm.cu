@@ -705,6 +705,10 @@ ks_gemm_map gemm_map(const ks_ctx* ctx, ks_dtype wdtype, const size_t* rows, int
   for (int i = 0; i < n_seg; i++) total_rows += rows[i];
   if (wdtype == KS_Q4K && n_tok <= KS_GEMM_SKINNY && (m.splits = ks_gemm_skinny_splits(ctx, total_rows, (unsigned)cols)) != 0) return m;
   if (wdtype == KS_Q4K) return ks_gemm_q4k_map(ctx, rows, n_seg, (unsigned)cols, gemm_np(n_tok));
+  if (n_tok <= KS_GEMM_SKINNY && n_seg == 1 && ks_gemm_q6k_skinny_covers(ctx, total_rows, (unsigned)cols)) {
+    m.splits = 1;
+    return m;
+  }
   const unsigned ksteps = (unsigned)(cols / GM_KSTEP), s = gemm_splits(ctx, total_rows, cols, n_tok), per = (ksteps + s - 1) / s;
   m.splits = (ksteps + per - 1) / per;
   return m;
@@ -714,6 +718,7 @@ bool gemm_covers(ks_dtype wdtype, size_t cols, int n_tok) {
 }
 }  // namespace
 
+bool ks_gemm_few_rows_q6k(const ks_ctx* ctx, size_t rows, size_t cols) { return ks_gemm_q6k_skinny_covers(ctx, rows, (unsigned)cols); }
 unsigned ks_gemm_np(int n_tok) { return gemm_np(n_tok); }
 
 // Bytes of the B image of n_tok rows of `cols` values (hi + lo halves, token count padded to 16).
@@ -781,7 +786,9 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
     }
   }
   int rc;
-  if (wdtype == KS_Q4K) {
+  const bool skinny6 = wdtype == KS_Q6K && n_tok <= KS_GEMM_SKINNY && n_seg == 1 && direct && ((uintptr_t)W[0] & 15) == 0 &&
+                       ks_gemm_q6k_skinny_covers(ctx, rows[0], (unsigned)cols);
+  if (wdtype == KS_Q4K || skinny6) {
     ks_gemm_job job{};
     job.n_seg = n_seg;
     for (int i = 0; i < n_seg; i++) {
@@ -796,7 +803,7 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
     job.np = np;
     job.xt = (const __half*)xt;
     job.map = map;
-    rc = map.G ? ks_launch_gemm_q4k(ctx, job) : ks_launch_gemm_skinny(ctx, job);
+    rc = skinny6 ? ks_launch_gemm_q6k_skinny(ctx, job) : map.G ? ks_launch_gemm_q4k(ctx, job) : ks_launch_gemm_skinny(ctx, job);
   } else {
     GemmArgs a{};
     for (int i = 0; i < 3; i++) {

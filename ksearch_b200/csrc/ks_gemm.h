@@ -1,4 +1,4 @@
-// Between ks_gemm.cu (images, epilogues, dispatch), ks_gemm_q4k.cu (the Q4_K kernel) and ks_gemm_skinny.cu (Q4_K, few rows).
+// Between ks_gemm.cu (images, epilogues, dispatch), ks_gemm_q4k.cu (the Q4_K kernel) and ks_gemm_skinny.cu (up to 8 token rows).
 #pragma once
 #include "ks_gemm_common.cuh"
 
@@ -18,3 +18,5 @@ ks_gemm_map ks_gemm_q4k_map(const ks_ctx* ctx, const size_t* rows, int n_seg, un
 int ks_launch_gemm_q4k(ks_ctx* ctx, const ks_gemm_job& job);
 unsigned ks_gemm_skinny_splits(const ks_ctx* ctx, size_t rows, unsigned cols);  // column shares; 0: not covered
 int ks_launch_gemm_skinny(ks_ctx* ctx, const ks_gemm_job& job);
+bool ks_gemm_q6k_skinny_covers(const ks_ctx* ctx, size_t rows, unsigned cols);
+int ks_launch_gemm_q6k_skinny(ks_ctx* ctx, const ks_gemm_job& job);

@@ -150,6 +150,7 @@ bool ks_sdpa_chunk_covers(size_t n_q, size_t n_kv, size_t hd, const void* K, con
 int ks_launch_sdpa_chunk(ks_ctx* ctx, int n_tok, size_t n_q, size_t n_kv, size_t hd, float scale, const float* q, const uint8_t* K,
                          const uint8_t* V, const float* meta, float* tmp, int n_splits);
 int ks_launch_sdpa_merge_split(ks_ctx* ctx, int n_tok, unsigned np, size_t n_q, size_t hd, const float* tmp, int n_splits, void* xt);
+bool ks_gemm_few_rows_q6k(const ks_ctx* ctx, size_t rows, size_t cols);  // ks_gemm_skinny.cu has a kernel for up to 8 token rows
 unsigned ks_gemm_np(int n_tok);  // token rows of an operand image: n_tok padded
 int ks_launch_copy_scale_indexed(ks_ctx* ctx, size_t n, size_t batch, float scale, ks_dtype src_dtype,
                                  const void* src, const float* idx, ks_dtype act, void* dst);
