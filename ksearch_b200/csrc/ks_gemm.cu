@@ -62,7 +62,7 @@ struct GemmArgs {
 };
 
 // x[token, k] (f32, row stride ldx) -> the B image.  One block per (padded) token row; rows past n_tok become zeros.
-__global__ void __launch_bounds__(1024) x_split_kernel(const float* x, size_t ldx, unsigned n_tok, unsigned np, unsigned cols, __half* xt, int q4k) {
+__global__ void __launch_bounds__(1024) x_split_kernel(const float* x, size_t ldx, unsigned n_tok, unsigned np, unsigned tbn, unsigned cols, __half* xt, int q4k) {
   ks_pdl_entry();
   __shared__ float red[32];
   const unsigned t = blockIdx.x, chunks = cols / 8u;
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(1024) x_split_kernel(const float* x, size_t ld
 #pragma unroll
       for (int e = 0; e < 8; e++) v[e] = 0.0f;
     }
-    put_split8(xt, np, t, ck, chunks, v, q4k != 0);
+    put_split8(xt, np, tbn, t, ck, chunks, v, q4k != 0);
   }
 }
 
@@ -502,7 +502,7 @@ __global__ void gemm_finish_norm_split_kernel(const EpiNormArgs e) {
   if (ck < chunks) {
 #pragma unroll
     for (int i = 0; i < 8; i++) xn[i] *= down;
-    put_split8(e.xt, e.np, t, ck, chunks, xn, e.q4k != 0);
+    put_split8(e.xt, e.np, q4k_block(e.np), t, ck, chunks, xn, e.q4k != 0);
   }
 }
 
@@ -544,7 +544,7 @@ __global__ void __cluster_dims__(GM_GELU_CL, 1, 1) __launch_bounds__(GM_GELU_THR
   if (ck < chunks) {
 #pragma unroll
     for (int k = 0; k < 8; k++) v[k] *= down;
-    put_split8(xt, np, t, ck, chunks, v, true);  // a down-projection is always Q4_K
+    put_split8(xt, np, q4k_block(np), t, ck, chunks, v, true);  // a down-projection is always Q4_K
   }
 }
 
@@ -699,12 +699,21 @@ unsigned gemm_splits(const ks_ctx* ctx, size_t rows, size_t cols, int n_tok) {
   }
   return best;
 }
-ks_gemm_map gemm_map(const ks_ctx* ctx, ks_dtype wdtype, const size_t* rows, int n_seg, size_t cols, int n_tok) {
+// Token rows per block of the image, and all of them padded to whole blocks.
+struct Blocks {
+  unsigned tbn, np;
+};
+Blocks gemm_blocks(int n_tok) { return {q4k_block(gemm_np(n_tok)), gemm_np(n_tok)}; }
+Blocks gemm_small_blocks(int n_tok) {
+  const unsigned tb = ((unsigned)n_tok + 63u) / 64u, tbn = (((unsigned)n_tok + tb - 1) / tb + 15u) / 16u * 16u;
+  return {tbn, tb * tbn};
+}
+ks_gemm_map gemm_map(const ks_ctx* ctx, ks_dtype wdtype, const size_t* rows, int n_seg, size_t cols, int n_tok, Blocks b, bool plain) {
   ks_gemm_map m{};
   size_t total_rows = 0;
   for (int i = 0; i < n_seg; i++) total_rows += rows[i];
   if (wdtype == KS_Q4K && n_tok <= KS_GEMM_SKINNY && (m.splits = ks_gemm_skinny_splits(ctx, total_rows, (unsigned)cols)) != 0) return m;
-  if (wdtype == KS_Q4K) return ks_gemm_q4k_map(ctx, rows, n_seg, (unsigned)cols, gemm_np(n_tok));
+  if (wdtype == KS_Q4K) return ks_gemm_q4k_map(ctx, rows, n_seg, (unsigned)cols, b.np, b.tbn, plain);
   if (n_tok <= KS_GEMM_SKINNY && n_seg == 1 && ks_gemm_q6k_skinny_covers(ctx, total_rows, (unsigned)cols)) {
     m.splits = 1;
     return m;
@@ -712,6 +721,18 @@ ks_gemm_map gemm_map(const ks_ctx* ctx, ks_dtype wdtype, const size_t* rows, int
   const unsigned ksteps = (unsigned)(cols / GM_KSTEP), s = gemm_splits(ctx, total_rows, cols, n_tok), per = (ksteps + s - 1) / s;
   m.splits = (ksteps + per - 1) / per;
   return m;
+}
+// One Q4_K matrix against more than 64 token rows: pairs of row tiles against blocks of up to 128 read the token rows half as
+// often; where that leaves few units for the SMs, single tiles against blocks of up to 64 are four times as many.  By the
+// estimate both maps are chosen by.
+Blocks gemm_pick_blocks(const ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_t cols, int n_tok) {
+  const Blocks wide = gemm_blocks(n_tok);
+  if (wdtype != KS_Q4K || wide.tbn <= 64u) return wide;
+  const Blocks small = gemm_small_blocks(n_tok);
+  double cw, cs;
+  ks_gemm_q4k_map(ctx, &rows, 1, (unsigned)cols, wide.np, wide.tbn, true, &cw);
+  ks_gemm_q4k_map(ctx, &rows, 1, (unsigned)cols, small.np, small.tbn, true, &cs);
+  return cs < cw ? small : wide;
 }
 bool gemm_covers(ks_dtype wdtype, size_t cols, int n_tok) {
   return (wdtype == KS_Q4K || wdtype == KS_Q6K) && cols % 256 == 0 && n_tok >= 1 && n_tok <= 256;
@@ -722,30 +743,35 @@ bool ks_gemm_few_rows_q6k(const ks_ctx* ctx, size_t rows, size_t cols) { return 
 unsigned ks_gemm_np(int n_tok) { return gemm_np(n_tok); }
 
 // Bytes of the B image of n_tok rows of `cols` values (hi + lo halves, token count padded to 16).
-size_t ks_gemm_xt_bytes(size_t cols, int n_tok) { return cols / 256 * 288 * gemm_np(n_tok) * 4 + (size_t)gemm_np(n_tok) * 4; }  // image + one factor per row
+size_t ks_gemm_xt_bytes(size_t cols, int n_tok) {  // image + one factor per row, whatever the blocks
+  const size_t np = n_tok > 64 ? ((size_t)n_tok + 63) / 64 * 64 : gemm_np(n_tok);
+  return cols / 256 * 288 * np * 4 + np * 4;
+}
 
 // x[t * ldx + k] (f32) -> the B image in xt.
-int ks_launch_gemm_split(ks_ctx* ctx, ks_dtype wdtype, const float* x, size_t ldx, int n_tok, size_t cols, void* xt) {
+static int launch_split(ks_ctx* ctx, ks_dtype wdtype, const float* x, size_t ldx, int n_tok, size_t cols, void* xt, Blocks b) {
   if (cols % 256 || n_tok < 1 || n_tok > 256 || ldx % 4) return ks_fail(ctx, KS_ERR_INVALID, "gemm: bad operand shape");
-  const unsigned np = gemm_np(n_tok);
-  KS_LAUNCH(ctx, (x_split_kernel), np, GM_ROW_THREADS, 0, x, ldx, (unsigned)n_tok, np, (unsigned)cols, (__half*)xt, (int)(wdtype == KS_Q4K));
+  KS_LAUNCH(ctx, (x_split_kernel), b.np, GM_ROW_THREADS, 0, x, ldx, (unsigned)n_tok, b.np, b.tbn, (unsigned)cols, (__half*)xt, (int)(wdtype == KS_Q4K));
   return ks_after_launch(ctx, "x_split");
+}
+int ks_launch_gemm_split(ks_ctx* ctx, ks_dtype wdtype, const float* x, size_t ldx, int n_tok, size_t cols, void* xt) {
+  return launch_split(ctx, wdtype, x, ldx, n_tok, cols, xt, gemm_blocks(n_tok));
 }
 
 // Up to three matrices over the same columns in one launch.  With one k split matrix i's result goes straight to
 // y[i] (row stride ldy[i]); otherwise the partials go to P (dense [split][token][row] per matrix, matrix after
 // matrix) and a second launch sums them in split order into y.  mode 1 (two matrices, gate and up): y[0] =
 // gelu(gate) * up, always through P.  `xt` is the image ks_launch_gemm_split made of the same token rows.
-int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* const* W, const size_t* rows, size_t cols, const void* xt,
-                        int n_tok, float* const* y, const size_t* ldy, float* P, int mode, const ks_gemm_epi* epi) {
+static int launch_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* const* W, const size_t* rows, size_t cols, const void* xt,
+                       int n_tok, float* const* y, const size_t* ldy, float* P, int mode, const ks_gemm_epi* epi, Blocks blocks) {
   if (!gemm_covers(wdtype, cols, n_tok) || n_seg < 1 || n_seg > 3) return ks_fail(ctx, KS_ERR_UNSUPPORTED, "gemm: shape not covered");
   if ((mode == KS_GEMM_NORM_SPLIT && (n_seg != 1 || !epi || rows[0] % 8 || rows[0] > 8192)) ||
       (mode == KS_GEMM_QKV && (n_seg != 3 || !epi || (epi->hd != 128 && epi->hd != 256) || rows[0] != (size_t)epi->n_q * epi->hd ||
                                rows[1] != (size_t)epi->n_kv * epi->hd || rows[2] != rows[1])) ||
       (mode == KS_GEMM_GELU_SPLIT && (n_seg != 2 || !epi || rows[0] != rows[1] || rows[0] % 8 || rows[0] > 8u * GM_GELU_CL * GM_GELU_THREADS || rows[0] % 256)))
     return ks_fail(ctx, KS_ERR_INVALID, "gemm: bad epilogue arguments");
-  const unsigned np = gemm_np(n_tok);
-  const ks_gemm_map map = gemm_map(ctx, wdtype, rows, n_seg, cols, n_tok);
+  const unsigned np = blocks.np;
+  const ks_gemm_map map = gemm_map(ctx, wdtype, rows, n_seg, cols, n_tok, blocks, mode == KS_GEMM_PLAIN);
   unsigned tiles = 0, tile0[4], groups = 0, group0[3] = {0, 0, 0};
   size_t total_rows = 0;
   for (int i = 0; i < 3; i++) {
@@ -916,29 +942,43 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
   return ks_after_launch(ctx, "gemm_finish");
 }
 
+int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* const* W, const size_t* rows, size_t cols, const void* xt,
+                        int n_tok, float* const* y, const size_t* ldy, float* P, int mode, const ks_gemm_epi* epi) {
+  return launch_segs(ctx, wdtype, n_seg, W, rows, cols, xt, n_tok, y, ldy, P, mode, epi, gemm_blocks(n_tok));
+}
+
 // Floats of partials ks_launch_gemm_segs may write for up to three matrices of `total_rows` rows in all (either dtype).
 size_t ks_gemm_part_floats(const ks_ctx* ctx, size_t total_rows, size_t cols, int n_tok) {
-  unsigned slots = gemm_map(ctx, KS_Q6K, &total_rows, 1, cols, n_tok).splits;
+  unsigned slots = gemm_map(ctx, KS_Q6K, &total_rows, 1, cols, n_tok, gemm_blocks(n_tok), true).splits;
   if (n_tok <= KS_GEMM_SKINNY) {
     const unsigned n = ks_gemm_skinny_splits(ctx, total_rows, (unsigned)cols);
     slots = n > slots ? n : slots;
   }
-  for (int extra = 0; extra < 3; extra++) {  // the matrices of a launch round their tiles up one by one
-    const size_t r = total_rows + (size_t)extra * 2 * GM_ROWS;
-    const ks_gemm_map m = ks_gemm_q4k_map(ctx, &r, 1, (unsigned)cols, gemm_np(n_tok));
+  const Blocks b = gemm_blocks(n_tok);
+  for (int extra = 0; extra < 6; extra++) {  // the matrices of a launch round their tiles up one by one; with and without an epilogue
+    const size_t r = total_rows + (size_t)(extra % 3) * 2 * GM_ROWS;
+    const ks_gemm_map m = ks_gemm_q4k_map(ctx, &r, 1, (unsigned)cols, b.np, b.tbn, extra >= 3);
     const unsigned n = (m.S + m.base - 1) / m.base + 1;  // a CTA has at least `base` units, a work tile may begin inside one
     slots = n > slots ? n : slots;
   }
   return (size_t)slots * (size_t)n_tok * total_rows;
 }
 
+// Scratch of ks_launch_gemm_kq: the image and the partials of that one launch.
+size_t ks_gemm_kq_bytes(const ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_t cols, int n_tok) {
+  const ks_gemm_map m = gemm_map(ctx, wdtype, &rows, 1, cols, n_tok, gemm_pick_blocks(ctx, wdtype, rows, cols, n_tok), true);
+  const size_t slots = m.G ? (m.S + m.base - 1) / m.base + 1 : m.splits;
+  return ks_gemm_xt_bytes(cols, n_tok) + 4 * slots * n_tok * rows;
+}
+
 // y[t * ldy + r] = sum_k W[r, k] x[t * ldx + k] for t < n_tok (<= 256), f32 x and y: operand split, GEMM and, when
-// the k range was split, the ordered sum of the partials.  `scratch`: ks_gemm_xt_bytes + 4 * ks_gemm_part_floats.
+// the k range was split, the ordered sum of the partials.  `scratch`: ks_gemm_kq_bytes.
 int ks_launch_gemm_kq(ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_t cols, const uint8_t* W, const float* x, size_t ldx, float* y,
                       size_t ldy, int n_tok, void* scratch) {
   if (!gemm_covers(wdtype, cols, n_tok) || ldx % 4) return 1;
-  int rc = ks_launch_gemm_split(ctx, wdtype, x, ldx, n_tok, cols, scratch);
+  const Blocks b = gemm_pick_blocks(ctx, wdtype, rows, cols, n_tok);
+  int rc = launch_split(ctx, wdtype, x, ldx, n_tok, cols, scratch, b);
   if (rc) return rc;
   float* P = (float*)((char*)scratch + ks_gemm_xt_bytes(cols, n_tok));
-  return ks_launch_gemm_segs(ctx, wdtype, 1, &W, &rows, cols, scratch, n_tok, &y, &ldy, P, KS_GEMM_PLAIN, nullptr);
+  return launch_segs(ctx, wdtype, 1, &W, &rows, cols, scratch, n_tok, &y, &ldy, P, KS_GEMM_PLAIN, nullptr, b);
 }

@@ -14,7 +14,10 @@ struct ks_gemm_job {
   const __half* xt;
   ks_gemm_map map;
 };
-ks_gemm_map ks_gemm_q4k_map(const ks_ctx* ctx, const size_t* rows, int n_seg, unsigned cols, unsigned np);
+// `tbn`: token rows of a block; more than 64 take row tiles in pairs.  `plain`: undivided sums need no second launch.  `cost`:
+// the estimate the map was chosen by, in us.
+ks_gemm_map ks_gemm_q4k_map(const ks_ctx* ctx, const size_t* rows, int n_seg, unsigned cols, unsigned np, unsigned tbn, bool plain,
+                            double* cost = nullptr);
 int ks_launch_gemm_q4k(ks_ctx* ctx, const ks_gemm_job& job);
 unsigned ks_gemm_skinny_splits(const ks_ctx* ctx, size_t rows, unsigned cols);  // column shares; 0: not covered
 int ks_launch_gemm_skinny(ks_ctx* ctx, const ks_gemm_job& job);

@@ -62,17 +62,15 @@ __device__ __forceinline__ void split8(const float (&w)[8], uint4& hi, uint4& lo
 //                          order in which masking the packed nibbles in place leaves the weights.  Chunks 32..35 carry the
 //                          sub-block sums the minima multiply: chunk 32 + g holds, with S = 2^-5 (sum of a 32-value
 //                          sub-block), (S_hi, S_hi', S_lo, S_lo', S_hi, S_hi', 0, 0) of sub-blocks 2 g and 2 g + 1.
-//                          More than 128 token rows are two such images of half the rows, one behind the other.
-__device__ __host__ __forceinline__ unsigned q4k_block(unsigned np) { return np > 128u ? np / 2u : np; }  // token rows of one image
-__device__ __forceinline__ void put_split8(__half* xt, unsigned np, unsigned t, unsigned ck, unsigned chunks, const float (&v)[8], bool q4k) {
+//                          Token rows come in blocks of `tbn`, each an image like this of its own, one behind the other.
+__device__ __host__ __forceinline__ unsigned q4k_block(unsigned np) { return np > 128u ? np / 2u : np; }  // tbn where nothing else is said
+__device__ __forceinline__ void put_split8(__half* xt, unsigned np, unsigned tbn, unsigned t, unsigned ck, unsigned chunks, const float (&v)[8], bool q4k) {
   unsigned at = ck;
   if (q4k) {
     at = (ck >> 5) * 36u + (ck & 31u);
-    const unsigned tbn = q4k_block(np);
-    if (t >= tbn) {
-      t -= tbn;
-      xt += (size_t)(chunks / 32u * 36u) * 2u * tbn * 8u;
-    }
+    const unsigned blk = t / tbn;
+    t -= blk * tbn;
+    xt += (size_t)(chunks / 32u * 36u) * 2u * (blk * tbn) * 8u;
     np = tbn;
     const float w[8] = {v[0], v[2], v[1], v[3], v[4], v[6], v[5], v[7]};
     uint4 hi, lo;

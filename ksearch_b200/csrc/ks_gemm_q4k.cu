@@ -158,7 +158,7 @@ __device__ __forceinline__ Seg pick_seg(const Q4Args& a, unsigned grp) {
   return s;
 }
 
-// Up to 64 token rows.  TQ: token rows per worker thread at most (tbn / 4: the four warps of a lane quadrant share the
+// Token rows in blocks of up to 64.  TQ: token rows per worker thread at most (tbn / 4: the four warps of a lane quadrant share the
 // accumulator's columns).
 template <int TQ>
 __global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_constant__ Q4Args a) {
@@ -291,14 +291,15 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_
         __syncwarp();
         if (lane == 0) mb_arrive(bar(QB_D_FREE + buf));
         if (last) {
-          const Seg sg = pick_seg(a, prev_wt);
-          const unsigned out_row = (prev_wt - sg.group0) * GM_ROWS + row;
+          const unsigned grp = prev_wt / a.map.tb, tok0 = (prev_wt - grp * a.map.tb) * tbn + g * tq;
+          const Seg sg = pick_seg(a, grp);
+          const unsigned out_row = (grp - sg.group0) * GM_ROWS + row;
           const unsigned pslot = blockIdx.x - ks_gemm_owner(a.map, prev_wt * a.map.S);
           float* y = sg.y + (size_t)pslot * sg.part + out_row;
           const bool live = out_row < sg.rows;
 #pragma unroll
           for (int k = 0; k < TQ; k++) {
-            const unsigned tok = g * tq + k;
+            const unsigned tok = tok0 + k;
             if ((unsigned)k < tq && tok < a.n_tok && live) y[(size_t)tok * sg.ldy] = acc[k] * up_s[tok];
             acc[k] = 0.0f;
           }
@@ -384,7 +385,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_
         break;
       }
       if (leader) {
-        const unsigned grp = wt;
+        const unsigned grp = wt / a.map.tb;
         const int k = (grp >= a.group0[1]) + (grp >= a.group0[2]);
         const unsigned g0 = k == 0 ? a.group0[0] : k == 1 ? a.group0[1] : a.group0[2];
         mb_expect(bar(QB_RAW_FULL + st), Q_RAW);  // rows past the matrix come as zeros and count
@@ -410,7 +411,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_
     const float* up = reinterpret_cast<const float*>(a.xt + xt_scale_off(a.cols, a.np));
     for (unsigned t = lane; t < a.np; t += 32u) up_s[t] = up[t];  // read behind the first accumulator, which waits for the copies below
     __syncwarp();
-    unsigned issued = 0, sb = u0 % a.map.S, st = 0, ph = 1;
+    unsigned issued = 0, wt = u0 / a.map.S, sb = u0 - wt * a.map.S, st = 0, ph = 1;
     for (unsigned j = 0; j < n_units; j++) {  // a super-block each
       const bool got = j < a.n_b || mb_wait(bar(QB_B_FREE + st), ph, a.wait_limit);
       if (!__all_sync(0xffffffffu, got)) {
@@ -420,14 +421,18 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_
       if (a.test_stall && j + 1u == a.test_stall) break;  // test hook: this unit's token rows never arrive
       if (leader) {
         mb_expect(bar(QB_B_FULL + st), b_stage);
-        bulk_in(b0 + st * b_stage, reinterpret_cast<const unsigned char*>(a.xt) + (size_t)sb * b_stage, b_stage, bar(QB_B_FULL + st));
+        const size_t at = ((size_t)(wt % a.map.tb) * a.map.S + sb) * b_stage;
+        bulk_in(b0 + st * b_stage, reinterpret_cast<const unsigned char*>(a.xt) + at, b_stage, bar(QB_B_FULL + st));
       }
       issued++;
       if (++st == a.n_b) {
         st = 0;
         ph ^= 1u;
       }
-      if (++sb == a.map.S) sb = 0;
+      if (++sb == a.map.S) {
+        sb = 0;
+        wt++;
+      }
       __syncwarp();
     }
     for (unsigned j = issued > a.n_b ? issued - a.n_b : 0u; j < issued; j++) mb_wait(bar(QB_B_FULL + j % a.n_b), (j / a.n_b) & 1u, a.wait_limit);
@@ -439,7 +444,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_
   if (warp == 0) tc_dealloc(tmem, 512);
 }
 
-// More than 64 token rows, in blocks of up to 128.  A unit is a super-block of TWO row tiles: the token rows of a half super-block
+// Token rows in blocks of 65 to 128.  A unit is a super-block of TWO row tiles: the token rows of a half super-block
 // (4 groups of 32 k, or 5 with the minima's) are brought in once and the MMAs of the tiles alternate between two accumulators,
 //   (tile 0, half 0) (tile 1, half 0) (tile 0, half 1) (tile 1, half 1),
 // which halves the traffic of B from L2 (one tile against 256 rows at once read B at 8.9 TB/s and could not go faster).
@@ -770,32 +775,48 @@ size_t q4_rings(const ks_ctx* ctx, unsigned tbn, unsigned nt, unsigned* n_raw, u
 }
 }  // namespace
 
-// How many CTAs a launch of `tiles` tiles takes.  A CTA's time is its units (t_u each) plus writing its shares of tiles; the
-// partials are then read once more.  More CTAs mean fewer units each and more partials.
-ks_gemm_map ks_gemm_q4k_map(const ks_ctx* ctx, const size_t* rows, int n_seg, unsigned cols, unsigned np) {
+// How many CTAs a launch takes, by an estimate in us.  A CTA's time is its units and writing its shares of work tiles; sums that
+// several CTAs share are then read once more by a second launch.  The constants are fitted to 300..18363 rows x 512..10240
+// columns x 70..256 token rows, measured with single tiles and with pairs: choosing between the two by this estimate loses
+// 0.5 % against the better one.
+ks_gemm_map ks_gemm_q4k_map(const ks_ctx* ctx, const size_t* rows, int n_seg, unsigned cols, unsigned np, unsigned tbn, bool plain,
+                            double* cost_out) {
   ks_gemm_map m{};
   m.S = cols / 256u;
-  m.tbn = q4k_block(np);
+  m.tbn = tbn;
   m.tb = np / m.tbn;
-  m.nt = np > 64u ? 2u : 1u;
+  m.nt = tbn > 64u ? 2u : 1u;
   unsigned wtiles = 0;
   for (int i = 0; i < n_seg; i++) wtiles += (unsigned)(((rows[i] + GM_ROWS - 1) / GM_ROWS + m.nt - 1) / m.nt);
   wtiles *= m.tb;
   const unsigned U = wtiles * m.S, most = (unsigned)ctx->sm_count < U ? (unsigned)ctx->sm_count : U;
-  const double t_u = (0.45 + m.tbn * 0.0085) * m.nt, t_w = (0.1 + m.tbn * 0.005) * m.nt;
-  double best = 1e30;
-  for (unsigned G = 1; G <= most; G++) {
-    if (G < most && wtiles % G && G * 4u < most * 3u) continue;
-    const unsigned per = (U + G - 1) / G, shares = (per + m.S - 2) / m.S + 1;
-    const double slots = (double)G / wtiles + 1.0;
-    const double cost = per * t_u + shares * t_w + slots * wtiles * m.nt * m.tbn * (GM_ROWS * 4e-6 / 5.0);
-    if (cost < best) {
-      best = cost;
-      m.G = G;
+  // the choice of the last few shapes is kept (a call asks three to seven times: 0.6 us each)
+  struct Kept {
+    unsigned most = 0, wtiles = 0, S = 0, tbn = 0, plain = 0, G = 0;
+    double cost = 0;
+  };
+  static thread_local Kept kept[64];
+  Kept& k = kept[(wtiles * 31u + m.S * 7u + m.tbn / 8u + plain) % 64u];
+  if (k.most != most || k.wtiles != wtiles || k.S != m.S || k.tbn != m.tbn || k.plain != (unsigned)plain) {
+    const double t_u = m.nt == 2 ? 0.95 + m.tbn * 0.0316 : 1.0 + m.tbn * 0.011, t_w = (0.15 + m.tbn * 0.0075) * m.nt, start = m.nt == 2 ? 2.0 : 0.0;
+    double best = 1e30;
+    for (unsigned G = 1; G <= most; G++) {
+      if (G < most && wtiles % G && G * 4u < most * 3u) continue;
+      const bool whole = plain && wtiles % G == 0;  // no work tile is shared
+      const unsigned per = (U + G - 1) / G, shares = whole ? wtiles / G : (per + m.S - 2) / m.S + 1;
+      const double again = whole ? 0.0 : 2.5 + ((double)G / wtiles + 2.0) * wtiles * m.nt * m.tbn * (GM_ROWS * 4e-6 / 4.0);
+      const double cost = start + per * t_u + shares * t_w + again;
+      if (cost < best) {
+        best = cost;
+        m.G = G;
+      }
     }
+    k = {most, wtiles, m.S, m.tbn, (unsigned)plain, m.G, best};
   }
+  m.G = k.G;
   m.base = U / m.G;
   m.rem = U % m.G;
+  if (cost_out) *cost_out = k.cost;
   return m;
 }
 
@@ -825,7 +846,8 @@ int ks_launch_gemm_q4k(ks_ctx* ctx, const ks_gemm_job& job) {
   a.cols = job.cols;
   a.n_tok = job.n_tok;
   a.np = job.np;
-  const int c = job.np <= 16 ? 0 : job.np <= 32 ? 1 : job.np <= 64 ? 2 : 3;
+  const unsigned tbn = job.map.tbn;
+  const int c = tbn <= 16 ? 0 : tbn <= 32 ? 1 : tbn <= 64 ? 2 : 3;
   const size_t smem = q4_rings(ctx, job.map.tbn, job.map.nt, &a.n_raw, &a.n_b);
   a.err = (unsigned*)ctx->ws + KS_WS_ERR_WORD;
   a.wait_limit = Q_WAIT;

@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(512) sdpa_merge_split_kernel(unsigned n_tok, u
     if (ck < chunks) {
 #pragma unroll
       for (int e = 0; e < 8; e++) v[kk][e] *= down;
-      put_split8(xt, np, t, ck, chunks, v[kk], true);
+      put_split8(xt, np, q4k_block(np), t, ck, chunks, v[kk], true);
     }
   }
 }
