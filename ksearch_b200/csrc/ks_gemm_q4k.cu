@@ -15,17 +15,19 @@
 //   * 16 warps: warp w owns the 32 rows of tensor-memory lane quadrant w % 4 and the 64 weights g = w / 4 of each: one
 //     LOP3 and one HFMA2 make two weights out of packed nibbles ((1024 + q) sc - 1024 sc, exact), tcgen05.st puts them where
 //     the MMA reads A.  Shared memory then carries only packed weights and B: A never passes through it;
-//   * one elected lane issues the MMAs; after a super-block tcgen05.commit hands the accumulator to the 16 warps, which
-//     fold it into registers (s times) while the next super-block's MMAs run in the other accumulator.
-// Tensor memory (512 columns): A ring of three half super-blocks (3 x 64) and two blocks of minima (2 x 16) below 224, two
-// accumulators of up to 128 columns above: up to 64 token rows x_hi and x_lo are ONE MMA of 2 NP columns, up to 128 rows two
-// MMAs of NP; more rows have one accumulator of up to 256 columns.
+//   * one elected lane issues the MMAs; after a super-block tcgen05.commit hands the accumulator to the warps that fold it into
+//     registers (s times) while the next super-block's MMAs run in the other accumulator.
+// Token rows come in blocks (the image has one part per block), two kernels by the block's rows:
+//   up to 64   one row tile per unit, the same 16 warps convert and fold, x_hi and x_lo are ONE MMA of 2 tbn columns;
+//   65 to 128  two row tiles per unit share the block's token rows, converting and folding in warps of their own.
+// Tensor memory (512 columns): A ring of three half super-blocks (3 x 64) and blocks of minima (16 each) below 224 or 256, two
+// accumulators of up to 128 columns above.
 // One CTA per SM walks its units (ks_gemm_map) without a gap between tiles: the copies of the next tile are in flight while
 // the last one is written out.
 //
 // Bound by: few token rows, the packed weights from memory and the issue slots of the dequantisation (about 1.7 instructions
-// per weight and lane of 16 warps); 256 rows, the tensor core (34 MMAs of 128x256x16 per unit, 4350 cycles) and B through
-// shared memory (64 B per cycle in, 64 B per cycle out).
+// per weight and lane of 16 warps); blocks of 128, the tensor core (73 % busy at 20480 x 2560 x 256 rows: 132 -> 72 us against
+// the kernel that wrote split weights to shared memory); few tiles, the latency of one unit and of the launches around it.
 // Every wait is bounded; on expiry the CTA raises the context's status word, waits (bounded) for what it has in flight, frees
 // its tensor memory and returns.
 #include <cuda.h>

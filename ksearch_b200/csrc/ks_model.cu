@@ -11,8 +11,8 @@
 //     (the reference runs slots serially, scheduler.rs:163-231);
 //   * the residual update after the FFN and the next layer's attention norm
 //     run as one launch (the same two-output kernel as after attention).
-// Per-layer embeddings, sliding windows and shared-KV layers of real Gemma-4
-// checkpoints are not part of this driver.
+// Per-layer embeddings and shared-KV layers of real Gemma-4 checkpoints are
+// not part of this driver.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>

@@ -1,0 +1,48 @@
+"""Decode attention on the tensor cores at the edges of its tiles, and prompt chunks against the same attention taken row by
+row.  Oracle and tolerances are those of the other attention tests (crates/ksearch_kernels/src/lib.rs:1117-1237): q and p enter
+as two f16 terms and K, V as exact integers with f32 scales, so the bound is that of f32 sums in another order."""
+import numpy as np
+import pytest
+
+from ksearch_b200 import F16, F32, Eng, synth
+from ksearch_b200 import model as ksm
+from tests.test_gpu_ops import _attn_case
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("act", [F32, F16])
+@pytest.mark.parametrize("n_q,n_kv,hd", [(8, 1, 256), (8, 2, 256), (8, 4, 256), (8, 8, 256), (4, 2, 128), (8, 1, 128)])
+def test_decode_attention_tile_edges(ctx, oracle, act, n_q, n_kv, hd):
+    """Context lengths around the 16-position tiles and the 128-position splits, windows that start off a tile."""
+    tlens = [1, 15, 16, 17, 127, 128, 129, 300]
+    starts = [0, 0, 3, 0, 1, 0, 17, 83]
+    for ns in (1, 3):
+        _attn_case(ctx, oracle, Eng(act), len(tlens), n_q, n_kv, hd, 512, tlens, starts, hd ** -0.5, ns, act=act)
+
+
+@pytest.mark.parametrize("hd,n_kv,window", [(256, 1, 0), (256, 2, 40), (128, 2, 0)])
+def test_prompt_chunks_at_odd_sizes(ctx, oracle, hd, n_kv, window):
+    """Chunks whose rows and positions end inside a tile, whole context and window: logits after the prompt match the CPU
+    decoder's (the model's bound: 1e-3 of the logit scale)."""
+    cfg = ksm.tiny_config(max_seq=320, n_kv=n_kv)
+    cfg.hd = hd
+    if window:
+        cfg.sliding_window, cfg.swa_layers = window, 1
+    model, T = ksm.GemmaCudaModel.synthetic(ctx, cfg, seed=31, keep=True)
+    model.slot_alloc()
+    toks = [int(t) for t in synth.token_ids(31, "p", 212, cfg.vocab)]
+    cpu = oracle.CpuDecoder(oracle.decoder_cfg(cfg), T)
+    at = 0
+    for n in (3, 17, 65, 126):
+        model.prefill(0, toks[at:at + n])
+        for t in toks[at:at + n]:
+            cpu.forward_token(t, False)
+        at += n
+    model.forward(0, 1, [toks[at]], True)
+    ctx.synchronize()
+    cpu.forward_token(toks[at], True)
+    want, got = cpu.logits().astype(np.float64), model.read_debug(1, 0).astype(np.float64)
+    assert np.abs(got - want).max() <= 1e-3 * np.abs(want).max()
+    cpu.close()
+    model.close()
