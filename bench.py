@@ -333,8 +333,8 @@ def gemm_shape(ctx, dtype, rows, cols, n_tok, tag):
     flops = 2.0 * rows * cols * n_tok
     return {"shape": f"{'Q4_K' if dtype == Q4K else 'Q6_K'} {rows}x{cols} x {n_tok} rows, fp32 x/y", "us": ms * 1e3,
             "weight_gbs": one.nbytes / ms / 1e6, "tflops_useful": flops / ms / 1e9,
-            "tflops_issued": 3.0 * flops / ms / 1e9,
-            "note": "three f16 products per weight and x (hi.hi + hi.lo + lo.hi) keep f32 accuracy; bound by the CUDA-core dequantisation and instruction issue"}
+            "tflops_issued": 2.0 * flops / ms / 1e9,
+            "note": "two f16 products per weight and x (exact integer weight x hi and lo of x) keep f32 accuracy; few tiles: launches and the latency of a unit, many: the tensor core"}
 
 
 def attention_shapes(ctx, peak):
