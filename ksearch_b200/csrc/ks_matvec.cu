@@ -489,9 +489,10 @@ static int check_w(ks_ctx* ctx, const char* what, ks_dtype wd, const ks_buf* W, 
 // the matvec's extra rows.  Measured, matvec against GEMM: Q4_K 256x512 8 rows 7.9 / 8.9 us, 1000x1536 4 rows 8.7 / 9.0,
 // 6 rows 12.4 / 8.9, 4096x1536 2 rows 7.1 / 7.3, 3 rows 9.5 / 7.3, 20480x2560 8 rows 104 / 17; Q6_K 512x1536 2 rows
 // 7.0 / 7.2, 3 rows 10.5 / 6.9, and where the few-row kernel does not reach 20480x4096 2 rows 68 / 79, 3 rows 129 / 79.
-// A captured stream keeps the matvec: the context's scratch may be replaced before the graph is replayed.
-static bool few_rows_gemm(const ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_t cols, ks_dtype act, size_t x_off, int n_tok) {
-  if (n_tok < 2 || act != KS_F32 || x_off % 4) return false;
+// A captured stream keeps the matvec: the context's scratch may be replaced before the graph is replayed.  So do token rows that
+// do not start on 16 bytes (a wrapped buffer, an odd offset): the operand split reads them 16 bytes at a time, the matvec needs not.
+static bool few_rows_gemm(const ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_t cols, ks_dtype act, const void* x, int n_tok) {
+  if (n_tok < 2 || act != KS_F32 || ((uintptr_t)x & 15)) return false;
   const double work = (double)rows * (double)cols * n_tok;
   if (wdtype == KS_Q4K ? work < (n_tok == 2 ? 14e6 : 6.5e6) : !ks_gemm_few_rows_q6k(ctx, rows, cols) ? n_tok == 2 || work < 64e6 : work < (n_tok == 2 ? 3e6 : 2e6))
     return false;
@@ -511,17 +512,18 @@ int ks_matvec(ks_ctx* ctx, size_t rows, size_t cols, ks_dtype wdtype, const ks_b
   const size_t ab = ks_act_bytes(act);
   KS_REQUIRE(ctx, ks_fits(x, x_off * ab, (size_t)n_tok * cols * ab), "matvec: x buffer too small");
   KS_REQUIRE(ctx, ks_fits(y, y_off * ab, (size_t)n_tok * rows * ab), "matvec: y buffer too small");
-  if (n_tok > 8 || few_rows_gemm(ctx, wdtype, rows, cols, act, x_off, n_tok)) {  // the reference's mul_mm route (lib.rs:1414): a tensor-core GEMM over all rows at once
-    KS_REQUIRE(ctx, act == KS_F32 && (wdtype == KS_Q4K || wdtype == KS_Q6K) && cols % 256 == 0 && x_off % 4 == 0,
-               "matvec: batches of more than 8 rows need f32 activations, Q4K/Q6K weights, cols %% 256 == 0 and x_off %% 4 == 0");
+  const void* xp = (const char*)x->dptr + x_off * ab;
+  if (n_tok > 8 || few_rows_gemm(ctx, wdtype, rows, cols, act, xp, n_tok)) {  // the reference's mul_mm route (lib.rs:1414): a tensor-core GEMM over all rows at once
+    KS_REQUIRE(ctx, n_tok <= 8 || (act == KS_F32 && x_off % 4 == 0 && ((uintptr_t)xp & 15) == 0),
+               "matvec: batches of more than 8 rows need f32 activations, x_off %% 4 == 0 and an x that starts on 16 bytes");
     void* scratch = nullptr;
     if ((rc = ks_ctx_gemm_scratch(ctx, ks_gemm_kq_bytes(ctx, wdtype, rows, cols, n_tok), &scratch))) return rc;
-    rc = ks_launch_gemm_kq(ctx, wdtype, rows, cols, (const uint8_t*)W->dptr + w_byte_off, (const float*)x->dptr + x_off, cols,
+    rc = ks_launch_gemm_kq(ctx, wdtype, rows, cols, (const uint8_t*)W->dptr + w_byte_off, (const float*)xp, cols,
                            (float*)y->dptr + y_off, rows, n_tok, scratch);
     return rc == 1 ? ks_fail(ctx, KS_ERR_UNSUPPORTED, "matvec: %zux%zu with %d rows does not fit the GEMM kernel", rows, cols, n_tok) : rc;
   }
   ks_mv_seg seg{(const uint8_t*)W->dptr + w_byte_off, (char*)y->dptr + y_off * ab, (unsigned)rows};
-  return ks_launch_matvec(ctx, wdtype, &seg, 1, KS_EPI_PLAIN, cols, act, (const char*)x->dptr + x_off * ab, n_tok, nullptr);
+  return ks_launch_matvec(ctx, wdtype, &seg, 1, KS_EPI_PLAIN, cols, act, xp, n_tok, nullptr);
 }
 
 int ks_matvec_qkv(ks_ctx* ctx, size_t q_rows, size_t kv_rows, size_t cols, ks_dtype dq, ks_dtype dk, ks_dtype dv,

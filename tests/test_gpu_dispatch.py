@@ -1,0 +1,44 @@
+"""Calls at the edges of the dispatch: what the fast kernels do not take has to reach the kernel that does, or be refused on
+the host.  Oracle and bounds are those of the op's own tests."""
+import numpy as np
+import pytest
+
+from ksearch_b200 import Q4K, Q6K, KsError, _lib, synth
+from tests.test_gpu_gemm import _check
+from tests.test_gpu_matvec import _gen
+
+pytestmark = pytest.mark.gpu
+
+
+def _view(ctx, buf, byte_off):
+    """The library's handle of a caller's memory that starts byte_off bytes into buf."""
+    return ctx.lib.ks_buf_wrap(ctx.h, buf.ptr + byte_off, buf.nbytes - byte_off)
+
+
+@pytest.mark.parametrize("dtype,rows,cols,batch", [(Q4K, 4096, 1536, 3), (Q6K, 2048, 1536, 3), (Q4K, 4096, 512, 8)])
+def test_few_rows_off_16_bytes(ctx, oracle, dtype, rows, cols, batch):
+    """Shapes whose 2..8 token rows go through the GEMM when they start on 16 bytes.  Where they do not (a wrapped buffer, an
+    odd element offset), the batch matvec takes the call in its one launch; a batch of more than 8 is refused."""
+    W = _gen(dtype, 71, "W", rows, cols)
+    x = synth.normals(71, "x", 9 * cols).reshape(9, cols).astype(np.float32)
+    bw, y = ctx.buffer_bytes(W), ctx.buffer_empty_f32(9 * rows)
+    bx = ctx.buffer_bytes(np.concatenate([np.zeros(4, np.float32), x.ravel(), np.zeros(4, np.float32)]))
+    y32, y64 = oracle.matvec(dtype, W, rows, cols, x[:batch])
+    for floats, x_off, launches in ((4, 0, (2, 3)), (3, 1, (2, 3)), (1, 3, (2, 3)), (0, 4, (2, 3))):   # all of them name x itself
+        h = _view(ctx, bx, 4 * floats)
+        before = ctx.launch_count()
+        ctx.check(ctx.lib.ks_matvec(ctx.h, rows, cols, dtype, bw.h, 0, 0, h, x_off, y.h, 0, batch))
+        assert ctx.launch_count() - before in launches
+        _check(ctx.read_f32(y, batch * rows).reshape(batch, rows), y32, y64, f"view at {floats} floats, offset {x_off}")
+        ctx.lib.ks_buf_free(ctx.h, h)
+    moved = ctx.buffer_bytes(np.concatenate([np.zeros(5, np.float32), x.ravel()]))                     # x at 20 bytes past a 256-byte boundary
+    for floats, x_off in ((5, 0), (0, 5), (1, 4)):
+        h = _view(ctx, moved, 4 * floats)
+        before = ctx.launch_count()
+        ctx.check(ctx.lib.ks_matvec(ctx.h, rows, cols, dtype, bw.h, 0, 0, h, x_off, y.h, 0, batch))
+        assert ctx.launch_count() - before == 1
+        _check(ctx.read_f32(y, batch * rows).reshape(batch, rows), y32, y64, f"view at {floats} floats, offset {x_off}")
+        with pytest.raises(KsError) as ei:
+            ctx.check(ctx.lib.ks_matvec(ctx.h, rows, cols, dtype, bw.h, 0, 0, h, x_off, y.h, 0, 9))
+        assert ei.value.code == _lib.ERR_INVALID
+        ctx.lib.ks_buf_free(ctx.h, h)
