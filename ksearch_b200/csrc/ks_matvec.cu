@@ -482,6 +482,7 @@ static int check_w(ks_ctx* ctx, const char* what, ks_dtype wd, const ks_buf* W, 
   KS_REQUIRE(ctx, ks_fits(W, off, need), "%s: weight buffer too small: need %zu B at offset %zu, have %zu", what, need, off,
              W ? W->bytes : 0);
   KS_REQUIRE(ctx, off % (wd == KS_Q4K ? 16 : 2) == 0, "%s: weight byte offset %zu misaligned", what, off);
+  KS_REQUIRE(ctx, ((uintptr_t)W->dptr + off) % (wd == KS_Q4K ? 16 : 2) == 0, "%s: weight pointer misaligned", what);  // a wrapped buffer may start anywhere
   return KS_OK;
 }
 

@@ -42,3 +42,19 @@ def test_few_rows_off_16_bytes(ctx, oracle, dtype, rows, cols, batch):
             ctx.check(ctx.lib.ks_matvec(ctx.h, rows, cols, dtype, bw.h, 0, 0, h, x_off, y.h, 0, 9))
         assert ei.value.code == _lib.ERR_INVALID
         ctx.lib.ks_buf_free(ctx.h, h)
+
+
+@pytest.mark.parametrize("dtype,byte_off", [(Q4K, 8), (Q6K, 1)])
+@pytest.mark.parametrize("batch", [1, 3, 9])
+def test_weights_off_their_alignment_are_refused(ctx, dtype, byte_off, batch):
+    """Q4_K rows start on 16 bytes, Q6_K rows on 2: a wrapped buffer that starts elsewhere is refused before any launch."""
+    rows, cols = 2048, 1536
+    W = _gen(dtype, 72, "W", rows, cols)
+    bw = ctx.buffer_bytes(np.concatenate([np.zeros(16, np.uint8), np.frombuffer(W, np.uint8)]))
+    bx, y = ctx.buffer_empty_f32(batch * cols), ctx.buffer_empty_f32(batch * rows)
+    h = _view(ctx, bw, byte_off)
+    before = ctx.launch_count()
+    with pytest.raises(KsError) as ei:
+        ctx.check(ctx.lib.ks_matvec(ctx.h, rows, cols, dtype, h, 0, 0, bx.h, 0, y.h, 0, batch))
+    assert ei.value.code == _lib.ERR_INVALID and ctx.launch_count() == before
+    ctx.lib.ks_buf_free(ctx.h, h)
