@@ -511,6 +511,8 @@ constexpr int GM_ROW_THREADS = 1024;  // threads of a block that writes one toke
 // blocks per (padded) token row, 8 values per thread: the row maximum that scales the image meets in distributed shared memory,
 // and few token rows still make enough blocks (8 rows of 10240 values: 64 blocks instead of 16).
 constexpr unsigned GM_GELU_CL = 4, GM_GELU_THREADS = 512;
+// The longest rows the two epilogues take: eight values per thread of one block, and of a cluster.
+constexpr size_t GM_NORM_MOST = 8 * 1024, GM_GELU_MOST = 8 * GM_GELU_CL * GM_GELU_THREADS;
 __global__ void __cluster_dims__(GM_GELU_CL, 1, 1) __launch_bounds__(GM_GELU_THREADS)
     gemm_finish_gelu_split_kernel(const float* P0, const float* P1, size_t part_stride, ks_gemm_map map, unsigned n_tok, unsigned np, unsigned rows,
                                   __half* xt) {
@@ -741,6 +743,9 @@ bool gemm_covers(ks_dtype wdtype, size_t cols, int n_tok) {
 
 bool ks_gemm_few_rows_q6k(const ks_ctx* ctx, size_t rows, size_t cols) { return ks_gemm_q6k_skinny_covers(ctx, rows, (unsigned)cols); }
 unsigned ks_gemm_np(int n_tok) { return gemm_np(n_tok); }
+bool ks_gemm_layers_cover(size_t hidden, size_t ffn, size_t q_cols) {
+  return hidden % 256 == 0 && ffn % 256 == 0 && q_cols % 256 == 0 && hidden <= GM_NORM_MOST && ffn <= GM_GELU_MOST;
+}
 
 // Bytes of the B image of n_tok rows of `cols` values (hi + lo halves, token count padded to 16).
 size_t ks_gemm_xt_bytes(size_t cols, int n_tok) {  // image + one factor per row, whatever the blocks
@@ -765,10 +770,10 @@ int ks_launch_gemm_split(ks_ctx* ctx, ks_dtype wdtype, const float* x, size_t ld
 static int launch_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* const* W, const size_t* rows, size_t cols, const void* xt,
                        int n_tok, float* const* y, const size_t* ldy, float* P, int mode, const ks_gemm_epi* epi, Blocks blocks) {
   if (!gemm_covers(wdtype, cols, n_tok) || n_seg < 1 || n_seg > 3) return ks_fail(ctx, KS_ERR_UNSUPPORTED, "gemm: shape not covered");
-  if ((mode == KS_GEMM_NORM_SPLIT && (n_seg != 1 || !epi || rows[0] % 8 || rows[0] > 8192)) ||
+  if ((mode == KS_GEMM_NORM_SPLIT && (n_seg != 1 || !epi || rows[0] % 8 || rows[0] > GM_NORM_MOST)) ||
       (mode == KS_GEMM_QKV && (n_seg != 3 || !epi || (epi->hd != 128 && epi->hd != 256) || rows[0] != (size_t)epi->n_q * epi->hd ||
                                rows[1] != (size_t)epi->n_kv * epi->hd || rows[2] != rows[1])) ||
-      (mode == KS_GEMM_GELU_SPLIT && (n_seg != 2 || !epi || rows[0] != rows[1] || rows[0] % 8 || rows[0] > 8u * GM_GELU_CL * GM_GELU_THREADS || rows[0] % 256)))
+      (mode == KS_GEMM_GELU_SPLIT && (n_seg != 2 || !epi || rows[0] != rows[1] || rows[0] % 8 || rows[0] > GM_GELU_MOST || rows[0] % 256)))
     return ks_fail(ctx, KS_ERR_INVALID, "gemm: bad epilogue arguments");
   const unsigned np = blocks.np;
   const ks_gemm_map map = gemm_map(ctx, wdtype, rows, n_seg, cols, n_tok, blocks, mode == KS_GEMM_PLAIN);

@@ -205,6 +205,8 @@ struct ks_gemm_epi {
 };
 int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* const* W, const size_t* rows, size_t cols, const void* xt,
                         int n_tok, float* const* y, const size_t* ldy, float* P, int mode, const ks_gemm_epi* epi);
+// Do the epilogues take every matrix of a layer of these widths?
+bool ks_gemm_layers_cover(size_t hidden, size_t ffn, size_t q_cols);
 // Split + GEMM for one matrix.  Returns 1 when the shape is not covered (cols not a multiple of 256, more than
 // 256 rows).  scratch: ks_gemm_kq_bytes.
 size_t ks_gemm_kq_bytes(const ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_t cols, int n_tok);

@@ -823,9 +823,9 @@ ks_model* ks_model_create(ks_ctx* ctx, const ks_model_config* cfg) {
     if (qn > maxcols) maxcols = qn;
     m->chunk = KS_PREFILL_CHUNK;
     while (m->chunk > 1 && (size_t)m->chunk * (maxcols / 64) * 280 + (64u << 10) > ctx->smem_optin) m->chunk--;
-    // block-aligned columns: larger batches go through the tensor-core GEMM, which computes in f32 (a chunk of an f16 model
-    // too: its rows meet f16 vectors nowhere)
-    if (H % 256 == 0 && F % 256 == 0 && qn % 256 == 0 && !getenv("KSEARCH_NO_GEMM")) {
+    // widths its epilogues take: larger batches go through the tensor-core GEMM, which computes in f32 (a chunk of an f16 model
+    // too: its rows meet f16 vectors nowhere); wider models keep the batch matvec for every batch
+    if (ks_gemm_layers_cover(H, F, qn) && !getenv("KSEARCH_NO_GEMM")) {
       const int G = KS_GEMM_CHUNK;
       m->gemm_chunk = G;
       // one launch each: q|k|v, o, gate|up, down, head

@@ -756,3 +756,29 @@ def test_f16_activation_model_runs_close(ctx, oracle):
     assert np.abs(got - want).max() <= 0.05 * np.abs(want).max()
     cpu.close()
     model.close()
+
+
+@pytest.mark.parametrize("act", [F32, F16])
+@pytest.mark.parametrize("hidden,ffn", [(512, 21504), (8448, 512)])
+def test_prompt_of_a_model_wider_than_the_gemm_epilogues(ctx, oracle, act, hidden, ffn):
+    """GeGLU rows above 16384 values and hidden rows above 8192 do not fit the GEMM's epilogues: such a model's prompts (and
+    steps of several slots) stay with the batch matvec, and its logits match the CPU decoder's: 1e-3 of their scale in f32 (the
+    model's bound), about ten f16 roundings of 2^-11 along the residual stream in f16."""
+    cfg = ksm.ModelConfig(1, hidden, ffn, 2, 1, 128, max(hidden, 1024), 32, 3, sigma_w=3e-5 if act == F16 else 0.01, sigma_embd=5e-5, act=act)
+    model, T = ksm.GemmaCudaModel.synthetic(ctx, cfg, seed=61, keep=True)
+    slots = [model.slot_alloc() for _ in range(3)]
+    toks = [int(t) for t in synth.token_ids(61, "p", 12, cfg.vocab)]
+    cpu = oracle.CpuDecoder(oracle.decoder_cfg(cfg), T)
+    for t in toks[:-1]:
+        cpu.forward_token(t, False)
+    cpu.forward_token(toks[-1], True)
+    want = cpu.logits().astype(np.float64)
+    for s in slots:
+        model.prefill(s, toks[:-1])
+    model.forward(0, 3, [toks[-1]] * 3, True)
+    ctx.synchronize()
+    for s in slots:
+        got = model.read_debug(1, s).astype(np.float64)
+        assert np.abs(got - want).max() <= (1e-3 if act == F32 else 5e-3) * np.abs(want).max()
+    cpu.close()
+    model.close()
