@@ -1314,7 +1314,7 @@ int ks_model_sample_step(ks_model* m, int first, int n, const int* tokens, const
   const size_t S = g.n_slots, head_b = S * sizeof(ks_cand_head), list_b = S * KS_CAND_MAX * sizeof(ks_cand);
   int rc;
   if (!m->cand_head && (rc = dev_alloc(m, (void**)&m->cand_head, head_b + list_b))) return rc;
-  if (!m->host_cand && cudaMallocHost(&m->host_cand, head_b + list_b) != cudaSuccess) {
+  if (!m->host_cand && cudaMallocHost(&m->host_cand, head_b + list_b + sizeof(unsigned)) != cudaSuccess) {  // lists, then the status word
     m->host_cand = nullptr;
     return ks_fail(c, KS_ERR_OOM, "sample_step: pinned allocation failed");
   }
@@ -1337,7 +1337,10 @@ int ks_model_sample_step(ks_model* m, int first, int n, const int* tokens, const
   KS_CUDA(c, cudaMemcpyAsync(host, dev, n * sizeof(ks_cand_head), cudaMemcpyDeviceToHost, c->stream));
   KS_CUDA(c, cudaMemcpy2DAsync(hlist, KS_CAND_MAX * sizeof(ks_cand), dlist, KS_CAND_MAX * sizeof(ks_cand), FEW * sizeof(ks_cand), n, cudaMemcpyDeviceToHost,
                                c->stream));
-  if ((rc = ks_synchronize(c))) return rc;
+  unsigned* status = (unsigned*)(host + head_b + list_b);
+  KS_CUDA(c, cudaMemcpyAsync(status, (unsigned*)c->ws + KS_WS_ERR_WORD, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+  KS_CUDA(c, cudaStreamSynchronize(c->stream));
+  if ((rc = check_device_status(m, status, first, n, 1))) return rc;
   const ks_cand_head* hh = (const ks_cand_head*)host;
   for (int s = 0; s < n; s++) {
     ks_cand* l = hlist + (size_t)s * KS_CAND_MAX;

@@ -4,7 +4,7 @@ filter off, with more survivors than the list holds, and greedy."""
 import numpy as np
 import pytest
 
-from ksearch_b200 import F16, F32, CudaContext, synth
+from ksearch_b200 import F16, F32, CudaContext, KsError, _lib, synth
 from ksearch_b200 import model as ksm
 from ksearch_b200.sample import sample_softcap_min_p
 
@@ -28,5 +28,38 @@ def test_sample_step_takes_the_cpu_samplers_tokens(n, act):
         assert got == want, (temp, min_p)
         ids = got
     assert [model.seq_len(s) for s in slots] == [8] * n
+    model.close()
+    c.close()
+
+
+def test_sample_step_rewinds_after_a_wait_that_gave_up():
+    """The persistent kernel told to wait for something nobody writes: the blocking step reports KS_ERR_TIMEOUT and leaves the
+    slot where it was, as decode_token does; the same step afterwards gives the token it gives without the stall."""
+    c = CudaContext(0, flags=1)
+    cfg = ksm.tiny_config(max_seq=48)
+    model = ksm.GemmaCudaModel.synthetic(c, cfg, seed=32)
+    ids = [int(t) for t in synth.token_ids(32, "ids", 6, cfg.vocab)]
+    args = (0, [0.8], [0.05], [77])
+
+    def run(stall):
+        model.slot_reset(0)
+        model.prefill(0, ids[:4])
+        model.sample_step([ids[4]], *args)
+        if stall:
+            model.debug_set(model.POLL_LIMIT, 2000)
+            model.debug_set(model.STALL, 1)
+            with pytest.raises(KsError) as ei:
+                model.sample_step([ids[5]], *args)
+            assert ei.value.code == _lib.ERR_TIMEOUT and model.seq_len(0) == 5
+            model.debug_set(model.STALL, 0)
+            model.debug_set(model.POLL_LIMIT, 1 << 21)
+        tok = model.sample_step([ids[5]], *args)
+        assert model.seq_len(0) == 6
+        return tok, model.read_debug(1, 0)
+
+    model.slot_alloc()
+    tok, logits = run(False)
+    again, after = run(True)
+    assert again == tok and np.array_equal(after, logits)
     model.close()
     c.close()
