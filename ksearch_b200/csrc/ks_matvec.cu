@@ -492,8 +492,10 @@ static int check_w(ks_ctx* ctx, const char* what, ks_dtype wd, const ks_buf* W, 
 // 7.0 / 7.2, 3 rows 10.5 / 6.9, and where the few-row kernel does not reach 20480x4096 2 rows 68 / 79, 3 rows 129 / 79.
 // A captured stream keeps the matvec: the context's scratch may be replaced before the graph is replayed.  So do token rows that
 // do not start on 16 bytes (a wrapped buffer, an odd offset): the operand split reads them 16 bytes at a time, the matvec needs not.
+// And so do calls that an override or a stored plan speaks for: plans name matvec kernels.
 static bool few_rows_gemm(const ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_t cols, ks_dtype act, const void* x, int n_tok) {
   if (n_tok < 2 || act != KS_F32 || ((uintptr_t)x & 15)) return false;
+  if (ctx->has_override || (!ctx->plans.empty() && ks_plan_lookup(ctx, wdtype == KS_Q4K ? "mv_q4k" : "mv_q6k", rows, cols, n_tok))) return false;
   const double work = (double)rows * (double)cols * n_tok;
   if (wdtype == KS_Q4K ? work < (n_tok == 2 ? 14e6 : 6.5e6) : !ks_gemm_few_rows_q6k(ctx, rows, cols) ? n_tok == 2 || work < 64e6 : work < (n_tok == 2 ? 3e6 : 2e6))
     return false;

@@ -1,9 +1,11 @@
 """Calls at the edges of the dispatch: what the fast kernels do not take has to reach the kernel that does, or be refused on
 the host.  Oracle and bounds are those of the op's own tests."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
-from ksearch_b200 import Q4K, Q6K, KsError, _lib, synth
+from ksearch_b200 import Q4K, Q6K, CudaContext, KsError, _lib, synth
 from tests.test_gpu_gemm import _check
 from tests.test_gpu_matvec import _gen
 
@@ -58,3 +60,35 @@ def test_weights_off_their_alignment_are_refused(ctx, dtype, byte_off, batch):
         ctx.check(ctx.lib.ks_matvec(ctx.h, rows, cols, dtype, h, 0, 0, bx.h, 0, y.h, 0, batch))
     assert ei.value.code == _lib.ERR_INVALID and ctx.launch_count() == before
     ctx.lib.ks_buf_free(ctx.h, h)
+
+
+@pytest.mark.parametrize("dtype,op", [(Q4K, "mv_q4k"), (Q6K, "mv_q6k")])
+@pytest.mark.parametrize("batch", [3, 8])
+def test_plans_speak_for_few_rows_too(oracle, dtype, op, batch):
+    """A shape whose 3..8 token rows go through the GEMM by themselves: with an override, or a plan stored for that row count,
+    the matvec kernel the plan names runs (one launch), whatever the other row counts do."""
+    rows, cols = 4096, 1536
+    c = CudaContext(0)
+    W = _gen(dtype, 73, "W", rows, cols)
+    x = synth.normals(73, "x", batch * cols).reshape(batch, cols).astype(np.float32)
+    bw, bx, y = c.buffer_bytes(W), c.buffer_bytes(x), c.buffer_empty_f32(batch * rows)
+    y32, y64 = oracle.matvec(dtype, W, rows, cols, x)
+
+    def launches(n=batch):
+        before = c.launch_count()
+        c.check(c.lib.ks_matvec(c.h, rows, cols, dtype, bw.h, 0, 0, bx.h, 0, y.h, 0, n))
+        _check(c.read_f32(y, n * rows).reshape(n, rows), y32[:n], y64[:n], f"{op} x {n}")
+        return c.launch_count() - before
+
+    assert launches() > 1
+    for variant in (0, 1):
+        plan = _lib.Plan(variant=variant, nr=1 if variant == 0 else 2, nwarps=4, ctas_per_sm=2, ms=0.0)
+        c.check(c.lib.ks_plan_override(c.h, C.byref(plan)))
+        assert launches() == 1
+        c.check(c.lib.ks_plan_override(c.h, None))
+        assert launches() > 1
+        c.check(c.lib.ks_plan_set(c.h, op.encode(), rows, cols, batch, C.byref(plan)))
+        assert launches() == 1 and (batch == 3 or launches(batch - 1) > 1)
+        c.check(c.lib.ks_plan_set(c.h, op.encode(), rows, cols, batch, None))
+    assert launches() > 1
+    c.close()
