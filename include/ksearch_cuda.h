@@ -141,8 +141,10 @@ int ks_quantize_q4k(ks_ctx* ctx, ks_dtype src_dtype, const ks_buf* src, size_t s
  * y is [n_tok, rows].  K:137 matvec_wd, K:1446 matvec_wd_at (offsets),
  * K:1414 matvec_batch: up to 8 rows share one GEMV pass over the weights; 9..256 rows take the route the
  * reference gives to mul_mm (crates/ksearch_codegen/src/render.rs:1073-1291), here a tensor-core GEMM
- * (f32 activations, Q4K / Q6K weights, cols a multiple of 256, x_off a multiple of 4, x on a 16-byte boundary).  The first such call
- * grows a scratch buffer inside the context: make it outside any ks_graph capture. */
+ * (f32 activations, Q4K / Q6K weights, cols a multiple of 256, x_off a multiple of 4, x on a 16-byte boundary).
+ * Such a call may have to grow a scratch buffer of the context: make the first of a shape outside any ks_graph capture.
+ * 2..8 rows of f32 take the GEMM too where it is faster, out of scratch the context starts with (32 MB): no call of up
+ * to 8 rows allocates.  Scratch that a captured graph uses stays valid until the context goes. */
 int ks_matvec(ks_ctx* ctx, size_t rows, size_t cols, ks_dtype wdtype, const ks_buf* W, size_t w_byte_off,
               ks_dtype act, const ks_buf* x, size_t x_off, ks_buf* y, size_t y_off, int n_tok);
 /* K:227 matvec_qkv_wds: three outputs in one launch. */

@@ -67,12 +67,14 @@ ks_ctx* ks_ctx_create(int device, uint64_t flags) {
     delete c;
     return nullptr;
   }
-  if (cudaMalloc(&c->ws, 16384) != cudaSuccess || cudaMemset(c->ws, 0, 16384) != cudaSuccess) {
+  if (cudaMalloc(&c->ws, 16384) != cudaSuccess || cudaMemset(c->ws, 0, 16384) != cudaSuccess || cudaMalloc(&c->gemm_ws, KS_FEW_WS) != cudaSuccess) {
     g_create_err = "workspace allocation failed";
+    cudaFree(c->ws);
     cudaStreamDestroy(c->stream);
     delete c;
     return nullptr;
   }
+  c->gemm_ws_bytes = KS_FEW_WS;
   return c;
 }
 
@@ -86,6 +88,7 @@ void ks_ctx_destroy(ks_ctx* c) {
   if (c->stage_y) ks_buf_free(c, c->stage_y);
   if (c->ws) cudaFree(c->ws);
   if (c->gemm_ws) cudaFree(c->gemm_ws);
+  for (void* p : c->gemm_ws_old) cudaFree(p);
   if (c->t0) cudaEventDestroy(c->t0);
   if (c->t1) cudaEventDestroy(c->t1);
   cudaStreamDestroy(c->stream);
@@ -304,12 +307,17 @@ int ks_ctx_gemm_scratch(ks_ctx* c, size_t bytes, void** out) {
     if (st != cudaStreamCaptureStatusNone)
       return ks_fail(c, KS_ERR_STATE, "gemm: scratch of %zu bytes must exist before the stream is captured", bytes);
     cudaSetDevice(c->device);
-    cudaStreamSynchronize(c->stream);  // launches that still read the old scratch
-    if (c->gemm_ws) cudaFree(c->gemm_ws);
-    c->gemm_ws = nullptr;
-    c->gemm_ws_bytes = 0;
-    if (cudaMalloc(&c->gemm_ws, bytes) != cudaSuccess) return ks_fail(c, KS_ERR_OOM, "gemm: cudaMalloc(%zu) failed", bytes);
-    c->gemm_ws_bytes = bytes;
+    // at least twice the old one: what the old ones keep then never exceeds the scratch in use
+    void* p = nullptr;
+    size_t n = bytes > 2 * c->gemm_ws_bytes ? bytes : 2 * c->gemm_ws_bytes;
+    if (cudaMalloc(&p, n) != cudaSuccess) {
+      cudaGetLastError();
+      n = bytes;
+      if (cudaMalloc(&p, n) != cudaSuccess) return ks_fail(c, KS_ERR_OOM, "gemm: cudaMalloc(%zu) failed", bytes);
+    }
+    c->gemm_ws_old.push_back(c->gemm_ws);
+    c->gemm_ws = p;
+    c->gemm_ws_bytes = n;
   }
   *out = c->gemm_ws;
   return KS_OK;

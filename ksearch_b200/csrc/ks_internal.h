@@ -8,6 +8,7 @@
 #include <deque>
 #include <map>
 #include <string>
+#include <vector>
 
 #include "../../include/ksearch_cuda.h"
 
@@ -27,8 +28,12 @@ struct ks_ctx {
   ks_plan override_plan{};
   std::map<std::string, ks_plan> plans;  // op_rowsxcols[_bN] -> plan (searched, loaded or set)
   void* ws = nullptr;  // small zero-initialised device workspace (cross-block reductions)
-  void* gemm_ws = nullptr;  // token rows split into f16 terms for the tensor-core GEMM (grown outside stream capture)
+  // token rows split into f16 terms for the tensor-core GEMM, and its partials: KS_FEW_WS bytes from the start, grown (outside
+  // stream capture) only by batches of more than 8 rows.  What growth replaces stays until the context goes: captured graphs
+  // hold its address.
+  void* gemm_ws = nullptr;
   size_t gemm_ws_bytes = 0;
+  std::vector<void*> gemm_ws_old;
   // pinned staging for the *_host convenience calls
   void* stage_h = nullptr;
   size_t stage_h_bytes = 0;
@@ -181,7 +186,9 @@ uint32_t ks_sample_candidates(const ks_cand* c, size_t n, float cap, float tempe
 int ks_launch_quantize_q4k(ks_ctx* ctx, ks_dtype src_dtype, const void* src, size_t nelem, void* dst);
 size_t ks_gemm_xt_bytes(size_t cols, int n_tok);  // bytes of the split image of n_tok rows of `cols` values
 size_t ks_gemm_part_floats(const ks_ctx* ctx, size_t total_rows, size_t cols, int n_tok);  // k-split partials, at most
-// The context's scratch, grown to `bytes` (fails inside a stream capture when it would have to grow).
+// The context's scratch, grown to `bytes` (fails inside a stream capture when it would have to grow).  Batches of 2..8 rows never
+// grow it: KS_FEW_WS holds their image (4.7 MB at 65536 columns) and partials (8 rows of 262144 outputs: 8 MB a share).
+constexpr size_t KS_FEW_WS = 32u << 20;
 int ks_ctx_gemm_scratch(ks_ctx* ctx, size_t bytes, void** out);
 // x[t * ldx + k] (f32) -> the image the GEMM over weights of that dtype reads its token rows from.
 int ks_launch_gemm_split(ks_ctx* ctx, ks_dtype wdtype, const float* x, size_t ldx, int n_tok, size_t cols, void* xt);

@@ -490,7 +490,8 @@ static int check_w(ks_ctx* ctx, const char* what, ks_dtype wd, const ks_buf* W, 
 // the matvec's extra rows.  Measured, matvec against GEMM: Q4_K 256x512 8 rows 7.9 / 8.9 us, 1000x1536 4 rows 8.7 / 9.0,
 // 6 rows 12.4 / 8.9, 4096x1536 2 rows 7.1 / 7.3, 3 rows 9.5 / 7.3, 20480x2560 8 rows 104 / 17; Q6_K 512x1536 2 rows
 // 7.0 / 7.2, 3 rows 10.5 / 6.9, and where the few-row kernel does not reach 20480x4096 2 rows 68 / 79, 3 rows 129 / 79.
-// A captured stream keeps the matvec: the context's scratch may be replaced before the graph is replayed.  So do token rows that
+// No such call allocates or waits: what would not fit the scratch that every context starts with keeps the matvec, and so does a
+// captured stream (the GEMM has not been measured inside a graph of few-row calls).  So do token rows that
 // do not start on 16 bytes (a wrapped buffer, an odd offset): the operand split reads them 16 bytes at a time, the matvec needs not.
 // And so do calls that an override or a stored plan speaks for: plans name matvec kernels.
 static bool few_rows_gemm(const ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_t cols, ks_dtype act, const void* x, int n_tok) {
@@ -500,7 +501,8 @@ static bool few_rows_gemm(const ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_
   if (wdtype == KS_Q4K ? work < (n_tok == 2 ? 14e6 : 6.5e6) : !ks_gemm_few_rows_q6k(ctx, rows, cols) ? n_tok == 2 || work < 64e6 : work < (n_tok == 2 ? 3e6 : 2e6))
     return false;
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(ctx->stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(ctx->stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone &&
+         ks_gemm_kq_bytes(ctx, wdtype, rows, cols, n_tok) <= KS_FEW_WS;
 }
 
 extern "C" {

@@ -92,3 +92,44 @@ def test_plans_speak_for_few_rows_too(oracle, dtype, op, batch):
         c.check(c.lib.ks_plan_set(c.h, op.encode(), rows, cols, batch, None))
     assert launches() > 1
     c.close()
+
+
+def test_few_rows_never_allocate_and_graphs_outlive_growth(oracle):
+    """2..8 rows work out of the scratch the context starts with: device memory in use does not change, and a shape that would
+    need more takes the matvec.  A graph captured over the scratch still gives its results after a larger batch has grown it."""
+    import torch
+    c = CudaContext(0)
+    rows, cols = 2048, 1536
+    W, x = _gen(Q4K, 74, "W", rows, cols), synth.normals(74, "x", 16 * cols).reshape(16, cols).astype(np.float32)
+    y32, y64 = oracle.matvec(Q4K, W, rows, cols, x)
+    bw, bx, y, y2 = c.buffer_bytes(W), c.buffer_bytes(x), c.buffer_empty_f32(16 * rows), c.buffer_empty_f32(16 * rows)
+    most = 1 << 20                                            # rows: 8 x 2^20 sums are 32 MB by themselves
+    big, bigx, bigy = c.buffer_empty_f32(most * 72), c.buffer_empty_f32(256 * 512), c.buffer_empty_f32(256 * (most // 4))
+    c.synchronize()
+
+    def call(r, k, bW, bX, bY, n):
+        before = c.launch_count()
+        c.check(c.lib.ks_matvec(c.h, r, k, Q4K, bW.h, 0, 0, bX.h, 0, bY.h, 0, n))
+        return c.launch_count() - before
+
+    call(rows, cols, bw, bx, y, 8)                            # the driver loads kernels on their first use
+    call(most, 512, big, bigx, bigy, 8)
+    c.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    assert call(rows, cols, bw, bx, y, 8) > 1                 # the GEMM
+    _check(c.read_f32(y, 8 * rows).reshape(8, rows), y32[:8], y64[:8], "8 rows")
+    assert call(most // 2, 512, big, bigx, bigy, 8) > 1 and call(most, 512, big, bigx, bigy, 8) == 1
+    c.synchronize()
+    assert torch.cuda.mem_get_info()[0] == free
+    call(rows, cols, bw, bx, y, 16)
+    c.check(c.lib.ks_graph_begin(c.h))
+    c.check(c.lib.ks_matvec(c.h, rows, cols, Q4K, bw.h, 0, 0, bx.h, 0, y2.h, 0, 16))
+    g = c.lib.ks_graph_end(c.h)
+    assert g
+    call(most // 4, 512, big, bigx, bigy, 256)
+    c.synchronize()
+    assert torch.cuda.mem_get_info()[0] < free - (200 << 20)  # the scratch has grown
+    c.check(c.lib.ks_graph_launch(c.h, g))
+    _check(c.read_f32(y2, 16 * rows).reshape(16, rows), y32, y64, "graph after growth")
+    c.lib.ks_graph_free(c.h, g)
+    c.close()
