@@ -6,10 +6,12 @@
 //   * its share of the token rows, two f16 terms of each value, sits in 32 registers as B fragments and is loaded once;
 //   * packed rows come by cp.async into a ring of the warp's own (16 rows x 80 bytes per tile), requested before the wait for
 //     the previous kernel; no warp waits for another inside a tile;
-//   * A is the packed nibble itself: masked in place it is the f16 subnormal q 2^-24 (q 2^-20 in the high half), which the
-//     tensor core multiplies exactly, so two weights cost one LOP3.  Tokens are the 8 columns; their first and second terms
-//     go into the same f32 sums of a 32-column sub-block, which then take the sub-block's scale in f32.  The minima are one
-//     more mma: A = m 2^-24, B = the image's sub-block sums;
+//   * A is q - 8 as f16, exact, by one LOP3 and one HADD2 (HFMA2) per two weights.  Tokens are the 8 columns; their second and
+//     first terms go into the same f32 sums of a 32-column sub-block, the small ones first, which then take the sub-block's
+//     scale in f32.  The eights and the minima are two more mmas: A = scales, minima, B = the image's sub-block sums.
+//     (The nibble masked in place is the f16 subnormal q 2^-24 and saves the HADD2, but products seem to be aligned by their
+//     operands' exponents, not by their own leading bits: the error against 64 bits was 4 times the matvec's on normal rows and
+//     20 to 40 times on rows with outliers.  Centred operands keep the sums as small as the result.);
 //   * the warps' sums of a tile meet in shared memory, four tiles at a time, in warp order.
 // The block's columns are one of `splits` shares of the row (at most 20 warps of 128); every share leaves one partial.
 // Bound by instructions (about 190 per warp and tile of 16 x 128 weights) where there are many rows, else by the latency of
@@ -49,6 +51,15 @@ __device__ __forceinline__ void header_half(const uint4 h, unsigned half, uint32
     sc = (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u);
     mn = ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u);
   }
+}
+// The nibbles 0 (1) of bytes 0 and 2 as two halves n - 8.
+__device__ __forceinline__ uint32_t nib_lo(uint32_t w) { return pack_h2(__hadd2(as_h2((w & 0x000F000Fu) | 0x64006400u), __float2half2_rn(-1032.0f))); }
+__device__ __forceinline__ uint32_t nib_hi(uint32_t w) {
+  return pack_h2(__hfma2(as_h2((w & 0x00F000F0u) | 0x64006400u), __float2half2_rn(0.0625f), __float2half2_rn(-72.0f)));
+}
+// Two of four bytes below 64 as halves (sel: 0x4140 the first two, 0x4342 the last two).
+__device__ __forceinline__ uint32_t bytes_h2(uint32_t v, uint32_t sel) {
+  return pack_h2(__hsub2(as_h2(__byte_perm(v, 0x64646464u, sel)), __float2half2_rn(1024.0f)));
 }
 // Byte j of v as a float.
 __device__ __forceinline__ float byte_f(uint32_t v, unsigned j) { return __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7540u + j)) - 8388608.0f; }
@@ -108,7 +119,7 @@ __global__ void __launch_bounds__(SK_MAX_WARPS * 32, 1) gemm_q4k_skinny_kernel(c
     bs = *reinterpret_cast<const uint32_t*>(x + (size_t)(32u + 2u * half + (t & 1u)) * 2u * a.np * 8u + g * 8u + 2u * (t >> 1));
   }
   const float* up = reinterpret_cast<const float*>(a.xt + xt_scale_off(a.cols, a.np));
-  const uint32_t msel = (t & 1u) ? 0x4342u : 0x4140u;  // this lane's two minima as halves
+  const uint32_t msel = (t & 1u) ? 0x4342u : 0x4140u;  // this lane's two scales and minima
   unsigned buf = 0;
 
   for (unsigned k0 = 0; k0 < n; k0 += SK_GROUP) {
@@ -124,23 +135,26 @@ __global__ void __launch_bounds__(SK_MAX_WARPS * 32, 1) gemm_q4k_skinny_kernel(c
       uint32_t sca, mna, scb, mnb;
       header_half(ha, half, sca, mna);
       header_half(hb, half, scb, mnb);
-      float cm[4] = {0.f, 0.f, 0.f, 0.f}, tot[4];
-      mma16816(cm, __byte_perm(mna, 0u, msel), __byte_perm(mnb, 0u, msel), 0u, 0u, bs, 0u);
+      float cm[4] = {0.f, 0.f, 0.f, 0.f}, cs[4] = {0.f, 0.f, 0.f, 0.f}, tot[4];
+      mma16816(cm, bytes_h2(mna, msel), bytes_h2(mnb, msel), 0u, 0u, bs, 0u);
+      mma16816(cs, bytes_h2(sca, msel), bytes_h2(scb, msel), 0u, 0u, bs, 0u);
 #pragma unroll
       for (unsigned uu = 0; uu < 2; uu++) {
         const uint2 qa = *reinterpret_cast<const uint2*>(ra + 8u * t + 16u + 32u * uu), qb = *reinterpret_cast<const uint2*>(rb + 8u * t + 16u + 32u * uu);
         const uint32_t a8 = qa.x >> 8, b8 = qb.x >> 8, a9 = qa.y >> 8, b9 = qb.y >> 8;
 #pragma unroll
         for (unsigned hn = 0; hn < 2; hn++) {
-          constexpr uint32_t LO = 0x000F000Fu;
-          const uint32_t M = hn ? LO << 4 : LO;
           const unsigned j = 2u * uu + hn;
+          const uint32_t xa = hn ? nib_hi(qa.x) : nib_lo(qa.x), xb = hn ? nib_hi(qb.x) : nib_lo(qb.x), xa8 = hn ? nib_hi(a8) : nib_lo(a8),
+                         xb8 = hn ? nib_hi(b8) : nib_lo(b8);
+          const uint32_t ya = hn ? nib_hi(qa.y) : nib_lo(qa.y), yb = hn ? nib_hi(qb.y) : nib_lo(qb.y), ya8 = hn ? nib_hi(a9) : nib_lo(a9),
+                         yb8 = hn ? nib_hi(b9) : nib_lo(b9);
           float c[4] = {0.f, 0.f, 0.f, 0.f};
-          mma16816(c, qa.x & M, qb.x & M, a8 & M, b8 & M, bh[j].x, bh[j].y);
-          mma16816(c, qa.y & M, qb.y & M, a9 & M, b9 & M, bh[j].z, bh[j].w);
-          mma16816(c, qa.x & M, qb.x & M, a8 & M, b8 & M, bl[j].x, bl[j].y);
-          mma16816(c, qa.y & M, qb.y & M, a9 & M, b9 & M, bl[j].z, bl[j].w);
-          const float fa = byte_f(sca, j) * (hn ? 0.0625f : 1.0f), fb = byte_f(scb, j) * (hn ? 0.0625f : 1.0f);
+          mma16816(c, xa, xb, xa8, xb8, bl[j].x, bl[j].y);
+          mma16816(c, ya, yb, ya8, yb8, bl[j].z, bl[j].w);
+          mma16816(c, xa, xb, xa8, xb8, bh[j].x, bh[j].y);
+          mma16816(c, ya, yb, ya8, yb8, bh[j].z, bh[j].w);
+          const float fa = byte_f(sca, j), fb = byte_f(scb, j);
           tot[0] = j ? fmaf(fa, c[0], tot[0]) : fa * c[0];
           tot[1] = j ? fmaf(fa, c[1], tot[1]) : fa * c[1];
           tot[2] = j ? fmaf(fb, c[2], tot[2]) : fb * c[2];
@@ -148,8 +162,9 @@ __global__ void __launch_bounds__(SK_MAX_WARPS * 32, 1) gemm_q4k_skinny_kernel(c
         }
       }
       float2 da = __half22float2(as_h2(ha.x)), db = __half22float2(as_h2(hb.x));  // (d, dmin)
-      da.x *= 16777216.0f; db.x *= 16777216.0f;      // the weights' 2^24
-      da.y *= 536870912.0f; db.y *= 536870912.0f;    // and 2^5 of the sums
+      da.y *= 32.0f; db.y *= 32.0f;                                               // the sums carry 2^-5
+#pragma unroll
+      for (int e = 0; e < 4; e++) tot[e] = fmaf(256.0f, cs[e], tot[e]);
       float* ps = psum + (size_t)((buf + kk) * a.warps + warp) * 128u + g * 8u + 2u * t;
       *reinterpret_cast<float2*>(ps) = make_float2(da.x * tot[0] - da.y * cm[0], da.x * tot[1] - da.y * cm[1]);
       *reinterpret_cast<float2*>(ps + 64) = make_float2(db.x * tot[2] - db.y * cm[2], db.x * tot[3] - db.y * cm[3]);

@@ -133,3 +133,24 @@ def test_few_rows_never_allocate_and_graphs_outlive_growth(oracle):
     _check(c.read_f32(y2, 16 * rows).reshape(16, rows), y32, y64, "graph after growth")
     c.lib.ks_graph_free(c.h, g)
     c.close()
+
+
+@pytest.mark.parametrize("dtype,rows,cols,batch,launches", [
+    (Q4K, 4096, 1536, 3, (2, 3)), (Q4K, 1024, 10240, 4, (2, 3)), (Q4K, 16384, 512, 8, (2, 3)),   # the few-row kernels
+    (Q6K, 4096, 1536, 3, (2,)), (Q6K, 2048, 2560, 8, (2,)),
+])
+def test_few_rows_are_as_exact_as_the_matvec(ctx, oracle, dtype, rows, cols, batch, launches):
+    """2..8 token rows with a few channels a thousand times the rest, as activations have them, against 64 bits.  The batch
+    matvec is 1.5e-7 off (relative 2-norm): f32 operands and sums of up to 10240 terms in 32-term blocks, a few 2^-24.  The
+    bound is 3.5e-7, six units of 2^-24; sums that lose low bits against the large channels are ten times that."""
+    W = _gen(dtype, 75, f"W{rows}x{cols}", rows, cols)
+    x = synth.normals(75, f"x{cols}", batch * cols).reshape(batch, cols).astype(np.float32)
+    x[:, 7::251] *= 1000.0
+    bw, bx, y = ctx.buffer_bytes(W), ctx.buffer_bytes(x), ctx.buffer_empty_f32(batch * rows)
+    before = ctx.launch_count()
+    ctx.check(ctx.lib.ks_matvec(ctx.h, rows, cols, dtype, bw.h, 0, 0, bx.h, 0, y.h, 0, batch))
+    assert ctx.launch_count() - before in launches
+    got = ctx.read_f32(y, batch * rows).reshape(batch, rows).astype(np.float64)
+    want = x.astype(np.float64) @ oracle.dequant(dtype, W, rows * cols).astype(np.float64).reshape(rows, cols).T
+    err = np.linalg.norm(got - want, axis=1) / np.linalg.norm(want, axis=1)
+    assert err.max() <= 3.5e-7, err
