@@ -138,6 +138,8 @@ def test_few_rows_never_allocate_and_graphs_outlive_growth(oracle):
 @pytest.mark.parametrize("dtype,rows,cols,batch,launches", [
     (Q4K, 4096, 1536, 3, (2, 3)), (Q4K, 1024, 10240, 4, (2, 3)), (Q4K, 16384, 512, 8, (2, 3)),   # the few-row kernels
     (Q6K, 4096, 1536, 3, (2,)), (Q6K, 2048, 2560, 8, (2,)),
+    (Q6K, 2048, 10240, 4, (1,)), (Q6K, 2007, 2048, 8, (1,)),                                     # outside the Q6_K one: the matvec
+    (Q6K, 512, 10240, 8, (2, 3)),                                                                # more than the matvec can stage
 ])
 def test_few_rows_are_as_exact_as_the_matvec(ctx, oracle, dtype, rows, cols, batch, launches):
     """2..8 token rows with a few channels a thousand times the rest, as activations have them, against 64 bits.  The batch
@@ -153,4 +155,4 @@ def test_few_rows_are_as_exact_as_the_matvec(ctx, oracle, dtype, rows, cols, bat
     got = ctx.read_f32(y, batch * rows).reshape(batch, rows).astype(np.float64)
     want = x.astype(np.float64) @ oracle.dequant(dtype, W, rows * cols).astype(np.float64).reshape(rows, cols).T
     err = np.linalg.norm(got - want, axis=1) / np.linalg.norm(want, axis=1)
-    assert err.max() <= 3.5e-7, err
+    assert err.max() <= (3.5e-7 if (dtype, cols, batch) != (Q6K, 10240, 8) else 1e-5), err   # there the tcgen05 kernel: f32 sums over all columns
