@@ -489,7 +489,7 @@ static int check_w(ks_ctx* ctx, const char* what, ks_dtype wd, const ks_buf* W, 
 // 2..8 token rows: the tensor cores, whose time hardly depends on the row count, from where their three launches cost less than
 // the matvec's extra rows.  Measured, matvec against GEMM: Q4_K 256x512 8 rows 7.9 / 8.9 us, 1000x1536 4 rows 8.7 / 9.0,
 // 6 rows 12.4 / 8.9, 4096x1536 2 rows 7.1 / 7.3, 3 rows 9.5 / 7.3, 20480x2560 8 rows 104 / 17; Q6_K 512x1536 2 rows
-// 7.0 / 7.2, 3 rows 10.5 / 6.9.  Where the few-row Q6_K kernel does not reach (more than 2560 columns, rows not a multiple of 8)
+// 7.0 / 7.2, 3 rows 10.5 / 6.9.  Where the few-row Q6_K kernel does not reach (more than 2560 columns, rows not a multiple of 8, packed rows off 16 bytes)
 // the matvec keeps the call although the tcgen05 kernel is faster from 3 rows on (20480x4096 129 / 79 us): that kernel's f32
 // sums over many columns are 15 times as far from 64 bits (2048x10240 x 4: 1.5e-7 / 2.4e-6).  It takes only rows that the
 // matvec cannot stage side by side (80 bytes of shared memory per 16 columns and row).
@@ -497,12 +497,12 @@ static int check_w(ks_ctx* ctx, const char* what, ks_dtype wd, const ks_buf* W, 
 // captured stream (the GEMM has not been measured inside a graph of few-row calls).  So do token rows that
 // do not start on 16 bytes (a wrapped buffer, an odd offset): the operand split reads them 16 bytes at a time, the matvec needs not.
 // And so do calls that an override or a stored plan speaks for: plans name matvec kernels.
-static bool few_rows_gemm(const ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_t cols, ks_dtype act, const void* x, int n_tok) {
+static bool few_rows_gemm(const ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_t cols, const uint8_t* W, ks_dtype act, const void* x, int n_tok) {
   if (n_tok < 2 || act != KS_F32 || ((uintptr_t)x & 15)) return false;
   if (ctx->has_override || (!ctx->plans.empty() && ks_plan_lookup(ctx, wdtype == KS_Q4K ? "mv_q4k" : "mv_q6k", rows, cols, n_tok))) return false;
   const double work = (double)rows * (double)cols * n_tok;
   const bool staged = (size_t)n_tok * (cols / 16) * 80 <= ctx->smem_optin;
-  if (wdtype == KS_Q4K ? work < (n_tok == 2 ? 14e6 : 6.5e6) : !ks_gemm_few_rows_q6k(ctx, rows, cols) ? staged : work < (n_tok == 2 ? 3e6 : 2e6))
+  if (wdtype == KS_Q4K ? work < (n_tok == 2 ? 14e6 : 6.5e6) : !ks_gemm_few_rows_q6k(ctx, rows, cols) || ((uintptr_t)W & 15) ? staged : work < (n_tok == 2 ? 3e6 : 2e6))
     return false;
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   return cudaStreamIsCapturing(ctx->stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone &&
@@ -522,7 +522,7 @@ int ks_matvec(ks_ctx* ctx, size_t rows, size_t cols, ks_dtype wdtype, const ks_b
   KS_REQUIRE(ctx, ks_fits(x, x_off * ab, (size_t)n_tok * cols * ab), "matvec: x buffer too small");
   KS_REQUIRE(ctx, ks_fits(y, y_off * ab, (size_t)n_tok * rows * ab), "matvec: y buffer too small");
   const void* xp = (const char*)x->dptr + x_off * ab;
-  if (n_tok > 8 || few_rows_gemm(ctx, wdtype, rows, cols, act, xp, n_tok)) {  // the reference's mul_mm route (lib.rs:1414): a tensor-core GEMM over all rows at once
+  if (n_tok > 8 || few_rows_gemm(ctx, wdtype, rows, cols, (const uint8_t*)W->dptr + w_byte_off, act, xp, n_tok)) {  // the reference's mul_mm route (lib.rs:1414): a tensor-core GEMM over all rows at once
     KS_REQUIRE(ctx, n_tok <= 8 || (act == KS_F32 && x_off % 4 == 0 && ((uintptr_t)xp & 15) == 0),
                "matvec: batches of more than 8 rows need f32 activations, x_off %% 4 == 0 and an x that starts on 16 bytes");
     void* scratch = nullptr;
