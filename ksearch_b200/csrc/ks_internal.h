@@ -178,8 +178,8 @@ struct ks_cand_cut {
 // Logit rows [n_slots][n] -> head[n_slots], list[n_slots][KS_CAND_MAX] (in no order).
 int ks_launch_candidates(ks_ctx* ctx, ks_dtype act, const void* logits, size_t n, int n_slots, float cap, const ks_cand_cut& cuts, ks_cand_head* head,
                          ks_cand* list);
-// The draw over candidates in index order; the others' probabilities fall under the min-p threshold.
-uint32_t ks_sample_candidates(const ks_cand* c, size_t n, float cap, float temperature, float min_p, uint32_t seed);
+// The draw over the n candidates of a row of n_all in index order; the others' probabilities fall under the min-p threshold.
+uint32_t ks_sample_candidates(const ks_cand* c, size_t n, size_t n_all, float cap, float temperature, float min_p, uint32_t seed);
 
 // ---- tensor-core GEMM for batches of more than 8 token rows (ks_gemm.cu) ---------------------------
 // nelem (a multiple of 256) elements of src (Q6K, Q4K, F16, F32) -> Q4_K blocks, as the reference's load-time quantizer.

@@ -1348,7 +1348,7 @@ int ks_model_sample_step(ks_model* m, int first, int n, const int* tokens, const
     if (listed[s] && !hh[s].odd && count >= 1 && count <= KS_CAND_MAX) {
       if (count > FEW) KS_CUDA(c, cudaMemcpy(l, dlist + (size_t)s * KS_CAND_MAX, count * sizeof(ks_cand), cudaMemcpyDeviceToHost));
       std::sort(l, l + count, [](const ks_cand& a, const ks_cand& b) { return a.index < b.index; });
-      next[s] = (int)ks_sample_candidates(l, count, g.softcap, temperature[s], min_p[s], seed[s]);
+      next[s] = (int)ks_sample_candidates(l, count, V, g.softcap, temperature[s], min_p[s], seed[s]);
       continue;
     }
     std::vector<unsigned char> row(V * ab);

@@ -89,7 +89,7 @@ uint32_t sample_impl(size_t n, Get get, float cap, float temperature, float min_
 // sample.rs:9-81 over the tokens that can survive its min-p filter (a superset, in index order).  A dropped token adds to
 // nothing but the softmax's normaliser, which scales the probabilities, their threshold and the drawn number alike, so it is
 // left out on both sides.
-uint32_t ks_sample_candidates(const ks_cand* c, size_t n, float cap, float temperature, float min_p, uint32_t seed) {
+uint32_t ks_sample_candidates(const ks_cand* c, size_t n, size_t n_all, float cap, float temperature, float min_p, uint32_t seed) {
   size_t best = 0;
   float best_v = -INFINITY;
   std::vector<float> xs(n);
@@ -109,16 +109,15 @@ uint32_t ks_sample_candidates(const ks_cand* c, size_t n, float cap, float tempe
     if (x < threshold) x = 0.0f;
     else filtered += x;
   }
+  if (filtered <= 0.0f) return c[best].index;
   uint32_t rng = seed | 1u;
   const float r = ((float)splitmix32(&rng) / 4294967296.0f) * filtered;
   float cdf = 0.0f;
-  size_t last = best;
   for (size_t i = 0; i < n; i++) {
     cdf += xs[i];
-    if (xs[i] > 0.0f) last = i;
     if (r < cdf) return c[i].index;
   }
-  return c[last].index;
+  return (uint32_t)(n_all - 1);  // a draw that rounds to 1 passes every token: the row's last one, as over the whole row
 }
 
 extern "C" {

@@ -63,3 +63,16 @@ def test_sample_step_rewinds_after_a_wait_that_gave_up():
     assert again == tok and np.array_equal(after, logits)
     model.close()
     c.close()
+
+
+@pytest.mark.parametrize("min_p", [0.05, 0.9, 2.0, 0.0])
+def test_sample_step_with_a_draw_that_rounds_to_one(ctx, min_p):
+    """splitmix32 within 128 of 2^32 is 1.0 as a float: the CPU sampler then runs past every token and takes the row's last."""
+    cfg = ksm.tiny_config(max_seq=32)
+    model = ksm.GemmaCudaModel.synthetic(ctx, cfg, seed=35)
+    model.slot_alloc()
+    for seed in (1109269, 138204815, 280706243, 1109268):
+        got = model.sample_step([7], 0, [0.8], [min_p], [seed])
+        want = sample_softcap_min_p(model.read_debug(1, 0), cfg.softcap, 0.8, min_p, seed)
+        assert got == [want] and (min_p == 2.0 or want == cfg.vocab - 1)
+    model.close()
