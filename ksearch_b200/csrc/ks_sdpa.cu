@@ -692,12 +692,10 @@ int launch_part_g(ks_ctx* ctx, int G, dim3 grid, unsigned n_q, unsigned n_kv, fl
     case 1: return launch_part<1, DPL, T>(ctx, grid, n_q, n_kv, scale, q, K, V, slot_stride, meta, tmp, out, n_splits);
     case 2: return launch_part<2, DPL, T>(ctx, grid, n_q, n_kv, scale, q, K, V, slot_stride, meta, tmp, out, n_splits);
     case 4: return launch_part<4, DPL, T>(ctx, grid, n_q, n_kv, scale, q, K, V, slot_stride, meta, tmp, out, n_splits);
-    case 8:
-    case 16:  // four heads per block, G / 4 blocks per KV head
+    default:  // 8 and 16: four heads per block, G / 4 blocks per KV head
       grid.y *= (unsigned)(G / 4);
       return launch_part<4, DPL, T>(ctx, grid, n_q, n_kv, scale, q, K, V, slot_stride, meta, tmp, out, n_splits);
   }
-  return ks_fail(ctx, KS_ERR_UNSUPPORTED, "sdpa: n_q/n_kv = %d not supported (1, 2, 4, 8, 16)", G);
 }
 
 }  // namespace
@@ -706,6 +704,8 @@ int ks_launch_sdpa(ks_ctx* ctx, size_t n_slots, size_t n_q, size_t n_kv, size_t 
                    const void* q, const uint8_t* K, const uint8_t* V, size_t slot_stride_bytes, const float* meta,
                    float* tmp, void* out, int n_splits, bool records_only) {
   const int G = (int)(n_q / n_kv);
+  if (G != 1 && G != 2 && G != 4 && G != 8 && G != 16)  // one set of groups, whichever kernel the operands' alignment leads to
+    return ks_fail(ctx, KS_ERR_UNSUPPORTED, "sdpa: n_q/n_kv = %d not supported (1, 2, 4, 8, 16)", G);
   dim3 grid((unsigned)n_splits, (unsigned)n_kv, (unsigned)n_slots);
   int rc = 1;
   static const bool per_row = getenv("KSEARCH_SDPA_PER_ROW") != nullptr;  // keep the per-row kernel (comparison runs)

@@ -457,9 +457,10 @@ int ks_sdpa_chunk_splits(const ks_ctx* ctx, int n_tok, size_t n_q, size_t n_kv, 
 }
 
 bool ks_sdpa_merge_split_covers(size_t n_q, size_t hd) { return n_q * hd <= 8192 && n_q * hd % 256 == 0 && n_q <= 64; }
+// Groups of query heads: those of decode attention.
 bool ks_sdpa_chunk_covers(size_t n_q, size_t n_kv, size_t hd, const void* K, const void* V) {
   const size_t G = n_q / n_kv;
-  return (hd == 256 || hd == 128) && G <= CH_BM && CH_BM % G == 0 && ks_sdpa_merge_split_covers(n_q, hd) && (((uintptr_t)K | (uintptr_t)V) & 3u) == 0;
+  return (hd == 256 || hd == 128) && G <= 16 && CH_BM % G == 0 && ks_sdpa_merge_split_covers(n_q, hd) && (((uintptr_t)K | (uintptr_t)V) & 3u) == 0;
 }
 
 // Rows of one slot: q [n_tok, n_q hd] f32, meta [n_tok][4] = (tlen, start, -, -) with both ends growing along the rows

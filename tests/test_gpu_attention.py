@@ -4,7 +4,7 @@ as two f16 terms and K, V as exact integers with f32 scales, so the bound is tha
 import numpy as np
 import pytest
 
-from ksearch_b200 import F16, F32, Eng, synth
+from ksearch_b200 import F16, F32, Eng, KsError, Q40, _lib, synth
 from ksearch_b200 import model as ksm
 from tests.test_gpu_ops import _attn_case
 
@@ -46,3 +46,17 @@ def test_prompt_chunks_at_odd_sizes(ctx, oracle, hd, n_kv, window):
     assert np.abs(got - want).max() <= 1e-3 * np.abs(want).max()
     cpu.close()
     model.close()
+
+
+@pytest.mark.parametrize("n_q,n_kv", [(3, 1), (6, 1), (32, 1), (24, 2)])
+@pytest.mark.parametrize("byte_off", [0, 2])
+def test_head_groups_outside_the_set_are_refused(ctx, n_q, n_kv, byte_off):
+    """1, 2, 4, 8 or 16 query heads per KV head, wherever the cache starts."""
+    hd, max_t = 256, 64
+    row = n_kv * hd // 32 * 18
+    q, out, tmp = (ctx.buffer_empty_f32(n) for n in (n_q * hd, n_q * hd, 4))
+    K, V, meta = ctx.buffer_empty_f32(max_t * row // 4 + 4), ctx.buffer_empty_f32(max_t * row // 4 + 4), ctx.buffer_bytes(np.array([9, 0, 0, 0], np.float32))
+    before = ctx.launch_count()
+    with pytest.raises(KsError) as ei:
+        ctx.check(ctx.lib.ks_sdpa_decode(ctx.h, 1, n_q, n_kv, hd, max_t, Q40, 1.0, F32, q.h, K.h, V.h, byte_off, max_t * row, meta.h, tmp.h, out.h, 1))
+    assert ei.value.code == _lib.ERR_UNSUPPORTED and ctx.launch_count() == before
