@@ -380,9 +380,13 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
 __device__ __forceinline__ float half_at(const unsigned char* p) { return __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short*>(p))); }
 
-template <int HD, typename T>
+// CH: bytes per copy of a cached row: 16 (8 for rows of 72 bytes) where the cache is aligned for it, else 4.
+template <int HD, typename T, unsigned CH>
 __global__ void __launch_bounds__(kMmaWarps * 32, 2)
 sdpa_mma_kernel(unsigned n_q, unsigned n_kv, unsigned gb, float scale, const T* q, const uint8_t* K, const uint8_t* V, size_t slot_stride,
                 const float* meta, float* tmp, T* out, int n_splits) {
@@ -417,7 +421,7 @@ sdpa_mma_kernel(unsigned n_q, unsigned n_kv, unsigned gb, float scale, const T* 
   auto fetch = [&](unsigned i, unsigned stage) {  // this warp's i-th tile (an empty group past the end; rows past the split repeat its last)
     const unsigned tile = warp + i * kMmaWarps;
     if (tile < n_tiles) {
-      constexpr unsigned CH = HD == 256 ? 16u : 8u, PER = ROWB / CH;  // rows of 144 (72) bytes
+      constexpr unsigned PER = ROWB / CH;
       const unsigned first = p0 + tile * kMmaTile, last = p1 - 1u - first;
 #pragma unroll
       for (unsigned k = 0; k < (kMmaTile * PER + 31u) / 32u; k++) {
@@ -425,12 +429,15 @@ sdpa_mma_kernel(unsigned n_q, unsigned n_kv, unsigned gb, float scale, const T* 
         if (c >= kMmaTile * PER) break;
         const size_t src = (size_t)(first + min(r, last)) * rowstride + o;
         const uint32_t dst = ring_s + stage * S::TILE + r * ROWB + o;
-        if (CH == 16u) {
+        if constexpr (CH == 16u) {
           cp_async16(dst, Ks + src);
           cp_async16(dst + kMmaTile * ROWB, Vs + src);
-        } else {
+        } else if constexpr (CH == 8u) {
           cp_async8(dst, Ks + src);
           cp_async8(dst + kMmaTile * ROWB, Vs + src);
+        } else {
+          cp_async4(dst, Ks + src);
+          cp_async4(dst + kMmaTile * ROWB, Vs + src);
         }
       }
     }
@@ -653,13 +660,11 @@ sdpa_mma_kernel(unsigned n_q, unsigned n_kv, unsigned gb, float scale, const T* 
   }
 }
 
-// Returns 1 when the call is outside what the kernel takes.
-template <int HD, typename T>
+template <int HD, typename T, unsigned CH>
 int launch_mma(ks_ctx* ctx, unsigned hpk, dim3 grid, unsigned n_q, unsigned n_kv, float scale, const void* q, const uint8_t* K, const uint8_t* V,
                size_t slot_stride, const float* meta, float* tmp, void* out, int n_splits) {
   const unsigned gb = hpk % 4 == 0 ? 4u : hpk % 2 == 0 ? 2u : 1u;
-  if (((uintptr_t)K | (uintptr_t)V | (uintptr_t)slot_stride) & (HD == 256 ? 15u : 7u)) return 1;
-  auto kern = sdpa_mma_kernel<HD, T>;
+  auto kern = sdpa_mma_kernel<HD, T, CH>;
   constexpr size_t smem = MmaSmem<HD>::total;
   static bool set[16] = {false};
   if (!set[ctx->device & 15]) {
@@ -709,10 +714,14 @@ int ks_launch_sdpa(ks_ctx* ctx, size_t n_slots, size_t n_q, size_t n_kv, size_t 
   dim3 grid((unsigned)n_splits, (unsigned)n_kv, (unsigned)n_slots);
   int rc = 1;
   static const bool per_row = getenv("KSEARCH_SDPA_PER_ROW") != nullptr;  // keep the per-row kernel (comparison runs)
-  if (!per_row && (hd == 256 || hd == 128)) {
-#define KS_MMA(HD_, T_) launch_mma<HD_, T_>(ctx, (unsigned)G, grid, (unsigned)n_q, (unsigned)n_kv, scale, q, K, V, slot_stride_bytes, meta, tmp, out, n_splits)
-    if (hd == 256) rc = act == KS_F32 ? KS_MMA(256, float) : KS_MMA(256, __half);
-    else rc = act == KS_F32 ? KS_MMA(128, float) : KS_MMA(128, __half);
+  const uintptr_t at = (uintptr_t)K | (uintptr_t)V | (uintptr_t)slot_stride_bytes;
+  if (!per_row && (hd == 256 || hd == 128) && at % 4 == 0) {  // a cache that starts on 2 bytes is left to the per-row kernel
+    const bool wide = at % (hd == 256 ? 16 : 8) == 0;
+#define KS_MMA(HD_, T_, CH_) launch_mma<HD_, T_, CH_>(ctx, (unsigned)G, grid, (unsigned)n_q, (unsigned)n_kv, scale, q, K, V, slot_stride_bytes, meta, tmp, out, n_splits)
+#define KS_MMA_CH(HD_, CH_) (act == KS_F32 ? KS_MMA(HD_, float, CH_) : KS_MMA(HD_, __half, CH_))
+    if (hd == 256) rc = wide ? KS_MMA_CH(256, 16u) : KS_MMA_CH(256, 4u);
+    else rc = wide ? KS_MMA_CH(128, 8u) : KS_MMA_CH(128, 4u);
+#undef KS_MMA_CH
 #undef KS_MMA
   }
   if (rc != 1) {

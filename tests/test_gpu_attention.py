@@ -60,3 +60,36 @@ def test_head_groups_outside_the_set_are_refused(ctx, n_q, n_kv, byte_off):
     with pytest.raises(KsError) as ei:
         ctx.check(ctx.lib.ks_sdpa_decode(ctx.h, 1, n_q, n_kv, hd, max_t, Q40, 1.0, F32, q.h, K.h, V.h, byte_off, max_t * row, meta.h, tmp.h, out.h, 1))
     assert ei.value.code == _lib.ERR_UNSUPPORTED and ctx.launch_count() == before
+
+
+@pytest.mark.parametrize("act", [F32, F16])
+@pytest.mark.parametrize("hd,byte_off,pad", [(256, 4, 0), (256, 8, 0), (256, 0, 4), (128, 4, 0), (128, 0, 12), (256, 2, 0), (128, 0, 6)])
+def test_caches_off_16_bytes(ctx, oracle, act, hd, byte_off, pad):
+    """Caches that start, or follow one another, on 2, 4 or 8 bytes: the same answers as at 16, bit for bit on multiples of 4,
+    where the same kernel takes them."""
+    n_q, n_kv, max_t, scale, tlens, starts = 8, 2, 320, hd ** -0.5, [5, 280, 129], [2, 0, 40]
+    npdt, n = np.float32 if act == F32 else np.float16, len(tlens)
+    slot = max_t * n_kv * hd // 32 * 18
+    K, V = (np.frombuffer(synth.q40_rows(53, k, n * max_t * n_kv * hd, sigma=0.05), np.uint8).reshape(n, slot) for k in "KV")
+    q = synth.normals(53, "q", n * n_q * hd).astype(npdt)
+    bq, meta = ctx.buffer_bytes(q), ctx.buffer_bytes(np.array([[t, s, 0, 0] for t, s in zip(tlens, starts)], np.float32))
+    e = Eng(act)
+
+    def run(off, gap, ns):
+        def place(x):
+            out = np.zeros(off + n * (slot + gap), np.uint8)
+            out[off:].reshape(n, slot + gap)[:, :slot] = x
+            return ctx.buffer_bytes(out)
+        bK, bV, out = place(K), place(V), ctx.buffer_empty_bytes(q.nbytes)
+        tmp = ctx.buffer_empty_f32(max(1, e.sdpa_tmp_floats(n_q, hd, ns, n)))
+        ctx.check(ctx.lib.ks_sdpa_decode(ctx.h, n, n_q, n_kv, hd, max_t, Q40, scale, act, bq.h, bK.h, bV.h, off, slot + gap, meta.h, tmp.h, out.h, ns))
+        return ctx.read_act(out, q.size, act).reshape(n, -1).astype(np.float64)
+
+    for ns in (1, 3):
+        got, plain = run(byte_off, pad, ns), run(0, 0, ns)
+        if (byte_off | pad) % 4 == 0:
+            assert np.array_equal(got, plain)
+        for s in range(n):
+            want = oracle.sdpa_decode(n_q, n_kv, hd, q.astype(np.float32).reshape(n, -1)[s], K[s], V[s], tlens[s], starts[s], scale, 0)
+            rtol, atol = (1e-3, 1e-4) if act == F32 else (3e-3, 1e-3)
+            assert (np.abs(got[s] - want) <= atol + rtol * np.abs(want)).all()
