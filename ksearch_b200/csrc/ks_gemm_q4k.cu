@@ -105,7 +105,7 @@ __device__ __forceinline__ void q4_header(const uint4 h, unsigned g, Q4Hdr& o) {
   const float ad = fabsf(d), am = fabsf(dm);
   __half2 s0 = small_int_h2(sc0), s1 = small_int_h2(sc1);
   float s = d, mu = ad > 0.0f ? __fdividef(32.0f * dm, d) : 0.0f;
-  if (am > 32.0f * ad) {
+  if (am > 32.0f * ad && (h.z | (h.w & 0xF0F0F0F0u)) != 0u) {  // (a block without minima has nothing to make room for, whatever its dmin)
     // j: the smallest power of two with dmin <= 32 d 2^j; beyond 2^20 (or d = 0) the d part is below the last bit of the minima
     float p = 0.0f;
     if (am <= 32.0f * 1048576.0f * ad) {

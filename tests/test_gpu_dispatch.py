@@ -158,3 +158,21 @@ def test_few_rows_are_as_exact_as_the_matvec(ctx, oracle, dtype, rows, cols, bat
     want = x.astype(np.float64) @ oracle.dequant(dtype, W, rows * cols).astype(np.float64).reshape(rows, cols).T
     err = np.linalg.norm(got - want, axis=1) / np.linalg.norm(want, axis=1)
     assert err.max() <= (3.5e-7 if (dtype, cols, batch) != (Q6K, 10240, 8) else 1e-5), err   # there the tcgen05 kernel: f32 sums over all columns
+
+
+@pytest.mark.parametrize("batch", [5, 24, 100])
+def test_a_large_dmin_without_minima_changes_nothing(ctx, oracle, batch):
+    """Super-blocks whose minima are all 0 with dmin 2^26 times d: the weights are d sc q, as with dmin = 0."""
+    rows, cols = 130, 512
+    W = np.frombuffer(_gen(Q4K, 77, "W", rows, cols), np.uint8).reshape(rows, cols // 256, 144).copy()
+    sc = np.random.default_rng(77).integers(0, 64, (rows, cols // 256, 8), np.uint8)
+    W[:, :, 4:8], W[:, :, 8:12] = (sc[:, :, :4] & 63) | ((sc[:, :, 4:] >> 4) << 6), 0
+    W[:, :, 12:16] = sc[:, :, 4:] & 15
+    W[0::2, :, 0:4] = np.frombuffer(np.array([2.0 ** -20, 64.0], np.float16).tobytes(), np.uint8)
+    W[1::2, :, 0:4] = np.frombuffer(np.array([2.0 ** -20, 2.0 ** -3], np.float16).tobytes(), np.uint8)
+    x = synth.normals(77, f"x{batch}", batch * cols).reshape(batch, cols).astype(np.float32)
+    raw = W.tobytes()
+    bw, bx, y = ctx.buffer_bytes(np.frombuffer(raw, np.uint8)), ctx.buffer_bytes(x), ctx.buffer_empty_f32(batch * rows)
+    ctx.check(ctx.lib.ks_matvec(ctx.h, rows, cols, Q4K, bw.h, 0, 0, bx.h, 0, y.h, 0, batch))
+    y32, y64 = oracle.matvec(Q4K, np.frombuffer(raw, np.uint8), rows, cols, x)
+    _check(ctx.read_f32(y, batch * rows).reshape(batch, rows) * 2.0 ** 20, y32 * np.float32(2.0 ** 20), y64 * 2.0 ** 20, f"{batch} rows")
