@@ -444,8 +444,8 @@ struct EpiNormArgs {
   const float* P;
   size_t part_stride;
   ks_gemm_map map;
-  unsigned n_tok, np, rows;
-  int q4k;      // form of the image written
+  unsigned n_tok, np, tbn, rows;  // np, tbn: blocks of the image written
+  int q4k;      // its form
   const float *res, *w_post, *w_norm;
   float eps;
   float* out_x;
@@ -502,7 +502,7 @@ __global__ void gemm_finish_norm_split_kernel(const EpiNormArgs e) {
   if (ck < chunks) {
 #pragma unroll
     for (int i = 0; i < 8; i++) xn[i] *= down;
-    put_split8(e.xt, e.np, q4k_block(e.np), t, ck, chunks, xn, e.q4k != 0);
+    put_split8(e.xt, e.np, e.tbn, t, ck, chunks, xn, e.q4k != 0);
   }
 }
 
@@ -514,8 +514,8 @@ constexpr unsigned GM_GELU_CL = 4, GM_GELU_THREADS = 512;
 // The longest rows the two epilogues take: eight values per thread of one block, and of a cluster.
 constexpr size_t GM_NORM_MOST = 8 * 1024, GM_GELU_MOST = 8 * GM_GELU_CL * GM_GELU_THREADS;
 __global__ void __cluster_dims__(GM_GELU_CL, 1, 1) __launch_bounds__(GM_GELU_THREADS)
-    gemm_finish_gelu_split_kernel(const float* P0, const float* P1, size_t part_stride, ks_gemm_map map, unsigned n_tok, unsigned np, unsigned rows,
-                                  __half* xt) {
+    gemm_finish_gelu_split_kernel(const float* P0, const float* P1, size_t part_stride, ks_gemm_map map, unsigned n_tok, unsigned np, unsigned tbn,
+                                  unsigned rows, __half* xt) {
   ks_pdl_entry();
   __shared__ float red[32], maxima[GM_GELU_CL];
   namespace cg = cooperative_groups;
@@ -546,7 +546,7 @@ __global__ void __cluster_dims__(GM_GELU_CL, 1, 1) __launch_bounds__(GM_GELU_THR
   if (ck < chunks) {
 #pragma unroll
     for (int k = 0; k < 8; k++) v[k] *= down;
-    put_split8(xt, np, q4k_block(np), t, ck, chunks, v, true);  // a down-projection is always Q4_K
+    put_split8(xt, np, tbn, t, ck, chunks, v, true);  // a down-projection is always Q4_K
   }
 }
 
@@ -701,10 +701,7 @@ unsigned gemm_splits(const ks_ctx* ctx, size_t rows, size_t cols, int n_tok) {
   }
   return best;
 }
-// Token rows per block of the image, and all of them padded to whole blocks.
-struct Blocks {
-  unsigned tbn, np;
-};
+typedef ks_gemm_blocks Blocks;
 Blocks gemm_blocks(int n_tok) { return {q4k_block(gemm_np(n_tok)), gemm_np(n_tok)}; }
 Blocks gemm_small_blocks(int n_tok) {
   const unsigned tb = ((unsigned)n_tok + 63u) / 64u, tbn = (((unsigned)n_tok + tb - 1) / tb + 15u) / 16u * 16u;
@@ -724,25 +721,26 @@ ks_gemm_map gemm_map(const ks_ctx* ctx, ks_dtype wdtype, const size_t* rows, int
   m.splits = (ksteps + per - 1) / per;
   return m;
 }
-// One Q4_K matrix against more than 64 token rows: pairs of row tiles against blocks of up to 128 read the token rows half as
-// often; where that leaves few units for the SMs, single tiles against blocks of up to 64 are four times as many.  By the
-// estimate both maps are chosen by.
-Blocks gemm_pick_blocks(const ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_t cols, int n_tok) {
-  const Blocks wide = gemm_blocks(n_tok);
-  if (wdtype != KS_Q4K || wide.tbn <= 64u) return wide;
-  const Blocks small = gemm_small_blocks(n_tok);
-  double cw, cs;
-  ks_gemm_q4k_map(ctx, &rows, 1, (unsigned)cols, wide.np, wide.tbn, true, &cw);
-  ks_gemm_q4k_map(ctx, &rows, 1, (unsigned)cols, small.np, small.tbn, true, &cs);
-  return cs < cw ? small : wide;
-}
 bool gemm_covers(ks_dtype wdtype, size_t cols, int n_tok) {
   return (wdtype == KS_Q4K || wdtype == KS_Q6K) && cols % 256 == 0 && n_tok >= 1 && n_tok <= 256;
 }
 }  // namespace
 
 bool ks_gemm_few_rows_q6k(const ks_ctx* ctx, size_t rows, size_t cols) { return ks_gemm_q6k_skinny_covers(ctx, rows, (unsigned)cols); }
-unsigned ks_gemm_np(int n_tok) { return gemm_np(n_tok); }
+// Q4_K matrices against more than 64 token rows: pairs of row tiles against blocks of up to 128 read the token rows half as
+// often; where that leaves few units for the SMs, single tiles against blocks of up to 64 are four times as many.  By the
+// estimate both maps are chosen by; with an epilogue behind it (sums always read once more) only where it promises a tenth: a
+// whole E2B layer of 256 rows took 142 us with wide blocks and 145 with the four small ones the bare estimate picks; of 128
+// rows 117 with wide blocks, 105 with small ones, of the tiny shape 87 and 60.
+ks_gemm_blocks ks_gemm_pick(const ks_ctx* ctx, ks_dtype wdtype, int n_seg, const size_t* rows, size_t cols, int n_tok, bool plain) {
+  const Blocks wide = gemm_blocks(n_tok);
+  if (wdtype != KS_Q4K || wide.tbn <= 64u) return wide;
+  const Blocks small = gemm_small_blocks(n_tok);
+  double cw, cs;
+  ks_gemm_q4k_map(ctx, rows, n_seg, (unsigned)cols, wide.np, wide.tbn, plain, &cw);
+  ks_gemm_q4k_map(ctx, rows, n_seg, (unsigned)cols, small.np, small.tbn, plain, &cs);
+  return cs < (plain ? cw : 0.9 * cw) ? small : wide;
+}
 bool ks_gemm_layers_cover(size_t hidden, size_t ffn, size_t q_cols) {
   return hidden % 256 == 0 && ffn % 256 == 0 && q_cols % 256 == 0 && hidden <= GM_NORM_MOST && ffn <= GM_GELU_MOST;
 }
@@ -754,21 +752,18 @@ size_t ks_gemm_xt_bytes(size_t cols, int n_tok) {  // image + one factor per row
 }
 
 // x[t * ldx + k] (f32) -> the B image in xt.
-static int launch_split(ks_ctx* ctx, ks_dtype wdtype, const float* x, size_t ldx, int n_tok, size_t cols, void* xt, Blocks b) {
+int ks_launch_gemm_split(ks_ctx* ctx, ks_dtype wdtype, const float* x, size_t ldx, int n_tok, size_t cols, void* xt, ks_gemm_blocks b) {
   if (cols % 256 || n_tok < 1 || n_tok > 256 || ldx % 4) return ks_fail(ctx, KS_ERR_INVALID, "gemm: bad operand shape");
   KS_LAUNCH(ctx, (x_split_kernel), b.np, GM_ROW_THREADS, 0, x, ldx, (unsigned)n_tok, b.np, b.tbn, (unsigned)cols, (__half*)xt, (int)(wdtype == KS_Q4K));
   return ks_after_launch(ctx, "x_split");
-}
-int ks_launch_gemm_split(ks_ctx* ctx, ks_dtype wdtype, const float* x, size_t ldx, int n_tok, size_t cols, void* xt) {
-  return launch_split(ctx, wdtype, x, ldx, n_tok, cols, xt, gemm_blocks(n_tok));
 }
 
 // Up to three matrices over the same columns in one launch.  With one k split matrix i's result goes straight to
 // y[i] (row stride ldy[i]); otherwise the partials go to P (dense [split][token][row] per matrix, matrix after
 // matrix) and a second launch sums them in split order into y.  mode 1 (two matrices, gate and up): y[0] =
-// gelu(gate) * up, always through P.  `xt` is the image ks_launch_gemm_split made of the same token rows.
-static int launch_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* const* W, const size_t* rows, size_t cols, const void* xt,
-                       int n_tok, float* const* y, const size_t* ldy, float* P, int mode, const ks_gemm_epi* epi, Blocks blocks) {
+// gelu(gate) * up, always through P.  `xt` is the image of the token rows in these blocks.
+int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* const* W, const size_t* rows, size_t cols, const void* xt,
+                        int n_tok, float* const* y, const size_t* ldy, float* P, int mode, const ks_gemm_epi* epi, ks_gemm_blocks blocks) {
   if (!gemm_covers(wdtype, cols, n_tok) || n_seg < 1 || n_seg > 3) return ks_fail(ctx, KS_ERR_UNSUPPORTED, "gemm: shape not covered");
   if ((mode == KS_GEMM_NORM_SPLIT && (n_seg != 1 || !epi || rows[0] % 8 || rows[0] > GM_NORM_MOST)) ||
       (mode == KS_GEMM_QKV && (n_seg != 3 || !epi || (epi->hd != 128 && epi->hd != 256) || rows[0] != (size_t)epi->n_q * epi->hd ||
@@ -881,7 +876,8 @@ static int launch_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* c
     e.part_stride = part_stride[0];
     e.map = map;
     e.n_tok = (unsigned)n_tok;
-    e.np = np;
+    e.np = epi->next.np;
+    e.tbn = epi->next.tbn;
     e.q4k = epi->next_dtype == KS_Q4K;
     e.rows = (unsigned)rows[0];
     e.res = epi->res;
@@ -890,7 +886,7 @@ static int launch_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* c
     e.eps = epi->eps;
     e.out_x = epi->out_x;
     e.xt = (__half*)epi->xt_out;
-    KS_LAUNCH(ctx, (gemm_finish_norm_split_kernel), np, (unsigned)((rows[0] / 8 + 31) / 32 * 32), 0, e);
+    KS_LAUNCH(ctx, (gemm_finish_norm_split_kernel), e.np, (unsigned)((rows[0] / 8 + 31) / 32 * 32), 0, e);
     return ks_after_launch(ctx, "gemm_finish_norm_split");
   }
   if (mode == KS_GEMM_QKV) {
@@ -922,8 +918,8 @@ static int launch_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* c
   if (mode == KS_GEMM_GELU_SPLIT) {
     // whole warps per block: a 32-value sub-block of the image is four neighbouring lanes of one
     const unsigned threads = ((unsigned)rows[0] / 8u / GM_GELU_CL + 31u) / 32u * 32u;
-    KS_LAUNCH(ctx, (gemm_finish_gelu_split_kernel), np * GM_GELU_CL, threads, 0, (const float*)out[0], (const float*)out[1], part_stride[0], map,
-              (unsigned)n_tok, np, (unsigned)rows[0], (__half*)epi->xt_out);
+    KS_LAUNCH(ctx, (gemm_finish_gelu_split_kernel), epi->next.np * GM_GELU_CL, threads, 0, (const float*)out[0], (const float*)out[1], part_stride[0], map,
+              (unsigned)n_tok, epi->next.np, epi->next.tbn, (unsigned)rows[0], (__half*)epi->xt_out);
     return ks_after_launch(ctx, "gemm_finish_gelu_split");
   }
   f.n_seg = (unsigned)n_seg;
@@ -947,11 +943,6 @@ static int launch_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* c
   return ks_after_launch(ctx, "gemm_finish");
 }
 
-int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* const* W, const size_t* rows, size_t cols, const void* xt,
-                        int n_tok, float* const* y, const size_t* ldy, float* P, int mode, const ks_gemm_epi* epi) {
-  return launch_segs(ctx, wdtype, n_seg, W, rows, cols, xt, n_tok, y, ldy, P, mode, epi, gemm_blocks(n_tok));
-}
-
 // Floats of partials ks_launch_gemm_segs may write for up to three matrices of `total_rows` rows in all (either dtype).
 size_t ks_gemm_part_floats(const ks_ctx* ctx, size_t total_rows, size_t cols, int n_tok) {
   unsigned slots = gemm_map(ctx, KS_Q6K, &total_rows, 1, cols, n_tok, gemm_blocks(n_tok), true).splits;
@@ -959,10 +950,11 @@ size_t ks_gemm_part_floats(const ks_ctx* ctx, size_t total_rows, size_t cols, in
     const unsigned n = ks_gemm_skinny_splits(ctx, total_rows, (unsigned)cols);
     slots = n > slots ? n : slots;
   }
-  const Blocks b = gemm_blocks(n_tok);
-  for (int extra = 0; extra < 6; extra++) {  // the matrices of a launch round their tiles up one by one; with and without an epilogue
-    const size_t r = total_rows + (size_t)(extra % 3) * 2 * GM_ROWS;
-    const ks_gemm_map m = ks_gemm_q4k_map(ctx, &r, 1, (unsigned)cols, b.np, b.tbn, extra >= 3);
+  const Blocks both[2] = {gemm_blocks(n_tok), n_tok > 64 ? gemm_small_blocks(n_tok) : gemm_blocks(n_tok)};
+  for (int extra = 0; extra < 20; extra++) {  // the matrices of a launch round their tiles up one by one; with and without an epilogue
+    const Blocks b = both[extra / 10];
+    const size_t r = total_rows + (size_t)(extra % 5) * GM_ROWS;
+    const ks_gemm_map m = ks_gemm_q4k_map(ctx, &r, 1, (unsigned)cols, b.np, b.tbn, extra % 10 >= 5);
     const unsigned n = (m.S + m.base - 1) / m.base + 1;  // a CTA has at least `base` units, a work tile may begin inside one
     slots = n > slots ? n : slots;
   }
@@ -971,7 +963,7 @@ size_t ks_gemm_part_floats(const ks_ctx* ctx, size_t total_rows, size_t cols, in
 
 // Scratch of ks_launch_gemm_kq: the image and the partials of that one launch.
 size_t ks_gemm_kq_bytes(const ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_t cols, int n_tok) {
-  const ks_gemm_map m = gemm_map(ctx, wdtype, &rows, 1, cols, n_tok, gemm_pick_blocks(ctx, wdtype, rows, cols, n_tok), true);
+  const ks_gemm_map m = gemm_map(ctx, wdtype, &rows, 1, cols, n_tok, ks_gemm_pick(ctx, wdtype, 1, &rows, cols, n_tok, true), true);
   const size_t slots = m.G ? (m.S + m.base - 1) / m.base + 1 : m.splits;
   return ks_gemm_xt_bytes(cols, n_tok) + 4 * slots * n_tok * rows;
 }
@@ -981,9 +973,9 @@ size_t ks_gemm_kq_bytes(const ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_t 
 int ks_launch_gemm_kq(ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_t cols, const uint8_t* W, const float* x, size_t ldx, float* y,
                       size_t ldy, int n_tok, void* scratch) {
   if (!gemm_covers(wdtype, cols, n_tok) || ldx % 4) return 1;
-  const Blocks b = gemm_pick_blocks(ctx, wdtype, rows, cols, n_tok);
-  int rc = launch_split(ctx, wdtype, x, ldx, n_tok, cols, scratch, b);
+  const Blocks b = ks_gemm_pick(ctx, wdtype, 1, &rows, cols, n_tok, true);
+  int rc = ks_launch_gemm_split(ctx, wdtype, x, ldx, n_tok, cols, scratch, b);
   if (rc) return rc;
   float* P = (float*)((char*)scratch + ks_gemm_xt_bytes(cols, n_tok));
-  return launch_segs(ctx, wdtype, 1, &W, &rows, cols, scratch, n_tok, &y, &ldy, P, KS_GEMM_PLAIN, nullptr, b);
+  return ks_launch_gemm_segs(ctx, wdtype, 1, &W, &rows, cols, scratch, n_tok, &y, &ldy, P, KS_GEMM_PLAIN, nullptr, b);
 }

@@ -154,9 +154,12 @@ bool ks_sdpa_merge_split_covers(size_t n_q, size_t hd);
 bool ks_sdpa_chunk_covers(size_t n_q, size_t n_kv, size_t hd, const void* K, const void* V);
 int ks_launch_sdpa_chunk(ks_ctx* ctx, int n_tok, size_t n_q, size_t n_kv, size_t hd, float scale, const float* q, const uint8_t* K,
                          const uint8_t* V, const float* meta, float* tmp, int n_splits);
-int ks_launch_sdpa_merge_split(ks_ctx* ctx, int n_tok, unsigned np, size_t n_q, size_t hd, const float* tmp, int n_splits, void* xt);
+// Token rows per block of an operand image and all of them padded to whole blocks: a choice of the GEMM that reads the image.
+struct ks_gemm_blocks {
+  unsigned tbn, np;
+};
+int ks_launch_sdpa_merge_split(ks_ctx* ctx, int n_tok, ks_gemm_blocks b, size_t n_q, size_t hd, const float* tmp, int n_splits, void* xt);
 bool ks_gemm_few_rows_q6k(const ks_ctx* ctx, size_t rows, size_t cols);  // ks_gemm_skinny.cu has a kernel for up to 8 token rows
-unsigned ks_gemm_np(int n_tok);  // token rows of an operand image: n_tok padded
 int ks_launch_copy_scale_indexed(ks_ctx* ctx, size_t n, size_t batch, float scale, ks_dtype src_dtype,
                                  const void* src, const float* idx, ks_dtype act, void* dst);
 int ks_launch_softcap_argmax(ks_ctx* ctx, size_t n, float cap, ks_dtype act, const void* logits, float* out_idx);
@@ -190,8 +193,10 @@ size_t ks_gemm_part_floats(const ks_ctx* ctx, size_t total_rows, size_t cols, in
 // grow it: KS_FEW_WS holds their image (4.7 MB at 65536 columns) and partials (8 rows of 262144 outputs: 8 MB a share).
 constexpr size_t KS_FEW_WS = 32u << 20;
 int ks_ctx_gemm_scratch(ks_ctx* ctx, size_t bytes, void** out);
+// The blocks a launch over these matrices wants (`plain`: nothing is done to its sums).
+ks_gemm_blocks ks_gemm_pick(const ks_ctx* ctx, ks_dtype wdtype, int n_seg, const size_t* rows, size_t cols, int n_tok, bool plain);
 // x[t * ldx + k] (f32) -> the image the GEMM over weights of that dtype reads its token rows from.
-int ks_launch_gemm_split(ks_ctx* ctx, ks_dtype wdtype, const float* x, size_t ldx, int n_tok, size_t cols, void* xt);
+int ks_launch_gemm_split(ks_ctx* ctx, ks_dtype wdtype, const float* x, size_t ldx, int n_tok, size_t cols, void* xt, ks_gemm_blocks b);
 // Up to three matrices over the same columns and token rows (q, k, v; gate, up) in one launch.  What becomes of
 // the sums: PLAIN y[i] = W[i] x; GELU (two matrices) y[0] = gelu(W[0] x) * (W[1] x); NORM_SPLIT (one matrix)
 // out_x = res + rms(W x) * w_post and the image of rms(out_x) * w_norm for the next GEMM in xt_out; GELU_SPLIT
@@ -204,6 +209,7 @@ struct ks_gemm_epi {
   float* out_x;                        // NORM_SPLIT: the updated residual rows
   void* xt_out;                        // the image written for the next GEMM (may be the image this GEMM read)
   ks_dtype next_dtype;                 // NORM_SPLIT: weights of that next GEMM
+  ks_gemm_blocks next;                 // *_SPLIT: its blocks
   unsigned n_q, n_kv, hd;              // QKV: heads; row t's cache entry: position pos[t] of the cache at t * slot_stride
   const float *qw, *kw, *rope;
   const int* pos;
@@ -211,7 +217,7 @@ struct ks_gemm_epi {
   size_t slot_stride;
 };
 int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* const* W, const size_t* rows, size_t cols, const void* xt,
-                        int n_tok, float* const* y, const size_t* ldy, float* P, int mode, const ks_gemm_epi* epi);
+                        int n_tok, float* const* y, const size_t* ldy, float* P, int mode, const ks_gemm_epi* epi, ks_gemm_blocks b);
 // Do the epilogues take every matrix of a layer of these widths?
 bool ks_gemm_layers_cover(size_t hidden, size_t ffn, size_t q_cols);
 // Split + GEMM for one matrix.  Returns 1 when the shape is not covered (cols not a multiple of 256, more than

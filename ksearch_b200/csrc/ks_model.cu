@@ -360,7 +360,12 @@ int enqueue_forward_gemm(ks_model* m, const Lane& L_, int n, bool want_logits) {
   if ((rc = lane_begin(m, L_, n))) return rc;
   if ((rc = ks_launch_copy_scale_indexed(c, H, n, sqrtf((float)H), (ks_dtype)g.embd_dtype, m->token_embd.dptr, L_.tok_in, act, x))) return rc;
   if ((rc = ks_launch_rmsnorm(c, H, n, g.eps, act, x, m->layers[0].attn32, nullptr, 0, 0.f, x2))) return rc;
-  if ((rc = ks_launch_gemm_split(c, KS_Q4K, (const float*)x2, H, n, H, m->gemm_xt))) return rc;
+  // every image is written in the blocks the GEMM that reads it wants
+  const size_t qkv_rows[3] = {qn, kvn, kvn}, gu_rows[2] = {F, F}, V = (size_t)g.vocab;
+  const ks_gemm_blocks b_qkv = ks_gemm_pick(c, KS_Q4K, 3, qkv_rows, H, n, false), b_o = ks_gemm_pick(c, KS_Q4K, 1, &H, qn, n, false),
+                       b_gu = ks_gemm_pick(c, KS_Q4K, 2, gu_rows, H, n, false), b_down = ks_gemm_pick(c, KS_Q4K, 1, &H, F, n, false),
+                       b_head = ks_gemm_pick(c, (ks_dtype)g.embd_dtype, 1, &V, H, n, true);
+  if ((rc = ks_launch_gemm_split(c, KS_Q4K, (const float*)x2, H, n, H, m->gemm_xt, b_qkv))) return rc;
   // From here on the normed rows exist only as the image the next GEMM reads: the sums of the o-proj and
   // down-proj partials go straight through the residual update and the next norm into that image.
   ks_gemm_epi epi{};
@@ -375,7 +380,6 @@ int enqueue_forward_gemm(ks_model* m, const Lane& L_, int n, bool want_logits) {
     {  // q, k and v rows in one launch (lib.rs:227); their sums go through the per-head norms, RoPE and the pack (lib.rs:1257)
       const uint8_t* Ws[3] = {(const uint8_t*)L.wq.dptr, (const uint8_t*)L.wk.dptr, (const uint8_t*)L.wv.dptr};
       float* ys[3] = {nullptr, nullptr, nullptr};
-      const size_t rs[3] = {qn, kvn, kvn};
       ks_gemm_epi head{};
       head.eps = g.eps;
       head.out_x = (float*)q;
@@ -389,42 +393,44 @@ int enqueue_forward_gemm(ks_model* m, const Lane& L_, int n, bool want_logits) {
       head.kv_k = kk;
       head.kv_v = kv;
       head.slot_stride = L_.kv_stride;
-      if ((rc = ks_launch_gemm_segs(c, KS_Q4K, 3, Ws, rs, H, m->gemm_xt, n, ys, rs, m->gemm_p0, KS_GEMM_QKV, &head))) return rc;
+      if ((rc = ks_launch_gemm_segs(c, KS_Q4K, 3, Ws, qkv_rows, H, m->gemm_xt, n, ys, qkv_rows, m->gemm_p0, KS_GEMM_QKV, &head, b_qkv))) return rc;
     }
     if (L_.chunk_base && n >= KS_CHUNK_ATT_MIN && ks_sdpa_chunk_covers(nq, nkv, hd, kk, kv)) {  // the rows of a chunk share their context
       if ((rc = ks_launch_sdpa_chunk(c, n, nq, nkv, hd, g.attn_scale, (const float*)q, kk, kv, layer_meta(m, L_, l), L_.attn_tmp, chunk_splits)) ||
-          (rc = ks_launch_sdpa_merge_split(c, n, ks_gemm_np(n), nq, hd, L_.attn_tmp, chunk_splits, m->gemm_xt)))
+          (rc = ks_launch_sdpa_merge_split(c, n, b_o, nq, hd, L_.attn_tmp, chunk_splits, m->gemm_xt)))
         return rc;
     } else if (att_splits > 1 && ks_sdpa_merge_split_covers(nq, hd)) {
       if ((rc = ks_launch_sdpa(c, n, nq, nkv, hd, g.attn_scale, act, q, kk, kv, L_.kv_stride, layer_meta(m, L_, l), L_.attn_tmp, o, att_splits, true)) ||
-          (rc = ks_launch_sdpa_merge_split(c, n, ks_gemm_np(n), nq, hd, L_.attn_tmp, att_splits, m->gemm_xt)))
+          (rc = ks_launch_sdpa_merge_split(c, n, b_o, nq, hd, L_.attn_tmp, att_splits, m->gemm_xt)))
         return rc;
     } else {
       if ((rc = ks_launch_sdpa(c, n, nq, nkv, hd, g.attn_scale, act, q, kk, kv, L_.kv_stride, layer_meta(m, L_, l), L_.attn_tmp, o, att_splits)))
         return rc;
-      if ((rc = ks_launch_gemm_split(c, KS_Q4K, (const float*)o, qn, n, qn, m->gemm_xt))) return rc;
+      if ((rc = ks_launch_gemm_split(c, KS_Q4K, (const float*)o, qn, n, qn, m->gemm_xt, b_o))) return rc;
     }
     {  // o-proj, x += rms(.) * w_post_attn, image of rms(x) * w_ffn_norm (lib.rs:539)
       const uint8_t* Ws[1] = {(const uint8_t*)L.wo.dptr};
       float* ys[1] = {nullptr};
       epi.next_dtype = KS_Q4K;
+      epi.next = b_gu;
       epi.w_post = L.post_attn32;
       epi.w_norm = L.ffn32;
-      if ((rc = ks_launch_gemm_segs(c, KS_Q4K, 1, Ws, &H, qn, m->gemm_xt, n, ys, &H, m->gemm_p0, KS_GEMM_NORM_SPLIT, &epi))) return rc;
+      if ((rc = ks_launch_gemm_segs(c, KS_Q4K, 1, Ws, &H, qn, m->gemm_xt, n, ys, &H, m->gemm_p0, KS_GEMM_NORM_SPLIT, &epi, b_o))) return rc;
     }
     {  // gate and up share the operand image; their partials meet in the GeGLU epilogue (lib.rs:953)
       const uint8_t* Ws[2] = {(const uint8_t*)L.wgate.dptr, (const uint8_t*)L.wup.dptr};
       float* ys[2] = {nullptr, nullptr};
-      const size_t rs[2] = {F, F};
-      if ((rc = ks_launch_gemm_segs(c, KS_Q4K, 2, Ws, rs, H, m->gemm_xt, n, ys, rs, m->gemm_p0, KS_GEMM_GELU_SPLIT, &epi))) return rc;
+      epi.next = b_down;
+      if ((rc = ks_launch_gemm_segs(c, KS_Q4K, 2, Ws, gu_rows, H, m->gemm_xt, n, ys, gu_rows, m->gemm_p0, KS_GEMM_GELU_SPLIT, &epi, b_gu))) return rc;
     }
     {  // down-proj, x += rms(.) * w_post_ffw, image of the NEXT norm (next layer's attn norm, or the output norm)
       const uint8_t* Ws[1] = {(const uint8_t*)L.wdown.dptr};
       float* ys[1] = {nullptr};
       epi.next_dtype = l + 1 < g.n_layers ? KS_Q4K : (ks_dtype)g.embd_dtype;
+      epi.next = l + 1 < g.n_layers ? b_qkv : b_head;
       epi.w_post = L.post_ffw32;
       epi.w_norm = l + 1 < g.n_layers ? m->layers[l + 1].attn32 : m->output32;
-      if ((rc = ks_launch_gemm_segs(c, KS_Q4K, 1, Ws, &H, F, m->gemm_xt, n, ys, &H, m->gemm_p0, KS_GEMM_NORM_SPLIT, &epi))) return rc;
+      if ((rc = ks_launch_gemm_segs(c, KS_Q4K, 1, Ws, &H, F, m->gemm_xt, n, ys, &H, m->gemm_p0, KS_GEMM_NORM_SPLIT, &epi, b_down))) return rc;
     }
   }
   if ((rc = lane_end(m, L_, n))) return rc;
@@ -432,8 +438,7 @@ int enqueue_forward_gemm(ks_model* m, const Lane& L_, int n, bool want_logits) {
   {
     const uint8_t* Ws[1] = {(const uint8_t*)m->token_embd.dptr};
     float* ys[1] = {(float*)logits};
-    const size_t V = (size_t)g.vocab;
-    if ((rc = ks_launch_gemm_segs(c, (ks_dtype)g.embd_dtype, 1, Ws, &V, H, m->gemm_xt, n, ys, &V, m->gemm_p0, KS_GEMM_PLAIN, nullptr))) return rc;
+    if ((rc = ks_launch_gemm_segs(c, (ks_dtype)g.embd_dtype, 1, Ws, &V, H, m->gemm_xt, n, ys, &V, m->gemm_p0, KS_GEMM_PLAIN, nullptr, b_head))) return rc;
   }
   for (int s = 0; s < n; s++)
     if ((rc = ks_launch_softcap_argmax(c, g.vocab, g.softcap, act, logits + (size_t)s * g.vocab * 4, tok_out + s))) return rc;

@@ -347,7 +347,7 @@ sdpa_chunk_kernel(unsigned n_tok, unsigned n_q, unsigned n_kv, float scale, cons
 // the operand split in one).  One block per (padded) token row, 8 neighbouring dims per thread and step.  The first splits' O are
 // requested before the (m, l) pairs are looked at; a warp makes the factors of a head.
 constexpr unsigned MG_FLY = 4;
-__global__ void __launch_bounds__(512) sdpa_merge_split_kernel(unsigned n_tok, unsigned np, unsigned n_q, unsigned hd, const float* tmp, unsigned n_splits,
+__global__ void __launch_bounds__(512) sdpa_merge_split_kernel(unsigned n_tok, unsigned np, unsigned tbn, unsigned n_q, unsigned hd, const float* tmp, unsigned n_splits,
                                                                __half* xt) {
   ks_pdl_entry();
   extern __shared__ float fac[];  // [n_q][n_splits]: exp(m - M) / L, 0 for an empty split (which may have left no O)
@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(512) sdpa_merge_split_kernel(unsigned n_tok, u
     if (ck < chunks) {
 #pragma unroll
       for (int e = 0; e < 8; e++) v[kk][e] *= down;
-      put_split8(xt, np, q4k_block(np), t, ck, chunks, v[kk], true);
+      put_split8(xt, np, tbn, t, ck, chunks, v[kk], true);
     }
   }
 }
@@ -473,8 +473,8 @@ int ks_launch_sdpa_chunk(ks_ctx* ctx, int n_tok, size_t n_q, size_t n_kv, size_t
 }
 
 // Records of n_tok rows -> the Q4_K form of the operand image (rows past n_tok as zeros).
-int ks_launch_sdpa_merge_split(ks_ctx* ctx, int n_tok, unsigned np, size_t n_q, size_t hd, const float* tmp, int n_splits, void* xt) {
+int ks_launch_sdpa_merge_split(ks_ctx* ctx, int n_tok, ks_gemm_blocks b, size_t n_q, size_t hd, const float* tmp, int n_splits, void* xt) {
   const unsigned chunks = (unsigned)(n_q * hd / 8), threads = chunks < 512u ? (chunks + 31u) / 32u * 32u : 512u;
-  KS_LAUNCH(ctx, sdpa_merge_split_kernel, np, threads, (size_t)n_q * n_splits * sizeof(float), (unsigned)n_tok, np, (unsigned)n_q, (unsigned)hd, tmp, (unsigned)n_splits, (__half*)xt);
+  KS_LAUNCH(ctx, sdpa_merge_split_kernel, b.np, threads, (size_t)n_q * n_splits * sizeof(float), (unsigned)n_tok, b.np, b.tbn, (unsigned)n_q, (unsigned)hd, tmp, (unsigned)n_splits, (__half*)xt);
   return ks_after_launch(ctx, "sdpa_merge_split");
 }

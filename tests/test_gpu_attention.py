@@ -93,3 +93,26 @@ def test_caches_off_16_bytes(ctx, oracle, act, hd, byte_off, pad):
             want = oracle.sdpa_decode(n_q, n_kv, hd, q.astype(np.float32).reshape(n, -1)[s], K[s], V[s], tlens[s], starts[s], scale, 0)
             rtol, atol = (1e-3, 1e-4) if act == F32 else (3e-3, 1e-3)
             assert (np.abs(got[s] - want) <= atol + rtol * np.abs(want)).all()
+
+
+@pytest.mark.parametrize("act", [F32, F16])
+@pytest.mark.parametrize("shape", ["tiny", "e2b_rows"])
+@pytest.mark.parametrize("n", [65, 96, 97, 131, 145, 193, 256])
+def test_prompt_chunks_in_blocks_of_either_size(ctx, oracle, act, shape, n):
+    """65..256 prompt rows: every matrix of a layer reads its token rows in blocks of its own choice (wide ones, or several of up
+    to 64), and the epilogues write the next matrix's.  The slot that took the rows in one chunk and one that took them 60 at a
+    time leave the same next logits."""
+    H, F, hd = (512, 1024, 128) if shape == "tiny" else (1536, 6144, 256)
+    cfg = ksm.ModelConfig(2, H, F, 8, 1, hd, 2048, 320, 2, sigma_w=0.01 if act == F32 else 2e-5, sigma_embd=5e-5, act=act)
+    model = ksm.GemmaCudaModel.synthetic(ctx, cfg, seed=33)
+    toks = [int(t) for t in synth.token_ids(33, "p", n + 1, cfg.vocab)]
+    got = []
+    for slot, step in ((model.slot_alloc(), n), (model.slot_alloc(), 60)):
+        for at in range(0, n, step):
+            model.prefill(slot, toks[at:min(at + step, n)])
+        model.forward(slot, 1, toks[n:], True)
+        ctx.synchronize()
+        got.append(model.read_debug(1, slot).astype(np.float64))
+    # f32 sums in another order through two layers and 4-bit caches (the model's own bound); an f16 head rounds to 2^-11
+    assert np.abs(got[0] - got[1]).max() <= (1e-3 if act == F32 else 2e-3) * np.abs(got[1]).max()
+    model.close()
