@@ -147,7 +147,7 @@ struct ks_model {
   // sampled steps (built on first use): candidates of every slot on the device and in pinned memory
   ks_cand_head* cand_head = nullptr;  // [n_slots] heads, then [n_slots][KS_CAND_MAX] pairs
   void* host_cand = nullptr;
-  // graphs keyed by (first slot, n slots, src parity, want_logits)
+  // graphs keyed by (first slot, n slots, src parity, want_logits); of prompt chunks by (slot, rows, attention forms)
   std::map<uint64_t, cudaGraphExec_t> graphs;
   std::map<uint64_t, size_t> graph_nodes;
   std::vector<void*> owned;
@@ -195,8 +195,22 @@ int dev_alloc(ks_model* m, void** p, size_t bytes) {
 
 constexpr int KS_PREFILL_CHUNK = 8;  // tokens per pass over the weights (the matvec kernels take up to 8)
 constexpr int KS_GEMM_CHUNK = 256;   // rows per pass when the tensor-core GEMM takes the matrices (f32 activations)
-constexpr int KS_CHUNK_ATT_MIN = 4;  // prompt rows from which they share one pass over their context (a block takes 64 rows x heads)
 constexpr size_t KS_STAGE_IDS = 256; // pinned words that stage host token ids
+
+// Do the rows of a prompt chunk share one pass over their context (ks_sdpa_chunk.cu: 64 rows x heads a block, few blocks), or does
+// each take the decode kernel (a block per row and up to four heads, spread over the chip)?  By the work of the second form:
+// rows x blocks x positions a row sees on average, in units of 256 dims.  Microseconds per layer, shared / per row:
+//   tiny (4 heads, 1 KV head of 128)   24 rows at 0: 50 / 44, 256 at 512 (82k): 97 / 86, 128 at 960 (65k): 94 / 93, 96 at 2048 (100k): 94 / 103
+//   E2B (8, 1 of 256)                  32 rows at 0: 70 / 63, 131 at 192 (67k): 115 / 108, 192 at 192 (110k): 124 / 131, 64 at 960 (127k): 89 / 90
+//   E4B (8, 2 of 256)                  131 rows at 0: 157 / 147, 96 at 512 (107k): 140 / 140, 192 at 192 (110k): 169 / 179
+// so 64k is where the per-row form stops winning.  A block of one head does the work of four: with a KV head per query head (8, 8
+// of 128) the line lies near 16k (96 rows at 0: 97 / 97, 131: 106 / 110, 48 at 192: 76 / 76).
+bool rows_share_context(const ks_model_config& g, int n, int base, int window) {
+  const int hpk = g.n_q / g.n_kv, gb = hpk % 4 == 0 ? 4 : hpk % 2 == 0 ? 2 : 1;
+  double seen = base + 0.5 * (n + 1);
+  if (window > 0 && seen > window) seen = window;
+  return n >= 4 && (double)n * (g.n_q / gb) * seen * g.hd >= 256.0 * (gb == 1 ? 16384.0 : 65536.0);
+}
 
 // Where a forward pass reads and writes: n rows of activations, their positions, and the KV caches
 // behind them.  Decode steps map row s to slot first + s (one cache per row); a prompt chunk maps
@@ -213,6 +227,7 @@ struct Lane {
   size_t kv_off;     // byte offset of row 0's cache inside every layer's K / V allocation
   size_t kv_stride;  // bytes between the caches of consecutive rows
   int* chunk_base;   // prompt chunk: the slot's position word (rows take base, base + 1, ...); else nullptr
+  bool share_full, share_swa;  // prompt chunk: do its rows share one pass over their context in a full / sliding-window layer?
 };
 
 Lane slot_lane(ks_model* m, int first, int src) {
@@ -241,8 +256,10 @@ Lane slot_lane(ks_model* m, int first, int src) {
   return L;
 }
 
-Lane chunk_lane(ks_model* m, int slot) {
+Lane chunk_lane(ks_model* m, int slot, bool share_full, bool share_swa) {
   Lane L{};
+  L.share_full = share_full;
+  L.share_swa = share_swa;
   L.x = (char*)m->cx; L.xb = (char*)m->cxb; L.x2 = (char*)m->cx2; L.xn = nullptr;
   L.q = (char*)m->cq; L.k = (char*)m->ck; L.v = (char*)m->cv; L.o = (char*)m->co; L.ff = (char*)m->cff;
   L.logits = nullptr;
@@ -395,7 +412,8 @@ int enqueue_forward_gemm(ks_model* m, const Lane& L_, int n, bool want_logits) {
       head.slot_stride = L_.kv_stride;
       if ((rc = ks_launch_gemm_segs(c, KS_Q4K, 3, Ws, qkv_rows, H, m->gemm_xt, n, ys, qkv_rows, m->gemm_p0, KS_GEMM_QKV, &head, b_qkv))) return rc;
     }
-    if (L_.chunk_base && n >= KS_CHUNK_ATT_MIN && ks_sdpa_chunk_covers(nq, nkv, hd, kk, kv)) {  // the rows of a chunk share their context
+    const bool share = layer_meta(m, L_, l) == L_.meta ? L_.share_full : L_.share_swa;
+    if (share && ks_sdpa_chunk_covers(nq, nkv, hd, kk, kv)) {
       if ((rc = ks_launch_sdpa_chunk(c, n, nq, nkv, hd, g.attn_scale, (const float*)q, kk, kv, layer_meta(m, L_, l), L_.attn_tmp, chunk_splits)) ||
           (rc = ks_launch_sdpa_merge_split(c, n, b_o, nq, hd, L_.attn_tmp, chunk_splits, m->gemm_xt)))
         return rc;
@@ -670,13 +688,15 @@ int run_forward(ks_model* m, int first, int n, int src, bool want_logits) {
 // A chunk of n prompt tokens of one slot (ids already in m->ctok) through every layer, no head.
 int run_prefill_chunk(ks_model* m, int slot, int n, bool gemm) {
   ks_ctx* c = m->ctx;
-  const uint64_t key = (1ull << 63) | ((uint64_t)slot << 32) | ((uint64_t)n << 8);
+  const bool share_full = rows_share_context(m->cfg, n, m->seq_len[slot], 0);
+  const bool share_swa = rows_share_context(m->cfg, n, m->seq_len[slot], m->cfg.sliding_window);
+  const uint64_t key = (1ull << 63) | ((uint64_t)slot << 32) | ((uint64_t)n << 8) | (gemm && share_full ? 1 : 0) | (gemm && share_swa && has_window(m->cfg) ? 2 : 0);
   auto it = m->graphs.find(key);
   if (it == m->graphs.end()) {
     cudaGraph_t graph = nullptr;
     KS_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     const uint64_t before = c->launches;
-    const Lane lane = chunk_lane(m, slot);
+    const Lane lane = chunk_lane(m, slot, share_full, share_swa);
     int rc = gemm       ? enqueue_forward_gemm(m, lane, n, false)
              : m->fused ? enqueue_forward_fused(m, lane, n, false)
                         : enqueue_forward(m, lane, n, false);

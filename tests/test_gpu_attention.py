@@ -116,3 +116,31 @@ def test_prompt_chunks_in_blocks_of_either_size(ctx, oracle, act, shape, n):
     # f32 sums in another order through two layers and 4-bit caches (the model's own bound); an f16 head rounds to 2^-11
     assert np.abs(got[0] - got[1]).max() <= (1e-3 if act == F32 else 2e-3) * np.abs(got[1]).max()
     model.close()
+
+
+@pytest.mark.parametrize("n_q,n_kv,hd,window", [(4, 1, 128, 0), (8, 8, 128, 0), (8, 2, 256, 700)])
+def test_prompt_rows_on_both_sides_of_the_sharing_rule(ctx, oracle, n_q, n_kv, hd, window):
+    """Chunks whose rows take their context one by one, chunks that share it, and both again at other positions (the graph of a
+    row count serves one form only): logits as the CPU decoder's after every chunk (the model's bound)."""
+    cfg = ksm.tiny_config(max_seq=1600, n_kv=n_kv)
+    cfg.n_q, cfg.hd, cfg.n_layers = n_q, hd, 2
+    if window:
+        cfg.sliding_window, cfg.swa_layers = window, 1
+    model, T = ksm.GemmaCudaModel.synthetic(ctx, cfg, seed=34, keep=True)
+    model.slot_alloc()
+    toks = [int(t) for t in synth.token_ids(34, "p", 1500, cfg.vocab)]
+    cpu = oracle.CpuDecoder(oracle.decoder_cfg(cfg), T)
+    at = 0
+    for n in (64, 20, 128, 200, 256, 256, 128, 20, 64, 200):
+        model.prefill(0, toks[at:at + n])
+        for t in toks[at:at + n]:
+            cpu.forward_token(t, False)
+        at += n
+        model.forward(0, 1, [toks[at]], True)
+        ctx.synchronize()
+        cpu.forward_token(toks[at], True)
+        at += 1
+        want, got = cpu.logits().astype(np.float64), model.read_debug(1, 0).astype(np.float64)
+        assert np.abs(got - want).max() <= 1e-3 * np.abs(want).max(), (n, at)
+    cpu.close()
+    model.close()
