@@ -134,6 +134,7 @@ int ks_launch_matvec_q4k_fx(ks_ctx* ctx, const ks_mv_seg* segs, int n_seg, ks_mv
                             const void* x, int n_tok, const ks_plan* plan);
 // Device error word raised by a kernel whose bounded wait gave up (index into ctx->ws, in words).
 #define KS_WS_ERR_WORD 4000
+#define KS_WS_FENCE_WORD 4001  // cleared behind the load-time quantiser and otherwise unused
 
 int ks_launch_rmsnorm(ks_ctx* ctx, size_t n, size_t rows, float eps, ks_dtype act, const void* x, const void* w,
                       const void* res, int has_scale, float scale, void* y);

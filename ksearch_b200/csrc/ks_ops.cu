@@ -608,7 +608,12 @@ int ks_launch_quantize_q4k(ks_ctx* ctx, ks_dtype src_dtype, const void* src, siz
   if (nelem % 256 || (threads + 127) / 128 >= (1ull << 31)) return ks_fail(ctx, KS_ERR_INVALID, "quantize_q4k: bad element count %zu", nelem);
   if (n_sb == 0) return KS_OK;
   KS_LAUNCH(ctx, (quantize_q4k_kernel), (unsigned)((threads + 127) / 128), 128, 0, (int)src_dtype, (const uint8_t*)src, n_sb, (uint8_t*)dst);
-  return ks_after_launch(ctx, "quantize_q4k");
+  // The matvec and GEMM kernels fetch weights before they wait for the kernel in front of them.  What this one writes are
+  // weights: a node that is no kernel keeps every later launch behind its end.
+  const int rc = ks_after_launch(ctx, "quantize_q4k");
+  if (rc) return rc;
+  KS_CUDA(ctx, cudaMemsetAsync((unsigned*)ctx->ws + KS_WS_FENCE_WORD, 0, sizeof(unsigned), ctx->stream));
+  return KS_OK;
 }
 
 extern "C" {

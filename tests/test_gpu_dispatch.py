@@ -176,3 +176,27 @@ def test_a_large_dmin_without_minima_changes_nothing(ctx, oracle, batch):
     ctx.check(ctx.lib.ks_matvec(ctx.h, rows, cols, Q4K, bw.h, 0, 0, bx.h, 0, y.h, 0, batch))
     y32, y64 = oracle.matvec(Q4K, np.frombuffer(raw, np.uint8), rows, cols, x)
     _check(ctx.read_f32(y, batch * rows).reshape(batch, rows) * 2.0 ** 20, y32 * np.float32(2.0 ** 20), y64 * 2.0 ** 20, f"{batch} rows")
+
+
+@pytest.mark.parametrize("batch", [1, 3, 9])
+def test_weights_quantised_just_before(batch):
+    """Weights written by the quantiser and read by the next op of the same stream, without a wait between (programmatic
+    dependent launch on): the same bits as after a wait, every time."""
+    rows, cols = 8192, 2560
+    c = CudaContext(0, flags=1)
+    rng = np.random.default_rng(76)
+    w = [c.buffer_bytes(rng.standard_normal(rows * cols, np.float32)) for _ in range(2)]
+    W, x = c.buffer_empty_bytes(rows * cols // 256 * 144), c.buffer_bytes(rng.standard_normal(batch * cols, np.float32))
+    y = c.buffer_empty_f32(batch * rows)
+
+    def run(i, wait):
+        c.check(c.lib.ks_quantize_q4k(c.h, 0, w[i].h, 0, rows * cols, W.h, 0))
+        if wait:
+            c.synchronize()
+        c.check(c.lib.ks_matvec(c.h, rows, cols, Q4K, W.h, 0, 0, x.h, 0, y.h, 0, batch))
+        return c.read_f32(y, batch * rows)
+
+    want = [run(i, True) for i in range(2)]
+    for k in range(6):
+        assert np.array_equal(run(k % 2, False), want[k % 2])
+    c.close()
