@@ -351,16 +351,14 @@ __global__ void __launch_bounds__(GM_THREADS + 64, 2) gemm_q6k_tc_kernel(const G
   if (warp == 0) tc_dealloc(tmem, a.tmem_cols);
 }
 
-// Sum of the k-split partials in split order (the result does not depend on how the CTAs were scheduled), then
-// the epilogue.  mode 0: up to three matrices, y[i] = sum of P[i]; mode 1: y[0] = gelu(sum of P[0]) * (sum of P[1])
-// (lib.rs:953, the GeGLU of gate and up).
+// Sum of the k-split partials in split order (the result does not depend on how the CTAs were scheduled) into y[i], for up
+// to three matrices.
 struct FinishArgs {
   const float* P[3];
   float* y[3];
   size_t ldy[3], part_stride[3];
   unsigned rows[3], tile0[3], group0[3], n_seg, n_tok;
   ks_gemm_map map;
-  int mode;
 };
 // One block per row tile and a few token rows (the tile's partial count is the block's); a thread sums four neighbouring rows
 // where row counts and addresses allow 16-byte accesses, else one.
@@ -389,7 +387,7 @@ template <int V>
 __global__ void __launch_bounds__(256) gemm_finish_kernel(const FinishArgs f) {
   ks_pdl_entry();
   constexpr unsigned PER = GM_ROWS / V, TOK = 256u / PER;  // threads per token row, token rows per block
-  const unsigned bx = blockIdx.x, seg = f.mode == 1 ? 0u : (bx >= f.tile0[1]) + (bx >= f.tile0[2]);
+  const unsigned bx = blockIdx.x, seg = (bx >= f.tile0[1]) + (bx >= f.tile0[2]);
   const unsigned rows = seg == 0 ? f.rows[0] : seg == 1 ? f.rows[1] : f.rows[2];
   const unsigned tile0 = seg == 0 ? f.tile0[0] : seg == 1 ? f.tile0[1] : f.tile0[2];
   const float* P = seg == 0 ? f.P[0] : seg == 1 ? f.P[1] : f.P[2];
@@ -400,12 +398,7 @@ __global__ void __launch_bounds__(256) gemm_finish_kernel(const FinishArgs f) {
   if (t >= f.n_tok || r >= rows) return;
   const size_t at = (size_t)t * rows + r;  // partials are dense [split][token][row]
   const unsigned group0 = seg == 0 ? f.group0[0] : seg == 1 ? f.group0[1] : f.group0[2];
-  FinVec<V> g = sum_slots<V>(P, ps, ks_gemm_slots(f.map, group0, bx - tile0, t), at);
-  if (f.mode == 1) {
-    const FinVec<V> u = sum_slots<V>(f.P[1], f.part_stride[1], ks_gemm_slots(f.map, f.group0[1], bx, t), at);
-#pragma unroll
-    for (int k = 0; k < V; k++) g.v[k] = gelu_mul(g.v[k], u.v[k]);
-  }
+  const FinVec<V> g = sum_slots<V>(P, ps, ks_gemm_slots(f.map, group0, bx - tile0, t), at);
   float* o = y + (size_t)t * ldy + r;
   if constexpr (V == 4) *reinterpret_cast<float4*>(o) = make_float4(g.v[0], g.v[1], g.v[2], g.v[3]);
   else *o = g.v[0];
@@ -730,8 +723,8 @@ bool ks_gemm_few_rows_q6k(const ks_ctx* ctx, size_t rows, size_t cols) { return 
 // Q4_K matrices against more than 64 token rows: pairs of row tiles against blocks of up to 128 read the token rows half as
 // often; where that leaves few units for the SMs, single tiles against blocks of up to 64 are four times as many.  By the
 // estimate both maps are chosen by; with an epilogue behind it (sums always read once more) only where it promises a tenth: a
-// whole E2B layer of 256 rows took 142 us with wide blocks and 145 with the four small ones the bare estimate picks; of 128
-// rows 117 with wide blocks, 105 with small ones, of the tiny shape 87 and 60.
+// whole E2B layer of 256 rows took 142 us with wide blocks, 145 with the four small ones the bare estimate picks, 139 with this
+// line; of 128 rows 117 with wide blocks and 105 with small ones, of the tiny shape 87 and 60.
 ks_gemm_blocks ks_gemm_pick(const ks_ctx* ctx, ks_dtype wdtype, int n_seg, const size_t* rows, size_t cols, int n_tok, bool plain) {
   const Blocks wide = gemm_blocks(n_tok);
   if (wdtype != KS_Q4K || wide.tbn <= 64u) return wide;
@@ -760,8 +753,7 @@ int ks_launch_gemm_split(ks_ctx* ctx, ks_dtype wdtype, const float* x, size_t ld
 
 // Up to three matrices over the same columns in one launch.  With one k split matrix i's result goes straight to
 // y[i] (row stride ldy[i]); otherwise the partials go to P (dense [split][token][row] per matrix, matrix after
-// matrix) and a second launch sums them in split order into y.  mode 1 (two matrices, gate and up): y[0] =
-// gelu(gate) * up, always through P.  `xt` is the image of the token rows in these blocks.
+// matrix) and a second launch sums them in split order into y, or takes them through an epilogue.  `xt` is the image of the token rows in these blocks.
 int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* const* W, const size_t* rows, size_t cols, const void* xt,
                         int n_tok, float* const* y, const size_t* ldy, float* P, int mode, const ks_gemm_epi* epi, ks_gemm_blocks blocks) {
   if (!gemm_covers(wdtype, cols, n_tok) || n_seg < 1 || n_seg > 3) return ks_fail(ctx, KS_ERR_UNSUPPORTED, "gemm: shape not covered");
@@ -804,10 +796,8 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
       f.P[i] = out[i];
       f.part_stride[i] = part_stride[i];
       f.rows[i] = (unsigned)rows[i];
-      if (mode == KS_GEMM_PLAIN || mode == KS_GEMM_GELU) {
-        f.y[i] = mode == KS_GEMM_GELU ? y[0] : y[i];
-        f.ldy[i] = mode == KS_GEMM_GELU ? ldy[0] : ldy[i];
-      }
+      f.y[i] = y[i];  // null where an epilogue takes the sums
+      f.ldy[i] = ldy[i];
       poff += (size_t)slots * n_tok * rows[i];
     }
   }
@@ -929,15 +919,12 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
     f.group0[i] = group0[i];
   }
   f.n_tok = (unsigned)n_tok;
-  f.mode = mode;
-  const unsigned out_tiles = mode == KS_GEMM_GELU ? tile0[1] : tiles;
   bool vec = true;
   for (int i = 0; i < n_seg; i++) {
-    vec = vec && rows[i] % 4 == 0 && ((uintptr_t)out[i] & 15) == 0;
-    if (mode == KS_GEMM_PLAIN || i == 0) vec = vec && ((uintptr_t)f.y[i] & 15) == 0 && f.ldy[i] % 4 == 0;
+    vec = vec && rows[i] % 4 == 0 && ((uintptr_t)out[i] & 15) == 0 && ((uintptr_t)f.y[i] & 15) == 0 && f.ldy[i] % 4 == 0;
   }
   const unsigned tok = vec ? 8u : 2u;
-  const dim3 grid(out_tiles, ((unsigned)n_tok + tok - 1) / tok);
+  const dim3 grid(tiles, ((unsigned)n_tok + tok - 1) / tok);
   if (vec) KS_LAUNCH(ctx, (gemm_finish_kernel<4>), grid, 256, 0, f);
   else KS_LAUNCH(ctx, (gemm_finish_kernel<1>), grid, 256, 0, f);
   return ks_after_launch(ctx, "gemm_finish");

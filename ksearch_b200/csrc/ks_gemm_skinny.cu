@@ -191,8 +191,9 @@ __global__ void __launch_bounds__(SK_MAX_WARPS * 32, 1) gemm_q4k_skinny_kernel(c
 // One matrix, direct output.  A tile is 16 whole rows: 3360 bytes per 256 columns, contiguous and a multiple of 16, so one bulk
 // copy brings it into a ring of `stages` (rows of 210-byte blocks start on any even address: words are read aligned and shifted
 // into place).  A = q - 32 as f16, exact; a 16-column run (one scale) is one k step, its two mmas (the tokens' two terms) share
-// f32 sums that then take the scale.  Bound by instructions (about 350 per warp and tile of 16 x 128 weights), close to the
-// time its bytes take; the tcgen05 kernel spends its time on hand-overs: 262144 x 2560 x 8 rows 450 us.
+// f32 sums that then take the scale.  Bound by instructions, about 350 per warp and tile of 16 x 128 weights, most on the
+// integer pipe: 262144 x 2560 x 8 rows 204 us where the bytes take 84 (the tcgen05 kernel, which spends its time on hand-overs:
+// 450 us).
 constexpr unsigned S6_PITCH = 10, S6_PSUM = 16 * S6_PITCH, S6_GROUP = 2, S6_MAX_STAGES = 6;
 constexpr unsigned S6_TILE = 16u * 210u;  // bytes of a tile per 256 columns
 constexpr unsigned S6_WAIT = 1u << 20;

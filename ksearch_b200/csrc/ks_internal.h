@@ -185,7 +185,7 @@ int ks_launch_candidates(ks_ctx* ctx, ks_dtype act, const void* logits, size_t n
 // The draw over the n candidates of a row of n_all in index order; the others' probabilities fall under the min-p threshold.
 uint32_t ks_sample_candidates(const ks_cand* c, size_t n, size_t n_all, float cap, float temperature, float min_p, uint32_t seed);
 
-// ---- tensor-core GEMM for batches of more than 8 token rows (ks_gemm.cu) ---------------------------
+// ---- tensor-core GEMM for batches of token rows (ks_gemm.cu) -----------------------------------------
 // nelem (a multiple of 256) elements of src (Q6K, Q4K, F16, F32) -> Q4_K blocks, as the reference's load-time quantizer.
 int ks_launch_quantize_q4k(ks_ctx* ctx, ks_dtype src_dtype, const void* src, size_t nelem, void* dst);
 size_t ks_gemm_xt_bytes(size_t cols, int n_tok);  // bytes of the split image of n_tok rows of `cols` values
@@ -199,11 +199,11 @@ ks_gemm_blocks ks_gemm_pick(const ks_ctx* ctx, ks_dtype wdtype, int n_seg, const
 // x[t * ldx + k] (f32) -> the image the GEMM over weights of that dtype reads its token rows from.
 int ks_launch_gemm_split(ks_ctx* ctx, ks_dtype wdtype, const float* x, size_t ldx, int n_tok, size_t cols, void* xt, ks_gemm_blocks b);
 // Up to three matrices over the same columns and token rows (q, k, v; gate, up) in one launch.  What becomes of
-// the sums: PLAIN y[i] = W[i] x; GELU (two matrices) y[0] = gelu(W[0] x) * (W[1] x); NORM_SPLIT (one matrix)
+// the sums: PLAIN y[i] = W[i] x; NORM_SPLIT (one matrix)
 // out_x = res + rms(W x) * w_post and the image of rms(out_x) * w_norm for the next GEMM in xt_out; GELU_SPLIT
 // (two matrices) the image of gelu(W[0] x) * (W[1] x) in xt_out.  P: ks_gemm_part_floats(sum of rows) floats.
 // QKV (three matrices): per-head norm and RoPE of q into out_x, of k and v into the cache rows (Q4_0).
-enum { KS_GEMM_PLAIN = 0, KS_GEMM_GELU = 1, KS_GEMM_NORM_SPLIT = 2, KS_GEMM_GELU_SPLIT = 3, KS_GEMM_QKV = 4 };
+enum { KS_GEMM_PLAIN, KS_GEMM_NORM_SPLIT, KS_GEMM_GELU_SPLIT, KS_GEMM_QKV };
 struct ks_gemm_epi {
   const float *res, *w_post, *w_norm;  // NORM_SPLIT: residual rows [n_tok, rows], the two norm weights
   float eps;
@@ -241,7 +241,7 @@ struct ks_mega_desc {
   const float* rope;  // [max_seq, hd]
   const int* pos;     // device: position of the token being processed
   float *x_a, *x_b;   // residual stream ping-pong; the token's embedding is in x_a on entry
-  float *yb, *q, *k, *v, *o, *ff;
+  float* yb;
   float* att_tmp;     // n_q * n_splits * (hd + 2) floats
   int n_splits;
 };

@@ -60,7 +60,7 @@ struct MegaArgs {
   const float* rope;        // [max_seq, hd]
   const int* pos;           // [1]
   float *x_a, *x_b;         // residual stream: layers read x_a / write x_b at the FFN, the reverse at the next qkv
-  float *yb, *q, *k, *v;
+  float* yb;
   unsigned char *ox, *ffx;  // attention output and GeGLU output, written by their producers in the staged fixed-point layout
   float* att_tmp;           // [n_q * n_splits * (hd + 2)]
   float4* nsum;             // [grid] per-block sums of the last o-proj / down phase: (sum y^2, sum x*y*wp, sum (y*wp)^2, sum x^2)
@@ -601,62 +601,6 @@ __device__ __forceinline__ void mg_issue_ent(const ItemEnt& e, const MegaLayer& 
     const int m = lane / MG_RL, rr = lane % MG_RL;
     if ((unsigned)rr < valid)
       bulk_in(slot_addr + (uint32_t)lane * seg_bytes, L.W[e.widx + m] + e.src_off + (size_t)rr * row_bytes, seg_bytes, bar);
-  }
-}
-
-// Multiply-accumulate one item: MATS row slots per lane, units of this lane in the segment.
-template <int MATS>
-__device__ __forceinline__ void mg_item_compute(uint32_t slot_addr, uint32_t xs_s, unsigned units, unsigned seg_blocks,
-                                                unsigned cs, int cl, int rl, float (&yacc)[2]) {
-  const int g = cl & 3;
-  const unsigned seg_bytes = seg_blocks * KS_Q4K_BLOCK_BYTES, seg_units = seg_blocks * 4, upl = seg_units / MG_LPR;
-  uint32_t waddr = slot_addr + (uint32_t)rl * seg_bytes + (uint32_t)(cl >> 2) * KS_Q4K_BLOCK_BYTES + (uint32_t)g * 32u;
-  uint32_t xaddr = xs_s + (cs * seg_units + (unsigned)cl) * (Q4K_XS * 4u);
-  uint32_t saddr = xs_s + units * (Q4K_XS * 4u) + (cs * seg_units + (unsigned)cl) * 8u;
-  for (unsigned it = 0; it < upl; it++) {
-    const float2 sx = lds_f2a(saddr);
-    u64 acc[MATS][2];
-#pragma unroll
-    for (int r = 0; r < MATS; r++) acc[r][0] = acc[r][1] = 0ull;
-    {
-      u64 xf[16];
-      lds_p2o<0>(xaddr, xf[0], xf[1]);     lds_p2o<16>(xaddr, xf[2], xf[3]);
-      lds_p2o<32>(xaddr, xf[4], xf[5]);    lds_p2o<48>(xaddr, xf[6], xf[7]);
-      lds_p2o<64>(xaddr, xf[8], xf[9]);    lds_p2o<80>(xaddr, xf[10], xf[11]);
-      lds_p2o<96>(xaddr, xf[12], xf[13]);  lds_p2o<112>(xaddr, xf[14], xf[15]);
-#pragma unroll
-      for (int r = 0; r < MATS; r++) {
-        const uint4 q = lds_u4o<16>(waddr + (uint32_t)(r * MG_RL) * seg_bytes);
-        q4_word_p(q.x, xf[0], xf[1], xf[2], xf[3], acc[r][0], acc[r][1]);
-        q4_word_p(q.y, xf[4], xf[5], xf[6], xf[7], acc[r][0], acc[r][1]);
-        q4_word_p(q.z, xf[8], xf[9], xf[10], xf[11], acc[r][0], acc[r][1]);
-        q4_word_p(q.w, xf[12], xf[13], xf[14], xf[15], acc[r][0], acc[r][1]);
-      }
-    }
-    {
-      u64 xf[16];
-      lds_p2o<128>(xaddr, xf[0], xf[1]);    lds_p2o<144>(xaddr, xf[2], xf[3]);
-      lds_p2o<160>(xaddr, xf[4], xf[5]);    lds_p2o<176>(xaddr, xf[6], xf[7]);
-      lds_p2o<192>(xaddr, xf[8], xf[9]);    lds_p2o<208>(xaddr, xf[10], xf[11]);
-      lds_p2o<224>(xaddr, xf[12], xf[13]);  lds_p2o<240>(xaddr, xf[14], xf[15]);
-#pragma unroll
-      for (int r = 0; r < MATS; r++) {
-        const uint4 q = lds_u4o<32>(waddr + (uint32_t)(r * MG_RL) * seg_bytes);
-        q4_word_p(q.x, xf[0], xf[1], xf[2], xf[3], acc[r][0], acc[r][1]);
-        q4_word_p(q.y, xf[4], xf[5], xf[6], xf[7], acc[r][0], acc[r][1]);
-        q4_word_p(q.z, xf[8], xf[9], xf[10], xf[11], acc[r][0], acc[r][1]);
-        q4_word_p(q.w, xf[12], xf[13], xf[14], xf[15], acc[r][0], acc[r][1]);
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < MATS; r++) {
-      const uint4 hdr = lds_u4o<0>(waddr + (uint32_t)(r * MG_RL) * seg_bytes - (uint32_t)g * 32u);
-      const float2 a01 = unpack2(padd2(acc[r][0], acc[r][1]));
-      yacc[r] = q4k_apply_scales(hdr, g, a01.x, a01.y, sx.x, sx.y, yacc[r]);
-    }
-    waddr += (MG_LPR / 4) * KS_Q4K_BLOCK_BYTES;
-    xaddr += MG_LPR * Q4K_XS * 4u;
-    saddr += MG_LPR * 8u;
   }
 }
 
@@ -1482,7 +1426,7 @@ int ks_mega_create(ks_ctx* ctx, const ks_mega_desc* d, const ks_mega_layer* laye
   a.eps = d->eps; a.attn_scale = d->attn_scale;
   a.rope = d->rope; a.pos = d->pos;
   a.x_a = d->x_a; a.x_b = d->x_b;
-  a.yb = d->yb; a.q = d->q; a.k = d->k; a.v = d->v;
+  a.yb = d->yb;
   a.ox = mg->d_fx;
   a.ffx = mg->d_fx + (size_t)qn / 64 * 256;
   a.att_tmp = d->att_tmp;

@@ -194,7 +194,7 @@ int dev_alloc(ks_model* m, void** p, size_t bytes) {
 }
 
 constexpr int KS_PREFILL_CHUNK = 8;  // tokens per pass over the weights (the matvec kernels take up to 8)
-constexpr int KS_GEMM_CHUNK = 256;   // rows per pass when the tensor-core GEMM takes the matrices (f32 activations)
+constexpr int KS_GEMM_CHUNK = 256;   // rows per pass when the tensor-core GEMM takes the matrices
 constexpr size_t KS_STAGE_IDS = 256; // pinned words that stage host token ids
 
 // Do the rows of a prompt chunk share one pass over their context (ks_sdpa_chunk.cu: 64 rows x heads a block, few blocks), or does
@@ -361,9 +361,9 @@ int enqueue_forward(ks_model* m, const Lane& L_, int n, bool want_logits) {
   return ks_after_launch(c, "collect");
 }
 
-// The same op order for 9..KS_GEMM_CHUNK rows (a prompt chunk, or more slots than the batch matvec stages side by
-// side): the matrices go through the tensor-core GEMM, the reference's mul_mm route (forward_prefill_chunk,
-// gemma_prim.rs:1317-1607); norms, RoPE/KV pack, attention and GELU are the row-wise kernels above.  f32 only.
+// The same op order for 3..KS_GEMM_CHUNK rows (a prompt chunk of a model of either activation dtype, or a step of several slots
+// of an f32 model): the matrices go through the tensor-core GEMM, the reference's mul_mm route (forward_prefill_chunk,
+// gemma_prim.rs:1317-1607), norms, RoPE, KV pack and GELU through its epilogues.  f32 between the ops.
 int enqueue_forward_gemm(ks_model* m, const Lane& L_, int n, bool want_logits) {
   ks_ctx* c = m->ctx;
   const ks_model_config& g = m->cfg;
@@ -607,7 +607,7 @@ int get_mega(ks_model* m, int first, ks_model::Mega* out) {
     return KS_OK;
   }
   const ks_model_config& g = m->cfg;
-  const size_t H = g.hidden, F = g.ffn, qn = (size_t)g.n_q * g.hd, kvn = (size_t)g.n_kv * g.hd;
+  const size_t H = g.hidden, F = g.ffn;
   ks_mega_desc d{};
   d.n_layers = g.n_layers;
   d.hidden = (unsigned)H; d.ffn = (unsigned)F; d.n_q = (unsigned)g.n_q; d.n_kv = (unsigned)g.n_kv; d.hd = (unsigned)g.hd;
@@ -617,11 +617,6 @@ int get_mega(ks_model* m, int first, ks_model::Mega* out) {
   d.x_a = m->step32 ? m->step32 + (size_t)first * 3 * H : (float*)m->x + (size_t)first * H;
   d.x_b = m->step32 ? d.x_a + H : (float*)m->xb + (size_t)first * H;
   d.yb = m->step32 ? d.x_a + 2 * H : (float*)m->x2 + (size_t)first * H;
-  d.q = (float*)m->q + (size_t)first * qn;
-  d.k = (float*)m->k + (size_t)first * kvn;
-  d.v = (float*)m->v + (size_t)first * kvn;
-  d.o = (float*)m->o + (size_t)first * qn;
-  d.ff = (float*)m->ff + (size_t)first * F;
   d.att_tmp = m->attn_tmp + (size_t)first * g.n_q * m->n_splits * (g.hd + 2);
   d.n_splits = m->n_splits;
   std::vector<ks_mega_layer> ls(g.n_layers);
@@ -1244,11 +1239,10 @@ static int check_device_status(ks_model* m, const unsigned* status, int first, i
   return ks_fail(c, KS_ERR_TIMEOUT, "a device-side wait gave up during decode (status word 0x%x); the slots were rewound", flag);
 }
 
-// Prompt tokens of one slot, KS_PREFILL_CHUNK at a time: the rows of a chunk share one pass over the
-// weights (the batch form of the matvec kernels, K:1414) and attend causally inside the chunk.  This is
-// the reference's GEMV fallback for prompts (forward_prefill_chunk, gemma_prim.rs:1317-1607, runs its
-// mul_mm GEMM instead); no logits are produced.  Enqueues only, apart from the wait for the pinned
-// staging words between chunks.
+// Prompt tokens of one slot, up to KS_GEMM_CHUNK at a time through the tensor-core GEMM (a last pair, and models it does not
+// cover: as many rows as the batch matvec stages): the rows of a chunk share one pass over the weights and attend causally
+// inside the chunk (forward_prefill_chunk, gemma_prim.rs:1317-1607); no logits are produced.  Enqueues only, apart from the
+// wait for the pinned staging words between chunks.
 int ks_model_prefill(ks_model* m, int slot, const int* tokens, int n_tokens) {
   if (!m) return KS_ERR_INVALID;
   ks_ctx* c = m->ctx;

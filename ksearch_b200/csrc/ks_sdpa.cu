@@ -7,14 +7,15 @@
 // dispatched by Eng::sdpa_hybrid_kv (crates/ksearch_kernels/src/lib.rs:1157-1178).
 //
 // Layout.  K and V: [max_t, n_kv, hd] in Q4_0 (18-byte blocks of 32 values), per
-// slot.  One block of the grid handles (split, kv head, slot); its warps take
-// the positions of the split round-robin.  A warp serves ALL query heads of the
-// KV head's group from one read of the K/V row: lane L owns the dims that live
-// in bytes [ (L % LPB)*BPL, +BPL ) of Q4_0 block L / LPB (low nibbles = dims i,
-// high nibbles = dims i+16), so a row is read once, 2 bytes at a time, and is
-// never dequantised to memory.  Running (m, l, O) per head stay in registers;
-// warps are merged through shared memory, splits through `tmp` with the
-// reference's (m, l, O[hd]) record layout, stride hd+2, m initialised to -1e30.
+// slot.  Splits are merged through `tmp` with the reference's (m, l, O[hd])
+// record layout, stride hd+2, m initialised to -1e30.  Two kernels leave such
+// records: sdpa_mma_kernel (tensor cores; caches that start on 4 bytes, further
+// below) and, for the others, sdpa_part_kernel: one block per (split, kv head,
+// slot), its warps take the positions of the split round-robin.  A warp serves
+// up to four query heads of the KV head's group from one read of the K/V row:
+// lane L owns the dims that live in bytes [ (L % LPB)*BPL, +BPL ) of Q4_0 block
+// L / LPB (low nibbles = dims i, high nibbles = dims i+16), so a row is read
+// once, 2 bytes at a time, and is never dequantised to memory.
 #include <cstdlib>
 
 #include "ks_internal.h"
@@ -37,25 +38,8 @@ __device__ __forceinline__ void st_act<__half>(__half* p, size_t i, float v) { p
 constexpr int kWarps = 4;
 constexpr float kNegInit = -1.0e30f;
 
-// Load this lane's DPL values of one Q4_0 row: dims (lo nibbles) then dims+16 (hi nibbles).
-template <int DPL>
-__device__ __forceinline__ void load_row(const uint8_t* row, int lane, float (&out)[DPL]) {
-  constexpr int BPL = DPL / 2;        // bytes per lane
-  constexpr int LPB = 16 / BPL;       // lanes per 32-value block
-  const uint8_t* blk = row + (lane / LPB) * KS_Q40_BLOCK_BYTES;
-  const float d = __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short*>(blk)));
-  const unsigned short* qs = reinterpret_cast<const unsigned short*>(blk + 2 + (lane % LPB) * BPL);
-#pragma unroll
-  for (int w = 0; w < BPL / 2; w++) {
-    const unsigned v = qs[w];
-    out[2 * w] = (float)((int)(v & 0xF) - 8) * d;
-    out[2 * w + 1] = (float)((int)((v >> 8) & 0xF) - 8) * d;
-    out[BPL + 2 * w] = (float)((int)((v >> 4) & 0xF) - 8) * d;
-    out[BPL + 2 * w + 1] = (float)((int)(v >> 12) - 8) * d;
-  }
-}
-// The same DPL values as plain nibbles (0..15 as floats) and the block's scale: the -8 offset and the scale are
-// applied once per (row, head) by the caller instead of once per value.
+// This lane's DPL values of one Q4_0 row, dims (low nibbles) then dims + 16 (high nibbles), as plain nibbles (0..15 as floats),
+// and the block's scale: the -8 offset and the scale are applied once per (row, head) by the caller.
 template <int DPL>
 __device__ __forceinline__ float load_row_raw(const uint8_t* row, int lane, float (&out)[DPL]) {
   constexpr int BPL = DPL / 2;
