@@ -487,12 +487,13 @@ static int check_w(ks_ctx* ctx, const char* what, ks_dtype wd, const ks_buf* W, 
 }
 
 // 2..8 token rows: the tensor cores, whose time hardly depends on the row count, from where their three launches cost less than
-// the matvec's extra rows.  Measured, matvec against GEMM: Q4_K 256x512 8 rows 7.9 / 8.9 us, 1000x1536 4 rows 8.7 / 9.0,
-// 6 rows 12.4 / 8.9, 4096x1536 2 rows 7.1 / 7.3, 3 rows 9.5 / 7.3, 20480x2560 8 rows 104 / 17; Q6_K 512x1536 2 rows
-// 7.0 / 7.2, 3 rows 10.5 / 6.9.  Where the few-row Q6_K kernel does not reach (more than 2560 columns, rows not a multiple of 8, packed rows off 16 bytes)
-// the matvec keeps the call although the tcgen05 kernel is faster from 3 rows on (20480x4096 129 / 79 us): that kernel's f32
-// sums over many columns are 15 times as far from 64 bits (2048x10240 x 4: 1.5e-7 / 2.4e-6).  It takes only rows that the
-// matvec cannot stage side by side (80 bytes of shared memory per 16 columns and row).
+// the matvec's extra rows.  Measured through the entry point, us, matvec against GEMM: Q4_K 2 rows 4096x1536 7.1 / 7.2, 1536x6144
+// 14.5 / 13.6, 2560x10240 31.9 / 16.7; 3 rows 4500x512 5.1 / 6.4, 1536x1536 9.4 / 11.2, 3000x1024 6.9 / 6.7, 1536x2048 11.4 / 7.2,
+// 2560x2560 11.8 / 10.2; 4 rows 1536x1536 11.6 / 9.1; 5 rows 1000x1536 11.3 / 9.1; 8 rows 20480x2560 100 / 20; Q6_K 512x1536 2 rows
+// 7.0 / 7.2, 3 rows 10.5 / 6.9.  Where the few-row Q6_K kernel does not reach (more than 2560 columns, rows not a multiple of 8,
+// packed rows off 16 bytes) the matvec keeps the call although the tcgen05 kernel is faster from 3 rows on (20480x4096 129 / 79):
+// that kernel's f32 sums over many columns are 15 times as far from 64 bits (2048x10240 x 4: 1.5e-7 / 2.4e-6).  It takes only
+// rows that the matvec cannot stage side by side (80 bytes of shared memory per 16 columns and row).
 // No such call allocates or waits: what would not fit the scratch that every context starts with keeps the matvec, and so does a
 // captured stream (the GEMM has not been measured inside a graph of few-row calls).  So do token rows that
 // do not start on 16 bytes (a wrapped buffer, an odd offset): the operand split reads them 16 bytes at a time, the matvec needs not.
@@ -502,7 +503,7 @@ static bool few_rows_gemm(const ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_
   if (ctx->has_override || (!ctx->plans.empty() && ks_plan_lookup(ctx, wdtype == KS_Q4K ? "mv_q4k" : "mv_q6k", rows, cols, n_tok))) return false;
   const double work = (double)rows * (double)cols * n_tok;
   const bool staged = (size_t)n_tok * (cols / 16) * 80 <= ctx->smem_optin;
-  if (wdtype == KS_Q4K ? work < (n_tok == 2 ? 14e6 : 6.5e6) : !ks_gemm_few_rows_q6k(ctx, rows, cols) || ((uintptr_t)W & 15) ? staged : work < (n_tok == 2 ? 3e6 : 2e6))
+  if (wdtype == KS_Q4K ? work < (n_tok == 2 ? 14e6 : n_tok == 3 && cols <= 2048 ? 9e6 : 6.5e6) : !ks_gemm_few_rows_q6k(ctx, rows, cols) || ((uintptr_t)W & 15) ? staged : work < (n_tok == 2 ? 3e6 : 2e6))
     return false;
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   return cudaStreamIsCapturing(ctx->stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone &&

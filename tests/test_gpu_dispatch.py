@@ -137,6 +137,7 @@ def test_few_rows_never_allocate_and_graphs_outlive_growth(oracle):
 
 @pytest.mark.parametrize("dtype,rows,cols,batch,launches", [
     (Q4K, 4096, 1536, 3, (2, 3)), (Q4K, 1024, 10240, 4, (2, 3)), (Q4K, 16384, 512, 8, (2, 3)),   # the few-row kernels
+    (Q4K, 1536, 1536, 3, (1,)), (Q4K, 2048, 1536, 3, (2, 3)), (Q4K, 1536, 1536, 4, (2, 3)),      # either side of the line for 3 rows
     (Q6K, 4096, 1536, 3, (2,)), (Q6K, 2048, 2560, 8, (2,)),
     (Q6K, 2048, 10240, 4, (1,)), (Q6K, 2007, 2048, 8, (1,)), (Q6K, 2056, 2048, 3, (1,)),         # outside the Q6_K one: the matvec
     (Q6K, 512, 10240, 8, (2, 3)),                                                                # more than the matvec can stage
