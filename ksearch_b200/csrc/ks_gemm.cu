@@ -654,7 +654,7 @@ __global__ void __launch_bounds__(256) gemm_finish_qkv_kernel(const EpiQkvArgs e
 }  // namespace
 
 namespace {
-// Token rows padded to what the MMAs take (N a multiple of 16; beyond 128 the Q4_K kernel takes them in two halves).
+// Token rows of the Q6_K kernel, padded to what its MMAs take.
 unsigned gemm_np(int n_tok) { return n_tok > 128 ? ((unsigned)n_tok + 31u) / 32u * 32u : ((unsigned)n_tok + 15u) / 16u * 16u; }
 // Shared memory of one CTA and its stage count (A and B rings have the same depth): two stages when that lets two
 // CTAs share an SM (measured: a third stage that still lets them does not pay), else as many (up to four) as one CTA fits.
@@ -695,9 +695,9 @@ unsigned gemm_splits(const ks_ctx* ctx, size_t rows, size_t cols, int n_tok) {
   return best;
 }
 typedef ks_gemm_blocks Blocks;
-Blocks gemm_blocks(int n_tok) { return {q4k_block(gemm_np(n_tok)), gemm_np(n_tok)}; }
-Blocks gemm_small_blocks(int n_tok) {
-  const unsigned tb = ((unsigned)n_tok + 63u) / 64u, tbn = (((unsigned)n_tok + tb - 1) / tb + 15u) / 16u * 16u;
+// Q4_K: the fewest blocks of at most `most` rows, all alike, a multiple of 16.
+Blocks gemm_blocks(int n_tok, unsigned most = 128u) {
+  const unsigned tb = ((unsigned)n_tok + most - 1u) / most, tbn = (((unsigned)n_tok + tb - 1) / tb + 15u) / 16u * 16u;
   return {tbn, tb * tbn};
 }
 ks_gemm_map gemm_map(const ks_ctx* ctx, ks_dtype wdtype, const size_t* rows, int n_seg, size_t cols, int n_tok, Blocks b, bool plain) {
@@ -714,8 +714,17 @@ ks_gemm_map gemm_map(const ks_ctx* ctx, ks_dtype wdtype, const size_t* rows, int
   m.splits = (ksteps + per - 1) / per;
   return m;
 }
+// The most partials a work tile of the launch leaves.
+unsigned map_slots(const ks_gemm_map& map, unsigned groups) {
+  unsigned slots = map.G ? 0 : map.splits;
+  for (unsigned w = 0; map.G && w < groups * map.tb; w++) {
+    const unsigned n = ks_gemm_owner(map, w * map.S + map.S - 1u) - ks_gemm_owner(map, w * map.S) + 1u;
+    slots = n > slots ? n : slots;
+  }
+  return slots;
+}
 bool gemm_covers(ks_dtype wdtype, size_t cols, int n_tok) {
-  return (wdtype == KS_Q4K || wdtype == KS_Q6K) && cols % 256 == 0 && n_tok >= 1 && n_tok <= 256;
+  return (wdtype == KS_Q4K || wdtype == KS_Q6K) && cols % 256 == 0 && n_tok >= 1 && n_tok <= (wdtype == KS_Q4K ? KS_GEMM_ROWS : 256);
 }
 }  // namespace
 
@@ -726,9 +735,10 @@ bool ks_gemm_few_rows_q6k(const ks_ctx* ctx, size_t rows, size_t cols) { return 
 // whole E2B layer of 256 rows took 142 us with wide blocks, 145 with the four small ones the bare estimate picks, 139 with this
 // line; of 128 rows 117 with wide blocks and 105 with small ones, of the tiny shape 87 and 60.
 ks_gemm_blocks ks_gemm_pick(const ks_ctx* ctx, ks_dtype wdtype, int n_seg, const size_t* rows, size_t cols, int n_tok, bool plain) {
+  if (wdtype != KS_Q4K) return {gemm_np(n_tok), gemm_np(n_tok)};
   const Blocks wide = gemm_blocks(n_tok);
-  if (wdtype != KS_Q4K || wide.tbn <= 64u) return wide;
-  const Blocks small = gemm_small_blocks(n_tok);
+  if (wide.tbn <= 64u) return wide;
+  const Blocks small = gemm_blocks(n_tok, 64u);
   double cw, cs;
   ks_gemm_q4k_map(ctx, rows, n_seg, (unsigned)cols, wide.np, wide.tbn, plain, &cw);
   ks_gemm_q4k_map(ctx, rows, n_seg, (unsigned)cols, small.np, small.tbn, plain, &cs);
@@ -740,13 +750,13 @@ bool ks_gemm_layers_cover(size_t hidden, size_t ffn, size_t q_cols) {
 
 // Bytes of the B image of n_tok rows of `cols` values (hi + lo halves, token count padded to 16).
 size_t ks_gemm_xt_bytes(size_t cols, int n_tok) {  // image + one factor per row, whatever the blocks
-  const size_t np = n_tok > 64 ? ((size_t)n_tok + 63) / 64 * 64 : gemm_np(n_tok);
+  const size_t np = n_tok > 128 ? ((size_t)n_tok + 127) / 128 * 128 : n_tok > 64 ? 128 : gemm_np(n_tok);
   return cols / 256 * 288 * np * 4 + np * 4;
 }
 
 // x[t * ldx + k] (f32) -> the B image in xt.
 int ks_launch_gemm_split(ks_ctx* ctx, ks_dtype wdtype, const float* x, size_t ldx, int n_tok, size_t cols, void* xt, ks_gemm_blocks b) {
-  if (cols % 256 || n_tok < 1 || n_tok > 256 || ldx % 4) return ks_fail(ctx, KS_ERR_INVALID, "gemm: bad operand shape");
+  if (cols % 256 || n_tok < 1 || n_tok > KS_GEMM_ROWS || ldx % 4) return ks_fail(ctx, KS_ERR_INVALID, "gemm: bad operand shape");
   KS_LAUNCH(ctx, (x_split_kernel), b.np, GM_ROW_THREADS, 0, x, ldx, (unsigned)n_tok, b.np, b.tbn, (unsigned)cols, (__half*)xt, (int)(wdtype == KS_Q4K));
   return ks_after_launch(ctx, "x_split");
 }
@@ -776,11 +786,7 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
     total_rows += rows[i];
   }
   tile0[3] = tiles;
-  unsigned slots = map.G ? 0 : map.splits;
-  for (unsigned w = 0; map.G && w < groups * map.tb; w++) {
-    const unsigned n = ks_gemm_owner(map, w * map.S + map.S - 1u) - ks_gemm_owner(map, w * map.S) + 1u;
-    slots = n > slots ? n : slots;
-  }
+  const unsigned slots = map_slots(map, groups);
   const bool direct = slots == 1 && mode == KS_GEMM_PLAIN;
   FinishArgs f{};
   float* out[3] = {nullptr, nullptr, nullptr};
@@ -930,22 +936,16 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
   return ks_after_launch(ctx, "gemm_finish");
 }
 
-// Floats of partials ks_launch_gemm_segs may write for up to three matrices of `total_rows` rows in all (either dtype).
-size_t ks_gemm_part_floats(const ks_ctx* ctx, size_t total_rows, size_t cols, int n_tok) {
-  unsigned slots = gemm_map(ctx, KS_Q6K, &total_rows, 1, cols, n_tok, gemm_blocks(n_tok), true).splits;
-  if (n_tok <= KS_GEMM_SKINNY) {
-    const unsigned n = ks_gemm_skinny_splits(ctx, total_rows, (unsigned)cols);
-    slots = n > slots ? n : slots;
+// Floats of partials ks_launch_gemm_segs writes for these matrices and token rows.
+size_t ks_gemm_part_floats(const ks_ctx* ctx, ks_dtype wdtype, int n_seg, const size_t* rows, size_t cols, int n_tok, bool plain) {
+  const ks_gemm_map m = gemm_map(ctx, wdtype, rows, n_seg, cols, n_tok, ks_gemm_pick(ctx, wdtype, n_seg, rows, cols, n_tok, plain), plain);
+  size_t total = 0;
+  unsigned groups = 0;
+  for (int i = 0; i < n_seg; i++) {
+    total += rows[i];
+    if (m.G) groups += (unsigned)(((rows[i] + GM_ROWS - 1) / GM_ROWS + m.nt - 1) / m.nt);
   }
-  const Blocks both[2] = {gemm_blocks(n_tok), n_tok > 64 ? gemm_small_blocks(n_tok) : gemm_blocks(n_tok)};
-  for (int extra = 0; extra < 20; extra++) {  // the matrices of a launch round their tiles up one by one; with and without an epilogue
-    const Blocks b = both[extra / 10];
-    const size_t r = total_rows + (size_t)(extra % 5) * GM_ROWS;
-    const ks_gemm_map m = ks_gemm_q4k_map(ctx, &r, 1, (unsigned)cols, b.np, b.tbn, extra % 10 >= 5);
-    const unsigned n = (m.S + m.base - 1) / m.base + 1;  // a CTA has at least `base` units, a work tile may begin inside one
-    slots = n > slots ? n : slots;
-  }
-  return (size_t)slots * (size_t)n_tok * total_rows;
+  return (size_t)map_slots(m, groups) * (size_t)n_tok * total;
 }
 
 // Scratch of ks_launch_gemm_kq: the image and the partials of that one launch.

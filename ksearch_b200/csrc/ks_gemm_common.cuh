@@ -63,7 +63,6 @@ __device__ __forceinline__ void split8(const float (&w)[8], uint4& hi, uint4& lo
 //                          sub-block sums the minima multiply: chunk 32 + g holds, with S = 2^-5 (sum of a 32-value
 //                          sub-block), (S_hi, S_hi', S_lo, S_lo', S_hi, S_hi', 0, 0) of sub-blocks 2 g and 2 g + 1.
 //                          Token rows come in blocks of `tbn`, each an image like this of its own, one behind the other.
-__device__ __host__ __forceinline__ unsigned q4k_block(unsigned np) { return np > 128u ? np / 2u : np; }  // the widest blocks
 __device__ __forceinline__ void put_split8(__half* xt, unsigned np, unsigned tbn, unsigned t, unsigned ck, unsigned chunks, const float (&v)[8], bool q4k) {
   unsigned at = ck;
   if (q4k) {

@@ -55,6 +55,7 @@ struct __align__(64) Q4Args {
   const __half* xt;        // the q4k form of the B image
   unsigned cols, n_tok, np;
   unsigned n_raw, n_b;     // ring depths
+  unsigned head;           // bytes in front of the rings: barriers, scale factors, wide: s of the last tiles' rows
   unsigned wait_limit, test_stall;
   unsigned* err;
 };
@@ -62,8 +63,8 @@ struct __align__(64) Q4Args {
 // barriers (8 bytes each) at the start of shared memory
 enum { QB_RAW_FULL = 0, QB_RAW_FREE = QB_RAW_FULL + Q_MAX_RAW, QB_B_FULL = QB_RAW_FREE + Q_MAX_RAW, QB_B_FREE = QB_B_FULL + Q_MAX_B,
        QB_A_FULL = QB_B_FREE + Q_MAX_B, QB_A_FREE = QB_A_FULL + 3, QB_D_FULL = QB_A_FREE + 3, QB_D_FREE = QB_D_FULL + 2, QB_DONE = QB_D_FREE + 2,
-       QB_COUNT };
-constexpr unsigned Q_HEAD = 2048;  // barriers, then from 512 the token rows' scale factors
+       QB_UP, QB_COUNT };
+constexpr unsigned Q_HEAD = 512;  // barriers; behind them the token rows' scale factors
 static_assert(QB_COUNT * 8 + 16 <= 512, "barriers fit the head of shared memory");
 
 __device__ __forceinline__ void mb_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
@@ -173,8 +174,8 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_
   constexpr unsigned Q_D = 224;                     // first accumulator
   const unsigned tbn = a.map.tbn;                   // token rows of a unit
   const unsigned b_group = 4u * 2u * tbn * 16u, b_stage = 9u * b_group;
-  float* up_s = reinterpret_cast<float*>(smem + 512);   // 2^e of every token row
-  const uint32_t raw0 = bars + Q_HEAD, b0 = raw0 + a.n_raw * Q_RAW;
+  float* up_s = reinterpret_cast<float*>(smem + Q_HEAD);   // 2^e of every token row
+  const uint32_t raw0 = bars + a.head, b0 = raw0 + a.n_raw * Q_RAW;
   const unsigned u0 = ks_gemm_first(a.map, blockIdx.x), n_units = a.map.base + (blockIdx.x < a.map.rem ? 1u : 0u);
 
   if (threadIdx.x == 0) {
@@ -195,6 +196,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_
       mb_init(bar(QB_D_FREE + i), Q_WARPS);
     }
     mb_init(bar(QB_DONE), 1);
+    mb_init(bar(QB_UP), 1);
     *fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -299,6 +301,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_
           const unsigned pslot = blockIdx.x - ks_gemm_owner(a.map, prev_wt * a.map.S);
           float* y = sg.y + (size_t)pslot * sg.part + out_row;
           const bool live = out_row < sg.rows;
+          if (!__all_sync(0xffffffffu, mb_wait(bar(QB_UP), 0u, a.wait_limit))) { ok = false; break; }
 #pragma unroll
           for (int k = 0; k < TQ; k++) {
             const unsigned tok = tok0 + k;
@@ -411,7 +414,10 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_
     const unsigned leader = elect_one();
     asm volatile("griddepcontrol.wait;" ::: "memory");  // the image comes from the kernel before this one
     const float* up = reinterpret_cast<const float*>(a.xt + xt_scale_off(a.cols, a.np));
-    for (unsigned t = lane; t < a.np; t += 32u) up_s[t] = up[t];  // read behind the first accumulator, which waits for the copies below
+    if (leader) {
+      mb_expect(bar(QB_UP), a.np * 4u);  // np: a multiple of 16
+      bulk_in(sm32(up_s), up, a.np * 4u, bar(QB_UP));
+    }
     __syncwarp();
     unsigned issued = 0, wt = u0 / a.map.S, sb = u0 - wt * a.map.S, st = 0, ph = 1;
     for (unsigned j = 0; j < n_units; j++) {  // a super-block each
@@ -438,6 +444,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_
       __syncwarp();
     }
     for (unsigned j = issued > a.n_b ? issued - a.n_b : 0u; j < issued; j++) mb_wait(bar(QB_B_FULL + j % a.n_b), (j / a.n_b) & 1u, a.wait_limit);
+    mb_wait(bar(QB_UP), 0u, a.wait_limit);
   }
   tc_fence_before();
   __syncthreads();
@@ -454,7 +461,7 @@ __global__ void __launch_bounds__(Q_THREADS, 1) gemm_q4k_tc_kernel(const __grid_
 // accumulator whose folders stood before a slot of A (13.4k cycles per unit, MMAs 4.5k).  Eight warps convert (32 rows x 128 k
 // each), eight fold (32 rows x half the tokens of both tiles: 128 sums per thread, hence the register split 56 / 168 / 32 of the
 // 96 a thread is launched with).
-constexpr unsigned QW_THREADS = 640, QW_HEAD = 4096;  // 5 groups of 4 warps; barriers, from 512 the scale factors, from 1536 s
+constexpr unsigned QW_THREADS = 640;  // 5 groups of 4 warps
 constexpr unsigned QW_D = 256;
 __global__ void __launch_bounds__(QW_THREADS, 1) gemm_q4k_wide_kernel(const __grid_constant__ Q4Args a) {
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -465,9 +472,9 @@ __global__ void __launch_bounds__(QW_THREADS, 1) gemm_q4k_wide_kernel(const __gr
   const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
   const unsigned tbn = a.map.tbn;
   const unsigned b_group = 4u * 2u * tbn * 16u, b_stage = 5u * b_group;
-  float* up_s = reinterpret_cast<float*>(smem + 512);    // 2^e of every token row
-  float* s_s = reinterpret_cast<float*>(smem + 1536);    // [4][128]: s of the rows of the last tiles, converters to folders
-  const uint32_t raw0 = bars + QW_HEAD, b0 = raw0 + a.n_raw * Q_RAW;
+  float* s_s = reinterpret_cast<float*>(smem + Q_HEAD);    // [4][128]: s of the rows of the last tiles, converters to folders
+  float* up_s = s_s + 4 * GM_ROWS;                         // 2^e of every token row
+  const uint32_t raw0 = bars + a.head, b0 = raw0 + a.n_raw * Q_RAW;
   const unsigned u0 = ks_gemm_first(a.map, blockIdx.x), n_units = a.map.base + (blockIdx.x < a.map.rem ? 1u : 0u);
 
   if (threadIdx.x == 0) {
@@ -488,6 +495,7 @@ __global__ void __launch_bounds__(QW_THREADS, 1) gemm_q4k_wide_kernel(const __gr
       mb_init(bar(QB_D_FREE + i), 8);
     }
     mb_init(bar(QB_DONE), 1);
+    mb_init(bar(QB_UP), 1);
     *fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -598,6 +606,7 @@ __global__ void __launch_bounds__(QW_THREADS, 1) gemm_q4k_wide_kernel(const __gr
           const unsigned pslot = blockIdx.x - ks_gemm_owner(a.map, wt * a.map.S);
           float* y = sg.y + (size_t)pslot * sg.part + (size_t)tok0 * sg.ldy + out_row;
           const unsigned n_tok = out_row < sg.rows ? a.n_tok : 0u;
+          if (!__all_sync(0xffffffffu, mb_wait(bar(QB_UP), 0u, a.wait_limit))) { ok = false; break; }
 #pragma unroll
           for (int k = 0; k < 64; k++) {
             if ((unsigned)k < tq && tok0 + k < n_tok) *y = acc[t][k] * up_s[tok0 + k];
@@ -711,7 +720,10 @@ __global__ void __launch_bounds__(QW_THREADS, 1) gemm_q4k_wide_kernel(const __gr
     const unsigned leader = elect_one();
     asm volatile("griddepcontrol.wait;" ::: "memory");  // the image comes from the kernel before this one
     const float* up = reinterpret_cast<const float*>(a.xt + xt_scale_off(a.cols, a.np));
-    for (unsigned t = lane; t < a.np; t += 32u) up_s[t] = up[t];  // read behind the first accumulator, which waits for the copies below
+    if (leader) {
+      mb_expect(bar(QB_UP), a.np * 4u);  // np: a multiple of 16
+      bulk_in(sm32(up_s), up, a.np * 4u, bar(QB_UP));
+    }
     __syncwarp();
     unsigned issued = 0, wt = u0 / a.map.S, sb = u0 - wt * a.map.S, hf = 0, st = 0, ph = 1;
     for (unsigned j = 0; j < 2u * n_units; j++) {  // halves of a super-block: 4 and 5 groups
@@ -742,6 +754,7 @@ __global__ void __launch_bounds__(QW_THREADS, 1) gemm_q4k_wide_kernel(const __gr
       __syncwarp();
     }
     for (unsigned j = issued > a.n_b ? issued - a.n_b : 0u; j < issued; j++) mb_wait(bar(QB_B_FULL + j % a.n_b), (j / a.n_b) & 1u, a.wait_limit);
+    mb_wait(bar(QB_UP), 0u, a.wait_limit);
     }
   }
   tc_fence_before();
@@ -765,15 +778,17 @@ encode_fn tensor_map_encoder() {
 
 // Ring depths: two B stages at least, then packed rows up to the four units that cover the latency of memory, then whatever
 // of either still fits.
-size_t q4_rings(const ks_ctx* ctx, unsigned tbn, unsigned nt, unsigned* n_raw, unsigned* n_b) {
-  const size_t head = nt == 1 ? Q_HEAD : QW_HEAD, room = ctx->smem_optin - head, stage = (size_t)(nt == 1 ? 9 : 5) * tbn * 128u;
-  *n_raw = 2;
-  *n_b = 2;
+size_t q4_rings(const ks_ctx* ctx, unsigned tbn, unsigned nt, unsigned np, Q4Args& a) {
+  a.head = (Q_HEAD + (nt == 1 ? 0u : 4u * GM_ROWS * 4u) + np * 4u + 1023u) & ~1023u;
+  const size_t room = ctx->smem_optin - a.head, stage = (size_t)(nt == 1 ? 9 : 5) * tbn * 128u;
+  unsigned n_raw = 2, n_b = 2;
   auto fits = [&](unsigned r, unsigned b) { return r <= Q_MAX_RAW && b <= Q_MAX_B && b * stage + r * Q_RAW <= room; };
-  while (*n_raw < 4 && fits(*n_raw + 1, *n_b)) ++*n_raw;
-  while (fits(*n_raw, *n_b + 1)) ++*n_b;
-  while (fits(*n_raw + 1, *n_b)) ++*n_raw;
-  return head + *n_b * stage + *n_raw * Q_RAW;
+  while (n_raw < 4 && fits(n_raw + 1, n_b)) ++n_raw;
+  while (fits(n_raw, n_b + 1)) ++n_b;
+  while (fits(n_raw + 1, n_b)) ++n_raw;
+  a.n_raw = n_raw;
+  a.n_b = n_b;
+  return a.head + n_b * stage + n_raw * Q_RAW;
 }
 }  // namespace
 
@@ -850,7 +865,7 @@ int ks_launch_gemm_q4k(ks_ctx* ctx, const ks_gemm_job& job) {
   a.np = job.np;
   const unsigned tbn = job.map.tbn;
   const int c = tbn <= 16 ? 0 : tbn <= 32 ? 1 : tbn <= 64 ? 2 : 3;
-  const size_t smem = q4_rings(ctx, job.map.tbn, job.map.nt, &a.n_raw, &a.n_b);
+  const size_t smem = q4_rings(ctx, job.map.tbn, job.map.nt, job.np, a);
   a.err = (unsigned*)ctx->ws + KS_WS_ERR_WORD;
   a.wait_limit = Q_WAIT;
   if (const char* t = getenv("KSEARCH_GEMM_TEST_STALL")) {  // exercises the give-up path: short waits, one operand withheld

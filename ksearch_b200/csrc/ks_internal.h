@@ -188,20 +188,21 @@ uint32_t ks_sample_candidates(const ks_cand* c, size_t n, size_t n_all, float ca
 // ---- tensor-core GEMM for batches of token rows (ks_gemm.cu) -----------------------------------------
 // nelem (a multiple of 256) elements of src (Q6K, Q4K, F16, F32) -> Q4_K blocks, as the reference's load-time quantizer.
 int ks_launch_quantize_q4k(ks_ctx* ctx, ks_dtype src_dtype, const void* src, size_t nelem, void* dst);
+constexpr int KS_GEMM_ROWS = 2048;  // token rows of one launch, Q4_K weights (Q6_K: 256)
 size_t ks_gemm_xt_bytes(size_t cols, int n_tok);  // bytes of the split image of n_tok rows of `cols` values
-size_t ks_gemm_part_floats(const ks_ctx* ctx, size_t total_rows, size_t cols, int n_tok);  // k-split partials, at most
 // The context's scratch, grown to `bytes` (fails inside a stream capture when it would have to grow).  Batches of 2..8 rows never
 // grow it: KS_FEW_WS holds their image (4.7 MB at 65536 columns) and partials (8 rows of 262144 outputs: 8 MB a share).
 constexpr size_t KS_FEW_WS = 32u << 20;
 int ks_ctx_gemm_scratch(ks_ctx* ctx, size_t bytes, void** out);
 // The blocks a launch over these matrices wants (`plain`: nothing is done to its sums).
 ks_gemm_blocks ks_gemm_pick(const ks_ctx* ctx, ks_dtype wdtype, int n_seg, const size_t* rows, size_t cols, int n_tok, bool plain);
+size_t ks_gemm_part_floats(const ks_ctx* ctx, ks_dtype wdtype, int n_seg, const size_t* rows, size_t cols, int n_tok, bool plain);  // its partials
 // x[t * ldx + k] (f32) -> the image the GEMM over weights of that dtype reads its token rows from.
 int ks_launch_gemm_split(ks_ctx* ctx, ks_dtype wdtype, const float* x, size_t ldx, int n_tok, size_t cols, void* xt, ks_gemm_blocks b);
 // Up to three matrices over the same columns and token rows (q, k, v; gate, up) in one launch.  What becomes of
 // the sums: PLAIN y[i] = W[i] x; NORM_SPLIT (one matrix)
 // out_x = res + rms(W x) * w_post and the image of rms(out_x) * w_norm for the next GEMM in xt_out; GELU_SPLIT
-// (two matrices) the image of gelu(W[0] x) * (W[1] x) in xt_out.  P: ks_gemm_part_floats(sum of rows) floats.
+// (two matrices) the image of gelu(W[0] x) * (W[1] x) in xt_out.  P: ks_gemm_part_floats floats.
 // QKV (three matrices): per-head norm and RoPE of q into out_x, of k and v into the cache rows (Q4_0).
 enum { KS_GEMM_PLAIN, KS_GEMM_NORM_SPLIT, KS_GEMM_GELU_SPLIT, KS_GEMM_QKV };
 struct ks_gemm_epi {
@@ -221,8 +222,7 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
                         int n_tok, float* const* y, const size_t* ldy, float* P, int mode, const ks_gemm_epi* epi, ks_gemm_blocks b);
 // Do the epilogues take every matrix of a layer of these widths?
 bool ks_gemm_layers_cover(size_t hidden, size_t ffn, size_t q_cols);
-// Split + GEMM for one matrix.  Returns 1 when the shape is not covered (cols not a multiple of 256, more than
-// 256 rows).  scratch: ks_gemm_kq_bytes.
+// Split + GEMM for one matrix.  Returns 1 when the shape is not covered (cols not a multiple of 256, too many rows).  scratch: ks_gemm_kq_bytes.
 size_t ks_gemm_kq_bytes(const ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_t cols, int n_tok);
 int ks_launch_gemm_kq(ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_t cols, const uint8_t* W, const float* x, size_t ldx, float* y,
                       size_t ldy, int n_tok, void* scratch);

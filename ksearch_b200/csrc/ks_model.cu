@@ -82,7 +82,7 @@ __global__ void set_state_kernel(int slot, int pos_value, int* pos) { ks_pdl_ent
 // A prompt chunk: row t of the chunk sits at position base + t of ONE slot (causal: it sees base + t + 1 positions).
 __global__ void begin_chunk_kernel(int n, const int* base, int* cpos, float* meta, float* meta_swa, int window) {
   ks_pdl_entry();
-  const int t = threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < n) {
     cpos[t] = base[0] + t;
     write_meta_pair(meta, meta_swa, t, base[0] + t + 1, window);
@@ -194,8 +194,11 @@ int dev_alloc(ks_model* m, void** p, size_t bytes) {
 }
 
 constexpr int KS_PREFILL_CHUNK = 8;  // tokens per pass over the weights (the matvec kernels take up to 8)
-constexpr int KS_GEMM_CHUNK = 256;   // rows per pass when the tensor-core GEMM takes the matrices
-constexpr size_t KS_STAGE_IDS = 256; // pinned words that stage host token ids
+// Rows per pass when the tensor-core GEMM takes the matrices.  A layer of 256 rows is a chain of ten launches of 6 to 31 us that
+// leave most of the chip idle; prompts of 2047 rows E2B / 4000 rows E4B / 776 rows E2B with a window, by rows per pass:
+// 256: 41.8 / 163 / 16.3 ms, 512: 32.6 / 136 / 12.6, 1024: 30.9 / 127 / 11.1, 2048: 24.7 / 112 / 11.1.
+constexpr int KS_GEMM_CHUNK = KS_GEMM_ROWS;
+constexpr size_t KS_STAGE_IDS = KS_GEMM_CHUNK; // pinned words that stage host token ids
 
 // Do the rows of a prompt chunk share one pass over their context (ks_sdpa_chunk.cu: 64 rows x heads a block, few blocks), or does
 // each take the decode kernel (a block per row and up to four heads, spread over the chip)?  By the work of the second form:
@@ -286,7 +289,7 @@ unsigned row_threads(int n) { return (unsigned)((n + 1 + 31) / 32 * 32); }  // o
 
 int lane_begin(ks_model* m, const Lane& L, int n) {
   if (L.chunk_base)
-    KS_LAUNCH(m->ctx, (begin_chunk_kernel), 1, row_threads(n), 0, n, (const int*)L.chunk_base, L.pos, L.meta, L.meta_swa, (int)m->cfg.sliding_window);
+    KS_LAUNCH(m->ctx, (begin_chunk_kernel), (unsigned)(n + 255) / 256u, 256, 0, n, (const int*)L.chunk_base, L.pos, L.meta, L.meta_swa, (int)m->cfg.sliding_window);
   else
     KS_LAUNCH(m->ctx, (begin_token_kernel), 1, row_threads(n), 0, n, (const int*)L.pos, L.meta, L.meta_swa, (int)m->cfg.sliding_window);
   return ks_after_launch(m->ctx, "begin_token");
@@ -846,18 +849,20 @@ ks_model* ks_model_create(ks_ctx* ctx, const ks_model_config* cfg) {
     // widths its epilogues take: larger batches go through the tensor-core GEMM, which computes in f32 (a chunk of an f16 model
     // too: its rows meet f16 vectors nowhere); wider models keep the batch matvec for every batch
     if (ks_gemm_layers_cover(H, F, qn) && !getenv("KSEARCH_NO_GEMM")) {
-      const int G = KS_GEMM_CHUNK;
+      // no prompt is longer than the cache; decode steps bring a row per slot
+      const int cap = (g.max_seq + 127) / 128 * 128, G = cap < KS_GEMM_CHUNK ? (cap > 256 ? cap : 256) : KS_GEMM_CHUNK;
       m->gemm_chunk = G;
       // one launch each: q|k|v, o, gate|up, down, head
-      const size_t rows_of[5] = {qn + 2 * kvn, H, 2 * F, H, (size_t)g.vocab}, cols_of[5] = {H, qn, H, F, H};
+      const size_t rows_of[5][3] = {{qn, kvn, kvn}, {H}, {F, F}, {H}, {(size_t)g.vocab}}, cols_of[5] = {H, qn, H, F, H};
+      const int segs_of[5] = {3, 1, 2, 1, 1};
       size_t xt = 0, part = 0;
       for (int i = 0; i < 5; i++) {
         const int most = i < 4 ? G : g.n_slots;  // only decode steps reach the head
         const size_t a = ks_gemm_xt_bytes(cols_of[i], most);
         xt = a > xt ? a : xt;
-        for (int n = 8; n < most + 16; n += n < 16 ? 8 : 16) {  // fewer rows are split finer, up to 8 take a kernel of their own
-          const int rows = n < most ? n : most;
-          const size_t b = 4 * ks_gemm_part_floats(ctx, rows_of[i], cols_of[i], rows);
+        // the work is dealt alike for all counts that pad to the same multiple of 16; up to 8 rows take a kernel of their own
+        for (int n = 8; n < most + 16; n += n < 16 ? 8 : 16) {
+          const size_t b = 4 * ks_gemm_part_floats(ctx, i < 4 ? KS_Q4K : (ks_dtype)g.embd_dtype, segs_of[i], rows_of[i], cols_of[i], n < most ? n : most, i == 4);
           part = b > part ? b : part;
         }
       }
@@ -891,7 +896,14 @@ ks_model* ks_model_create(ks_ctx* ctx, const ks_model_config* cfg) {
   if (ok) {
     m->n_splits = ks_sdpa_pick_splits(ctx, 1, g.n_kv, g.max_seq);
     const size_t C = m->gemm_chunk > KS_PREFILL_CHUNK ? m->gemm_chunk : KS_PREFILL_CHUNK;
-    ok = dev_alloc(m, (void**)&m->cattn_tmp, (C * g.n_q * (size_t)m->n_splits * (g.hd + 2) + 4) * sizeof(float)) == KS_OK;
+    // records of a chunk's rows: fewer splits a row, the more rows there are
+    size_t recs = 0;
+    for (size_t n = 1; n <= C; n++) {
+      const int a = att_splits_for(m, (int)n), b = ks_sdpa_chunk_splits(ctx, (int)n, g.n_q, g.n_kv, (size_t)g.max_seq, m->n_splits);
+      const size_t r = n * (size_t)(a > b ? a : b);
+      recs = r > recs ? r : recs;
+    }
+    ok = dev_alloc(m, (void**)&m->cattn_tmp, (recs * g.n_q * (g.hd + 2) + 4) * sizeof(float)) == KS_OK;
   }
   if (ok) {
     ok = dev_alloc(m, (void**)&m->attn_tmp, (S * g.n_q * (size_t)m->n_splits * (g.hd + 2) + 4) * sizeof(float)) == KS_OK;
@@ -922,7 +934,7 @@ ks_model* ks_model_create(ks_ctx* ctx, const ks_model_config* cfg) {
     ok = false;
   }
   if (m->host_ret) memset(m->host_ret, 0, ((size_t)g.n_slots + 4) * sizeof(float));
-  m->host_tok_n = 8192;
+  m->host_tok_n = 8192 - 256 + KS_STAGE_IDS;  // read-back words of a generate call and the staged prompt ids
   if (ok && cudaMallocHost((void**)&m->host_tok, m->host_tok_n * sizeof(float)) != cudaSuccess) {
     ks_fail(ctx, KS_ERR_OOM, "model_create: pinned allocation failed");
     ok = false;

@@ -1,4 +1,4 @@
-// Attention of a prompt chunk: up to 256 token rows of one slot against its Q4_0 cache, causal (and windowed) by row.
+// Attention of a prompt chunk: many token rows of one slot against its Q4_0 cache, causal (and windowed) by row.
 //
 // The reference runs its decode attention once per prompt row (forward_prefill_chunk, crates/ksearch_gemma/src/
 // gemma_prim.rs:1463-1472, over crates/ksearch_codegen/src/lower.rs:4897-6088), so every row reads the whole context again.
@@ -83,7 +83,8 @@ sdpa_chunk_kernel(unsigned n_tok, unsigned n_q, unsigned n_kv, float scale, cons
   extern __shared__ __align__(128) unsigned char smem[];
   ks_pdl_entry();
   const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, rg = warp >> 1, h = warp & 1u;
-  const unsigned G = n_q / n_kv, kvh = blockIdx.y, split = blockIdx.z, row0 = blockIdx.x * CH_BM;
+  const unsigned G = n_q / n_kv, kvh = blockIdx.y, split = blockIdx.z;
+  const unsigned row0 = (gridDim.x - 1u - blockIdx.x) * CH_BM;  // the last rows see the most: they start first
   const uint32_t sb = sm32(smem);
   float* row_scale = reinterpret_cast<float*>(smem + S::row);
   int* row_first = reinterpret_cast<int*>(smem + S::row + CH_BM * 4);

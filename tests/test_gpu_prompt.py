@@ -1,0 +1,38 @@
+"""Prompt chunks of up to 2048 rows against the same prompt in short pieces."""
+import numpy as np
+import pytest
+
+from ksearch_b200 import synth
+from ksearch_b200 import model as ksm
+
+pytestmark = pytest.mark.gpu
+
+
+def _logits_after(model, ctx, pieces, last):
+    model.slot_reset(0)
+    for p in pieces:
+        model.prefill(0, p)
+    model.forward(0, 1, [int(last)], True)
+    ctx.synchronize()
+    return model.read_debug(1, 0).astype(np.float64)
+
+
+@pytest.mark.parametrize("window", [0, 100])
+@pytest.mark.parametrize("n_kv", [1, 2])
+def test_long_chunks_equal_short_pieces(ctx, n_kv, window):
+    """One call with the whole prompt (chunks of up to 2048 rows: many blocks of token rows a launch, the rest behind a full
+    chunk) and calls of 200 rows, which tests/test_gpu_model.py holds to the CPU decoder, leave the same cache: the next
+    token's logits agree to the bound of those tests."""
+    cfg = ksm.tiny_config(max_seq=2432, n_kv=n_kv)
+    if window:
+        cfg.sliding_window, cfg.swa_layers = window, 0b101
+    model, _ = ksm.GemmaCudaModel.synthetic(ctx, cfg, seed=41, keep=True)
+    model.slot_alloc()
+    for n in (257, 640, 1025, 2047, 2048, 2049, 2051, 2400):
+        toks = [int(t) for t in synth.token_ids(41, f"p{n}", n + 1, cfg.vocab)]
+        want = _logits_after(model, ctx, [toks[i:min(i + 200, n)] for i in range(0, n, 200)], toks[n])
+        got = _logits_after(model, ctx, [toks[:n]], toks[n])
+        assert model.seq_len(0) == n + 1
+        scale, err = np.abs(want).max(), np.abs(got - want)
+        assert err.max() <= 1e-3 * scale and np.sqrt((err ** 2).mean()) <= 1e-4 * scale, n
+    model.close()
