@@ -5,20 +5,28 @@
 // chain of ~180 dependent steps, each a few hundred kilobytes to ten megabytes of weights, and a
 // kernel boundary costs more than most of those steps take.  Here one block per SM stays resident
 // for the whole token:
-//   * the weight stream never stops: every warp owns a ring of shared-memory stages fed by
-//     cp.async.bulk, and walks ONE item list for the whole token (all its row groups of all phases);
-//     the copies of the next phases are already in flight while the block waits at a barrier;
+//   * the weight stream never stops: one warp copies the block's row groups of all phases, in the order they are
+//     needed, into a ring in shared memory (cp.async.bulk, one mbarrier per row group); the next phases' groups are
+//     already there while the block waits at a barrier.  Fifteen other warps multiply: an item is a row group's share
+//     of the columns, so a group is split over as many warps as that evens out;
 //   * phases (qkv | attention | o-proj | gate-up | down, per layer) are separated by a grid barrier
 //     on one global counter; activations cross it through global memory (L2), read with ld.cg;
 //     one hop has no barrier: q/k/v go to the attention blocks as 64-bit (value, tag) words written
 //     with relaxed stores and polled by their consumers (a hop of ~1 us instead of ~2 us);
-//   * the norms are applied while x is staged; their weights are fetched BEFORE the barrier wait,
-//     because the acquire that ends the wait drops the SM's L1 and every later plain load of a
-//     constant would be a full round trip to L2;
+//   * the norms are applied while x is staged; their weights come through the ring as well, because the acquire that
+//     ends a wait drops the SM's L1 and every later plain load of a constant would be a full round trip to L2 (for the
+//     same reason nothing may be spilled: local memory lives in L1);
 //   * for the same reason nothing on the critical path reads a descriptor from global memory: the
 //     five phase shapes and the per-layer pointers are copied to shared memory once;
 //   * attention: per-head RMS + RoPE + Q4_0 pack of the new K/V row, split-context online softmax
-//     and the merge of the splits (last arriving block) happen inside one phase.
+//     and, for long contexts, the merge of the splits (last arriving block) happen inside one phase; a few splits are merged
+//     by whoever stages them.
+// Bound by the chain: a layer of the E2B shape is 25.5 us (32.5 before the copying warp, with eight warps of 242 registers), its
+// weights 3 us of HBM.  Microseconds at 100 positions, E2B, before / now: q|k|v 4.8 / 3.8, attention 10.9 / 5.1, o 4.1 / 5.1,
+// gate|up 7.7 / 5.9, down 5.1 / 5.7; E4B at 4000 positions: 6.0 / 5.1, 25.4 / 12.3, 4.7 / 4.4, 16.4 / 10.2, 8.6 / 9.2.  A phase
+// is 1 to 2 us of waiting (barrier and slower blocks), 0.8 to 2 of staging, the rest multiplication.  Fifteen warps instead of
+// eight, row groups dealt one by one instead of in runs of eight (a block had up to 64 gate|up rows where 42 is the mean) and no
+// register spilled are what they owe it to: arrays left undefined in some lanes stayed live around the phase loop and spilled.
 // Every spin (barrier, tagged word, mbarrier) is bounded; on expiry the block raises the context's status word,
 // drains its copies and leaves, and the other blocks time out the same way.
 #include <utility>
@@ -31,14 +39,17 @@ namespace {
 enum { MG_MATVEC = 0, MG_GATE_UP = 1, MG_ATTN = 2 };
 enum { PH_QKV = 0, PH_ATTN = 1, PH_OPROJ = 2, PH_GATEUP = 3, PH_DOWN = 4, PH_PER_LAYER = 5 };
 
+constexpr unsigned MG_WARPS = 15, MG_THREADS = MG_WARPS * 32;  // that multiply; a sixteenth warp copies
+constexpr unsigned MG_JOBS = 64;                               // row groups in the ring at a time, at most (a power of two)
+constexpr unsigned MG_EMPTY = 1024;                            // arrivals that free one: its items' shares add up to this
+
 struct MegaShape {          // one of the five phases of a layer; the same for every layer
   int type;
   int n_seg;                // matvec: 1 or 3 (q, k, v)
   unsigned rows[3];
   unsigned grp_start[4];    // first group of each segment, [n_seg] = total groups (0 for attention)
   unsigned cols, row_bytes, seg_blocks, n_cseg;
-  int oct;                  // 1: a block owns runs of 8 consecutive groups (32 rows = one sub-block of the next phase's x)
-  int split;                // gate-up only, 1: the gate rows and the up rows of a group are two items (rows too long for one slot)
+  unsigned mats, w0;        // matrices of a group (2: gate and up), MegaLayer::W index of the first segment's
 };
 
 struct MegaLayer {          // per-layer pointers, copied to shared memory when the kernel starts
@@ -52,17 +63,17 @@ struct MegaArgs {
   const void* tables;       // MegaShape[5] then MegaLayer[n_layers], 16-byte aligned; copied to shared memory at start
   unsigned tables_bytes;    // multiple of 16
   int n_layers;
-  int stages;               // ring slots per warp
-  unsigned slot_bytes;      // bytes per ring slot
-  unsigned x_bytes;         // staging area for x (also the attention scratch)
+  unsigned ring_bytes;
+  unsigned x_off, ring_off; // shared memory: staging area for x (also the attention scratch), the ring
   unsigned n_q, n_kv, hd, n_splits;
   float eps, attn_scale;
   const float* rope;        // [max_seq, hd]
   const int* pos;           // [1]
   float *x_a, *x_b;         // residual stream: layers read x_a / write x_b at the FFN, the reverse at the next qkv
   float* yb;
-  unsigned char *ox, *ffx;  // attention output and GeGLU output, written by their producers in the staged fixed-point layout
-  float* att_tmp;           // [n_q * n_splits * (hd + 2)]
+  unsigned char* ox;        // merged attention output, written in the staged fixed-point layout
+  float* ff;                // GeGLU output
+  float* att_tmp;           // [n_q][n_splits] records
   float4* nsum;             // [grid] per-block sums of the last o-proj / down phase: (sum y^2, sum x*y*wp, sum (y*wp)^2, sum x^2)
   unsigned* att_cnt;        // [n_q] arrival counters of the attention blocks, per head
   unsigned* bar;            // [0] running barrier counter, [1] its value when the previous token ended
@@ -83,7 +94,7 @@ __device__ __forceinline__ void mb_expect(uint32_t bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ bool mb_wait(uint32_t bar, unsigned parity) {
-  for (unsigned i = 0; i < (1u << 22); i++) {
+  for (unsigned i = 0; i < (1u << 21); i++) {
     unsigned ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -117,33 +128,46 @@ __device__ __forceinline__ unsigned long long tag_load(const unsigned long long*
   asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
   return w;
 }
-// Four tagged words per lane until every tag matches; false when the limit ran out.
-__device__ __forceinline__ bool tag_wait4(const unsigned long long* base, int i0, int i1, int i2, int i3, unsigned tag, unsigned limit,
-                                          float& o0, float& o1, float& o2, float& o3) {
+// Tagged words p[i], i = at[0..N), per lane until every tag matches; false when the limit ran out.
+template <int N>
+__device__ __forceinline__ bool tag_wait(const unsigned long long* p, const int (&at)[N], unsigned tag, unsigned limit, float (&v)[N]) {
   for (unsigned it = 0; it < limit; it++) {
-    const unsigned long long w0 = tag_load(base + i0), w1 = tag_load(base + i1), w2 = tag_load(base + i2), w3 = tag_load(base + i3);
-    if ((unsigned)(w0 >> 32) == tag && (unsigned)(w1 >> 32) == tag && (unsigned)(w2 >> 32) == tag && (unsigned)(w3 >> 32) == tag) {
-      o0 = __uint_as_float((unsigned)w0);
-      o1 = __uint_as_float((unsigned)w1);
-      o2 = __uint_as_float((unsigned)w2);
-      o3 = __uint_as_float((unsigned)w3);
-      return true;
+    unsigned long long w[N];
+    unsigned bad = 0;
+#pragma unroll
+    for (int j = 0; j < N; j++) w[j] = tag_load(p + at[j]);
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+      bad |= (unsigned)(w[j] >> 32) ^ tag;
+      v[j] = __uint_as_float((unsigned)w[j]);
     }
+    if (bad == 0) return true;
   }
-  o0 = o1 = o2 = o3 = 0.0f;
+#pragma unroll
+  for (int j = 0; j < N; j++) v[j] = 0.0f;
   return false;
 }
 
+// The thread's index, read anew: what is computed from it stays where it is used.  Hoisted out of the phase loop, the addresses and
+// predicates of all phases together do not fit the registers, and a spilled one comes back from L2.
+__device__ __forceinline__ unsigned mg_tid() {
+  unsigned t;
+  asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+  return t;
+}
+// The warps that multiply; the copying warp never joins them.
+__device__ __forceinline__ void cta_sync() { asm volatile("bar.sync 1, %0;" ::"n"(MG_THREADS) : "memory"); }
+
 // Grid-wide barrier on a monotonically increasing counter, in two halves so that loads which do not
 // depend on other blocks can be issued in between.
-// wsum != nullptr: the eight warps left their partial norm sums there; thread 0 folds them (fixed order) into nsum[block].
-__device__ __forceinline__ void grid_arrive(unsigned* counter, const float4* wsum, float4* nsum) {
-  __syncthreads();  // every store of this block is issued
-  if (threadIdx.x == 0) {
-    if (wsum) {
+// n_wsum: that many warps left partial norm sums in wsum; thread 0 folds them (fixed order) into nsum[block].
+__device__ __forceinline__ void grid_arrive(unsigned* counter, const float4* wsum, unsigned n_wsum, float4* nsum) {
+  const unsigned tid = mg_tid();
+  cta_sync();  // every store of this block is issued
+  if (tid == 0) {
+    if (n_wsum) {
       float4 t = wsum[0];
-#pragma unroll
-      for (int w = 1; w < 8; w++) {
+      for (unsigned w = 1; w < n_wsum; w++) {
         const float4 u = wsum[w];
         t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w;
       }
@@ -159,9 +183,10 @@ __device__ __forceinline__ void grid_arrive(unsigned* counter, const float4* wsu
 // seen sooner than one poller's round trip allows.  sflag: 0 = waiting, 1 = released, 2 = gave up.
 // Two flag words alternate between consecutive barriers, so a word is cleared a whole phase after its last reader.
 __device__ __forceinline__ bool grid_wait(unsigned* counter, unsigned target, unsigned* err, int* flags, int parity, unsigned limit) {
+  const unsigned tid = mg_tid();
   int* sflag = flags + parity;
-  if (threadIdx.x == 0) flags[parity ^ 1] = 0;
-  if ((threadIdx.x & 31) == 0 && threadIdx.x < 128) {
+  if (tid == 0) flags[parity ^ 1] = 0;
+  if ((tid & 31) == 0 && tid < 128) {
     volatile int* vf = sflag;
     int state = 0;
     for (unsigned i = 0; i < limit; i++) {  // a second or two of polling at most
@@ -183,7 +208,7 @@ __device__ __forceinline__ bool grid_wait(unsigned* counter, unsigned target, un
       *vf = 2;
     }
   }
-  __syncthreads();
+  cta_sync();
   return *sflag == 1;
 }
 
@@ -220,7 +245,7 @@ __device__ __forceinline__ void fx_put_chunk(unsigned char* xs, unsigned units, 
   *reinterpret_cast<uint32_t*>(base) = __byte_perm(__byte_perm(X0, X1, 0x0040), __byte_perm(X2, X3, 0x0040), 0x5410);
   *reinterpret_cast<uint32_t*>(base + plane) = __byte_perm(__byte_perm(X0, X1, 0x0051), __byte_perm(X2, X3, 0x0051), 0x5410);
   *reinterpret_cast<uint32_t*>(base + 2 * plane) = __byte_perm(__byte_perm(X0, X1, 0x0062), __byte_perm(X2, X3, 0x0062), 0x5410);
-  if ((threadIdx.x & 7u) == 0) {
+  if ((c & 7u) == 0) {
     float* mt = reinterpret_cast<float*>(xs + 3 * plane + (size_t)u * 16u);
     mt[hi] = s;
     mt[2 + hi] = sc;
@@ -252,17 +277,18 @@ __device__ __forceinline__ void fx_store_subblock(unsigned char* dst, unsigned u
 }
 // Bring a vector a producer left in that layout into shared memory (units * 256 bytes; the pad words travel too).
 __device__ __forceinline__ void fx_copy_in(unsigned char* xs, const unsigned char* src, unsigned units) {
+  const unsigned tid = mg_tid();
   const unsigned n16 = units * 16u;  // 3 planes of 80 bytes + 16 bytes of sums and scales per unit
-  for (unsigned base = 0; base < n16; base += 6u * blockDim.x) {
-    uint4 v[6];
+  for (unsigned base = 0; base < n16; base += 2u * MG_THREADS) {
+    uint4 v[2];
 #pragma unroll
-    for (int k = 0; k < 6; k++) {
-      const unsigned i = base + threadIdx.x + k * blockDim.x;
-      if (i < n16) v[k] = __ldcg(reinterpret_cast<const uint4*>(src) + i);
+    for (int k = 0; k < 2; k++) {
+      const unsigned i = base + tid + k * MG_THREADS;
+      v[k] = i < n16 ? __ldcg(reinterpret_cast<const uint4*>(src) + i) : make_uint4(0u, 0u, 0u, 0u);
     }
 #pragma unroll
-    for (int k = 0; k < 6; k++) {
-      const unsigned i = base + threadIdx.x + k * blockDim.x;
+    for (int k = 0; k < 2; k++) {
+      const unsigned i = base + tid + k * MG_THREADS;
       if (i < n16) reinterpret_cast<uint4*>(xs)[i] = v[k];
     }
   }
@@ -295,41 +321,47 @@ __device__ __forceinline__ void fx_word(uint32_t w, unsigned xl0, unsigned xl1, 
   ahi[1] = dp4a_uu(hi, xh1, ahi[1]);
   ahi2 = dp4a_us(hi, xh2, ahi2);
 }
-// Multiply-accumulate one item against the fixed-point x: MATS row slots per lane.
+// Multiply-accumulate one item (column segment cs of the four rows at slot_addr, MATS matrices) against the fixed-point x.
 template <int MATS>
-__device__ __forceinline__ void mg_item_compute_fx(uint32_t slot_addr, uint32_t xs_s, unsigned units, unsigned seg_blocks,
+__device__ __forceinline__ void mg_item_compute_fx(uint32_t slot_addr, unsigned row_bytes, uint32_t xs_s, unsigned units, unsigned seg_blocks,
                                                    unsigned cs, int cl, int rl, float (&yacc)[2]) {
   const int g = cl & 3;
-  const unsigned seg_bytes = seg_blocks * KS_Q4K_BLOCK_BYTES, seg_units = seg_blocks * 4, upl = seg_units / MG_LPR;
+  const unsigned seg_units = seg_blocks * 4, upl = seg_units / MG_LPR;
   const uint32_t plane = units * MG_XU;
-  uint32_t waddr = slot_addr + (uint32_t)rl * seg_bytes + (uint32_t)(cl >> 2) * KS_Q4K_BLOCK_BYTES + (uint32_t)g * 32u;
+  uint32_t waddr = slot_addr + (uint32_t)rl * row_bytes + (cs * seg_blocks + (uint32_t)(cl >> 2)) * KS_Q4K_BLOCK_BYTES + (uint32_t)g * 32u;
   uint32_t xaddr = xs_s + (cs * seg_units + (unsigned)cl) * MG_XU;
   uint32_t maddr = xs_s + 3u * plane + (cs * seg_units + (unsigned)cl) * 16u;
+#pragma unroll 1
   for (unsigned it = 0; it < upl; it++) {
-    const float4 mt = lds_f4o<0>(maddr);
-    // 16 words per plane: [0..7] low sub-block, [8..15] high sub-block
-    const uint4 a0 = lds_u4o<0>(xaddr), a1 = lds_u4o<16>(xaddr), a2 = lds_u4o<32>(xaddr), a3 = lds_u4o<48>(xaddr);
-    const uint4 b0 = lds_u4o<0>(xaddr + plane), b1 = lds_u4o<16>(xaddr + plane), b2 = lds_u4o<32>(xaddr + plane),
-                b3 = lds_u4o<48>(xaddr + plane);
-    const uint4 c0 = lds_u4o<0>(xaddr + 2 * plane), c1 = lds_u4o<16>(xaddr + 2 * plane), c2 = lds_u4o<32>(xaddr + 2 * plane),
-                c3 = lds_u4o<48>(xaddr + 2 * plane);
+    unsigned alo[MATS][2], ahi[MATS][2];
+    int alo2[MATS], ahi2[MATS];
 #pragma unroll
     for (int r = 0; r < MATS; r++) {
-      const uint32_t wa = waddr + (uint32_t)(r * MG_RL) * seg_bytes;
-      const uint4 q0 = lds_u4o<16>(wa), q1 = lds_u4o<32>(wa);
-      const uint4 hdr = lds_u4o<0>(wa - (uint32_t)g * 32u);
-      unsigned alo[2] = {0u, 0u}, ahi[2] = {0u, 0u};
-      int alo2 = 0, ahi2 = 0;
-      fx_word(q0.x, a0.x, b0.x, c0.x, a2.x, b2.x, c2.x, alo, alo2, ahi, ahi2);
-      fx_word(q0.y, a0.y, b0.y, c0.y, a2.y, b2.y, c2.y, alo, alo2, ahi, ahi2);
-      fx_word(q0.z, a0.z, b0.z, c0.z, a2.z, b2.z, c2.z, alo, alo2, ahi, ahi2);
-      fx_word(q0.w, a0.w, b0.w, c0.w, a2.w, b2.w, c2.w, alo, alo2, ahi, ahi2);
-      fx_word(q1.x, a1.x, b1.x, c1.x, a3.x, b3.x, c3.x, alo, alo2, ahi, ahi2);
-      fx_word(q1.y, a1.y, b1.y, c1.y, a3.y, b3.y, c3.y, alo, alo2, ahi, ahi2);
-      fx_word(q1.z, a1.z, b1.z, c1.z, a3.z, b3.z, c3.z, alo, alo2, ahi, ahi2);
-      fx_word(q1.w, a1.w, b1.w, c1.w, a3.w, b3.w, c3.w, alo, alo2, ahi, ahi2);
-      const float flo = fmaf((float)alo2, 65536.0f, fmaf((float)alo[1], 256.0f, (float)alo[0])) * mt.z;
-      const float fhi = fmaf((float)ahi2, 65536.0f, fmaf((float)ahi[1], 256.0f, (float)ahi[0])) * mt.w;
+      alo[r][0] = alo[r][1] = ahi[r][0] = ahi[r][1] = 0u;
+      alo2[r] = ahi2[r] = 0;
+    }
+    // 16 words per plane: [0..7] low sub-block, [8..15] high sub-block.  Half of each at a time: with all 48 words of x in registers
+    // the kernel spills, and what is spilled has to come back from L2 (shared memory leaves no L1, an acquire empties it).
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const uint32_t xa = xaddr + 16u * h;
+      const uint4 a0 = lds_u4o<0>(xa), a2 = lds_u4o<32>(xa), b0 = lds_u4o<0>(xa + plane), b2 = lds_u4o<32>(xa + plane),
+                  c0 = lds_u4o<0>(xa + 2 * plane), c2 = lds_u4o<32>(xa + 2 * plane);
+#pragma unroll
+      for (int r = 0; r < MATS; r++) {
+        const uint4 q = lds_u4o<16>(waddr + (uint32_t)(r * MG_RL) * row_bytes + 16u * h);
+        fx_word(q.x, a0.x, b0.x, c0.x, a2.x, b2.x, c2.x, alo[r], alo2[r], ahi[r], ahi2[r]);
+        fx_word(q.y, a0.y, b0.y, c0.y, a2.y, b2.y, c2.y, alo[r], alo2[r], ahi[r], ahi2[r]);
+        fx_word(q.z, a0.z, b0.z, c0.z, a2.z, b2.z, c2.z, alo[r], alo2[r], ahi[r], ahi2[r]);
+        fx_word(q.w, a0.w, b0.w, c0.w, a2.w, b2.w, c2.w, alo[r], alo2[r], ahi[r], ahi2[r]);
+      }
+    }
+    const float4 mt = lds_f4o<0>(maddr);
+#pragma unroll
+    for (int r = 0; r < MATS; r++) {
+      const uint4 hdr = lds_u4o<0>(waddr + (uint32_t)(r * MG_RL) * row_bytes - (uint32_t)g * 32u);
+      const float flo = fmaf((float)alo2[r], 65536.0f, fmaf((float)alo[r][1], 256.0f, (float)alo[r][0])) * mt.z;
+      const float fhi = fmaf((float)ahi2[r], 65536.0f, fmaf((float)ahi[r][1], 256.0f, (float)ahi[r][0])) * mt.w;
       yacc[r] = q4k_apply_scales(hdr, g, flo, fhi, mt.x, mt.y, yacc[r]);
     }
     waddr += (MG_LPR / 4) * KS_Q4K_BLOCK_BYTES;
@@ -340,107 +372,52 @@ __device__ __forceinline__ void mg_item_compute_fx(uint32_t slot_addr, uint32_t 
 
 
 // ---- staging of x (with the fused norm prologues), reads through L2 ---------------------------
-// Norm weights of the next matvec phase, fetched into registers before the barrier wait.
-template <int PC>
-struct NormPre {  // PC chunks of 4 elements per thread: cols <= PC * 4 * blockDim
-  float4 w[PC], wp[PC];
-};
-template <int PC>
-__device__ __forceinline__ void mg_prefetch_norm(NormPre<PC>& n, int mode, const float* w, const float* wp, unsigned cols) {
-  const unsigned nchunk = cols >> 2;
-  if (mode == KS_PRO_NONE) return;
+constexpr int MG_XMAX = 4;  // plain staging keeps up to 4 chunks per thread in flight (8192 columns), loops beyond
+// x' = x
+__device__ __forceinline__ void mg_stage_plain(unsigned char* xs, unsigned cols, const float* x) {
+  const unsigned tid = mg_tid();
+  const unsigned units = cols >> 6, nchunk = cols >> 2;
+  for (unsigned base = 0; base < nchunk; base += MG_XMAX * MG_THREADS) {
+    float4 v[MG_XMAX];
 #pragma unroll
-  for (int k = 0; k < PC; k++) {
-    const unsigned c = threadIdx.x + k * blockDim.x;
-    if (c < nchunk) {
-      n.w[k] = reinterpret_cast<const float4*>(w)[c];
-      if (mode == KS_PRO_ADD_NORM) n.wp[k] = reinterpret_cast<const float4*>(wp)[c];
+    for (int k = 0; k < MG_XMAX; k++) {
+      const unsigned c = base + tid + k * MG_THREADS;
+      v[k] = c < nchunk ? ldcg4(x, c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int k = 0; k < MG_XMAX; k++) {
+      const unsigned c = base + tid + k * MG_THREADS;
+      if (c < nchunk) fx_put_chunk(xs, units, c, v[k]);
     }
   }
 }
-
-constexpr int MG_XMAX = 8;  // plain staging keeps up to 8 chunks per thread in flight (cols <= 8192), loops beyond
-
-// mode NONE: x' = x.  NORM: x' = rms(x)*w.  ADD_NORM: r = x + rms(y)*wp (block 0 stores r to out_x); x' = rms(r)*w.
+// x' = rms(x) * w  (the first layer)
 template <int PC>
-__device__ __forceinline__ void mg_stage_x(unsigned char* xs, float* red, int mode, unsigned cols, const float* x,
-                                           const float* y, float* out_x, float eps, const NormPre<PC>& n) {
+__device__ __forceinline__ void mg_stage_norm(unsigned char* xs, float* red, unsigned cols, const float* x, float eps, const float4* w) {
+  const unsigned tid = mg_tid();
   const unsigned units = cols >> 6, nchunk = cols >> 2;
-  if (mode == KS_PRO_NONE) {
-    for (unsigned base = 0; base < nchunk; base += MG_XMAX * blockDim.x) {
-      float4 v[MG_XMAX];
-#pragma unroll
-      for (int k = 0; k < MG_XMAX; k++) {
-        const unsigned c = base + threadIdx.x + k * blockDim.x;
-        if (c < nchunk) v[k] = ldcg4(x, c);
-      }
-#pragma unroll
-      for (int k = 0; k < MG_XMAX; k++) {
-        const unsigned c = base + threadIdx.x + k * blockDim.x;
-        if (c < nchunk) fx_put_chunk(xs, units, c, v[k]);
-      }
-    }
-    return;
-  }
-  const float invn = 1.0f / (float)cols;
-  float4 v[PC], yv[PC];
+  float4 v[PC];
   float ss = 0.0f;
-  if (mode == KS_PRO_ADD_NORM) {
-#pragma unroll
-    for (int k = 0; k < PC; k++) {
-      const unsigned c = threadIdx.x + k * blockDim.x;
-      if (c < nchunk) {
-        yv[k] = ldcg4(y, c);
-        v[k] = ldcg4(x, c);
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < PC; k++) {
-      const unsigned c = threadIdx.x + k * blockDim.x;
-      if (c < nchunk) {
-        ss = fmaf(yv[k].x, yv[k].x, ss); ss = fmaf(yv[k].y, yv[k].y, ss);
-        ss = fmaf(yv[k].z, yv[k].z, ss); ss = fmaf(yv[k].w, yv[k].w, ss);
-      }
-    }
-    ss = block_sum_f(ss, red);
-    const float inv = 1.0f / sqrtf(ss * invn + eps);
-    ss = 0.0f;
-#pragma unroll
-    for (int k = 0; k < PC; k++) {
-      const unsigned c = threadIdx.x + k * blockDim.x;
-      if (c < nchunk) {
-        const float4 p4 = n.wp[k];
-        float4 r = v[k];
-        r.x = __fadd_rn(r.x, __fmul_rn(__fmul_rn(yv[k].x, inv), p4.x));
-        r.y = __fadd_rn(r.y, __fmul_rn(__fmul_rn(yv[k].y, inv), p4.y));
-        r.z = __fadd_rn(r.z, __fmul_rn(__fmul_rn(yv[k].z, inv), p4.z));
-        r.w = __fadd_rn(r.w, __fmul_rn(__fmul_rn(yv[k].w, inv), p4.w));
-        if (blockIdx.x == 0) reinterpret_cast<float4*>(out_x)[c] = r;
-        v[k] = r;
-      }
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < PC; k++) {
-      const unsigned c = threadIdx.x + k * blockDim.x;
-      if (c < nchunk) v[k] = ldcg4(x, c);
-    }
-  }
 #pragma unroll
   for (int k = 0; k < PC; k++) {
-    const unsigned c = threadIdx.x + k * blockDim.x;
-    if (c < nchunk) {
-      ss = fmaf(v[k].x, v[k].x, ss); ss = fmaf(v[k].y, v[k].y, ss);
-      ss = fmaf(v[k].z, v[k].z, ss); ss = fmaf(v[k].w, v[k].w, ss);
-    }
+    const unsigned c = tid + k * MG_THREADS;
+    v[k] = c < nchunk ? ldcg4(x, c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    ss = fmaf(v[k].x, v[k].x, ss); ss = fmaf(v[k].y, v[k].y, ss);
+    ss = fmaf(v[k].z, v[k].z, ss); ss = fmaf(v[k].w, v[k].w, ss);
   }
-  ss = block_sum_f(ss, red);
-  const float inv2 = 1.0f / sqrtf(ss * invn + eps);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if ((tid & 31) == 0) red[tid >> 5] = ss;
+  cta_sync();
+  ss = 0.0f;
+#pragma unroll
+  for (unsigned w = 0; w < MG_WARPS; w++) ss += red[w];
+  const float inv2 = 1.0f / sqrtf(ss * (1.0f / (float)cols) + eps);
 #pragma unroll
   for (int k = 0; k < PC; k++) {
-    const unsigned c = threadIdx.x + k * blockDim.x;
+    const unsigned c = tid + k * MG_THREADS;
     if (c < nchunk) {
-      const float4 w4 = n.w[k];
+      const float4 w4 = w[c];
       float4 r;
       r.x = __fmul_rn(__fmul_rn(v[k].x, inv2), w4.x);
       r.y = __fmul_rn(__fmul_rn(v[k].y, inv2), w4.y);
@@ -451,38 +428,40 @@ __device__ __forceinline__ void mg_stage_x(unsigned char* xs, float* red, int mo
   }
 }
 
-// ADD_NORM without any block-wide reduction: the blocks that produced y left the four sums that both
-// norms need (K:539 expands to  sum r^2 = sum x^2 + 2 inv sum x y wp + inv^2 sum (y wp)^2,  r = x + inv y wp).
+// r = x + rms(y) * wp (block 0 stores r to out_x); x' = rms(r) * w.  Without a block-wide reduction over the vector: the blocks that
+// produced y left the four sums that both norms need (K:539 expands to  sum r^2 = sum x^2 + 2 inv sum x y wp + inv^2 sum (y wp)^2,
+// r = x + inv y wp).  A lane folds a block's sums while the loads of x and y are on their way.
 template <int PC>
-__device__ __forceinline__ void mg_stage_addnorm(unsigned char* xs, unsigned cols, const float* x, const float* y, float* out_x,
-                                                 float eps, const NormPre<PC>& n, const float4* nsum, unsigned nblocks) {
+__device__ __forceinline__ void mg_stage_addnorm(unsigned char* xs, float* red, unsigned cols, const float* x, const float* y, float* out_x,
+                                                 float eps, const float4* w, const float4* wp, const float4* nsum, unsigned nblocks) {
+  const unsigned tid = mg_tid();
   const unsigned units = cols >> 6, nchunk = cols >> 2;
-  const int lane = threadIdx.x & 31;
-  float4 v[PC], yv[PC], ps[8];
-#pragma unroll
-  for (int j = 0; j < 8; j++) {
-    const unsigned i = (unsigned)lane + 32u * j;
-    ps[j] = i < nblocks ? __ldcg(nsum + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
+  float4 v[PC], yv[PC];
 #pragma unroll
   for (int k = 0; k < PC; k++) {
-    const unsigned c = threadIdx.x + k * blockDim.x;
-    if (c < nchunk) {
-      yv[k] = ldcg4(y, c);
-      v[k] = ldcg4(x, c);
+    const unsigned c = tid + k * MG_THREADS;
+    yv[k] = c < nchunk ? ldcg4(y, c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    v[k] = c < nchunk ? ldcg4(x, c) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  const unsigned fold = (nblocks + 31u) / 32u;
+  float4* sums = reinterpret_cast<float4*>(red);
+  if ((tid >> 5) < fold) {
+    float4 t = tid < nblocks ? __ldcg(nsum + tid) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
+      t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
+      t.z += __shfl_xor_sync(0xffffffffu, t.z, o);
+      t.w += __shfl_xor_sync(0xffffffffu, t.w, o);
     }
+    if ((tid & 31) == 0) sums[tid >> 5] = t;
   }
-  float4 t = ps[0];
-#pragma unroll
-  for (int j = 1; j < 8; j++) {
-    t.x += ps[j].x; t.y += ps[j].y; t.z += ps[j].z; t.w += ps[j].w;
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
-    t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
-    t.z += __shfl_xor_sync(0xffffffffu, t.z, o);
-    t.w += __shfl_xor_sync(0xffffffffu, t.w, o);
+  cta_sync();
+  float4 t = sums[0];
+#pragma unroll 1
+  for (unsigned w = 1; w < fold; w++) {
+    const float4 u = sums[w];
+    t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w;
   }
   const float invn = 1.0f / (float)cols;
   const float inv = __frsqrt_rn(t.x * invn + eps);
@@ -490,9 +469,9 @@ __device__ __forceinline__ void mg_stage_addnorm(unsigned char* xs, unsigned col
   const float inv2 = __frsqrt_rn(fmaxf(rr, 0.0f) * invn + eps);
 #pragma unroll
   for (int k = 0; k < PC; k++) {
-    const unsigned c = threadIdx.x + k * blockDim.x;
+    const unsigned c = tid + k * MG_THREADS;
     if (c < nchunk) {
-      const float4 p4 = n.wp[k], w4 = n.w[k];
+      const float4 p4 = wp[c], w4 = w[c];
       float4 r = v[k];
       r.x = __fadd_rn(r.x, __fmul_rn(__fmul_rn(yv[k].x, inv), p4.x));
       r.y = __fadd_rn(r.y, __fmul_rn(__fmul_rn(yv[k].y, inv), p4.y));
@@ -509,100 +488,21 @@ __device__ __forceinline__ void mg_stage_addnorm(unsigned char* xs, unsigned col
   }
 }
 
-// ---- the per-warp item list of a whole token -----------------------------------------------------
-// Item = (phase, row group, column segment).
-
-// The items of a warp repeat layer after layer (same shapes, other pointers), so the walk over the
-// shapes is done once per kernel: each warp records its items of ONE layer, in phase order, and the
-// issue and consume positions are (layer, entry) pairs.
-constexpr int MG_MAX_ENT = 16;
-struct ItemEnt {
-  uint32_t src_off;  // byte offset of the first copy inside its weight matrix
-  uint32_t pslot;    // index of this item among the block's items of the phase (where its partial sums go)
-  uint16_t seg16;    // bytes of one row segment / 16
-  uint8_t kind, seg, cs, valid;
-  uint8_t widx;      // MegaLayer::W index of the first matrix
-  uint8_t flags;     // bit 0: two matrices (gate, up) in one item; bit 1: whole rows (one copy per matrix);
-                     // bit 2: this item is the second matrix (up) of a split gate-up group
-};
-struct ItemPos {
-  int layer, e;
-};
-__device__ __forceinline__ void pos_next(ItemPos& c, int n_ent) {
-  if (++c.e >= n_ent) {
-    c.e = 0;
-    c.layer++;
-  }
-}
-// Groups of a phase go to blocks round-robin (block c owns groups c, c + grid, ...); the block's items
-// -- its groups x the column segments -- go to its warps round-robin.  A row's column segments may
-// therefore be multiplied by different warps; the partial sums meet in shared memory (slot pslot).
-constexpr int MG_MAX_P = 64;  // items of one block in one phase
+// ---- the row groups of a block -------------------------------------------------------------------
+// Groups of four rows go to blocks round-robin (block c owns groups c, c + grid, ...); each is one job of the copying warp.  A
+// phase's items are its groups x column segments, item i to warp i % MG_WARPS; the partial sums of a row's segments meet in
+// shared memory (slot i).
+constexpr int MG_MAX_P = 192;  // items of one block in one phase
 __device__ __forceinline__ unsigned block_groups(const MegaShape& sh) {
   const unsigned total = sh.type == MG_ATTN ? 0u : sh.grp_start[sh.n_seg];
-  if (sh.oct) {
-    const unsigned octs = (total + 7u) / 8u;
-    return octs > blockIdx.x ? (octs - blockIdx.x + gridDim.x - 1) / gridDim.x * 8u : 0u;
-  }
   return total > blockIdx.x ? (total - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u;
 }
 // global group index of this block's k-th group
-__device__ __forceinline__ unsigned block_group_id(const MegaShape& sh, unsigned k) {
-  return sh.oct ? (blockIdx.x + (k >> 3) * gridDim.x) * 8u + (k & 7u) : blockIdx.x + k * gridDim.x;
-}
-// lane 0 of each warp fills its table; returns the entry count (0 when the warp owns nothing, -1 on overflow)
-__device__ __forceinline__ int build_items(ItemEnt* ent, const MegaShape* shapes, int warp) {
-  int n = 0;
-  for (int kind = 0; kind < PH_PER_LAYER; kind++) {
-    const MegaShape& sh = shapes[kind];
-    const unsigned C = sh.n_cseg, n_slots = block_groups(sh) * C;
-    if (n_slots > (unsigned)MG_MAX_P) return -1;
-    const unsigned seg_bytes = sh.seg_blocks * KS_Q4K_BLOCK_BYTES;
-    const bool split = sh.type == MG_GATE_UP && sh.split;
-    const int mats = (sh.type == MG_GATE_UP && !split) ? 2 : 1;
-    const int w0 = kind == PH_QKV ? 0 : kind == PH_OPROJ ? 3 : kind == PH_GATEUP ? 4 : 6;
-    const unsigned n_items = split ? n_slots * 2u : n_slots;
-    for (unsigned jj = (unsigned)warp; jj < n_items; jj += 8u) {
-      if (n >= MG_MAX_ENT) return -1;
-      const unsigned j = split ? jj >> 1 : jj, second = split ? jj & 1u : 0u;
-      const unsigned k = j / C, cs = j - k * C;
-      const unsigned g = block_group_id(sh, k);
-      if (g >= sh.grp_start[sh.n_seg]) continue;
-      int seg = 0;
-      if (sh.n_seg > 1 && g >= sh.grp_start[1]) seg = 1;
-      if (sh.n_seg > 2 && g >= sh.grp_start[2]) seg = 2;
-      const unsigned row0 = (g - sh.grp_start[seg]) * MG_RL;
-      ItemEnt e;
-      e.src_off = row0 * sh.row_bytes + cs * seg_bytes;
-      e.pslot = j;
-      e.seg16 = (uint16_t)(seg_bytes / 16u);
-      e.kind = (uint8_t)kind;
-      e.seg = (uint8_t)seg;
-      e.cs = (uint8_t)cs;
-      e.valid = (uint8_t)min((unsigned)MG_RL, sh.rows[seg] - row0);
-      e.widx = (uint8_t)(w0 + (mats == 2 ? 0 : split ? second : seg));
-      e.flags = (uint8_t)((mats == 2 ? 1 : 0) | (C == 1 ? 2 : 0) | (second ? 4 : 0));
-      ent[n++] = e;
-    }
-  }
-  return n;
-}
-
-// Start the copies of one item into a ring slot (all lanes call).
-__device__ __forceinline__ void mg_issue_ent(const ItemEnt& e, const MegaLayer& L, unsigned row_bytes, uint32_t slot_addr,
-                                             uint32_t bar, int lane) {
-  const unsigned seg_bytes = (unsigned)e.seg16 * 16u, valid = e.valid;
-  const int mats = (e.flags & 1) ? 2 : 1;
-  if (lane == 0) mb_expect(bar, valid * mats * seg_bytes);
-  if (e.flags & 2) {
-    if (lane < mats)
-      bulk_in(slot_addr + (uint32_t)lane * MG_RL * seg_bytes, L.W[e.widx + lane] + e.src_off, valid * seg_bytes, bar);
-  } else if (lane < MG_RL * mats) {
-    const int m = lane / MG_RL, rr = lane % MG_RL;
-    if ((unsigned)rr < valid)
-      bulk_in(slot_addr + (uint32_t)lane * seg_bytes, L.W[e.widx + m] + e.src_off + (size_t)rr * row_bytes, seg_bytes, bar);
-  }
-}
+__device__ __forceinline__ unsigned block_group_id(unsigned k) { return blockIdx.x + k * gridDim.x; }
+// jobs in front of a phase's row groups
+__device__ __forceinline__ unsigned norm_jobs(int kind) { return kind == PH_QKV || kind == PH_GATEUP ? 1u : 0u; }
+// arrivals of item cs of a job with C items
+__device__ __forceinline__ unsigned empty_share(unsigned cs, unsigned C) { return cs == 0 ? MG_EMPTY - C + 1u : 1u; }
 
 // ---- attention phase ------------------------------------------------------------------------------
 constexpr float kNegInit = -1.0e30f;
@@ -644,19 +544,24 @@ __device__ __forceinline__ void raw_load(const uint8_t* row, int lane, RawRow<DP
 #pragma unroll
   for (int w = 0; w < BPL / 2; w++) r.q[w] = qs[w];
 }
+// Its values n - 8, each times the power of two its nibble sits at (q comes divided by it, o is divided by it at the end): a mask
+// and an OR make the float 2^23 + n 2^k, a subtraction the rest, all exact.  The block's scale is applied to the sums.
 template <int DPL>
-__device__ __forceinline__ void raw_decode(const RawRow<DPL>& r, float (&out)[DPL]) {
+__device__ __forceinline__ constexpr float raw_unit(int j) {
   constexpr int BPL = DPL / 2;
-  const float d = __half2float(__ushort_as_half(r.d));
+  return (j < BPL ? 1.0f : 16.0f) * (j & 1 ? 256.0f : 1.0f);
+}
+template <int DPL>
+__device__ __forceinline__ void raw_ints(const RawRow<DPL>& r, float (&out)[DPL]) {
+  constexpr int BPL = DPL / 2;
 #pragma unroll
-  for (int w = 0; w < BPL / 2; w++) {
-    const unsigned v = r.q[w];
-    out[2 * w] = (float)((int)(v & 0xF) - 8) * d;
-    out[2 * w + 1] = (float)((int)((v >> 8) & 0xF) - 8) * d;
-    out[BPL + 2 * w] = (float)((int)((v >> 4) & 0xF) - 8) * d;
-    out[BPL + 2 * w + 1] = (float)((int)(v >> 12) - 8) * d;
+  for (int j = 0; j < DPL; j++) {
+    const unsigned v = r.q[(j % BPL) / 2], mask = 0xFu * (unsigned)raw_unit<DPL>(j);
+    out[j] = __uint_as_float((v & mask) | 0x4B000000u) - (8388608.0f + 8.0f * raw_unit<DPL>(j));
   }
 }
+template <int DPL>
+__device__ __forceinline__ float raw_scale(const RawRow<DPL>& r) { return __half2float(__ushort_as_half(r.d)); }
 template <int DPL>
 __device__ __forceinline__ int mg_lane_dim(int lane, int j) {
   constexpr int BPL = DPL / 2, LPB = 16 / BPL;
@@ -664,56 +569,107 @@ __device__ __forceinline__ int mg_lane_dim(int lane, int j) {
   return j < BPL ? base + j : base + 16 + (j - BPL);
 }
 
-constexpr int MG_MAX_SPLITS = 16;  // context splits per head (the final merge keeps one record per split in registers)
+__host__ __device__ constexpr unsigned mg_rec(unsigned hd) { return hd + 4u; }  // floats of a record: O[hd], m, l, two unused
+constexpr int MG_MAX_SPLITS = 18;  // context splits per head (the final merge keeps one record per split in registers)
+constexpr int MG_FLY = 4;  // positions of a warp in flight
+// Up to MG_DIRECT splits are merged by every block while it stages the o-projection's input (mg_stage_merge): no block waits for
+// another one's merge, and a block reads at most n_q x 4 records (2.0 us of staging instead of 0.8).  A token of the E2B shape at
+// 64..128 positions: one split 1017 us, two 1003, four 998; with a window of 512: 1203, 1188, 1096.
+constexpr unsigned MG_DIRECT = 4, MG_SINGLE_TLEN = MG_FLY * MG_WARPS, MG_DIRECT_TLEN = 1024;
 
 // Shared memory the attention phase needs (it reuses the x staging area).
 __host__ __device__ inline unsigned mg_att_bytes(unsigned hd) {
-  return 8u * (hd + 2u) * 4u + 2u * ((hd / 32u) * KS_Q40_BLOCK_BYTES + 16u) + 32u;
+  return MG_WARPS * (hd + 2u) * 4u + hd * 4u + 2u * ((hd / 32u) * KS_Q40_BLOCK_BYTES + 16u) + 32u;
 }
 
-// Splits in use for a context of tlen positions: one row per warp (8 per block) until every split is
-// in use, more rows per warp beyond that.
+// Splits in use for a context of tlen positions: one block per head while its warps get by with a few rows each, a few that every
+// block merges for itself, then all of them and a merge by the head's last block.
 __host__ __device__ inline unsigned mg_active_splits(unsigned tlen, unsigned max_splits) {
-  unsigned ns = (tlen + 7u) / 8u;
-  return ns < 1u ? 1u : ns > max_splits ? max_splits : ns;
+  const unsigned ns = tlen <= MG_SINGLE_TLEN ? 1u : tlen <= MG_DIRECT_TLEN ? MG_DIRECT : max_splits;
+  return ns < max_splits ? ns : max_splits;
+}
+// The positions a layer attends to: [first, pos].
+__device__ __forceinline__ unsigned mg_first(const MegaLayer& L, unsigned pos) {
+  const unsigned win = (unsigned)L.window;
+  return win && pos + 1u > win ? pos + 1u - win : 0u;
+}
+// A run of bytes into L2, as far as whole 16-byte pieces of it go.
+__device__ __forceinline__ void l2_prefetch(const void* p, size_t bytes) {
+  const uintptr_t a = ((uintptr_t)p + 15u) & ~(uintptr_t)15u, e = ((uintptr_t)p + bytes) & ~(uintptr_t)15u;
+  if (e > a) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((unsigned)(e - a)) : "memory");
+}
+// The weights of a token push everything else out of L2 (they are five times its size), so the cached rows a layer's attention
+// reads are asked for a phase or more ahead; one thread per block, each split's rows once.
+__device__ __forceinline__ void mg_prefetch_kv(const MegaArgs& a, const MegaLayer& L, unsigned pos) {
+  const unsigned NSMAX = a.n_splits, first = mg_first(L, pos), tlen = pos + 1u - first;
+  const unsigned NS = mg_active_splits(tlen, NSMAX), split = blockIdx.x % NSMAX, head = blockIdx.x / NSMAX;
+  if (head == 0 && split < NS) {
+    const unsigned chunk = (tlen + NS - 1) / NS, p0 = first + split * chunk, p1 = min(p0 + chunk, pos);
+    const size_t row = (size_t)a.n_kv * (a.hd / 32u) * KS_Q40_BLOCK_BYTES;
+    if (p0 < p1) {
+      l2_prefetch(L.kv_k + p0 * row, (p1 - p0) * row);
+      l2_prefetch(L.kv_v + p0 * row, (p1 - p0) * row);
+    }
+  }
+  if (blockIdx.x >= gridDim.x - 2u) l2_prefetch(L.norm[gridDim.x - blockIdx.x], a.hd * 4u);  // the head norms
 }
 
 // One block per (query head, context split): the work of a short context is tiny, so it is spread
 // as widely as the grid allows and every serial step stays short.
-//   1. every warp builds the roped, normed, scaled q of the head in registers (no exchange needed);
-//      in the blocks of the split that holds the newest position, warps 0.. pack the new K row and
-//      warps 4.. the new V row to Q4_0 in shared memory (lower.rs:4231-4702), block pairs (b, b+NB/2)
-//      per warp because RoPE pairs those halves; the block of the KV group's first head stores them;
+//   1. one warp polls for the head's q and leaves it roped, normed and scaled in shared memory; in the blocks of the split that
+//      holds the newest position, four others pack the new K row and four the new V row to Q4_0 in shared memory
+//      (lower.rs:4231-4702), block pairs (b, b+NB/2) per warp because RoPE pairs those halves; the block of the KV group's
+//      first head stores them;
 //   2. warps take the positions of the split round-robin, online softmax per warp;
-//   3. the eight warps' (m, l, O) meet in shared memory, thread d folds dimension d;
-//   4. the block leaves a (m, l, O[hd]) record; the last block of a head to arrive merges the
-//      head's records (lower.rs:5897-6088).
+//   3. the warps' (m, l, O) meet in shared memory, thread d folds dimension d;
+//   4. the block leaves a (m, l, O[hd]) record; few records of a head are merged by their readers, more by the last block of
+//      the head to arrive (lower.rs:5897-6088).
 template <int DPL>
 __device__ __forceinline__ void mg_attention(const MegaArgs& a, const MegaLayer& L, unsigned char* sm, int* sflag, long long* pf,
-                                             unsigned tag) {
+                                             unsigned tag, unsigned pos) {
+  const unsigned tid = mg_tid();
   constexpr int HD = DPL * 32, HALF = HD / 2, NB = HD / 32;
   constexpr unsigned ROWB = NB * KS_Q40_BLOCK_BYTES;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = tid & 31, warp = tid >> 5;
   const unsigned NSMAX = a.n_splits;
   if (blockIdx.x >= a.n_q * NSMAX) return;
   const unsigned head = blockIdx.x / NSMAX, split = blockIdx.x % NSMAX;
   const unsigned G = a.n_q / a.n_kv, kvh = head / G;
-  const unsigned pos = (unsigned)a.pos[0], win = (unsigned)L.window, first = win && pos + 1u > win ? pos + 1u - win : 0u, tlen = pos + 1u - first;
+  const unsigned first = mg_first(L, pos), tlen = pos + 1u - first;
   const unsigned NS = mg_active_splits(tlen, NSMAX);
   if (split >= NS) return;
   const unsigned chunk = (tlen + NS - 1) / NS;
   const unsigned p0 = first + split * chunk, p1 = min(p0 + chunk, pos + 1u);
   const bool owner = pos >= p0 && pos < p1;  // the split that holds the newest position
-  float* part = reinterpret_cast<float*>(sm);     // [8][HD + 2]
-  uint8_t* skrow = reinterpret_cast<uint8_t*>(part + 8 * (HD + 2));
+  float* part = reinterpret_cast<float*>(sm);     // [MG_WARPS][HD + 2]
+  float* sq = part + MG_WARPS * (HD + 2);         // the head's q
+  uint8_t* skrow = reinterpret_cast<uint8_t*>(sq + HD);
   uint8_t* svrow = skrow + ROWB + 16u;
   const float* cs = a.rope + (size_t)pos * HD;
+  const size_t rowstride = (size_t)a.n_kv * ROWB;
+  uint8_t* Kc = L.kv_k + (size_t)kvh * ROWB;
+  uint8_t* Vc = L.kv_v + (size_t)kvh * ROWB;
+  // MG_FLY positions of this warp at a time (t, t + MG_WARPS, ...): K of the next ones is asked for as soon as the scores are
+  // there, V once it is summed, and the first do not wait for q.  (One position at a time, its successor in flight: 640 ns a
+  // position; 250 positions a block took 20 us.)
+  constexpr int FLY = MG_FLY;
+  RawRow<DPL> kn[FLY], vn[FLY];
+  auto row_at = [&](unsigned t, int i) { return min(t + MG_WARPS * i, p1 - 1u); };  // past the split's end: loaded, not used
+  auto load_rows = [&](unsigned t, RawRow<DPL>(&r)[FLY], const uint8_t* cache, const uint8_t* newest) {
+#pragma unroll
+    for (int i = 0; i < FLY; i++) {
+      const unsigned p = row_at(t, i);
+      raw_load<DPL>(p == pos ? newest : cache + (size_t)p * rowstride, lane, r[i]);
+    }
+  };
+  unsigned t = p0 + warp;
+  load_rows(t, kn, Kc, skrow);
+  load_rows(t, vn, Vc, svrow);
 
-  float qr[DPL];
-  {
-    const int pb = warp & 3;  // block pair of the K / V job
-    const bool kjob = owner && warp < 4 && pb < NB / 2, vjob = owner && warp >= 4 && pb < NB / 2;
-    float qv[DPL], qw[DPL], qc[DPL], qs[DPL], rv[DPL], r_w0 = 0.f, r_w1 = 0.f, r_c = 0.f, r_s = 0.f;
+  const int pb = (warp - 1) & 3;  // block pair of the K / V job
+  const bool kjob = owner && warp >= 1 && warp < 5 && pb < NB / 2, vjob = owner && warp >= 5 && warp < 9 && pb < NB / 2;
+  if (warp == 0) {
+    float qv[DPL], qw[DPL], qc[DPL], qs[DPL];
     const float* qnw = L.norm[1];
 #pragma unroll
     for (int j = 0; j < DPL; j++) {  // constants first: they are on their way while the tagged words are polled
@@ -723,85 +679,78 @@ __device__ __forceinline__ void mg_attention(const MegaArgs& a, const MegaLayer&
       qs[j] = cs[HALF + (d & (HALF - 1))];
     }
     // q (and, in the owner split, k / v) arrive as tagged words straight from the blocks that computed them
-    bool got = true;
-    {
-      const unsigned long long* qsrc = a.qkv_t + (size_t)head * HD;
+    int at[DPL];
 #pragma unroll
-      for (int j = 0; j < DPL; j += 4)
-        got = tag_wait4(qsrc, mg_lane_dim<DPL>(lane, j), mg_lane_dim<DPL>(lane, j + 1), mg_lane_dim<DPL>(lane, j + 2),
-                        mg_lane_dim<DPL>(lane, j + 3), tag, a.poll_limit, qv[j], qv[j + 1], qv[j + 2], qv[j + 3]) && got;
-    }
-    if (kjob || vjob) {
-      const unsigned long long* src = a.qkv_t + (size_t)a.n_q * HD + (kjob ? 0u : (size_t)a.n_kv * HD) + (size_t)kvh * HD;
-#pragma unroll
-      for (int j = 0; j < DPL; j += 4)
-        got = tag_wait4(src, lane + 32 * j, lane + 32 * (j + 1), lane + 32 * (j + 2), lane + 32 * (j + 3), tag, a.poll_limit, rv[j],
-                        rv[j + 1], rv[j + 2], rv[j + 3]) && got;
-      if (kjob) {
-        const float* w = L.norm[2];
-        r_w0 = w[32 * pb + lane];
-        r_w1 = w[HALF + 32 * pb + lane];
-        r_c = cs[32 * pb + lane];
-        r_s = cs[HALF + 32 * pb + lane];
-      }
-    }
+    for (int j = 0; j < DPL; j++) at[j] = mg_lane_dim<DPL>(lane, j);
+    const bool got = tag_wait<DPL>(a.qkv_t + (size_t)head * HD, at, tag, a.poll_limit, qv);
     if (!got) atomicOr(a.err, 2u);  // a tagged word never came: the values are zeros, the status word tells the host
-    {
-      float ss = 0.0f;
+    float ss = 0.0f;
 #pragma unroll
-      for (int j = 0; j < DPL; j++) ss = fmaf(qv[j], qv[j], ss);
-      ss = mg_warp_sum(ss);
-      const float inv = 1.0f / sqrtf(ss / (float)HD + a.eps);
-      // lanes 0..15 hold dims of the first half, lanes 16..31 their RoPE partners (dim + HD/2)
+    for (int j = 0; j < DPL; j++) ss = fmaf(qv[j], qv[j], ss);
+    ss = mg_warp_sum(ss);
+    const float inv = 1.0f / sqrtf(ss / (float)HD + a.eps);
+    // lanes 0..15 hold dims of the first half, lanes 16..31 their RoPE partners (dim + HD/2)
 #pragma unroll
-      for (int j = 0; j < DPL; j++) {
-        const float u = __fmul_rn(__fmul_rn(qv[j], inv), qw[j]);
-        const float pu = __shfl_xor_sync(0xffffffffu, u, 16);
-        const float r = lane < 16 ? __fsub_rn(__fmul_rn(u, qc[j]), __fmul_rn(pu, qs[j]))
-                                  : __fadd_rn(__fmul_rn(pu, qs[j]), __fmul_rn(u, qc[j]));
-        qr[j] = r * a.attn_scale;
-      }
+    for (int j = 0; j < DPL; j++) {
+      const float u = __fmul_rn(__fmul_rn(qv[j], inv), qw[j]);
+      const float pu = __shfl_xor_sync(0xffffffffu, u, 16);
+      const float r = lane < 16 ? __fsub_rn(__fmul_rn(u, qc[j]), __fmul_rn(pu, qs[j]))
+                                : __fadd_rn(__fmul_rn(pu, qs[j]), __fmul_rn(u, qc[j]));
+      sq[mg_lane_dim<DPL>(lane, j)] = r * a.attn_scale;
     }
-    if (kjob || vjob) {
-      float ss = 0.0f;
-#pragma unroll
-      for (int j = 0; j < DPL; j++) ss = fmaf(rv[j], rv[j], ss);
-      ss = mg_warp_sum(ss);
-      const float inv = 1.0f / sqrtf(ss / (float)HD + a.eps);
-      float x0 = 0.f, x1 = 0.f;  // this lane's element of block pb and of block pb + NB/2
-#pragma unroll
-      for (int j = 0; j < DPL / 2; j++)
-        if (j == pb) {
-          x0 = rv[j];
-          x1 = rv[j + DPL / 2];
-        }
-      float lo, hi;
-      if (kjob) {
-        const float u = __fmul_rn(__fmul_rn(x0, inv), r_w0), vv = __fmul_rn(__fmul_rn(x1, inv), r_w1);
-        lo = __fsub_rn(__fmul_rn(u, r_c), __fmul_rn(vv, r_s));
-        hi = __fadd_rn(__fmul_rn(u, r_s), __fmul_rn(vv, r_c));
-      } else {
-        lo = __fmul_rn(x0, inv);
-        hi = __fmul_rn(x1, inv);
-      }
-      uint8_t* dst = kjob ? skrow : svrow;
-      // values pass through f16 before packing (render.rs:1046)
-      mg_pack_q40(__half2float(__float2half_rn(lo)), dst + pb * KS_Q40_BLOCK_BYTES, lane);
-      mg_pack_q40(__half2float(__float2half_rn(hi)), dst + (pb + NB / 2) * KS_Q40_BLOCK_BYTES, lane);
+  } else if (kjob || vjob) {
+    float rv[DPL], r_w0 = 0.f, r_w1 = 0.f, r_c = 0.f, r_s = 0.f;
+    if (kjob) {
+      const float* w = L.norm[2];
+      r_w0 = w[32 * pb + lane];
+      r_w1 = w[HALF + 32 * pb + lane];
+      r_c = cs[32 * pb + lane];
+      r_s = cs[HALF + 32 * pb + lane];
     }
+    const unsigned long long* src = a.qkv_t + (size_t)a.n_q * HD + (kjob ? 0u : (size_t)a.n_kv * HD) + (size_t)kvh * HD;
+    int at[DPL];
+#pragma unroll
+    for (int j = 0; j < DPL; j++) at[j] = lane + 32 * j;
+    const bool got = tag_wait<DPL>(src, at, tag, a.poll_limit, rv);
+    if (!got) atomicOr(a.err, 2u);
+    float ss = 0.0f;
+#pragma unroll
+    for (int j = 0; j < DPL; j++) ss = fmaf(rv[j], rv[j], ss);
+    ss = mg_warp_sum(ss);
+    const float inv = 1.0f / sqrtf(ss / (float)HD + a.eps);
+    float x0 = 0.f, x1 = 0.f;  // this lane's element of block pb and of block pb + NB/2
+#pragma unroll
+    for (int j = 0; j < DPL / 2; j++)
+      if (j == pb) {
+        x0 = rv[j];
+        x1 = rv[j + DPL / 2];
+      }
+    float lo, hi;
+    if (kjob) {
+      const float u = __fmul_rn(__fmul_rn(x0, inv), r_w0), vv = __fmul_rn(__fmul_rn(x1, inv), r_w1);
+      lo = __fsub_rn(__fmul_rn(u, r_c), __fmul_rn(vv, r_s));
+      hi = __fadd_rn(__fmul_rn(u, r_s), __fmul_rn(vv, r_c));
+    } else {
+      lo = __fmul_rn(x0, inv);
+      hi = __fmul_rn(x1, inv);
+    }
+    uint8_t* dst = kjob ? skrow : svrow;
+    // values pass through f16 before packing (render.rs:1046)
+    mg_pack_q40(__half2float(__float2half_rn(lo)), dst + pb * KS_Q40_BLOCK_BYTES, lane);
+    mg_pack_q40(__half2float(__float2half_rn(hi)), dst + (pb + NB / 2) * KS_Q40_BLOCK_BYTES, lane);
   }
-  const size_t rowstride = (size_t)a.n_kv * ROWB;
-  uint8_t* Kc = L.kv_k + (size_t)kvh * ROWB;
-  uint8_t* Vc = L.kv_v + (size_t)kvh * ROWB;
+  cta_sync();
+  float qr[DPL];
+#pragma unroll
+  for (int j = 0; j < DPL; j++) qr[j] = sq[mg_lane_dim<DPL>(lane, j)] * (1.0f / raw_unit<DPL>(j));
   if (owner) {
-    __syncthreads();
     if (head == kvh * G) {
       const unsigned n16 = ROWB / 2;
-      if (threadIdx.x < n16)
-        reinterpret_cast<unsigned short*>(Kc + (size_t)pos * rowstride)[threadIdx.x] = reinterpret_cast<const unsigned short*>(skrow)[threadIdx.x];
-      else if (threadIdx.x < 2 * n16)
-        reinterpret_cast<unsigned short*>(Vc + (size_t)pos * rowstride)[threadIdx.x - n16] =
-            reinterpret_cast<const unsigned short*>(svrow)[threadIdx.x - n16];
+      if (tid < n16)
+        reinterpret_cast<unsigned short*>(Kc + (size_t)pos * rowstride)[tid] = reinterpret_cast<const unsigned short*>(skrow)[tid];
+      else if (tid < 2 * n16)
+        reinterpret_cast<unsigned short*>(Vc + (size_t)pos * rowstride)[tid - n16] =
+            reinterpret_cast<const unsigned short*>(svrow)[tid - n16];
     }
   }
   if (pf) pf[4] = clock64();
@@ -809,36 +758,52 @@ __device__ __forceinline__ void mg_attention(const MegaArgs& a, const MegaLayer&
   float o[DPL], m = kNegInit, l = 0.0f;
 #pragma unroll
   for (int j = 0; j < DPL; j++) o[j] = 0.0f;
-  {
-    RawRow<DPL> kn, vn;  // next row, in flight while the current one is processed
-    unsigned t = p0 + warp;
-    if (t < p1) {
-      raw_load<DPL>(t == pos ? skrow : Kc + (size_t)t * rowstride, lane, kn);
-      raw_load<DPL>(t == pos ? svrow : Vc + (size_t)t * rowstride, lane, vn);
-    }
-#pragma unroll 1
-    for (; t < p1; t += 8) {
-      const RawRow<DPL> kr = kn, vr = vn;
-      const unsigned t2 = t + 8;
-      if (t2 < p1) {
-        raw_load<DPL>(t2 == pos ? skrow : Kc + (size_t)t2 * rowstride, lane, kn);
-        raw_load<DPL>(t2 == pos ? svrow : Vc + (size_t)t2 * rowstride, lane, vn);
+  if (owner && t < p1) {  // the row packed above
+#pragma unroll
+    for (int i = 0; i < FLY; i++)
+      if (row_at(t, i) == pos) {
+        raw_load<DPL>(skrow, lane, kn[i]);
+        raw_load<DPL>(svrow, lane, vn[i]);
       }
-      float kv[DPL];
-      raw_decode<DPL>(kr, kv);
-      float sc = 0.0f;
+  }
+#pragma unroll 1
+  for (; t < p1; t += MG_WARPS * FLY) {
+    float kv[DPL], sc[FLY], m2 = m;
 #pragma unroll
-      for (int j = 0; j < DPL; j++) sc = fmaf(qr[j], kv[j], sc);
-      sc = mg_warp_sum(sc);
-      raw_decode<DPL>(vr, kv);
-      const float m2 = fmaxf(m, sc);
-      const float alpha = __expf(m - m2);
-      const float e = __expf(sc - m2);
-      l = l * alpha + e;
-      m = m2;
+    for (int i = 0; i < FLY; i++) {
+      raw_ints<DPL>(kn[i], kv);
+      sc[i] = 0.0f;
 #pragma unroll
-      for (int j = 0; j < DPL; j++) o[j] = fmaf(e, kv[j], o[j] * alpha);
+      for (int j = 0; j < DPL; j++) sc[i] = fmaf(qr[j], kv[j], sc[i]);
+      sc[i] *= raw_scale<DPL>(kn[i]);
     }
+    const bool more = t + MG_WARPS * FLY < p1;
+    if (more) load_rows(t + MG_WARPS * FLY, kn, Kc, skrow);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+      for (int i = 0; i < FLY; i++) sc[i] += __shfl_xor_sync(0xffffffffu, sc[i], off);
+#pragma unroll
+    for (int i = 0; i < FLY; i++) {
+      sc[i] = t + MG_WARPS * i < p1 ? sc[i] : -INFINITY;
+      m2 = fmaxf(m2, sc[i]);
+    }
+    const float alpha = __expf(m - m2);
+    l *= alpha;
+    m = m2;
+#pragma unroll
+    for (int j = 0; j < DPL; j++) o[j] *= alpha;
+#pragma unroll
+    for (int i = 0; i < FLY; i++) {
+      if (t + MG_WARPS * i >= p1) break;
+      const float e = __expf(sc[i] - m2);
+      l += e;
+      raw_ints<DPL>(vn[i], kv);
+      const float ed = e * raw_scale<DPL>(vn[i]);
+#pragma unroll
+      for (int j = 0; j < DPL; j++) o[j] = fmaf(ed, kv[j], o[j]);
+    }
+    if (more) load_rows(t + MG_WARPS * FLY, vn, Vc, svrow);
   }
   {
     float* dst = part + warp * (HD + 2);
@@ -847,65 +812,67 @@ __device__ __forceinline__ void mg_attention(const MegaArgs& a, const MegaLayer&
       dst[1] = l;
     }
 #pragma unroll
-    for (int j = 0; j < DPL; j++) dst[2 + j * 32 + lane] = o[j];
+    for (int j = 0; j < DPL; j++) dst[2 + j * 32 + lane] = o[j] * (1.0f / raw_unit<DPL>(j));
   }
-  __syncthreads();
+  cta_sync();
   if (pf) pf[5] = clock64();
-  // thread d folds head dimension d over the eight warps; it sits in slot j * 32 + lane of the warps' layout
-  const int d = threadIdx.x;
+  // thread d folds head dimension d over the warps; it sits in slot j * 32 + lane of the warps' layout
+  const int d = tid;
   int dslot;
   {
     constexpr int BPL = DPL / 2, LPB = 16 / BPL;
     const int within = d & 31, hh = within >> 4, w16 = within & 15;
     dslot = (hh * BPL + (w16 % BPL)) * 32 + ((d >> 5) * LPB + w16 / BPL);
   }
-  const unsigned ounits = (a.n_q * HD) >> 6;
   float M = kNegInit, Lsum = 0.0f, O = 0.0f;
   if (d < HD) {
-    float mw[8];
+    float mw[MG_WARPS];
 #pragma unroll
-    for (int w = 0; w < 8; w++) {
+    for (unsigned w = 0; w < MG_WARPS; w++) {
       mw[w] = part[w * (HD + 2)];
       M = fmaxf(M, mw[w]);
     }
 #pragma unroll
-    for (int w = 0; w < 8; w++) {
+    for (unsigned w = 0; w < MG_WARPS; w++) {
       const float f = __expf(mw[w] - M);
       Lsum = fmaf(part[w * (HD + 2) + 1], f, Lsum);
       O = fmaf(part[w * (HD + 2) + 2 + dslot], f, O);
     }
   }
   if (pf) pf[6] = clock64();
+  const unsigned ounits = (a.n_q * HD) >> 6;
   if (NS == 1) {  // one split: this block's result is final
     if (d < HD) fx_store_subblock(a.ox, ounits, head * HD + (d & ~31), O / Lsum, lane);
     return;
   }
-  float* rec = a.att_tmp + ((size_t)head * NSMAX + split) * (HD + 2);
+  float* rec = a.att_tmp + ((size_t)head * NSMAX + split) * mg_rec(HD);
   if (d < HD) {
-    rec[2 + d] = O;  // records are kept in dimension order
+    rec[d] = O;  // records are kept in dimension order
     if (d == 0) {
-      rec[0] = M;
-      rec[1] = Lsum;
+      rec[HD] = M;
+      rec[HD + 1] = Lsum;
     }
-    __threadfence();
   }
-  __syncthreads();
-  if (threadIdx.x == 0) *sflag = (atomicAdd(a.att_cnt + head, 1u) == NS - 1) ? 1 : 0;
-  __syncthreads();
+  if (NS <= MG_DIRECT) return;  // merged by whoever reads them, behind the grid barrier
+  __threadfence();
+  cta_sync();
+  if (tid == 0) *sflag = (atomicAdd(a.att_cnt + head, 1u) == NS - 1) ? 1 : 0;
+  cta_sync();
   if (pf) pf[7] = clock64();
   if (*sflag) {
     // last block of this head to arrive: merge the head's records, every load first
     __threadfence();
     if (d < HD) {
-      const float* rec0 = a.att_tmp + (size_t)head * NSMAX * (HD + 2);
+      const float* rec0 = a.att_tmp + (size_t)head * NSMAX * mg_rec(HD);
       float mp[MG_MAX_SPLITS], lp[MG_MAX_SPLITS], ov[MG_MAX_SPLITS];
 #pragma unroll
       for (int p = 0; p < MG_MAX_SPLITS; p++) {
         if ((unsigned)p < NS) {
-          const float* r = rec0 + (size_t)p * (HD + 2);
-          mp[p] = __ldcg(r);
-          lp[p] = __ldcg(r + 1);
-          ov[p] = __ldcg(r + 2 + d);
+          const float* r = rec0 + (size_t)p * mg_rec(HD);
+          const float2 u = __ldcg(reinterpret_cast<const float2*>(r + HD));
+          mp[p] = u.x;
+          lp[p] = u.y;
+          ov[p] = __ldcg(r + d);
         } else {
           mp[p] = kNegInit;
           lp[p] = 0.0f;
@@ -924,136 +891,204 @@ __device__ __forceinline__ void mg_attention(const MegaArgs& a, const MegaLayer&
       }
       fx_store_subblock(a.ox, ounits, head * HD + (d & ~31), OO / LL, lane);
     }
-    if (threadIdx.x == 0) a.att_cnt[head] = 0u;
+    if (tid == 0) a.att_cnt[head] = 0u;
+  }
+}
+
+// The o-projection's input out of the records of at most MG_DIRECT splits: each thread merges four neighbouring dims of a head at
+// a time, every load of a round first.
+__device__ __forceinline__ void mg_stage_merge(unsigned char* xs, const MegaArgs& a, unsigned NS, unsigned cols) {
+  const unsigned tid = mg_tid();
+  const unsigned units = cols >> 6, nchunk = cols >> 2, rec_len = mg_rec(a.hd);
+  constexpr int PER = 1;
+  for (unsigned base = tid; base < nchunk; base += PER * MG_THREADS) {  // (whole warps: nchunk is a multiple of 128)
+    float2 ml[PER][MG_DIRECT];
+    float4 o[PER][MG_DIRECT];
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+      const unsigned c = base + (unsigned)k * MG_THREADS, head = (c << 2) / a.hd, d = (c << 2) - head * a.hd;
+      const float* rec = a.att_tmp + (size_t)head * a.n_splits * rec_len;
+#pragma unroll
+      for (unsigned s = 0; s < MG_DIRECT; s++) {
+        const bool there = c < nchunk && s < NS;
+        const float* r = rec + s * rec_len;
+        ml[k][s] = there ? __ldcg(reinterpret_cast<const float2*>(r + a.hd)) : make_float2(kNegInit, 0.0f);
+        o[k][s] = there ? __ldcg(reinterpret_cast<const float4*>(r + d)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+      const unsigned c = base + (unsigned)k * MG_THREADS;
+      float M = kNegInit, Ls = 0.0f;
+      float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+      for (unsigned s = 0; s < MG_DIRECT; s++) M = fmaxf(M, ml[k][s].x);
+#pragma unroll
+      for (unsigned s = 0; s < MG_DIRECT; s++) {
+        const float f = __expf(ml[k][s].x - M);
+        Ls = fmaf(ml[k][s].y, f, Ls);
+        v.x = fmaf(o[k][s].x, f, v.x);
+        v.y = fmaf(o[k][s].y, f, v.y);
+        v.z = fmaf(o[k][s].z, f, v.z);
+        v.w = fmaf(o[k][s].w, f, v.w);
+      }
+      const float inv = 1.0f / Ls;
+      v.x *= inv; v.y *= inv; v.z *= inv; v.w *= inv;
+      if (c < nchunk) fx_put_chunk(xs, units, c, v);
+    }
   }
 }
 
 // ---- the kernel -------------------------------------------------------------------------------------
-struct MegaSmem {
-  unsigned ring_off, bar_off, red_off, flag_off, tab_off, ent_off, total;
-};
-__host__ __device__ inline MegaSmem mg_smem(unsigned x_bytes, unsigned slot_bytes, int stages, unsigned tables_bytes) {
-  MegaSmem L;
-  L.ring_off = (x_bytes + 127u) & ~127u;
-  L.bar_off = L.ring_off + 8u * (unsigned)stages * slot_bytes;
-  L.red_off = (L.bar_off + 8u * 8u * (unsigned)stages + 15u) & ~15u;
-  L.flag_off = L.red_off + 256u + MG_MAX_P * 32u;  // 32 floats for block sums, 8 float4 of per-warp norm sums, partial sums [MG_MAX_P][2][4]
-  L.tab_off = L.flag_off + 48u;  // 4 flag words, then 8 words of per-kind group counts
-  L.ent_off = L.tab_off + tables_bytes;
-  L.total = L.ent_off + 8u * MG_MAX_ENT * (unsigned)sizeof(ItemEnt);
-  return L;
+// Shared memory: what has a fixed size first, so that its addresses are constants; then the tables, x (and the attention
+// scratch) and the ring.
+constexpr unsigned SM_BAR = 0, SM_RED = SM_BAR + 2u * MG_JOBS * 8u,    // per job: its rows are there; its items are done
+                   SM_WSUM = SM_RED + 256u, SM_PSUM = SM_WSUM + MG_WARPS * 16u,
+                   SM_FLAG = SM_PSUM + MG_MAX_P * 32u,                 // 4 flag words, the copying warp's stop word, 8 words of group counts
+                   SM_JOB = SM_FLAG + 64u,                             // a job's place in the ring; bytes it takes there
+                   SM_TAB = SM_JOB + 2u * MG_JOBS * 4u;
+constexpr unsigned SM_LAYERS = SM_TAB + ((PH_PER_LAYER * (unsigned)sizeof(MegaShape) + 15u) & ~15u);
+static_assert(SM_TAB % 16u == 0 && SM_PSUM % 16u == 0, "vector access");
+
+// One thread copies the row groups of the whole token in the order they are multiplied, as far ahead as the ring has room.
+__device__ __forceinline__ void mg_copy_jobs(const MegaArgs& a, const MegaShape* shapes, const MegaLayer* layers, const unsigned* ngrp, uint32_t ring_s,
+                                             uint32_t full, uint32_t empty, unsigned* joff, unsigned* jbytes, volatile int* stop, unsigned H, unsigned pos) {
+  unsigned head = 0, tail = 0, used = 0, at = 0;
+  for (int layer = 0; layer < a.n_layers; layer++) {
+    const MegaLayer& L = layers[layer];
+    mg_prefetch_kv(a, L, pos);
+    for (int kind = 0; kind < PH_PER_LAYER; kind++) {
+      const MegaShape& sh = shapes[kind];
+      const unsigned n = ngrp[kind], row_bytes = sh.row_bytes, mats = sh.mats;
+      // in front of a phase that stages a norm: its weights, those of the norm inside the residual update behind them
+      const unsigned norms = norm_jobs(kind);
+      for (unsigned kk = 0; kk < n + norms; kk++) {
+        const bool norm = kk < norms;
+        const unsigned k = kk - norms, g = norm ? 0u : block_group_id(k);
+        unsigned seg = 0;
+        if (sh.n_seg > 1 && g >= sh.grp_start[1]) seg = 1;
+        if (sh.n_seg > 2 && g >= sh.grp_start[2]) seg = 2;
+        const unsigned row0 = (g - sh.grp_start[seg]) * MG_RL, valid = min((unsigned)MG_RL, sh.rows[seg] - row0);
+        const unsigned room = norm ? 8u * H : mats * MG_RL * row_bytes;
+        unsigned skip = at + room > a.ring_bytes ? a.ring_bytes - at : 0u, need = room + skip;  // nothing wraps
+        while (head - tail >= MG_JOBS || used + need > a.ring_bytes) {
+          const uint32_t bar = empty + (tail & (MG_JOBS - 1u)) * 8u;
+          const unsigned parity = (tail / MG_JOBS) & 1u;
+          bool ok = false;
+          for (unsigned i = 0; i < (1u << 22) && !ok && !*stop; i++) {
+            unsigned r;
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                "selp.u32 %0, 1, 0, p;\n\t}"
+                : "=r"(r)
+                : "r"(bar), "r"(parity)
+                : "memory");
+            ok = r != 0;
+          }
+          if (!ok) {
+            if (!*stop) atomicOr(a.err, 1u);
+            goto out;
+          }
+          used -= jbytes[tail & (MG_JOBS - 1u)];
+          tail++;
+          if (used == 0) {  // empty: start over, or a job of more than half the ring might never fit
+            at = 0;
+            skip = 0;
+            need = room;
+          }
+        }
+        if (skip) at = 0;
+        const unsigned b = head & (MG_JOBS - 1u);
+        joff[b] = at;
+        jbytes[b] = need;
+        mb_expect(full + b * 8u, norm ? room : mats * valid * row_bytes);  // (its arrival publishes joff)
+        if (norm) {
+          bulk_in(ring_s + at, kind == PH_QKV ? L.norm[0] : L.norm[4], 4u * H, full + b * 8u);
+          // (the first layer has no residual update in front of it: any weights)
+          bulk_in(ring_s + at + 4u * H, kind == PH_QKV ? layers[max(layer - 1, 0)].norm[5] : L.norm[3], 4u * H, full + b * 8u);
+        }
+        for (unsigned m = 0; m < mats && !norm; m++)
+          bulk_in(ring_s + at + m * MG_RL * row_bytes, L.W[sh.w0 + seg + m] + (size_t)row0 * row_bytes, valid * row_bytes, full + b * 8u);
+        at += room;
+        used += need;
+        head++;
+      }
+    }
+  }
+out:
+  // copies still in flight must land before this block's shared memory goes away (bounded)
+  for (unsigned j = tail; j < head; j++) mb_wait(full + (j & (MG_JOBS - 1u)) * 8u, (j / MG_JOBS) & 1u);
 }
 
 template <int DPL, int PC>
-__global__ void __launch_bounds__(256, 1) mega_kernel(const MegaArgs a) {
+__global__ void __launch_bounds__(MG_THREADS + 32, 1) mega_kernel(const MegaArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int cl = lane % MG_LPR, rl = lane / MG_LPR;
-  const int S = a.stages;
-  const MegaSmem SL = mg_smem(a.x_bytes, a.slot_bytes, S, a.tables_bytes);
-  const uint32_t ring_s = sm32(smem + SL.ring_off) + (uint32_t)(warp * S) * a.slot_bytes;
-  const uint32_t bars = sm32(smem + SL.bar_off) + (uint32_t)(warp * S) * 8u;
-  float* red = reinterpret_cast<float*>(smem + SL.red_off);
-  float4* wsum = reinterpret_cast<float4*>(smem + SL.red_off + 128u);
-  float* psum = reinterpret_cast<float*>(smem + SL.red_off + 256u);
-  int* sflag = reinterpret_cast<int*>(smem + SL.flag_off);
-  const MegaShape* shapes = reinterpret_cast<const MegaShape*>(smem + SL.tab_off);
-  const MegaLayer* layers = reinterpret_cast<const MegaLayer*>(smem + SL.tab_off + ((PH_PER_LAYER * sizeof(MegaShape) + 15u) & ~15u));
-  const uint32_t xs_s = sm32(smem);
+  const uint32_t ring_s = sm32(smem) + a.ring_off, full = sm32(smem) + SM_BAR, empty = full + MG_JOBS * 8u, xs_s = sm32(smem) + a.x_off;
+  unsigned char* xs = smem + a.x_off;
+  float* red = reinterpret_cast<float*>(smem + SM_RED);
+  float4* wsum = reinterpret_cast<float4*>(smem + SM_WSUM);
+  float* psum = reinterpret_cast<float*>(smem + SM_PSUM);
+  int* sflag = reinterpret_cast<int*>(smem + SM_FLAG);
+  volatile int* stop = sflag + 4;
+  unsigned* ngrp = reinterpret_cast<unsigned*>(smem + SM_FLAG + 32u);  // this block's group count per phase kind
+  unsigned* joff = reinterpret_cast<unsigned*>(smem + SM_JOB);
+  const MegaShape* shapes = reinterpret_cast<const MegaShape*>(smem + SM_TAB);
+  const MegaLayer* layers = reinterpret_cast<const MegaLayer*>(smem + SM_LAYERS);
   const unsigned bar_base = a.bar[1];
   const int n_phases = a.n_layers * PH_PER_LAYER;
+  // tag of this token's words: position and layer; a slot reset clears the words, so a replayed position never
+  // meets its own old tags
+  const unsigned pos = (unsigned)a.pos[0], tag_base = ((pos + 1u) << 8) + 1u;
 
   for (unsigned i = threadIdx.x; i < a.tables_bytes / 16u; i += blockDim.x)
-    reinterpret_cast<uint4*>(smem + SL.tab_off)[i] = reinterpret_cast<const uint4*>(a.tables)[i];
-  if (threadIdx.x == 0) sflag[2] = sflag[3] = 0;  // barrier flag words ([0] belongs to the attention phase)
-  unsigned* ngrp = reinterpret_cast<unsigned*>(smem + SL.flag_off + 16u);  // this block's group count per phase kind
-  if (threadIdx.x < PH_PER_LAYER) ngrp[threadIdx.x] = 0;
-  if (lane == 0) {
-    for (int s = 0; s < S; s++) mb_init(bars + s * 8u, 1);
+    reinterpret_cast<uint4*>(smem + SM_TAB)[i] = reinterpret_cast<const uint4*>(a.tables)[i];
+  if (threadIdx.x < MG_JOBS) {
+    mb_init(full + threadIdx.x * 8u, 1);
+    mb_init(empty + threadIdx.x * 8u, MG_EMPTY);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  if (threadIdx.x == 0) {
+    sflag[2] = sflag[3] = 0;  // barrier flag words ([0] belongs to the attention phase)
+    *stop = 0;
+  }
   __syncthreads();
   if (threadIdx.x < PH_PER_LAYER) ngrp[threadIdx.x] = block_groups(shapes[threadIdx.x]);
-  const unsigned H = shapes[PH_QKV].cols;
-
-  ItemEnt* ent = reinterpret_cast<ItemEnt*>(smem + SL.ent_off) + warp * MG_MAX_ENT;
-  int n_ent = 0;
-  if (lane == 0) n_ent = build_items(ent, shapes, warp);
-  n_ent = __shfl_sync(0xffffffffu, n_ent, 0);
-  bool dead = false;  // this warp gave up (a copy never landed, or its item table overflowed): it keeps the block-level steps only
-  if (n_ent < 0) {
-    dead = true;
-    if (lane == 0) atomicOr(a.err, 4u);
-    n_ent = 0;
-  }
-  __syncwarp();
-  ItemPos ic{n_ent > 0 ? 0 : a.n_layers, 0}, cc = ic;
-  unsigned issued = 0, consumed = 0;
-  while (issued < (unsigned)S && ic.layer < a.n_layers) {
-    const ItemEnt e = ent[ic.e];
-    mg_issue_ent(e, layers[ic.layer], shapes[e.kind].row_bytes, ring_s + issued * a.slot_bytes, bars + issued * 8u, lane);
-    issued++;
-    pos_next(ic, n_ent);
+  __syncthreads();
+  const unsigned hidden = shapes[PH_QKV].cols;
+  if (threadIdx.x >= MG_THREADS) {
+    if (threadIdx.x == MG_THREADS) mg_copy_jobs(a, shapes, layers, ngrp, ring_s, full, empty, joff, joff + MG_JOBS, stop, hidden, pos);
+    return;
   }
 
+  bool dead = false;  // this warp gave up (a copy never landed): it keeps the block-level steps only
+  unsigned job0 = 0;  // jobs of the phases before this one
   long long* prof = nullptr;
   if (threadIdx.x == 0 && (blockIdx.x == 0 || blockIdx.x == gridDim.x - 1))
     prof = a.prof + (size_t)(blockIdx.x == 0 ? 0 : 1) * n_phases * 8;
   int p = 0, layer = 0, kind = 0;
-  // tag of this token's words: position and layer; a slot reset clears the words, so a replayed position never
-  // meets its own old tags
-  const unsigned tag_base = (((unsigned)a.pos[0] + 1u) << 8) + 1u;
   for (; p < n_phases; p++) {
+    unsigned H = hidden;
+    asm volatile("" : "+r"(H));
+    const unsigned tid = mg_tid();
+    const int lane = (int)(tid & 31u), warp = (int)(tid >> 5), cl = lane % MG_LPR, rl = lane / MG_LPR;
     const MegaLayer& L = layers[layer];
-    // constants of this phase, fetched while the other blocks arrive at the barrier before it
-    NormPre<PC> npre;
-    if (kind == PH_QKV)
-      mg_prefetch_norm(npre, layer == 0 ? KS_PRO_NORM : KS_PRO_ADD_NORM, L.norm[0], layers[layer > 0 ? layer - 1 : 0].norm[5], H);
-    else if (kind == PH_GATEUP)
-      mg_prefetch_norm(npre, KS_PRO_ADD_NORM, L.norm[4], L.norm[3], H);
     // No barrier in front of attention: its inputs are tagged words.  Every block still ARRIVES after every phase,
     // so the targets of the barriers that remain are unchanged; the flag word this wait would have cleared is
-    // cleared all the same.  (The parity stays `p & 1`: written as a separate counter the same logic compiles into
-    // a kernel that is 40 % slower.)
+    // cleared all the same.
     if (p > 0 && kind == PH_ATTN) {
-      if (threadIdx.x == 0) sflag[2 + ((p & 1) ^ 1)] = 0;
+      if (tid == 0) sflag[2 + ((p & 1) ^ 1)] = 0;
     } else if (p > 0) {
       if (!grid_wait(a.bar, bar_base + (unsigned)p * gridDim.x + (p == 2 ? a.test_stall : 0u), a.err, sflag + 2, p & 1, a.poll_limit)) break;
       if (prof) prof[(p - 1) * 8 + 3] = clock64();
     }
     if (prof) prof[p * 8 + 0] = clock64();
+    unsigned n_wsum = 0;
     if (kind == PH_ATTN) {
-      mg_attention<DPL>(a, L, smem, sflag, prof ? prof + p * 8 : nullptr, tag_base + (unsigned)layer);
+      mg_attention<DPL>(a, L, xs, sflag, prof ? prof + p * 8 : nullptr, tag_base + (unsigned)layer, pos);
     } else {
       const MegaShape& sh = shapes[kind];
-      // input, prologue and outputs of this phase
-      int mode = KS_PRO_NONE;
-      const float* x;
-      const float* yin = a.yb;
-      float* out_x = nullptr;
-      if (kind == PH_QKV) {
-        mode = layer == 0 ? KS_PRO_NORM : KS_PRO_ADD_NORM;
-        x = layer == 0 ? a.x_a : a.x_b;
-        out_x = a.x_a;
-      } else if (kind == PH_OPROJ) {
-        x = nullptr;
-      } else if (kind == PH_GATEUP) {
-        mode = KS_PRO_ADD_NORM;
-        x = a.x_a;
-        out_x = a.x_b;
-      } else {
-        x = nullptr;
-      }
-      if (kind == PH_OPROJ || kind == PH_DOWN)
-        fx_copy_in(smem, kind == PH_OPROJ ? a.ox : a.ffx, sh.cols >> 6);
-      else if (mode == KS_PRO_ADD_NORM)
-        mg_stage_addnorm(smem, sh.cols, x, yin, out_x, a.eps, npre, a.nsum, gridDim.x);
-      else
-        mg_stage_x(smem, red, mode, sh.cols, x, yin, out_x, a.eps, npre);
-      __syncthreads();
-      if (prof) prof[p * 8 + 1] = clock64();
-      const unsigned units = sh.cols >> 6;
       // o-proj and down feed a residual-add + norm: their rows also leave the sums that norm needs
       const bool sums = kind == PH_OPROJ || kind == PH_DOWN;
       // Thread f finishes row (f & 3) of this block's group (f >> 2): it adds the column segments'
@@ -1063,33 +1098,66 @@ __global__ void __launch_bounds__(256, 1) mega_kernel(const MegaArgs a) {
       int fseg = 0;
       bool fin = false;
       float xr = 0.0f, wpr = 0.0f;
-      if ((threadIdx.x >> 2) < n_g) {
-        const unsigned g = block_group_id(sh, threadIdx.x >> 2);
+      if ((tid >> 2) < n_g) {
+        const unsigned g = block_group_id(tid >> 2);
         if (sh.n_seg > 1 && g >= sh.grp_start[1]) fseg = 1;
         if (sh.n_seg > 2 && g >= sh.grp_start[2]) fseg = 2;
-        frow = (g - sh.grp_start[fseg]) * MG_RL + (threadIdx.x & 3u);
-        fin = g < sh.grp_start[sh.n_seg] && frow < sh.rows[fseg];
-        if (fin && sums) {  // in flight while the items are multiplied
+        frow = (g - sh.grp_start[fseg]) * MG_RL + (tid & 3u);
+        fin = frow < sh.rows[fseg];
+        if (fin && sums) {  // in flight while x is staged
           xr = __ldcg((kind == PH_OPROJ ? a.x_a : a.x_b) + frow);
           wpr = (kind == PH_OPROJ ? L.norm[3] : L.norm[5])[frow];
         }
       }
-      while (cc.layer == layer && !dead) {
-        const ItemEnt e = ent[cc.e];
-        if (e.kind != kind) break;
-        const unsigned st = consumed % (unsigned)S;
-        if (!mb_wait(bars + st * 8u, (consumed / (unsigned)S) & 1u)) {
+      unsigned ik = (unsigned)warp / C, ics = (unsigned)warp - ik * C;  // this warp's first item
+      const unsigned dk = MG_WARPS / C, dcs = MG_WARPS - dk * C;        // from one to the next
+      // input and prologue of this phase
+      const unsigned ns_att = mg_active_splits(pos + 1u - mg_first(L, pos), a.n_splits);
+      const unsigned nb = job0 & (MG_JOBS - 1u);
+      if (norm_jobs(kind)) {
+        if (!dead && !mb_wait(full + nb * 8u, (job0 / MG_JOBS) & 1u)) {
+          dead = true;
+          if (lane == 0) atomicOr(a.err, 1u);
+        }
+        const float4* w = reinterpret_cast<const float4*>(smem + a.ring_off + (dead ? 0u : joff[nb]));
+        if (layer == 0 && kind == PH_QKV)
+          mg_stage_norm<PC>(xs, red, H, a.x_a, a.eps, w);
+        else
+          mg_stage_addnorm<PC>(xs, red, H, kind == PH_QKV ? a.x_b : a.x_a, a.yb, kind == PH_QKV ? a.x_a : a.x_b, a.eps, w, w + H / 4u, a.nsum, gridDim.x);
+      } else if (kind == PH_DOWN)
+        mg_stage_plain(xs, sh.cols, a.ff);
+      else if (ns_att > 1u && ns_att <= MG_DIRECT)
+        mg_stage_merge(xs, a, ns_att, sh.cols);
+      else
+        fx_copy_in(xs, a.ox, sh.cols >> 6);
+      cta_sync();
+      if (norm_jobs(kind)) {
+        if (tid == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(empty + nb * 8u), "n"(MG_EMPTY) : "memory");
+        job0++;
+      }
+      if (prof) prof[p * 8 + 1] = clock64();
+      const unsigned units = sh.cols >> 6;
+      for (unsigned i = (unsigned)warp; ik < n_g && !dead; i += MG_WARPS) {
+        const unsigned cs = ics, job = job0 + ik, b = job & (MG_JOBS - 1u);
+        ik += dk;
+        ics += dcs;
+        if (ics >= C) {
+          ics -= C;
+          ik++;
+        }
+        if (!mb_wait(full + b * 8u, (job / MG_JOBS) & 1u)) {
           dead = true;
           if (lane == 0) atomicOr(a.err, 1u);
           break;
         }
-        const uint32_t slot = ring_s + st * a.slot_bytes;
+        const uint32_t slot = ring_s + joff[b];
         float yacc[2] = {0.0f, 0.0f};
-        if (e.flags & 1)
-          mg_item_compute_fx<2>(slot, xs_s, units, sh.seg_blocks, e.cs, cl, rl, yacc);
+        if (kind == PH_GATEUP)
+          mg_item_compute_fx<2>(slot, sh.row_bytes, xs_s, units, sh.seg_blocks, cs, cl, rl, yacc);
         else
-          mg_item_compute_fx<1>(slot, xs_s, units, sh.seg_blocks, e.cs, cl, rl, yacc);
-        consumed++;
+          mg_item_compute_fx<1>(slot, sh.row_bytes, xs_s, units, sh.seg_blocks, cs, cl, rl, yacc);
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(empty + b * 8u), "r"(empty_share(cs, C)) : "memory");
         float v0 = yacc[0], v1 = yacc[1];
 #pragma unroll
         for (int o = MG_LPR / 2; o > 0; o >>= 1) {
@@ -1097,65 +1165,46 @@ __global__ void __launch_bounds__(256, 1) mega_kernel(const MegaArgs a) {
           v1 += __shfl_xor_sync(0xffffffffu, v1, o);
         }
         if (cl == 0) {
-          if (e.flags & 4) {
-            psum[e.pslot * 8u + 4u + (unsigned)rl] = v0;  // the up rows of a split gate-up group
-          } else {
-            psum[e.pslot * 8u + (unsigned)rl] = v0;
-            if (e.flags & 1) psum[e.pslot * 8u + 4u + (unsigned)rl] = v1;
-          }
-        }
-        pos_next(cc, n_ent);
-        // Refill now only when the next item of THIS phase is not in flight yet; everything else is
-        // refilled after the barrier arrival below, off the critical path.
-        if (ic.layer == layer && ent[ic.e].kind == kind) {
-          __syncwarp();
-          if (lane == 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the slot was read through the generic proxy
-          __syncwarp();
-          const ItemEnt ne = ent[ic.e];
-          mg_issue_ent(ne, layers[ic.layer], sh.row_bytes, slot, bars + st * 8u, lane);
-          issued++;
-          pos_next(ic, n_ent);
+          psum[i * 8u + (unsigned)rl] = v0;
+          if (kind == PH_GATEUP) psum[i * 8u + 4u + (unsigned)rl] = v1;
         }
       }
-      __syncthreads();  // the partial sums of every item of this block are in shared memory
-      float ns0 = 0.0f, ns1 = 0.0f, ns2 = 0.0f, ns3 = 0.0f, fval = 0.0f;
+      job0 += n_g;
+      cta_sync();  // the partial sums of every item of this block are in shared memory
+      float ns0 = 0.0f, ns1 = 0.0f, ns2 = 0.0f, ns3 = 0.0f;
       if (fin) {
-        const float* ps = psum + (size_t)(threadIdx.x >> 2) * C * 8u + (threadIdx.x & 3u);
+        const float* ps = psum + (size_t)(tid >> 2) * C * 8u + (tid & 3u);
         float v0 = 0.0f, v1 = 0.0f;
         for (unsigned cs = 0; cs < C; cs++) {
           v0 += ps[cs * 8u];
-          v1 += ps[cs * 8u + 4u];
+          if (kind == PH_GATEUP) v1 += ps[cs * 8u + 4u];
         }
-        fval = sh.type == MG_GATE_UP ? gelu_mul(v0, v1) : v0;
-        const float val = fval;
         if (kind == PH_QKV) {  // handed to the attention blocks as tagged words (no barrier follows this phase)
           const size_t at = fseg == 0 ? 0u : fseg == 1 ? (size_t)a.n_q * a.hd : (size_t)(a.n_q + a.n_kv) * a.hd;
-          tag_store(a.qkv_t + at + frow, val, tag_base + (unsigned)layer);
-        } else if (kind != PH_GATEUP) {
-          a.yb[frow] = val;
-        }
-        if (sums) {
-          const float t = val * wpr;
-          ns0 = val * val;
+          tag_store(a.qkv_t + at + frow, v0, tag_base + (unsigned)layer);
+        } else if (kind == PH_GATEUP) {
+          a.ff[frow] = gelu_mul(v0, v1);
+        } else {
+          a.yb[frow] = v0;
+          const float t = v0 * wpr;
+          ns0 = v0 * v0;
           ns1 = xr * t;
           ns2 = t * t;
           ns3 = xr * xr;
         }
       }
-      if (kind == PH_GATEUP && (threadIdx.x >> 2) < n_g) {
-        // this warp's 32 threads hold 32 consecutive rows (a run of 8 groups): one sub-block of the next phase's x
-        const unsigned g0 = block_group_id(sh, (threadIdx.x >> 2) & ~7u);
-        if (g0 < sh.grp_start[1]) fx_store_subblock(a.ffx, sh.rows[0] >> 6, g0 * MG_RL, fval, lane);
-      }
       if (sums) {
+        n_wsum = n_g ? (n_g * MG_RL + 31u) / 32u : 1u;
+        if ((unsigned)warp < n_wsum) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          ns0 += __shfl_xor_sync(0xffffffffu, ns0, o);
-          ns1 += __shfl_xor_sync(0xffffffffu, ns1, o);
-          ns2 += __shfl_xor_sync(0xffffffffu, ns2, o);
-          ns3 += __shfl_xor_sync(0xffffffffu, ns3, o);
+          for (int o = 16; o > 0; o >>= 1) {
+            ns0 += __shfl_xor_sync(0xffffffffu, ns0, o);
+            ns1 += __shfl_xor_sync(0xffffffffu, ns1, o);
+            ns2 += __shfl_xor_sync(0xffffffffu, ns2, o);
+            ns3 += __shfl_xor_sync(0xffffffffu, ns3, o);
+          }
+          if (lane == 0) wsum[warp] = make_float4(ns0, ns1, ns2, ns3);
         }
-        if (lane == 0) wsum[warp] = make_float4(ns0, ns1, ns2, ns3);
       }
     }
     if (prof) prof[p * 8 + 2] = clock64();
@@ -1163,27 +1212,14 @@ __global__ void __launch_bounds__(256, 1) mega_kernel(const MegaArgs a) {
       p++;
       break;
     }
-    grid_arrive(a.bar, (kind == PH_OPROJ || kind == PH_DOWN) ? wsum : nullptr, a.nsum);
-    // refill the ring while the other blocks arrive
-    if (!dead && issued - consumed < (unsigned)S && ic.layer < a.n_layers) {
-      if (lane == 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      while (issued - consumed < (unsigned)S && ic.layer < a.n_layers) {
-        const unsigned st = issued % (unsigned)S;
-        const ItemEnt ne = ent[ic.e];
-        mg_issue_ent(ne, layers[ic.layer], shapes[ne.kind].row_bytes, ring_s + st * a.slot_bytes, bars + st * 8u, lane);
-        issued++;
-        pos_next(ic, n_ent);
-      }
-    }
+    grid_arrive(a.bar, wsum, n_wsum, a.nsum);
     if (++kind == PH_PER_LAYER) {
       kind = 0;
       layer++;
     }
   }
   if (p == n_phases && blockIdx.x == 0 && threadIdx.x == 0) a.bar[1] = bar_base + (unsigned)(n_phases - 1) * gridDim.x;
-  // copies still in flight must land before this block's shared memory goes away (bounded)
-  for (unsigned j = consumed; j < issued; j++) mb_wait(bars + (j % (unsigned)S) * 8u, (j / (unsigned)S) & 1u);
+  if (p < n_phases || dead) *stop = 1;  // the copying warp need not wait for the rest to be used
 }
 
 }  // namespace
@@ -1197,10 +1233,11 @@ struct ks_mega {
   long long* d_prof = nullptr;
   unsigned long long* d_qkv = nullptr;  // tagged q | k | v words
   size_t qkv_words = 0;
-  unsigned char* d_fx = nullptr;  // attention output and GeGLU output in the staged layout
+  unsigned char* d_fx = nullptr;  // merged attention output in the staged layout, GeGLU output
+  float* d_att = nullptr;         // records of the attention splits
   unsigned grid = 0;
   size_t smem = 0;
-  int G = 0, dpl = 0, pc = 4;  // pc: 4-element chunks of the hidden vector per thread (2 up to 2048 columns)
+  int G = 0, dpl = 0, pc = 2;  // pc: 4-element chunks of the hidden vector per thread (480 threads)
   float* residual = nullptr;  // buffer that holds the residual stream when the kernel ends
 };
 
@@ -1216,7 +1253,7 @@ int mega_launch_t(ks_ctx* ctx, ks_mega* mg) {
   }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(mg->grid);
-  cfg.blockDim = dim3(256);
+  cfg.blockDim = dim3(MG_THREADS + 32);
   cfg.dynamicSmemBytes = mg->smem;
   cfg.stream = ctx->stream;
   cudaLaunchAttribute attr[1];
@@ -1231,8 +1268,8 @@ int mega_launch_t(ks_ctx* ctx, ks_mega* mg) {
 }  // namespace
 
 int ks_mega_launch(ks_ctx* ctx, ks_mega* mg) {
-  if (mg->dpl == 4) return mg->pc == 2 ? mega_launch_t<4, 2>(ctx, mg) : mega_launch_t<4, 4>(ctx, mg);
-  if (mg->dpl == 8) return mg->pc == 2 ? mega_launch_t<8, 2>(ctx, mg) : mega_launch_t<8, 4>(ctx, mg);
+  if (mg->dpl == 4) return mg->pc == 1 ? mega_launch_t<4, 1>(ctx, mg) : mg->pc == 2 ? mega_launch_t<4, 2>(ctx, mg) : mega_launch_t<4, 3>(ctx, mg);
+  if (mg->dpl == 8) return mg->pc == 1 ? mega_launch_t<8, 1>(ctx, mg) : mg->pc == 2 ? mega_launch_t<8, 2>(ctx, mg) : mega_launch_t<8, 3>(ctx, mg);
   return ks_fail(ctx, KS_ERR_UNSUPPORTED, "decode kernel: head size not supported");
 }
 
@@ -1266,6 +1303,7 @@ void ks_mega_destroy(ks_mega* mg) {
   if (mg->d_qkv) cudaFree(mg->d_qkv);
   if (mg->d_prof) cudaFree(mg->d_prof);
   if (mg->d_fx) cudaFree(mg->d_fx);
+  if (mg->d_att) cudaFree(mg->d_att);
   delete mg;
 }
 
@@ -1280,41 +1318,38 @@ int ks_mega_create(ks_ctx* ctx, const ks_mega_desc* d, const ks_mega_layer* laye
   if (!even_blocks(H) || !even_blocks(F) || !even_blocks(qn)) return KS_OK;
   if (H > 16u * 256u) return KS_OK;  // the fused norms hold the vector in registers
   if (G < 1 || nq % nkv || !(hd == 128 || hd == 256)) return KS_OK;
-  // one block per (query head, split): fewer splits than the caller's record layout allows if the grid is small
-  unsigned n_splits = (unsigned)d->n_splits;
-  if (n_splits > (unsigned)ctx->sm_count / nq) n_splits = (unsigned)ctx->sm_count / nq;
+  // one block per (query head, split)
+  unsigned n_splits = (unsigned)ctx->sm_count / nq;
   if (n_splits > (unsigned)MG_MAX_SPLITS) n_splits = MG_MAX_SPLITS;
   if (n_splits < 1 || nq > 48) return KS_OK;
   if (d->n_layers < 1 || d->n_layers > 128) return KS_OK;
 
-  const int stages = 3;
-  const unsigned shapes_bytes = (unsigned)((PH_PER_LAYER * sizeof(MegaShape) + 15u) & ~15u);
+  const unsigned shapes_bytes = SM_LAYERS - SM_TAB;
   const unsigned tables_bytes = (unsigned)((shapes_bytes + d->n_layers * sizeof(MegaLayer) + 15u) & ~15u);
   unsigned maxcols = H > F ? H : F;
   if (qn > maxcols) maxcols = qn;
-  unsigned x_bytes = (maxcols / 64u) * Q4K_XTOK * 4u;
+  unsigned x_bytes = (maxcols / 64u) * (3u * MG_XU + 16u);
   const unsigned att = mg_att_bytes(hd);
   if (att > x_bytes) x_bytes = att;
-  const unsigned budget = (unsigned)ctx->smem_optin;
-  const MegaSmem fixed = mg_smem(x_bytes, 0, stages, tables_bytes);
-  if (fixed.total + 8u * stages * 4u * KS_Q4K_BLOCK_BYTES * 2u > budget) return KS_OK;
-  unsigned slot_cap = (budget - fixed.total) / (8u * stages);
-  slot_cap &= ~15u;
-  if (slot_cap > 8192u) slot_cap = 8192u;
-  // Blocks per column segment.  A block's items (its groups x column segments) are shared by its 8
-  // warps, so more segments shorten the longest warp until the per-item overhead (measured: a little more
-  // than one unit's worth of time) wins; segments hold an even number of blocks (8 lanes per row) and must fit a ring slot.
+  const unsigned x_off = (SM_TAB + tables_bytes + 127u) & ~127u, head = (x_off + x_bytes + 127u) & ~127u;
+  unsigned most_job = 4u * (maxcols > 2u * H ? maxcols : 2u * H) / 256u * KS_Q4K_BLOCK_BYTES;  // (gate and up rows are one job)
+  if (most_job < 8u * H) most_job = 8u * H;
+  if (head + most_job + 128u > (unsigned)ctx->smem_optin) return KS_OK;
+  const unsigned ring_bytes = ((unsigned)ctx->smem_optin - head) & ~127u;
+  // Blocks per column segment.  A block's items (its groups x column segments) are shared by its warps, so more segments shorten
+  // the longest warp until the per-item overhead (measured: a little more than one unit's worth of time) wins; segments hold an
+  // even number of blocks (8 lanes per row).
   const unsigned grid = (unsigned)ctx->sm_count;
-  auto pick_seg = [&](unsigned cols, unsigned mats, unsigned total_groups, bool oct = false) {
-    const unsigned nb = cols / 256u;
-    const unsigned n_g = oct ? ((total_groups + 7) / 8 + grid - 1) / grid * 8 : (total_groups + grid - 1) / grid;
+  if (grid > MG_THREADS) return KS_OK;  // a thread folds the norm sums of a block
+  auto pick_seg = [&](unsigned cols, unsigned mats, unsigned total_groups) {
+    const unsigned nb = cols / 256u, n_g = (total_groups + grid - 1) / grid;
     unsigned best = 0;
     float best_cost = 0.f;
-    for (unsigned C = 1; C <= nb; C++) {
+    for (unsigned C = 1; C <= nb && C < MG_EMPTY; C++) {
       if (nb % C) continue;
       const unsigned sb = nb / C;
-      if (sb % 2 || 4u * mats * sb * KS_Q4K_BLOCK_BYTES > slot_cap || n_g * C > (unsigned)MG_MAX_P) continue;
-      const float cost = (float)((n_g * C + 7u) / 8u) * ((float)(sb * mats) * 0.5f + 1.2f);
+      if (sb % 2 || n_g * C > (unsigned)MG_MAX_P) continue;
+      const float cost = (float)((n_g * C + MG_WARPS - 1u) / MG_WARPS) * ((float)(sb * mats) * 0.5f + 1.2f);
       if (!best || cost < best_cost) {
         best = sb;
         best_cost = cost;
@@ -1323,44 +1358,16 @@ int ks_mega_create(ks_ctx* ctx, const ks_mega_desc* d, const ks_mega_layer* laye
     return best;
   };
   const unsigned g_qkv = (qn + 3) / 4 + 2 * ((kvn + 3) / 4), g_h = (H + 3) / 4, g_f = (F + 3) / 4;
-  if (g_qkv > 64u * grid || g_f > 64u * grid || g_h > 64u * grid) return KS_OK;  // a block finishes at most 64 groups per phase
-  const unsigned sb_h = pick_seg(H, 1, g_qkv), sb_q = pick_seg(qn, 1, g_h), sb_f = pick_seg(F, 1, g_h);
-  // gate-up: gate and up rows of a group in one item (x read once for both) when they fit a slot, else as two items
-  unsigned sb_h2 = pick_seg(H, 2, g_f, true);
-  bool gu_split = false;
-  if (!sb_h2) {
-    gu_split = true;
-    const unsigned n_g = ((g_f + 7) / 8 + grid - 1) / grid * 8, nb = H / 256u;
-    float best_cost = 0.f;
-    for (unsigned C = 1; C <= nb; C++) {
-      if (nb % C) continue;
-      const unsigned sb = nb / C;
-      if (sb % 2 || 4u * sb * KS_Q4K_BLOCK_BYTES > slot_cap || n_g * C > (unsigned)MG_MAX_P) continue;
-      const float cost = (float)((n_g * C * 2u + 7u) / 8u) * ((float)sb * 0.5f + 1.2f);
-      if (!sb_h2 || cost < best_cost) {
-        sb_h2 = sb;
-        best_cost = cost;
-      }
-    }
-  }
+  const unsigned most_g = MG_THREADS / MG_RL * grid;  // a block finishes a row per thread
+  if (g_qkv > most_g || g_f > most_g || g_h > most_g) return KS_OK;
+  const unsigned sb_h = pick_seg(H, 1, g_qkv), sb_q = pick_seg(qn, 1, g_h), sb_f = pick_seg(F, 1, g_h), sb_h2 = pick_seg(H, 2, g_f);
   if (!sb_h || !sb_h2 || !sb_q || !sb_f) return KS_OK;
-  unsigned slot_bytes = 0;
-  auto upd = [&](unsigned sb, unsigned mats) {
-    const unsigned b = 4u * mats * sb * KS_Q4K_BLOCK_BYTES;
-    if (b > slot_bytes) slot_bytes = b;
-  };
-  upd(sb_h, 1); upd(sb_h2, gu_split ? 1 : 2); upd(sb_q, 1); upd(sb_f, 1);
-
-  {  // every warp's items of one layer must fit its table
-    auto per_warp = [&](unsigned total_groups, unsigned ncs) { return ((total_groups + grid - 1) / grid * ncs + 7u) / 8u; };
-    const unsigned worst = per_warp(g_qkv, H / 256 / sb_h) + per_warp(g_h, qn / 256 / sb_q) +
-                           (((g_f + 7) / 8 + grid - 1) / grid * 8 * (H / 256 / sb_h2) * (gu_split ? 2u : 1u) + 7u) / 8u +
-                           per_warp(g_h, F / 256 / sb_f);
-    if (worst > (unsigned)MG_MAX_ENT) return KS_OK;
-  }
   std::vector<unsigned char> tab(tables_bytes, 0);
   MegaShape* sh = reinterpret_cast<MegaShape*>(tab.data());
   MegaLayer* ly = reinterpret_cast<MegaLayer*>(tab.data() + shapes_bytes);
+  for (int k = 0; k < PH_PER_LAYER; k++) sh[k].mats = 1;
+  sh[PH_OPROJ].w0 = 3;
+  sh[PH_DOWN].w0 = 6;
   auto set_rows = [](MegaShape& p, unsigned cols, unsigned sb) {
     p.cols = cols;
     p.row_bytes = cols / 256u * KS_Q4K_BLOCK_BYTES;
@@ -1379,7 +1386,7 @@ int ks_mega_create(ks_ctx* ctx, const ks_mega_desc* d, const ks_mega_layer* laye
   sh[PH_ATTN].type = MG_ATTN; sh[PH_ATTN].n_seg = 1; sh[PH_ATTN].n_cseg = 1;
   sh[PH_OPROJ].type = MG_MATVEC; sh[PH_OPROJ].n_seg = 1; sh[PH_OPROJ].rows[0] = H;
   set_rows(sh[PH_OPROJ], qn, sb_q);
-  sh[PH_GATEUP].type = MG_GATE_UP; sh[PH_GATEUP].n_seg = 1; sh[PH_GATEUP].rows[0] = F; sh[PH_GATEUP].oct = 1; sh[PH_GATEUP].split = gu_split ? 1 : 0;
+  sh[PH_GATEUP].type = MG_GATE_UP; sh[PH_GATEUP].n_seg = 1; sh[PH_GATEUP].rows[0] = F; sh[PH_GATEUP].mats = 2; sh[PH_GATEUP].w0 = 4;
   set_rows(sh[PH_GATEUP], H, sb_h2);
   sh[PH_DOWN].type = MG_MATVEC; sh[PH_DOWN].n_seg = 1; sh[PH_DOWN].rows[0] = H;
   set_rows(sh[PH_DOWN], F, sb_f);
@@ -1399,14 +1406,15 @@ int ks_mega_create(ks_ctx* ctx, const ks_mega_desc* d, const ks_mega_layer* laye
   const size_t n_phases = (size_t)d->n_layers * PH_PER_LAYER;
   if (cudaMalloc(&mg->d_tables, tables_bytes) != cudaSuccess || cudaMalloc((void**)&mg->d_sync, 512 + 16 * (size_t)ctx->sm_count) != cudaSuccess ||
       cudaMalloc((void**)&mg->d_prof, n_phases * 16 * sizeof(long long)) != cudaSuccess ||
-      cudaMalloc((void**)&mg->d_fx, ((size_t)qn / 64 + (size_t)F / 64) * 256) != cudaSuccess ||
+      cudaMalloc((void**)&mg->d_fx, (size_t)qn / 64 * 256 + F * sizeof(float)) != cudaSuccess ||
+      cudaMalloc((void**)&mg->d_att, (size_t)nq * n_splits * mg_rec(hd) * sizeof(float)) != cudaSuccess ||
       cudaMalloc((void**)&mg->d_qkv, ((size_t)qn + 2 * (size_t)kvn) * sizeof(unsigned long long)) != cudaSuccess) {
     ks_mega_destroy(mg);
     return ks_fail(ctx, KS_ERR_OOM, "decode kernel: cannot allocate its tables");
   }
   cudaError_t e = cudaMemcpyAsync(mg->d_tables, tab.data(), tables_bytes, cudaMemcpyHostToDevice, ctx->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(mg->d_sync, 0, 512 + 16 * (size_t)ctx->sm_count, ctx->stream);
-  if (e == cudaSuccess) e = cudaMemsetAsync(mg->d_fx, 0, ((size_t)qn / 64 + (size_t)F / 64) * 256, ctx->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(mg->d_fx, 0, (size_t)qn / 64 * 256 + F * sizeof(float), ctx->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(mg->d_prof, 0, n_phases * 16 * sizeof(long long), ctx->stream);
   mg->qkv_words = (size_t)qn + 2 * (size_t)kvn;
   if (e == cudaSuccess) e = cudaMemsetAsync(mg->d_qkv, 0, mg->qkv_words * sizeof(unsigned long long), ctx->stream);
@@ -1419,17 +1427,17 @@ int ks_mega_create(ks_ctx* ctx, const ks_mega_desc* d, const ks_mega_layer* laye
   a.tables = mg->d_tables;
   a.tables_bytes = tables_bytes;
   a.n_layers = d->n_layers;
-  a.stages = stages;
-  a.slot_bytes = slot_bytes;
-  a.x_bytes = x_bytes;
+  a.ring_bytes = ring_bytes;
+  a.x_off = x_off;
+  a.ring_off = head;
   a.n_q = nq; a.n_kv = nkv; a.hd = hd; a.n_splits = n_splits;
   a.eps = d->eps; a.attn_scale = d->attn_scale;
   a.rope = d->rope; a.pos = d->pos;
   a.x_a = d->x_a; a.x_b = d->x_b;
   a.yb = d->yb;
   a.ox = mg->d_fx;
-  a.ffx = mg->d_fx + (size_t)qn / 64 * 256;
-  a.att_tmp = d->att_tmp;
+  a.ff = reinterpret_cast<float*>(mg->d_fx + (size_t)qn / 64 * 256);
+  a.att_tmp = mg->d_att;
   a.bar = mg->d_sync;
   a.qkv_t = mg->d_qkv;
   a.att_cnt = mg->d_sync + 64;
@@ -1439,10 +1447,10 @@ int ks_mega_create(ks_ctx* ctx, const ks_mega_desc* d, const ks_mega_layer* laye
   a.test_stall = 0;
   a.prof = mg->d_prof;
   mg->grid = grid;
-  mg->smem = mg_smem(x_bytes, slot_bytes, stages, tables_bytes).total;
+  mg->smem = head + ring_bytes;
   mg->G = (int)G;
   mg->dpl = (int)(hd / 32);
-  mg->pc = H <= 2048 ? 2 : 4;
+  mg->pc = (int)((H / 4u + MG_THREADS - 1u) / MG_THREADS);
   mg->residual = d->x_b;
   *out = mg;
   return KS_OK;
