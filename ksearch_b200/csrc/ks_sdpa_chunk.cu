@@ -2,95 +2,95 @@
 //
 // The reference runs its decode attention once per prompt row (forward_prefill_chunk, crates/ksearch_gemma/src/
 // gemma_prim.rs:1463-1472, over crates/ksearch_codegen/src/lower.rs:4897-6088), so every row reads the whole context again.
-// Here a block takes 64 query rows that share a KV head (64 / G tokens x the head's G query heads), brings each tile of 64
-// positions in once and multiplies on the tensor cores (mma.sync m16n8k16, f16 in, f32 out) without giving up f32 accuracy:
-//   scores   a cached K value is d (n - 8) with a 4-bit n: the integer n - 8 is exact in f16, q is split into two f16 terms
-//            (scaled per row by a power of two), and each 32-dim block's integer product is multiplied by its d in f32;
-//   values   d (n - 8) has 15 significant bits: two f16 terms hold it exactly; the probabilities are split the same way and
-//            p_hi v_hi + p_lo v_hi + p_hi v_lo leaves out 2^-22.
-// Eight warps: warp (r, h) owns rows 16 r .. +16; it scores half h of the tile's positions and gathers half h of the
-// dims.  Probabilities cross between the two through shared memory; the running maximum does too.
+// Here a block takes 128 query rows that share a KV head (128 / G tokens x the head's G query heads), brings each tile of 64
+// positions in once and multiplies on tcgen05 (f16 in, f32 out) without giving up f32 accuracy: q (scaled per row by a power of
+// two), the cached values d (n - 8), exactly, and the probabilities are two f16 terms each, a product is hi hi + hi lo + lo hi.
+//   * q's first term and the probabilities lie in TENSOR memory as the A operand, q's second term and the decoded tile in shared
+//     memory; scores and a tile's values are the accumulators (HD = 256 fills the 512 columns);
+//   * four warps own a row of scores per thread: mask, running maximum, probabilities;
+//   * eight decode: K as positions x dims, V as dims x positions (a thread takes one byte of eight neighbouring rows), and add each
+//     tile's values, scaled as the maximum moved, to f32 registers, half a row per thread (184 registers);
+//   * one issues.  The scores of the next tile follow the values of this one in the tensor pipe, and meanwhile the decoders work;
+//     what the pipe waits for is the probabilities.
+// The sums leave tensor memory after every tile and small terms come first, because the accumulator truncates: against 64 bits the
+// result is off by 1.3..1.8e-7 (2-norm) whatever the context, where accumulating on gave 3e-6 over 2047 positions, 1e-5 over 4000.
 // The context is split over blockIdx.z; (m, l, O) records go to `tmp` as the decode kernels leave them and
-// sdpa_chunk_merge_kernel folds them straight into the operand image of the output projection.
+// sdpa_merge_split_kernel folds them straight into the operand image of the output projection.
 //
-// Bound by shared-memory reads of the operands (about 4300 cycles per 64 x 64 tile) and mma issue (about 5100 cycles at
-// 1024 MAC per cycle and SM); decoding the cache is a tenth of that.
+// Bound by the chain scores -> probabilities -> values of a tile: about 2.2 us for 128 x 64, 1.5 of them MMAs.  2047 rows of 8
+// heads: 109 us; 2000 rows behind 2000 positions, 2 KV heads: 299.  On mma.sync (64 rows a block) the same took 336 and 809.
 #include "ks_gemm_common.cuh"
 
 namespace {
 
-constexpr int CH_BM = 64, CH_BN = 64, CH_THREADS = 256;
+constexpr int CH_BM = 128, CH_BN = 64;                 // query rows, positions of a tile
+constexpr int CH_ROW_WARPS = 4, CH_DEC_WARPS = 8, CH_WORK = (CH_ROW_WARPS + CH_DEC_WARPS) * 32, CH_THREADS = CH_WORK + 128;
+constexpr unsigned CH_WAIT = 1u << 20;
+constexpr float CH_P = 256.0f;                         // probabilities carry 2^8
 constexpr float kNegInit = -1.0e30f;
+
+// barriers: operands ready (decoders, row warps), the tile's O taken (decoders), products ready (commits: scores done = K free;
+// values done = V and P free)
+enum { CB_K_FULL, CB_V_FULL, CB_P_FULL, CB_O_FREE, CB_S_FULL, CB_K_FREE, CB_V_FREE, CB_DONE, CB_COUNT };
 
 template <int HD>
 struct ChunkSmem {
   static constexpr unsigned NB = HD / 32, ROWB = NB * KS_Q40_BLOCK_BYTES, RP = ROWB + 4;
-  static constexpr unsigned LD = HD + 8;            // halves per row of q, K, V: 16 bytes off a multiple of 128
-  static constexpr unsigned LP = CH_BN + 8;         // halves per row of p
-  static constexpr unsigned qh = 0, ql = qh + CH_BM * LD * 2, k = ql + CH_BM * LD * 2, vh = k + CH_BN * LD * 2, vl = vh + CH_BN * LD * 2,
-                            ph = vl + CH_BN * LD * 2, pl = ph + CH_BM * LP * 2, dk = pl + CH_BM * LP * 2, raw = dk + NB * CH_BN * 4,
-                            row = raw + 2 * CH_BN * RP,   // per row: scale, first, past the last position
-                            red = row + CH_BM * 12, total = red + 4 * CH_BM * 4;
+  static constexpr unsigned slot = 64, row = 128;     // tensor-memory address, failure flag; per row: scale, first, past the last position, maximum,
+                                                      // then what the sums so far are multiplied by, of two tiles
+  static constexpr unsigned raw = 4096;
+  static constexpr unsigned ql = (raw + 2 * CH_BN * RP + 1023u) & ~1023u, kh = ql + CH_BM * HD * 2, kl = kh + CH_BN * HD * 2, vh = kl + CH_BN * HD * 2,
+                            vl = vh + CH_BN * HD * 2, total = vl + CH_BN * HD * 2;
+  static constexpr unsigned o = ql, OP = HD + 4;      // the result on its way out: rows of OP floats
+  static_assert(o + CH_BM * OP * 4 <= total, "the result fits the operands");
+  // tensor memory: first term of q, scores, the probabilities' two terms, O
+  static constexpr unsigned t_q = 0, t_s = HD / 2, t_ph = t_s + CH_BN, t_pl = t_ph + CH_BN / 2, t_o = t_pl + CH_BN / 2;
+  static_assert(t_o + HD <= 512, "tensor memory");
 };
 
-__device__ __forceinline__ void ldsm4(uint32_t a, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
-}
-__device__ __forceinline__ void ldsm4t(uint32_t a, uint32_t (&r)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
-}
-__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
+__device__ __forceinline__ void mb_arrive1(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ void cp4(uint32_t dst, const void* src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory"); }
-
-// Two neighbouring Q4_0 blocks (36 bytes, nine words) -> their scales and 2 x 32 values n - 8 as half2 pairs in dim order.
-struct Pair40 {
-  __half d[2];
-  __half2 v[2][16];
-};
-__device__ __forceinline__ void decode_pair(const uint32_t* w, Pair40& o) {
-  uint32_t q[2][4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    q[0][i] = __funnelshift_r(w[i], w[i + 1], 16);
-    q[1][i] = w[5 + i];
-  }
-  o.d[0] = __ushort_as_half((unsigned short)(w[0] & 0xFFFFu));
-  o.d[1] = __ushort_as_half((unsigned short)(w[4] >> 16));
-  const __half2 off = __float2half2_rn(1032.0f);
-#pragma unroll
-  for (int b = 0; b < 2; b++)
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const uint32_t lo = q[b][i] & 0x0F0F0F0Fu, hi = (q[b][i] >> 4) & 0x0F0F0F0Fu;  // dims 4 i .. +3 and 16 + 4 i .. +3
-      o.v[b][2 * i] = __hsub2(as_h2(__byte_perm(lo, 0, 0x4140) | 0x64006400u), off);
-      o.v[b][2 * i + 1] = __hsub2(as_h2(__byte_perm(lo, 0, 0x4342) | 0x64006400u), off);
-      o.v[b][8 + 2 * i] = __hsub2(as_h2(__byte_perm(hi, 0, 0x4140) | 0x64006400u), off);
-      o.v[b][8 + 2 * i + 1] = __hsub2(as_h2(__byte_perm(hi, 0, 0x4342) | 0x64006400u), off);
-    }
+// The decoders meet; true if every one of them says so.
+__device__ __forceinline__ bool dec_all(bool ok) {
+  unsigned r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "barrier.cta.red.and.pred q, 1, %2, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"((unsigned)ok), "n"(CH_DEC_WARPS * 32)
+      : "memory");
+  return r != 0;
 }
+// d (n - 8) of two values as two f16 terms, exactly.
+__device__ __forceinline__ void split_d(__half2 n, __half2 d, uint32_t& hi, uint32_t& lo) {
+  const __half2 x = __hmul2(n, d);
+  hi = pack_h2(x);
+  lo = pack_h2(__hfma2(n, d, __hneg2(x)));
+}
+__device__ __forceinline__ __half2 nib_h2(uint32_t w) { return __hsub2(as_h2((w & 0x000F000Fu) | 0x64006400u), __float2half2_rn(1032.0f)); }  // nibbles 0 of bytes 0 and 2
 
 template <int HD>
 __global__ void __launch_bounds__(CH_THREADS, 1)
 sdpa_chunk_kernel(unsigned n_tok, unsigned n_q, unsigned n_kv, float scale, const float* q, const uint8_t* K, const uint8_t* V, const float* meta,
-                  float* tmp, unsigned n_splits) {
+                  float* tmp, unsigned n_splits, unsigned* err) {
   using S = ChunkSmem<HD>;
-  constexpr unsigned NB = S::NB, LD = S::LD, LP = S::LP, RP = S::RP, ROWB = S::ROWB;
-  constexpr int NT = HD / 16;   // 8-dim output tiles of a warp (half the head)
-  extern __shared__ __align__(128) unsigned char smem[];
+  constexpr unsigned NB = S::NB, RP = S::RP, ROWB = S::ROWB;
+  extern __shared__ __align__(1024) unsigned char smem[];
   ks_pdl_entry();
-  const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, rg = warp >> 1, h = warp & 1u;
+  const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const unsigned G = n_q / n_kv, kvh = blockIdx.y, split = blockIdx.z;
   const unsigned row0 = (gridDim.x - 1u - blockIdx.x) * CH_BM;  // the last rows see the most: they start first
   const uint32_t sb = sm32(smem);
+  auto bar = [&](unsigned i) { return sb + 8u * i; };
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + S::slot);
+  volatile unsigned* fail = reinterpret_cast<volatile unsigned*>(smem + S::slot + 8);
   float* row_scale = reinterpret_cast<float*>(smem + S::row);
   int* row_first = reinterpret_cast<int*>(smem + S::row + CH_BM * 4);
   int* row_end = reinterpret_cast<int*>(smem + S::row + CH_BM * 8);
-  float* red = reinterpret_cast<float*>(smem + S::red);
-  float* dk = reinterpret_cast<float*>(smem + S::dk);
+  unsigned* row_max = reinterpret_cast<unsigned*>(smem + S::row + CH_BM * 12);
+  float* row_alpha = reinterpret_cast<float*>(smem + S::row + CH_BM * 16);
 
   // ---- the block's rows: row r is query head kvh G + r % G of token (row0 + r) / G; positions they see at all
   const unsigned tok_a = row0 / G, tok_b = min((row0 + CH_BM - 1u) / G, n_tok - 1u);
@@ -98,250 +98,325 @@ sdpa_chunk_kernel(unsigned n_tok, unsigned n_q, unsigned n_kv, float scale, cons
   const int pmax = (int)meta[tok_b * 4 + 0] + (int)meta[tok_b * 4 + 1];
   const int span = (pmax - pmin + CH_BN - 1) / CH_BN, per = (span + (int)n_splits - 1) / (int)n_splits;
   const int t_begin = pmin + (int)split * per * CH_BN, t_end = min(pmin + (int)(split + 1u) * per * CH_BN, pmax);
-
-  auto fetch = [&](int t0) {  // the packed rows of positions t0 .. +64 (zeros past the end are masked, rows are clamped)
-    for (unsigned r = warp; r < 2u * CH_BN; r += CH_THREADS / 32) {
-      const unsigned p = r & (CH_BN - 1u);
-      const int pos = min(t0 + (int)p, pmax - 1);
+  const unsigned n_tiles = t_begin < t_end ? (unsigned)((t_end - t_begin + CH_BN - 1) / CH_BN) : 0u;
+  if (n_tiles == 0u) {  // an empty record is all the merge needs
+    for (unsigned r = tid; r < CH_BM; r += CH_THREADS) {
+      const unsigned t = (row0 + r) / G, head = kvh * G + (row0 + r) % G;
+      if (t < n_tok) *reinterpret_cast<float2*>(tmp + (((size_t)t * n_q + head) * n_splits + split) * (HD + 2)) = make_float2(kNegInit, 0.0f);
+    }
+    return;
+  }
+  const bool decoder = warp >= CH_ROW_WARPS && warp < CH_ROW_WARPS + CH_DEC_WARPS;
+  const unsigned dt = tid - CH_ROW_WARPS * 32;  // decoders: 0..255
+  auto fetch = [&](int t0) {  // the packed rows of positions t0 .. +64 (rows past the end repeat the last, their scores are masked)
+    for (unsigned r = dt >> 5; r < 2u * CH_BN; r += CH_DEC_WARPS) {
+      const int pos = min(t0 + (int)(r & (CH_BN - 1u)), pmax - 1);
       const uint8_t* src = (r < CH_BN ? K : V) + ((size_t)pos * n_kv + kvh) * ROWB;
       const uint32_t dst = sb + S::raw + r * RP;
       for (unsigned w = lane; w < ROWB / 4u; w += 32u) cp4(dst + 4u * w, src + 4u * w);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  if (t_begin < t_end) fetch(t_begin);
+  if (decoder) fetch(t_begin);
 
-  for (unsigned r = warp; r < CH_BM; r += CH_THREADS / 32) {
-    const unsigned t = (row0 + r) / G, head = kvh * G + (row0 + r) % G;
-    float v[HD / 32];
+  if (tid == 0) {
+    mb_init(bar(CB_K_FULL), CH_DEC_WARPS);
+    mb_init(bar(CB_V_FULL), CH_DEC_WARPS);
+    mb_init(bar(CB_P_FULL), CH_ROW_WARPS);
+    mb_init(bar(CB_O_FREE), CH_DEC_WARPS);
+    for (unsigned i = CB_S_FULL; i < CB_COUNT; i++) mb_init(bar(i), 1);
+    *fail = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (tid < CH_BM) row_max[tid] = 0u;
+  if (warp == CH_ROW_WARPS + CH_DEC_WARPS) tc_alloc(sm32(tslot), 512);
+  __syncthreads();
+
+  // ---- q: a thread takes every third chunk of 8 dims of a row; the row maximum sets a power of two, then two f16 terms per value.
+  // The second term stays in shared memory as core matrices, the first passes through there (K's place) to tensor memory.
+  {
+    constexpr unsigned PARTS = CH_WORK / CH_BM, PER = (HD / 8 + PARTS - 1) / PARTS;
+    const unsigned r = tid % CH_BM, part = tid / CH_BM, t = (row0 + r) / G, head = kvh * G + (row0 + r) % G;
+    float v[PER][8];
     float m = 0.0f;
+    if (tid < CH_WORK) {
+      const float* src = q + ((size_t)t * n_q + head) * HD;
 #pragma unroll
-    for (int j = 0; j < HD / 32; j++) {
-      v[j] = t < n_tok ? q[((size_t)t * n_q + head) * HD + lane * (HD / 32) + j] : 0.0f;
-      m = fmaxf(m, fabsf(v[j]));
+      for (unsigned k = 0; k < PER; k++) {
+        const unsigned c = part + k * PARTS;
+        const bool in = c < HD / 8u && t < n_tok;
+        const float4 a = in ? *reinterpret_cast<const float4*>(src + 8u * c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 b = in ? *reinterpret_cast<const float4*>(src + 8u * c + 4u) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[k][0] = a.x; v[k][1] = a.y; v[k][2] = a.z; v[k][3] = a.w;
+        v[k][4] = b.x; v[k][5] = b.y; v[k][6] = b.z; v[k][7] = b.w;
+        m = fmaxf(m, absmax8(v[k]));
+      }
+      atomicMax(row_max + r, __float_as_uint(m));
     }
+    __syncthreads();
+    if (tid < CH_WORK) {
+      float up;
+      const float down = row_scale_down(__uint_as_float(row_max[r]), &up);
+      if (part == 0) {
+        row_scale[r] = up * scale;
+        row_first[r] = t < n_tok ? (int)meta[t * 4 + 1] : 0;
+        row_end[r] = t < n_tok ? (int)meta[t * 4 + 1] + (int)meta[t * 4 + 0] : 0;
+      }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    float up;
-    const float down = row_scale_down(m, &up);
-    uint32_t hi[HD / 64], lo[HD / 64];
+      for (unsigned k = 0; k < PER; k++) {
+        const unsigned c = part + k * PARTS;
+        if (c < HD / 8u) {
 #pragma unroll
-    for (int j = 0; j < HD / 64; j++) {
-      const float a = v[2 * j] * down, b = v[2 * j + 1] * down;
-      const __half2 hh = __floats2half2_rn(a, b);
-      const float2 hf = __half22float2(hh);
-      hi[j] = pack_h2(hh);
-      lo[j] = pack_h2(__floats2half2_rn(a - hf.x, b - hf.y));
+          for (int e = 0; e < 8; e++) v[k][e] *= down;
+          uint4 hi, lo;
+          split8(v[k], hi, lo);
+          *reinterpret_cast<uint4*>(smem + S::kh + (c * CH_BM + r) * 16u) = hi;
+          *reinterpret_cast<uint4*>(smem + S::ql + (c * CH_BM + r) * 16u) = lo;
+        }
+      }
     }
-    uint32_t* dh = reinterpret_cast<uint32_t*>(smem + S::qh + (size_t)r * LD * 2) + lane * (HD / 64);
-    uint32_t* dl = reinterpret_cast<uint32_t*>(smem + S::ql + (size_t)r * LD * 2) + lane * (HD / 64);
-#pragma unroll
-    for (int j = 0; j < HD / 64; j++) {
-      dh[j] = hi[j];
-      dl[j] = lo[j];
-    }
-    if (lane == 0) {
-      row_scale[r] = up * scale;
-      row_first[r] = t < n_tok ? (int)meta[t * 4 + 1] : 0;
-      row_end[r] = t < n_tok ? (int)meta[t * 4 + 1] + (int)meta[t * 4 + 0] : 0;
-    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  __syncthreads();
+  const uint32_t tmem = *tslot;
+  if (tmem != 0u && tid == 0) *fail = 1;  // all 512 columns were asked for: they start at 0
+  const uint32_t tlane = (warp & 3u) << 21;   // 32 rows per warp, in the address bits of the lane
+  if (warp < CH_ROW_WARPS) {
+#pragma unroll
+    for (unsigned c = 0; c < HD / 8u; c += 2u) {
+      const uint4 a = *reinterpret_cast<const uint4*>(smem + S::kh + (c * CH_BM + tid) * 16u), b = *reinterpret_cast<const uint4*>(smem + S::kh + ((c + 1u) * CH_BM + tid) * 16u);
+      const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+      tc_st8(tlane + S::t_q + c * 4u, w);
+    }
+    tc_wait_st();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
 
-  float o[NT][4];
+  if (warp < CH_ROW_WARPS) {
+    // ---- a row of scores per thread
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 120;");
+    const float sc = row_scale[tid];
+    const int first = row_first[tid], end = row_end[tid];
+    float ref = kNegInit, l = 0.0f;
+    bool ok = true;
+    for (unsigned i = 0; i < n_tiles; i++) {
+      if (!__all_sync(0xffffffffu, mb_wait(bar(CB_S_FULL), i & 1u, CH_WAIT))) { ok = false; break; }
+      tc_fence_after();
+      uint32_t s[4][16];
 #pragma unroll
-  for (int i = 0; i < NT; i++)
+      for (int k = 0; k < 4; k++) tc_ld16(tlane + S::t_s + 16u * k, s[k]);
 #pragma unroll
-    for (int e = 0; e < 4; e++) o[i][e] = 0.0f;
-  float m0 = kNegInit, m1 = kNegInit, l0 = 0.0f, l1 = 0.0f;  // rows 16 rg + g and + 8; l over this warp's half of the positions
-  const unsigned gr = lane >> 2, tc = lane & 3u, ra = 16u * rg + gr, rb = ra + 8u;
-
-  for (int t0 = t_begin; t0 < t_end; t0 += CH_BN) {
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();  // the raw rows are there; the previous tile's operands are used up
-    {
-      const unsigned p = tid & (CH_BN - 1u);
-      for (unsigned pr = tid >> 6; pr < NB / 2; pr += CH_THREADS / CH_BN) {
-        Pair40 d;
-        const uint32_t* wk = reinterpret_cast<const uint32_t*>(smem + S::raw + (size_t)p * RP) + 9u * pr;
-        uint32_t w[9];
+      for (int k = 0; k < 4; k++) tc_wait_ld16(s[k]);
+      const int p0 = t_begin + (int)i * CH_BN, a = first - p0, b = min(end, t_end) - p0;  // columns [a, b) are seen
+      float mx = -INFINITY;
 #pragma unroll
-        for (int i = 0; i < 9; i++) w[i] = wk[i];
-        decode_pair(w, d);
-        uint4* kd = reinterpret_cast<uint4*>(smem + S::k + (size_t)p * LD * 2 + pr * 128u);
+      for (int j = 0; j < CH_BN; j++) {
+        const float x = j >= a && j < b ? __uint_as_float(s[j / 16][j % 16]) * sc : -INFINITY;
+        s[j / 16][j % 16] = __float_as_uint(x);
+        mx = fmaxf(mx, x);
+      }
+      mx = fmaxf(mx, ref);
+      const float alpha = __expf(ref - mx);
+      ref = mx;
+      row_alpha[(i & 1u) * CH_BM + tid] = alpha;
+      if (i > 0) {  // P is free
+        if (!__all_sync(0xffffffffu, mb_wait(bar(CB_V_FREE), (i - 1u) & 1u, CH_WAIT))) { ok = false; break; }
+        tc_fence_after();
+      }
+      float sum = 0.0f;
 #pragma unroll
-        for (int b = 0; b < 2; b++) {
-          dk[(2u * pr + b) * CH_BN + p] = __half2float(d.d[b]);
+      for (int k = 0; k < 4; k++) {
+        uint32_t ph[8], pl[8];
 #pragma unroll
-          for (int i = 0; i < 4; i++)
-            kd[4 * b + i] = make_uint4(pack_h2(d.v[b][4 * i]), pack_h2(d.v[b][4 * i + 1]), pack_h2(d.v[b][4 * i + 2]), pack_h2(d.v[b][4 * i + 3]));
+        for (int j = 0; j < 8; j++) {  // a masked score is -infinity: its probability is 0 whatever the maximum
+          const float x = __expf(__uint_as_float(s[k][2 * j]) - ref), y = __expf(__uint_as_float(s[k][2 * j + 1]) - ref);
+          sum += x + y;
+          const __half2 h = __floats2half2_rn(x * CH_P, y * CH_P);
+          const float2 f = __half22float2(h);
+          ph[j] = pack_h2(h);
+          pl[j] = pack_h2(__floats2half2_rn(x * CH_P - f.x, y * CH_P - f.y));
         }
-        const uint32_t* wv = reinterpret_cast<const uint32_t*>(smem + S::raw + (size_t)(CH_BN + p) * RP) + 9u * pr;
-#pragma unroll
-        for (int i = 0; i < 9; i++) w[i] = wv[i];
-        decode_pair(w, d);
-        uint4* hd4 = reinterpret_cast<uint4*>(smem + S::vh + (size_t)p * LD * 2 + pr * 128u);
-        uint4* ld4 = reinterpret_cast<uint4*>(smem + S::vl + (size_t)p * LD * 2 + pr * 128u);
-#pragma unroll
-        for (int b = 0; b < 2; b++) {
-          const __half2 dd = __half2half2(d.d[b]);
-#pragma unroll
-          for (int i = 0; i < 4; i++) {
-            uint32_t hh[4], ll[4];
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-              const __half2 x = __hmul2(d.v[b][4 * i + e], dd);
-              hh[e] = pack_h2(x);
-              ll[e] = pack_h2(__hfma2(d.v[b][4 * i + e], dd, __hneg2(x)));
-            }
-            hd4[4 * b + i] = make_uint4(hh[0], hh[1], hh[2], hh[3]);
-            ld4[4 * b + i] = make_uint4(ll[0], ll[1], ll[2], ll[3]);
-          }
-        }
+        tc_st8(tlane + S::t_ph + 8u * k, ph);
+        tc_st8(tlane + S::t_pl + 8u * k, pl);
       }
+      l = l * alpha + sum;
+      tc_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mb_arrive1(bar(CB_P_FULL));
     }
-    __syncthreads();
-    if (t0 + CH_BN < t_end) fetch(t0 + CH_BN);  // flies while this tile is multiplied
-
-    // ---- scores of rows 16 rg .. +16 and positions 32 h .. +32 of the tile
-    float s[4][4];
+    if (!ok && lane == 0) *fail = 1;
+    row_scale[tid] = ref;
+    reinterpret_cast<float*>(row_max)[tid] = l;
+  } else if (decoder) {
+    // ---- packed rows -> two f16 terms of K (positions x dims) and of V transposed (dims x positions); a tile's values are added to
+    // half a row per thread
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 184;");
+    constexpr unsigned HALF = HD / 2;
+    const unsigned orow = (warp & 3u) * 32u + lane, ocol = (warp >> 2 & 1u) * HALF;  // (warps 4..7 and 8..11)
+    float acc[HALF];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (unsigned c = 0; c < HALF; c++) acc[c] = 0.0f;
+    auto fold = [&](unsigned i) {
+      tc_fence_after();
+      const float alpha = row_alpha[(i & 1u) * CH_BM + orow];
 #pragma unroll
-      for (int e = 0; e < 4; e++) s[i][e] = 0.0f;
-    const uint32_t qa = sb + ((16u * rg + (lane & 15u)) * LD + (lane >> 4) * 8u) * 2u;
-    const uint32_t ka = sb + S::k + ((32u * h + (lane & 7u)) * LD + (lane >> 3) * 8u) * 2u;
-#pragma unroll 2
-    for (unsigned b = 0; b < NB; b++) {
-      uint32_t ah0[4], ah1[4], al0[4], al1[4], kb[4][4];
-      ldsm4(qa + S::qh + b * 64u, ah0);
-      ldsm4(qa + S::qh + b * 64u + 32u, ah1);
-      ldsm4(qa + S::ql + b * 64u, al0);
-      ldsm4(qa + S::ql + b * 64u + 32u, al1);
+      for (unsigned c = 0; c < HALF; c += 16u) {
+        uint32_t o[16];
+        tc_ld16(tlane + S::t_o + ocol + c, o);
+        tc_wait_ld16(o);
 #pragma unroll
-      for (int i = 0; i < 4; i++) ldsm4(ka + (unsigned)i * 8u * LD * 2u + b * 64u, kb[i]);
-      float c[4][4];
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int e = 0; e < 4; e++) c[i][e] = 0.0f;
-#pragma unroll
-      for (int i = 0; i < 4; i++) mma16816(c[i], ah0, kb[i][0], kb[i][1]);
-#pragma unroll
-      for (int i = 0; i < 4; i++) mma16816(c[i], ah1, kb[i][2], kb[i][3]);
-#pragma unroll
-      for (int i = 0; i < 4; i++) mma16816(c[i], al0, kb[i][0], kb[i][1]);
-#pragma unroll
-      for (int i = 0; i < 4; i++) mma16816(c[i], al1, kb[i][2], kb[i][3]);
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const float2 d = *reinterpret_cast<const float2*>(dk + b * CH_BN + 32u * h + 8u * i + 2u * tc);
-        s[i][0] = fmaf(c[i][0], d.x, s[i][0]);
-        s[i][1] = fmaf(c[i][1], d.y, s[i][1]);
-        s[i][2] = fmaf(c[i][2], d.x, s[i][2]);
-        s[i][3] = fmaf(c[i][3], d.y, s[i][3]);
+        for (unsigned e = 0; e < 16u; e++) acc[c + e] = fmaf(acc[c + e], alpha, __uint_as_float(o[e]));
       }
-    }
-    const float sa = row_scale[ra], sbk = row_scale[rb];
-    const int fa = row_first[ra], ea = row_end[ra], fb = row_first[rb], eb = row_end[rb];
-    float xa = kNegInit, xb = kNegInit;
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-      for (int e = 0; e < 2; e++) {
-        const int pos = t0 + (int)(32u * h + 8u * i + 2u * tc) + e;
-        s[i][e] = pos >= fa && pos < ea ? s[i][e] * sa : -INFINITY;
-        s[i][2 + e] = pos >= fb && pos < eb ? s[i][2 + e] * sbk : -INFINITY;
-        xa = fmaxf(xa, s[i][e]);
-        xb = fmaxf(xb, s[i][2 + e]);
-      }
-#pragma unroll
-    for (int off = 1; off <= 2; off <<= 1) {
-      xa = fmaxf(xa, __shfl_xor_sync(0xffffffffu, xa, off));
-      xb = fmaxf(xb, __shfl_xor_sync(0xffffffffu, xb, off));
-    }
-    if (tc == 0) {
-      red[h * CH_BM + ra] = xa;
-      red[h * CH_BM + rb] = xb;
-    }
-    __syncthreads();
-    const float na = fmaxf(m0, fmaxf(red[ra], red[CH_BM + ra])), nb = fmaxf(m1, fmaxf(red[rb], red[CH_BM + rb]));
-    const float alpha_a = __expf(m0 - na), alpha_b = __expf(m1 - nb);
-    m0 = na;
-    m1 = nb;
-    float suma = 0.0f, sumb = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      // a masked score is -infinity: its probability is 0 whatever the maximum
-      const float p0 = __expf(s[i][0] - na), p1 = __expf(s[i][1] - na), p2 = __expf(s[i][2] - nb), p3 = __expf(s[i][3] - nb);
-      suma += p0 + p1;
-      sumb += p2 + p3;
-      // 2^8 keeps the low terms of small probabilities out of the denormals; taken off with the sum
-      const __half2 ha = __floats2half2_rn(p0 * 256.0f, p1 * 256.0f), hb = __floats2half2_rn(p2 * 256.0f, p3 * 256.0f);
-      const float2 fa2 = __half22float2(ha), fb2 = __half22float2(hb);
-      const unsigned col = 32u * h + 8u * i + 2u * tc;
-      *reinterpret_cast<uint32_t*>(smem + S::ph + (ra * LP + col) * 2u) = pack_h2(ha);
-      *reinterpret_cast<uint32_t*>(smem + S::ph + (rb * LP + col) * 2u) = pack_h2(hb);
-      *reinterpret_cast<uint32_t*>(smem + S::pl + (ra * LP + col) * 2u) = pack_h2(__floats2half2_rn(p0 * 256.0f - fa2.x, p1 * 256.0f - fa2.y));
-      *reinterpret_cast<uint32_t*>(smem + S::pl + (rb * LP + col) * 2u) = pack_h2(__floats2half2_rn(p2 * 256.0f - fb2.x, p3 * 256.0f - fb2.y));
-    }
-    l0 = l0 * alpha_a + suma;
-    l1 = l1 * alpha_b + sumb;
-#pragma unroll
-    for (int i = 0; i < NT; i++) {
-      o[i][0] *= alpha_a;
-      o[i][1] *= alpha_a;
-      o[i][2] *= alpha_b;
-      o[i][3] *= alpha_b;
-    }
-    __syncthreads();
-    // ---- values: all 64 positions, dims of half h
-    const uint32_t pa = sb + ((16u * rg + (lane & 15u)) * LP + (lane >> 4) * 8u) * 2u;
-    const uint32_t va = sb + (((lane & 15u)) * LD + h * (HD / 2) + (lane >> 4) * 8u) * 2u;
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mb_arrive1(bar(CB_O_FREE));
+    };
+    bool ok = true;
+    for (unsigned i = 0; i < n_tiles; i++) {
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      if (i > 0) ok = mb_wait(bar(CB_K_FREE), (i - 1u) & 1u, CH_WAIT);
+      if (!dec_all(ok)) { ok = false; break; }  // the raw rows are there, K is free
 #pragma unroll 1
-    for (unsigned ks = 0; ks < CH_BN / 16; ks++) {
-      uint32_t ph[4], pl[4];
-      ldsm4(pa + S::ph + ks * 32u, ph);
-      ldsm4(pa + S::pl + ks * 32u, pl);
+      for (unsigned job = dt; job < CH_BN * NB; job += CH_DEC_WARPS * 32) {  // a block of a row
+        const unsigned p = job % CH_BN, b = job / CH_BN;
+        const unsigned char* src = smem + S::raw + p * RP + b * KS_Q40_BLOCK_BYTES;
+        const __half2 d = __half2half2(__ushort_as_half(*reinterpret_cast<const unsigned short*>(src)));
+        uint32_t w[4];
 #pragma unroll
-      for (int i = 0; i < NT; i += 2) {
-        uint32_t vh[4], vl[4];
-        ldsm4t(va + S::vh + (ks * 16u * LD + 8u * i) * 2u, vh);
-        ldsm4t(va + S::vl + (ks * 16u * LD + 8u * i) * 2u, vl);
-        mma16816(o[i], ph, vh[0], vh[1]);
-        mma16816(o[i + 1], ph, vh[2], vh[3]);
-        mma16816(o[i], pl, vh[0], vh[1]);
-        mma16816(o[i + 1], pl, vh[2], vh[3]);
-        mma16816(o[i], ph, vl[0], vl[1]);
-        mma16816(o[i + 1], ph, vl[2], vl[3]);
+        for (int k = 0; k < 4; k++)
+          w[k] = *reinterpret_cast<const unsigned short*>(src + 2 + 4 * k) | (uint32_t)*reinterpret_cast<const unsigned short*>(src + 4 + 4 * k) << 16;
+#pragma unroll 1
+        for (int half = 0; half < 2; half++)  // dims 0..15 of the block are the low nibbles
+#pragma unroll
+          for (int c = 0; c < 2; c++) {
+            uint32_t hi[4], lo[4];
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+              const uint32_t x = half ? w[2 * c + k] >> 4 : w[2 * c + k];
+              split_d(nib_h2(__byte_perm(x, 0u, 0x4140)), d, hi[2 * k], lo[2 * k]);
+              split_d(nib_h2(__byte_perm(x, 0u, 0x4342)), d, hi[2 * k + 1], lo[2 * k + 1]);
+            }
+            const unsigned at = ((4u * b + 2u * half + c) * CH_BN + p) * 16u;
+            *reinterpret_cast<uint4*>(smem + S::kh + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            *reinterpret_cast<uint4*>(smem + S::kl + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          }
       }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mb_arrive1(bar(CB_K_FULL));
+      if (i > 0) ok = mb_wait(bar(CB_V_FREE), (i - 1u) & 1u, CH_WAIT);
+      if (!dec_all(ok)) { ok = false; break; }
+      if (i > 0) fold(i - 1u);
+#pragma unroll 1
+      for (unsigned job = dt; job < 16u * NB * (CH_BN / 8); job += CH_DEC_WARPS * 32) {  // byte j of a block in eight neighbouring rows
+        const unsigned j = job % 16u, b = job / 16u % NB, pg = job / (16u * NB);
+        const unsigned char* src = smem + S::raw + (CH_BN + 8u * pg) * RP + b * KS_Q40_BLOCK_BYTES;
+        uint32_t hl[4], ll[4], hh[4], lh[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const unsigned char *x = src + 2 * k * RP, *y = x + RP;
+          const uint32_t n = x[2 + j] | (uint32_t)y[2 + j] << 16;
+          const __half2 d = as_h2(*reinterpret_cast<const unsigned short*>(x) | (uint32_t)*reinterpret_cast<const unsigned short*>(y) << 16);
+          split_d(nib_h2(n), d, hl[k], ll[k]);
+          split_d(nib_h2(n >> 4), d, hh[k], lh[k]);
+        }
+        const unsigned at = (pg * HD + 32u * b + j) * 16u;
+        *reinterpret_cast<uint4*>(smem + S::vh + at) = make_uint4(hl[0], hl[1], hl[2], hl[3]);
+        *reinterpret_cast<uint4*>(smem + S::vl + at) = make_uint4(ll[0], ll[1], ll[2], ll[3]);
+        *reinterpret_cast<uint4*>(smem + S::vh + at + 256u) = make_uint4(hh[0], hh[1], hh[2], hh[3]);
+        *reinterpret_cast<uint4*>(smem + S::vl + at + 256u) = make_uint4(lh[0], lh[1], lh[2], lh[3]);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mb_arrive1(bar(CB_V_FULL));
+      if (!dec_all(true)) break;  // (meets only: the raw rows are used up)
+      if (i + 1u < n_tiles) fetch(t_begin + (int)(i + 1u) * CH_BN);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    ok = ok && __all_sync(0xffffffffu, mb_wait(bar(CB_V_FREE), (n_tiles - 1u) & 1u, CH_WAIT));
+    if (!ok && lane == 0) *fail = 1;
+    if (ok) {  // the rows through shared memory, so that they leave in whole lines; every product that read it is done
+      fold(n_tiles - 1u);
+      float* out = reinterpret_cast<float*>(smem + S::o) + orow * S::OP + ocol;
+#pragma unroll
+      for (unsigned c = 0; c < HALF; c += 4u)
+        *reinterpret_cast<float4*>(out + c) = make_float4(acc[c] * (1.0f / CH_P), acc[c + 1] * (1.0f / CH_P), acc[c + 2] * (1.0f / CH_P), acc[c + 3] * (1.0f / CH_P));
+    }
+  } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+    if (warp == CH_ROW_WARPS + CH_DEC_WARPS) {
+    // ---- products: the whole warp runs the loop, one elected lane issues; the trip count out of a warp reduction, so that it and
+    // the descriptors stay in uniform registers
+    const unsigned leader = elect_one(), tiles = __reduce_max_sync(0xffffffffu, n_tiles);
+    constexpr uint32_t idesc_s = (1u << 4) | ((CH_BN >> 3) << 17) | ((CH_BM >> 4) << 24), idesc_o = (1u << 4) | ((HD >> 3) << 17) | ((CH_BM >> 4) << 24);
+    const uint64_t d_ql = tc_desc(sb + S::ql, CH_BM * 16u, 128u), d_kh = tc_desc(sb + S::kh, CH_BN * 16u, 128u), d_kl = tc_desc(sb + S::kl, CH_BN * 16u, 128u),
+                   d_vh = tc_desc(sb + S::vh, HD * 16u, 128u), d_vl = tc_desc(sb + S::vl, HD * 16u, 128u);
+    bool ok = false;
+    // Within a tile the small terms come first: the accumulator drops bits below its largest term at every step.
+    for (unsigned i = 0; i < tiles; i++) {
+      if (!__all_sync(0xffffffffu, mb_wait(bar(CB_K_FULL), i & 1u, CH_WAIT))) goto out;
+      tc_fence_after();
+      if (leader) {
+#pragma unroll
+        for (unsigned ks = 0; ks < HD / 16u; ks++) {  // (address fields count 16 bytes; two chunks a step)
+          tc_mma_f16_ta(S::t_s, S::t_q + 8u * ks, d_kl + (uint64_t)(2u * ks * CH_BN), idesc_s, ks ? 1u : 0u);
+          tc_mma_f16(S::t_s, d_ql + (uint64_t)(2u * ks * CH_BM), d_kh + (uint64_t)(2u * ks * CH_BN), idesc_s, 1u);
+        }
+#pragma unroll
+        for (unsigned ks = 0; ks < HD / 16u; ks++) tc_mma_f16_ta(S::t_s, S::t_q + 8u * ks, d_kh + (uint64_t)(2u * ks * CH_BN), idesc_s, 1u);
+        tc_commit(bar(CB_S_FULL));
+        tc_commit(bar(CB_K_FREE));
+      }
+      __syncwarp();
+      {
+        const bool got = mb_wait(bar(CB_V_FULL), i & 1u, CH_WAIT) && (i == 0u || mb_wait(bar(CB_O_FREE), (i - 1u) & 1u, CH_WAIT)) &&
+                         mb_wait(bar(CB_P_FULL), i & 1u, CH_WAIT);
+        if (!__all_sync(0xffffffffu, got)) goto out;
+      }
+      tc_fence_after();
+      if (leader) {
+#pragma unroll
+        for (unsigned ks = 0; ks < CH_BN / 16u; ks++) {
+          tc_mma_f16_ta(S::t_o, S::t_pl + 8u * ks, d_vh + (uint64_t)(2u * ks * HD), idesc_o, ks ? 1u : 0u);
+          tc_mma_f16_ta(S::t_o, S::t_ph + 8u * ks, d_vl + (uint64_t)(2u * ks * HD), idesc_o, 1u);
+        }
+#pragma unroll
+        for (unsigned ks = 0; ks < CH_BN / 16u; ks++) tc_mma_f16_ta(S::t_o, S::t_ph + 8u * ks, d_vh + (uint64_t)(2u * ks * HD), idesc_o, 1u);
+        tc_commit(bar(CB_V_FREE));
+      }
+      __syncwarp();
+    }
+    ok = true;
+  out:
+    if (leader) {  // every product issued must finish before shared and tensor memory go away (bounded)
+      if (!ok) *fail = 1;
+      tc_commit(bar(CB_DONE));
+    }
+    __syncwarp();
+    mb_wait(bar(CB_DONE), 0u, CH_WAIT);
     }
   }
-  // ---- records: l of the two halves together, O of this warp's dims
-#pragma unroll
-  for (int off = 1; off <= 2; off <<= 1) {
-    l0 += __shfl_xor_sync(0xffffffffu, l0, off);
-    l1 += __shfl_xor_sync(0xffffffffu, l1, off);
-  }
+  tc_fence_before();
   __syncthreads();
-  if (tc == 0) {
-    red[(2u + h) * CH_BM + ra] = l0;
-    red[(2u + h) * CH_BM + rb] = l1;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int half = 0; half < 2; half++) {
-    const unsigned r = half ? rb : ra, t = (row0 + r) / G, head = kvh * G + (row0 + r) % G;
-    if (t >= n_tok) continue;
-    float* rec = tmp + (((size_t)t * n_q + head) * n_splits + split) * (HD + 2);
-    if (h == 0 && tc == 0) {
-      rec[0] = half ? m1 : m0;
-      rec[1] = red[2u * CH_BM + r] + red[3u * CH_BM + r];
+  tc_fence_after();
+  if (*fail) {
+    if (tid == 0) atomicOr(err, 8u);
+  } else {
+    for (unsigned r = warp; r < CH_BM; r += CH_THREADS / 32) {
+      const unsigned t = (row0 + r) / G, head = kvh * G + (row0 + r) % G;
+      if (t >= n_tok) continue;
+      float* rec = tmp + (((size_t)t * n_q + head) * n_splits + split) * (HD + 2);
+      const float2* o = reinterpret_cast<const float2*>(smem + S::o) + r * (S::OP / 2);
+      for (unsigned d = lane; d < HD / 2u; d += 32u) *reinterpret_cast<float2*>(rec + 2 + 2u * d) = o[d];
+      if (lane == 0) *reinterpret_cast<float2*>(rec) = make_float2(row_scale[r], reinterpret_cast<float*>(row_max)[r]);
     }
-#pragma unroll
-    for (int i = 0; i < NT; i++)
-      *reinterpret_cast<float2*>(rec + 2 + h * (HD / 2) + 8 * i + 2 * tc) =
-          make_float2(o[i][2 * half] * (1.0f / 256.0f), o[i][2 * half + 1] * (1.0f / 256.0f));
   }
+  __syncthreads();
+  if (warp == CH_ROW_WARPS + CH_DEC_WARPS) tc_dealloc(tmem, 512);
 }
 
 // The (m, l, O) records of a token's heads -> the image the output projection reads its rows from (lower.rs:5897-6088 and
@@ -441,16 +516,19 @@ int launch_chunk(ks_ctx* ctx, dim3 grid, unsigned n_tok, unsigned n_q, unsigned 
     if (e != cudaSuccess) return ks_fail(ctx, KS_ERR_CUDA, "sdpa_chunk: cannot set %zu B shared memory: %s", smem, cudaGetErrorString(e));
     set[ctx->device & 15] = true;
   }
-  KS_LAUNCH(ctx, sdpa_chunk_kernel<HD>, grid, CH_THREADS, smem, n_tok, n_q, n_kv, scale, q, K, V, meta, tmp, n_splits);
+  KS_LAUNCH(ctx, sdpa_chunk_kernel<HD>, grid, CH_THREADS, smem, n_tok, n_q, n_kv, scale, q, K, V, meta, tmp, n_splits,
+            (unsigned*)ctx->ws + KS_WS_ERR_WORD);
   return ks_after_launch(ctx, "sdpa_chunk");
 }
 }  // namespace
 
-// Context splits of a chunk: enough blocks for every SM, at least two tiles each.  `ctx_len` may exceed what the rows see.
+// Context splits of a chunk: enough blocks for every SM, at least two tiles each.  A nearly empty second wave costs more than fewer
+// splits, except against one: the later rows see most of the context, and half a chip waits for them (2047 rows of 8 heads, 128
+// blocks: 162 us, twice as many halves 109).  `ctx_len` may exceed what the rows see.
 int ks_sdpa_chunk_splits(const ks_ctx* ctx, int n_tok, size_t n_q, size_t n_kv, size_t ctx_len, int most) {
   const size_t blocks = ((size_t)n_tok * (n_q / n_kv) + CH_BM - 1) / CH_BM * n_kv;
   size_t s = ((size_t)ctx->sm_count + blocks - 1) / blocks;
-  if (s > 1 && s * blocks > (size_t)ctx->sm_count + (size_t)ctx->sm_count / 8) s--;  // a nearly empty second wave costs more than fewer splits
+  if (s > 2 && s * blocks > (size_t)ctx->sm_count + (size_t)ctx->sm_count / 8) s--;
   const size_t by_len = (ctx_len + 2 * CH_BN - 1) / (2 * CH_BN);
   if (s > by_len) s = by_len;
   if (s > (size_t)most) s = most;

@@ -36,3 +36,31 @@ def test_long_chunks_equal_short_pieces(ctx, n_kv, window):
         scale, err = np.abs(want).max(), np.abs(got - want)
         assert err.max() <= 1e-3 * scale and np.sqrt((err ** 2).mean()) <= 1e-4 * scale, n
     model.close()
+
+
+@pytest.mark.parametrize("n_q,n_kv,hd", [(8, 1, 256), (8, 2, 256), (4, 4, 256), (16, 1, 128), (8, 4, 128)])
+def test_chunk_attention_equals_row_attention(monkeypatch, n_q, n_kv, hd):
+    """Prompt rows that share their context (tiles of 128 query rows x 64 positions) against a model whose prompts go row by row
+    through the decode attention: one tile and less, its edges, several tiles behind a context, windowed layers."""
+    from ksearch_b200 import CudaContext
+    out = []
+    for no_gemm in (False, True):
+        if no_gemm:
+            monkeypatch.setenv("KSEARCH_NO_GEMM", "1")
+        else:
+            monkeypatch.delenv("KSEARCH_NO_GEMM", raising=False)
+        cfg = ksm.tiny_config(max_seq=768, n_kv=n_kv)
+        cfg.n_q, cfg.hd, cfg.n_layers = n_q, hd, 2
+        cfg.sliding_window, cfg.swa_layers = 70, 0b10
+        c = CudaContext(0, flags=1)
+        model, _ = ksm.GemmaCudaModel.synthetic(c, cfg, seed=47, keep=True)
+        model.slot_alloc()
+        toks = [int(t) for t in synth.token_ids(47, "p", 700, cfg.vocab)]
+        for first, n in ((0, 63), (0, 64), (0, 129), (0, 333), (65, 128), (300, 257), (600, 90)):
+            out.append(_logits_after(model, c, ([toks[:first]] if first else []) + [toks[first:first + n]], toks[first + n]))
+        model.close()
+        c.close()
+    half = len(out) // 2
+    for got, want in zip(out[:half], out[half:]):
+        scale, err = np.abs(want).max(), np.abs(got - want)
+        assert err.max() <= 1e-3 * scale and np.sqrt((err ** 2).mean()) <= 1e-4 * scale
