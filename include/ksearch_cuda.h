@@ -318,12 +318,15 @@ int ks_model_slot_reset(ks_model* m, int slot);                              /* 
 int ks_model_slot_seq_len(const ks_model* m, int slot);                      /* KV:161 seq_len */
 int ks_model_slot_active(const ks_model* m);                                 /* KV:179 active_batch().len() */
 int ks_model_forward(ks_model* m, int first_slot, int n_slots, const int* tokens, int want_logits);   /* GP:881 forward_token, enqueue only */
-/* Prompt tokens of one slot without logits, up to 128 per pass over the weights (the rows of a chunk attend
+/* Prompt tokens of one slot without logits, up to 2048 per pass over the weights (the rows of a chunk attend
  * causally inside the chunk).  GemmaPrimModel::prefill_chunk (crates/ksearch_gemma/src/gemma_prim.rs:1305-1315):
  * chunks of more than 8 rows run every matrix through the tensor-core GEMM (the reference's mul_mm), shorter
  * ones through the batch GEMV (crates/ksearch_kernels/src/lib.rs:1414).  The slot advances by n_tokens;
  * enqueues only, apart from the wait for the pinned staging words between chunks. */
 int ks_model_prefill(ks_model* m, int slot, const int* tokens, int n_tokens);
+/* The same for several slots at once: counts[i] tokens for slots[i], behind one another in `tokens`; their rows share
+ * passes over the weights.  Arguments are checked before anything runs. */
+int ks_model_prefill_slots(ks_model* m, int n, const int* slots, const int* tokens, const int* counts);
 int ks_model_decode_token(ks_model* m, int first_slot, int n_slots, const int* tokens, int* next);    /* GP:1616 decode_token, blocking */
 /* One blocking step of slots first..first+n-1 whose tokens are sampled (GP:1622 decode_token_sampled + sample.rs:9-81 per slot):
  * ks_model_forward with logits, then ks_sample_softcap_min_p over each slot's row, with only the logits that can survive

@@ -554,7 +554,7 @@ struct EpiQkvArgs {
   unsigned n_tok, n_q, n_kv;
   float eps;
   const float *qw, *kw, *rope;
-  const int* pos;
+  const int *pos, *row_slot;
   float* q_out;
   uint8_t *kv_k, *kv_v;
   size_t slot_stride;
@@ -621,7 +621,7 @@ __global__ void __launch_bounds__(256) gemm_finish_qkv_kernel(const EpiQkvArgs e
       else *reinterpret_cast<float2*>(o + h * (HD / 2)) = make_float2(y[h][0], y[h][1]);
     return;
   }
-  uint8_t* dst = (seg == 1 ? e.kv_k : e.kv_v) + (size_t)tok * e.slot_stride + (p * e.n_kv + head) * ROWB;
+  uint8_t* dst = (seg == 1 ? e.kv_k : e.kv_v) + (size_t)(e.row_slot ? (unsigned)e.row_slot[tok] : tok) * e.slot_stride + (p * e.n_kv + head) * ROWB;
 #pragma unroll
   for (int h = 0; h < 2; h++) {
     float amax = 0.0f, val[V];
@@ -902,6 +902,7 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
     e.kw = epi->kw;
     e.rope = epi->rope;
     e.pos = epi->pos;
+    e.row_slot = epi->row_slot;
     e.q_out = epi->out_x;
     e.kv_k = epi->kv_k;
     e.kv_v = epi->kv_v;

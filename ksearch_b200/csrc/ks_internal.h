@@ -153,8 +153,13 @@ int ks_launch_sdpa(ks_ctx* ctx, size_t n_slots, size_t n_q, size_t n_kv, size_t 
 int ks_sdpa_chunk_splits(const ks_ctx* ctx, int n_tok, size_t n_q, size_t n_kv, size_t ctx_len, int most);
 bool ks_sdpa_merge_split_covers(size_t n_q, size_t hd);
 bool ks_sdpa_chunk_covers(size_t n_q, size_t n_kv, size_t hd, const void* K, const void* V);
+// Rows [row0[p], row0[p + 1]) of a pass belong to slot[p]; no slot twice.
+struct ks_row_parts {
+  unsigned n, row0[65], slot[64];
+};
+// parts == nullptr: all rows belong to the cache at K and V; else part p's cache is slot[p] * slot_stride bytes on.
 int ks_launch_sdpa_chunk(ks_ctx* ctx, int n_tok, size_t n_q, size_t n_kv, size_t hd, float scale, const float* q, const uint8_t* K,
-                         const uint8_t* V, const float* meta, float* tmp, int n_splits);
+                         const uint8_t* V, const float* meta, float* tmp, int n_splits, const ks_row_parts* parts = nullptr, size_t slot_stride = 0);
 // Token rows per block of an operand image and all of them padded to whole blocks: a choice of the GEMM that reads the image.
 struct ks_gemm_blocks {
   unsigned tbn, np;
@@ -212,9 +217,9 @@ struct ks_gemm_epi {
   void* xt_out;                        // the image written for the next GEMM (may be the image this GEMM read)
   ks_dtype next_dtype;                 // NORM_SPLIT: weights of that next GEMM
   ks_gemm_blocks next;                 // *_SPLIT: its blocks
-  unsigned n_q, n_kv, hd;              // QKV: heads; row t's cache entry: position pos[t] of the cache at t * slot_stride
+  unsigned n_q, n_kv, hd;              // QKV: heads; row t's cache entry: position pos[t] of the cache at (row_slot ? row_slot[t] : t) * slot_stride
   const float *qw, *kw, *rope;
-  const int* pos;
+  const int *pos, *row_slot;
   uint8_t *kv_k, *kv_v;
   size_t slot_stride;
 };

@@ -93,6 +93,24 @@ __global__ void end_chunk_kernel(int n, int* base) {
   if (threadIdx.x == 0) base[0] += n;
 }
 
+// Prompt rows of several slots: row t belongs to the part it lies in and sits behind what its slot holds.
+__global__ void begin_parts_kernel(const __grid_constant__ ks_row_parts parts, const int* pos, int* cpos, int* row_slot, float* meta, float* meta_swa, int window) {
+  ks_pdl_entry();
+  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= parts.row0[parts.n]) return;
+  unsigned p = 0;
+  while (t >= parts.row0[p + 1]) p++;
+  const int at = pos[parts.slot[p]] + (int)(t - parts.row0[p]);
+  cpos[t] = at;
+  row_slot[t] = (int)parts.slot[p];
+  write_meta_pair(meta, meta_swa, (int)t, at + 1, window);
+}
+__global__ void end_parts_kernel(const __grid_constant__ ks_row_parts parts, int* pos) {
+  ks_pdl_entry();
+  const unsigned p = threadIdx.x;
+  if (p < parts.n) pos[parts.slot[p]] += (int)(parts.row0[p + 1] - parts.row0[p]);
+}
+
 struct Tensor {
   void* dptr = nullptr;
   size_t bytes = 0;
@@ -168,7 +186,7 @@ struct ks_model {
   // prompt chunks (ks_model_prefill): KS_PREFILL_CHUNK rows of activations of their own
   void *cx = nullptr, *cxb = nullptr, *cx2 = nullptr, *cq = nullptr, *ck = nullptr, *cv = nullptr, *co = nullptr, *cff = nullptr;
   float* ctok = nullptr;
-  int* cpos = nullptr;
+  int *cpos = nullptr, *crow_slot = nullptr;
   float* cmeta = nullptr;
   float* cmeta_swa = nullptr;
   float* cattn_tmp = nullptr;
@@ -230,6 +248,7 @@ struct Lane {
   size_t kv_off;     // byte offset of row 0's cache inside every layer's K / V allocation
   size_t kv_stride;  // bytes between the caches of consecutive rows
   int* chunk_base;   // prompt chunk: the slot's position word (rows take base, base + 1, ...); else nullptr
+  const ks_row_parts* parts; // prompt rows of several slots (kv_stride is then between slots); else nullptr
   bool share_full, share_swa;  // prompt chunk: do its rows share one pass over their context in a full / sliding-window layer?
 };
 
@@ -288,14 +307,18 @@ int att_splits_for(const ks_model* m, int n) {
 unsigned row_threads(int n) { return (unsigned)((n + 1 + 31) / 32 * 32); }  // one thread per row and one more
 
 int lane_begin(ks_model* m, const Lane& L, int n) {
-  if (L.chunk_base)
+  if (L.parts)
+    KS_LAUNCH(m->ctx, (begin_parts_kernel), (unsigned)(n + 255) / 256u, 256, 0, *L.parts, (const int*)m->pos, L.pos, m->crow_slot, L.meta, L.meta_swa, (int)m->cfg.sliding_window);
+  else if (L.chunk_base)
     KS_LAUNCH(m->ctx, (begin_chunk_kernel), (unsigned)(n + 255) / 256u, 256, 0, n, (const int*)L.chunk_base, L.pos, L.meta, L.meta_swa, (int)m->cfg.sliding_window);
   else
     KS_LAUNCH(m->ctx, (begin_token_kernel), 1, row_threads(n), 0, n, (const int*)L.pos, L.meta, L.meta_swa, (int)m->cfg.sliding_window);
   return ks_after_launch(m->ctx, "begin_token");
 }
 int lane_end(ks_model* m, const Lane& L, int n) {
-  if (L.chunk_base)
+  if (L.parts)
+    KS_LAUNCH(m->ctx, (end_parts_kernel), 1, 64, 0, *L.parts, m->pos);
+  else if (L.chunk_base)
     KS_LAUNCH(m->ctx, (end_chunk_kernel), 1, 32, 0, n, L.chunk_base);
   else
     KS_LAUNCH(m->ctx, (end_token_kernel), 1, row_threads(n), 0, n, L.pos);
@@ -410,6 +433,7 @@ int enqueue_forward_gemm(ks_model* m, const Lane& L_, int n, bool want_logits) {
       head.kw = L.k32;
       head.rope = m->rope;
       head.pos = L_.pos;
+      head.row_slot = L_.parts ? m->crow_slot : nullptr;
       head.kv_k = kk;
       head.kv_v = kv;
       head.slot_stride = L_.kv_stride;
@@ -417,7 +441,7 @@ int enqueue_forward_gemm(ks_model* m, const Lane& L_, int n, bool want_logits) {
     }
     const bool share = layer_meta(m, L_, l) == L_.meta ? L_.share_full : L_.share_swa;
     if (share && ks_sdpa_chunk_covers(nq, nkv, hd, kk, kv)) {
-      if ((rc = ks_launch_sdpa_chunk(c, n, nq, nkv, hd, g.attn_scale, (const float*)q, kk, kv, layer_meta(m, L_, l), L_.attn_tmp, chunk_splits)) ||
+      if ((rc = ks_launch_sdpa_chunk(c, n, nq, nkv, hd, g.attn_scale, (const float*)q, kk, kv, layer_meta(m, L_, l), L_.attn_tmp, chunk_splits, L_.parts, L_.kv_stride)) ||
           (rc = ks_launch_sdpa_merge_split(c, n, b_o, nq, hd, L_.attn_tmp, chunk_splits, m->gemm_xt)))
         return rc;
     } else if (att_splits > 1 && ks_sdpa_merge_split_covers(nq, hd)) {
@@ -849,8 +873,8 @@ ks_model* ks_model_create(ks_ctx* ctx, const ks_model_config* cfg) {
     // widths its epilogues take: larger batches go through the tensor-core GEMM, which computes in f32 (a chunk of an f16 model
     // too: its rows meet f16 vectors nowhere); wider models keep the batch matvec for every batch
     if (ks_gemm_layers_cover(H, F, qn) && !getenv("KSEARCH_NO_GEMM")) {
-      // no prompt is longer than the cache; decode steps bring a row per slot
-      const int cap = (g.max_seq + 127) / 128 * 128, G = cap < KS_GEMM_CHUNK ? (cap > 256 ? cap : 256) : KS_GEMM_CHUNK;
+      // prompts are no longer than the caches; decode steps bring a row per slot
+      const int cap = (int)std::min<size_t>(((size_t)g.max_seq * S + 127) / 128 * 128, KS_GEMM_CHUNK), G = cap < KS_GEMM_CHUNK ? (cap > 256 ? cap : 256) : KS_GEMM_CHUNK;
       m->gemm_chunk = G;
       // one launch each: q|k|v, o, gate|up, down, head
       const size_t rows_of[5][3] = {{qn, kvn, kvn}, {H}, {F, F}, {H}, {(size_t)g.vocab}}, cols_of[5] = {H, qn, H, F, H};
@@ -890,6 +914,7 @@ ks_model* ks_model_create(ks_ctx* ctx, const ks_model_config* cfg) {
          dev_alloc(m, &m->ck, C * kvn * cb) == KS_OK && dev_alloc(m, &m->cv, C * kvn * cb) == KS_OK &&
          dev_alloc(m, &m->co, C * qn * cb) == KS_OK && dev_alloc(m, &m->cff, C * F * cb) == KS_OK &&
          dev_alloc(m, (void**)&m->ctok, C * sizeof(float)) == KS_OK && dev_alloc(m, (void**)&m->cpos, C * sizeof(int)) == KS_OK &&
+         dev_alloc(m, (void**)&m->crow_slot, C * sizeof(int)) == KS_OK &&
          dev_alloc(m, (void**)&m->cmeta, C * 4 * sizeof(float)) == KS_OK &&
          (!has_window(g) || dev_alloc(m, (void**)&m->cmeta_swa, C * 4 * sizeof(float)) == KS_OK);
   }
@@ -1275,6 +1300,77 @@ int ks_model_prefill(ks_model* m, int slot, const int* tokens, int n_tokens) {
     if ((rc = run_prefill_chunk(m, slot, n, prompt_gemm(m, n)))) return rc;
     m->seq_len[slot] += n;
     t0 += n;
+  }
+  return KS_OK;
+}
+
+// Prompt tokens of several slots (counts[i] of them for slots[i], behind one another in `tokens`): their rows share passes over the
+// weights, up to KS_GEMM_CHUNK a pass.  Everything is checked before anything runs.  A pass of one slot's rows is ks_model_prefill;
+// passes that mix slots are launched as they are (their shapes hardly repeat, and a capture costs more than the launches).
+int ks_model_prefill_slots(ks_model* m, int n, const int* slots, const int* tokens, const int* counts) {
+  if (!m) return KS_ERR_INVALID;
+  ks_ctx* c = m->ctx;
+  KS_REQUIRE(c, n >= 0 && n <= m->cfg.n_slots && (n == 0 || (slots && counts)), "prefill_slots: bad arguments");
+  int rc;
+  if ((rc = check_ready(m))) return rc;
+  size_t total = 0;
+  std::vector<char> seen(m->cfg.n_slots, 0);
+  for (int i = 0; i < n; i++) {
+    if ((rc = check_slots(m, slots[i], 1))) return rc;
+    KS_REQUIRE(c, !seen[slots[i]], "prefill_slots: slot %d twice", slots[i]);
+    seen[slots[i]] = 1;
+    KS_REQUIRE(c, counts[i] >= 0, "prefill_slots: negative token count");
+    if (m->seq_len[slots[i]] + counts[i] > m->cfg.max_seq) return ks_fail(c, KS_ERR_STATE, "max_seq exceeded");
+    total += (size_t)counts[i];
+  }
+  KS_REQUIRE(c, tokens || total == 0, "prefill_slots: null tokens");
+  for (size_t t = 0; t < total; t++)
+    KS_REQUIRE(c, tokens[t] >= 0 && tokens[t] < m->cfg.vocab, "token id %d outside the vocabulary", tokens[t]);
+  const ks_model_config& g = m->cfg;
+  bool mix = m->gemm_chunk > 0 && m->slot_stride % 4 == 0;
+  for (int l = 0; l < g.n_layers; l++) mix = mix && ks_sdpa_chunk_covers(g.n_q, g.n_kv, g.hd, m->kv_k[l], m->kv_v[l]);
+  float* stage = m->host_tok + m->host_tok_n - 16 - KS_STAGE_IDS;
+  const int* next = tokens;
+  int i = 0, used = 0;  // `used` tokens of part i have run
+  while (i < n) {
+    // the parts of this pass
+    ks_row_parts parts{};
+    int rows = 0;
+    while (i < n && (int)parts.n < (mix ? 64 : 1) && rows < (mix ? m->gemm_chunk : 1 << 30)) {
+      const int left = counts[i] - used, take = mix ? std::min(left, m->gemm_chunk - rows) : left;
+      if (take > 0) {
+        parts.slot[parts.n] = (unsigned)slots[i];
+        parts.row0[parts.n++] = (unsigned)rows;
+        rows += take;
+        parts.row0[parts.n] = (unsigned)rows;
+      }
+      if (take < left) {
+        used += take;
+        break;
+      }
+      i++;
+      used = 0;
+    }
+    if (parts.n == 0) break;
+    if (parts.n == 1 || !prompt_gemm(m, rows)) {
+      for (unsigned p = 0; p < parts.n; p++) {
+        const int len = (int)(parts.row0[p + 1] - parts.row0[p]);
+        if ((rc = ks_model_prefill(m, (int)parts.slot[p], next, len))) return rc;
+        next += len;
+      }
+      continue;
+    }
+    KS_CUDA(c, cudaStreamSynchronize(c->stream));  // the staging words may still be in flight
+    for (int t = 0; t < rows; t++) stage[t] = (float)next[t];
+    KS_CUDA(c, cudaMemcpyAsync(m->ctok, stage, rows * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+    Lane lane = chunk_lane(m, 0, true, true);
+    lane.chunk_base = nullptr;
+    lane.kv_off = 0;
+    lane.kv_stride = m->slot_stride;
+    lane.parts = &parts;
+    if ((rc = enqueue_forward_gemm(m, lane, rows, false))) return rc;
+    for (unsigned p = 0; p < parts.n; p++) m->seq_len[parts.slot[p]] += (int)(parts.row0[p + 1] - parts.row0[p]);
+    next += rows;
   }
   return KS_OK;
 }

@@ -1,4 +1,4 @@
-// Attention of a prompt chunk: many token rows of one slot against its Q4_0 cache, causal (and windowed) by row.
+// Attention of a prompt chunk: many token rows of one slot, or of several, against their Q4_0 caches, causal (and windowed) by row.
 //
 // The reference runs its decode attention once per prompt row (forward_prefill_chunk, crates/ksearch_gemma/src/
 // gemma_prim.rs:1463-1472, over crates/ksearch_codegen/src/lower.rs:4897-6088), so every row reads the whole context again.
@@ -71,17 +71,29 @@ __device__ __forceinline__ void split_d(__half2 n, __half2 d, uint32_t& hi, uint
 }
 __device__ __forceinline__ __half2 nib_h2(uint32_t w) { return __hsub2(as_h2((w & 0x000F000Fu) | 0x64006400u), __float2half2_rn(1032.0f)); }  // nibbles 0 of bytes 0 and 2
 
+struct ChunkParts {  // part p: rows from row0[p] on, row tiles from tile0[p] on
+  unsigned n, row0[65], tile0[65], slot[64];
+};
+
 template <int HD>
 __global__ void __launch_bounds__(CH_THREADS, 1)
-sdpa_chunk_kernel(unsigned n_tok, unsigned n_q, unsigned n_kv, float scale, const float* q, const uint8_t* K, const uint8_t* V, const float* meta,
-                  float* tmp, unsigned n_splits, unsigned* err) {
+sdpa_chunk_kernel(const __grid_constant__ ChunkParts parts, size_t slot_stride, unsigned n_q, unsigned n_kv, float scale, const float* q, const uint8_t* K,
+                  const uint8_t* V, const float* meta, float* tmp, unsigned n_splits, unsigned* err) {
   using S = ChunkSmem<HD>;
   constexpr unsigned NB = S::NB, RP = S::RP, ROWB = S::ROWB;
   extern __shared__ __align__(1024) unsigned char smem[];
   ks_pdl_entry();
   const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const unsigned G = n_q / n_kv, kvh = blockIdx.y, split = blockIdx.z;
-  const unsigned row0 = (gridDim.x - 1u - blockIdx.x) * CH_BM;  // the last rows see the most: they start first
+  const unsigned bx = gridDim.x - 1u - blockIdx.x;  // the last rows see the most: they start first
+  unsigned part_id = 0;
+  while (part_id + 1u < parts.n && bx >= parts.tile0[part_id + 1u]) part_id++;
+  const unsigned row0 = (bx - parts.tile0[part_id]) * CH_BM, first_tok = parts.row0[part_id], n_tok = parts.row0[part_id + 1u] - first_tok;
+  q += (size_t)first_tok * n_q * HD;  // from here on rows are counted inside the part
+  meta += (size_t)first_tok * 4u;
+  tmp += (size_t)first_tok * n_q * n_splits * (HD + 2);
+  K += parts.slot[part_id] * slot_stride;
+  V += parts.slot[part_id] * slot_stride;
   const uint32_t sb = sm32(smem);
   auto bar = [&](unsigned i) { return sb + 8u * i; };
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + S::slot);
@@ -507,7 +519,7 @@ __global__ void __launch_bounds__(512) sdpa_merge_split_kernel(unsigned n_tok, u
 }
 
 template <int HD>
-int launch_chunk(ks_ctx* ctx, dim3 grid, unsigned n_tok, unsigned n_q, unsigned n_kv, float scale, const float* q, const uint8_t* K, const uint8_t* V,
+int launch_chunk(ks_ctx* ctx, dim3 grid, const ChunkParts& parts, size_t slot_stride, unsigned n_q, unsigned n_kv, float scale, const float* q, const uint8_t* K, const uint8_t* V,
                  const float* meta, float* tmp, unsigned n_splits) {
   constexpr size_t smem = ChunkSmem<HD>::total;
   static bool set[16] = {false};
@@ -516,7 +528,7 @@ int launch_chunk(ks_ctx* ctx, dim3 grid, unsigned n_tok, unsigned n_q, unsigned 
     if (e != cudaSuccess) return ks_fail(ctx, KS_ERR_CUDA, "sdpa_chunk: cannot set %zu B shared memory: %s", smem, cudaGetErrorString(e));
     set[ctx->device & 15] = true;
   }
-  KS_LAUNCH(ctx, sdpa_chunk_kernel<HD>, grid, CH_THREADS, smem, n_tok, n_q, n_kv, scale, q, K, V, meta, tmp, n_splits,
+  KS_LAUNCH(ctx, sdpa_chunk_kernel<HD>, grid, CH_THREADS, smem, parts, slot_stride, n_q, n_kv, scale, q, K, V, meta, tmp, n_splits,
             (unsigned*)ctx->ws + KS_WS_ERR_WORD);
   return ks_after_launch(ctx, "sdpa_chunk");
 }
@@ -542,13 +554,24 @@ bool ks_sdpa_chunk_covers(size_t n_q, size_t n_kv, size_t hd, const void* K, con
   return (hd == 256 || hd == 128) && G <= 16 && CH_BM % G == 0 && ks_sdpa_merge_split_covers(n_q, hd) && (((uintptr_t)K | (uintptr_t)V) & 3u) == 0;
 }
 
-// Rows of one slot: q [n_tok, n_q hd] f32, meta [n_tok][4] = (tlen, start, -, -) with both ends growing along the rows
+// q [n_tok, n_q hd] f32, meta [n_tok][4] = (tlen, start, -, -) with both ends growing along the rows of a slot
 // -> records in tmp [n_tok][n_q][n_splits][hd + 2].
 int ks_launch_sdpa_chunk(ks_ctx* ctx, int n_tok, size_t n_q, size_t n_kv, size_t hd, float scale, const float* q, const uint8_t* K, const uint8_t* V,
-                         const float* meta, float* tmp, int n_splits) {
-  const dim3 grid((unsigned)(((size_t)n_tok * (n_q / n_kv) + CH_BM - 1) / CH_BM), (unsigned)n_kv, (unsigned)n_splits);
-  return hd == 256 ? launch_chunk<256>(ctx, grid, (unsigned)n_tok, (unsigned)n_q, (unsigned)n_kv, scale, q, K, V, meta, tmp, (unsigned)n_splits)
-                   : launch_chunk<128>(ctx, grid, (unsigned)n_tok, (unsigned)n_q, (unsigned)n_kv, scale, q, K, V, meta, tmp, (unsigned)n_splits);
+                         const float* meta, float* tmp, int n_splits, const ks_row_parts* parts, size_t slot_stride) {
+  ChunkParts cp{};
+  cp.n = parts ? parts->n : 1u;
+  unsigned tiles = 0;
+  for (unsigned p = 0; p < cp.n; p++) {
+    cp.row0[p] = parts ? parts->row0[p] : 0u;
+    cp.row0[p + 1] = parts ? parts->row0[p + 1] : (unsigned)n_tok;
+    cp.slot[p] = parts ? parts->slot[p] : 0u;
+    cp.tile0[p] = tiles;
+    tiles += (unsigned)(((cp.row0[p + 1] - cp.row0[p]) * (n_q / n_kv) + CH_BM - 1) / CH_BM);
+  }
+  cp.tile0[cp.n] = tiles;
+  const dim3 grid(tiles, (unsigned)n_kv, (unsigned)n_splits);
+  return hd == 256 ? launch_chunk<256>(ctx, grid, cp, slot_stride, (unsigned)n_q, (unsigned)n_kv, scale, q, K, V, meta, tmp, (unsigned)n_splits)
+                   : launch_chunk<128>(ctx, grid, cp, slot_stride, (unsigned)n_q, (unsigned)n_kv, scale, q, K, V, meta, tmp, (unsigned)n_splits);
 }
 
 // Records of n_tok rows -> the Q4_K form of the operand image (rows past n_tok as zeros).

@@ -190,6 +190,14 @@ class GemmaCudaModel:
         arr = (C.c_int * max(1, len(toks)))(*toks)
         self.ctx.check(self.lib.ks_model_prefill(self.h, slot, arr, len(toks)))
 
+    def prefill_many(self, parts):
+        """Prompt tokens of several slots, (slot, tokens) each: their rows share passes over the weights."""
+        toks = [[int(t) for t in p[1]] for p in parts]
+        flat = [t for p in toks for t in p]
+        n = len(toks)
+        self.ctx.check(self.lib.ks_model_prefill_slots(self.h, n, (C.c_int * max(1, n))(*[int(p[0]) for p in parts]),
+                                                       (C.c_int * max(1, len(flat)))(*flat), (C.c_int * max(1, n))(*[len(p) for p in toks])))
+
     def decode_token(self, tokens, first: int = 0):
         toks = [int(t) for t in np.atleast_1d(tokens)]
         n = len(toks)

@@ -186,6 +186,7 @@ class Scheduler:
         decoding = any(not a.finished and a.last_token is not None for a in self.active)
         budget = max(self.cfg.prefill_tokens_per_tick, self.cfg.prefill_chunk)
         idx = self._prefill_next % n
+        together = [] if hasattr(self.model, "prefill_many") else None
         for _ in range(n):
             if budget == 0:
                 break
@@ -199,14 +200,46 @@ class Scheduler:
                 continue
             cap = self.cfg.prefill_chunk if decoding else budget
             take = min(budget, cap, end - a.cursor)
-            try:
-                self.model.prefill(a.slot, a.req.prompt_ids[a.cursor:a.cursor + take])
-            except Exception as e:
-                a.req.emit("error", str(e))
-                self._finish(a, "error")
-                continue
-            budget -= take
-            a.cursor += take
-            if a.cursor >= end:
-                a.last_token = int(a.req.prompt_ids[-1])
+            if together is not None:
+                together.append((a, take))
+                budget -= take
+            elif self._prefill_one(a, take):
+                budget -= take
         self._prefill_next = idx
+        if together:
+            self._prefill_together(together)
+
+    def _prefill_one(self, a: _Active, take: int) -> bool:
+        try:
+            self.model.prefill(a.slot, a.req.prompt_ids[a.cursor:a.cursor + take])
+        except Exception as e:
+            a.req.emit("error", str(e))
+            self._finish(a, "error")
+            return False
+        self._advance(a, take)
+        return True
+
+    def _advance(self, a: _Active, take: int):
+        a.cursor += take
+        if a.cursor >= len(a.req.prompt_ids) - 1:
+            a.last_token = int(a.req.prompt_ids[-1])
+
+    def _prefill_together(self, parts):
+        """The round's prompt pieces in shared passes over the weights; one by one where that is refused, so that an
+        error meets the request it belongs to."""
+        if len(parts) > 1:
+            before = [self.model.seq_len(a.slot) for a, _ in parts]
+            try:
+                self.model.prefill_many([(a.slot, a.req.prompt_ids[a.cursor:a.cursor + take]) for a, take in parts])
+            except Exception as e:
+                if [self.model.seq_len(a.slot) for a, _ in parts] != before:
+                    for a, _ in parts:
+                        a.req.emit("error", str(e))
+                        self._finish(a, "error")
+                    return
+            else:
+                for a, take in parts:
+                    self._advance(a, take)
+                return
+        for a, take in parts:
+            self._prefill_one(a, take)

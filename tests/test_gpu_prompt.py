@@ -64,3 +64,42 @@ def test_chunk_attention_equals_row_attention(monkeypatch, n_q, n_kv, hd):
     for got, want in zip(out[:half], out[half:]):
         scale, err = np.abs(want).max(), np.abs(got - want)
         assert err.max() <= 1e-3 * scale and np.sqrt((err ** 2).mean()) <= 1e-4 * scale
+
+
+@pytest.mark.parametrize("n_kv,window", [(1, 0), (2, 60)])
+def test_prompts_of_several_slots_share_passes(ctx, n_kv, window):
+    """prefill_many against one prefill call per slot: ragged pieces in any slot order, pieces behind a context, an empty one, more
+    rows than a pass takes; what is refused leaves every slot where it was."""
+    from ksearch_b200 import KsError
+    cfg = ksm.tiny_config(max_seq=800, n_slots=4, n_kv=n_kv)
+    cfg.sliding_window, cfg.swa_layers = window, 0b101 if window else 0
+    model, _ = ksm.GemmaCudaModel.synthetic(ctx, cfg, seed=53, keep=True)
+    slots = [model.slot_alloc() for _ in range(4)]
+    toks = [[int(t) for t in synth.token_ids(53, f"s{s}", 801, cfg.vocab)] for s in slots]
+    for rounds in ([(5, 130, 1, 300)], [(64, 17, 128, 3), (1, 1, 0, 1), (90, 0, 257, 40)], [(700, 690, 710, 705)]):
+        logits = []
+        for together in (True, False):
+            at = [0] * 4
+            for s in slots:
+                model.slot_reset(s)
+            for counts in rounds:
+                parts = [(s, toks[s][at[s]:at[s] + counts[s]]) for s in (2, 0, 3, 1)]
+                if together:
+                    model.prefill_many(parts)
+                else:
+                    for s, p in parts:
+                        model.prefill(s, p)
+                at = [a + c for a, c in zip(at, counts)]
+            assert [model.seq_len(s) for s in slots] == at
+            model.forward(0, 4, [toks[s][at[s]] for s in slots], True)
+            ctx.synchronize()
+            logits.append([model.read_debug(1, s).astype(np.float64) for s in slots])
+        for got, want in zip(*logits):
+            scale, err = np.abs(want).max(), np.abs(got - want)
+            assert err.max() <= 1e-3 * scale and np.sqrt((err ** 2).mean()) <= 1e-4 * scale
+    before = [model.seq_len(s) for s in slots]
+    for bad in ([(0, [1]), (1, [cfg.vocab])], [(0, [1]), (0, [2])], [(0, [1]), (1, [1] * 800)]):
+        with pytest.raises(KsError):
+            model.prefill_many(bad)
+        assert [model.seq_len(s) for s in slots] == before
+    model.close()
