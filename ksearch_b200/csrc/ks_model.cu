@@ -218,19 +218,20 @@ constexpr int KS_PREFILL_CHUNK = 8;  // tokens per pass over the weights (the ma
 constexpr int KS_GEMM_CHUNK = KS_GEMM_ROWS;
 constexpr size_t KS_STAGE_IDS = KS_GEMM_CHUNK; // pinned words that stage host token ids
 
-// Do the rows of a prompt chunk share one pass over their context (ks_sdpa_chunk.cu: 64 rows x heads a block, few blocks), or does
-// each take the decode kernel (a block per row and up to four heads, spread over the chip)?  By the work of the second form:
-// rows x blocks x positions a row sees on average, in units of 256 dims.  Microseconds per layer, shared / per row:
-//   tiny (4 heads, 1 KV head of 128)   24 rows at 0: 50 / 44, 256 at 512 (82k): 97 / 86, 128 at 960 (65k): 94 / 93, 96 at 2048 (100k): 94 / 103
-//   E2B (8, 1 of 256)                  32 rows at 0: 70 / 63, 131 at 192 (67k): 115 / 108, 192 at 192 (110k): 124 / 131, 64 at 960 (127k): 89 / 90
-//   E4B (8, 2 of 256)                  131 rows at 0: 157 / 147, 96 at 512 (107k): 140 / 140, 192 at 192 (110k): 169 / 179
-// so 64k is where the per-row form stops winning.  A block of one head does the work of four: with a KV head per query head (8, 8
-// of 128) the line lies near 16k (96 rows at 0: 97 / 97, 131: 106 / 110, 48 at 192: 76 / 76).
+// Do the rows of a prompt chunk share one pass over their context (ks_sdpa_chunk.cu: 128 rows x heads a block, few blocks of 25 us
+// and more), or does each take the decode kernel (a block per row and up to four heads, spread over the chip)?  By the work of the
+// second form: rows x blocks x positions a row sees on average, in units of 256 dims.  Microseconds per layer, shared / per row:
+//   tiny (4 heads, 1 KV head of 128)   256 rows at 0 (16k): 81 / 69, 512 at 0 (66k): 98 / 100, 256 at 512 (82k): 81 / 77, 320 at 512 (108k): 91 / 91
+//   E2B (8, 1 of 256)                  256 at 0 (66k): 130 / 123, 320 (102k): 140 / 141, 384 (148k): 145 / 155, 128 at 512 (148k): 107 / 97,
+//                                      192 at 512 (234k): 121 / 127, 64 at 1024 (135k): 93 / 88, 96 (206k): 104 / 108
+//   E4B (8, 2 of 256)                  256 at 0: 187 / 181, 320: 229 / 233, 384: 241 / 253, 128 at 512: 146 / 138, 192: 169 / 180, 96 at 1024: 143 / 146
+// so the line lies near 128k.  A block of one head does the work of four: with a KV head per query head (8, 8 of 128) near 48k
+// (128 rows at 0, 33k: 75 / 74, 192, 74k: 77 / 90, 32 at 512, 68k: 61 / 58, 32 at 1024, 133k: 64 / 66).
 bool rows_share_context(const ks_model_config& g, int n, int base, int window) {
   const int hpk = g.n_q / g.n_kv, gb = hpk % 4 == 0 ? 4 : hpk % 2 == 0 ? 2 : 1;
   double seen = base + 0.5 * (n + 1);
   if (window > 0 && seen > window) seen = window;
-  return n >= 4 && (double)n * (g.n_q / gb) * seen * g.hd >= 256.0 * (gb == 1 ? 16384.0 : 65536.0);
+  return n >= 4 && (double)n * (g.n_q / gb) * seen * g.hd >= 256.0 * (gb == 1 ? 49152.0 : 131072.0);
 }
 
 // Where a forward pass reads and writes: n rows of activations, their positions, and the KV caches
