@@ -1237,7 +1237,7 @@ struct ks_mega {
   float* d_att = nullptr;         // records of the attention splits
   unsigned grid = 0;
   size_t smem = 0;
-  int G = 0, dpl = 0, pc = 2;  // pc: 4-element chunks of the hidden vector per thread (480 threads)
+  int dpl = 0, pc = 2;  // pc: 4-element chunks of the hidden vector per thread (480 threads)
   float* residual = nullptr;  // buffer that holds the residual stream when the kernel ends
 };
 
@@ -1448,7 +1448,6 @@ int ks_mega_create(ks_ctx* ctx, const ks_mega_desc* d, const ks_mega_layer* laye
   a.prof = mg->d_prof;
   mg->grid = grid;
   mg->smem = head + ring_bytes;
-  mg->G = (int)G;
   mg->dpl = (int)(hd / 32);
   mg->pc = (int)((H / 4u + MG_THREADS - 1u) / MG_THREADS);
   mg->residual = d->x_b;
