@@ -343,6 +343,12 @@ const void* ks_model_debug_ptr(const ks_model* m, int which, int slot);      /* 
  * of KSEARCH_PROFILE, GP:885,924-929,1260-1273; also switched on by that environment variable; the default
  * kernel always records its stamps). */
 int ks_model_debug_set(ks_model* m, int slot, int what, unsigned value);
+/* Test hook, no GPU needed: where one block of the persistent decode kernel keeps its jobs (runs of weight rows, norm weights) in
+ * shared memory while a token of a model of these widths runs on sm_count SMs with smem_optin bytes a block.  out[3 j] = place of
+ * job j in the ring, [3 j + 1] = its bytes, [3 j + 2] = the oldest job still there when it is placed; at most max_jobs of them are
+ * written.  Returns their number, 0 when the kernel does not take the shape. */
+int ks_debug_decode_ring(int hidden, int ffn, int n_q, int n_kv, int hd, int n_layers, int sm_count, size_t smem_optin, int block,
+                         unsigned* ring_bytes, unsigned* out, int max_jobs);
 /* One slot's rows of a layer's KV cache on the device, [max_seq, n_kv, hd] in Q4_0 (KV:24-60 holds one such
  * buffer per owning layer); which: 0 = K, 1 = V.  For tests and for hosts that snapshot or restore a slot. */
 void* ks_model_kv_ptr(const ks_model* m, int layer, int which, int slot);

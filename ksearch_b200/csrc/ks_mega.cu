@@ -29,6 +29,7 @@
 // register spilled are what they owe it to: arrays left undefined in some lanes stayed live around the phase loop and spilled.
 // Every spin (barrier, tagged word, mbarrier) is bounded; on expiry the block raises the context's status word,
 // drains its copies and leaves, and the other blocks time out the same way.
+#include <cstring>
 #include <utility>
 #include <vector>
 
@@ -493,14 +494,35 @@ __device__ __forceinline__ void mg_stage_addnorm(unsigned char* xs, float* red, 
 // phase's items are its groups x column segments, item i to warp i % MG_WARPS; the partial sums of a row's segments meet in
 // shared memory (slot i).
 constexpr int MG_MAX_P = 192;  // items of one block in one phase
-__device__ __forceinline__ unsigned block_groups(const MegaShape& sh) {
+__host__ __device__ __forceinline__ unsigned block_groups(const MegaShape& sh, unsigned block, unsigned grid) {
   const unsigned total = sh.type == MG_ATTN ? 0u : sh.grp_start[sh.n_seg];
-  return total > blockIdx.x ? (total - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u;
+  return total > block ? (total - block + grid - 1) / grid : 0u;
 }
 // global group index of this block's k-th group
 __device__ __forceinline__ unsigned block_group_id(unsigned k) { return blockIdx.x + k * gridDim.x; }
-// jobs in front of a phase's row groups
-__device__ __forceinline__ unsigned norm_jobs(int kind) { return kind == PH_QKV || kind == PH_GATEUP ? 1u : 0u; }
+// jobs in front of a phase's row groups: two vectors of norm weights
+__host__ __device__ __forceinline__ unsigned norm_jobs(int kind) { return kind == PH_QKV || kind == PH_GATEUP ? 1u : 0u; }
+__host__ __device__ __forceinline__ unsigned job_bytes(const MegaShape& sh, bool norm, unsigned hidden) {
+  return norm ? 8u * hidden : sh.mats * MG_RL * sh.row_bytes;
+}
+// The ring: jobs lie one behind the other and leave in that order.  None wraps: one that does not fit behind the last starts over,
+// and the bytes it passes by are its own until it leaves.  Where a job lies depends on the shape and the block, never on timing.
+struct MegaRing {
+  unsigned bytes, at, used;
+  __host__ __device__ unsigned takes(unsigned room) const { return at + room > bytes ? bytes - at + room : room; }
+  __host__ __device__ bool fits(unsigned room) const { return used + takes(room) <= bytes; }
+  __host__ __device__ unsigned put(unsigned room, unsigned& taken) {
+    taken = takes(room);
+    const unsigned place = at + room > bytes ? 0u : at;
+    at = place + room;
+    used += taken;
+    return place;
+  }
+  __host__ __device__ void drop(unsigned taken) {
+    used -= taken;
+    if (used == 0) at = 0;  // start over, or a job of more than half the ring might never fit
+  }
+};
 // arrivals of item cs of a job with C items
 __device__ __forceinline__ unsigned empty_share(unsigned cs, unsigned C) { return cs == 0 ? MG_EMPTY - C + 1u : 1u; }
 
@@ -953,7 +975,8 @@ static_assert(SM_TAB % 16u == 0 && SM_PSUM % 16u == 0, "vector access");
 // One thread copies the row groups of the whole token in the order they are multiplied, as far ahead as the ring has room.
 __device__ __forceinline__ void mg_copy_jobs(const MegaArgs& a, const MegaShape* shapes, const MegaLayer* layers, const unsigned* ngrp, uint32_t ring_s,
                                              uint32_t full, uint32_t empty, unsigned* joff, unsigned* jbytes, volatile int* stop, unsigned H, unsigned pos) {
-  unsigned head = 0, tail = 0, used = 0, at = 0;
+  unsigned head = 0, tail = 0;
+  MegaRing ring{a.ring_bytes, 0u, 0u};
   for (int layer = 0; layer < a.n_layers; layer++) {
     const MegaLayer& L = layers[layer];
     mg_prefetch_kv(a, L, pos);
@@ -969,9 +992,8 @@ __device__ __forceinline__ void mg_copy_jobs(const MegaArgs& a, const MegaShape*
         if (sh.n_seg > 1 && g >= sh.grp_start[1]) seg = 1;
         if (sh.n_seg > 2 && g >= sh.grp_start[2]) seg = 2;
         const unsigned row0 = (g - sh.grp_start[seg]) * MG_RL, valid = min((unsigned)MG_RL, sh.rows[seg] - row0);
-        const unsigned room = norm ? 8u * H : mats * MG_RL * row_bytes;
-        unsigned skip = at + room > a.ring_bytes ? a.ring_bytes - at : 0u, need = room + skip;  // nothing wraps
-        while (head - tail >= MG_JOBS || used + need > a.ring_bytes) {
+        const unsigned room = job_bytes(sh, norm, H);
+        while (head - tail >= MG_JOBS || !ring.fits(room)) {
           const uint32_t bar = empty + (tail & (MG_JOBS - 1u)) * 8u;
           const unsigned parity = (tail / MG_JOBS) & 1u;
           bool ok = false;
@@ -990,18 +1012,14 @@ __device__ __forceinline__ void mg_copy_jobs(const MegaArgs& a, const MegaShape*
             if (!*stop) atomicOr(a.err, 1u);
             goto out;
           }
-          used -= jbytes[tail & (MG_JOBS - 1u)];
+          ring.drop(jbytes[tail & (MG_JOBS - 1u)]);
           tail++;
-          if (used == 0) {  // empty: start over, or a job of more than half the ring might never fit
-            at = 0;
-            skip = 0;
-            need = room;
-          }
         }
-        if (skip) at = 0;
         const unsigned b = head & (MG_JOBS - 1u);
+        unsigned taken;
+        const unsigned at = ring.put(room, taken);
         joff[b] = at;
-        jbytes[b] = need;
+        jbytes[b] = taken;
         mb_expect(full + b * 8u, norm ? room : mats * valid * row_bytes);  // (its arrival publishes joff)
         if (norm) {
           bulk_in(ring_s + at, kind == PH_QKV ? L.norm[0] : L.norm[4], 4u * H, full + b * 8u);
@@ -1010,8 +1028,6 @@ __device__ __forceinline__ void mg_copy_jobs(const MegaArgs& a, const MegaShape*
         }
         for (unsigned m = 0; m < mats && !norm; m++)
           bulk_in(ring_s + at + m * MG_RL * row_bytes, L.W[sh.w0 + seg + m] + (size_t)row0 * row_bytes, valid * row_bytes, full + b * 8u);
-        at += room;
-        used += need;
         head++;
       }
     }
@@ -1054,7 +1070,7 @@ __global__ void __launch_bounds__(MG_THREADS + 32, 1) mega_kernel(const MegaArgs
     *stop = 0;
   }
   __syncthreads();
-  if (threadIdx.x < PH_PER_LAYER) ngrp[threadIdx.x] = block_groups(shapes[threadIdx.x]);
+  if (threadIdx.x < PH_PER_LAYER) ngrp[threadIdx.x] = block_groups(shapes[threadIdx.x], blockIdx.x, gridDim.x);
   __syncthreads();
   const unsigned hidden = shapes[PH_QKV].cols;
   if (threadIdx.x >= MG_THREADS) {
@@ -1307,40 +1323,42 @@ void ks_mega_destroy(ks_mega* mg) {
   delete mg;
 }
 
-// Returns KS_OK and *out == nullptr when the shape is outside what the kernel covers (the caller keeps
-// the launch-per-op path), a negative code on a CUDA failure.
-int ks_mega_create(ks_ctx* ctx, const ks_mega_desc* d, const ks_mega_layer* layers, ks_mega** out) {
-  *out = nullptr;
-  const unsigned H = d->hidden, F = d->ffn, hd = d->hd, nq = d->n_q, nkv = d->n_kv;
+namespace {
+struct MegaPlan {
+  MegaShape sh[PH_PER_LAYER];
+  unsigned grid, n_splits, tables_bytes, x_off, ring_off, ring_bytes;
+};
+// Phases, splits and shared memory for a model on a chip of `sms` SMs; false: the kernel does not take the shape.
+bool mega_plan(unsigned sms, unsigned smem, const ks_mega_desc& d, MegaPlan& p) {
+  const unsigned H = d.hidden, F = d.ffn, hd = d.hd, nq = d.n_q, nkv = d.n_kv;
   const unsigned qn = nq * hd, kvn = nkv * hd;
-  const unsigned G = nq / nkv;
-  auto even_blocks = [](unsigned cols) { return cols % 512 == 0; };
-  if (!even_blocks(H) || !even_blocks(F) || !even_blocks(qn)) return KS_OK;
-  if (H > 16u * 256u) return KS_OK;  // the fused norms hold the vector in registers
-  if (G < 1 || nq % nkv || !(hd == 128 || hd == 256)) return KS_OK;
+  auto even_blocks = [](unsigned cols) { return cols && cols % 512 == 0; };
+  if (!even_blocks(H) || !even_blocks(F) || !even_blocks(qn)) return false;
+  if (H > 16u * 256u) return false;  // the fused norms hold the vector in registers
+  if (nkv < 1 || nq < nkv || nq % nkv || !(hd == 128 || hd == 256)) return false;
   // one block per (query head, split)
-  unsigned n_splits = (unsigned)ctx->sm_count / nq;
-  if (n_splits > (unsigned)MG_MAX_SPLITS) n_splits = MG_MAX_SPLITS;
-  if (n_splits < 1 || nq > 48) return KS_OK;
-  if (d->n_layers < 1 || d->n_layers > 128) return KS_OK;
+  p.n_splits = sms / nq;
+  if (p.n_splits > (unsigned)MG_MAX_SPLITS) p.n_splits = MG_MAX_SPLITS;
+  if (p.n_splits < 1 || nq > 48) return false;
+  if (d.n_layers < 1 || d.n_layers > 128) return false;
 
-  const unsigned shapes_bytes = SM_LAYERS - SM_TAB;
-  const unsigned tables_bytes = (unsigned)((shapes_bytes + d->n_layers * sizeof(MegaLayer) + 15u) & ~15u);
+  p.tables_bytes = (unsigned)((SM_LAYERS - SM_TAB + d.n_layers * sizeof(MegaLayer) + 15u) & ~15u);
   unsigned maxcols = H > F ? H : F;
   if (qn > maxcols) maxcols = qn;
   unsigned x_bytes = (maxcols / 64u) * (3u * MG_XU + 16u);
   const unsigned att = mg_att_bytes(hd);
   if (att > x_bytes) x_bytes = att;
-  const unsigned x_off = (SM_TAB + tables_bytes + 127u) & ~127u, head = (x_off + x_bytes + 127u) & ~127u;
+  p.x_off = (SM_TAB + p.tables_bytes + 127u) & ~127u;
+  p.ring_off = (p.x_off + x_bytes + 127u) & ~127u;
   unsigned most_job = 4u * (maxcols > 2u * H ? maxcols : 2u * H) / 256u * KS_Q4K_BLOCK_BYTES;  // (gate and up rows are one job)
   if (most_job < 8u * H) most_job = 8u * H;
-  if (head + most_job + 128u > (unsigned)ctx->smem_optin) return KS_OK;
-  const unsigned ring_bytes = ((unsigned)ctx->smem_optin - head) & ~127u;
+  if (p.ring_off + most_job + 128u > smem) return false;
+  p.ring_bytes = (smem - p.ring_off) & ~127u;
   // Blocks per column segment.  A block's items (its groups x column segments) are shared by its warps, so more segments shorten
   // the longest warp until the per-item overhead (measured: a little more than one unit's worth of time) wins; segments hold an
   // even number of blocks (8 lanes per row).
-  const unsigned grid = (unsigned)ctx->sm_count;
-  if (grid > MG_THREADS) return KS_OK;  // a thread folds the norm sums of a block
+  const unsigned grid = p.grid = sms;
+  if (grid > MG_THREADS) return false;  // a thread folds the norm sums of a block
   auto pick_seg = [&](unsigned cols, unsigned mats, unsigned total_groups) {
     const unsigned nb = cols / 256u, n_g = (total_groups + grid - 1) / grid;
     unsigned best = 0;
@@ -1359,13 +1377,14 @@ int ks_mega_create(ks_ctx* ctx, const ks_mega_desc* d, const ks_mega_layer* laye
   };
   const unsigned g_qkv = (qn + 3) / 4 + 2 * ((kvn + 3) / 4), g_h = (H + 3) / 4, g_f = (F + 3) / 4;
   const unsigned most_g = MG_THREADS / MG_RL * grid;  // a block finishes a row per thread
-  if (g_qkv > most_g || g_f > most_g || g_h > most_g) return KS_OK;
+  if (g_qkv > most_g || g_f > most_g || g_h > most_g) return false;
   const unsigned sb_h = pick_seg(H, 1, g_qkv), sb_q = pick_seg(qn, 1, g_h), sb_f = pick_seg(F, 1, g_h), sb_h2 = pick_seg(H, 2, g_f);
-  if (!sb_h || !sb_h2 || !sb_q || !sb_f) return KS_OK;
-  std::vector<unsigned char> tab(tables_bytes, 0);
-  MegaShape* sh = reinterpret_cast<MegaShape*>(tab.data());
-  MegaLayer* ly = reinterpret_cast<MegaLayer*>(tab.data() + shapes_bytes);
-  for (int k = 0; k < PH_PER_LAYER; k++) sh[k].mats = 1;
+  if (!sb_h || !sb_h2 || !sb_q || !sb_f) return false;
+  MegaShape* sh = p.sh;
+  for (int k = 0; k < PH_PER_LAYER; k++) {
+    sh[k] = MegaShape{};
+    sh[k].mats = 1;
+  }
   sh[PH_OPROJ].w0 = 3;
   sh[PH_DOWN].w0 = 6;
   auto set_rows = [](MegaShape& p, unsigned cols, unsigned sb) {
@@ -1390,6 +1409,49 @@ int ks_mega_create(ks_ctx* ctx, const ks_mega_desc* d, const ks_mega_layer* laye
   set_rows(sh[PH_GATEUP], H, sb_h2);
   sh[PH_DOWN].type = MG_MATVEC; sh[PH_DOWN].n_seg = 1; sh[PH_DOWN].rows[0] = H;
   set_rows(sh[PH_DOWN], F, sb_f);
+  return true;
+}
+}  // namespace
+
+// The places block `block`'s jobs take in its ring during a token, in order: out[3 j] = place, [3 j + 1] = bytes, [3 j + 2] = the first
+// job still there (`max_jobs` of them at most).  Returns their number, 0 where the kernel does not take the shape.  Host only.
+extern "C" int ks_debug_decode_ring(int hidden, int ffn, int n_q, int n_kv, int hd, int n_layers, int sm_count, size_t smem_optin, int block,
+                                    unsigned* ring_bytes, unsigned* out, int max_jobs) {
+  ks_mega_desc d{};
+  d.n_layers = n_layers;
+  d.hidden = (unsigned)hidden; d.ffn = (unsigned)ffn; d.n_q = (unsigned)n_q; d.n_kv = (unsigned)n_kv; d.hd = (unsigned)hd;
+  MegaPlan p;
+  if (hidden < 1 || ffn < 1 || n_q < 1 || n_kv < 1 || hd < 1 || block < 0 || block >= sm_count || !mega_plan((unsigned)sm_count, (unsigned)smem_optin, d, p)) return 0;
+  if (ring_bytes) *ring_bytes = p.ring_bytes;
+  MegaRing ring{p.ring_bytes, 0u, 0u};
+  unsigned taken[MG_JOBS], head = 0, tail = 0;
+  for (int layer = 0; layer < n_layers; layer++)
+    for (int kind = 0; kind < PH_PER_LAYER; kind++) {
+      const unsigned norms = norm_jobs(kind), n = block_groups(p.sh[kind], (unsigned)block, p.grid) + norms;
+      for (unsigned k = 0; k < n; k++, head++) {
+        const unsigned room = job_bytes(p.sh[kind], k < norms, d.hidden);
+        for (; head - tail >= MG_JOBS || !ring.fits(room); tail++) ring.drop(taken[tail & (MG_JOBS - 1u)]);
+        const unsigned at = ring.put(room, taken[head & (MG_JOBS - 1u)]);
+        if (out && head < (unsigned)max_jobs) {
+          out[3 * head] = at;
+          out[3 * head + 1] = room;
+          out[3 * head + 2] = tail;
+        }
+      }
+    }
+  return (int)head;
+}
+
+// Returns KS_OK and *out == nullptr when the shape is outside what the kernel covers (the caller keeps
+// the launch-per-op path), a negative code on a CUDA failure.
+int ks_mega_create(ks_ctx* ctx, const ks_mega_desc* d, const ks_mega_layer* layers, ks_mega** out) {
+  *out = nullptr;
+  MegaPlan p;
+  if (!mega_plan((unsigned)ctx->sm_count, (unsigned)ctx->smem_optin, *d, p)) return KS_OK;
+  const unsigned H = d->hidden, F = d->ffn, hd = d->hd, nq = d->n_q, nkv = d->n_kv, qn = nq * hd, kvn = nkv * hd, n_splits = p.n_splits;
+  std::vector<unsigned char> tab(p.tables_bytes, 0);
+  memcpy(tab.data(), p.sh, sizeof(p.sh));
+  MegaLayer* ly = reinterpret_cast<MegaLayer*>(tab.data() + (SM_LAYERS - SM_TAB));
   for (int l = 0; l < d->n_layers; l++) {
     const ks_mega_layer& L = layers[l];
     MegaLayer& o = ly[l];
@@ -1404,7 +1466,7 @@ int ks_mega_create(ks_ctx* ctx, const ks_mega_desc* d, const ks_mega_layer* laye
   ks_mega* mg = new ks_mega();
   cudaSetDevice(ctx->device);
   const size_t n_phases = (size_t)d->n_layers * PH_PER_LAYER;
-  if (cudaMalloc(&mg->d_tables, tables_bytes) != cudaSuccess || cudaMalloc((void**)&mg->d_sync, 512 + 16 * (size_t)ctx->sm_count) != cudaSuccess ||
+  if (cudaMalloc(&mg->d_tables, p.tables_bytes) != cudaSuccess || cudaMalloc((void**)&mg->d_sync, 512 + 16 * (size_t)ctx->sm_count) != cudaSuccess ||
       cudaMalloc((void**)&mg->d_prof, n_phases * 16 * sizeof(long long)) != cudaSuccess ||
       cudaMalloc((void**)&mg->d_fx, (size_t)qn / 64 * 256 + F * sizeof(float)) != cudaSuccess ||
       cudaMalloc((void**)&mg->d_att, (size_t)nq * n_splits * mg_rec(hd) * sizeof(float)) != cudaSuccess ||
@@ -1412,7 +1474,7 @@ int ks_mega_create(ks_ctx* ctx, const ks_mega_desc* d, const ks_mega_layer* laye
     ks_mega_destroy(mg);
     return ks_fail(ctx, KS_ERR_OOM, "decode kernel: cannot allocate its tables");
   }
-  cudaError_t e = cudaMemcpyAsync(mg->d_tables, tab.data(), tables_bytes, cudaMemcpyHostToDevice, ctx->stream);
+  cudaError_t e = cudaMemcpyAsync(mg->d_tables, tab.data(), p.tables_bytes, cudaMemcpyHostToDevice, ctx->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(mg->d_sync, 0, 512 + 16 * (size_t)ctx->sm_count, ctx->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(mg->d_fx, 0, (size_t)qn / 64 * 256 + F * sizeof(float), ctx->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(mg->d_prof, 0, n_phases * 16 * sizeof(long long), ctx->stream);
@@ -1425,11 +1487,11 @@ int ks_mega_create(ks_ctx* ctx, const ks_mega_desc* d, const ks_mega_layer* laye
   }
   MegaArgs& a = mg->args;
   a.tables = mg->d_tables;
-  a.tables_bytes = tables_bytes;
+  a.tables_bytes = p.tables_bytes;
   a.n_layers = d->n_layers;
-  a.ring_bytes = ring_bytes;
-  a.x_off = x_off;
-  a.ring_off = head;
+  a.ring_bytes = p.ring_bytes;
+  a.x_off = p.x_off;
+  a.ring_off = p.ring_off;
   a.n_q = nq; a.n_kv = nkv; a.hd = hd; a.n_splits = n_splits;
   a.eps = d->eps; a.attn_scale = d->attn_scale;
   a.rope = d->rope; a.pos = d->pos;
@@ -1446,8 +1508,8 @@ int ks_mega_create(ks_ctx* ctx, const ks_mega_desc* d, const ks_mega_layer* laye
   a.poll_limit = 1u << 21;
   a.test_stall = 0;
   a.prof = mg->d_prof;
-  mg->grid = grid;
-  mg->smem = head + ring_bytes;
+  mg->grid = p.grid;
+  mg->smem = p.ring_off + p.ring_bytes;
   mg->dpl = (int)(hd / 32);
   mg->pc = (int)((H / 4u + MG_THREADS - 1u) / MG_THREADS);
   mg->residual = d->x_b;

@@ -45,3 +45,17 @@ def test_attention_forms_and_widths(monkeypatch, hidden, n_q, n_kv, hd, window):
     for g, w in zip(got, want):
         scale, err = np.abs(w).max(), np.abs(g - w)
         assert err.max() <= 1e-3 * scale and np.sqrt((err ** 2).mean()) <= 1e-4 * scale   # the bound of tests/test_gpu_model.py
+
+
+@pytest.mark.parametrize("hidden,ffn,n_q,n_kv,hd,layers", [(512, 1024, 4, 1, 128, 18), (1536, 6144, 8, 1, 256, 3), (2560, 10240, 8, 2, 256, 9)])
+def test_jobs_that_end_where_the_ring_ends(monkeypatch, hidden, ffn, n_q, n_kv, hd, layers):
+    """Depths at which a run of weight rows fills the ring to its last byte (tests/test_decode_ring.py holds the places)."""
+    cfg = ksm.tiny_config(max_seq=64, n_kv=n_kv)
+    cfg.hidden, cfg.ffn, cfg.n_q, cfg.hd, cfg.n_layers, cfg.sigma_w = hidden, ffn, n_q, hd, layers, 2e-4
+    toks = [int(t) for t in synth.token_ids(44, "p", 20, cfg.vocab)]
+    got, persistent = _logits(cfg, "1", monkeypatch, toks, (0, 9))
+    assert persistent
+    want, _ = _logits(cfg, "0", monkeypatch, toks, (0, 9))
+    for g, w in zip(got, want):
+        scale, err = np.abs(w).max(), np.abs(g - w)
+        assert err.max() <= 1e-3 * scale and np.sqrt((err ** 2).mean()) <= 1e-4 * scale
