@@ -343,6 +343,13 @@ const void* ks_model_debug_ptr(const ks_model* m, int which, int slot);      /* 
  * of KSEARCH_PROFILE, GP:885,924-929,1260-1273; also switched on by that environment variable; the default
  * kernel always records its stamps). */
 int ks_model_debug_set(ks_model* m, int slot, int what, unsigned value);
+/* Test hook: the attention of prompt rows that share passes over their contexts, alone.  Rows row0[p]..row0[p + 1] - 1 of q
+ * [rows, n_q hd] f32 read the Q4_0 cache at slots[p] * slot_stride_bytes of K and V ([max_t, n_kv, hd] each); meta [rows][4] =
+ * (tlen, start, -, -), both ends growing along a part and start + tlen <= max_t (trusted); tmp gets [rows][n_q][n_splits][hd + 2]
+ * records (m, l, O). */
+int ks_debug_sdpa_chunk(ks_ctx* ctx, size_t n_q, size_t n_kv, size_t hd, size_t max_t, float scale, int n_parts, const int* row0,
+                        const int* slots, size_t slot_stride_bytes, const ks_buf* q, const ks_buf* K, const ks_buf* V,
+                        const ks_buf* meta, ks_buf* tmp, int n_splits);
 /* Test hook, no GPU needed: where one block of the persistent decode kernel keeps its jobs (runs of weight rows, norm weights) in
  * shared memory while a token of a model of these widths runs on sm_count SMs with smem_optin bytes a block.  out[3 j] = place of
  * job j in the ring, [3 j + 1] = its bytes, [3 j + 2] = the oldest job still there when it is placed; at most max_jobs of them are

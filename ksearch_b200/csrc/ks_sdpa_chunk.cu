@@ -27,6 +27,7 @@ constexpr int CH_BM = 128, CH_BN = 64;                 // query rows, positions 
 constexpr int CH_ROW_WARPS = 4, CH_DEC_WARPS = 8, CH_WORK = (CH_ROW_WARPS + CH_DEC_WARPS) * 32, CH_THREADS = CH_WORK + 128;
 constexpr unsigned CH_WAIT = 1u << 20;
 constexpr float CH_P = 256.0f;                         // probabilities carry 2^8
+constexpr float CH_K_MOST = 8188.0f;                   // the largest scale with 8 d in f16
 constexpr float kNegInit = -1.0e30f;
 
 // barriers: operands ready (decoders, row warps), the tile's O taken (decoders), products ready (commits: scores done = K free;
@@ -38,7 +39,9 @@ struct ChunkSmem {
   static constexpr unsigned NB = HD / 32, ROWB = NB * KS_Q40_BLOCK_BYTES, RP = ROWB + 4;
   static constexpr unsigned slot = 64, row = 128;     // tensor-memory address, failure flag; per row: scale, first, past the last position, maximum,
                                                       // then what the sums so far are multiplied by, of two tiles
+  static constexpr unsigned up = row + CH_BM * 24;    // of two tiles: what their scores are multiplied by
   static constexpr unsigned raw = 4096;
+  static_assert(up + 8 <= raw, "the rows' words fit in front of the packed rows");
   static constexpr unsigned ql = (raw + 2 * CH_BN * RP + 1023u) & ~1023u, kh = ql + CH_BM * HD * 2, kl = kh + CH_BN * HD * 2, vh = kl + CH_BN * HD * 2,
                             vl = vh + CH_BN * HD * 2, total = vl + CH_BN * HD * 2;
   static constexpr unsigned o = ql, OP = HD + 4;      // the result on its way out: rows of OP floats
@@ -103,6 +106,7 @@ sdpa_chunk_kernel(const __grid_constant__ ChunkParts parts, size_t slot_stride, 
   int* row_end = reinterpret_cast<int*>(smem + S::row + CH_BM * 8);
   unsigned* row_max = reinterpret_cast<unsigned*>(smem + S::row + CH_BM * 12);
   float* row_alpha = reinterpret_cast<float*>(smem + S::row + CH_BM * 16);
+  float* tile_up = reinterpret_cast<float*>(smem + S::up);
 
   // ---- the block's rows: row r is query head kvh G + r % G of token (row0 + r) / G; positions they see at all
   const unsigned tok_a = row0 / G, tok_b = min((row0 + CH_BM - 1u) / G, n_tok - 1u);
@@ -223,10 +227,11 @@ sdpa_chunk_kernel(const __grid_constant__ ChunkParts parts, size_t slot_stride, 
 #pragma unroll
       for (int k = 0; k < 4; k++) tc_wait_ld16(s[k]);
       const int p0 = t_begin + (int)i * CH_BN, a = first - p0, b = min(end, t_end) - p0;  // columns [a, b) are seen
+      const float st = sc * tile_up[i & 1u];
       float mx = -INFINITY;
 #pragma unroll
       for (int j = 0; j < CH_BN; j++) {
-        const float x = j >= a && j < b ? __uint_as_float(s[j / 16][j % 16]) * sc : -INFINITY;
+        const float x = j >= a && j < b ? __uint_as_float(s[j / 16][j % 16]) * st : -INFINITY;
         s[j / 16][j % 16] = __float_as_uint(x);
         mx = fmaxf(mx, x);
       }
@@ -292,31 +297,43 @@ sdpa_chunk_kernel(const __grid_constant__ ChunkParts parts, size_t slot_stride, 
       asm volatile("cp.async.wait_all;" ::: "memory");
       if (i > 0) ok = mb_wait(bar(CB_K_FREE), (i - 1u) & 1u, CH_WAIT);
       if (!dec_all(ok)) { ok = false; break; }  // the raw rows are there, K is free
+      // A tile with a scale whose products leave f16 is decoded again at an eighth and its scores multiplied by 8; what that rounds
+      // off (2^-22 of a value at most) is nothing beside a value of 57000.
+      float tile = 1.0f;
+      for (;;) {
+        const __half down = __float2half_rn(1.0f / tile);
+        bool fits = true;
 #pragma unroll 1
-      for (unsigned job = dt; job < CH_BN * NB; job += CH_DEC_WARPS * 32) {  // a block of a row
-        const unsigned p = job % CH_BN, b = job / CH_BN;
-        const unsigned char* src = smem + S::raw + p * RP + b * KS_Q40_BLOCK_BYTES;
-        const __half2 d = __half2half2(__ushort_as_half(*reinterpret_cast<const unsigned short*>(src)));
-        uint32_t w[4];
+        for (unsigned job = dt; job < CH_BN * NB; job += CH_DEC_WARPS * 32) {  // a block of a row
+          const unsigned p = job % CH_BN, b = job / CH_BN;
+          const unsigned char* src = smem + S::raw + p * RP + b * KS_Q40_BLOCK_BYTES;
+          const __half raw_d = __ushort_as_half(*reinterpret_cast<const unsigned short*>(src));
+          fits = fits && !(__habs(raw_d) > __float2half_rn(CH_K_MOST));
+          const __half2 d = __half2half2(__hmul(raw_d, down));
+          uint32_t w[4];
 #pragma unroll
-        for (int k = 0; k < 4; k++)
-          w[k] = *reinterpret_cast<const unsigned short*>(src + 2 + 4 * k) | (uint32_t)*reinterpret_cast<const unsigned short*>(src + 4 + 4 * k) << 16;
+          for (int k = 0; k < 4; k++)
+            w[k] = *reinterpret_cast<const unsigned short*>(src + 2 + 4 * k) | (uint32_t)*reinterpret_cast<const unsigned short*>(src + 4 + 4 * k) << 16;
 #pragma unroll 1
-        for (int half = 0; half < 2; half++)  // dims 0..15 of the block are the low nibbles
+          for (int half = 0; half < 2; half++)  // dims 0..15 of the block are the low nibbles
 #pragma unroll
-          for (int c = 0; c < 2; c++) {
-            uint32_t hi[4], lo[4];
+            for (int c = 0; c < 2; c++) {
+              uint32_t hi[4], lo[4];
 #pragma unroll
-            for (int k = 0; k < 2; k++) {
-              const uint32_t x = half ? w[2 * c + k] >> 4 : w[2 * c + k];
-              split_d(nib_h2(__byte_perm(x, 0u, 0x4140)), d, hi[2 * k], lo[2 * k]);
-              split_d(nib_h2(__byte_perm(x, 0u, 0x4342)), d, hi[2 * k + 1], lo[2 * k + 1]);
+              for (int k = 0; k < 2; k++) {
+                const uint32_t x = half ? w[2 * c + k] >> 4 : w[2 * c + k];
+                split_d(nib_h2(__byte_perm(x, 0u, 0x4140)), d, hi[2 * k], lo[2 * k]);
+                split_d(nib_h2(__byte_perm(x, 0u, 0x4342)), d, hi[2 * k + 1], lo[2 * k + 1]);
+              }
+              const unsigned at = ((4u * b + 2u * half + c) * CH_BN + p) * 16u;
+              *reinterpret_cast<uint4*>(smem + S::kh + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+              *reinterpret_cast<uint4*>(smem + S::kl + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
             }
-            const unsigned at = ((4u * b + 2u * half + c) * CH_BN + p) * 16u;
-            *reinterpret_cast<uint4*>(smem + S::kh + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            *reinterpret_cast<uint4*>(smem + S::kl + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-          }
+        }
+        if (tile != 1.0f || dec_all(fits)) break;
+        tile = 8.0f;
       }
+      if (dt == 0) tile_up[i & 1u] = tile;
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) mb_arrive1(bar(CB_K_FULL));
@@ -579,4 +596,28 @@ int ks_launch_sdpa_merge_split(ks_ctx* ctx, int n_tok, ks_gemm_blocks b, size_t 
   const unsigned chunks = (unsigned)(n_q * hd / 8), threads = chunks < 512u ? (chunks + 31u) / 32u * 32u : 512u;
   KS_LAUNCH(ctx, sdpa_merge_split_kernel, b.np, threads, (size_t)n_q * n_splits * sizeof(float), (unsigned)n_tok, b.np, b.tbn, (unsigned)n_q, (unsigned)hd, tmp, (unsigned)n_splits, (__half*)xt);
   return ks_after_launch(ctx, "sdpa_merge_split");
+}
+
+// Chunk attention alone, for tests.
+extern "C" int ks_debug_sdpa_chunk(ks_ctx* ctx, size_t n_q, size_t n_kv, size_t hd, size_t max_t, float scale, int n_parts, const int* row0, const int* slots,
+                                   size_t slot_stride_bytes, const ks_buf* q, const ks_buf* K, const ks_buf* V, const ks_buf* meta, ks_buf* tmp, int n_splits) {
+  if (!ctx) return KS_ERR_INVALID;
+  KS_REQUIRE(ctx, n_q > 0 && n_kv > 0 && n_q % n_kv == 0 && hd % 32 == 0 && max_t > 0 && n_splits >= 1 && n_splits < 65536, "sdpa_chunk: bad shape");
+  KS_REQUIRE(ctx, n_parts >= 1 && n_parts <= 64 && row0 && slots && row0[0] == 0 && slot_stride_bytes % 4 == 0, "sdpa_chunk: bad parts");
+  const size_t cache = max_t * n_kv * (hd / 32) * KS_Q40_BLOCK_BYTES;
+  ks_row_parts parts{};
+  parts.n = (unsigned)n_parts;
+  size_t last = 0;
+  for (int p = 0; p < n_parts; p++) {
+    KS_REQUIRE(ctx, row0[p + 1] > row0[p] && row0[p + 1] <= KS_GEMM_ROWS && slots[p] >= 0, "sdpa_chunk: bad parts");
+    parts.row0[p + 1] = (unsigned)row0[p + 1];
+    parts.slot[p] = (unsigned)slots[p];
+    last = (size_t)slots[p] > last ? (size_t)slots[p] : last;
+  }
+  const size_t n = (size_t)row0[n_parts], need = last * slot_stride_bytes + cache;
+  KS_REQUIRE(ctx, ks_fits(K, 0, need) && ks_fits(V, 0, need) && ks_fits(q, 0, n * n_q * hd * 4) && ks_fits(meta, 0, n * 16) &&
+             ks_fits(tmp, 0, n * n_q * (size_t)n_splits * (hd + 2) * 4), "sdpa_chunk: a buffer is too small");
+  if (!ks_sdpa_chunk_covers(n_q, n_kv, hd, K->dptr, V->dptr)) return ks_fail(ctx, KS_ERR_UNSUPPORTED, "sdpa_chunk: shape not covered");
+  return ks_launch_sdpa_chunk(ctx, (int)n, n_q, n_kv, hd, scale, (const float*)q->dptr, (const uint8_t*)K->dptr, (const uint8_t*)V->dptr, (const float*)meta->dptr,
+                              (float*)tmp->dptr, n_splits, &parts, slot_stride_bytes);
 }
