@@ -343,6 +343,8 @@ const void* ks_model_debug_ptr(const ks_model* m, int which, int slot);      /* 
  * of KSEARCH_PROFILE, GP:885,924-929,1260-1273; also switched on by that environment variable; the default
  * kernel always records its stamps). */
 int ks_model_debug_set(ks_model* m, int slot, int what, unsigned value);
+/* Test hook: captured launch sequences the model holds. */
+int ks_model_debug_graphs(const ks_model* m);
 /* Test hook: the attention of prompt rows that share passes over their contexts, alone.  Rows row0[p]..row0[p + 1] - 1 of q
  * [rows, n_q hd] f32 read the Q4_0 cache at slots[p] * slot_stride_bytes of K and V ([max_t, n_kv, hd] each); meta [rows][4] =
  * (tlen, start, -, -), both ends growing along a part and start + tlen <= max_t (trusted); tmp gets [rows][n_q][n_splits][hd + 2]

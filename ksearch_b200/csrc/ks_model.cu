@@ -165,9 +165,19 @@ struct ks_model {
   // sampled steps (built on first use): candidates of every slot on the device and in pinned memory
   ks_cand_head* cand_head = nullptr;  // [n_slots] heads, then [n_slots][KS_CAND_MAX] pairs
   void* host_cand = nullptr;
-  // graphs keyed by (first slot, n slots, src parity, want_logits); of prompt chunks by (slot, rows, attention forms)
-  std::map<uint64_t, cudaGraphExec_t> graphs;
-  std::map<uint64_t, size_t> graph_nodes;
+  // graphs keyed by (first slot, n slots, src parity, want_logits); of prompt rows that go through the batch matvec by (slot, rows)
+  struct Graph {
+    cudaGraphExec_t exec = nullptr;
+    size_t nodes = 0;
+  };
+  std::map<uint64_t, Graph> graphs;
+  // the prompt passes through the GEMM that came last, by (slot, rows, attention forms); one that came again has its graph
+  struct PromptGraph {
+    uint64_t key = 0, last = 0;  // last: number of the pass that used it
+    Graph graph;
+  };
+  std::vector<PromptGraph> prompt_graphs;
+  uint64_t prompt_passes = 0;
   std::vector<void*> owned;
   std::vector<char> tok_src;  // per slot: which half of the ping-pong holds its next input id
   // ids that come from the host are read by the embedding kernel straight out of this pinned, device-visible array
@@ -667,6 +677,41 @@ int get_mega(ks_model* m, int first, ks_model::Mega* out) {
   return KS_OK;
 }
 
+// What `enqueue` launches, as a graph.  Nothing runs.
+template <class F>
+int capture(ks_ctx* c, F&& enqueue, ks_model::Graph* out) {
+  cudaGraph_t graph = nullptr;
+  KS_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+  const uint64_t before = c->launches;
+  const int rc = enqueue();
+  cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
+  c->launches = before;  // captured launches are counted when the graph replays
+  if (rc) {
+    if (graph) cudaGraphDestroy(graph);
+    return rc;
+  }
+  if (e != cudaSuccess) return ks_fail(c, KS_ERR_CUDA, "model: graph capture failed: %s", cudaGetErrorString(e));
+  ks_model::Graph g;
+  e = cudaGraphInstantiate(&g.exec, graph, 0);
+  cudaGraphGetNodes(graph, nullptr, &g.nodes);
+  cudaGraphDestroy(graph);
+  if (e != cudaSuccess) return ks_fail(c, KS_ERR_CUDA, "model: graph instantiate failed: %s", cudaGetErrorString(e));
+  *out = g;
+  return KS_OK;
+}
+int replay(ks_ctx* c, const ks_model::Graph& g) {
+  KS_CUDA(c, cudaGraphLaunch(g.exec, c->stream));
+  c->launches += g.nodes;
+  return KS_OK;
+}
+void drop_graphs(ks_model* m) {
+  for (auto& kv : m->graphs) cudaGraphExecDestroy(kv.second.exec);
+  m->graphs.clear();
+  for (auto& p : m->prompt_graphs)
+    if (p.graph.exec) cudaGraphExecDestroy(p.graph.exec);
+  m->prompt_graphs.clear();
+}
+
 // Launch the forward pass through a cached graph (captured on first use).
 int run_forward(ks_model* m, int first, int n, int src, bool want_logits) {
   ks_ctx* c = m->ctx;
@@ -674,75 +719,71 @@ int run_forward(ks_model* m, int first, int n, int src, bool want_logits) {
   auto it = m->graphs.find(key);
   if (it == m->graphs.end()) {
     ks_model::Mega mg;
-    if (n == 1) {
-      int rcm = get_mega(m, first, &mg);
-      if (rcm) return rcm;
-    }
-    cudaGraph_t graph = nullptr;
-    KS_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    const uint64_t before = c->launches;
+    int rc = n == 1 ? get_mega(m, first, &mg) : KS_OK;
+    if (rc) return rc;
     const Lane lane = slot_lane(m, first, src);
-    int rc = mg ? enqueue_forward_mega(m, mg, first, src, want_logits)
+    ks_model::Graph g;
+    rc = capture(c, [&] {
+      return mg ? enqueue_forward_mega(m, mg, first, src, want_logits)
              : n > m->chunk ? enqueue_forward_gemm(m, lane, n, want_logits)
              : m->fused ? enqueue_forward_fused(m, lane, n, want_logits)
                         : enqueue_forward(m, lane, n, want_logits);
-    cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
-    c->launches = before;  // captured launches are counted when the graph replays
-    if (rc) {
-      if (graph) cudaGraphDestroy(graph);
-      return rc;
-    }
-    if (e != cudaSuccess) return ks_fail(c, KS_ERR_CUDA, "model: graph capture failed: %s", cudaGetErrorString(e));
-    cudaGraphExec_t exec = nullptr;
-    e = cudaGraphInstantiate(&exec, graph, 0);
-    size_t nodes = 0;
-    cudaGraphGetNodes(graph, nullptr, &nodes);
-    cudaGraphDestroy(graph);
-    if (e != cudaSuccess) return ks_fail(c, KS_ERR_CUDA, "model: graph instantiate failed: %s", cudaGetErrorString(e));
-    m->graphs[key] = exec;
-    m->graph_nodes[key] = nodes;
-    it = m->graphs.find(key);
+    }, &g);
+    if (rc) return rc;
+    it = m->graphs.emplace(key, g).first;
   }
-  KS_CUDA(c, cudaGraphLaunch(it->second, c->stream));
-  c->launches += m->graph_nodes[key];
-  return KS_OK;
+  return replay(c, it->second);
 }
 
-// A chunk of n prompt tokens of one slot (ids already in m->ctok) through every layer, no head.
+// Prompt passes through the GEMM hardly repeat their row counts, and a capture (1.2 to 2 ms of host time, now and then 10 to 25) costs
+// more than the launches (0.7 to 1.4 ms, behind which the GPU works).  So a pass is launched as it is; one that comes again among the
+// last KS_PROMPT_GRAPHS different ones gets a graph, which saves 0.1 to 0.2 ms of every later pass.  E2B, captured at once / launched /
+// replayed: 20 rows 3.3 / 2.16 / 2.04 ms, 300 rows 6.0 / 4.84 / 4.71, 600 rows 8.7 / 7.31 / 7.22, 2047 rows 20.6 / 19.5 / 19.3; E4B 300
+// rows 11.1 / 9.6 / 9.3.
+constexpr size_t KS_PROMPT_GRAPHS = 64;
+
+// A chunk of n prompt tokens of one slot (ids already in m->ctok) through every layer, no head.  The stream is idle but for the ids'
+// copy, so a graph may be dropped.
 int run_prefill_chunk(ks_model* m, int slot, int n, bool gemm) {
   ks_ctx* c = m->ctx;
-  const bool share_full = rows_share_context(m->cfg, n, m->seq_len[slot], 0);
-  const bool share_swa = rows_share_context(m->cfg, n, m->seq_len[slot], m->cfg.sliding_window);
-  const uint64_t key = (1ull << 63) | ((uint64_t)slot << 32) | ((uint64_t)n << 8) | (gemm && share_full ? 1 : 0) | (gemm && share_swa && has_window(m->cfg) ? 2 : 0);
-  auto it = m->graphs.find(key);
-  if (it == m->graphs.end()) {
-    cudaGraph_t graph = nullptr;
-    KS_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    const uint64_t before = c->launches;
-    const Lane lane = chunk_lane(m, slot, share_full, share_swa);
-    int rc = gemm       ? enqueue_forward_gemm(m, lane, n, false)
-             : m->fused ? enqueue_forward_fused(m, lane, n, false)
-                        : enqueue_forward(m, lane, n, false);
-    cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
-    c->launches = before;
-    if (rc) {
-      if (graph) cudaGraphDestroy(graph);
-      return rc;
+  const bool share_full = gemm && rows_share_context(m->cfg, n, m->seq_len[slot], 0);
+  const bool share_swa = gemm && rows_share_context(m->cfg, n, m->seq_len[slot], m->cfg.sliding_window);
+  const Lane lane = chunk_lane(m, slot, share_full, share_swa);
+  const uint64_t key = (1ull << 63) | ((uint64_t)slot << 32) | ((uint64_t)n << 8) | (share_full ? 1 : 0) | (share_swa && has_window(m->cfg) ? 2 : 0);
+  if (!gemm) {  // 1..8 rows: few different passes
+    auto it = m->graphs.find(key);
+    if (it == m->graphs.end()) {
+      ks_model::Graph g;
+      const int rc = capture(c, [&] { return m->fused ? enqueue_forward_fused(m, lane, n, false) : enqueue_forward(m, lane, n, false); }, &g);
+      if (rc) return rc;
+      it = m->graphs.emplace(key, g).first;
     }
-    if (e != cudaSuccess) return ks_fail(c, KS_ERR_CUDA, "model: graph capture failed: %s", cudaGetErrorString(e));
-    cudaGraphExec_t exec = nullptr;
-    e = cudaGraphInstantiate(&exec, graph, 0);
-    size_t nodes = 0;
-    cudaGraphGetNodes(graph, nullptr, &nodes);
-    cudaGraphDestroy(graph);
-    if (e != cudaSuccess) return ks_fail(c, KS_ERR_CUDA, "model: graph instantiate failed: %s", cudaGetErrorString(e));
-    m->graphs[key] = exec;
-    m->graph_nodes[key] = nodes;
-    it = m->graphs.find(key);
+    return replay(c, it->second);
   }
-  KS_CUDA(c, cudaGraphLaunch(it->second, c->stream));
-  c->launches += m->graph_nodes[key];
-  return KS_OK;
+  ks_model::PromptGraph *at = nullptr, *oldest = nullptr;
+  for (auto& p : m->prompt_graphs) {
+    if (p.key == key) at = &p;
+    if (!oldest || p.last < oldest->last) oldest = &p;
+  }
+  const bool again = at != nullptr;
+  if (!at) {
+    if (m->prompt_graphs.size() < KS_PROMPT_GRAPHS) {
+      m->prompt_graphs.emplace_back();
+      at = &m->prompt_graphs.back();
+    } else {
+      at = oldest;
+      if (at->graph.exec) cudaGraphExecDestroy(at->graph.exec);
+      at->graph = {};
+    }
+    at->key = key;
+  }
+  at->last = ++m->prompt_passes;
+  if (!again) return enqueue_forward_gemm(m, lane, n, false);
+  if (!at->graph.exec) {
+    const int rc = capture(c, [&] { return enqueue_forward_gemm(m, lane, n, false); }, &at->graph);
+    if (rc) return rc;
+  }
+  return replay(c, at->graph);
 }
 
 }  // namespace
@@ -988,9 +1029,7 @@ int ks_model_warm_plans(ks_model* m, int n_tok) {
   found += ks_plan_search(c, g.embd_dtype == KS_Q6K ? "mv_q6k" : "mv_q4k", (size_t)g.vocab, 0, H, n_tok, nullptr) == KS_OK;
   // plans change the captured launches: drop graphs recorded before
   cudaStreamSynchronize(c->stream);
-  for (auto& kv : m->graphs) cudaGraphExecDestroy(kv.second);
-  m->graphs.clear();
-  m->graph_nodes.clear();
+  drop_graphs(m);
   return found;
 }
 
@@ -998,7 +1037,7 @@ void ks_model_destroy(ks_model* m) {
   if (!m) return;
   cudaSetDevice(m->ctx->device);
   cudaStreamSynchronize(m->ctx->stream);
-  for (auto& kv : m->graphs) cudaGraphExecDestroy(kv.second);
+  drop_graphs(m);
   for (auto& kv : m->mega) {
     if (kv.second.bar) ks_mega_destroy(kv.second.bar);
     if (kv.second.flow) ks_flow_destroy(kv.second.flow);
@@ -1307,7 +1346,7 @@ int ks_model_prefill(ks_model* m, int slot, const int* tokens, int n_tokens) {
 
 // Prompt tokens of several slots (counts[i] of them for slots[i], behind one another in `tokens`): their rows share passes over the
 // weights, up to KS_GEMM_CHUNK a pass.  Everything is checked before anything runs.  A pass of one slot's rows is ks_model_prefill;
-// passes that mix slots are launched as they are (their shapes hardly repeat, and a capture costs more than the launches).
+// passes that mix slots are launched as they are (run_prefill_chunk says what a capture costs).
 int ks_model_prefill_slots(ks_model* m, int n, const int* slots, const int* tokens, const int* counts) {
   if (!m) return KS_ERR_INVALID;
   ks_ctx* c = m->ctx;
@@ -1586,10 +1625,15 @@ int ks_model_debug_set(ks_model* m, int slot, int what, unsigned value) {
   if ((rc = mg.bar ? ks_mega_set(mg.bar, what, value) : ks_flow_set(mg.flow, what, value)))
     return ks_fail(c, rc, "debug_set: unknown knob %d", what);
   cudaStreamSynchronize(c->stream);
-  for (auto& kv : m->graphs) cudaGraphExecDestroy(kv.second);
-  m->graphs.clear();
-  m->graph_nodes.clear();
+  drop_graphs(m);
   return KS_OK;
+}
+
+int ks_model_debug_graphs(const ks_model* m) {
+  if (!m) return KS_ERR_INVALID;
+  size_t n = m->graphs.size();
+  for (const auto& p : m->prompt_graphs) n += p.graph.exec != nullptr;
+  return (int)n;
 }
 
 // Device address of one slot's rows of a layer's cache ([max_seq, n_kv, hd] Q4_0); which: 0 = K, 1 = V.

@@ -103,3 +103,32 @@ def test_prompts_of_several_slots_share_passes(ctx, n_kv, window):
             model.prefill_many(bad)
         assert [model.seq_len(s) for s in slots] == before
     model.close()
+
+
+def test_lengths_that_do_not_repeat_leave_no_graph(ctx):
+    """A prompt length is launched the first time, captured the second and replayed from then on, always with the same result; lengths
+    that come once leave nothing behind, and what repeated ones leave is bounded."""
+    cfg = ksm.tiny_config(max_seq=1280)
+    model, _ = ksm.GemmaCudaModel.synthetic(ctx, cfg, seed=59, keep=True)
+    model.slot_alloc()
+    toks = [int(t) for t in synth.token_ids(59, "p", 1280, cfg.vocab)]
+    held = lambda: model.lib.ks_model_debug_graphs(model.h)
+    first = {n: _logits_after(model, ctx, [toks[:n]], toks[n]) for n in (9, 130, 700, 1100)}   # (the decode step is a graph)
+    before = held()
+    for n in range(20, 220):
+        model.slot_reset(0)
+        model.prefill(0, toks[:n])
+    assert held() == before
+    for _ in range(3):
+        for n, want in first.items():
+            assert np.array_equal(_logits_after(model, ctx, [toks[:n]], toks[n]), want), n
+    assert held() == before + len(first)
+    for n in range(300, 400):
+        for _ in range(2):
+            model.slot_reset(0)
+            model.prefill(0, toks[:n])
+    assert held() == before + 64
+    for n, want in first.items():
+        assert np.array_equal(_logits_after(model, ctx, [toks[:n]], toks[n]), want), n
+    assert held() <= before + 64
+    model.close()
