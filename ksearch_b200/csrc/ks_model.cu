@@ -193,7 +193,8 @@ struct ks_model {
   std::map<int, Mega> mega;
   bool use_mega = false;
   int decode_kernel = 1;
-  // prompt chunks (ks_model_prefill): KS_PREFILL_CHUNK rows of activations of their own
+  // prompt chunks (ks_model_prefill): activations of their own; x, x2, q and o as many rows as a pass through the GEMM takes, the
+  // others KS_PREFILL_CHUNK
   void *cx = nullptr, *cxb = nullptr, *cx2 = nullptr, *cq = nullptr, *ck = nullptr, *cv = nullptr, *co = nullptr, *cff = nullptr;
   float* ctok = nullptr;
   int *cpos = nullptr, *crow_slot = nullptr;
@@ -407,7 +408,7 @@ int enqueue_forward_gemm(ks_model* m, const Lane& L_, int n, bool want_logits) {
   const ks_dtype act = KS_F32;
   const size_t H = g.hidden, F = g.ffn, hd = g.hd, nq = g.n_q, nkv = g.n_kv;
   const size_t qn = nq * hd, kvn = nkv * hd;
-  char *x = L_.x, *x2 = L_.x2, *q = L_.q, *k = L_.k, *v = L_.v, *o = L_.o, *logits = L_.logits;
+  char *x = L_.x, *x2 = L_.x2, *q = L_.q, *o = L_.o, *logits = L_.logits;
   float* tok_out = L_.tok_out;
   int rc;
   const int att_splits = att_splits_for(m, n), chunk_splits = ks_sdpa_chunk_splits(c, n, nq, nkv, (size_t)g.max_seq, m->n_splits);
@@ -951,10 +952,11 @@ ks_model* ks_model_create(ks_ctx* ctx, const ks_model_config* cfg) {
     }
     const size_t C = m->gemm_chunk > KS_PREFILL_CHUNK ? m->gemm_chunk : KS_PREFILL_CHUNK;
     const size_t cb = m->gemm_chunk ? sizeof(float) : ab;  // the batch matvec's rows fit as well
-    ok = ok && dev_alloc(m, &m->cx, C * H * cb) == KS_OK && dev_alloc(m, &m->cxb, C * H * cb) == KS_OK &&
-         dev_alloc(m, &m->cx2, C * H * cb) == KS_OK && dev_alloc(m, &m->cq, C * qn * cb) == KS_OK &&
-         dev_alloc(m, &m->ck, C * kvn * cb) == KS_OK && dev_alloc(m, &m->cv, C * kvn * cb) == KS_OK &&
-         dev_alloc(m, &m->co, C * qn * cb) == KS_OK && dev_alloc(m, &m->cff, C * F * cb) == KS_OK &&
+    constexpr size_t B = KS_PREFILL_CHUNK;                 // what only the batch matvec's passes read and write
+    ok = ok && dev_alloc(m, &m->cx, C * H * cb) == KS_OK && dev_alloc(m, &m->cx2, C * H * cb) == KS_OK &&
+         dev_alloc(m, &m->cq, C * qn * cb) == KS_OK && dev_alloc(m, &m->co, C * qn * cb) == KS_OK &&
+         dev_alloc(m, &m->cxb, B * H * ab) == KS_OK && dev_alloc(m, &m->ck, B * kvn * ab) == KS_OK &&
+         dev_alloc(m, &m->cv, B * kvn * ab) == KS_OK && dev_alloc(m, &m->cff, B * F * ab) == KS_OK &&
          dev_alloc(m, (void**)&m->ctok, C * sizeof(float)) == KS_OK && dev_alloc(m, (void**)&m->cpos, C * sizeof(int)) == KS_OK &&
          dev_alloc(m, (void**)&m->crow_slot, C * sizeof(int)) == KS_OK &&
          dev_alloc(m, (void**)&m->cmeta, C * 4 * sizeof(float)) == KS_OK &&
