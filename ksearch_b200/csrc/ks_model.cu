@@ -231,18 +231,22 @@ constexpr size_t KS_STAGE_IDS = KS_GEMM_CHUNK; // pinned words that stage host t
 
 // Do the rows of a prompt chunk share one pass over their context (ks_sdpa_chunk.cu: 128 rows x heads a block, few blocks of 25 us
 // and more), or does each take the decode kernel (a block per row and up to four heads, spread over the chip)?  By the work of the
-// second form: rows x blocks x positions a row sees on average, in units of 256 dims.  Microseconds per layer, shared / per row:
-//   tiny (4 heads, 1 KV head of 128)   256 rows at 0 (16k): 81 / 69, 512 at 0 (66k): 98 / 100, 256 at 512 (82k): 81 / 77, 320 at 512 (108k): 91 / 91
-//   E2B (8, 1 of 256)                  256 at 0 (66k): 130 / 123, 320 (102k): 140 / 141, 384 (148k): 145 / 155, 128 at 512 (148k): 107 / 97,
-//                                      192 at 512 (234k): 121 / 127, 64 at 1024 (135k): 93 / 88, 96 (206k): 104 / 108
-//   E4B (8, 2 of 256)                  256 at 0: 187 / 181, 320: 229 / 233, 384: 241 / 253, 128 at 512: 146 / 138, 192: 169 / 180, 96 at 1024: 143 / 146
-// so the line lies near 128k.  A block of one head does the work of four: with a KV head per query head (8, 8 of 128) near 48k
-// (128 rows at 0, 33k: 75 / 74, 192, 74k: 77 / 90, 32 at 512, 68k: 61 / 58, 32 at 1024, 133k: 64 / 66).
+// second form, rows x blocks x positions a row sees on average in units of 256 dims, against a line that lies the higher the fewer
+// rows there are: few rows are few blocks of the first form.  Microseconds per layer of 24, shared / per row, with the work:
+//   E2B (8 heads, 1 KV head of 256)  256 rows at 0: 132 / 123 (65k), 320: 143 / 142 (102k), 384: 154 / 156 (147k); 128 at 512: 105 / 98 (147k),
+//                                    160: 122 / 125 (189k); 96 at 1024: 109 / 110 (205k); 48 at 2048: 101 / 101 (198k), 64: 114 / 104 (266k);
+//                                    window 128, 256 rows: 131 / 121 (65k), 512: 175 / 185 (131k), 768: 214 / 242 (196k)
+//   E4B (8, 2 of 256)                256 at 0: 198 / 188, 320: 232 / 234, 384: 241 / 253; 128 at 512: 145 / 139, 160: 167 / 180; 96 at 1024:
+//                                    143 / 148; 64 at 2048: 138 / 125; window 512 at 1024: 128 rows 144 / 135 (131k), 256: 196 / 208 (262k)
+//   tiny (4, 1 of 128)               384 at 0: 72 / 68 (37k), 192 at 512: 66 / 59 (58k), 128 at 1024: 70 / 64 (70k)
+// A block of one head does the work of four, so with a KV head per query head (8, 8 of 128) the line lies lower: 128 at 0: 67 / 65
+// (33k), 192: 66 / 80 (74k); 24 at 2048: 60 / 78 (197k); 16 at 3500: 71 / 72 (225k); 32 at 512: 61 / 58 (68k).
 bool rows_share_context(const ks_model_config& g, int n, int base, int window) {
   const int hpk = g.n_q / g.n_kv, gb = hpk % 4 == 0 ? 4 : hpk % 2 == 0 ? 2 : 1;
   double seen = base + 0.5 * (n + 1);
   if (window > 0 && seen > window) seen = window;
-  return n >= 4 && (double)n * (g.n_q / gb) * seen * g.hd >= 256.0 * (gb == 1 ? 49152.0 : 131072.0);
+  const double work = (double)n * (g.n_q / gb) * seen * g.hd / 256.0;
+  return n >= 4 && work >= (gb == 1 ? 45e3 + 1e6 / n : 75e3 + 13e6 / n);
 }
 
 // Where a forward pass reads and writes: n rows of activations, their positions, and the KV caches
@@ -1349,6 +1353,10 @@ int ks_model_prefill(ks_model* m, int slot, const int* tokens, int n_tokens) {
 // Prompt tokens of several slots (counts[i] of them for slots[i], behind one another in `tokens`): their rows share passes over the
 // weights, up to KS_GEMM_CHUNK a pass.  Everything is checked before anything runs.  A pass of one slot's rows is ks_model_prefill;
 // passes that mix slots are launched as they are (run_prefill_chunk says what a capture costs).
+// A pass that mixes slots shares contexts whatever its pieces: the decode kernel takes rows of one cache or of one cache each.  Short
+// pieces would do better row by row, but one by one they read the weights again.  Microseconds per layer, mixed / one by one / as many
+// rows of one slot that see as much, row by row: E2B 3 x 5 rows at 0: 76 / 174 / 61, 8 x 16: 106 / 487 / 82, 8 x 40: 152 / 568 / 133,
+// 8 x 128: 275 / 658 / 310, 4 x 64 at 512: 133 / 322 / 147; E4B 8 x 16: 142 / 618 / 121, 8 x 128: 493 / 973 / 527.
 int ks_model_prefill_slots(ks_model* m, int n, const int* slots, const int* tokens, const int* counts) {
   if (!m) return KS_ERR_INVALID;
   ks_ctx* c = m->ctx;
