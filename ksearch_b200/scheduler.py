@@ -185,8 +185,24 @@ class Scheduler:
             return
         decoding = any(not a.finished and a.last_token is not None for a in self.active)
         budget = max(self.cfg.prefill_tokens_per_tick, self.cfg.prefill_chunk)
-        idx = self._prefill_next % n
-        together = [] if hasattr(self.model, "prefill_many") else None
+        start = self._prefill_next % n
+        if hasattr(self.model, "prefill_many"):
+            parts = []
+
+            def later(a, take):
+                parts.append((a, take))
+                return True
+
+            self._prefill_next = self._hand_out(start, budget, decoding, later)
+            if not parts or self._prefill_together(parts):
+                return
+        # (also where the shared call was refused: an error meets the request it belongs to and leaves its tokens to those behind)
+        self._prefill_next = self._hand_out(start, budget, decoding, self._prefill_one)
+
+    def _hand_out(self, idx: int, budget: int, decoding: bool, run) -> int:
+        """Deals the round's budget to the requests from idx on; `run` takes a piece and says whether it counts.  Where the next
+        round starts."""
+        n = len(self.active)
         for _ in range(n):
             if budget == 0:
                 break
@@ -200,14 +216,9 @@ class Scheduler:
                 continue
             cap = self.cfg.prefill_chunk if decoding else budget
             take = min(budget, cap, end - a.cursor)
-            if together is not None:
-                together.append((a, take))
+            if run(a, take):
                 budget -= take
-            elif self._prefill_one(a, take):
-                budget -= take
-        self._prefill_next = idx
-        if together:
-            self._prefill_together(together)
+        return idx
 
     def _prefill_one(self, a: _Active, take: int) -> bool:
         try:
@@ -224,22 +235,25 @@ class Scheduler:
         if a.cursor >= len(a.req.prompt_ids) - 1:
             a.last_token = int(a.req.prompt_ids[-1])
 
-    def _prefill_together(self, parts):
-        """The round's prompt pieces in shared passes over the weights; one by one where that is refused, so that an
-        error meets the request it belongs to."""
-        if len(parts) > 1:
-            before = [self.model.seq_len(a.slot) for a, _ in parts]
-            try:
-                self.model.prefill_many([(a.slot, a.req.prompt_ids[a.cursor:a.cursor + take]) for a, take in parts])
-            except Exception as e:
-                if [self.model.seq_len(a.slot) for a, _ in parts] != before:
-                    for a, _ in parts:
-                        a.req.emit("error", str(e))
-                        self._finish(a, "error")
-                    return
-            else:
-                for a, take in parts:
+    def _prefill_together(self, parts) -> bool:
+        """The round's prompt pieces in shared passes over the weights; False if they are refused and none has run.  Where a call
+        fails half way, what ran counts, the request it failed in ends, and the others keep their place in the next round."""
+        if len(parts) == 1:
+            return False
+        before = [self.model.seq_len(a.slot) for a, _ in parts]
+        try:
+            self.model.prefill_many([(a.slot, a.req.prompt_ids[a.cursor:a.cursor + take]) for a, take in parts])
+        except Exception as e:
+            went = [self.model.seq_len(a.slot) - was for (a, _), was in zip(parts, before)]
+            if not any(went):
+                return False
+            for (a, take), n in zip(parts, went):
+                if n == take:
                     self._advance(a, take)
-                return
-        for a, take in parts:
-            self._prefill_one(a, take)
+                elif n:
+                    a.req.emit("error", str(e))
+                    self._finish(a, "error")
+        else:
+            for a, take in parts:
+                self._advance(a, take)
+        return True

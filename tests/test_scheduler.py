@@ -37,6 +37,7 @@ class FakeModel:
         return self.len[s]
 
     def prefill(self, s, toks):
+        assert all(t < self.cfg.vocab for t in toks), "refused"
         assert s in self.used and self.len[s] + len(toks) <= self.cfg.max_seq
         self.prefills.append((s, len(toks)))
         self.len[s] += len(toks)
@@ -50,6 +51,31 @@ class FakeModel:
             out.append(self.rule(t, self.len[s]))
             self.len[s] += 1
         return out
+
+
+class SharedModel(FakeModel):
+    """The same with the prompt pieces of several slots in one call, as GemmaCudaModel has it: all of them are looked at before any
+    runs; `stop_after` pieces of a call, the device fails."""
+
+    stop_after = None
+
+    def prefill_many(self, parts):
+        self.calls = getattr(self, "calls", 0) + 1
+        for s, toks in parts:
+            if self.len[s] + len(toks) > self.cfg.max_seq or any(t >= self.cfg.vocab for t in toks):
+                raise ValueError("refused")
+        for i, (s, toks) in enumerate(parts):
+            if i == self.stop_after:
+                self.len[s] += len(toks) // 2
+                raise RuntimeError("device said no")
+            self.prefill(s, toks)
+
+
+@pytest.fixture(autouse=True, params=["one by one", "together"])
+def both_ways(request, monkeypatch):
+    if request.param == "together":
+        monkeypatch.setitem(globals(), "FakeModel", SharedModel)
+    return request.param
 
 
 def _tokens(req):
@@ -231,3 +257,38 @@ def test_sampled_requests_read_logits_and_use_the_reference_sampler():
         m3.forward(1, 1, [tok], True)
         tok = int(np.argmax(30.0 * np.tanh(m3.read_debug(1, 1) / 30.0)))
         assert got[step] == tok
+
+
+def test_a_refused_prompt_piece_costs_the_others_nothing(both_ways):
+    """One request of a round is refused: it alone ends, and its share of the round's budget goes to those behind it."""
+    m = FakeModel(n_slots=4, max_seq=64)
+    s = Scheduler(m, SchedulerConfig(slots=4, prefill_chunk=4, prefill_tokens_per_tick=40))
+    bad = InferenceRequest([5000] * 21, max_tokens=2)
+    good = [InferenceRequest(list(range(300, 300 + n)), max_tokens=2) for n in (11, 21, 16)]
+    for r in (good[0], bad, good[1], good[2]):
+        s.submit(r)
+    s.tick()
+    assert m.prefills == [(0, 10), (2, 20), (3, 10)] and [a.req for a in s.active] == [good[0], good[1], good[2]]
+    s.run(100)
+    assert [e[0] for e in bad.events] == ["error"] and all(_done(r) == ("length", len(r.prompt_ids), 2) for r in good) and m.used == set()
+
+
+@pytest.mark.parametrize("stop_after", [0, 1, 2])
+def test_a_call_that_fails_half_way(stop_after):
+    """The device fails inside a shared call: pieces that ran count, the one it failed in ends its request, the others go on."""
+    m = SharedModel(n_slots=3)
+    m.stop_after = stop_after
+    s = Scheduler(m, SchedulerConfig(slots=3, prefill_chunk=4, prefill_tokens_per_tick=100))
+    reqs = [InferenceRequest(list(range(300, 300 + n)), max_tokens=2) for n in (9, 7, 12)]
+    for r in reqs:
+        s.submit(r)
+    s.tick()
+    m.stop_after = None
+    s.run(100)
+    assert m.calls >= 1 and m.used == set()
+    for i, r in enumerate(reqs):
+        if i == stop_after:
+            assert r.events == [("error", "device said no")]
+        else:
+            assert _done(r) == ("length", len(r.prompt_ids), 2)
+            assert _tokens(r)[0] == m.rule(r.prompt_ids[-1], len(r.prompt_ids) - 1)
