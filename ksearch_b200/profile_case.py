@@ -6,6 +6,7 @@ profiler captures are taken on.
     python -m ksearch_b200.profile_case matvec --dtype q4k --rows 20480 --cols 2560 --copies 6 --iters 2 --batch 128
     python -m ksearch_b200.profile_case decode --layers 4 --tokens 4
     python -m ksearch_b200.profile_case attn --kv 1 --ctx 16384 --slots 4 --copies 8 --iters 2
+    python -m ksearch_b200.profile_case chunk --rows 2047 --ctx 0 --kv 1 --splits 2 --iters 4
 
 `--copies` distinct weight copies are cycled so that a launch never finds its weights in L2
 (copies * matrix bytes should exceed the 126 MB L2).  Prints the CUDA-event time per launch.
@@ -22,7 +23,7 @@ from . import model as ksm
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("op", choices=["matvec", "gate_up", "decode", "attn"])
+    ap.add_argument("op", choices=["matvec", "gate_up", "decode", "attn", "chunk"])
     ap.add_argument("--dtype", default="q4k", choices=["q4k", "q6k"])
     ap.add_argument("--rows", type=int, default=4096)
     ap.add_argument("--cols", type=int, default=4096)
@@ -31,8 +32,9 @@ def main():
     ap.add_argument("--layers", type=int, default=4)
     ap.add_argument("--tokens", type=int, default=4)
     ap.add_argument("--pdl", type=int, default=0)
-    ap.add_argument("--kv", type=int, default=1, help="attn: KV heads (8 query heads)")
-    ap.add_argument("--ctx", type=int, default=16384, help="attn: positions per slot")
+    ap.add_argument("--kv", type=int, default=1, help="attn, chunk: KV heads (8 query heads)")
+    ap.add_argument("--ctx", type=int, default=16384, help="attn: positions per slot; chunk: positions in front of its rows")
+    ap.add_argument("--splits", type=int, default=1, help="chunk: context splits")
     ap.add_argument("--slots", type=int, default=4, help="attn: slots")
     ap.add_argument("--batch", type=int, default=1, help="token rows per matvec call (more than 8: the tensor-core GEMM)")
     args = ap.parse_args()
@@ -51,6 +53,28 @@ def main():
             m.forward(0, 1, None, True)
         ms = ctx.timer_end_ms()
         print(f"decode: {ms / args.tokens * 1e3:.1f} us/token over {args.tokens} tokens ({args.layers} layers, vocab {cfg.vocab})")
+        return
+    if args.op == "chunk":
+        n_q, hd = 8, 256
+        top = args.ctx + args.rows
+        bK, bV = (ctx.buffer_bytes(synth.q40_rows(1, k, top * args.kv * hd, sigma=0.05)) for k in "KV")
+        q = ctx.buffer_bytes(synth.normals(1, "q", args.rows * n_q * hd))
+        meta = np.zeros((args.rows, 4), np.float32)
+        meta[:, 0] = np.arange(args.ctx + 1, top + 1)
+        bmeta = ctx.buffer_bytes(meta)
+        tmp = ctx.buffer_empty_f32(args.rows * n_q * args.splits * (hd + 2))
+        row0, slot = np.array([0, args.rows], np.int32), np.zeros(1, np.int32)
+
+        def chunk():
+            ctx.check(ctx.lib.ks_debug_sdpa_chunk(ctx.h, n_q, args.kv, hd, top, 1.0 / 16.0, 1, row0.ctypes.data, slot.ctypes.data, 0,
+                                                  q.h, bK.h, bV.h, bmeta.h, tmp.h, args.splits))
+        chunk()
+        ctx.synchronize()
+        ctx.timer_begin()
+        for _ in range(args.iters):
+            chunk()
+        us = ctx.timer_end_ms() / args.iters * 1e3
+        print(f"chunk: {args.rows} rows behind {args.ctx} positions, {args.kv} KV heads, {args.splits} splits: {us:.1f} us/launch")
         return
     if args.op == "attn":
         from .eng import write_meta

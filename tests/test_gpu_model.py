@@ -242,8 +242,7 @@ def test_device_wait_gives_up_and_recovers(oracle, monkeypatch, decode_kernel):
 @pytest.mark.parametrize("decode_kernel", ["1", "2", "0"])
 def test_e4b_like_shapes(oracle, monkeypatch, decode_kernel):
     """Two layers with the E4B row and column counts (hidden 2560, GeGLU 10240, 8 q / 2 kv heads of
-    256): ten blocks per row, gate and up rows too long for one ring slot, four 4-element chunks per
-    thread in the fused norms, two KV heads.  Both the persistent kernel and the launch-per-op path."""
+    256): ten blocks per row, two 4-element chunks per thread in the fused norms, two KV heads.  Both the persistent kernel and the launch-per-op path."""
     from ksearch_b200 import CudaContext
     monkeypatch.setenv("KSEARCH_DECODE_KERNEL", decode_kernel)
     c = CudaContext(0, flags=1)
@@ -366,7 +365,7 @@ def test_logits_tight_when_kv_bytes_agree(oracle, monkeypatch, shape, decode_ker
 def test_prefill_chunks_match_token_by_token(ctx, oracle, monkeypatch, n_kv, batch_rows):
     """ks_model_prefill: prompt rows share a pass over the weights and attend causally inside a chunk: up to 2
     rows through the batch matvec (up to 8 with KSEARCH_BATCH_ROWS=8, the limit before the GEMM path proved faster
-    from 3 rows on), longer prompts in chunks of up to 256 rows through the tensor-core GEMM.
+    from 3 rows on), longer prompts in chunks of up to 2048 rows (here: as many as the cache holds) through the tensor-core GEMM.
     After the prompt, the next-token logits must match the CPU decoder, and the KV rows it wrote must
     serve later decode steps (teacher-forced continuation)."""
     if batch_rows is None:
@@ -377,7 +376,7 @@ def test_prefill_chunks_match_token_by_token(ctx, oracle, monkeypatch, n_kv, bat
     model, T = ksm.GemmaCudaModel.synthetic(ctx, cfg, seed=31, keep=True)
     cpu = oracle.CpuDecoder(oracle.decoder_cfg(cfg), T)
     model.slot_alloc()
-    # batch matvec; GEMM chunks of 16..256 rows (up to 128: hi|lo rows in one MMA); full chunks + ragged rest
+    # batch matvec; GEMM chunks of one and of several blocks of token rows, whole and ragged
     for n_prompt in (1, 2, 3, 7, 8, 9, 21, 128, 150, 137, 256, 300, 530):
         toks = synth.token_ids(31, f"p{n_prompt}", n_prompt + 6, cfg.vocab)
         model.slot_reset(0)

@@ -2,7 +2,7 @@
 import numpy as np
 import pytest
 
-from ksearch_b200 import synth
+from ksearch_b200 import F16, F32, synth
 from ksearch_b200 import model as ksm
 
 pytestmark = pytest.mark.gpu
@@ -41,7 +41,8 @@ def test_long_chunks_equal_short_pieces(ctx, n_kv, window):
 @pytest.mark.parametrize("n_q,n_kv,hd", [(8, 1, 256), (8, 2, 256), (4, 4, 256), (16, 1, 128), (8, 4, 128)])
 def test_chunk_attention_equals_row_attention(monkeypatch, n_q, n_kv, hd):
     """Prompt rows that share their context (tiles of 128 query rows x 64 positions) against a model whose prompts go row by row
-    through the decode attention: one tile and less, its edges, several tiles behind a context, windowed layers."""
+    through the decode attention: one tile and less, its edges, several tiles behind a context, windowed layers.  A pass that mixes
+    slots always shares, so the piece brings a few rows of a second slot along."""
     from ksearch_b200 import CudaContext
     out = []
     for no_gemm in (False, True):
@@ -49,15 +50,22 @@ def test_chunk_attention_equals_row_attention(monkeypatch, n_q, n_kv, hd):
             monkeypatch.setenv("KSEARCH_NO_GEMM", "1")
         else:
             monkeypatch.delenv("KSEARCH_NO_GEMM", raising=False)
-        cfg = ksm.tiny_config(max_seq=768, n_kv=n_kv)
+        cfg = ksm.tiny_config(max_seq=768, n_slots=2, n_kv=n_kv)
         cfg.n_q, cfg.hd, cfg.n_layers = n_q, hd, 2
         cfg.sliding_window, cfg.swa_layers = 70, 0b10
         c = CudaContext(0, flags=1)
         model, _ = ksm.GemmaCudaModel.synthetic(c, cfg, seed=47, keep=True)
-        model.slot_alloc()
+        slots = [model.slot_alloc(), model.slot_alloc()]
         toks = [int(t) for t in synth.token_ids(47, "p", 700, cfg.vocab)]
-        for first, n in ((0, 63), (0, 64), (0, 129), (0, 333), (65, 128), (300, 257), (600, 90)):
-            out.append(_logits_after(model, c, ([toks[:first]] if first else []) + [toks[first:first + n]], toks[first + n]))
+        for first, n in ((0, 1), (0, 63), (0, 64), (0, 129), (0, 333), (65, 128), (300, 257), (600, 90)):
+            for s in slots:
+                model.slot_reset(s)
+            if first:
+                model.prefill(0, toks[:first])
+            model.prefill_many([(0, toks[first:first + n]), (1, toks[:5])])
+            model.forward(0, 2, [toks[first + n], toks[5]], True)
+            c.synchronize()
+            out.append(np.concatenate([model.read_debug(1, s).astype(np.float64) for s in slots]))
         model.close()
         c.close()
     half = len(out) // 2
@@ -131,4 +139,42 @@ def test_lengths_that_do_not_repeat_leave_no_graph(ctx):
     for n, want in first.items():
         assert np.array_equal(_logits_after(model, ctx, [toks[:n]], toks[n]), want), n
     assert held() <= before + 64
+    model.close()
+
+
+@pytest.mark.parametrize("n_slots,n_kv,hd,act,window", [(4, 2, 256, F32, 60), (4, 1, 256, F16, 0), (4, 2, 128, F16, 40), (12, 1, 128, F32, 50), (64, 1, 128, F32, 0)])
+def test_mixed_passes_of_other_models(ctx, n_slots, n_kv, hd, act, window):
+    """prefill_many against one prefill call per slot: head size 256, f16 activations, up to as many slots as a model has.  In f16 both
+    sides run the prompt in f32; the step behind it rounds to f16 (2^-11 an op, ten ops a layer, three layers)."""
+    cfg = ksm.tiny_config(max_seq=256, n_slots=n_slots, n_kv=n_kv, act=act)
+    cfg.hd = hd
+    if act == F16:
+        cfg.sigma_w = 3e-5   # random weights of one sign: larger ones leave the f16 range in the FFN
+    if window:
+        cfg.sliding_window, cfg.swa_layers = window, 0b101
+    model, _ = ksm.GemmaCudaModel.synthetic(ctx, cfg, seed=61, keep=True)
+    slots = [model.slot_alloc() for _ in range(n_slots)]
+    toks = [[int(t) for t in synth.token_ids(61, f"s{s}", 256, cfg.vocab)] for s in slots]
+    rounds = [[(7 * s) % 61 + 1 for s in slots], [(11 * s) % 19 for s in slots]]
+    sides = []
+    for together in (True, False):
+        at = [0] * n_slots
+        for s in slots:
+            model.slot_reset(s)
+        for counts in rounds:
+            parts = [(s, toks[s][at[s]:at[s] + counts[s]]) for s in reversed(slots)]
+            if together:
+                model.prefill_many(parts)
+            else:
+                for s, p in parts:
+                    model.prefill(s, p)
+            at = [a + c for a, c in zip(at, counts)]
+        model.forward(0, n_slots, [toks[s][at[s]] for s in slots], True)
+        ctx.synchronize()
+        sides.append([model.read_debug(1, s).astype(np.float64) for s in slots])
+    worst, mean = (1e-3, 1e-4) if act == F32 else (30 * 2.0 ** -11, 30 ** 0.5 * 2.0 ** -11)
+    for got, want in zip(*sides):
+        scale, err = np.abs(want).max(), np.abs(got - want)
+        assert 0 < scale < np.inf
+        assert err.max() <= worst * scale and np.sqrt((err ** 2).mean()) <= mean * scale
     model.close()
