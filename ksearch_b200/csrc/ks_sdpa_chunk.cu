@@ -27,7 +27,7 @@ constexpr int CH_BM = 128, CH_BN = 64;                 // query rows, positions 
 constexpr int CH_ROW_WARPS = 4, CH_DEC_WARPS = 8, CH_WORK = (CH_ROW_WARPS + CH_DEC_WARPS) * 32, CH_THREADS = CH_WORK + 128;
 constexpr unsigned CH_WAIT = 1u << 20;
 constexpr float CH_P = 256.0f;                         // probabilities carry 2^8
-constexpr float CH_K_MOST = 8188.0f;                   // the largest scale with 8 d in f16
+constexpr unsigned CH_K_MOST = 0x6FFFu;                // the largest scale with 8 d in f16, 8188
 constexpr float kNegInit = -1.0e30f;
 
 // barriers: operands ready (decoders, row warps), the tile's O taken (decoders), products ready (commits: scores done = K free;
@@ -132,6 +132,21 @@ sdpa_chunk_kernel(const __grid_constant__ ChunkParts parts, size_t slot_stride, 
       for (unsigned w = lane; w < ROWB / 4u; w += 32u) cp4(dst + 4u * w, src + 4u * w);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // The largest scale (its f16 bits) of the K rows this thread copied.  Block b's scale is half of word 18 b / 4, and those words are
+  // all among a lane's first.
+  static_assert((NB - 1u) * KS_Q40_BLOCK_BYTES < 128u, "scales lie in the first 32 words of a row");
+  const unsigned scale_at = (lane * 4u + KS_Q40_BLOCK_BYTES - 1u) / KS_Q40_BLOCK_BYTES * KS_Q40_BLOCK_BYTES;
+  const bool has_scale = scale_at < lane * 4u + 4u && scale_at < ROWB;
+  const unsigned scale_off = S::raw + ((warp - CH_ROW_WARPS) & (CH_DEC_WARPS - 1u)) * RP + (has_scale ? scale_at : lane * 4u);
+  auto most_scale = [&] {
+    unsigned m = 0;
+#pragma unroll
+    for (unsigned k = 0; k < CH_BN / CH_DEC_WARPS; k++) {
+      const unsigned d = *reinterpret_cast<const unsigned short*>(smem + scale_off + k * CH_DEC_WARPS * RP) & 0x7FFFu;
+      m = d > m ? d : m;
+    }
+    return has_scale ? m : 0u;
   };
   if (decoder) fetch(t_begin);
 
@@ -295,43 +310,41 @@ sdpa_chunk_kernel(const __grid_constant__ ChunkParts parts, size_t slot_stride, 
     bool ok = true;
     for (unsigned i = 0; i < n_tiles; i++) {
       asm volatile("cp.async.wait_all;" ::: "memory");
+      const bool fits = most_scale() <= CH_K_MOST;
       if (i > 0) ok = mb_wait(bar(CB_K_FREE), (i - 1u) & 1u, CH_WAIT);
-      if (!dec_all(ok)) { ok = false; break; }  // the raw rows are there, K is free
-      // A tile with a scale whose products leave f16 is decoded again at an eighth and its scores multiplied by 8; what that rounds
-      // off (2^-22 of a value at most) is nothing beside a value of 57000.
+      // The raw rows are there, K is free.  A tile with a scale whose products leave f16 is decoded at an eighth and its scores are
+      // multiplied by 8; what that rounds off (2^-22 of a value at most) is nothing beside a value of 57000.  Every thread looks at
+      // the scales that it copied itself.
       float tile = 1.0f;
-      for (;;) {
-        const __half down = __float2half_rn(1.0f / tile);
-        bool fits = true;
-#pragma unroll 1
-        for (unsigned job = dt; job < CH_BN * NB; job += CH_DEC_WARPS * 32) {  // a block of a row
-          const unsigned p = job % CH_BN, b = job / CH_BN;
-          const unsigned char* src = smem + S::raw + p * RP + b * KS_Q40_BLOCK_BYTES;
-          const __half raw_d = __ushort_as_half(*reinterpret_cast<const unsigned short*>(src));
-          fits = fits && !(__habs(raw_d) > __float2half_rn(CH_K_MOST));
-          const __half2 d = __half2half2(__hmul(raw_d, down));
-          uint32_t w[4];
-#pragma unroll
-          for (int k = 0; k < 4; k++)
-            w[k] = *reinterpret_cast<const unsigned short*>(src + 2 + 4 * k) | (uint32_t)*reinterpret_cast<const unsigned short*>(src + 4 + 4 * k) << 16;
-#pragma unroll 1
-          for (int half = 0; half < 2; half++)  // dims 0..15 of the block are the low nibbles
-#pragma unroll
-            for (int c = 0; c < 2; c++) {
-              uint32_t hi[4], lo[4];
-#pragma unroll
-              for (int k = 0; k < 2; k++) {
-                const uint32_t x = half ? w[2 * c + k] >> 4 : w[2 * c + k];
-                split_d(nib_h2(__byte_perm(x, 0u, 0x4140)), d, hi[2 * k], lo[2 * k]);
-                split_d(nib_h2(__byte_perm(x, 0u, 0x4342)), d, hi[2 * k + 1], lo[2 * k + 1]);
-              }
-              const unsigned at = ((4u * b + 2u * half + c) * CH_BN + p) * 16u;
-              *reinterpret_cast<uint4*>(smem + S::kh + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-              *reinterpret_cast<uint4*>(smem + S::kl + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-            }
-        }
-        if (tile != 1.0f || dec_all(fits)) break;
+      if (!dec_all(ok && fits)) {
+        if (!dec_all(ok)) { ok = false; break; }
         tile = 8.0f;
+      }
+      const __half2 down = __float2half2_rn(1.0f / tile);
+#pragma unroll 1
+      for (unsigned job = dt; job < CH_BN * NB; job += CH_DEC_WARPS * 32) {  // a block of a row
+        const unsigned p = job % CH_BN, b = job / CH_BN;
+        const unsigned char* src = smem + S::raw + p * RP + b * KS_Q40_BLOCK_BYTES;
+        const __half2 d = __hmul2(__half2half2(__ushort_as_half(*reinterpret_cast<const unsigned short*>(src))), down);
+        uint32_t w[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          w[k] = *reinterpret_cast<const unsigned short*>(src + 2 + 4 * k) | (uint32_t)*reinterpret_cast<const unsigned short*>(src + 4 + 4 * k) << 16;
+#pragma unroll 1
+        for (int half = 0; half < 2; half++)  // dims 0..15 of the block are the low nibbles
+#pragma unroll
+          for (int c = 0; c < 2; c++) {
+            uint32_t hi[4], lo[4];
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+              const uint32_t x = half ? w[2 * c + k] >> 4 : w[2 * c + k];
+              split_d(nib_h2(__byte_perm(x, 0u, 0x4140)), d, hi[2 * k], lo[2 * k]);
+              split_d(nib_h2(__byte_perm(x, 0u, 0x4342)), d, hi[2 * k + 1], lo[2 * k + 1]);
+            }
+            const unsigned at = ((4u * b + 2u * half + c) * CH_BN + p) * 16u;
+            *reinterpret_cast<uint4*>(smem + S::kh + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            *reinterpret_cast<uint4*>(smem + S::kl + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          }
       }
       if (dt == 0) tile_up[i & 1u] = tile;
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
