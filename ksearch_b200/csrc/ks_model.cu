@@ -742,9 +742,9 @@ int run_forward(ks_model* m, int first, int n, int src, bool want_logits) {
 
 // Prompt passes through the GEMM hardly repeat their row counts, and a capture (1.2 to 2 ms of host time, now and then 10 to 25) costs
 // more than the launches (0.7 to 1.4 ms, behind which the GPU works).  So a pass is launched as it is; one that comes again among the
-// last KS_PROMPT_GRAPHS different ones gets a graph, which saves 0.1 to 0.2 ms of every later pass.  E2B, captured at once / launched /
-// replayed: 20 rows 3.3 / 2.16 / 2.04 ms, 300 rows 6.0 / 4.84 / 4.71, 600 rows 8.7 / 7.31 / 7.22, 2047 rows 20.6 / 19.5 / 19.3; E4B 300
-// rows 11.1 / 9.6 / 9.3.
+// last KS_PROMPT_GRAPHS different ones is captured behind its launches, while the GPU works on them, and replayed from then on, which
+// saves 0.1 to 0.2 ms a pass.  E2B, captured at once / launched / replayed: 20 rows 3.3 / 2.16 / 2.04 ms, 300 rows 6.0 / 4.84 / 4.71,
+// 600 rows 8.7 / 7.31 / 7.22, 2047 rows 20.6 / 19.5 / 19.3; E4B 300 rows 11.1 / 9.6 / 9.3.
 constexpr size_t KS_PROMPT_GRAPHS = 64;
 
 // A chunk of n prompt tokens of one slot (ids already in m->ctok) through every layer, no head.  The stream is idle but for the ids'
@@ -783,12 +783,12 @@ int run_prefill_chunk(ks_model* m, int slot, int n, bool gemm) {
     at->key = key;
   }
   at->last = ++m->prompt_passes;
-  if (!again) return enqueue_forward_gemm(m, lane, n, false);
-  if (!at->graph.exec) {
-    const int rc = capture(c, [&] { return enqueue_forward_gemm(m, lane, n, false); }, &at->graph);
-    if (rc) return rc;
-  }
-  return replay(c, at->graph);
+  if (at->graph.exec) return replay(c, at->graph);
+  const int rc = enqueue_forward_gemm(m, lane, n, false);
+  if (rc || !again) return rc;
+  // (a pass that cannot be captured is launched each time)
+  if (capture(c, [&] { return enqueue_forward_gemm(m, lane, n, false); }, &at->graph) || cudaGraphUpload(at->graph.exec, c->stream) != cudaSuccess) (void)cudaGetLastError();
+  return KS_OK;
 }
 
 }  // namespace
