@@ -373,7 +373,7 @@ __device__ __forceinline__ void mg_item_compute_fx(uint32_t slot_addr, unsigned 
 
 
 // ---- staging of x (with the fused norm prologues), reads through L2 ---------------------------
-constexpr int MG_XMAX = 4;  // plain staging keeps up to 4 chunks per thread in flight (8192 columns), loops beyond
+constexpr int MG_XMAX = 4;  // plain staging keeps up to 4 chunks per thread in flight (7680 columns), loops beyond
 // x' = x
 __device__ __forceinline__ void mg_stage_plain(unsigned char* xs, unsigned cols, const float* x) {
   const unsigned tid = mg_tid();
@@ -510,9 +510,8 @@ __host__ __device__ __forceinline__ unsigned job_bytes(const MegaShape& sh, bool
 struct MegaRing {
   unsigned bytes, at, used;
   __host__ __device__ unsigned takes(unsigned room) const { return at + room > bytes ? bytes - at + room : room; }
-  __host__ __device__ bool fits(unsigned room) const { return used + takes(room) <= bytes; }
-  __host__ __device__ unsigned put(unsigned room, unsigned& taken) {
-    taken = takes(room);
+  __host__ __device__ bool fits(unsigned taken) const { return used + taken <= bytes; }
+  __host__ __device__ unsigned put(unsigned room, unsigned taken) {
     const unsigned place = at + room > bytes ? 0u : at;
     at = place + room;
     used += taken;
@@ -993,7 +992,8 @@ __device__ __forceinline__ void mg_copy_jobs(const MegaArgs& a, const MegaShape*
         if (sh.n_seg > 2 && g >= sh.grp_start[2]) seg = 2;
         const unsigned row0 = (g - sh.grp_start[seg]) * MG_RL, valid = min((unsigned)MG_RL, sh.rows[seg] - row0);
         const unsigned room = job_bytes(sh, norm, H);
-        while (head - tail >= MG_JOBS || !ring.fits(room)) {
+        unsigned taken = ring.takes(room);
+        while (head - tail >= MG_JOBS || !ring.fits(taken)) {
           const uint32_t bar = empty + (tail & (MG_JOBS - 1u)) * 8u;
           const unsigned parity = (tail / MG_JOBS) & 1u;
           bool ok = false;
@@ -1014,10 +1014,9 @@ __device__ __forceinline__ void mg_copy_jobs(const MegaArgs& a, const MegaShape*
           }
           ring.drop(jbytes[tail & (MG_JOBS - 1u)]);
           tail++;
+          if (ring.used == 0) taken = room;
         }
-        const unsigned b = head & (MG_JOBS - 1u);
-        unsigned taken;
-        const unsigned at = ring.put(room, taken);
+        const unsigned b = head & (MG_JOBS - 1u), at = ring.put(room, taken);
         joff[b] = at;
         jbytes[b] = taken;
         mb_expect(full + b * 8u, norm ? room : mats * valid * row_bytes);  // (its arrival publishes joff)
@@ -1430,8 +1429,13 @@ extern "C" int ks_debug_decode_ring(int hidden, int ffn, int n_q, int n_kv, int 
       const unsigned norms = norm_jobs(kind), n = block_groups(p.sh[kind], (unsigned)block, p.grid) + norms;
       for (unsigned k = 0; k < n; k++, head++) {
         const unsigned room = job_bytes(p.sh[kind], k < norms, d.hidden);
-        for (; head - tail >= MG_JOBS || !ring.fits(room); tail++) ring.drop(taken[tail & (MG_JOBS - 1u)]);
-        const unsigned at = ring.put(room, taken[head & (MG_JOBS - 1u)]);
+        unsigned t = ring.takes(room);
+        for (; head - tail >= MG_JOBS || !ring.fits(t); tail++) {
+          ring.drop(taken[tail & (MG_JOBS - 1u)]);
+          if (ring.used == 0) t = room;
+        }
+        const unsigned at = ring.put(room, t);
+        taken[head & (MG_JOBS - 1u)] = t;
         if (out && head < (unsigned)max_jobs) {
           out[3 * head] = at;
           out[3 * head + 1] = room;
