@@ -594,9 +594,11 @@ __host__ __device__ constexpr unsigned mg_rec(unsigned hd) { return hd + 4u; }  
 constexpr int MG_MAX_SPLITS = 18;  // context splits per head (the final merge keeps one record per split in registers)
 constexpr int MG_FLY = 4;  // positions of a warp in flight
 // Up to MG_DIRECT splits are merged by every block while it stages the o-projection's input (mg_stage_merge): no block waits for
-// another one's merge, and a block reads at most n_q x 4 records (2.0 us of staging instead of 0.8).  A token of the E2B shape at
-// 64..128 positions: one split 1017 us, two 1003, four 998; with a window of 512: 1203, 1188, 1096.
-constexpr unsigned MG_DIRECT = 4, MG_SINGLE_TLEN = MG_FLY * MG_WARPS, MG_DIRECT_TLEN = 1024;
+// another one's merge, and a block reads at most n_q x 4 records (2.0 us of staging instead of 0.8).  From the second batch of
+// positions per warp on (4 x 60) the eighteen win.  A token at 200 / 300 / 500 / 1000 / 2000 positions, four splits: E2B 943 / 984 / 1024 /
+// 1131 / 1334 us, E4B 1516 / 1565 / 1612 / 1738 / 2020; all eighteen: 984 / 990 / 993 / 1001 / 1055 and 1562 / 1568 / 1572 / 1581 / 1679 (eight,
+// merged while staging: 964 / 967 / 994 / 1051 / 1156 and 1543 / 1546 / 1578 / 1645 / 1775).  E2B at 64..128: one split 1017, two 1003, four 998.
+constexpr unsigned MG_DIRECT = 4, MG_SINGLE_TLEN = MG_FLY * MG_WARPS, MG_DIRECT_TLEN = 320;
 
 // Shared memory the attention phase needs (it reuses the x staging area).
 __host__ __device__ inline unsigned mg_att_bytes(unsigned hd) {

@@ -38,7 +38,7 @@ def test_attention_forms_and_widths(monkeypatch, hidden, n_q, n_kv, hd, window):
     if window:
         cfg.sliding_window, cfg.swa_layers = window, 0b01
     toks = [int(t) for t in synth.token_ids(43, "p", 1210, cfg.vocab)]
-    starts = (0, 13, 57, 70, 86, 119, 240, 1021, 1200)      # 60 | 61 positions and 1024 | 1025, and the window's edge
+    starts = (0, 13, 57, 70, 86, 119, 240, 317, 1021, 1200)  # 60 | 61 positions and 320 | 321, and the window's edge
     got, persistent = _logits(cfg, "1", monkeypatch, toks, starts)
     assert persistent or window
     want, _ = _logits(cfg, "0", monkeypatch, toks, starts)
