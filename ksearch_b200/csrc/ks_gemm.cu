@@ -956,7 +956,7 @@ size_t ks_gemm_kq_bytes(const ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_t 
   return ks_gemm_xt_bytes(cols, n_tok) + 4 * slots * n_tok * rows;
 }
 
-// y[t * ldy + r] = sum_k W[r, k] x[t * ldx + k] for t < n_tok (<= 256), f32 x and y: operand split, GEMM and, when
+// y[t * ldy + r] = sum_k W[r, k] x[t * ldx + k] for t < n_tok (Q4_K: up to KS_GEMM_ROWS, Q6_K: 256), f32 x and y: operand split, GEMM and, when
 // the k range was split, the ordered sum of the partials.  `scratch`: ks_gemm_kq_bytes.
 int ks_launch_gemm_kq(ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_t cols, const uint8_t* W, const float* x, size_t ldx, float* y,
                       size_t ldy, int n_tok, void* scratch) {

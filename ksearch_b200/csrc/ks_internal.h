@@ -247,8 +247,7 @@ struct ks_mega_desc {
   const int* pos;     // device: position of the token being processed
   float *x_a, *x_b;   // residual stream ping-pong; the token's embedding is in x_a on entry
   float* yb;
-  float* att_tmp;     // n_q * n_splits * (hd + 2) floats
-  int n_splits;
+  int n_splits;       // ks_flow: at most so many context splits
 };
 // Two kernels take the same description.  ks_mega_* (ks_mega.cu): phases separated by grid-wide barriers,
 // inputs staged from plain global vectors.  ks_flow_* (ks_flow.cu): no barriers, every value that crosses

@@ -919,46 +919,37 @@ __device__ __forceinline__ void mg_attention(const MegaArgs& a, const MegaLayer&
 }
 
 // The o-projection's input out of the records of at most MG_DIRECT splits: each thread merges four neighbouring dims of a head at
-// a time, every load of a round first.
+// a time, every load first.
 __device__ __forceinline__ void mg_stage_merge(unsigned char* xs, const MegaArgs& a, unsigned NS, unsigned cols) {
   const unsigned tid = mg_tid();
   const unsigned units = cols >> 6, nchunk = cols >> 2, rec_len = mg_rec(a.hd);
-  constexpr int PER = 1;
-  for (unsigned base = tid; base < nchunk; base += PER * MG_THREADS) {  // (whole warps: nchunk is a multiple of 128)
-    float2 ml[PER][MG_DIRECT];
-    float4 o[PER][MG_DIRECT];
+  for (unsigned c = tid; c < nchunk; c += MG_THREADS) {  // (whole warps: nchunk is a multiple of 128)
+    const unsigned head = (c << 2) / a.hd, d = (c << 2) - head * a.hd;
+    const float* rec = a.att_tmp + (size_t)head * a.n_splits * rec_len;
+    float2 ml[MG_DIRECT];
+    float4 o[MG_DIRECT];
 #pragma unroll
-    for (int k = 0; k < PER; k++) {
-      const unsigned c = base + (unsigned)k * MG_THREADS, head = (c << 2) / a.hd, d = (c << 2) - head * a.hd;
-      const float* rec = a.att_tmp + (size_t)head * a.n_splits * rec_len;
-#pragma unroll
-      for (unsigned s = 0; s < MG_DIRECT; s++) {
-        const bool there = c < nchunk && s < NS;
-        const float* r = rec + s * rec_len;
-        ml[k][s] = there ? __ldcg(reinterpret_cast<const float2*>(r + a.hd)) : make_float2(kNegInit, 0.0f);
-        o[k][s] = there ? __ldcg(reinterpret_cast<const float4*>(r + d)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      }
+    for (unsigned s = 0; s < MG_DIRECT; s++) {
+      const float* r = rec + s * rec_len;
+      ml[s] = s < NS ? __ldcg(reinterpret_cast<const float2*>(r + a.hd)) : make_float2(kNegInit, 0.0f);
+      o[s] = s < NS ? __ldcg(reinterpret_cast<const float4*>(r + d)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
+    float M = kNegInit, Ls = 0.0f;
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-    for (int k = 0; k < PER; k++) {
-      const unsigned c = base + (unsigned)k * MG_THREADS;
-      float M = kNegInit, Ls = 0.0f;
-      float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (unsigned s = 0; s < MG_DIRECT; s++) M = fmaxf(M, ml[s].x);
 #pragma unroll
-      for (unsigned s = 0; s < MG_DIRECT; s++) M = fmaxf(M, ml[k][s].x);
-#pragma unroll
-      for (unsigned s = 0; s < MG_DIRECT; s++) {
-        const float f = __expf(ml[k][s].x - M);
-        Ls = fmaf(ml[k][s].y, f, Ls);
-        v.x = fmaf(o[k][s].x, f, v.x);
-        v.y = fmaf(o[k][s].y, f, v.y);
-        v.z = fmaf(o[k][s].z, f, v.z);
-        v.w = fmaf(o[k][s].w, f, v.w);
-      }
-      const float inv = 1.0f / Ls;
-      v.x *= inv; v.y *= inv; v.z *= inv; v.w *= inv;
-      if (c < nchunk) fx_put_chunk(xs, units, c, v);
+    for (unsigned s = 0; s < MG_DIRECT; s++) {
+      const float f = __expf(ml[s].x - M);
+      Ls = fmaf(ml[s].y, f, Ls);
+      v.x = fmaf(o[s].x, f, v.x);
+      v.y = fmaf(o[s].y, f, v.y);
+      v.z = fmaf(o[s].z, f, v.z);
+      v.w = fmaf(o[s].w, f, v.w);
     }
+    const float inv = 1.0f / Ls;
+    v.x *= inv; v.y *= inv; v.z *= inv; v.w *= inv;
+    fx_put_chunk(xs, units, c, v);
   }
 }
 

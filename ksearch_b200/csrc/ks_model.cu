@@ -660,7 +660,6 @@ int get_mega(ks_model* m, int first, ks_model::Mega* out) {
   d.x_a = m->step32 ? m->step32 + (size_t)first * 3 * H : (float*)m->x + (size_t)first * H;
   d.x_b = m->step32 ? d.x_a + H : (float*)m->xb + (size_t)first * H;
   d.yb = m->step32 ? d.x_a + 2 * H : (float*)m->x2 + (size_t)first * H;
-  d.att_tmp = m->attn_tmp + (size_t)first * g.n_q * m->n_splits * (g.hd + 2);
   d.n_splits = m->n_splits;
   std::vector<ks_mega_layer> ls(g.n_layers);
   for (int l = 0; l < g.n_layers; l++) {

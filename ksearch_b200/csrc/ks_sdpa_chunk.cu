@@ -17,8 +17,11 @@
 // The context is split over blockIdx.z; (m, l, O) records go to `tmp` as the decode kernels leave them and
 // sdpa_merge_split_kernel folds them straight into the operand image of the output projection.
 //
-// Bound by the chain scores -> probabilities -> values of a tile: about 2.2 us for 128 x 64, 1.5 of them MMAs.  2047 rows of 8
-// heads: 109 us; 2000 rows behind 2000 positions, 2 KV heads: 299.  On mma.sync (64 rows a block) the same took 336 and 809.
+// Bound by the decoders, who turn a tile's values, fold the one before and turn the next one's keys in a row: 5.7 us for 128 x 64,
+// 1.2 of them MMAs (2047 rows, 2 splits: tensor pipe 21 %, issue slots 38 %).  A block takes another 18 us for its start, q and
+// records.  Back to back: one block of 64 tiles 381 us; 2047 rows of 8 heads (128 blocks of up to 32 tiles) 205 us, in two splits 118;
+// 2000 rows behind 2000 positions, 2 KV heads (126 blocks of up to 63 tiles) 388, in two splits 344.  On mma.sync (64 rows a block) the
+// last two took 336 and 809.
 #include "ks_gemm_common.cuh"
 
 namespace {
@@ -566,7 +569,7 @@ int launch_chunk(ks_ctx* ctx, dim3 grid, const ChunkParts& parts, size_t slot_st
 
 // Context splits of a chunk: enough blocks for every SM, at least two tiles each.  A nearly empty second wave costs more than fewer
 // splits, except against one: the later rows see most of the context, and half a chip waits for them (2047 rows of 8 heads, 128
-// blocks: 162 us, twice as many halves 109).  `ctx_len` may exceed what the rows see.
+// blocks: 205 us, twice as many halves 118, three times as many thirds 151).  `ctx_len` may exceed what the rows see.
 int ks_sdpa_chunk_splits(const ks_ctx* ctx, int n_tok, size_t n_q, size_t n_kv, size_t ctx_len, int most) {
   const size_t blocks = ((size_t)n_tok * (n_q / n_kv) + CH_BM - 1) / CH_BM * n_kv;
   size_t s = ((size_t)ctx->sm_count + blocks - 1) / blocks;
