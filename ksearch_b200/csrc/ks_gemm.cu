@@ -444,7 +444,10 @@ struct EpiNormArgs {
   float* out_x;
   __half* xt;
 };
-__global__ void gemm_finish_norm_split_kernel(const EpiNormArgs e) {
+constexpr size_t GM_NORM_MOST = 8 * 1024;  // the longest rows: eight values per thread
+// THREADS: at most; more than 512 have half the registers each.
+template <unsigned THREADS>
+__global__ void __launch_bounds__(THREADS) gemm_finish_norm_split_kernel(const EpiNormArgs e) {
   ks_pdl_entry();
   __shared__ float red[32];
   const unsigned t = blockIdx.x, ck = threadIdx.x, chunks = e.rows / 8u;
@@ -504,8 +507,7 @@ constexpr int GM_ROW_THREADS = 1024;  // threads of a block that writes one toke
 // blocks per (padded) token row, 8 values per thread: the row maximum that scales the image meets in distributed shared memory,
 // and few token rows still make enough blocks (8 rows of 10240 values: 64 blocks instead of 16).
 constexpr unsigned GM_GELU_CL = 4, GM_GELU_THREADS = 512;
-// The longest rows the two epilogues take: eight values per thread of one block, and of a cluster.
-constexpr size_t GM_NORM_MOST = 8 * 1024, GM_GELU_MOST = 8 * GM_GELU_CL * GM_GELU_THREADS;
+constexpr size_t GM_GELU_MOST = 8 * GM_GELU_CL * GM_GELU_THREADS;
 __global__ void __cluster_dims__(GM_GELU_CL, 1, 1) __launch_bounds__(GM_GELU_THREADS)
     gemm_finish_gelu_split_kernel(const float* P0, const float* P1, size_t part_stride, ks_gemm_map map, unsigned n_tok, unsigned np, unsigned tbn,
                                   unsigned rows, __half* xt) {
@@ -882,7 +884,9 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
     e.eps = epi->eps;
     e.out_x = epi->out_x;
     e.xt = (__half*)epi->xt_out;
-    KS_LAUNCH(ctx, (gemm_finish_norm_split_kernel), e.np, (unsigned)((rows[0] / 8 + 31) / 32 * 32), 0, e);
+    const unsigned threads = (unsigned)((rows[0] / 8 + 31) / 32 * 32);
+    if (threads <= 512u) KS_LAUNCH(ctx, (gemm_finish_norm_split_kernel<512>), e.np, threads, 0, e);
+    else KS_LAUNCH(ctx, (gemm_finish_norm_split_kernel<1024>), e.np, threads, 0, e);
     return ks_after_launch(ctx, "gemm_finish_norm_split");
   }
   if (mode == KS_GEMM_QKV) {

@@ -757,6 +757,26 @@ def test_f16_activation_model_runs_close(ctx, oracle):
     model.close()
 
 
+@pytest.mark.parametrize("hidden", [5632, 8192])
+def test_prompt_of_the_widest_rows_the_gemm_epilogue_takes(ctx, oracle, hidden):
+    """Hidden rows of up to 8192 values take eight values per thread: blocks of more than 672 threads need the epilogue with fewer
+    registers, or the launch fails.  1e-3 of the logits' scale, the model's bound."""
+    cfg = ksm.ModelConfig(1, hidden, 512, 2, 1, 128, hidden, 32, 1, sigma_embd=5e-5)
+    model, T = ksm.GemmaCudaModel.synthetic(ctx, cfg, seed=67, keep=True)
+    model.slot_alloc()
+    toks = [int(t) for t in synth.token_ids(67, "p", 12, cfg.vocab)]
+    cpu = oracle.CpuDecoder(oracle.decoder_cfg(cfg), T)
+    for t in toks:
+        cpu.forward_token(t, True)
+    want = cpu.logits().astype(np.float64)
+    model.prefill(0, toks[:-1])
+    model.forward(0, 1, [toks[-1]], True)
+    ctx.synchronize()
+    assert np.abs(model.read_debug(1, 0).astype(np.float64) - want).max() <= 1e-3 * np.abs(want).max()
+    cpu.close()
+    model.close()
+
+
 @pytest.mark.parametrize("act", [F32, F16])
 @pytest.mark.parametrize("hidden,ffn", [(512, 21504), (8448, 512)])
 def test_prompt_of_a_model_wider_than_the_gemm_epilogues(ctx, oracle, act, hidden, ffn):
