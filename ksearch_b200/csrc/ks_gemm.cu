@@ -515,6 +515,7 @@ __global__ void __cluster_dims__(GM_GELU_CL, 1, 1) __launch_bounds__(GM_GELU_THR
   __shared__ float red[32], maxima[GM_GELU_CL];
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
+  cluster.barrier_arrive();  // (a block's shared memory is there once it has started)
   const unsigned rank = blockIdx.x % GM_GELU_CL, t = blockIdx.x / GM_GELU_CL, chunks = rows / 8u, ck = rank * blockDim.x + threadIdx.x;
   float v[8];
 #pragma unroll
@@ -530,6 +531,7 @@ __global__ void __cluster_dims__(GM_GELU_CL, 1, 1) __launch_bounds__(GM_GELU_THR
   }
   // gelu(gate) * up is where a random-weight model leaves the f16 range
   const float m = block_max_f(absmax8(v), red);
+  cluster.barrier_wait();
   if (threadIdx.x < GM_GELU_CL) *cluster.map_shared_rank(&maxima[rank], threadIdx.x) = m;
   cluster.sync();
   float row_max = maxima[0];
@@ -542,6 +544,94 @@ __global__ void __cluster_dims__(GM_GELU_CL, 1, 1) __launch_bounds__(GM_GELU_THR
 #pragma unroll
     for (int k = 0; k < 8; k++) v[k] *= down;
     put_split8(xt, np, tbn, t, ck, chunks, v, true);  // a down-projection is always Q4_K
+  }
+}
+
+// The same for passes of many rows: a cluster of eight blocks per FOUR token rows, two steps of 64 columns per warp
+// (put_split8_rows4).  Bound by loads in flight: all first partials are requested before anything is waited for, and 64 registers
+// keep five blocks of 192 threads on an SM (with 94 and three: 60 us instead of 47; with the second partials requested early as well
+// it spills: 51).  The partial counts, half a dozen divisions each, are a lane's work each (31 to 24 million instructions).
+// 2047 rows of 6144 values, 111 MB read and 57 written: 78 us with a cluster of four per row, 47 here; 1530 rows of 10240: 107, 60.
+constexpr unsigned GM_R4_CL = 8, GM_R4_S = 2, GM_R4_WARPS = 16;  // blocks of a cluster, steps of a warp, warps at most
+constexpr int GM_R4_ROWS = 128;  // from so many rows and values on: 129 rows of 6144 values 7.8 and 6.6 us, of 1024 5.1 and 6.4; 1025 of 1024 15.9 and 8.7
+constexpr size_t GM_R4_VALUES = 1u << 18;
+static_assert(GM_GELU_MOST <= GM_R4_CL * GM_R4_S * GM_R4_WARPS * 64, "the longest rows fit");
+__device__ __forceinline__ void ld8(const float* p, float (&v)[8]) {
+  *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p);
+  *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(p + 4);
+}
+// Partials 1 .. n - 1 on top of the first.
+__device__ __forceinline__ void add_slots(const float* p, size_t stride, unsigned n, float (&v)[8]) {
+  for (unsigned k = 1; k < n; k++) {
+    float x[8];
+    ld8(p + (size_t)k * stride, x);
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] += x[i];
+  }
+}
+__global__ void __cluster_dims__(GM_R4_CL, 1, 1) __launch_bounds__(GM_R4_WARPS * 32, 2)
+    gemm_finish_gelu_rows_kernel(const float* P0, const float* P1, size_t part_stride, ks_gemm_map map, unsigned n_tok, unsigned np, unsigned tbn,
+                                 unsigned rows, __half* xt) {
+  ks_pdl_entry();
+  __shared__ float red[GM_R4_WARPS][4], maxima[GM_R4_CL][4];
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.barrier_arrive();  // (a block's shared memory is there once it has started)
+  const unsigned rank = blockIdx.x % GM_R4_CL, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const unsigned t0 = blockIdx.x / GM_R4_CL * 4u, t = t0 + (lane & 3u);
+  const unsigned steps = rows / 64u, per = (steps + GM_R4_CL - 1u) / GM_R4_CL, first = rank * per, end = min(first + per, steps);
+  const unsigned groups = map.G ? ((rows + GM_ROWS - 1u) / GM_ROWS + map.nt - 1u) / map.nt : 0u;
+  float v[GM_R4_S][8], u[GM_R4_S][8];
+#pragma unroll
+  for (unsigned s = 0; s < GM_R4_S; s++) {
+    const unsigned st = first + warp + s * warps;
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[s][k] = u[s][k] = 0.0f;
+    if (st < end && t < n_tok) {
+      const size_t at = (size_t)t * rows + 64u * st + 8u * (lane >> 2);
+      ld8(P0 + at, v[s]);
+      ld8(P1 + at, u[s]);
+    }
+  }
+  const unsigned my_slots = ks_gemm_slots(map, lane & 1u ? groups : 0u, 64u * (first + warp + (lane >> 1) % GM_R4_S * warps) / GM_ROWS, t0);
+  float m = 0.0f;
+#pragma unroll
+  for (unsigned s = 0; s < GM_R4_S; s++) {
+    const unsigned st = first + warp + s * warps, ng = __shfl_sync(0xffffffffu, my_slots, 2 * s), nu = __shfl_sync(0xffffffffu, my_slots, 2 * s + 1);
+    if (st < end && t < n_tok) {
+      const size_t at = (size_t)t * rows + 64u * st + 8u * (lane >> 2);
+      add_slots(P0 + at, part_stride, ng, v[s]);
+      add_slots(P1 + at, part_stride, nu, u[s]);
+#pragma unroll
+      for (int k = 0; k < 8; k++) v[s][k] = gelu_mul(v[s][k], u[s][k]);
+      m = fmaxf(m, absmax8(v[s]));
+    }
+  }
+  // the rows' largest values: over the warp's lanes, the block, the cluster
+#pragma unroll
+  for (int o = 4; o <= 16; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (lane < 4u) red[warp][lane] = m;
+  __syncthreads();
+  m = 0.0f;
+#pragma unroll 4
+  for (unsigned w = 0; w < warps; w++) m = fmaxf(m, red[w][lane & 3u]);
+  cluster.barrier_wait();
+  if (threadIdx.x < 4u * GM_R4_CL) cluster.map_shared_rank(&maxima[rank][0], threadIdx.x >> 2)[lane & 3u] = m;
+  cluster.sync();
+  float row_max = maxima[0][lane & 3u];
+#pragma unroll
+  for (unsigned k = 1; k < GM_R4_CL; k++) row_max = fmaxf(row_max, maxima[k][lane & 3u]);
+  float up;
+  const float down = row_scale_down(row_max, &up);
+  if (rank == 0 && threadIdx.x < 4u) reinterpret_cast<float*>(xt + xt_scale_off(rows, np))[t] = up;
+#pragma unroll
+  for (unsigned s = 0; s < GM_R4_S; s++) {
+    const unsigned st = first + warp + s * warps;
+    if (st < end) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) v[s][k] *= down;
+      put_split8_rows4(xt, tbn, t0, 8u * st, rows / 8u, v[s]);
+    }
   }
 }
 
@@ -585,10 +675,11 @@ __global__ void __launch_bounds__(256) gemm_finish_qkv_kernel(const EpiQkvArgs e
     w[0][k] = seg == 0 ? e.qw[d] : seg == 1 ? e.kw[d] : 1.0f;
     w[1][k] = seg == 0 ? e.qw[HD / 2 + d] : seg == 1 ? e.kw[HD / 2 + d] : 1.0f;
   }
+  // (half a head is one row tile, or within one; how many partials it has takes half a dozen divisions: a lane each)
+  const unsigned my_slots = ks_gemm_slots(e.map, g0, (head * HD + (lane & 1u) * (HD / 2)) / GM_ROWS, tok);
 #pragma unroll
   for (int h = 0; h < 2; h++) {
-    const unsigned row = head * HD + (unsigned)h * (HD / 2) + lane * V;
-    const unsigned n = ks_gemm_slots(e.map, g0, row / GM_ROWS, tok);
+    const unsigned row = head * HD + (unsigned)h * (HD / 2) + lane * V, n = __shfl_sync(0xffffffffu, my_slots, h);
     const float* src = P + (size_t)tok * rows + row;
 #pragma unroll
     for (int k = 0; k < V; k++) x[h][k] = 0.0f;
@@ -917,6 +1008,12 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
     return ks_after_launch(ctx, "gemm_finish_qkv");
   }
   if (mode == KS_GEMM_GELU_SPLIT) {
+    if (n_tok >= GM_R4_ROWS && (size_t)n_tok * rows[0] >= GM_R4_VALUES) {
+      const unsigned per = ((unsigned)rows[0] / 64u + GM_R4_CL - 1u) / GM_R4_CL, warps = (per + GM_R4_S - 1u) / GM_R4_S;
+      KS_LAUNCH(ctx, gemm_finish_gelu_rows_kernel, epi->next.np / 4u * GM_R4_CL, warps * 32u, 0, (const float*)out[0], (const float*)out[1], part_stride[0], map,
+                (unsigned)n_tok, epi->next.np, epi->next.tbn, (unsigned)rows[0], (__half*)epi->xt_out);
+      return ks_after_launch(ctx, "gemm_finish_gelu_rows");
+    }
     // whole warps per block: a 32-value sub-block of the image is four neighbouring lanes of one
     const unsigned threads = ((unsigned)rows[0] / 8u / GM_GELU_CL + 31u) / 32u * 32u;
     KS_LAUNCH(ctx, (gemm_finish_gelu_split_kernel), epi->next.np * GM_GELU_CL, threads, 0, (const float*)out[0], (const float*)out[1], part_stride[0], map,

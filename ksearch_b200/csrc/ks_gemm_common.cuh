@@ -103,6 +103,36 @@ __device__ __forceinline__ void put_split8(__half* xt, unsigned np, unsigned tbn
   *reinterpret_cast<uint4*>(base + (size_t)np * 8u) = lo;
 }
 
+// The same for passes of many rows: a warp holds 64 columns (chunks ck0 .. ck0 + 7, ck0 a multiple of 8) of four neighbouring token
+// rows, lane = row t0 + lane % 4 (t0 a multiple of 4), chunk ck0 + lane / 4.  A chunk's four rows are then 64 neighbouring bytes of
+// the q4k image; one row per block leaves a warp's 16-byte stores in 32 lines, 4 KB apart.  The sums are added in the order of put_split8.
+__device__ __forceinline__ void put_split8_rows4(__half* xt, unsigned tbn, unsigned t0, unsigned ck0, unsigned chunks, const float (&v)[8]) {
+  const unsigned lane = threadIdx.x & 31u, c = lane >> 2, ck = ck0 + c, blk = t0 / tbn, t = t0 - blk * tbn + (lane & 3u);
+  xt += (size_t)(chunks / 32u * 36u) * 2u * (blk * tbn) * 8u + (size_t)t * 8u;
+  const float w[8] = {v[0], v[2], v[1], v[3], v[4], v[6], v[5], v[7]};
+  uint4 hi, lo;
+  split8(w, hi, lo);
+  __half* base = xt + (size_t)((ck >> 5) * 36u + (ck & 31u)) * 2u * tbn * 8u;
+  *reinterpret_cast<uint4*>(base) = hi;
+  *reinterpret_cast<uint4*>(base + (size_t)tbn * 8u) = lo;
+  float s = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+  s += __shfl_xor_sync(0xffffffffu, s, 4);
+  s += __shfl_xor_sync(0xffffffffu, s, 8);
+  const float s1 = __shfl_xor_sync(0xffffffffu, s, 16);
+  if (c < 2u) {
+    uint4 e = make_uint4(0u, 0u, 0u, 0u);
+    if (c == 0u) {
+      const __half2 h = __floats2half2_rn(s * 0.03125f, s1 * 0.03125f);
+      const float2 hf = __half22float2(h);
+      e.x = pack_h2(h);
+      e.y = pack_h2(__floats2half2_rn(s * 0.03125f - hf.x, s1 * 0.03125f - hf.y));
+      e.z = e.x;
+    }
+    __half* ext = xt + (size_t)((ck0 >> 5) * 36u + 32u + ((ck0 & 31u) >> 3)) * 2u * tbn * 8u;
+    *reinterpret_cast<uint4*>(ext + (c ? (size_t)tbn * 8u : 0)) = e;  // chunk 1's lanes clear the lo row
+  }
+}
+
 // Range.  f16 ends at 65504 and loses its low term below ~1e-3 (the low half of a small value is a denormal);
 // activations do neither.  Every token row is therefore stored as x * 2^-e with e = exponent(largest magnitude) - 14,
 // so the scaled row peaks in [2^14, 2^15), and the GEMM multiplies that token's outputs by 2^e (both exact).

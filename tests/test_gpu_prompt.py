@@ -178,3 +178,19 @@ def test_mixed_passes_of_other_models(ctx, n_slots, n_kv, hd, act, window):
         assert 0 < scale < np.inf
         assert err.max() <= worst * scale and np.sqrt((err ** 2).mean()) <= mean * scale
     model.close()
+
+
+@pytest.mark.parametrize("ffn", [2304, 3328, 16384])
+def test_gelu_of_four_rows_per_cluster(ctx, ffn):
+    """From 128 rows and 2^18 values on four token rows share a cluster of blocks: row counts around a multiple of four, widths that
+    leave warps of a block and blocks of the cluster without work, the widest rows.  Against pieces of 100 rows, which have a cluster per row."""
+    cfg = ksm.ModelConfig(2, 256, ffn, 2, 1, 128, 1024, 256, 1, sigma_w=0.01, sigma_embd=1e-4)
+    model, _ = ksm.GemmaCudaModel.synthetic(ctx, cfg, seed=43, keep=True)
+    model.slot_alloc()
+    toks = [int(t) for t in synth.token_ids(43, "p", 200, cfg.vocab)]
+    for n in (128, 129, 130, 131, 191):
+        want = _logits_after(model, ctx, [toks[i:min(i + 100, n)] for i in range(0, n, 100)], toks[n])
+        got = _logits_after(model, ctx, [toks[:n]], toks[n])
+        scale, err = np.abs(want).max(), np.abs(got - want)
+        assert err.max() <= 1e-3 * scale and np.sqrt((err ** 2).mean()) <= 1e-4 * scale, n
+    model.close()
