@@ -156,10 +156,21 @@ bool ks_sdpa_chunk_covers(size_t n_q, size_t n_kv, size_t hd, const void* K, con
 // Rows [row0[p], row0[p + 1]) of a pass belong to slot[p]; no slot twice.
 struct ks_row_parts {
   unsigned n, row0[65], slot[64];
+  unsigned image0[64];  // where a part's decoded tiles start in the image
 };
+// Room for `tiles` decoded tiles of 64 positions of every KV head (ks_kv_image_bytes); tile t of a part at image0 + t.  No part sees
+// more than `span` tiles.
+struct ks_kv_image {
+  void* base;
+  size_t tiles;
+  unsigned span;
+};
+size_t ks_kv_image_bytes(size_t tiles, size_t n_kv, size_t hd);
+unsigned ks_kv_image_tiles(size_t positions);
 // parts == nullptr: all rows belong to the cache at K and V; else part p's cache is slot[p] * slot_stride bytes on.
 int ks_launch_sdpa_chunk(ks_ctx* ctx, int n_tok, size_t n_q, size_t n_kv, size_t hd, float scale, const float* q, const uint8_t* K,
-                         const uint8_t* V, const float* meta, float* tmp, int n_splits, const ks_row_parts* parts = nullptr, size_t slot_stride = 0);
+                         const uint8_t* V, const float* meta, float* tmp, int n_splits, const ks_kv_image& image, const ks_row_parts* parts = nullptr,
+                         size_t slot_stride = 0);
 // Token rows per block of an operand image and all of them padded to whole blocks: a choice of the GEMM that reads the image.
 struct ks_gemm_blocks {
   unsigned tbn, np;

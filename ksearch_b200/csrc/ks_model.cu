@@ -206,6 +206,8 @@ struct ks_model {
   // operand image, the k-split partials
   int gemm_chunk = 0;
   int prompt_chunk = 1;  // prompt rows up to which the batch matvec takes them although the GEMM could
+  void* kv_image = nullptr;     // decoded tiles of one layer's caches for chunk attention: room for this many tiles of every KV head
+  size_t kv_image_tiles = 0;
   void* gemm_xt = nullptr;
   float* gemm_p0 = nullptr;
 };
@@ -229,25 +231,28 @@ constexpr int KS_PREFILL_CHUNK = 8;  // tokens per pass over the weights (the ma
 constexpr int KS_GEMM_CHUNK = KS_GEMM_ROWS;
 constexpr size_t KS_STAGE_IDS = KS_GEMM_CHUNK; // pinned words that stage host token ids
 
-// Do the rows of a prompt chunk share one pass over their context (ks_sdpa_chunk.cu: 128 rows x heads a block, few blocks of 25 us
+// Do the rows of a prompt chunk share one pass over their context (ks_sdpa_chunk.cu: 128 rows x heads a block, few blocks of 20 us
 // and more), or does each take the decode kernel (a block per row and up to four heads, spread over the chip)?  By the work of the
 // second form, rows x blocks x positions a row sees on average in units of 256 dims, against a line that lies the higher the fewer
 // rows there are: few rows are few blocks of the first form.  Microseconds per layer of 24, shared / per row, with the work:
-//   E2B (8 heads, 1 KV head of 256)  256 rows at 0: 132 / 123 (65k), 320: 143 / 142 (102k), 384: 154 / 156 (147k); 128 at 512: 105 / 98 (147k),
-//                                    160: 122 / 125 (189k); 96 at 1024: 109 / 110 (205k); 48 at 2048: 101 / 101 (198k), 64: 114 / 104 (266k);
-//                                    window 128, 256 rows: 131 / 121 (65k), 512: 175 / 185 (131k), 768: 214 / 242 (196k)
-//   E4B (8, 2 of 256)                256 at 0: 198 / 188, 320: 232 / 234, 384: 241 / 253; 128 at 512: 145 / 139, 160: 167 / 180; 96 at 1024:
-//                                    143 / 148; 64 at 2048: 138 / 125; window 512 at 1024: 128 rows 144 / 135 (131k), 256: 196 / 208 (262k)
-//   tiny (4, 1 of 128)               384 at 0: 72 / 68 (37k), 192 at 512: 66 / 59 (58k), 128 at 1024: 70 / 64 (70k)
-// A block of one head does the work of four, so with a KV head per query head (8, 8 of 128) the line lies lower: 128 at 0: 67 / 65
-// (33k), 192: 66 / 80 (74k); 24 at 2048: 60 / 78 (197k); 16 at 3500: 71 / 72 (225k); 32 at 512: 61 / 58 (68k).
+//   E2B (8 heads, 1 KV head of 256)  256 rows at 0: 124 / 118 (65k), 320: 130 / 133 (102k), 384: 136 / 147 (147k); 128 at 512: 100 / 96 (147k),
+//                                    160: 117 / 123 (189k); 96 at 1024: 103 / 106 (205k); 48 at 2048: 102 / 97 (198k), 64: 111 / 101 (266k);
+//                                    window 128, 256 rows: 124 / 116 (65k), 512: 167 / 178 (131k)
+//   E4B (8, 2 of 256)                256 at 0: 183 / 178, 320: 216 / 221, 384: 230 / 242; 128 at 512: 143 / 136, 160: 159 / 167; 96 at 1024:
+//                                    142 / 145; 64 at 2048: 146 / 123; window 512 at 1024: 128 rows 145 / 132 (131k), 192: 175 / 169 (196k)
+//   tiny (4, 1 of 128)               384 at 0: 65 / 63 (37k), 192 at 512: 60 / 56 (58k), 128 at 1024: 65 / 60 (70k)
+// A block of one head does the work of four, so with a KV head per query head (8, 8 of 128) the line lies lower: 128 at 0: 62 / 61
+// (33k), 192: 63 / 77 (74k); 24 at 2048: 58 / 74 (197k); 16 at 3500: 73 / 69 (225k); 32 at 512: 52 / 47 (68k).
 bool rows_share_context(const ks_model_config& g, int n, int base, int window) {
   const int hpk = g.n_q / g.n_kv, gb = hpk % 4 == 0 ? 4 : hpk % 2 == 0 ? 2 : 1;
   double seen = base + 0.5 * (n + 1);
   if (window > 0 && seen > window) seen = window;
   const double work = (double)n * (g.n_q / gb) * seen * g.hd / 256.0;
-  return n >= 4 && work >= (gb == 1 ? 45e3 + 1e6 / n : 75e3 + 13e6 / n);
+  return n >= 4 && work >= (gb == 1 ? 45e3 + 1e6 / n : 60e3 + 13e6 / n);
 }
+
+// Bytes of decoded tiles (chunk attention) a model has room for, beyond one slot's: a pass that mixes slots takes as many as fit.
+constexpr size_t KS_IMAGE_MOST = 256u << 20;
 
 // Where a forward pass reads and writes: n rows of activations, their positions, and the KV caches
 // behind them.  Decode steps map row s to slot first + s (one cache per row); a prompt chunk maps
@@ -266,6 +271,7 @@ struct Lane {
   int* chunk_base;   // prompt chunk: the slot's position word (rows take base, base + 1, ...); else nullptr
   const ks_row_parts* parts; // prompt rows of several slots (kv_stride is then between slots); else nullptr
   bool share_full, share_swa;  // prompt chunk: do its rows share one pass over their context in a full / sliding-window layer?
+  unsigned image_span;         // ... and at most how many tiles of 64 positions does a part see?
 };
 
 Lane slot_lane(ks_model* m, int first, int src) {
@@ -294,8 +300,9 @@ Lane slot_lane(ks_model* m, int first, int src) {
   return L;
 }
 
-Lane chunk_lane(ks_model* m, int slot, bool share_full, bool share_swa) {
+Lane chunk_lane(ks_model* m, int slot, bool share_full, bool share_swa, unsigned image_span) {
   Lane L{};
+  L.image_span = image_span;
   L.share_full = share_full;
   L.share_swa = share_swa;
   L.x = (char*)m->cx; L.xb = (char*)m->cxb; L.x2 = (char*)m->cx2; L.xn = nullptr;
@@ -457,7 +464,8 @@ int enqueue_forward_gemm(ks_model* m, const Lane& L_, int n, bool want_logits) {
     }
     const bool share = layer_meta(m, L_, l) == L_.meta ? L_.share_full : L_.share_swa;
     if (share && ks_sdpa_chunk_covers(nq, nkv, hd, kk, kv)) {
-      if ((rc = ks_launch_sdpa_chunk(c, n, nq, nkv, hd, g.attn_scale, (const float*)q, kk, kv, layer_meta(m, L_, l), L_.attn_tmp, chunk_splits, L_.parts, L_.kv_stride)) ||
+      const ks_kv_image image{m->kv_image, m->kv_image_tiles, L_.image_span};
+      if ((rc = ks_launch_sdpa_chunk(c, n, nq, nkv, hd, g.attn_scale, (const float*)q, kk, kv, layer_meta(m, L_, l), L_.attn_tmp, chunk_splits, image, L_.parts, L_.kv_stride)) ||
           (rc = ks_launch_sdpa_merge_split(c, n, b_o, nq, hd, L_.attn_tmp, chunk_splits, m->gemm_xt)))
         return rc;
     } else if (att_splits > 1 && ks_sdpa_merge_split_covers(nq, hd)) {
@@ -750,9 +758,10 @@ constexpr size_t KS_PROMPT_GRAPHS = 64;
 // copy, so a graph may be dropped.
 int run_prefill_chunk(ks_model* m, int slot, int n, bool gemm) {
   ks_ctx* c = m->ctx;
-  const bool share_full = gemm && rows_share_context(m->cfg, n, m->seq_len[slot], 0);
-  const bool share_swa = gemm && rows_share_context(m->cfg, n, m->seq_len[slot], m->cfg.sliding_window);
-  const Lane lane = chunk_lane(m, slot, share_full, share_swa);
+  const bool share_full = gemm && m->kv_image && rows_share_context(m->cfg, n, m->seq_len[slot], 0);
+  const bool share_swa = gemm && m->kv_image && rows_share_context(m->cfg, n, m->seq_len[slot], m->cfg.sliding_window);
+  // (a replay may stand further on than the pass that was captured: its tiles are those of the whole slot)
+  const Lane lane = chunk_lane(m, slot, share_full, share_swa, ks_kv_image_tiles((size_t)m->cfg.max_seq));
   const uint64_t key = (1ull << 63) | ((uint64_t)slot << 32) | ((uint64_t)n << 8) | (share_full ? 1 : 0) | (share_swa && has_window(m->cfg) ? 2 : 0);
   if (!gemm) {  // 1..8 rows: few different passes
     auto it = m->graphs.find(key);
@@ -976,6 +985,19 @@ ks_model* ks_model_create(ks_ctx* ctx, const ks_model_config* cfg) {
       recs = r > recs ? r : recs;
     }
     ok = dev_alloc(m, (void**)&m->cattn_tmp, (recs * g.n_q * (g.hd + 2) + 4) * sizeof(float)) == KS_OK;
+  }
+  if (ok && m->gemm_chunk && ks_sdpa_chunk_covers(g.n_q, g.n_kv, g.hd, nullptr, nullptr)) {
+    // as many tiles as the slots can hold, within a bound but not less than one slot's; a model that has no memory left for them
+    // takes its prompts row by row
+    const size_t one = ks_kv_image_bytes(1, g.n_kv, g.hd), slot = ks_kv_image_tiles((size_t)g.max_seq), all = (size_t)g.n_slots * slot;
+    const size_t tiles = all * one <= KS_IMAGE_MOST ? all : std::max(slot, KS_IMAGE_MOST / one);
+    if (cudaMalloc(&m->kv_image, ks_kv_image_bytes(tiles, g.n_kv, g.hd)) == cudaSuccess) {
+      m->owned.push_back(m->kv_image);
+      m->kv_image_tiles = tiles;
+    } else {
+      (void)cudaGetLastError();
+      m->kv_image = nullptr;
+    }
   }
   if (ok) {
     ok = dev_alloc(m, (void**)&m->attn_tmp, (S * g.n_q * (size_t)m->n_splits * (g.hd + 2) + 4) * sizeof(float)) == KS_OK;
@@ -1376,18 +1398,25 @@ int ks_model_prefill_slots(ks_model* m, int n, const int* slots, const int* toke
   for (size_t t = 0; t < total; t++)
     KS_REQUIRE(c, tokens[t] >= 0 && tokens[t] < m->cfg.vocab, "token id %d outside the vocabulary", tokens[t]);
   const ks_model_config& g = m->cfg;
-  bool mix = m->gemm_chunk > 0 && m->slot_stride % 4 == 0;
+  bool mix = m->gemm_chunk > 0 && m->slot_stride % 4 == 0 && m->kv_image;
   for (int l = 0; l < g.n_layers; l++) mix = mix && ks_sdpa_chunk_covers(g.n_q, g.n_kv, g.hd, m->kv_k[l], m->kv_v[l]);
   float* stage = m->host_tok + m->host_tok_n - 16 - KS_STAGE_IDS;
   const int* next = tokens;
   int i = 0, used = 0;  // `used` tokens of part i have run
   while (i < n) {
-    // the parts of this pass
+    // the parts of this pass; their decoded tiles lie one part's behind the other's
     ks_row_parts parts{};
     int rows = 0;
+    size_t tiles = 0;
+    unsigned span = 0;
     while (i < n && (int)parts.n < (mix ? 64 : 1) && rows < (mix ? m->gemm_chunk : 1 << 30)) {
       const int left = counts[i] - used, take = mix ? std::min(left, m->gemm_chunk - rows) : left;
+      const unsigned sees = ks_kv_image_tiles((size_t)m->seq_len[slots[i]] + take);
+      if (mix && parts.n && take > 0 && tiles + sees > m->kv_image_tiles) break;  // (one part always fits)
       if (take > 0) {
+        parts.image0[parts.n] = (unsigned)tiles;
+        tiles += sees;
+        span = std::max(span, sees);
         parts.slot[parts.n] = (unsigned)slots[i];
         parts.row0[parts.n++] = (unsigned)rows;
         rows += take;
@@ -1412,7 +1441,7 @@ int ks_model_prefill_slots(ks_model* m, int n, const int* slots, const int* toke
     KS_CUDA(c, cudaStreamSynchronize(c->stream));  // the staging words may still be in flight
     for (int t = 0; t < rows; t++) stage[t] = (float)next[t];
     KS_CUDA(c, cudaMemcpyAsync(m->ctok, stage, rows * sizeof(float), cudaMemcpyHostToDevice, c->stream));
-    Lane lane = chunk_lane(m, 0, true, true);
+    Lane lane = chunk_lane(m, 0, true, true, span);
     lane.chunk_base = nullptr;
     lane.kv_off = 0;
     lane.kv_stride = m->slot_stride;

@@ -2,51 +2,48 @@
 //
 // The reference runs its decode attention once per prompt row (forward_prefill_chunk, crates/ksearch_gemma/src/
 // gemma_prim.rs:1463-1472, over crates/ksearch_codegen/src/lower.rs:4897-6088), so every row reads the whole context again.
-// Here a block takes 128 query rows that share a KV head (128 / G tokens x the head's G query heads), brings each tile of 64
-// positions in once and multiplies on tcgen05 (f16 in, f32 out) without giving up f32 accuracy: q (scaled per row by a power of
-// two), the cached values d (n - 8), exactly, and the probabilities are two f16 terms each, a product is hi hi + hi lo + lo hi.
-//   * q's first term and the probabilities lie in TENSOR memory as the A operand, q's second term and the decoded tile in shared
-//     memory; scores and a tile's values are the accumulators (HD = 256 fills the 512 columns);
-//   * four warps own a row of scores per thread: mask, running maximum, probabilities;
-//   * eight decode: K as positions x dims, V as dims x positions (a thread takes one byte of eight neighbouring rows), and add each
-//     tile's values, scaled as the maximum moved, to f32 registers, half a row per thread (184 registers);
-//   * one issues.  The scores of the next tile follow the values of this one in the tensor pipe, and meanwhile the decoders work;
-//     what the pipe waits for is the probabilities.
+// Here the tiles of 64 positions that the rows see are decoded ONCE into an image (kv_image_kernel: K as positions x dims, V as dims x
+// positions, each value d (n - 8) exactly as two f16 terms, in the layout shared memory wants), and a block takes 128 query rows that
+// share a KV head (128 / G tokens x the head's G query heads), brings tile after tile in by bulk copies and multiplies on tcgen05 (f16
+// in, f32 out) without giving up f32 accuracy: q (scaled per row by a power of two) and the probabilities are two f16 terms each as
+// well, a product is hi hi + hi lo + lo hi.
+//   * q's first term and the probabilities lie in TENSOR memory as the A operand, q's second term and the tile in shared memory; scores
+//     and a tile's values are the accumulators (HD = 256 fills the 512 columns);
+//   * eight warps own half a row per thread: they add the values of the tile before, scaled as the maximum moved, to f32 registers while
+//     the scores of this one are made, then mask, running maximum (the two threads of a row trade theirs), probabilities;
+//   * one warp issues the products, one the copies.
 // The sums leave tensor memory after every tile and small terms come first, because the accumulator truncates: against 64 bits the
 // result is off by 1.3..1.8e-7 (2-norm) whatever the context, where accumulating on gave 3e-6 over 2047 positions, 1e-5 over 4000.
 // The context is split over blockIdx.z; (m, l, O) records go to `tmp` as the decode kernels leave them and
 // sdpa_merge_split_kernel folds them straight into the operand image of the output projection.
 //
-// Bound by the decoders, who turn a tile's values, fold the one before and turn the next one's keys in a row: 5.7 us for 128 x 64,
-// 1.2 of them MMAs (2047 rows, 2 splits: tensor pipe 21 %, issue slots 38 %).  A block takes another 18 us for its start, q and
-// records.  Back to back: one block of 64 tiles 381 us; 2047 rows of 8 heads (128 blocks of up to 32 tiles) 205 us, in two splits 118;
-// 2000 rows behind 2000 positions, 2 KV heads (126 blocks of up to 63 tiles) 388, in two splits 344.  On mma.sync (64 rows a block) the
-// last two took 336 and 809.
+// Bound by the chain of a tile: scores (48 MMAs), probabilities, values (12 MMAs of 256 columns), 3.2 us for 128 x 64.  When eight warps
+// of every block decoded its tiles it was 5.7 us, 2.2 of them waiting for keys; one thread per row of scores: 3.7.  Launches with their
+// image, back to back: 2047 rows of 8 heads (128 blocks of up to 32 tiles) 121 us, in two splits 84 (decoding in every block 205 and
+// 118); 2000 rows behind 2000 positions, 2 KV heads (126 blocks of up to 63 tiles) 218, in two splits 197 (387 and 343); 300 rows in
+// three splits 26.5 (30).
 #include "ks_gemm_common.cuh"
 
 namespace {
 
 constexpr int CH_BM = 128, CH_BN = 64;                 // query rows, positions of a tile
-constexpr int CH_ROW_WARPS = 4, CH_DEC_WARPS = 8, CH_WORK = (CH_ROW_WARPS + CH_DEC_WARPS) * 32, CH_THREADS = CH_WORK + 128;
+constexpr int CH_WORK_WARPS = 8, CH_THREADS = (CH_WORK_WARPS + 4) * 32;
 constexpr unsigned CH_WAIT = 1u << 20;
 constexpr float CH_P = 256.0f;                         // probabilities carry 2^8
 constexpr unsigned CH_K_MOST = 0x6FFFu;                // the largest scale with 8 d in f16, 8188
 constexpr float kNegInit = -1.0e30f;
 
-// barriers: operands ready (decoders, row warps), the tile's O taken (decoders), products ready (commits: scores done = K free;
-// values done = V and P free)
+// barriers: the tile's K and V there (copies), its probabilities, its O taken (workers), products ready (commits: scores done = K
+// free; values done = V and P free)
 enum { CB_K_FULL, CB_V_FULL, CB_P_FULL, CB_O_FREE, CB_S_FULL, CB_K_FREE, CB_V_FREE, CB_DONE, CB_COUNT };
 
 template <int HD>
 struct ChunkSmem {
-  static constexpr unsigned NB = HD / 32, ROWB = NB * KS_Q40_BLOCK_BYTES, RP = ROWB + 4;
-  static constexpr unsigned slot = 64, row = 128;     // tensor-memory address, failure flag; per row: scale, first, past the last position, maximum,
-                                                      // then what the sums so far are multiplied by, of two tiles
-  static constexpr unsigned up = row + CH_BM * 24;    // of two tiles: what their scores are multiplied by
-  static constexpr unsigned raw = 4096;
-  static_assert(up + 8 <= raw, "the rows' words fit in front of the packed rows");
-  static constexpr unsigned ql = (raw + 2 * CH_BN * RP + 1023u) & ~1023u, kh = ql + CH_BM * HD * 2, kl = kh + CH_BN * HD * 2, vh = kl + CH_BN * HD * 2,
+  static constexpr unsigned slot = 64, row = 128;     // tensor-memory address, failure flag; per row: scale, first, past the last position, then
+                                                      // the maxima and the sums of the two threads that share it, of two tiles
+  static constexpr unsigned ql = 4096, kh = ql + CH_BM * HD * 2, kl = kh + CH_BN * HD * 2, vh = kl + CH_BN * HD * 2,
                             vl = vh + CH_BN * HD * 2, total = vl + CH_BN * HD * 2;
+  static_assert(row + CH_BM * 28 <= ql, "the rows' words fit in front of the operands");
   static constexpr unsigned o = ql, OP = HD + 4;      // the result on its way out: rows of OP floats
   static_assert(o + CH_BM * OP * 4 <= total, "the result fits the operands");
   // tensor memory: first term of q, scores, the probabilities' two terms, O
@@ -55,17 +52,16 @@ struct ChunkSmem {
 };
 
 __device__ __forceinline__ void mb_arrive1(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
-__device__ __forceinline__ void cp4(uint32_t dst, const void* src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory"); }
-// The decoders meet; true if every one of them says so.
-__device__ __forceinline__ bool dec_all(bool ok) {
+// The two warps that share 32 query rows meet; true if every thread of both says so.
+__device__ __forceinline__ bool pair_all(unsigned quad, bool ok) {
   unsigned r;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.u32 p, %1, 0;\n\t"
-      "barrier.cta.red.and.pred q, 1, %2, p;\n\t"
+      "barrier.cta.red.and.pred q, %2, 64, p;\n\t"
       "selp.u32 %0, 1, 0, q;\n\t}"
       : "=r"(r)
-      : "r"((unsigned)ok), "n"(CH_DEC_WARPS * 32)
+      : "r"((unsigned)ok), "r"(1u + quad)
       : "memory");
   return r != 0;
 }
@@ -77,16 +73,93 @@ __device__ __forceinline__ void split_d(__half2 n, __half2 d, uint32_t& hi, uint
 }
 __device__ __forceinline__ __half2 nib_h2(uint32_t w) { return __hsub2(as_h2((w & 0x000F000Fu) | 0x64006400u), __float2half2_rn(1032.0f)); }  // nibbles 0 of bytes 0 and 2
 
-struct ChunkParts {  // part p: rows from row0[p] on, row tiles from tile0[p] on
-  unsigned n, row0[65], tile0[65], slot[64];
+struct ChunkParts {  // part p: rows from row0[p] on, row tiles from tile0[p] on; its decoded tiles start at image0[p] of the image
+  unsigned n, row0[65], tile0[65], slot[64], image0[64];
 };
+// Decoded tile t of KV head h in the image: K's first and second terms, V's, each as the kernel wants it in shared memory; behind all
+// tiles, what their scores are multiplied by.
+template <int HD>
+struct ChunkImage {
+  static constexpr unsigned HALF = 2 * CH_BN * HD * 2, TILE = 2 * HALF;  // bytes of a tile's K (V), and of both
+};
+
+// The tiles of 64 positions that some row of a part sees, decoded once for all its query tiles.  grid = (tiles, 4 n_kv, parts): a block
+// takes K or V of a tile, half the dims.
+template <int HD>
+__global__ void __launch_bounds__(256) kv_image_kernel(const __grid_constant__ ChunkParts parts, size_t slot_stride, unsigned n_kv, const uint8_t* K, const uint8_t* V,
+                                                        const float* meta, unsigned char* img, float* img_up) {
+  ks_pdl_entry();
+  constexpr unsigned NB = HD / 32, ROWB = NB * KS_Q40_BLOCK_BYTES;
+  const unsigned tid = threadIdx.x, part = blockIdx.z, kvh = blockIdx.y >> 2, half = blockIdx.y & 1u;
+  const float *m0 = meta + (size_t)parts.row0[part] * 4u, *m1 = meta + (size_t)(parts.row0[part + 1u] - 1u) * 4u;  // starts and ends grow with the row
+  const unsigned end = (unsigned)((int)m1[0] + (int)m1[1]), tile = (unsigned)(int)m0[1] / CH_BN + blockIdx.x, p0 = tile * CH_BN;
+  if (p0 >= end) return;
+  const size_t at = (size_t)(parts.image0[part] + tile) * n_kv + kvh;
+  unsigned char* out = img + at * ChunkImage<HD>::TILE;
+  const bool vals = (blockIdx.y & 2u) != 0u;
+  const uint8_t* src = (vals ? V : K) + parts.slot[part] * slot_stride + (size_t)kvh * ROWB;
+  auto row = [&](unsigned p) { return src + (size_t)min(p0 + p, end - 1u) * n_kv * ROWB; };  // (rows past the end repeat the last: their scores are masked)
+  if (!vals) {
+    // a tile with a scale whose products leave f16 is decoded at an eighth and its scores are multiplied by 8; what that rounds off
+    // (2^-22 of a value at most) is nothing beside a value of 57000
+    bool over = false;
+    for (unsigned i = tid; i < CH_BN * NB; i += 256u)
+      over |= (*reinterpret_cast<const unsigned short*>(row(i % CH_BN) + i / CH_BN * KS_Q40_BLOCK_BYTES) & 0x7FFFu) > CH_K_MOST;
+    const float up = __syncthreads_or(over) ? 8.0f : 1.0f;
+    if (tid == 0 && half == 0) img_up[at] = up;
+    const __half2 down = __float2half2_rn(1.0f / up);
+    for (unsigned job = tid; job < CH_BN * NB / 2u; job += 256u) {  // a block of a row
+      const unsigned p = job % CH_BN, b = half * (NB / 2u) + job / CH_BN;
+      const uint8_t* x = row(p) + b * KS_Q40_BLOCK_BYTES;
+      const __half2 d = __hmul2(__half2half2(__ushort_as_half(*reinterpret_cast<const unsigned short*>(x))), down);
+      uint32_t w[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        w[k] = *reinterpret_cast<const unsigned short*>(x + 2 + 4 * k) | (uint32_t)*reinterpret_cast<const unsigned short*>(x + 4 + 4 * k) << 16;
+#pragma unroll
+      for (int hn = 0; hn < 2; hn++)  // dims 0..15 of the block are the low nibbles
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+          uint32_t hi[4], lo[4];
+#pragma unroll
+          for (int k = 0; k < 2; k++) {
+            const uint32_t v = hn ? w[2 * c + k] >> 4 : w[2 * c + k];
+            split_d(nib_h2(__byte_perm(v, 0u, 0x4140)), d, hi[2 * k], lo[2 * k]);
+            split_d(nib_h2(__byte_perm(v, 0u, 0x4342)), d, hi[2 * k + 1], lo[2 * k + 1]);
+          }
+          unsigned char* o = out + ((4u * b + 2u * hn + c) * CH_BN + p) * 16u;
+          *reinterpret_cast<uint4*>(o) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+          *reinterpret_cast<uint4*>(o + ChunkImage<HD>::HALF / 2u) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        }
+    }
+    return;
+  }
+  out += ChunkImage<HD>::HALF;
+  for (unsigned job = tid; job < 16u * (NB / 2u) * (CH_BN / 8); job += 256u) {  // byte j of a block in eight neighbouring rows
+    const unsigned j = job % 16u, b = half * (NB / 2u) + job / 16u % (NB / 2u), pg = job / (16u * (NB / 2u));
+    uint32_t hl[4], ll[4], hh[4], lh[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const uint8_t *x = row(8u * pg + 2u * k) + b * KS_Q40_BLOCK_BYTES, *y = row(8u * pg + 2u * k + 1u) + b * KS_Q40_BLOCK_BYTES;
+      const uint32_t n = x[2 + j] | (uint32_t)y[2 + j] << 16;
+      const __half2 d = as_h2(*reinterpret_cast<const unsigned short*>(x) | (uint32_t)*reinterpret_cast<const unsigned short*>(y) << 16);
+      split_d(nib_h2(n), d, hl[k], ll[k]);
+      split_d(nib_h2(n >> 4), d, hh[k], lh[k]);
+    }
+    unsigned char* o = out + (pg * HD + 32u * b + j) * 16u;
+    *reinterpret_cast<uint4*>(o) = make_uint4(hl[0], hl[1], hl[2], hl[3]);
+    *reinterpret_cast<uint4*>(o + 256u) = make_uint4(hh[0], hh[1], hh[2], hh[3]);
+    *reinterpret_cast<uint4*>(o + ChunkImage<HD>::HALF / 2u) = make_uint4(ll[0], ll[1], ll[2], ll[3]);
+    *reinterpret_cast<uint4*>(o + ChunkImage<HD>::HALF / 2u + 256u) = make_uint4(lh[0], lh[1], lh[2], lh[3]);
+  }
+}
 
 template <int HD>
 __global__ void __launch_bounds__(CH_THREADS, 1)
-sdpa_chunk_kernel(const __grid_constant__ ChunkParts parts, size_t slot_stride, unsigned n_q, unsigned n_kv, float scale, const float* q, const uint8_t* K,
-                  const uint8_t* V, const float* meta, float* tmp, unsigned n_splits, unsigned* err) {
+sdpa_chunk_kernel(const __grid_constant__ ChunkParts parts, unsigned n_q, unsigned n_kv, float scale, const float* q, const float* meta, float* tmp, unsigned n_splits,
+                  const unsigned char* img, const float* img_up, unsigned* err) {
   using S = ChunkSmem<HD>;
-  constexpr unsigned NB = S::NB, RP = S::RP, ROWB = S::ROWB;
+  using Image = ChunkImage<HD>;
   extern __shared__ __align__(1024) unsigned char smem[];
   ks_pdl_entry();
   const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -98,8 +171,6 @@ sdpa_chunk_kernel(const __grid_constant__ ChunkParts parts, size_t slot_stride, 
   q += (size_t)first_tok * n_q * HD;  // from here on rows are counted inside the part
   meta += (size_t)first_tok * 4u;
   tmp += (size_t)first_tok * n_q * n_splits * (HD + 2);
-  K += parts.slot[part_id] * slot_stride;
-  V += parts.slot[part_id] * slot_stride;
   const uint32_t sb = sm32(smem);
   auto bar = [&](unsigned i) { return sb + 8u * i; };
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smem + S::slot);
@@ -107,13 +178,11 @@ sdpa_chunk_kernel(const __grid_constant__ ChunkParts parts, size_t slot_stride, 
   float* row_scale = reinterpret_cast<float*>(smem + S::row);
   int* row_first = reinterpret_cast<int*>(smem + S::row + CH_BM * 4);
   int* row_end = reinterpret_cast<int*>(smem + S::row + CH_BM * 8);
-  unsigned* row_max = reinterpret_cast<unsigned*>(smem + S::row + CH_BM * 12);
-  float* row_alpha = reinterpret_cast<float*>(smem + S::row + CH_BM * 16);
-  float* tile_up = reinterpret_cast<float*>(smem + S::up);
+  float* row_max = reinterpret_cast<float*>(smem + S::row + CH_BM * 12);  // [2 tiles][2 halves][CH_BM]
 
   // ---- the block's rows: row r is query head kvh G + r % G of token (row0 + r) / G; positions they see at all
   const unsigned tok_a = row0 / G, tok_b = min((row0 + CH_BM - 1u) / G, n_tok - 1u);
-  const int pmin = (int)meta[tok_a * 4 + 1];                                        // starts and ends grow with the token
+  const int pmin = (int)meta[tok_a * 4 + 1] & ~(CH_BN - 1);                         // starts and ends grow with the token; tiles start at multiples of 64
   const int pmax = (int)meta[tok_b * 4 + 0] + (int)meta[tok_b * 4 + 1];
   const int span = (pmax - pmin + CH_BN - 1) / CH_BN, per = (span + (int)n_splits - 1) / (int)n_splits;
   const int t_begin = pmin + (int)split * per * CH_BN, t_end = min(pmin + (int)(split + 1u) * per * CH_BN, pmax);
@@ -125,145 +194,145 @@ sdpa_chunk_kernel(const __grid_constant__ ChunkParts parts, size_t slot_stride, 
     }
     return;
   }
-  const bool decoder = warp >= CH_ROW_WARPS && warp < CH_ROW_WARPS + CH_DEC_WARPS;
-  const unsigned dt = tid - CH_ROW_WARPS * 32;  // decoders: 0..255
-  auto fetch = [&](int t0) {  // the packed rows of positions t0 .. +64 (rows past the end repeat the last, their scores are masked)
-    for (unsigned r = dt >> 5; r < 2u * CH_BN; r += CH_DEC_WARPS) {
-      const int pos = min(t0 + (int)(r & (CH_BN - 1u)), pmax - 1);
-      const uint8_t* src = (r < CH_BN ? K : V) + ((size_t)pos * n_kv + kvh) * ROWB;
-      const uint32_t dst = sb + S::raw + r * RP;
-      for (unsigned w = lane; w < ROWB / 4u; w += 32u) cp4(dst + 4u * w, src + 4u * w);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  // The largest scale (its f16 bits) of the K rows this thread copied.  Block b's scale is half of word 18 b / 4, and those words are
-  // all among a lane's first.
-  static_assert((NB - 1u) * KS_Q40_BLOCK_BYTES < 128u, "scales lie in the first 32 words of a row");
-  const unsigned scale_at = (lane * 4u + KS_Q40_BLOCK_BYTES - 1u) / KS_Q40_BLOCK_BYTES * KS_Q40_BLOCK_BYTES;
-  const bool has_scale = scale_at < lane * 4u + 4u && scale_at < ROWB;
-  const unsigned scale_off = S::raw + ((warp - CH_ROW_WARPS) & (CH_DEC_WARPS - 1u)) * RP + (has_scale ? scale_at : lane * 4u);
-  auto most_scale = [&] {
-    unsigned m = 0;
-#pragma unroll
-    for (unsigned k = 0; k < CH_BN / CH_DEC_WARPS; k++) {
-      const unsigned d = *reinterpret_cast<const unsigned short*>(smem + scale_off + k * CH_DEC_WARPS * RP) & 0x7FFFu;
-      m = d > m ? d : m;
-    }
-    return has_scale ? m : 0u;
-  };
-  if (decoder) fetch(t_begin);
+  const size_t img_at = (size_t)(parts.image0[part_id] + (unsigned)t_begin / CH_BN) * n_kv + kvh;  // tiles are n_kv apart
 
   if (tid == 0) {
-    mb_init(bar(CB_K_FULL), CH_DEC_WARPS);
-    mb_init(bar(CB_V_FULL), CH_DEC_WARPS);
-    mb_init(bar(CB_P_FULL), CH_ROW_WARPS);
-    mb_init(bar(CB_O_FREE), CH_DEC_WARPS);
+    mb_init(bar(CB_K_FULL), 1);
+    mb_init(bar(CB_V_FULL), 1);
+    mb_init(bar(CB_P_FULL), CH_WORK_WARPS);
+    mb_init(bar(CB_O_FREE), CH_WORK_WARPS);
     for (unsigned i = CB_S_FULL; i < CB_COUNT; i++) mb_init(bar(i), 1);
     *fail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (tid < CH_BM) row_max[tid] = 0u;
-  if (warp == CH_ROW_WARPS + CH_DEC_WARPS) tc_alloc(sm32(tslot), 512);
-  __syncthreads();
+  if (warp == CH_WORK_WARPS) tc_alloc(sm32(tslot), 512);
 
-  // ---- q: a thread takes every third chunk of 8 dims of a row; the row maximum sets a power of two, then two f16 terms per value.
-  // The second term stays in shared memory as core matrices, the first passes through there (K's place) to tensor memory.
-  {
-    constexpr unsigned PARTS = CH_WORK / CH_BM, PER = (HD / 8 + PARTS - 1) / PARTS;
-    const unsigned r = tid % CH_BM, part = tid / CH_BM, t = (row0 + r) / G, head = kvh * G + (row0 + r) % G;
-    float v[PER][8];
-    float m = 0.0f;
-    if (tid < CH_WORK) {
-      const float* src = q + ((size_t)t * n_q + head) * HD;
+  // ---- q: a warp takes eight rows at a time, lane = row lane % 8, chunk of 8 dims lane / 8 (+ 4 a step): a load touches 128 neighbouring
+  // bytes of eight rows, a store 128 bytes of a chunk.  The row maximum sets a power of two, then two f16 terms per value: the second
+  // stays in shared memory as core matrices, the first passes through there (K's place) to tensor memory.
+  for (unsigned grp = warp; grp < CH_BM / 8; grp += CH_THREADS / 32) {
+    constexpr int STEPS = HD / 32;
+    const unsigned r = grp * 8u + (lane & 7u), t = (row0 + r) / G, head = kvh * G + (row0 + r) % G;
+    const float* src = q + ((size_t)t * n_q + head) * HD + 8u * (lane >> 3);
+    float v[STEPS][8], m = 0.0f;
 #pragma unroll
-      for (unsigned k = 0; k < PER; k++) {
-        const unsigned c = part + k * PARTS;
-        const bool in = c < HD / 8u && t < n_tok;
-        const float4 a = in ? *reinterpret_cast<const float4*>(src + 8u * c) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 b = in ? *reinterpret_cast<const float4*>(src + 8u * c + 4u) : make_float4(0.f, 0.f, 0.f, 0.f);
-        v[k][0] = a.x; v[k][1] = a.y; v[k][2] = a.z; v[k][3] = a.w;
-        v[k][4] = b.x; v[k][5] = b.y; v[k][6] = b.z; v[k][7] = b.w;
-        m = fmaxf(m, absmax8(v[k]));
-      }
-      atomicMax(row_max + r, __float_as_uint(m));
+    for (int k = 0; k < STEPS; k++) {
+      const float4 a = t < n_tok ? *reinterpret_cast<const float4*>(src + 32 * k) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 b = t < n_tok ? *reinterpret_cast<const float4*>(src + 32 * k + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+      v[k][0] = a.x; v[k][1] = a.y; v[k][2] = a.z; v[k][3] = a.w;
+      v[k][4] = b.x; v[k][5] = b.y; v[k][6] = b.z; v[k][7] = b.w;
     }
-    __syncthreads();
-    if (tid < CH_WORK) {
-      float up;
-      const float down = row_scale_down(__uint_as_float(row_max[r]), &up);
-      if (part == 0) {
-        row_scale[r] = up * scale;
-        row_first[r] = t < n_tok ? (int)meta[t * 4 + 1] : 0;
-        row_end[r] = t < n_tok ? (int)meta[t * 4 + 1] + (int)meta[t * 4 + 0] : 0;
-      }
 #pragma unroll
-      for (unsigned k = 0; k < PER; k++) {
-        const unsigned c = part + k * PARTS;
-        if (c < HD / 8u) {
-#pragma unroll
-          for (int e = 0; e < 8; e++) v[k][e] *= down;
-          uint4 hi, lo;
-          split8(v[k], hi, lo);
-          *reinterpret_cast<uint4*>(smem + S::kh + (c * CH_BM + r) * 16u) = hi;
-          *reinterpret_cast<uint4*>(smem + S::ql + (c * CH_BM + r) * 16u) = lo;
-        }
-      }
+    for (int k = 0; k < STEPS; k++) m = fmaxf(m, absmax8(v[k]));
+    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
+    float up;
+    const float down = row_scale_down(m, &up);
+    if (lane < 8u) {
+      row_scale[r] = up * scale;
+      row_first[r] = t < n_tok ? (int)meta[t * 4 + 1] : 0;
+      row_end[r] = t < n_tok ? (int)meta[t * 4 + 1] + (int)meta[t * 4 + 0] : 0;
     }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+#pragma unroll
+    for (int k = 0; k < STEPS; k++) {
+#pragma unroll
+      for (int e = 0; e < 8; e++) v[k][e] *= down;
+      uint4 hi, lo;
+      split8(v[k], hi, lo);
+      const unsigned at = ((4u * k + (lane >> 3)) * CH_BM + r) * 16u;
+      *reinterpret_cast<uint4*>(smem + S::kh + at) = hi;
+      *reinterpret_cast<uint4*>(smem + S::ql + at) = lo;
+    }
   }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncthreads();
   const uint32_t tmem = *tslot;
   if (tmem != 0u && tid == 0) *fail = 1;  // all 512 columns were asked for: they start at 0
-  const uint32_t tlane = (warp & 3u) << 21;   // 32 rows per warp, in the address bits of the lane
-  if (warp < CH_ROW_WARPS) {
+  const unsigned quad = warp & 3u, half = warp >> 2 & 1u, row = quad * 32u + lane;  // workers: half the columns of a row
+  const uint32_t tlane = quad << 21;      // 32 rows per warp, in the address bits of the lane
+  if (warp < CH_WORK_WARPS) {
 #pragma unroll
-    for (unsigned c = 0; c < HD / 8u; c += 2u) {
-      const uint4 a = *reinterpret_cast<const uint4*>(smem + S::kh + (c * CH_BM + tid) * 16u), b = *reinterpret_cast<const uint4*>(smem + S::kh + ((c + 1u) * CH_BM + tid) * 16u);
+    for (unsigned k = 0; k < HD / 16u; k += 2u) {
+      const unsigned c = half * (HD / 16u) + k;
+      const uint4 a = *reinterpret_cast<const uint4*>(smem + S::kh + (c * CH_BM + row) * 16u), b = *reinterpret_cast<const uint4*>(smem + S::kh + ((c + 1u) * CH_BM + row) * 16u);
       const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
       tc_st8(tlane + S::t_q + c * 4u, w);
     }
     tc_wait_st();
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // K's place has been read: the first copy may write it
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
 
-  if (warp < CH_ROW_WARPS) {
-    // ---- a row of scores per thread
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 120;");
-    const float sc = row_scale[tid];
-    const int first = row_first[tid], end = row_end[tid];
-    float ref = kNegInit, l = 0.0f;
+  if (warp < CH_WORK_WARPS) {
+    // ---- half a row per thread: the tile before's values into f32 registers, then this tile's scores -> probabilities
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 232;");
+    constexpr unsigned HALF = HD / 2;
+    const float sc = row_scale[row];
+    const int first = row_first[row], end = row_end[row];
+    float acc[HALF], ref = kNegInit, l = 0.0f, alpha = 1.0f;
+#pragma unroll
+    for (unsigned c = 0; c < HALF; c++) acc[c] = 0.0f;
+    auto fold = [&] {
+      tc_fence_after();
+#pragma unroll
+      for (unsigned c = 0; c < HALF; c += 32u) {
+        uint32_t o[2][16];
+        tc_ld16(tlane + S::t_o + half * HALF + c, o[0]);
+        tc_ld16(tlane + S::t_o + half * HALF + c + 16u, o[1]);
+        tc_wait_ld16(o[0]);
+        tc_wait_ld16(o[1]);
+#pragma unroll
+        for (unsigned e = 0; e < 32u; e++) acc[c + e] = fmaf(acc[c + e], alpha, __uint_as_float(o[e / 16u][e % 16u]));
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mb_arrive1(bar(CB_O_FREE));
+    };
     bool ok = true;
     for (unsigned i = 0; i < n_tiles; i++) {
-      if (!__all_sync(0xffffffffu, mb_wait(bar(CB_S_FULL), i & 1u, CH_WAIT))) { ok = false; break; }
-      tc_fence_after();
-      uint32_t s[4][16];
-#pragma unroll
-      for (int k = 0; k < 4; k++) tc_ld16(tlane + S::t_s + 16u * k, s[k]);
-#pragma unroll
-      for (int k = 0; k < 4; k++) tc_wait_ld16(s[k]);
-      const int p0 = t_begin + (int)i * CH_BN, a = first - p0, b = min(end, t_end) - p0;  // columns [a, b) are seen
-      const float st = sc * tile_up[i & 1u];
+      const float up = img_up[img_at + (size_t)i * n_kv];
+      if (i > 0) {  // the scores of this tile are made meanwhile
+        ok = __all_sync(0xffffffffu, mb_wait(bar(CB_V_FREE), (i - 1u) & 1u, CH_WAIT));
+        if (ok) fold();
+      }
+      ok = ok && __all_sync(0xffffffffu, mb_wait(bar(CB_S_FULL), i & 1u, CH_WAIT));
       float mx = -INFINITY;
-#pragma unroll
-      for (int j = 0; j < CH_BN; j++) {
-        const float x = j >= a && j < b ? __uint_as_float(s[j / 16][j % 16]) * st : -INFINITY;
-        s[j / 16][j % 16] = __float_as_uint(x);
-        mx = fmaxf(mx, x);
-      }
-      mx = fmaxf(mx, ref);
-      const float alpha = __expf(ref - mx);
-      ref = mx;
-      row_alpha[(i & 1u) * CH_BM + tid] = alpha;
-      if (i > 0) {  // P is free
-        if (!__all_sync(0xffffffffu, mb_wait(bar(CB_V_FREE), (i - 1u) & 1u, CH_WAIT))) { ok = false; break; }
+      uint32_t s[2][16];
+      if (ok) {
         tc_fence_after();
+        tc_ld16(tlane + S::t_s + half * 32u, s[0]);
+        tc_ld16(tlane + S::t_s + half * 32u + 16u, s[1]);
+        tc_wait_ld16(s[0]);
+        tc_wait_ld16(s[1]);
+        const int p0 = t_begin + (int)i * CH_BN + (int)half * 32, a = first - p0, b = min(end, t_end) - p0;  // columns [a, b) are seen
+        const float st = sc * up;
+        if (__all_sync(0xffffffffu, a <= 0 && b >= 32)) {
+#pragma unroll
+          for (int j = 0; j < 32; j++) {
+            const float x = __uint_as_float(s[j / 16][j % 16]) * st;
+            s[j / 16][j % 16] = __float_as_uint(x);
+            mx = fmaxf(mx, x);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; j++) {
+            const float x = j >= a && j < b ? __uint_as_float(s[j / 16][j % 16]) * st : -INFINITY;
+            s[j / 16][j % 16] = __float_as_uint(x);
+            mx = fmaxf(mx, x);
+          }
+        }
+        row_max[((i & 1u) * 2u + half) * CH_BM + row] = mx;
       }
+      if (!pair_all(quad, ok)) { ok = false; break; }
+      mx = fmaxf(fmaxf(mx, row_max[((i & 1u) * 2u + (half ^ 1u)) * CH_BM + row]), ref);
+      alpha = __expf(ref - mx);
+      ref = mx;
       float sum = 0.0f;
 #pragma unroll
-      for (int k = 0; k < 4; k++) {
+      for (int k = 0; k < 2; k++) {
         uint32_t ph[8], pl[8];
 #pragma unroll
         for (int j = 0; j < 8; j++) {  // a masked score is -infinity: its probability is 0 whatever the maximum
@@ -274,8 +343,8 @@ sdpa_chunk_kernel(const __grid_constant__ ChunkParts parts, size_t slot_stride, 
           ph[j] = pack_h2(h);
           pl[j] = pack_h2(__floats2half2_rn(x * CH_P - f.x, y * CH_P - f.y));
         }
-        tc_st8(tlane + S::t_ph + 8u * k, ph);
-        tc_st8(tlane + S::t_pl + 8u * k, pl);
+        tc_st8(tlane + S::t_ph + half * 16u + 8u * k, ph);
+        tc_st8(tlane + S::t_pl + half * 16u + 8u * k, pl);
       }
       l = l * alpha + sum;
       tc_wait_st();
@@ -283,117 +352,20 @@ sdpa_chunk_kernel(const __grid_constant__ ChunkParts parts, size_t slot_stride, 
       __syncwarp();
       if (lane == 0) mb_arrive1(bar(CB_P_FULL));
     }
-    if (!ok && lane == 0) *fail = 1;
-    row_scale[tid] = ref;
-    reinterpret_cast<float*>(row_max)[tid] = l;
-  } else if (decoder) {
-    // ---- packed rows -> two f16 terms of K (positions x dims) and of V transposed (dims x positions); a tile's values are added to
-    // half a row per thread
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 184;");
-    constexpr unsigned HALF = HD / 2;
-    const unsigned orow = (warp & 3u) * 32u + lane, ocol = (warp >> 2 & 1u) * HALF;  // (warps 4..7 and 8..11)
-    float acc[HALF];
-#pragma unroll
-    for (unsigned c = 0; c < HALF; c++) acc[c] = 0.0f;
-    auto fold = [&](unsigned i) {
-      tc_fence_after();
-      const float alpha = row_alpha[(i & 1u) * CH_BM + orow];
-#pragma unroll
-      for (unsigned c = 0; c < HALF; c += 16u) {
-        uint32_t o[16];
-        tc_ld16(tlane + S::t_o + ocol + c, o);
-        tc_wait_ld16(o);
-#pragma unroll
-        for (unsigned e = 0; e < 16u; e++) acc[c + e] = fmaf(acc[c + e], alpha, __uint_as_float(o[e]));
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mb_arrive1(bar(CB_O_FREE));
-    };
-    bool ok = true;
-    for (unsigned i = 0; i < n_tiles; i++) {
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      const bool fits = most_scale() <= CH_K_MOST;
-      if (i > 0) ok = mb_wait(bar(CB_K_FREE), (i - 1u) & 1u, CH_WAIT);
-      // The raw rows are there, K is free.  A tile with a scale whose products leave f16 is decoded at an eighth and its scores are
-      // multiplied by 8; what that rounds off (2^-22 of a value at most) is nothing beside a value of 57000.  Every thread looks at
-      // the scales that it copied itself.
-      float tile = 1.0f;
-      if (!dec_all(ok && fits)) {
-        if (!dec_all(ok)) { ok = false; break; }
-        tile = 8.0f;
-      }
-      const __half2 down = __float2half2_rn(1.0f / tile);
-#pragma unroll 1
-      for (unsigned job = dt; job < CH_BN * NB; job += CH_DEC_WARPS * 32) {  // a block of a row
-        const unsigned p = job % CH_BN, b = job / CH_BN;
-        const unsigned char* src = smem + S::raw + p * RP + b * KS_Q40_BLOCK_BYTES;
-        const __half2 d = __hmul2(__half2half2(__ushort_as_half(*reinterpret_cast<const unsigned short*>(src))), down);
-        uint32_t w[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-          w[k] = *reinterpret_cast<const unsigned short*>(src + 2 + 4 * k) | (uint32_t)*reinterpret_cast<const unsigned short*>(src + 4 + 4 * k) << 16;
-#pragma unroll 1
-        for (int half = 0; half < 2; half++)  // dims 0..15 of the block are the low nibbles
-#pragma unroll
-          for (int c = 0; c < 2; c++) {
-            uint32_t hi[4], lo[4];
-#pragma unroll
-            for (int k = 0; k < 2; k++) {
-              const uint32_t x = half ? w[2 * c + k] >> 4 : w[2 * c + k];
-              split_d(nib_h2(__byte_perm(x, 0u, 0x4140)), d, hi[2 * k], lo[2 * k]);
-              split_d(nib_h2(__byte_perm(x, 0u, 0x4342)), d, hi[2 * k + 1], lo[2 * k + 1]);
-            }
-            const unsigned at = ((4u * b + 2u * half + c) * CH_BN + p) * 16u;
-            *reinterpret_cast<uint4*>(smem + S::kh + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            *reinterpret_cast<uint4*>(smem + S::kl + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-          }
-      }
-      if (dt == 0) tile_up[i & 1u] = tile;
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mb_arrive1(bar(CB_K_FULL));
-      if (i > 0) ok = mb_wait(bar(CB_V_FREE), (i - 1u) & 1u, CH_WAIT);
-      if (!dec_all(ok)) { ok = false; break; }
-      if (i > 0) fold(i - 1u);
-#pragma unroll 1
-      for (unsigned job = dt; job < 16u * NB * (CH_BN / 8); job += CH_DEC_WARPS * 32) {  // byte j of a block in eight neighbouring rows
-        const unsigned j = job % 16u, b = job / 16u % NB, pg = job / (16u * NB);
-        const unsigned char* src = smem + S::raw + (CH_BN + 8u * pg) * RP + b * KS_Q40_BLOCK_BYTES;
-        uint32_t hl[4], ll[4], hh[4], lh[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          const unsigned char *x = src + 2 * k * RP, *y = x + RP;
-          const uint32_t n = x[2 + j] | (uint32_t)y[2 + j] << 16;
-          const __half2 d = as_h2(*reinterpret_cast<const unsigned short*>(x) | (uint32_t)*reinterpret_cast<const unsigned short*>(y) << 16);
-          split_d(nib_h2(n), d, hl[k], ll[k]);
-          split_d(nib_h2(n >> 4), d, hh[k], lh[k]);
-        }
-        const unsigned at = (pg * HD + 32u * b + j) * 16u;
-        *reinterpret_cast<uint4*>(smem + S::vh + at) = make_uint4(hl[0], hl[1], hl[2], hl[3]);
-        *reinterpret_cast<uint4*>(smem + S::vl + at) = make_uint4(ll[0], ll[1], ll[2], ll[3]);
-        *reinterpret_cast<uint4*>(smem + S::vh + at + 256u) = make_uint4(hh[0], hh[1], hh[2], hh[3]);
-        *reinterpret_cast<uint4*>(smem + S::vl + at + 256u) = make_uint4(lh[0], lh[1], lh[2], lh[3]);
-      }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mb_arrive1(bar(CB_V_FULL));
-      if (!dec_all(true)) break;  // (meets only: the raw rows are used up)
-      if (i + 1u < n_tiles) fetch(t_begin + (int)(i + 1u) * CH_BN);
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
     ok = ok && __all_sync(0xffffffffu, mb_wait(bar(CB_V_FREE), (n_tiles - 1u) & 1u, CH_WAIT));
     if (!ok && lane == 0) *fail = 1;
     if (ok) {  // the rows through shared memory, so that they leave in whole lines; every product that read it is done
-      fold(n_tiles - 1u);
-      float* out = reinterpret_cast<float*>(smem + S::o) + orow * S::OP + ocol;
+      fold();
+      float* out = reinterpret_cast<float*>(smem + S::o) + row * S::OP + half * HALF;
 #pragma unroll
       for (unsigned c = 0; c < HALF; c += 4u)
         *reinterpret_cast<float4*>(out + c) = make_float4(acc[c] * (1.0f / CH_P), acc[c + 1] * (1.0f / CH_P), acc[c + 2] * (1.0f / CH_P), acc[c + 3] * (1.0f / CH_P));
+      row_max[((n_tiles & 1u) * 2u + half) * CH_BM + row] = l;  // (the tile before's maxima have been read by both)
+      if (half == 0) row_scale[row] = ref;
     }
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
-    if (warp == CH_ROW_WARPS + CH_DEC_WARPS) {
+    if (warp == CH_WORK_WARPS) {
     // ---- products: the whole warp runs the loop, one elected lane issues; the trip count out of a warp reduction, so that it and
     // the descriptors stay in uniform registers
     const unsigned leader = elect_one(), tiles = __reduce_max_sync(0xffffffffu, n_tiles);
@@ -443,6 +415,32 @@ sdpa_chunk_kernel(const __grid_constant__ ChunkParts parts, size_t slot_stride, 
     }
     __syncwarp();
     mb_wait(bar(CB_DONE), 0u, CH_WAIT);
+    } else if (warp == CH_WORK_WARPS + 1) {
+    // ---- decoded tiles: K of the next one when its scores are made, V when its values are
+    const unsigned leader = elect_one();
+    constexpr unsigned BYTES = Image::HALF;
+    const unsigned char* src = img + img_at * Image::TILE;
+    unsigned ks = 0, vs = 0;  // copies sent
+    for (unsigned i = 0; i < n_tiles; i++) {
+      if (i > 0 && !__all_sync(0xffffffffu, mb_wait(bar(CB_K_FREE), (i - 1u) & 1u, CH_WAIT))) break;
+      if (leader) {
+        mb_expect(bar(CB_K_FULL), BYTES);
+        bulk_in(sb + S::kh, src, BYTES, bar(CB_K_FULL));
+      }
+      ks++;
+      if (i > 0 && !__all_sync(0xffffffffu, mb_wait(bar(CB_V_FREE), (i - 1u) & 1u, CH_WAIT))) break;
+      if (leader) {
+        mb_expect(bar(CB_V_FULL), BYTES);
+        bulk_in(sb + S::vh, src + BYTES, BYTES, bar(CB_V_FULL));
+      }
+      vs++;
+      src += (size_t)n_kv * Image::TILE;
+      __syncwarp();
+    }
+    if ((ks < n_tiles || vs < n_tiles) && leader) *fail = 1;
+    // the copies must have landed before this block's shared memory goes away (bounded)
+    if (ks) mb_wait(bar(CB_K_FULL), (ks - 1u) & 1u, CH_WAIT);
+    if (vs) mb_wait(bar(CB_V_FULL), (vs - 1u) & 1u, CH_WAIT);
     }
   }
   tc_fence_before();
@@ -457,11 +455,12 @@ sdpa_chunk_kernel(const __grid_constant__ ChunkParts parts, size_t slot_stride, 
       float* rec = tmp + (((size_t)t * n_q + head) * n_splits + split) * (HD + 2);
       const float2* o = reinterpret_cast<const float2*>(smem + S::o) + r * (S::OP / 2);
       for (unsigned d = lane; d < HD / 2u; d += 32u) *reinterpret_cast<float2*>(rec + 2 + 2u * d) = o[d];
-      if (lane == 0) *reinterpret_cast<float2*>(rec) = make_float2(row_scale[r], reinterpret_cast<float*>(row_max)[r]);
+      const float* sums = row_max + (n_tiles & 1u) * 2u * CH_BM + r;
+      if (lane == 0) *reinterpret_cast<float2*>(rec) = make_float2(row_scale[r], sums[0] + sums[CH_BM]);
     }
   }
   __syncthreads();
-  if (warp == CH_ROW_WARPS + CH_DEC_WARPS) tc_dealloc(tmem, 512);
+  if (warp == CH_WORK_WARPS) tc_dealloc(tmem, 512);
 }
 
 // The (m, l, O) records of a token's heads -> the image the output projection reads its rows from (lower.rs:5897-6088 and
@@ -553,7 +552,7 @@ __global__ void __launch_bounds__(512) sdpa_merge_split_kernel(unsigned n_tok, u
 
 template <int HD>
 int launch_chunk(ks_ctx* ctx, dim3 grid, const ChunkParts& parts, size_t slot_stride, unsigned n_q, unsigned n_kv, float scale, const float* q, const uint8_t* K, const uint8_t* V,
-                 const float* meta, float* tmp, unsigned n_splits) {
+                 const float* meta, float* tmp, unsigned n_splits, const ks_kv_image& image) {
   constexpr size_t smem = ChunkSmem<HD>::total;
   static bool set[16] = {false};
   if (!set[ctx->device & 15]) {
@@ -561,7 +560,12 @@ int launch_chunk(ks_ctx* ctx, dim3 grid, const ChunkParts& parts, size_t slot_st
     if (e != cudaSuccess) return ks_fail(ctx, KS_ERR_CUDA, "sdpa_chunk: cannot set %zu B shared memory: %s", smem, cudaGetErrorString(e));
     set[ctx->device & 15] = true;
   }
-  KS_LAUNCH(ctx, sdpa_chunk_kernel<HD>, grid, CH_THREADS, smem, parts, slot_stride, n_q, n_kv, scale, q, K, V, meta, tmp, n_splits,
+  unsigned char* img = (unsigned char*)image.base;
+  float* img_up = (float*)(img + image.tiles * n_kv * (size_t)ChunkImage<HD>::TILE);
+  KS_LAUNCH(ctx, (kv_image_kernel<HD>), dim3(image.span, 4u * n_kv, parts.n), 256, 0, parts, slot_stride, n_kv, K, V, meta, img, img_up);
+  const int rc = ks_after_launch(ctx, "kv_image");
+  if (rc) return rc;
+  KS_LAUNCH(ctx, sdpa_chunk_kernel<HD>, grid, CH_THREADS, smem, parts, n_q, n_kv, scale, q, meta, tmp, n_splits, (const unsigned char*)img, (const float*)img_up,
             (unsigned*)ctx->ws + KS_WS_ERR_WORD);
   return ks_after_launch(ctx, "sdpa_chunk");
 }
@@ -587,10 +591,13 @@ bool ks_sdpa_chunk_covers(size_t n_q, size_t n_kv, size_t hd, const void* K, con
   return (hd == 256 || hd == 128) && G <= 16 && CH_BM % G == 0 && ks_sdpa_merge_split_covers(n_q, hd) && (((uintptr_t)K | (uintptr_t)V) & 3u) == 0;
 }
 
+size_t ks_kv_image_bytes(size_t tiles, size_t n_kv, size_t hd) { return tiles * n_kv * (hd == 256 ? ChunkImage<256>::TILE : ChunkImage<128>::TILE) + tiles * n_kv * sizeof(float); }
+unsigned ks_kv_image_tiles(size_t positions) { return (unsigned)((positions + CH_BN - 1) / CH_BN); }
+
 // q [n_tok, n_q hd] f32, meta [n_tok][4] = (tlen, start, -, -) with both ends growing along the rows of a slot
 // -> records in tmp [n_tok][n_q][n_splits][hd + 2].
 int ks_launch_sdpa_chunk(ks_ctx* ctx, int n_tok, size_t n_q, size_t n_kv, size_t hd, float scale, const float* q, const uint8_t* K, const uint8_t* V,
-                         const float* meta, float* tmp, int n_splits, const ks_row_parts* parts, size_t slot_stride) {
+                         const float* meta, float* tmp, int n_splits, const ks_kv_image& image, const ks_row_parts* parts, size_t slot_stride) {
   ChunkParts cp{};
   cp.n = parts ? parts->n : 1u;
   unsigned tiles = 0;
@@ -598,13 +605,14 @@ int ks_launch_sdpa_chunk(ks_ctx* ctx, int n_tok, size_t n_q, size_t n_kv, size_t
     cp.row0[p] = parts ? parts->row0[p] : 0u;
     cp.row0[p + 1] = parts ? parts->row0[p + 1] : (unsigned)n_tok;
     cp.slot[p] = parts ? parts->slot[p] : 0u;
+    cp.image0[p] = parts ? parts->image0[p] : 0u;
     cp.tile0[p] = tiles;
     tiles += (unsigned)(((cp.row0[p + 1] - cp.row0[p]) * (n_q / n_kv) + CH_BM - 1) / CH_BM);
   }
   cp.tile0[cp.n] = tiles;
   const dim3 grid(tiles, (unsigned)n_kv, (unsigned)n_splits);
-  return hd == 256 ? launch_chunk<256>(ctx, grid, cp, slot_stride, (unsigned)n_q, (unsigned)n_kv, scale, q, K, V, meta, tmp, (unsigned)n_splits)
-                   : launch_chunk<128>(ctx, grid, cp, slot_stride, (unsigned)n_q, (unsigned)n_kv, scale, q, K, V, meta, tmp, (unsigned)n_splits);
+  return hd == 256 ? launch_chunk<256>(ctx, grid, cp, slot_stride, (unsigned)n_q, (unsigned)n_kv, scale, q, K, V, meta, tmp, (unsigned)n_splits, image)
+                   : launch_chunk<128>(ctx, grid, cp, slot_stride, (unsigned)n_q, (unsigned)n_kv, scale, q, K, V, meta, tmp, (unsigned)n_splits, image);
 }
 
 // Records of n_tok rows -> the Q4_K form of the operand image (rows past n_tok as zeros).
@@ -628,12 +636,18 @@ extern "C" int ks_debug_sdpa_chunk(ks_ctx* ctx, size_t n_q, size_t n_kv, size_t 
     KS_REQUIRE(ctx, row0[p + 1] > row0[p] && row0[p + 1] <= KS_GEMM_ROWS && slots[p] >= 0, "sdpa_chunk: bad parts");
     parts.row0[p + 1] = (unsigned)row0[p + 1];
     parts.slot[p] = (unsigned)slots[p];
+    parts.image0[p] = (unsigned)p * ks_kv_image_tiles(max_t);
     last = (size_t)slots[p] > last ? (size_t)slots[p] : last;
   }
   const size_t n = (size_t)row0[n_parts], need = last * slot_stride_bytes + cache;
   KS_REQUIRE(ctx, ks_fits(K, 0, need) && ks_fits(V, 0, need) && ks_fits(q, 0, n * n_q * hd * 4) && ks_fits(meta, 0, n * 16) &&
              ks_fits(tmp, 0, n * n_q * (size_t)n_splits * (hd + 2) * 4), "sdpa_chunk: a buffer is too small");
   if (!ks_sdpa_chunk_covers(n_q, n_kv, hd, K->dptr, V->dptr)) return ks_fail(ctx, KS_ERR_UNSUPPORTED, "sdpa_chunk: shape not covered");
+  ks_kv_image image{};
+  image.span = ks_kv_image_tiles(max_t);
+  image.tiles = (size_t)n_parts * image.span;
+  const int rc = ks_ctx_gemm_scratch(ctx, ks_kv_image_bytes(image.tiles, n_kv, hd), &image.base);
+  if (rc) return rc;
   return ks_launch_sdpa_chunk(ctx, (int)n, n_q, n_kv, hd, scale, (const float*)q->dptr, (const uint8_t*)K->dptr, (const uint8_t*)V->dptr, (const float*)meta->dptr,
-                              (float*)tmp->dptr, n_splits, &parts, slot_stride_bytes);
+                              (float*)tmp->dptr, n_splits, image, &parts, slot_stride_bytes);
 }

@@ -194,3 +194,29 @@ def test_gelu_of_four_rows_per_cluster(ctx, ffn):
         scale, err = np.abs(want).max(), np.abs(got - want)
         assert err.max() <= 1e-3 * scale and np.sqrt((err ** 2).mean()) <= 1e-4 * scale, n
     model.close()
+
+
+def test_mixed_pass_with_more_context_than_its_decoded_tiles(ctx):
+    """Eight slots of 15 tiles of 64 positions and 32 KV heads are more than the 64 tiles such a model keeps decoded (256 MB): their short
+    pieces run in several passes.  Against the same pieces one by one, whose rows read the caches themselves: the model's bound."""
+    cfg = ksm.ModelConfig(1, 256, 512, 32, 32, 256, 1024, 1024, 8, sigma_w=0.01, sigma_embd=1e-4)
+    model, _ = ksm.GemmaCudaModel.synthetic(ctx, cfg, seed=53, keep=True)
+    slots = [model.slot_alloc() for _ in range(8)]
+    toks = [int(t) for t in synth.token_ids(53, "p", 1000, cfg.vocab)]
+    out = []
+    for together in (True, False):
+        for s in slots:
+            model.slot_reset(s)
+            model.prefill(s, toks[s:s + 900])
+        pieces = [(s, toks[s:s + 5 + s]) for s in slots]
+        if together:
+            model.prefill_many(pieces)
+        else:
+            for s, p in pieces:
+                model.prefill(s, p)
+        model.forward(0, 8, toks[:8], True)
+        ctx.synchronize()
+        out.append(np.concatenate([model.read_debug(1, s).astype(np.float64) for s in slots]))
+    scale, err = np.abs(out[1]).max(), np.abs(out[0] - out[1])
+    assert err.max() <= 1e-3 * scale and np.sqrt((err ** 2).mean()) <= 1e-4 * scale
+    model.close()
