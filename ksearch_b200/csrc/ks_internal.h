@@ -147,7 +147,8 @@ int ks_launch_per_head_qkv_q40(ks_ctx* ctx, size_t n_q, size_t n_kv, size_t hd, 
                                const int* pos_dev, size_t slot_stride_bytes);
 int ks_launch_sdpa(ks_ctx* ctx, size_t n_slots, size_t n_q, size_t n_kv, size_t hd, float scale, ks_dtype act,
                    const void* q, const uint8_t* K, const uint8_t* V, size_t slot_stride_bytes, const float* meta,
-                   float* tmp, void* out, int n_splits, bool records_only = false);  // records_only: the splits stay in tmp, unmerged
+                   float* tmp, void* out, int n_splits, bool records_only = false, size_t max_t = 0);
+// records_only: the splits stay in tmp, unmerged; max_t: no context is longer (0: slots keep n_splits each)
 // A prompt chunk's rows against one slot's cache on the tensor cores (ks_sdpa_chunk.cu), and the merge of its records into
 // the operand image of the output projection.
 int ks_sdpa_chunk_splits(const ks_ctx* ctx, int n_tok, size_t n_q, size_t n_kv, size_t ctx_len, int most);

@@ -258,17 +258,50 @@ sdpa_part_kernel(unsigned n_q, unsigned n_kv, float scale, const T* q, const uin
   }
 }
 
+// Slots of unequal contexts share their launch's splits by length: every slot gets as many chunks of one size as its context has, or the
+// launch lasts as long as a share of its longest context (four slots of 1024, 4096, 16384 and 16384 positions in 32 splits each: 27.8
+// us, dealt 24; with 4 KV heads 41.4 and 30.9; eight of 50, 100, .. 6400 with one 20.3 and 14.8).  Contexts that are short for the splits
+// (chunks of 128 positions) or average four fifths of the longest keep the plain layout (eight of 8192: 42.8 us either way); working the
+// rest out takes half a microsecond in each of the two launches (9000 and 30 positions: 16.4 and 16.8).  Chunk u of the launch leaves its
+// record at place u, one head behind the other.  A whole warp calls; lane s speaks for slot s.
+constexpr unsigned kDealSlots = 32;
+constexpr unsigned kMinChunk = 128;  // positions of a split at least: a tile of 16 per warp
+struct Deal {
+  unsigned chunk, count;  // positions of a chunk (0: not dealt); this lane's slot: how many
+};
+// tlen: of this lane's slot, 0 beyond the last
+__device__ __forceinline__ Deal deal_splits(unsigned tlen, unsigned n_slots, unsigned n_splits) {
+  const unsigned lane = threadIdx.x & 31u, most = n_slots * n_splits;
+  const unsigned sum = __reduce_add_sync(0xffffffffu, tlen), top = __reduce_max_sync(0xffffffffu, tlen);
+  Deal d{0u, 0u};
+  if (top <= kMinChunk * n_splits || (unsigned long long)top * n_slots * 4u <= (unsigned long long)sum * 5u) return d;
+  // the size that fills the launch if every context divides by it, else one with a chunk to spare for every slot: that always fits
+  // (reciprocals, and a step either way: four divisions one behind the other took longer than the rest)
+#pragma unroll
+  for (int again = 0; again < 2; again++) {
+    d.chunk = max(kMinChunk, ((unsigned)__fdividef((float)sum, (float)(again ? most - n_slots : most)) + 16u) & ~15u);
+    d.count = (unsigned)__fdividef((float)tlen, (float)d.chunk);
+    d.count += d.count * d.chunk < tlen;
+    d.count -= d.count > 0u && (d.count - 1u) * d.chunk >= tlen;
+    d.count = lane < n_slots ? max(1u, d.count) : 0u;
+    if (__reduce_add_sync(0xffffffffu, d.count) <= most) break;
+  }
+  return d;
+}
+
 // Merge the per-split records of one (slot, head): lower.rs:5897-6088.  A block takes 64 dims; four threads share a dim's splits
 // (p = part, part + 4, ...) and their sums meet in a fixed order.  The O values are requested before the (m, l) pairs are looked
 // at, so the two trips to memory are one.  Bound by that trip and the launch.
 constexpr int kRedDims = 64, kRedParts = 4, kRedFly = 8;
-template <typename T>
-__global__ void __launch_bounds__(kRedDims * kRedParts) sdpa_reduce_kernel(unsigned hd, const float* tmp, T* out, int n_splits) {
+// DEAL: the launch's splits may have been dealt among gridDim.x / n_q slots.
+template <typename T, bool DEAL>
+__global__ void __launch_bounds__(kRedDims * kRedParts) sdpa_reduce_kernel(unsigned hd, const float* tmp, T* out, int n_splits, unsigned n_q, const float* meta) {
   ks_pdl_entry();
   __shared__ float fac[KS_SDPA_MAX_SPLITS];
   __shared__ float part_sum[kRedDims * kRedParts];
   const size_t sh = blockIdx.x;  // slot * n_q + head
   const float* rec0 = tmp + sh * n_splits * (hd + 2);
+  size_t stride = hd + 2;
   const int part = threadIdx.x / kRedDims, lane = threadIdx.x & 31;
   const unsigned d = blockIdx.y * kRedDims + threadIdx.x % kRedDims;
   float v[kRedFly];
@@ -276,17 +309,27 @@ __global__ void __launch_bounds__(kRedDims * kRedParts) sdpa_reduce_kernel(unsig
 #pragma unroll
     for (int k = 0; k < kRedFly; k++) {
       const int p = p0 + k * kRedParts;
-      v[k] = p < n_splits ? rec0[(size_t)p * (hd + 2) + 2 + d] : 0.0f;
+      v[k] = p < n_splits ? rec0[p * stride + 2 + d] : 0.0f;
     }
   };
   request(part);
+  if constexpr (DEAL) {  // what was asked for above is right unless the splits were dealt
+    const unsigned n_slots = gridDim.x / n_q, slot = blockIdx.x / n_q;
+    const Deal g = deal_splits((unsigned)lane < n_slots ? (unsigned)meta[lane * 4] : 0u, n_slots, (unsigned)n_splits);
+    if (g.chunk) {
+      rec0 = tmp + ((size_t)__reduce_add_sync(0xffffffffu, (unsigned)lane < slot ? g.count : 0u) * n_q + blockIdx.x % n_q) * (hd + 2);
+      n_splits = (int)__shfl_sync(0xffffffffu, g.count, slot);
+      stride *= n_q;
+      request(part);
+    }
+  }
   if (threadIdx.x < 32) {  // exp(m - M) / L of every split; an empty one (l = 0) has no O and counts for nothing
     float m[KS_SDPA_MAX_SPLITS / 32], l[KS_SDPA_MAX_SPLITS / 32], M = kNegInit, L = 0.0f;
 #pragma unroll
     for (int k = 0; k < KS_SDPA_MAX_SPLITS / 32; k++) {
       const int p = lane + 32 * k;
-      m[k] = p < n_splits ? rec0[(size_t)p * (hd + 2)] : kNegInit;
-      l[k] = p < n_splits ? rec0[(size_t)p * (hd + 2) + 1] : 0.0f;
+      m[k] = p < n_splits ? rec0[p * stride] : kNegInit;
+      l[k] = p < n_splits ? rec0[p * stride + 1] : 0.0f;
       M = fmaxf(M, m[k]);
     }
 #pragma unroll
@@ -338,7 +381,7 @@ __global__ void __launch_bounds__(kRedDims * kRedParts) sdpa_reduce_kernel(unsig
 constexpr int kMmaWarps = 8;
 constexpr int kMmaTile = 16;
 constexpr int kMmaRing = 2;
-constexpr int kMinChunk = kMmaWarps * kMmaTile;  // positions of a split at least: one tile per warp
+static_assert(kMinChunk == kMmaWarps * kMmaTile, "one tile per warp");
 
 template <int HD>
 struct MmaSmem {
@@ -370,7 +413,8 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
 __device__ __forceinline__ float half_at(const unsigned char* p) { return __half2float(__ushort_as_half(*reinterpret_cast<const unsigned short*>(p))); }
 
 // CH: bytes per copy of a cached row: 16 (8 for rows of 72 bytes) where the cache is aligned for it, else 4.
-template <int HD, typename T, unsigned CH>
+// DEAL: splits go to the slots by the lengths of their contexts where those are unequal enough.
+template <int HD, typename T, unsigned CH, bool DEAL>
 __global__ void __launch_bounds__(kMmaWarps * 32, 2)
 sdpa_mma_kernel(unsigned n_q, unsigned n_kv, unsigned gb, float scale, const T* q, const uint8_t* K, const uint8_t* V, size_t slot_stride,
                 const float* meta, float* tmp, T* out, int n_splits) {
@@ -380,16 +424,43 @@ sdpa_mma_kernel(unsigned n_q, unsigned n_kv, unsigned gb, float scale, const T* 
   extern __shared__ __align__(128) unsigned char smem[];
   const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, g = lane >> 2, t = lane & 3u;
   const unsigned hpk = n_q / n_kv, gpk = hpk / gb;  // heads and blocks per KV head
-  const unsigned split = blockIdx.x, kvh = blockIdx.y / gpk, slot = blockIdx.z;
-  const unsigned head0 = kvh * hpk + (blockIdx.y % gpk) * gb;
-  const unsigned tlen = (unsigned)meta[slot * 4 + 0], start = (unsigned)meta[slot * 4 + 1];
+  const unsigned kvh = blockIdx.y / gpk, head0 = kvh * hpk + (blockIdx.y % gpk) * gb;
+  unsigned split = blockIdx.x, slot = blockIdx.z, dealt = 0;
+  unsigned tlen, start;
+  if constexpr (DEAL) {
+    const float4 m = lane < gridDim.z ? *reinterpret_cast<const float4*>(meta + lane * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const Deal d = deal_splits((unsigned)m.x, gridDim.z, gridDim.x);
+    dealt = d.chunk;
+    if (dealt) {
+      unsigned end = d.count;  // of the slot's chunks
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned x = __shfl_up_sync(0xffffffffu, end, o);
+        if (lane >= (unsigned)o) end += x;
+      }
+      const unsigned at = blockIdx.z * gridDim.x + blockIdx.x;  // of the launch's splits
+      const unsigned before = __ballot_sync(0xffffffffu, end <= at);  // slots whose chunks lie in front
+      slot = __popc(before);
+      if (slot >= gridDim.z) return;  // more blocks than chunks: the merge looks at none beyond them
+      split = at - __shfl_sync(0xffffffffu, end - d.count, slot);
+    }
+    tlen = (unsigned)__shfl_sync(0xffffffffu, m.x, slot);
+    start = (unsigned)__shfl_sync(0xffffffffu, m.y, slot);
+  } else {
+    tlen = (unsigned)meta[slot * 4 + 0];
+    start = (unsigned)meta[slot * 4 + 1];
+  }
   // a split never holds fewer than kMinChunk positions: on a short context the later splits are empty and their
   // blocks leave after writing an empty record, so a split count sized for the longest context costs little
-  const unsigned chunk = max((tlen + n_splits - 1) / n_splits, (unsigned)kMinChunk);
+  const unsigned chunk = dealt ? dealt : max((tlen + n_splits - 1) / n_splits, kMinChunk);
   const unsigned p0 = split * chunk, p1 = min(p0 + chunk, tlen);
+  auto record = [&](unsigned head) {
+    if (DEAL && dealt) return tmp + ((size_t)(blockIdx.z * gridDim.x + blockIdx.x) * n_q + head) * (HD + 2);
+    return tmp + (((size_t)slot * n_q + head) * n_splits + split) * (HD + 2);
+  };
   if (p0 >= p1 && n_splits > 1) {  // nothing to do: the empty record (m = -1e30, l = 0) is all the merge needs
     if (tid < gb) {
-      float* rec = tmp + (((size_t)slot * n_q + head0 + tid) * n_splits + split) * (HD + 2);
+      float* rec = record(head0 + tid);
       rec[0] = kNegInit;
       rec[1] = 0.0f;
     }
@@ -634,7 +705,7 @@ sdpa_mma_kernel(unsigned n_q, unsigned n_kv, unsigned gb, float scale, const T* 
     if (n_splits == 1) {
       st_act<T>(out, ((size_t)slot * n_q + head) * HD + d, a / fac[36u + h]);
     } else {
-      float* rec = tmp + (((size_t)slot * n_q + head) * n_splits + split) * (HD + 2);
+      float* rec = record(head);
       if (d == 0) {
         rec[0] = fac[32u + h];
         rec[1] = fac[36u + h];
@@ -644,11 +715,11 @@ sdpa_mma_kernel(unsigned n_q, unsigned n_kv, unsigned gb, float scale, const T* 
   }
 }
 
-template <int HD, typename T, unsigned CH>
+template <int HD, typename T, unsigned CH, bool DEAL>
 int launch_mma(ks_ctx* ctx, unsigned hpk, dim3 grid, unsigned n_q, unsigned n_kv, float scale, const void* q, const uint8_t* K, const uint8_t* V,
                size_t slot_stride, const float* meta, float* tmp, void* out, int n_splits) {
   const unsigned gb = hpk % 4 == 0 ? 4u : hpk % 2 == 0 ? 2u : 1u;
-  auto kern = sdpa_mma_kernel<HD, T, CH>;
+  auto kern = sdpa_mma_kernel<HD, T, CH, DEAL>;
   constexpr size_t smem = MmaSmem<HD>::total;
   static bool set[16] = {false};
   if (!set[ctx->device & 15]) {
@@ -691,22 +762,27 @@ int launch_part_g(ks_ctx* ctx, int G, dim3 grid, unsigned n_q, unsigned n_kv, fl
 
 int ks_launch_sdpa(ks_ctx* ctx, size_t n_slots, size_t n_q, size_t n_kv, size_t hd, float scale, ks_dtype act,
                    const void* q, const uint8_t* K, const uint8_t* V, size_t slot_stride_bytes, const float* meta,
-                   float* tmp, void* out, int n_splits, bool records_only) {
+                   float* tmp, void* out, int n_splits, bool records_only, size_t max_t) {
   const int G = (int)(n_q / n_kv);
   if (G != 1 && G != 2 && G != 4 && G != 8 && G != 16)  // one set of groups, whichever kernel the operands' alignment leads to
     return ks_fail(ctx, KS_ERR_UNSUPPORTED, "sdpa: n_q/n_kv = %d not supported (1, 2, 4, 8, 16)", G);
   dim3 grid((unsigned)n_splits, (unsigned)n_kv, (unsigned)n_slots);
   int rc = 1;
+  bool deal = false;
   static const bool per_row = getenv("KSEARCH_SDPA_PER_ROW") != nullptr;  // keep the per-row kernel (comparison runs)
   const uintptr_t at = (uintptr_t)K | (uintptr_t)V | (uintptr_t)slot_stride_bytes;
   if (!per_row && (hd == 256 || hd == 128) && at % 4 == 0) {  // a cache that starts on 2 bytes is left to the per-row kernel
     const bool wide = at % (hd == 256 ? 16 : 8) == 0;
-#define KS_MMA(HD_, T_, CH_) launch_mma<HD_, T_, CH_>(ctx, (unsigned)G, grid, (unsigned)n_q, (unsigned)n_kv, scale, q, K, V, slot_stride_bytes, meta, tmp, out, n_splits)
+    // (contexts that cannot be long for the splits need not be looked at)
+    deal = max_t > (size_t)n_splits * kMinChunk && n_slots > 1 && n_slots <= kDealSlots && n_splits > 1 && n_slots * n_splits <= KS_SDPA_MAX_SPLITS && !records_only && ((uintptr_t)meta & 15) == 0;
+#define KS_MMA_D(HD_, T_, CH_, D_) launch_mma<HD_, T_, CH_, D_>(ctx, (unsigned)G, grid, (unsigned)n_q, (unsigned)n_kv, scale, q, K, V, slot_stride_bytes, meta, tmp, out, n_splits)
+#define KS_MMA(HD_, T_, CH_) (deal ? KS_MMA_D(HD_, T_, CH_, true) : KS_MMA_D(HD_, T_, CH_, false))
 #define KS_MMA_CH(HD_, CH_) (act == KS_F32 ? KS_MMA(HD_, float, CH_) : KS_MMA(HD_, __half, CH_))
     if (hd == 256) rc = wide ? KS_MMA_CH(256, 16u) : KS_MMA_CH(256, 4u);
     else rc = wide ? KS_MMA_CH(128, 8u) : KS_MMA_CH(128, 4u);
 #undef KS_MMA_CH
 #undef KS_MMA
+#undef KS_MMA_D
   }
   if (rc != 1) {
     // the tensor-core kernel took it
@@ -721,10 +797,15 @@ int ks_launch_sdpa(ks_ctx* ctx, size_t n_slots, size_t n_q, size_t n_kv, size_t 
   }
   if (rc || n_splits == 1 || records_only) return rc;
   const dim3 blocks((unsigned)(n_slots * n_q), (unsigned)hd / kRedDims);
-  if (act == KS_F32)
-    KS_LAUNCH(ctx, (sdpa_reduce_kernel<float>), blocks, kRedDims * kRedParts, 0, (unsigned)hd, tmp, (float*)out, n_splits);
-  else
-    KS_LAUNCH(ctx, (sdpa_reduce_kernel<__half>), blocks, kRedDims * kRedParts, 0, (unsigned)hd, tmp, (__half*)out, n_splits);
+#define KS_RED(T_, D_) KS_LAUNCH(ctx, (sdpa_reduce_kernel<T_, D_>), blocks, kRedDims * kRedParts, 0, (unsigned)hd, tmp, (T_*)out, n_splits, (unsigned)n_q, meta)
+  if (act == KS_F32) {
+    if (deal) KS_RED(float, true);
+    else KS_RED(float, false);
+  } else {
+    if (deal) KS_RED(__half, true);
+    else KS_RED(__half, false);
+  }
+#undef KS_RED
   return ks_after_launch(ctx, "sdpa_reduce");
 }
 
@@ -774,7 +855,7 @@ int ks_sdpa_decode(ks_ctx* ctx, size_t n_slots, size_t n_q, size_t n_kv, size_t 
   // (tlen, start) are device-resident and trusted to satisfy start + tlen <= max_t, as in the reference.
   return ks_launch_sdpa(ctx, n_slots, n_q, n_kv, hd, scale, act, q->dptr, (const uint8_t*)K->dptr + kv_byte_off,
                         (const uint8_t*)V->dptr + kv_byte_off, slot_stride_bytes, (const float*)meta->dptr,
-                        n_splits > 1 ? (float*)tmp->dptr : nullptr, out->dptr, n_splits);
+                        n_splits > 1 ? (float*)tmp->dptr : nullptr, out->dptr, n_splits, false, max_t);
 }
 
 }  // extern "C"
