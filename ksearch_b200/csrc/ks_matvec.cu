@@ -312,15 +312,18 @@ int launch_q6k_nt(ks_ctx* ctx, const MvArgs& a, int grid, int threads, size_t sm
 // activation dtypes).  Q6_K: the ring kernel (262144x1536 91 -> 66 us, 8192x4096 27 -> 14 us against variant 2); two row sets
 // per tile while four tiles of them are within 40 KB (up to 2048 columns), and as many warps as keep the last round of a short
 // launch full.  Q4_K: the fixed-point kernel where its shorter inner loop pays for staging x (rows of 4096 columns on:
-// 1536x6144 11.4 -> 6.5 us; or many rows of at most 2048: 12288x1536 7.8 -> 6.7 us), else the streamed kernel with eight warps
-// and two blocks per SM (20480x2560 16.5 -> 14.6 us).
+// 1536x6144 11.4 -> 6.5 us; or many rows of 1280 to 2048: 12288x1536 7.2 -> 6.3 us, but of 512 5.6 against 4.0, of 1024 5.9 against
+// 5.6), else the streamed kernel, whose launcher picks the warps (stream_q4k_warps).
 static ks_plan single_token_default(const ks_ctx* ctx, ks_dtype wdtype, size_t rows, size_t cols, bool one_matrix) {
   ks_plan p{};
   if (wdtype == KS_Q4K) {
-    p.variant = one_matrix && (cols >= 4096 || (rows >= 8192 && cols <= 2048)) ? 3 : 0;
-    p.nr = p.variant == 3 ? 0 : 1;
-    p.nwarps = 8;
-    p.ctas_per_sm = 2;
+    p.variant = one_matrix && (cols >= 4096 || (rows >= 8192 && cols > 1024 && cols <= 2048)) ? 3 : 0;
+    if (p.variant == 3) {
+      p.nwarps = 8;
+      p.ctas_per_sm = 2;
+    } else {
+      p.nr = 1;
+    }
     return p;
   }
   p.nr = cols <= 2048 ? 2 : 1;

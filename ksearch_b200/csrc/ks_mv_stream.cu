@@ -576,6 +576,35 @@ int launch_q6k(ks_ctx* ctx, const MvsArgs& a, unsigned grid, int nwarps, size_t 
   return ks_after_launch(ctx, "matvec_q6k_stream");
 }
 
+// Warps of a block for one token without a plan, two blocks per SM.  A row group (four rows) is a warp's unit of work, so eight warps are
+// fewer or longer rounds than need be for many shapes.  Measured through the entry points, us, eight warps and what is picked here:
+//   few groups of long rows: four, so that more SMs take part (1536x2048 4.25 / 3.66, 512x2560 4.76 / 3.79, gate|up 1024x1536 4.98 / 4.39);
+//   more groups than one block of eight warps per SM: of seven, six or (two matrices) four warps what leaves the busiest SM the fewest
+//   groups, as long as two blocks fit an SM (eight warps of 12 blocks x two stages do not): 6144x3072 10.06 / 6.57, 6144x1536 5.02 / 4.60,
+//   20480x3072 19.3 / 15.8, gate|up 6144x1536 9.58 / 6.58, 10240x2560 17.9 / 14.0, 16384x4096 36.8 / 30.2;
+//   else eight (short rows: 20480x1024 7.0, six 7.5; gate|up 4096x1536 5.1, four 6.3; an odd number of blocks: 20480x3840 22.7, six 26.1).
+int stream_q4k_warps(const ks_ctx* ctx, unsigned groups, unsigned cols, unsigned x_bytes, unsigned stage_bytes, int mats) {
+  const unsigned sms = (unsigned)ctx->sm_count;
+  if (groups <= 8u * sms) {
+    const bool few = mats == 2 ? groups <= 2u * sms : cols >= 2048 && groups <= (cols <= 2560 ? 8u : 5u) * sms / 3u;
+    return few ? 4 : 8;
+  }
+  if (cols <= 1024 || cols % 512) return 8;
+  int best = 8;
+  unsigned least = 0xFFFFFFFFu;
+  for (const int nw : {8, 7, 6, 4}) {
+    if ((nw == 8 && mats == 2) || (nw == 4 && mats == 1)) continue;
+    if (2u * (make_layout(x_bytes, stage_bytes, nw, 2).total + 1024u) > (unsigned)ctx->smem_optin + 1024u) continue;
+    const unsigned blocks = (groups + nw - 1) / nw, rounds = (groups + 2u * sms * nw - 1) / (2u * sms * nw);
+    const unsigned load = rounds > 1 ? rounds * 2u * nw : (blocks + sms - 1) / sms * nw;
+    if (load <= least) {
+      least = load;
+      best = nw;
+    }
+  }
+  return best;
+}
+
 }  // namespace
 
 // Streamed Q4_K launch; plan fields: nr = rows per lane (1 or 2), nwarps, ctas_per_sm,
@@ -636,14 +665,16 @@ int ks_launch_matvec_stream_q4k(ks_ctx* ctx, const ks_mv_seg* segs, int n_seg, k
   a.grp_start[a.n_seg] = g0;
   const unsigned x_bytes = (unsigned)n_tok * (unsigned)(cols / 64) * Q4K_XTOK * 4u;
   const unsigned stage_bytes = (unsigned)(RL * R * mats) * seg_blocks * KS_Q4K_BLOCK_BYTES;
-  const int cps = (plan && plan->ctas_per_sm > 0) ? plan->ctas_per_sm : 1;
+  const bool own = plan && plan->nwarps == 0 && n_tok == 1 && a.pro.mode == KS_PRO_NONE;  // one token without a plan
+  if (own) nwarps = stream_q4k_warps(ctx, g0, (unsigned)cols, x_bytes, stage_bytes, mats);
+  const int cps = own ? 2 : (plan && plan->ctas_per_sm > 0) ? plan->ctas_per_sm : 1;
   if (auto_stages) {
     // Enough stages for a warp to start ALL of its copies before it waits for its input (the whole
     // weight stream of a decode-sized matrix is then in flight while the previous kernel still
     // runs), inside HALF of an SM's shared memory so that the blocks of two consecutive kernels fit
     // side by side: fewer stages first, then fewer warps (not below 4).
     const unsigned half = 108u * 1024u;
-    const bool pick_warps = !(plan && plan->nwarps > 0);
+    const bool pick_warps = !own && !(plan && plan->nwarps > 0);
     for (;;) {
       const unsigned gw_total = (unsigned)(ctx->sm_count * cps * nwarps);
       const unsigned items = ((g0 + gw_total - 1) / gw_total) * a.n_cseg;
