@@ -88,7 +88,7 @@ def test_quantize_q4k_edge_cases(ctx):
 
 
 @pytest.mark.parametrize("act", [F32, F16])
-@pytest.mark.parametrize("n,rows", [(1536, 1), (2560, 1), (256, 5), (4096, 3), (100, 2)])
+@pytest.mark.parametrize("n,rows", [(1536, 1), (2560, 1), (256, 5), (4096, 3), (100, 2), (8, 3), (264, 2), (1544, 2), (8192, 2), (8200, 2)])
 def test_rmsnorm_family(ctx, oracle, act, n, rows):
     e = Eng(act)
     npdt = np.float32 if act == F32 else np.float16
@@ -137,6 +137,31 @@ def test_rmsnorm_add_then_rmsnorm(ctx, oracle, act):
         e.rmsnorm_add_then_rmsnorm(ctx, 1 << 20, 1e-6, by, bwp, br, bwf, ox, ox2)
 
 
+@pytest.mark.parametrize("act", [F32, F16])
+@pytest.mark.parametrize("n", [8, 248, 2568, 8192, 8200, 1530])
+@pytest.mark.parametrize("off", [0, 4])
+def test_norms_at_the_edges_of_their_forms(ctx, oracle, act, n, off):
+    """Eight values a thread up to 8192, rows that are no multiple of eight or longer, and rows that start off 16 bytes (4 elements: f16
+    only; the reference's rounding, so the tolerances of the tests above)."""
+    e = Eng(act)
+    npdt = np.float32 if act == F32 else np.float16
+    rows = 2
+    y, res = ((synth.normals(44, k, n * rows + off) * 2).astype(npdt) for k in ("y", "r"))
+    wp, wf = (synth.norm_weight(44, k, n).astype(npdt) for k in ("wp", "wf"))
+    by, br, bwp, bwf = map(ctx.buffer_bytes, (y, res, wp, wf))
+    out = ctx.buffer_empty_bytes(y.nbytes)
+    tol = dict(rtol=1e-3, atol=1e-4) if act == F32 else dict(rtol=3e-3, atol=3e-3)
+    yf, rf = y[off:].astype(np.float32), res[off:].astype(np.float32)
+    ctx.check(ctx.lib.ks_rmsnorm(ctx.h, n, rows, 1e-6, act, by.h, off, bwp.h, br.h, off, 0, 0.0, out.h, off))
+    assert_close(ctx.read_act(out, n * rows + off, act)[off:], oracle.rmsnorm(yf, wp.astype(np.float32), 1e-6, res=rf, rows=rows), what="rmsnorm", **tol)
+    if off == 0 and n * 4 <= 48 * 1024:
+        ox, ox2 = ctx.buffer_empty_bytes(y.nbytes), ctx.buffer_empty_bytes(y.nbytes)
+        e.rmsnorm_add_then_rmsnorm_rows(ctx, n, rows, 1e-6, by, bwp, br, bwf, ox, ox2)
+        wx, wx2 = oracle.rmsnorm_add_then_rmsnorm(yf, wp.astype(np.float32), rf, wf.astype(np.float32), 1e-6, rows=rows)
+        assert_close(ctx.read_act(ox, n * rows, act), wx, what="out_x", **tol)
+        assert_close(ctx.read_act(ox2, n * rows, act), wx2, what="out_x2", **tol)
+
+
 def test_quantize_q40_bit_exact(ctx, oracle, golden_cases):
     e = Eng(F32)
     v = golden_cases["pack_q40.v"]
@@ -156,7 +181,7 @@ def test_quantize_q40_bit_exact(ctx, oracle, golden_cases):
 
 
 @pytest.mark.parametrize("act", [F32, F16])
-@pytest.mark.parametrize("n_q,n_kv,hd,n_tok", [(8, 1, 256, 1), (8, 2, 256, 1), (8, 1, 256, 5), (4, 2, 64, 3)])
+@pytest.mark.parametrize("n_q,n_kv,hd,n_tok", [(8, 1, 256, 1), (8, 2, 256, 1), (8, 1, 256, 5), (4, 2, 64, 3), (4, 2, 128, 3), (2, 2, 128, 1)])
 def test_per_head_qkv_q40(ctx, oracle, act, n_q, n_kv, hd, n_tok):
     e = Eng(act)
     npdt = np.float32 if act == F32 else np.float16
