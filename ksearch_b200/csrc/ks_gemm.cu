@@ -444,10 +444,12 @@ struct EpiNormArgs {
   float* out_x;
   __half* xt;
 };
+constexpr int GM_MANY_ROWS = 512;
 constexpr size_t GM_NORM_MOST = 8 * 1024;  // the longest rows: eight values per thread
-// THREADS: at most; more than 512 have half the registers each.
-template <unsigned THREADS>
-__global__ void __launch_bounds__(THREADS) gemm_finish_norm_split_kernel(const EpiNormArgs e) {
+// THREADS: at most; more than 512 have half the registers each.  AHEAD: the norm weights are asked for with the first partials: with few
+// rows that hides two trips to memory, with many it costs the registers that more blocks per SM need (2047 rows of 1536 19.4 us, without 17).
+template <unsigned THREADS, bool AHEAD>
+__global__ void __launch_bounds__(THREADS, AHEAD ? 1 : 1024 / THREADS) gemm_finish_norm_split_kernel(const EpiNormArgs e) {
   ks_pdl_entry();
   __shared__ float red[32];
   const unsigned t = blockIdx.x, ck = threadIdx.x, chunks = e.rows / 8u;
@@ -459,12 +461,14 @@ __global__ void __launch_bounds__(THREADS) gemm_finish_norm_split_kernel(const E
   if (live) {
     r0 = *reinterpret_cast<const float4*>(e.res + at);
     r1 = *reinterpret_cast<const float4*>(e.res + at + 4);
-    p0 = *reinterpret_cast<const float4*>(e.w_post + 8u * ck);
-    p1 = *reinterpret_cast<const float4*>(e.w_post + 8u * ck + 4);
-    n0 = *reinterpret_cast<const float4*>(e.w_norm + 8u * ck);
-    n1 = *reinterpret_cast<const float4*>(e.w_norm + 8u * ck + 4);
+    if constexpr (AHEAD) {
+      p0 = *reinterpret_cast<const float4*>(e.w_post + 8u * ck);
+      p1 = *reinterpret_cast<const float4*>(e.w_post + 8u * ck + 4);
+      n0 = *reinterpret_cast<const float4*>(e.w_norm + 8u * ck);
+      n1 = *reinterpret_cast<const float4*>(e.w_norm + 8u * ck + 4);
+    }
   }
-  sum8<4>(e.P + at, e.part_stride, live ? ks_gemm_slots(e.map, 0u, 8u * ck / GM_ROWS, t) : 0u, y);
+  sum8<AHEAD ? 4 : 2>(e.P + at, e.part_stride, live ? ks_gemm_slots(e.map, 0u, 8u * ck / GM_ROWS, t) : 0u, y);
   float ss = 0.0f;
 #pragma unroll
   for (int i = 0; i < 8; i++) ss = fmaf(y[i], y[i], ss);
@@ -474,6 +478,10 @@ __global__ void __launch_bounds__(THREADS) gemm_finish_norm_split_kernel(const E
 #pragma unroll
   for (int i = 0; i < 8; i++) v[i] = 0.0f;
   if (live) {
+    if constexpr (!AHEAD) {
+      p0 = *reinterpret_cast<const float4*>(e.w_post + 8u * ck);
+      p1 = *reinterpret_cast<const float4*>(e.w_post + 8u * ck + 4);
+    }
     const float rr[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w}, pp[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
 #pragma unroll
     for (int i = 0; i < 8; i++) v[i] = __fadd_rn(rr[i], __fmul_rn(__fmul_rn(y[i], inv), pp[i]));
@@ -488,6 +496,10 @@ __global__ void __launch_bounds__(THREADS) gemm_finish_norm_split_kernel(const E
 #pragma unroll
   for (int i = 0; i < 8; i++) xn[i] = 0.0f;
   if (live) {
+    if constexpr (!AHEAD) {
+      n0 = *reinterpret_cast<const float4*>(e.w_norm + 8u * ck);
+      n1 = *reinterpret_cast<const float4*>(e.w_norm + 8u * ck + 4);
+    }
     const float nn[8] = {n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, n1.z, n1.w};
 #pragma unroll
     for (int i = 0; i < 8; i++) xn[i] = __fmul_rn(__fmul_rn(v[i], inv2), nn[i]);
@@ -976,8 +988,9 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
     e.out_x = epi->out_x;
     e.xt = (__half*)epi->xt_out;
     const unsigned threads = (unsigned)((rows[0] / 8 + 31) / 32 * 32);
-    if (threads <= 512u) KS_LAUNCH(ctx, (gemm_finish_norm_split_kernel<512>), e.np, threads, 0, e);
-    else KS_LAUNCH(ctx, (gemm_finish_norm_split_kernel<1024>), e.np, threads, 0, e);
+    if (threads > 512u) KS_LAUNCH(ctx, (gemm_finish_norm_split_kernel<1024, false>), e.np, threads, 0, e);
+    else if (n_tok < GM_MANY_ROWS) KS_LAUNCH(ctx, (gemm_finish_norm_split_kernel<512, true>), e.np, threads, 0, e);
+    else KS_LAUNCH(ctx, (gemm_finish_norm_split_kernel<512, false>), e.np, threads, 0, e);
     return ks_after_launch(ctx, "gemm_finish_norm_split");
   }
   if (mode == KS_GEMM_QKV) {

@@ -180,7 +180,8 @@ int ks_launch_sdpa_merge_split(ks_ctx* ctx, int n_tok, ks_gemm_blocks b, size_t 
 bool ks_gemm_few_rows_q6k(const ks_ctx* ctx, size_t rows, size_t cols);  // ks_gemm_skinny.cu has a kernel for up to 8 token rows
 int ks_launch_copy_scale_indexed(ks_ctx* ctx, size_t n, size_t batch, float scale, ks_dtype src_dtype,
                                  const void* src, const float* idx, ks_dtype act, void* dst);
-int ks_launch_softcap_argmax(ks_ctx* ctx, size_t n, float cap, ks_dtype act, const void* logits, float* out_idx);
+// rows (up to 64) of n logits, one behind the other, in one launch
+int ks_launch_softcap_argmax(ks_ctx* ctx, size_t n, float cap, ks_dtype act, const void* logits, float* out_idx, unsigned rows = 1);
 
 // ---- sampling candidates (ks_sample_gpu.cu, ks_sample.cpp) -------------------------------------------
 constexpr unsigned KS_CAND_MAX = 2048;  // pairs kept per slot; more and the host takes the whole row

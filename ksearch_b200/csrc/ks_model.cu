@@ -404,8 +404,7 @@ int enqueue_forward(ks_model* m, const Lane& L_, int n, bool want_logits) {
   // head: logits = token_embd . rms(x, output_norm); next id = softcap argmax (gemma_prim.rs:1222-1242)
   ks_mv_seg sh{(const uint8_t*)m->token_embd.dptr, logits, (unsigned)g.vocab};
   if ((rc = ks_launch_matvec(c, (ks_dtype)g.embd_dtype, &sh, 1, KS_EPI_PLAIN, H, act, x2, n, nullptr))) return rc;
-  for (int s = 0; s < n; s++)
-    if ((rc = ks_launch_softcap_argmax(c, g.vocab, g.softcap, act, logits + (size_t)s * g.vocab * ab, tok_out + s))) return rc;
+  if ((rc = ks_launch_softcap_argmax(c, g.vocab, g.softcap, act, logits, tok_out, (unsigned)n))) return rc;
   KS_LAUNCH(c, (collect_kernel), 1, row_threads(n), 0, n, (const float*)tok_out, (const unsigned*)c->ws + KS_WS_ERR_WORD, L_.ret, (float*)m->host_ret, (int)g.n_slots);
   return ks_after_launch(c, "collect");
 }
@@ -509,8 +508,7 @@ int enqueue_forward_gemm(ks_model* m, const Lane& L_, int n, bool want_logits) {
     float* ys[1] = {(float*)logits};
     if ((rc = ks_launch_gemm_segs(c, (ks_dtype)g.embd_dtype, 1, Ws, &V, H, m->gemm_xt, n, ys, &V, m->gemm_p0, KS_GEMM_PLAIN, nullptr, b_head))) return rc;
   }
-  for (int s = 0; s < n; s++)
-    if ((rc = ks_launch_softcap_argmax(c, g.vocab, g.softcap, act, logits + (size_t)s * g.vocab * 4, tok_out + s))) return rc;
+  if ((rc = ks_launch_softcap_argmax(c, g.vocab, g.softcap, act, logits, tok_out, (unsigned)n))) return rc;
   KS_LAUNCH(c, (collect_kernel), 1, row_threads(n), 0, n, (const float*)tok_out, (const unsigned*)c->ws + KS_WS_ERR_WORD, L_.ret, (float*)m->host_ret, (int)g.n_slots);
   return ks_after_launch(c, "collect");
 }
@@ -583,8 +581,7 @@ int enqueue_forward_fused(ks_model* m, const Lane& L_, int n, bool want_logits) 
     return rc;
   ks_mv_seg sh{(const uint8_t*)m->token_embd.dptr, logits, (unsigned)g.vocab};
   if ((rc = ks_launch_matvec(c, (ks_dtype)g.embd_dtype, &sh, 1, KS_EPI_PLAIN, H, act, xn, n, nullptr))) return rc;
-  for (int s = 0; s < n; s++)
-    if ((rc = ks_launch_softcap_argmax(c, g.vocab, g.softcap, act, logits + (size_t)s * g.vocab * ab, tok_out + s))) return rc;
+  if ((rc = ks_launch_softcap_argmax(c, g.vocab, g.softcap, act, logits, tok_out, (unsigned)n))) return rc;
   KS_LAUNCH(c, (collect_kernel), 1, row_threads(n), 0, n, (const float*)tok_out, (const unsigned*)c->ws + KS_WS_ERR_WORD, L_.ret, (float*)m->host_ret, (int)g.n_slots);
   return ks_after_launch(c, "collect");
 }

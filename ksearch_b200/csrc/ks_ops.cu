@@ -643,6 +643,12 @@ template <typename T>
 __global__ void softcap_argmax_kernel(unsigned n, float cap, const T* x, float* out_idx, float* ws_val,
                                       unsigned* ws_idx, unsigned* counter) {
   ks_pdl_entry();
+  // a row of logits per blockIdx.y, each with workspace, counter and result of its own
+  x += (size_t)blockIdx.y * n;
+  out_idx += blockIdx.y;
+  ws_val += blockIdx.y * gridDim.x;
+  ws_idx += blockIdx.y * gridDim.x;
+  counter += blockIdx.y;
   __shared__ float sv[32];
   __shared__ unsigned si[32];
   __shared__ bool last;
@@ -803,19 +809,20 @@ int ks_launch_copy_scale_indexed(ks_ctx* ctx, size_t n, size_t batch, float scal
   return ks_after_launch(ctx, "copy_scale_indexed");
 }
 
-int ks_launch_softcap_argmax(ks_ctx* ctx, size_t n, float cap, ks_dtype act, const void* logits, float* out_idx) {
-  // workspace layout: [0,1024) f32 values, [1024,2048) u32 indices, [2048] counter
+int ks_launch_softcap_argmax(ks_ctx* ctx, size_t n, float cap, ks_dtype act, const void* logits, float* out_idx, unsigned rows) {
+  // workspace layout: [0,1024) f32 values, [1024,2048) u32 indices, [2048,2048+64) counters of the rows
+  if (rows < 1 || rows > 64) return ks_fail(ctx, KS_ERR_INVALID, "softcap_argmax: %u rows (1 .. 64)", rows);
   float* ws_val = (float*)ctx->ws;
   unsigned* ws_idx = (unsigned*)ctx->ws + 1024;
   unsigned* counter = (unsigned*)ctx->ws + 2048;
   unsigned grid = (unsigned)((n + 1023) / 1024);
-  const unsigned cap_grid = (unsigned)(ctx->sm_count * 2) < 1024u ? (unsigned)(ctx->sm_count * 2) : 1024u;
+  const unsigned cap_grid = (unsigned)(ctx->sm_count * 2) < 1024u / rows ? (unsigned)(ctx->sm_count * 2) : 1024u / rows;
   if (grid > cap_grid) grid = cap_grid;
   if (grid == 0) grid = 1;
   if (act == KS_F32)
-    KS_LAUNCH(ctx, (softcap_argmax_kernel<float>), grid, 256, 0, (unsigned)n, cap, (const float*)logits, out_idx, ws_val, ws_idx, counter);
+    KS_LAUNCH(ctx, (softcap_argmax_kernel<float>), dim3(grid, rows), 256, 0, (unsigned)n, cap, (const float*)logits, out_idx, ws_val, ws_idx, counter);
   else
-    KS_LAUNCH(ctx, (softcap_argmax_kernel<__half>), grid, 256, 0, (unsigned)n, cap, (const __half*)logits, out_idx, ws_val, ws_idx, counter);
+    KS_LAUNCH(ctx, (softcap_argmax_kernel<__half>), dim3(grid, rows), 256, 0, (unsigned)n, cap, (const __half*)logits, out_idx, ws_val, ws_idx, counter);
   return ks_after_launch(ctx, "softcap_argmax");
 }
 
