@@ -18,10 +18,10 @@
 // sdpa_merge_split_kernel folds them straight into the operand image of the output projection.
 //
 // Bound by the chain of a tile: scores (48 MMAs), probabilities, values (12 MMAs of 256 columns), 3.2 us for 128 x 64.  When eight warps
-// of every block decoded its tiles it was 5.7 us, 2.2 of them waiting for keys; one thread per row of scores: 3.7.  Launches with their
-// image, back to back: 2047 rows of 8 heads (128 blocks of up to 32 tiles) 121 us, in two splits 84 (decoding in every block 205 and
-// 118); 2000 rows behind 2000 positions, 2 KV heads (126 blocks of up to 63 tiles) 218, in two splits 197 (387 and 343); 300 rows in
-// three splits 26.5 (30).
+// of every block decoded its tiles it was 5.7 us, 2.2 of them waiting for keys; one thread per row of scores: 3.7.  A block takes another
+// 8 us: q 3.6, records 2, setting up 2.  Launches with their image, back to back: 2047 rows of 8 heads (128 blocks of up to 32 tiles) 119
+// us, in two splits 78 (decoding in every block 205 and 118); 2000 rows behind 2000 positions, 2 KV heads (126 blocks of up to 63 tiles)
+// 218, in two splits 192 (387 and 343); 300 rows in three splits 23.6 (30).
 #include "ks_gemm_common.cuh"
 
 namespace {
@@ -52,16 +52,16 @@ struct ChunkSmem {
 };
 
 __device__ __forceinline__ void mb_arrive1(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
-// The two warps that share 32 query rows meet; true if every thread of both says so.
-__device__ __forceinline__ bool pair_all(unsigned quad, bool ok) {
+// `threads` threads (whole warps) meet at barrier `id`; true if every one of them says so.
+__device__ __forceinline__ bool meet_all(unsigned id, unsigned threads, bool ok) {
   unsigned r;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.u32 p, %1, 0;\n\t"
-      "barrier.cta.red.and.pred q, %2, 64, p;\n\t"
+      "barrier.cta.red.and.pred q, %2, %3, p;\n\t"
       "selp.u32 %0, 1, 0, q;\n\t}"
       : "=r"(r)
-      : "r"((unsigned)ok), "r"(1u + quad)
+      : "r"((unsigned)ok), "r"(id), "r"(threads)
       : "memory");
   return r != 0;
 }
@@ -208,41 +208,53 @@ sdpa_chunk_kernel(const __grid_constant__ ChunkParts parts, unsigned n_q, unsign
   }
   if (warp == CH_WORK_WARPS) tc_alloc(sm32(tslot), 512);
 
-  // ---- q: a warp takes eight rows at a time, lane = row lane % 8, chunk of 8 dims lane / 8 (+ 4 a step): a load touches 128 neighbouring
-  // bytes of eight rows, a store 128 bytes of a chunk.  The row maximum sets a power of two, then two f16 terms per value: the second
-  // stays in shared memory as core matrices, the first passes through there (K's place) to tensor memory.
-  for (unsigned grp = warp; grp < CH_BM / 8; grp += CH_THREADS / 32) {
-    constexpr int STEPS = HD / 32;
-    const unsigned r = grp * 8u + (lane & 7u), t = (row0 + r) / G, head = kvh * G + (row0 + r) % G;
-    const float* src = q + ((size_t)t * n_q + head) * HD + 8u * (lane >> 3);
-    float v[STEPS][8], m = 0.0f;
+  // ---- q: a worker warp takes twice eight rows, lane = row lane % 8, chunk of 8 dims lane / 8 (+ 4 a step): a load touches 128 neighbouring
+  // bytes of eight rows, a store 128 bytes of a chunk; all loads come first (one trip instead of two: 5.7 -> 3.6 us a block).  The row
+  // maximum sets a power of two, then two f16 terms per value: the second stays in shared memory as core matrices, the first passes
+  // through there (K's place) to tensor memory.
+  if (warp < CH_WORK_WARPS) {
+    constexpr int STEPS = HD / 32, GROUPS = CH_BM / 8 / CH_WORK_WARPS;
+    float v[GROUPS][STEPS][8], first_pos[GROUPS], length[GROUPS];
 #pragma unroll
-    for (int k = 0; k < STEPS; k++) {
-      const float4 a = t < n_tok ? *reinterpret_cast<const float4*>(src + 32 * k) : make_float4(0.f, 0.f, 0.f, 0.f);
-      const float4 b = t < n_tok ? *reinterpret_cast<const float4*>(src + 32 * k + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-      v[k][0] = a.x; v[k][1] = a.y; v[k][2] = a.z; v[k][3] = a.w;
-      v[k][4] = b.x; v[k][5] = b.y; v[k][6] = b.z; v[k][7] = b.w;
+    for (int p = 0; p < GROUPS; p++) {
+      const unsigned r = (warp * GROUPS + p) * 8u + (lane & 7u), t = (row0 + r) / G, head = kvh * G + (row0 + r) % G;
+      const float* src = q + ((size_t)t * n_q + head) * HD + 8u * (lane >> 3);
+      const bool in = t < n_tok;
+      length[p] = in ? meta[t * 4] : 0.0f;
+      first_pos[p] = in ? meta[t * 4 + 1] : 0.0f;
+#pragma unroll
+      for (int k = 0; k < STEPS; k++) {
+        const float4 a = in ? *reinterpret_cast<const float4*>(src + 32 * k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 b = in ? *reinterpret_cast<const float4*>(src + 32 * k + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[p][k][0] = a.x; v[p][k][1] = a.y; v[p][k][2] = a.z; v[p][k][3] = a.w;
+        v[p][k][4] = b.x; v[p][k][5] = b.y; v[p][k][6] = b.z; v[p][k][7] = b.w;
+      }
     }
 #pragma unroll
-    for (int k = 0; k < STEPS; k++) m = fmaxf(m, absmax8(v[k]));
-    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
-    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
-    float up;
-    const float down = row_scale_down(m, &up);
-    if (lane < 8u) {
-      row_scale[r] = up * scale;
-      row_first[r] = t < n_tok ? (int)meta[t * 4 + 1] : 0;
-      row_end[r] = t < n_tok ? (int)meta[t * 4 + 1] + (int)meta[t * 4 + 0] : 0;
-    }
+    for (int p = 0; p < GROUPS; p++) {
+      const unsigned r = (warp * GROUPS + p) * 8u + (lane & 7u);
+      float m = 0.0f;
 #pragma unroll
-    for (int k = 0; k < STEPS; k++) {
+      for (int k = 0; k < STEPS; k++) m = fmaxf(m, absmax8(v[p][k]));
+      m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+      m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
+      float up;
+      const float down = row_scale_down(m, &up);
+      if (lane < 8u) {
+        row_scale[r] = up * scale;
+        row_first[r] = (int)first_pos[p];
+        row_end[r] = (int)first_pos[p] + (int)length[p];
+      }
 #pragma unroll
-      for (int e = 0; e < 8; e++) v[k][e] *= down;
-      uint4 hi, lo;
-      split8(v[k], hi, lo);
-      const unsigned at = ((4u * k + (lane >> 3)) * CH_BM + r) * 16u;
-      *reinterpret_cast<uint4*>(smem + S::kh + at) = hi;
-      *reinterpret_cast<uint4*>(smem + S::ql + at) = lo;
+      for (int k = 0; k < STEPS; k++) {
+#pragma unroll
+        for (int e = 0; e < 8; e++) v[p][k][e] *= down;
+        uint4 hi, lo;
+        split8(v[p][k], hi, lo);
+        const unsigned at = ((4u * k + (lane >> 3)) * CH_BM + r) * 16u;
+        *reinterpret_cast<uint4*>(smem + S::kh + at) = hi;
+        *reinterpret_cast<uint4*>(smem + S::ql + at) = lo;
+      }
     }
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -326,7 +338,7 @@ sdpa_chunk_kernel(const __grid_constant__ ChunkParts parts, unsigned n_q, unsign
         }
         row_max[((i & 1u) * 2u + half) * CH_BM + row] = mx;
       }
-      if (!pair_all(quad, ok)) { ok = false; break; }
+      if (!meet_all(1u + quad, 64u, ok)) { ok = false; break; }  // the two warps that share 32 query rows
       mx = fmaxf(fmaxf(mx, row_max[((i & 1u) * 2u + (half ^ 1u)) * CH_BM + row]), ref);
       alpha = __expf(ref - mx);
       ref = mx;
@@ -362,6 +374,28 @@ sdpa_chunk_kernel(const __grid_constant__ ChunkParts parts, unsigned n_q, unsign
         *reinterpret_cast<float4*>(out + c) = make_float4(acc[c] * (1.0f / CH_P), acc[c + 1] * (1.0f / CH_P), acc[c + 2] * (1.0f / CH_P), acc[c + 3] * (1.0f / CH_P));
       row_max[((n_tiles & 1u) * 2u + half) * CH_BM + row] = l;  // (the tile before's maxima have been read by both)
       if (half == 0) row_scale[row] = ref;
+    }
+    if (meet_all(5u, CH_WORK_WARPS * 32u, ok)) {
+      // here, where the registers are: four rows of a warp's in flight at a time (one after the other, in twelve warps, they took 5.5 us)
+      constexpr unsigned FLY = 4, PER = HD / 64;
+      const float* sums = row_max + (n_tiles & 1u) * 2u * CH_BM;
+#pragma unroll 1
+      for (unsigned r0 = warp; r0 < CH_BM; r0 += CH_WORK_WARPS * FLY) {
+        float2 o[FLY][PER];
+#pragma unroll
+        for (unsigned f = 0; f < FLY; f++)
+#pragma unroll
+          for (unsigned k = 0; k < PER; k++) o[f][k] = (reinterpret_cast<const float2*>(smem + S::o) + (r0 + f * CH_WORK_WARPS) * (S::OP / 2))[lane + 32u * k];
+#pragma unroll
+        for (unsigned f = 0; f < FLY; f++) {
+          const unsigned r = r0 + f * CH_WORK_WARPS, t = (row0 + r) / G, head = kvh * G + (row0 + r) % G;
+          if (t >= n_tok) continue;
+          float* rec = tmp + (((size_t)t * n_q + head) * n_splits + split) * (HD + 2);
+#pragma unroll
+          for (unsigned k = 0; k < PER; k++) *reinterpret_cast<float2*>(rec + 2 + 2u * (lane + 32u * k)) = o[f][k];
+          if (lane == 0) *reinterpret_cast<float2*>(rec) = make_float2(row_scale[r], sums[r] + sums[CH_BM + r]);
+        }
+      }
     }
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
@@ -446,20 +480,7 @@ sdpa_chunk_kernel(const __grid_constant__ ChunkParts parts, unsigned n_q, unsign
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (*fail) {
-    if (tid == 0) atomicOr(err, 8u);
-  } else {
-    for (unsigned r = warp; r < CH_BM; r += CH_THREADS / 32) {
-      const unsigned t = (row0 + r) / G, head = kvh * G + (row0 + r) % G;
-      if (t >= n_tok) continue;
-      float* rec = tmp + (((size_t)t * n_q + head) * n_splits + split) * (HD + 2);
-      const float2* o = reinterpret_cast<const float2*>(smem + S::o) + r * (S::OP / 2);
-      for (unsigned d = lane; d < HD / 2u; d += 32u) *reinterpret_cast<float2*>(rec + 2 + 2u * d) = o[d];
-      const float* sums = row_max + (n_tiles & 1u) * 2u * CH_BM + r;
-      if (lane == 0) *reinterpret_cast<float2*>(rec) = make_float2(row_scale[r], sums[0] + sums[CH_BM]);
-    }
-  }
-  __syncthreads();
+  if (tid == 0 && *fail) atomicOr(err, 8u);
   if (warp == CH_WORK_WARPS) tc_dealloc(tmem, 512);
 }
 
