@@ -582,14 +582,16 @@ int launch_q6k(ks_ctx* ctx, const MvsArgs& a, unsigned grid, int nwarps, size_t 
 //   more groups than one block of eight warps per SM: of seven, six or (two matrices) four warps what leaves the busiest SM the fewest
 //   groups, as long as two blocks fit an SM (eight warps of 12 blocks x two stages do not): 6144x3072 10.06 / 6.57, 6144x1536 5.02 / 4.60,
 //   20480x3072 19.3 / 15.8, gate|up 6144x1536 9.58 / 6.58, 10240x2560 17.9 / 14.0, 16384x4096 36.8 / 30.2;
-//   else eight (short rows: 20480x1024 7.0, six 7.5; gate|up 4096x1536 5.1, four 6.3; an odd number of blocks: 20480x3840 22.7, six 26.1).
+//   else eight (short rows: 20480x1024 7.0, six 7.5, but 12685x1024 6.1 and 5.6, where six warps end their second round together;
+//   gate|up 4096x1536 5.1, four 6.3; an odd number of blocks: 20480x3840 22.7, six 26.1).
 int stream_q4k_warps(const ks_ctx* ctx, unsigned groups, unsigned cols, unsigned x_bytes, unsigned stage_bytes, int mats) {
   const unsigned sms = (unsigned)ctx->sm_count;
   if (groups <= 8u * sms) {
     const bool few = mats == 2 ? groups <= 2u * sms : cols >= 2048 && groups <= (cols <= 2560 ? 8u : 5u) * sms / 3u;
     return few ? 4 : 8;
   }
-  if (cols <= 1024 || cols % 512) return 8;
+  if (cols % 512) return 8;
+  if (cols <= 1024) return mats == 1 && groups > 20u * sms && groups <= 24u * sms ? 6 : 8;
   int best = 8;
   unsigned least = 0xFFFFFFFFu;
   for (const int nw : {8, 7, 6, 4}) {
