@@ -26,8 +26,9 @@
 // the last one is written out.
 //
 // Bound by: few token rows, the packed weights from memory and the issue slots of the dequantisation (about 1.7 instructions
-// per weight and lane of 16 warps); blocks of 128, the tensor core (73 % busy at 20480 x 2560 x 256 rows: 132 -> 72 us against
-// the kernel that wrote split weights to shared memory); few tiles, the latency of one unit and of the launches around it.
+// per weight and lane of 16 warps); blocks of 128, the tensor core (20480 x 2560 x 256 rows: 93 % busy inside a work tile, at the 1.4
+// GHz that the power limit leaves; 132 -> 72 us against the kernel that wrote split weights to shared memory); few tiles, the latency
+// of one unit and of the launches around it.
 // Every wait is bounded; on expiry the CTA raises the context's status word, waits (bounded) for what it has in flight, frees
 // its tensor memory and returns.
 #include <cuda.h>
