@@ -62,34 +62,44 @@ struct GemmArgs {
 };
 
 // x[token, k] (f32, row stride ldx) -> the B image.  One block per (padded) token row; rows past n_tok become zeros.
+__device__ __forceinline__ void x_chunk(const float* row, unsigned ck, float (&v)[8]) {
+  const float4 a = *reinterpret_cast<const float4*>(row + (size_t)ck * 8u), b = *reinterpret_cast<const float4*>(row + (size_t)ck * 8u + 4u);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+  v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+// ONE: a thread per chunk, which it reads once (rows of up to 8192 values: one trip to memory, and no more warps than there is work for;
+// with the partial counts of the sums behind it worked out early, 55 rows against 4096x1536 in three launches 12.9 -> 10.6 us).
+template <bool ONE>
 __global__ void __launch_bounds__(1024) x_split_kernel(const float* x, size_t ldx, unsigned n_tok, unsigned np, unsigned tbn, unsigned cols, __half* xt, int q4k) {
   ks_pdl_entry();
   __shared__ float red[32];
   const unsigned t = blockIdx.x, chunks = cols / 8u;
   const bool live = t < n_tok;
   const float* row = x + (size_t)t * ldx;
-  float m = 0.0f;
-  if (live)
-    for (unsigned ck = threadIdx.x; ck < chunks; ck += blockDim.x) {
-      const float4 a = *reinterpret_cast<const float4*>(row + (size_t)ck * 8u), b = *reinterpret_cast<const float4*>(row + (size_t)ck * 8u + 4u);
-      const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-      m = fmaxf(m, absmax8(v));
+  float m = 0.0f, v[8];
+#pragma unroll
+  for (int e = 0; e < 8; e++) v[e] = 0.0f;
+  if (live) {
+    if constexpr (ONE) {
+      x_chunk(row, threadIdx.x, v);
+      m = absmax8(v);
+    } else {
+      for (unsigned ck = threadIdx.x; ck < chunks; ck += blockDim.x) {
+        x_chunk(row, ck, v);
+        m = fmaxf(m, absmax8(v));
+      }
     }
+  }
   m = block_max_f(m, red);
   float up;
   const float down = row_scale_down(m, &up);
   if (threadIdx.x == 0) reinterpret_cast<float*>(xt + xt_scale_off(cols, np))[t] = up;
   for (unsigned ck = threadIdx.x; ck < chunks; ck += blockDim.x) {
-    float v[8];
-    if (live) {
-      const float4 a = *reinterpret_cast<const float4*>(row + (size_t)ck * 8u), b = *reinterpret_cast<const float4*>(row + (size_t)ck * 8u + 4u);
-      v[0] = a.x * down; v[1] = a.y * down; v[2] = a.z * down; v[3] = a.w * down;
-      v[4] = b.x * down; v[5] = b.y * down; v[6] = b.z * down; v[7] = b.w * down;
-    } else {
+    if (!ONE && live) x_chunk(row, ck, v);
+    float w[8];
 #pragma unroll
-      for (int e = 0; e < 8; e++) v[e] = 0.0f;
-    }
-    put_split8(xt, np, tbn, t, ck, chunks, v, q4k != 0);
+    for (int e = 0; e < 8; e++) w[e] = v[e] * down;  // (zeros past n_tok)
+    put_split8(xt, np, tbn, t, ck, chunks, w, q4k != 0);
   }
 }
 
@@ -385,7 +395,6 @@ __device__ __forceinline__ FinVec<V> sum_slots(const float* P, size_t stride, un
 }
 template <int V>
 __global__ void __launch_bounds__(256) gemm_finish_kernel(const FinishArgs f) {
-  ks_pdl_entry();
   constexpr unsigned PER = GM_ROWS / V, TOK = 256u / PER;  // threads per token row, token rows per block
   const unsigned bx = blockIdx.x, seg = (bx >= f.tile0[1]) + (bx >= f.tile0[2]);
   const unsigned rows = seg == 0 ? f.rows[0] : seg == 1 ? f.rows[1] : f.rows[2];
@@ -398,7 +407,9 @@ __global__ void __launch_bounds__(256) gemm_finish_kernel(const FinishArgs f) {
   if (t >= f.n_tok || r >= rows) return;
   const size_t at = (size_t)t * rows + r;  // partials are dense [split][token][row]
   const unsigned group0 = seg == 0 ? f.group0[0] : seg == 1 ? f.group0[1] : f.group0[2];
-  const FinVec<V> g = sum_slots<V>(P, ps, ks_gemm_slots(f.map, group0, bx - tile0, t), at);
+  const unsigned slots = ks_gemm_slots(f.map, group0, bx - tile0, t);  // (half a dozen divisions: in front of the wait)
+  ks_pdl_entry();
+  const FinVec<V> g = sum_slots<V>(P, ps, slots, at);
   float* o = y + (size_t)t * ldy + r;
   if constexpr (V == 4) *reinterpret_cast<float4*>(o) = make_float4(g.v[0], g.v[1], g.v[2], g.v[3]);
   else *o = g.v[0];
@@ -450,10 +461,11 @@ constexpr size_t GM_NORM_MOST = 8 * 1024;  // the longest rows: eight values per
 // rows that hides two trips to memory, with many it costs the registers that more blocks per SM need (2047 rows of 1536 19.4 us, without 17).
 template <unsigned THREADS, bool AHEAD>
 __global__ void __launch_bounds__(THREADS, AHEAD ? 1 : 1024 / THREADS) gemm_finish_norm_split_kernel(const EpiNormArgs e) {
-  ks_pdl_entry();
   __shared__ float red[32];
   const unsigned t = blockIdx.x, ck = threadIdx.x, chunks = e.rows / 8u;
   const bool live = ck < chunks && t < e.n_tok;
+  const unsigned slots = live ? ks_gemm_slots(e.map, 0u, 8u * ck / GM_ROWS, t) : 0u;  // (half a dozen divisions: in front of the wait)
+  ks_pdl_entry();
   float y[8];
   const size_t at = (size_t)t * e.rows + 8u * ck;
   // everything that does not depend on the sums is requested first
@@ -468,7 +480,7 @@ __global__ void __launch_bounds__(THREADS, AHEAD ? 1 : 1024 / THREADS) gemm_fini
       n1 = *reinterpret_cast<const float4*>(e.w_norm + 8u * ck + 4);
     }
   }
-  sum8<AHEAD ? 4 : 2>(e.P + at, e.part_stride, live ? ks_gemm_slots(e.map, 0u, 8u * ck / GM_ROWS, t) : 0u, y);
+  sum8<AHEAD ? 4 : 2>(e.P + at, e.part_stride, slots, y);
   float ss = 0.0f;
 #pragma unroll
   for (int i = 0; i < 8; i++) ss = fmaf(y[i], y[i], ss);
@@ -523,21 +535,23 @@ constexpr size_t GM_GELU_MOST = 8 * GM_GELU_CL * GM_GELU_THREADS;
 __global__ void __cluster_dims__(GM_GELU_CL, 1, 1) __launch_bounds__(GM_GELU_THREADS)
     gemm_finish_gelu_split_kernel(const float* P0, const float* P1, size_t part_stride, ks_gemm_map map, unsigned n_tok, unsigned np, unsigned tbn,
                                   unsigned rows, __half* xt) {
-  ks_pdl_entry();
   __shared__ float red[32], maxima[GM_GELU_CL];
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   cluster.barrier_arrive();  // (a block's shared memory is there once it has started)
   const unsigned rank = blockIdx.x % GM_GELU_CL, t = blockIdx.x / GM_GELU_CL, chunks = rows / 8u, ck = rank * blockDim.x + threadIdx.x;
+  // how many partials (divisions: in front of the wait)
+  const unsigned tile = 8u * ck / GM_ROWS, groups = map.G ? ((rows + GM_ROWS - 1u) / GM_ROWS + map.nt - 1u) / map.nt : 0u;
+  const unsigned ng = ks_gemm_slots(map, 0u, tile, t), nu = ks_gemm_slots(map, groups, tile, t);
+  ks_pdl_entry();
   float v[8];
 #pragma unroll
   for (int k = 0; k < 8; k++) v[k] = 0.0f;
   if (t < n_tok && ck < chunks) {
     float g[8], u[8];
     const size_t at = (size_t)t * rows + 8u * ck;
-    const unsigned tile = 8u * ck / GM_ROWS, groups = map.G ? ((rows + GM_ROWS - 1u) / GM_ROWS + map.nt - 1u) / map.nt : 0u;
-    sum8<4>(P0 + at, part_stride, ks_gemm_slots(map, 0u, tile, t), g);
-    sum8<4>(P1 + at, part_stride, ks_gemm_slots(map, groups, tile, t), u);
+    sum8<4>(P0 + at, part_stride, ng, g);
+    sum8<4>(P1 + at, part_stride, nu, u);
 #pragma unroll
     for (int k = 0; k < 8; k++) v[k] = gelu_mul(g[k], u[k]);
   }
@@ -667,7 +681,6 @@ template <int HD>
 __global__ void __launch_bounds__(256) gemm_finish_qkv_kernel(const EpiQkvArgs e) {
   constexpr int V = HD / 64, LPB = 32 / V;  // values per lane and half, lanes per 32-value block
   constexpr unsigned ROWB = HD / 32 * KS_Q40_BLOCK_BYTES;
-  ks_pdl_entry();
   const unsigned lane = threadIdx.x & 31u, jobs = e.n_q + 2u * e.n_kv, id = blockIdx.x * 8u + (threadIdx.x >> 5);
   if (id >= e.n_tok * jobs) return;
   const unsigned tok = id / jobs, job = id - tok * jobs;
@@ -676,6 +689,9 @@ __global__ void __launch_bounds__(256) gemm_finish_qkv_kernel(const EpiQkvArgs e
   const float* P = seg == 0 ? e.P[0] : seg == 1 ? e.P[1] : e.P[2];
   const size_t ps = seg == 0 ? e.part_stride[0] : seg == 1 ? e.part_stride[1] : e.part_stride[2];
   const unsigned rows = seg == 0 ? e.rows[0] : seg == 1 ? e.rows[1] : e.rows[2], g0 = seg == 0 ? e.group0[0] : seg == 1 ? e.group0[1] : e.group0[2];
+  // (half a head is one row tile, or within one; how many partials it has takes half a dozen divisions: a lane each, in front of the wait)
+  const unsigned my_slots = ks_gemm_slots(e.map, g0, (head * HD + (lane & 1u) * (HD / 2)) / GM_ROWS, tok);
+  ks_pdl_entry();
   const size_t p = (size_t)e.pos[tok];
   const float* cs = e.rope + p * HD;
   float c[V], sn[V], w[2][V], x[2][V];
@@ -687,8 +703,6 @@ __global__ void __launch_bounds__(256) gemm_finish_qkv_kernel(const EpiQkvArgs e
     w[0][k] = seg == 0 ? e.qw[d] : seg == 1 ? e.kw[d] : 1.0f;
     w[1][k] = seg == 0 ? e.qw[HD / 2 + d] : seg == 1 ? e.kw[HD / 2 + d] : 1.0f;
   }
-  // (half a head is one row tile, or within one; how many partials it has takes half a dozen divisions: a lane each)
-  const unsigned my_slots = ks_gemm_slots(e.map, g0, (head * HD + (lane & 1u) * (HD / 2)) / GM_ROWS, tok);
 #pragma unroll
   for (int h = 0; h < 2; h++) {
     const unsigned row = head * HD + (unsigned)h * (HD / 2) + lane * V, n = __shfl_sync(0xffffffffu, my_slots, h);
@@ -862,7 +876,9 @@ size_t ks_gemm_xt_bytes(size_t cols, int n_tok) {  // image + one factor per row
 // x[t * ldx + k] (f32) -> the B image in xt.
 int ks_launch_gemm_split(ks_ctx* ctx, ks_dtype wdtype, const float* x, size_t ldx, int n_tok, size_t cols, void* xt, ks_gemm_blocks b) {
   if (cols % 256 || n_tok < 1 || n_tok > KS_GEMM_ROWS || ldx % 4) return ks_fail(ctx, KS_ERR_INVALID, "gemm: bad operand shape");
-  KS_LAUNCH(ctx, (x_split_kernel), b.np, GM_ROW_THREADS, 0, x, ldx, (unsigned)n_tok, b.np, b.tbn, (unsigned)cols, (__half*)xt, (int)(wdtype == KS_Q4K));
+  const bool one = cols <= 8u * GM_ROW_THREADS;
+  KS_LAUNCH(ctx, (one ? x_split_kernel<true> : x_split_kernel<false>), b.np, one ? (unsigned)(cols / 8) : (unsigned)GM_ROW_THREADS, 0, x, ldx, (unsigned)n_tok, b.np, b.tbn,
+            (unsigned)cols, (__half*)xt, (int)(wdtype == KS_Q4K));
   return ks_after_launch(ctx, "x_split");
 }
 

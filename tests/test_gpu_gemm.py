@@ -136,3 +136,19 @@ def test_gemm_token_rows_beyond_the_f16_range(ctx, oracle, dtype):
         scale = np.abs(y64[t]).max()
         err = np.abs(got[t] - y64[t])
         assert (err <= 1e-3 * np.abs(y64[t]) + 1e-5 * scale).all(), (t, err.max() / scale)
+
+
+@pytest.mark.parametrize("cols", [256, 8192, 8448])
+@pytest.mark.parametrize("batch", [9, 70])
+def test_operand_split_of_short_and_long_rows(ctx, oracle, cols, batch):
+    """A thread per eight values reads them once up to 8192 columns, longer rows are read twice; rows that pad a block are zeros, so the
+    sums of the last token row do not depend on what lies behind it."""
+    rows = 300
+    W = synth.q4k_matrix(71, "w", rows, cols)
+    x = synth.normals(71, "x", cols * batch)
+    y = ctx.buffer_empty_f32(rows * batch)
+    Eng().matvec_batch(ctx, rows, cols, batch, Q4K, ctx.buffer_bytes(W), ctx.buffer_bytes(np.concatenate([x, np.full(cols, np.nan, np.float32)])), y)
+    got = ctx.read_f32(y, rows * batch).reshape(batch, rows).astype(np.float64)
+    for t in (0, 1, batch - 1):
+        _, ref = oracle.matvec(Q4K, W, rows, cols, x[t * cols:(t + 1) * cols])
+        assert np.abs(got[t] - ref).max() <= 1e-5 * np.abs(ref).max() + 1e-4
