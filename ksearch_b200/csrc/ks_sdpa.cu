@@ -260,7 +260,7 @@ sdpa_part_kernel(unsigned n_q, unsigned n_kv, float scale, const T* q, const uin
 
 // Slots of unequal contexts share their launch's splits by length: every slot gets as many chunks of one size as its context has, or the
 // launch lasts as long as a share of its longest context (four slots of 1024, 4096, 16384 and 16384 positions in 32 splits each: 27.8
-// us, dealt 24; with 4 KV heads 41.4 and 30.9; eight of 50, 100, .. 6400 with one 20.3 and 14.8).  Contexts that are short for the splits
+// us, dealt 24; with 4 KV heads 41.4 and 30.9; eight of 50, 100, .. 6400 with one 20.3 and 14.8; figures before q was read in one trip).  Contexts that are short for the splits
 // (chunks of 128 positions) or average four fifths of the longest keep the plain layout (eight of 8192: 42.8 us either way); working the
 // rest out takes half a microsecond in each of the two launches (9000 and 30 positions: 16.4 and 16.8).  Chunk u of the launch leaves its
 // record at place u, one head behind the other.  A whole warp calls; lane s speaks for slot s.
@@ -500,43 +500,54 @@ sdpa_mma_kernel(unsigned n_q, unsigned n_kv, unsigned gb, float scale, const T* 
   };
   fetch(0, 0);
 
-  // ---- q: per head a power-of-two scale, then the B fragments of every block in the order the lanes read them
+  // ---- q: per head a power-of-two scale, then the B fragments of every block in the order the lanes read them.  A thread reads the
+  // eight values of its fragment once; their largest meet over the lanes of a block and, through shared memory, over the blocks.  (A warp
+  // per head looking for the maximum first made two trips to memory and a loop of 1.4 to 2 us: one slot of 16384 positions 15.9 -> 14.4
+  // us, eight of 300 13.1 -> 11.7, the four unequal ones above 24 -> 22.)
   float* qscale = reinterpret_cast<float*>(smem + S::st_off + kMmaWarps * 4 * 8);  // [0..4) down, [4..8) up
-  if (warp < gb) {
-    float m = 0.0f;
-    for (unsigned i = lane; i < HD; i += 32u) m = fmaxf(m, fabsf(ld_act<T>(q, ((size_t)slot * n_q + head0 + warp) * HD + i)));
+  float* bmax = reinterpret_cast<float*>(smem + S::st_off);                        // [NB][4] (the warps' (m, l) come here later)
+  static_assert(NB <= (unsigned)kMmaWarps && NB * 16u <= kMmaWarps * 4 * 8, "a warp per block, and its four largest values fit");
+  {
+    const unsigned n = lane >> 2, lt = lane & 3u, h = n & 3u;
+    const bool in = warp < NB && h < gb;
+    float x[2][4], m = 0.0f;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (lane == 0) {
-      int e = 0;
-      if (m > 0.0f && m < 3.0e38f) {
-        e = (int)((__float_as_uint(m) >> 23) & 0xFFu) - 127 - 14;
-        e = e < -100 ? -100 : e;
+    for (int half = 0; half < 2; half++)
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        x[half][k] = in ? ld_act<T>(q, ((size_t)slot * n_q + head0 + h) * HD + 32u * warp + 4u * lt + 16u * half + k) : 0.0f;
+        m = fmaxf(m, fabsf(x[half][k]));
       }
-      qscale[warp] = __uint_as_float((unsigned)(127 - e) << 23);
-      qscale[4 + warp] = __uint_as_float((unsigned)(127 + e) << 23);
+    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+    if (warp < NB && lt == 0 && n < 4u) bmax[warp * 4u + h] = m;
+    __syncthreads();
+    m = 0.0f;
+#pragma unroll
+    for (unsigned b = 0; b < NB; b++) m = fmaxf(m, bmax[b * 4u + h]);
+    int e = 0;
+    if (m > 0.0f && m < 3.0e38f) {
+      e = (int)((__float_as_uint(m) >> 23) & 0xFFu) - 127 - 14;
+      e = e < -100 ? -100 : e;
     }
-  } else if (warp < 4) {
-    if (lane == 0) qscale[warp] = qscale[4 + warp] = 0.0f;
-  }
-  __syncthreads();
-  for (unsigned i = tid; i < NB * 32u; i += kMmaWarps * 32) {
-    const unsigned b = i >> 5, l = i & 31u, n = l >> 2, lt = l & 3u, h = n & 3u;
-    uint32_t w[4] = {0u, 0u, 0u, 0u};
-    if (h < gb) {
-      const size_t at = ((size_t)slot * n_q + head0 + h) * HD + 32u * b + 4u * lt;
-      const float dn = qscale[h];
+    const float dn = __uint_as_float((unsigned)(127 - e) << 23);
+    if (warp == 0 && lt == 0 && n < 4u) {
+      qscale[h] = h < gb ? dn : 0.0f;
+      qscale[4 + h] = h < gb ? __uint_as_float((unsigned)(127 + e) << 23) : 0.0f;
+    }
+    if (warp < NB) {
+      uint32_t w[4];
 #pragma unroll
       for (int half = 0; half < 2; half++)
 #pragma unroll
         for (int k = 0; k < 2; k++) {
-          const float x0 = ld_act<T>(q, at + 16u * half + k) * dn, x1 = ld_act<T>(q, at + 16u * half + k + 2u) * dn;
+          const float x0 = x[half][k] * dn, x1 = x[half][k + 2] * dn;
           const __half2 hh = __floats2half2_rn(x0, x1);
           const float2 hf = __half22float2(hh);
           w[2 * half + k] = n < 4u ? h2_bits(hh) : h2_bits(__floats2half2_rn(x0 - hf.x, x1 - hf.y));
         }
+      reinterpret_cast<uint4*>(smem + S::q_off)[tid] = make_uint4(w[0], w[1], w[2], w[3]);
     }
-    reinterpret_cast<uint4*>(smem + S::q_off)[i] = make_uint4(w[0], w[1], w[2], w[3]);
   }
   __syncthreads();
   const uint4* qf = reinterpret_cast<const uint4*>(smem + S::q_off) + lane;
