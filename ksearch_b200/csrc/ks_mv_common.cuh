@@ -1,6 +1,7 @@
 // Device helpers shared by the matvec kernels: streaming loads, f32x2 arithmetic, the
 // nibble -> f32 extraction, scale unpacking and the staging of x in shared memory.
 #pragma once
+#include "ks_gelu.cuh"
 #include "ks_internal.h"
 
 #ifndef KS_F32X2
@@ -72,23 +73,6 @@ template <>
 __device__ __forceinline__ void act_store<float>(float* p, size_t i, float v) { p[i] = v; }
 template <>
 __device__ __forceinline__ void act_store<__half>(__half* p, size_t i, float v) { p[i] = __float2half_rn(v); }
-
-// tanh-GELU(gate) * up, gate clamped to +-20 (lower.rs:2926-2954).  tanh |t| = 1 - 2 / (1 + e), e = exp(2 |t|), in 25 instructions
-// without a branch, where tanhf has two paths that a warp usually takes both (a prompt's GELU launch spent most of its time there).
-// What 1 + e and the reciprocal round off is carried along: tanh comes out rounded to the last bit of 1 as tanhf gives it, so the
-// tail 1 + tanh (which the next norm may blow up) is the same multiple of 2^-24, and the 2-norm error against 64 bits for normal x
-// is 3.77e-8 (tanhf 3.79e-8; |x| below 0.01: 4.6e-8 and 3.8e-8).
-__device__ __forceinline__ float gelu_mul(float g, float u) {
-  const float ax = fminf(20.0f, fmaxf(-20.0f, g));
-  const float t = 0.79788456f * (ax + 0.044715f * ((ax * ax) * ax));
-  const float e = __expf(fminf(2.0f * fabsf(t), 87.0f));  // >= 1; beyond the limit tanh is 1 anyway
-  const float d = 1.0f + e, dl = 1.0f - (d - e);
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-  const float off = fmaf(-dl, r, fmaf(-d, r, 1.0f));  // 1 - (1 + e) r
-  const float th = fmaf(-2.0f * r, off, 1.0f - 2.0f * r);
-  return ((0.5f * ax) * (1.0f + copysignf(th, t))) * u;
-}
 
 struct MvArgs {
   const uint8_t* W[3];

@@ -4,6 +4,7 @@
 // Each kernel restates one lowering of the reference (file:line given at the
 // kernel); arithmetic order follows the lowering so that results stay within
 // rounding of its CPU restatement.
+#include "ks_gelu.cuh"
 #include "ks_internal.h"
 
 namespace {
@@ -705,11 +706,7 @@ __global__ void softcap_argmax_kernel(unsigned n, float cap, const T* x, float* 
 template <typename T>
 __global__ void gelu_mul_kernel(size_t n, const T* g, const T* u, T* y) {
   ks_pdl_entry();
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const float ax = fminf(20.0f, fmaxf(-20.0f, ld_act<T>(g, i)));
-    const float t = 0.79788456f * (ax + 0.044715f * ((ax * ax) * ax));
-    st_act<T>(y, i, ((0.5f * ax) * (1.0f + tanhf(t))) * ld_act<T>(u, i));
-  }
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) st_act<T>(y, i, gelu_mul(ld_act<T>(g, i), ld_act<T>(u, i)));
 }
 
 }  // namespace

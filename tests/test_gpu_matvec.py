@@ -148,6 +148,44 @@ def test_matvec_gate_up_gelu(ctx, oracle, rows, cols):
     assert np.all(np.abs(got - want) <= tol)
 
 
+def _rows_that_pick(cols, picks):
+    """A Q4_K matrix whose row r is 1 in column picks[r] and 0 elsewhere."""
+    w = np.zeros((len(picks), cols // 256, 144), np.uint8)
+    w[:, :, 0:2] = np.frombuffer(np.float16(1.0).tobytes(), np.uint8)
+    w[:, :, 4:8] = w[:, :, 12:16] = 1
+    for r, c in enumerate(picks):
+        w[r, c // 256, 16 + c % 256 // 64 * 32 + c % 32] = 16 if c % 64 >= 32 else 1
+    return w
+
+
+@pytest.mark.parametrize("lo,hi,times", [(-0.01, 0.01, 1.1), (-0.2, 0.0, 1.1), (-1.0, -0.2, 1.5), (-3.0, -1.0, 1.5), (-6.0, -3.0, 1.1), (0.0, 6.0, 1.1), (-25.0, 25.0, 1.1)])
+def test_fused_gelu_against_64_bits(ctx, lo, hi, times):
+    """Rows that pick one value each: what the fused kernel gives is the GELU alone.  The same bits as the op, and off 64 bits (2-norm)
+    by hardly more than the f32 formula with a correctly rounded tanh: tanhf is within one unit in the last place, which does not show
+    near 0 (1.04 times) and does where 1 + tanh cancels, its unit against half a unit (1.34 times measured on -1 .. -0.5)."""
+    cols, rows, e = 4096, 4095, Eng(F32)
+    gate, up = ctx.buffer_bytes(_rows_that_pick(cols, range(rows))), ctx.buffer_bytes(_rows_that_pick(cols, [rows] * rows))
+    one = ctx.buffer_bytes(np.ones(rows, np.float32))
+    y, z = ctx.buffer_empty_f32(rows), ctx.buffer_empty_f32(rows)
+    got, x = [], []
+    for k in range(4):
+        v = np.random.default_rng(83 + k).uniform(lo, hi, cols).astype(np.float32)
+        v[:2], v[rows] = (lo, hi), 1.0
+        bx = ctx.buffer_bytes(v)
+        e.matvec_gate_up_gelu_wd(ctx, rows, cols, Q4K, gate, up, bx, y)
+        e.gelu_mul(ctx, rows, bx, one, z)
+        got.append(ctx.read_f32(y, rows))
+        x.append(v[:rows])
+        assert np.array_equal(got[-1], ctx.read_f32(z, rows))
+    x, got = np.concatenate(x), np.concatenate(got).astype(np.float64)
+    ax, f32 = np.clip(x, np.float32(-20), np.float32(20)), np.float32
+    t = f32(0.79788456) * (ax + f32(0.044715) * ((ax * ax) * ax))
+    ideal = ((f32(0.5) * ax) * (f32(1) + np.tanh(t.astype(np.float64)).astype(f32))).astype(np.float64)
+    a = ax.astype(np.float64)
+    want = 0.5 * a * (1.0 + np.tanh(np.sqrt(2.0 / np.pi) * (a + 0.044715 * a ** 3)))
+    assert np.linalg.norm(got - want) <= times * np.linalg.norm(ideal - want)
+
+
 def test_matvec_f16_activations(ctx, oracle):
     """The reference's own mode: f16 x in, f16 y out, f32 accumulation (RE:2263-2274)."""
     rows, cols = 256, 1536
