@@ -251,6 +251,16 @@ bool rows_share_context(const ks_model_config& g, int n, int base, int window) {
   return n >= 4 && work >= (gb == 1 ? 45e3 + 1e6 / n : 60e3 + 13e6 / n);
 }
 
+// Tiles of 64 positions that the image launch of a one-slot pass covers: what the pass sees, rounded up to a power of two so that a graph
+// serves as long as its prompt grows within that, but no more than a slot has.  (Blocks beyond the context read two words and leave, but a
+// launch for all of a slot of 131072 positions is mostly such blocks: 384 rows 143.6 us a layer of E2B and 244 of E4B, with this 137 and 231.)
+unsigned image_span(const ks_model_config& g, int n, int base) {
+  const unsigned need = ks_kv_image_tiles((size_t)base + n), all = ks_kv_image_tiles((size_t)g.max_seq);
+  unsigned span = 1;
+  while (span < need) span *= 2;
+  return span < all ? span : all;
+}
+
 // Bytes of decoded tiles (chunk attention) a model has room for, beyond one slot's: a pass that mixes slots takes as many as fit.
 constexpr size_t KS_IMAGE_MOST = 256u << 20;
 
@@ -757,9 +767,10 @@ int run_prefill_chunk(ks_model* m, int slot, int n, bool gemm) {
   ks_ctx* c = m->ctx;
   const bool share_full = gemm && m->kv_image && rows_share_context(m->cfg, n, m->seq_len[slot], 0);
   const bool share_swa = gemm && m->kv_image && rows_share_context(m->cfg, n, m->seq_len[slot], m->cfg.sliding_window);
-  // (a replay may stand further on than the pass that was captured: its tiles are those of the whole slot)
-  const Lane lane = chunk_lane(m, slot, share_full, share_swa, ks_kv_image_tiles((size_t)m->cfg.max_seq));
-  const uint64_t key = (1ull << 63) | ((uint64_t)slot << 32) | ((uint64_t)n << 8) | (share_full ? 1 : 0) | (share_swa && has_window(m->cfg) ? 2 : 0);
+  const unsigned span = share_full || share_swa ? image_span(m->cfg, n, m->seq_len[slot]) : 0;
+  const Lane lane = chunk_lane(m, slot, share_full, share_swa, span);
+  // (a replay may stand further on than the pass that was captured, but not beyond its tiles)
+  const uint64_t key = (1ull << 63) | ((uint64_t)slot << 40) | ((uint64_t)n << 28) | (uint64_t)span << 2 | (share_full ? 1 : 0) | (share_swa && has_window(m->cfg) ? 2 : 0);
   if (!gemm) {  // 1..8 rows: few different passes
     auto it = m->graphs.find(key);
     if (it == m->graphs.end()) {
@@ -797,6 +808,17 @@ int run_prefill_chunk(ks_model* m, int slot, int n, bool gemm) {
 }
 
 }  // namespace
+
+// ---- test hooks that need no GPU ----------------------------------------------------------------
+extern "C" int ks_debug_prompt_pass(int n_q, int n_kv, int hd, int max_seq, int window, int n, int base, unsigned* span) {
+  ks_model_config g{};
+  g.n_q = n_q;
+  g.n_kv = n_kv;
+  g.hd = hd;
+  g.max_seq = max_seq;
+  if (span) *span = image_span(g, n, base);
+  return rows_share_context(g, n, base, window);
+}
 
 // ---- C ABI ------------------------------------------------------------------------------------
 extern "C" {

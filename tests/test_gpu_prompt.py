@@ -142,6 +142,24 @@ def test_lengths_that_do_not_repeat_leave_no_graph(ctx):
     model.close()
 
 
+@pytest.mark.parametrize("window", [0, 100])
+def test_equal_pieces_of_a_growing_prompt(ctx, window):
+    """Pieces of one length behind each other, three prompts: their passes are launched, captured and replayed while the context grows
+    past what the first of them saw.  The same logits every time, and those of shorter pieces to the bound above."""
+    cfg = ksm.tiny_config(max_seq=5000, n_kv=2)
+    if window:
+        cfg.sliding_window, cfg.swa_layers = window, 0b101
+    model, _ = ksm.GemmaCudaModel.synthetic(ctx, cfg, seed=71, keep=True)
+    model.slot_alloc()
+    toks = [int(t) for t in synth.token_ids(71, "p", 4097, cfg.vocab)]
+    got = [_logits_after(model, ctx, [toks[i:i + 512] for i in range(0, 4096, 512)], toks[4096]) for _ in range(3)]
+    want = _logits_after(model, ctx, [toks[i:min(i + 200, 4096)] for i in range(0, 4096, 200)], toks[4096])
+    assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
+    scale, err = np.abs(want).max(), np.abs(got[0] - want)
+    assert err.max() <= 1e-3 * scale and np.sqrt((err ** 2).mean()) <= 1e-4 * scale
+    model.close()
+
+
 @pytest.mark.parametrize("n_slots,n_kv,hd,act,window", [(4, 2, 256, F32, 60), (4, 1, 256, F16, 0), (4, 2, 128, F16, 40), (12, 1, 128, F32, 50), (64, 1, 128, F32, 0)])
 def test_mixed_passes_of_other_models(ctx, n_slots, n_kv, hd, act, window):
     """prefill_many against one prefill call per slot: head size 256, f16 activations, up to as many slots as a model has.  In f16 both
