@@ -235,20 +235,23 @@ constexpr size_t KS_STAGE_IDS = KS_GEMM_CHUNK; // pinned words that stage host t
 // and more), or does each take the decode kernel (a block per row and up to four heads, spread over the chip)?  By the work of the
 // second form, rows x blocks x positions a row sees on average in units of 256 dims, against a line that lies the higher the fewer
 // rows there are: few rows are few blocks of the first form.  Microseconds per layer of 24, shared / per row, with the work:
-//   E2B (8 heads, 1 KV head of 256)  256 rows at 0: 124 / 118 (65k), 320: 130 / 133 (102k), 384: 136 / 147 (147k); 128 at 512: 100 / 96 (147k),
-//                                    160: 117 / 123 (189k); 96 at 1024: 103 / 106 (205k); 48 at 2048: 102 / 97 (198k), 64: 111 / 101 (266k);
-//                                    window 128, 256 rows: 124 / 116 (65k), 512: 167 / 178 (131k)
-//   E4B (8, 2 of 256)                256 at 0: 183 / 178, 320: 216 / 221, 384: 230 / 242; 128 at 512: 143 / 136, 160: 159 / 167; 96 at 1024:
-//                                    142 / 145; 64 at 2048: 146 / 123; window 512 at 1024: 128 rows 145 / 132 (131k), 192: 175 / 169 (196k)
-//   tiny (4, 1 of 128)               384 at 0: 65 / 63 (37k), 192 at 512: 60 / 56 (58k), 128 at 1024: 65 / 60 (70k)
-// A block of one head does the work of four, so with a KV head per query head (8, 8 of 128) the line lies lower: 128 at 0: 62 / 61
-// (33k), 192: 63 / 77 (74k); 24 at 2048: 58 / 74 (197k); 16 at 3500: 73 / 69 (225k); 32 at 512: 52 / 47 (68k).
+//   E2B (8 heads, 1 KV head of 256)  256 rows at 0: 121 / 114 (65k), 320: 126 / 128 (102k), 384: 133 / 140 (147k); 128 at 512: 96 / 95 (147k),
+//                                    160: 113 / 118 (189k); 96 at 1024: 98 / 101 (205k); 64 at 2048: 110 / 97 (266k), 80: 98 / 125 (334k);
+//                                    48 at 4096: 98 / 124 (395k); window 128, 320 rows at 1024: 126 / 122 (81k), 640: 186 / 199 (163k)
+//   E4B (8, 2 of 256)                256 at 0: 177 / 171, 320: 212 / 213, 384: 227 / 232; 128 at 512: 134 / 132, 160: 153 / 163; 96 at 1024:
+//                                    138 / 141; 64 at 2048: 149 / 120, 80: 143 / 169; window 512 at 1024: 128 rows 139 / 131 (131k), 192: 169 / 164 (196k)
+//   tiny (4, 1 of 128)               384 at 0: 60 / 59 (37k), 192 at 512: 56 / 51 (58k), 448 at 512: 69 / 75 (164k), 160 at 2048: 60 / 74 (170k)
+// At a lower line (60k for 75k) the 64 rows behind 2048 share, a tenth (E2B) to a quarter (E4B) slower.  Where it still picks the slower form
+// by more than 5 %: 48 and 64 rows behind 4096 of E4B (152 / 142 and 157 / 147), 128 in a window of 1024 there (171 / 154), 256 at 1024 of tiny
+// (69 / 64) share; 80 behind 2048 and 48 behind 6000 of tiny (57 / 69 and 64 / 85), 128 at 512 of 8 heads over 4 of 128 (55 / 64) do not.
+// A block of one head does the work of four, so with a KV head per query head (8, 8 of 128) the line lies lower: 128 at 0: 57 / 53 (33k),
+// 192: 59 / 69 (74k); 24 at 512: 49 / 43 (50k), 48: 53 / 54 (103k); 24 at 2048: 55 / 70 (197k); 8 at 6000 shares all the same: 82 / 62 (192k).
 bool rows_share_context(const ks_model_config& g, int n, int base, int window) {
   const int hpk = g.n_q / g.n_kv, gb = hpk % 4 == 0 ? 4 : hpk % 2 == 0 ? 2 : 1;
   double seen = base + 0.5 * (n + 1);
   if (window > 0 && seen > window) seen = window;
   const double work = (double)n * (g.n_q / gb) * seen * g.hd / 256.0;
-  return n >= 4 && work >= (gb == 1 ? 45e3 + 1e6 / n : 60e3 + 13e6 / n);
+  return n >= 4 && work >= (gb == 1 ? 45e3 + 1e6 / n : 75e3 + 13e6 / n);
 }
 
 // Tiles of 64 positions that the image launch of a one-slot pass covers: what the pass sees, rounded up to a power of two so that a graph
