@@ -355,6 +355,9 @@ int ks_debug_sdpa_chunk(ks_ctx* ctx, size_t n_q, size_t n_kv, size_t hd, size_t 
 /* Test hook, no GPU needed: do n prompt rows behind `base` positions (seen through a window, if > 0) share their context?  *span = tiles of
  * 64 positions that the launch which decodes them covers, if they do. */
 int ks_debug_prompt_pass(int n_q, int n_kv, int hd, int max_seq, int window, int n, int base, unsigned* span);
+/* Test hook, no GPU needed: decoded tiles a model of these sizes takes memory for where free_bytes are left, spare of which it may not
+ * touch; 0: none, its prompts go row by row. */
+size_t ks_debug_image_tiles(int n_kv, int hd, int max_seq, int n_slots, size_t free_bytes, size_t spare);
 /* Test hook, no GPU needed: where one block of the persistent decode kernel keeps its jobs (runs of weight rows, norm weights) in
  * shared memory while a token of a model of these widths runs on sm_count SMs with smem_optin bytes a block.  out[3 j] = place of
  * job j in the ring, [3 j + 1] = its bytes, [3 j + 2] = the oldest job still there when it is placed; at most max_jobs of them are

@@ -126,6 +126,7 @@ SIGNATURES = {
     "ks_model_debug_graphs": (_i, [_vp]),
     "ks_debug_sdpa_chunk": (_i, [_vp, _sz, _sz, _sz, _sz, _f, _i, _vp, _vp, _sz, _vp, _vp, _vp, _vp, _vp, _i]),
     "ks_debug_prompt_pass": (_i, [_i, _i, _i, _i, _i, _i, _i, _vp]),
+    "ks_debug_image_tiles": (_sz, [_i, _i, _i, _i, _sz, _sz]),
     "ks_debug_decode_ring": (_i, [_i, _i, _i, _i, _i, _i, _i, _sz, _i, _vp, _vp, _i]),
     "ks_comm_unique_id": (_i, [_vp]),
     "ks_comm_init": (_vp, [_vp, _i, _i, _vp]),

@@ -264,8 +264,17 @@ unsigned image_span(const ks_model_config& g, int n, int base) {
   return span < all ? span : all;
 }
 
-// Bytes of decoded tiles (chunk attention) a model has room for, beyond one slot's: a pass that mixes slots takes as many as fit.
+// Decoded tiles (chunk attention) that a model takes memory for: as many as its slots can hold, up to KS_IMAGE_MOST bytes, but one slot's
+// in any case (8 hd bytes per position and KV head, where the slot's caches are 1.125 hd a layer: a fifth of them for 35 layers).  A pass
+// that mixes slots takes as many as fit.  Prompts run without them too, row by row, so nothing else may fail for want of their memory:
+// they are 0 where `free` bytes do not leave `spare` behind them.
 constexpr size_t KS_IMAGE_MOST = 256u << 20;
+constexpr size_t KS_IMAGE_SPARE = 1u << 30;  // decode kernels, plan search, GEMM scratch and the host's own buffers come later
+size_t image_tiles(const ks_model_config& g, size_t free, size_t spare) {
+  const size_t one = ks_kv_image_bytes(1, g.n_kv, g.hd), slot = ks_kv_image_tiles((size_t)g.max_seq), all = (size_t)g.n_slots * slot;
+  const size_t tiles = all * one <= KS_IMAGE_MOST ? all : std::max(slot, KS_IMAGE_MOST / one);
+  return free >= spare && ks_kv_image_bytes(tiles, g.n_kv, g.hd) <= free - spare ? tiles : 0;
+}
 
 // Where a forward pass reads and writes: n rows of activations, their positions, and the KV caches
 // behind them.  Decode steps map row s to slot first + s (one cache per row); a prompt chunk maps
@@ -822,6 +831,14 @@ extern "C" int ks_debug_prompt_pass(int n_q, int n_kv, int hd, int max_seq, int 
   if (span) *span = image_span(g, n, base);
   return rows_share_context(g, n, base, window);
 }
+extern "C" size_t ks_debug_image_tiles(int n_kv, int hd, int max_seq, int n_slots, size_t free_bytes, size_t spare) {
+  ks_model_config g{};
+  g.n_kv = n_kv;
+  g.hd = hd;
+  g.max_seq = max_seq;
+  g.n_slots = n_slots;
+  return image_tiles(g, free_bytes, spare);
+}
 
 // ---- C ABI ------------------------------------------------------------------------------------
 extern "C" {
@@ -1008,19 +1025,6 @@ ks_model* ks_model_create(ks_ctx* ctx, const ks_model_config* cfg) {
     }
     ok = dev_alloc(m, (void**)&m->cattn_tmp, (recs * g.n_q * (g.hd + 2) + 4) * sizeof(float)) == KS_OK;
   }
-  if (ok && m->gemm_chunk && ks_sdpa_chunk_covers(g.n_q, g.n_kv, g.hd, nullptr, nullptr)) {
-    // as many tiles as the slots can hold, within a bound but not less than one slot's; a model that has no memory left for them
-    // takes its prompts row by row
-    const size_t one = ks_kv_image_bytes(1, g.n_kv, g.hd), slot = ks_kv_image_tiles((size_t)g.max_seq), all = (size_t)g.n_slots * slot;
-    const size_t tiles = all * one <= KS_IMAGE_MOST ? all : std::max(slot, KS_IMAGE_MOST / one);
-    if (cudaMalloc(&m->kv_image, ks_kv_image_bytes(tiles, g.n_kv, g.hd)) == cudaSuccess) {
-      m->owned.push_back(m->kv_image);
-      m->kv_image_tiles = tiles;
-    } else {
-      (void)cudaGetLastError();
-      m->kv_image = nullptr;
-    }
-  }
   if (ok) {
     ok = dev_alloc(m, (void**)&m->attn_tmp, (S * g.n_q * (size_t)m->n_splits * (g.hd + 2) + 4) * sizeof(float)) == KS_OK;
   }
@@ -1058,6 +1062,22 @@ ks_model* ks_model_create(ks_ctx* ctx, const ks_model_config* cfg) {
   if (!ok) {
     ks_model_destroy(m);
     return nullptr;
+  }
+  const char* image = getenv("KSEARCH_KV_IMAGE");
+  if (m->gemm_chunk && ks_sdpa_chunk_covers(g.n_q, g.n_kv, g.hd, nullptr, nullptr) && !(image && image[0] == '0')) {
+    // last, and not at the expense of what an upload stages: a tensor in f32
+    size_t stage = 0, free = 0, all = 0;
+    for (const auto& kv : m->by_name)
+      if (kv.second->dtype == KS_Q4K) stage = std::max(stage, kv.second->bytes / KS_Q4K_BLOCK_BYTES * 256 * sizeof(float));
+    if (cudaMemGetInfo(&free, &all) != cudaSuccess) free = 0;
+    const size_t tiles = image_tiles(g, free, stage + KS_IMAGE_SPARE);
+    if (tiles && cudaMalloc(&m->kv_image, ks_kv_image_bytes(tiles, g.n_kv, g.hd)) == cudaSuccess) {
+      m->owned.push_back(m->kv_image);
+      m->kv_image_tiles = tiles;
+    } else {
+      m->kv_image = nullptr;
+    }
+    (void)cudaGetLastError();
   }
   return m;
 }

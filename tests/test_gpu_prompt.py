@@ -214,6 +214,34 @@ def test_gelu_of_four_rows_per_cluster(ctx, ffn):
     model.close()
 
 
+@pytest.mark.parametrize("window", [0, 100])
+def test_prompts_of_a_model_without_decoded_tiles(ctx, monkeypatch, window):
+    """A model that has no memory for decoded tiles takes prompts row by row and slots one by one: the same logits to the model's bound,
+    behind one prompt, pieces of it and pieces of several slots."""
+    cfg = ksm.tiny_config(max_seq=1280, n_slots=3, n_kv=2)
+    if window:
+        cfg.sliding_window, cfg.swa_layers = window, 0b101
+    toks = [int(t) for t in synth.token_ids(73, "p", 1280, cfg.vocab)]
+    out = []
+    for image in ("1", "0"):
+        monkeypatch.setenv("KSEARCH_KV_IMAGE", image)
+        model, _ = ksm.GemmaCudaModel.synthetic(ctx, cfg, seed=73, keep=True)
+        slots = [model.slot_alloc() for _ in range(3)]
+        got = [_logits_after(model, ctx, p, toks[0]) for p in ([toks[:1200]], [toks[:1200]], [toks[:1200]], [toks[:700], toks[700:1200]])]
+        for s in slots:
+            model.slot_reset(s)
+        for _ in range(2):
+            model.prefill_many([(s, toks[100 * s:100 * s + 150 + 90 * s]) for s in slots])
+        model.forward(0, 3, toks[:3], True)
+        ctx.synchronize()
+        out.append(got + [model.read_debug(1, s).astype(np.float64) for s in slots])
+        assert [model.seq_len(s) for s in slots] == [2 * (150 + 90 * s) + 1 for s in slots]
+        model.close()
+    for want, got in zip(*out):
+        scale, err = np.abs(want).max(), np.abs(got - want)
+        assert err.max() <= 1e-3 * scale and np.sqrt((err ** 2).mean()) <= 1e-4 * scale
+
+
 def test_mixed_pass_with_more_context_than_its_decoded_tiles(ctx):
     """Eight slots of 15 tiles of 64 positions and 32 KV heads are more than the 64 tiles such a model keeps decoded (256 MB): their short
     pieces run in several passes.  Against the same pieces one by one, whose rows read the caches themselves: the model's bound."""

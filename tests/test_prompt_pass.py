@@ -24,6 +24,20 @@ def test_the_image_launch_covers_what_the_pass_sees_and_little_more(max_seq):
             assert need <= span <= slot and span < 2 * need
 
 
+@pytest.mark.parametrize("n_kv,hd,max_seq,n_slots", [(1, 256, 4096, 1), (2, 256, 4096, 8), (2, 256, 131072, 1), (32, 256, 1024, 8), (1, 128, 64, 64)])
+def test_decoded_tiles_leave_the_memory_that_others_need(n_kv, hd, max_seq, n_slots):
+    """As many tiles as the slots hold, up to 256 MB but one slot's at least, and none where that would cut into the spare memory."""
+    lib, most, spare = _lib.load(), 1 << 62, 3 << 30
+    one, slot = n_kv * (64 * hd * 8 + 4), -(-max_seq // 64)
+    tiles = lib.ks_debug_image_tiles(n_kv, hd, max_seq, n_slots, most, spare)
+    assert slot <= tiles <= n_slots * slot
+    assert tiles == n_slots * slot or tiles == max(slot, (256 << 20) // one)
+    need = tiles * one
+    assert lib.ks_debug_image_tiles(n_kv, hd, max_seq, n_slots, spare + need, spare) == tiles
+    for free in (spare + need - 1, spare, spare - 1, need, 0):
+        assert lib.ks_debug_image_tiles(n_kv, hd, max_seq, n_slots, free, spare) == 0
+
+
 # microseconds per layer: rows share their context / every row by itself (E2B- and E4B-shaped layers, one slot)
 @pytest.mark.parametrize("shape,window,n,base,shared,rows", [
     (E2B, 0, 256, 0, 120.8, 114.3), (E2B, 0, 384, 0, 133.4, 140.4), (E2B, 0, 128, 256, 95.3, 87.6), (E2B, 0, 256, 256, 123.1, 127.6),
