@@ -118,7 +118,7 @@ bool ks_matvec_can_fuse_pro(ks_dtype wdtype, size_t cols);
 
 // variant (plan->variant & 0xFF): 0 = streamed through the bulk-copy engine, 1 = direct register loads
 int ks_launch_matvec_stream_q4k(ks_ctx* ctx, const ks_mv_seg* segs, int n_seg, ks_mv_epilogue epi, size_t cols,
-                                ks_dtype act, const void* x, int n_tok, const ks_plan* plan, const ks_mv_pro* pro);
+                                ks_dtype act, const void* x, int n_tok, const ks_plan* plan, const ks_mv_pro* pro, bool own = false);
 int ks_launch_matvec_stream_q6k(ks_ctx* ctx, const ks_mv_seg* segs, int n_seg, size_t cols, ks_dtype act, const void* x,
                                 int n_tok, const ks_plan* plan);   // returns 1 when the shape must use the direct kernel
 // variant 2 (Q6_K only): x as block fixed point, byte dot products; returns 1 when the call must use another variant

@@ -610,9 +610,10 @@ int stream_q4k_warps(const ks_ctx* ctx, unsigned groups, unsigned cols, unsigned
 }  // namespace
 
 // Streamed Q4_K launch; plan fields: nr = rows per lane (1 or 2), nwarps, ctas_per_sm,
-// variant bits 8..15 = stages (0 = default 3), bits 16..23 = blocks per column segment (0 = auto).
+// variant bits 8..15 = stages (0 = default 3), bits 16..23 = blocks per column segment (0 = auto).  own: one token without a plan of the
+// caller's, whose warps are picked here (a plan that leaves nwarps at 0 has its other fields obeyed).
 int ks_launch_matvec_stream_q4k(ks_ctx* ctx, const ks_mv_seg* segs, int n_seg, ks_mv_epilogue epi, size_t cols,
-                                ks_dtype act, const void* x, int n_tok, const ks_plan* plan, const ks_mv_pro* pro) {
+                                ks_dtype act, const void* x, int n_tok, const ks_plan* plan, const ks_mv_pro* pro, bool own) {
   const unsigned nb = (unsigned)(cols / 256);
   const int LPR = (nb % 2 == 0) ? 8 : 4;
   const int RL = 32 / LPR;
@@ -667,7 +668,6 @@ int ks_launch_matvec_stream_q4k(ks_ctx* ctx, const ks_mv_seg* segs, int n_seg, k
   a.grp_start[a.n_seg] = g0;
   const unsigned x_bytes = (unsigned)n_tok * (unsigned)(cols / 64) * Q4K_XTOK * 4u;
   const unsigned stage_bytes = (unsigned)(RL * R * mats) * seg_blocks * KS_Q4K_BLOCK_BYTES;
-  const bool own = plan && plan->nwarps == 0 && n_tok == 1 && a.pro.mode == KS_PRO_NONE;  // one token without a plan
   if (own) nwarps = stream_q4k_warps(ctx, g0, (unsigned)cols, x_bytes, stage_bytes, mats);
   const int cps = own ? 2 : (plan && plan->ctas_per_sm > 0) ? plan->ctas_per_sm : 1;
   if (auto_stages) {

@@ -94,6 +94,63 @@ def test_plans_speak_for_few_rows_too(oracle, dtype, op, batch):
     c.close()
 
 
+def _blocks_of(c, call):
+    """Blocks of the one launch that a call captures to on the context's stream."""
+    from cuda.bindings import driver as cu
+    stream = cu.CUstream(c.lib.ks_ctx_stream(c.h))
+    (err,) = cu.cuStreamBeginCapture(stream, cu.CUstreamCaptureMode.CU_STREAM_CAPTURE_MODE_THREAD_LOCAL)
+    assert err == cu.CUresult.CUDA_SUCCESS
+    try:
+        call()
+    finally:
+        err, graph = cu.cuStreamEndCapture(stream)
+    assert err == cu.CUresult.CUDA_SUCCESS
+    err, _, n = cu.cuGraphGetNodes(graph)
+    err, nodes, n = cu.cuGraphGetNodes(graph, n)
+    assert err == cu.CUresult.CUDA_SUCCESS and n == 1
+    err, at = cu.cuGraphKernelNodeGetParams(nodes[0])
+    assert err == cu.CUresult.CUDA_SUCCESS
+    blocks, threads = at.gridDimX, at.blockDimX
+    cu.cuGraphDestroy(graph)
+    return blocks, threads
+
+
+def test_a_plan_without_warps_keeps_its_other_fields(oracle):
+    """nwarps 0 in a plan is the kernel's default for that field and no more: its blocks per SM stand.  Without a plan the launch is
+    the shape's own."""
+    rows, cols = 20480, 1536
+    c = CudaContext(0)
+    sms = c.lib.ks_ctx_sm_count(c.h)
+    W, x = _gen(Q4K, 78, "W", rows, cols), synth.normals(78, "x", cols).astype(np.float32)
+    bw, bx, y = c.buffer_bytes(W), c.buffer_bytes(x), c.buffer_empty_f32(rows)
+    y32, y64 = oracle.matvec(Q4K, W, rows, cols, x)
+
+    def call():
+        c.check(c.lib.ks_matvec(c.h, rows, cols, Q4K, bw.h, 0, 0, bx.h, 0, y.h, 0, 1))
+
+    def launch(plan):
+        for how in ("override", "set"):
+            if how == "override":
+                c.check(c.lib.ks_plan_override(c.h, C.byref(plan)))
+            else:
+                c.check(c.lib.ks_plan_set(c.h, b"mv_q4k", rows, cols, 1, C.byref(plan)))
+            got = _blocks_of(c, call)
+            call()
+            _check(c.read_f32(y, rows), y32, y64, how)
+            c.check(c.lib.ks_plan_override(c.h, None))
+            c.check(c.lib.ks_plan_set(c.h, b"mv_q4k", rows, cols, 1, None))
+            yield got
+
+    own = _blocks_of(c, call)
+    for per_sm in (1, 2, 3):
+        for blocks, threads in launch(_lib.Plan(variant=0, nr=1, nwarps=0, ctas_per_sm=per_sm, ms=0.0)):
+            assert blocks == min(sms * per_sm, -(-rows // 4 // (threads // 32)))
+    for blocks, threads in launch(_lib.Plan(variant=0, nr=1, nwarps=6, ctas_per_sm=1, ms=0.0)):
+        assert (blocks, threads) == (sms, 192)
+    assert _blocks_of(c, call) == own
+    c.close()
+
+
 def test_few_rows_never_allocate_and_graphs_outlive_growth(oracle):
     """2..8 rows work out of the scratch the context starts with: device memory in use does not change, and a shape that would
     need more takes the matvec.  A graph captured over the scratch still gives its results after a larger batch has grown it."""
