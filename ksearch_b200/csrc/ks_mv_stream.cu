@@ -579,11 +579,15 @@ int launch_q6k(ks_ctx* ctx, const MvsArgs& a, unsigned grid, int nwarps, size_t 
 // Warps of a block for one token without a plan, two blocks per SM.  A row group (four rows) is a warp's unit of work, so eight warps are
 // fewer or longer rounds than need be for many shapes.  Measured through the entry points, us, eight warps and what is picked here:
 //   few groups of long rows: four, so that more SMs take part (1536x2048 4.25 / 3.66, 512x2560 4.76 / 3.79, gate|up 1024x1536 4.98 / 4.39);
-//   more groups than one block of eight warps per SM: of seven, six or (two matrices) four warps what leaves the busiest SM the fewest
-//   groups, as long as two blocks fit an SM (eight warps of 12 blocks x two stages do not): 6144x3072 10.06 / 6.57, 6144x1536 5.02 / 4.60,
-//   20480x3072 19.3 / 15.8, gate|up 6144x1536 9.58 / 6.58, 10240x2560 17.9 / 14.0, 16384x4096 36.8 / 30.2;
-//   else eight (short rows: 20480x1024 7.0, six 7.5, but 12685x1024 6.1 and 5.6, where six warps end their second round together;
-//   gate|up 4096x1536 5.1, four 6.3; an odd number of blocks: 20480x3840 22.7, six 26.1).
+//   more groups than one block of eight warps per SM, where two blocks of eight fit an SM: six if they end their last round nearly
+//   full and eight would not, 8 to 12 and 20 to 24 groups per SM (eight / six; 6144x1536 5.02 / 4.60, at 12 groups 2048 5.9 / 5.6, 2560 7.1 / 6.4,
+//   3584 11.1 / 11.0, gate|up of 3584 17.7 / 15.7; at 23 groups 1024 6.2 / 5.7, 2560 11.6 / 10.3, 3584 22.2 / 20.0, gate|up of 1024 9.4 / 8.5, 3584
+//   35.8 / 29.9; but at 10 groups of 1024 4.0 / 3.9, at 17 groups 2560 8.9 / 9.7, 3584 16.7 / 18.9, gate|up 24.8 / 29.0, at 28 groups 11.9 / 13.6,
+//   22.3 / 28 and 35.9 / 43; seven is at best 2 % ahead, at 14 groups of 3584 2.5 % behind);
+//   where they do not fit (twelve super-blocks a row, two matrices): of seven, six or (two matrices) four warps what leaves the busiest SM the
+//   fewest groups: 6144x3072 10.06 / 6.57, 20480x3072 19.3 / 15.8, gate|up 6144x1536 9.58 / 6.58, 10240x2560 17.9 / 14.0, 16384x4096 36.8 / 30.2,
+//   four only from three rounds on if another fits (gate|up of 1536, 15 groups: eight 9.9, six 9.8, four 11.0);
+//   else eight (gate|up 4096x1536 5.1, four 6.3; an odd number of super-blocks: 20480x3840 22.7, six 26.1).
 int stream_q4k_warps(const ks_ctx* ctx, unsigned groups, unsigned cols, unsigned x_bytes, unsigned stage_bytes, int mats) {
   const unsigned sms = (unsigned)ctx->sm_count;
   if (groups <= 8u * sms) {
@@ -591,13 +595,13 @@ int stream_q4k_warps(const ks_ctx* ctx, unsigned groups, unsigned cols, unsigned
     return few ? 4 : 8;
   }
   if (cols % 512) return 8;
-  if (cols <= 1024) return mats == 1 && groups > 20u * sms && groups <= 24u * sms ? 6 : 8;
+  auto two_fit = [&](int nw) { return 2u * (make_layout(x_bytes, stage_bytes, nw, 2).total + 1024u) <= (unsigned)ctx->smem_optin + 1024u; };
+  if (two_fit(8)) return (cols > 1024 && groups <= 12u * sms) || (groups > 20u * sms && groups <= 24u * sms) ? 6 : 8;
   int best = 8;
   unsigned least = 0xFFFFFFFFu;
-  for (const int nw : {8, 7, 6, 4}) {
-    if ((nw == 8 && mats == 2) || (nw == 4 && mats == 1)) continue;
-    if (2u * (make_layout(x_bytes, stage_bytes, nw, 2).total + 1024u) > (unsigned)ctx->smem_optin + 1024u) continue;
+  for (const int nw : {7, 6, 4}) {
     const unsigned blocks = (groups + nw - 1) / nw, rounds = (groups + 2u * sms * nw - 1) / (2u * sms * nw);
+    if (!two_fit(nw) || (nw == 4 && (mats == 1 || (rounds <= 2 && best != 8)))) continue;
     const unsigned load = rounds > 1 ? rounds * 2u * nw : (blocks + sms - 1) / sms * nw;
     if (load <= least) {
       least = load;

@@ -151,6 +151,28 @@ def test_a_plan_without_warps_keeps_its_other_fields(oracle):
     c.close()
 
 
+@pytest.mark.parametrize("gate_up,cols,per_sm,warps", [
+    (0, 2560, 2.5, 4), (0, 3584, 1.5, 4), (0, 3584, 3, 8), (0, 2560, 7.9, 8), (1, 1536, 1.9, 4), (1, 1536, 7.9, 8),     # few groups of four rows
+    (0, 2560, 8.1, 6), (0, 2560, 12, 6), (0, 2560, 12.1, 8), (0, 2560, 17, 8), (0, 3584, 17, 8), (0, 3584, 20, 8), (0, 2560, 20.1, 6), (0, 3584, 24, 6), (0, 2560, 28, 8), (0, 3584, 34, 8),
+    (0, 1024, 10, 8), (0, 1024, 13, 8), (0, 1024, 22, 6), (0, 1024, 25, 8), (0, 2048, 13, 8),
+    (1, 3584, 9, 6), (1, 3584, 15, 8), (1, 3584, 19, 8), (1, 3584, 22, 6), (1, 3584, 32, 8), (1, 1024, 10, 8), (1, 1024, 23, 6),
+    (0, 3072, 10, 6), (0, 3072, 13, 7), (1, 1536, 10, 6), (1, 1536, 13, 7), (1, 1536, 15, 6), (1, 1536, 17, 4), (1, 1536, 27, 7), (1, 2560, 9, 4), (1, 2560, 15, 4),   # two blocks of eight do not fit
+    (0, 3840, 24, 8), (1, 1280, 20, 8),                                                                                 # an odd number of super-blocks
+])
+def test_warps_of_a_streamed_matvec(ctx, gate_up, cols, per_sm, warps):
+    """One token without a plan takes the block size that was measured fastest for its groups per SM (on 148 SMs; see stream_q4k_warps)."""
+    rows = int(per_sm * ctx.lib.ks_ctx_sm_count(ctx.h)) * (8 if cols // 256 % 2 else 4)
+    bw, bx, y = (ctx.buffer_empty_bytes(n) for n in (rows * cols // 256 * 144, 4 * cols, 4 * rows))
+
+    def call():
+        if gate_up:
+            ctx.check(ctx.lib.ks_matvec_gate_up_gelu(ctx.h, rows, cols, Q4K, bw.h, bw.h, 0, bx.h, y.h))
+        else:
+            ctx.check(ctx.lib.ks_matvec(ctx.h, rows, cols, Q4K, bw.h, 0, 0, bx.h, 0, y.h, 0, 1))
+
+    assert _blocks_of(ctx, call)[1] == 32 * warps
+
+
 def test_few_rows_never_allocate_and_graphs_outlive_growth(oracle):
     """2..8 rows work out of the scratch the context starts with: device memory in use does not change, and a shape that would
     need more takes the matvec.  A graph captured over the scratch still gives its results after a larger batch has grown it."""
