@@ -255,11 +255,12 @@ bool rows_share_context(const ks_model_config& g, int n, int base, int window) {
 }
 
 // Tiles of 64 positions that the image launch of a one-slot pass covers: what the pass sees, rounded up to a power of two so that a graph
-// serves as long as its prompt grows within that, but no more than a slot has.  (Blocks beyond the context read two words and leave, but a
-// launch for all of a slot of 131072 positions is mostly such blocks: 384 rows 143.6 us a layer of E2B and 244 of E4B, with this 137 and 231.)
+// serves as long as its prompt grows within that, but no more than a slot has.  Blocks beyond the context read two words and leave, but a
+// launch for all of a slot of 131072 positions is mostly such blocks: 384 rows 143.6 us a layer of E2B and 244 of E4B, with this 137 and 231.
+// Below 32 tiles nothing is won (384 rows of E4B 222.5 us a layer at 32 and 64, 223.6 at 16, 225 at 8; E2B 132.8 at all of them).
 unsigned image_span(const ks_model_config& g, int n, int base) {
   const unsigned need = ks_kv_image_tiles((size_t)base + n), all = ks_kv_image_tiles((size_t)g.max_seq);
-  unsigned span = 1;
+  unsigned span = 32;
   while (span < need) span *= 2;
   return span < all ? span : all;
 }

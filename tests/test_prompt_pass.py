@@ -21,7 +21,7 @@ def test_the_image_launch_covers_what_the_pass_sees_and_little_more(max_seq):
             if base + n > max_seq:
                 continue
             need, span = -(-(base + n) // 64), _pass(E4B, max_seq, 0, n, base)[1]
-            assert need <= span <= slot and span < 2 * need
+            assert need <= span <= slot and span < max(2 * need, 33)
 
 
 @pytest.mark.parametrize("n_kv,hd,max_seq,n_slots", [(1, 256, 4096, 1), (2, 256, 4096, 8), (2, 256, 131072, 1), (32, 256, 1024, 8), (1, 128, 64, 64)])
