@@ -455,10 +455,12 @@ struct EpiNormArgs {
   float* out_x;
   __half* xt;
 };
-constexpr int GM_MANY_ROWS = 512;
+constexpr size_t GM_NORM_AHEAD = 3u << 18;  // values of a launch up to which the weights come early
 constexpr size_t GM_NORM_MOST = 8 * 1024;  // the longest rows: eight values per thread
 // THREADS: at most; more than 512 have half the registers each.  AHEAD: the norm weights are asked for with the first partials: with few
-// rows that hides two trips to memory, with many it costs the registers that more blocks per SM need (2047 rows of 1536 19.4 us, without 17).
+// rows that hides two trips to memory, with many it costs the registers that more blocks per SM need.  A layer with its two launches, us,
+// ahead / without: 1536 values 128 rows 80.5 / 84.1, 512 160.2 / 164.5, 768 203.1 / 201.8 (one launch of 2047 19.4 / 17); 2560 values 256 rows 171.0 /
+// 175.7, 300 208.7 / 209.1, 384 226.8 / 223.7, 1536 730 / 724; 4096 values 128 rows 126.9 / 130.2, 200 181.5 / 179.3, 512 322.9 / 314.4.
 template <unsigned THREADS, bool AHEAD>
 __global__ void __launch_bounds__(THREADS, AHEAD ? 1 : 1024 / THREADS) gemm_finish_norm_split_kernel(const EpiNormArgs e) {
   __shared__ float red[32];
@@ -1005,7 +1007,7 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
     e.xt = (__half*)epi->xt_out;
     const unsigned threads = (unsigned)((rows[0] / 8 + 31) / 32 * 32);
     if (threads > 512u) KS_LAUNCH(ctx, (gemm_finish_norm_split_kernel<1024, false>), e.np, threads, 0, e);
-    else if (n_tok < GM_MANY_ROWS) KS_LAUNCH(ctx, (gemm_finish_norm_split_kernel<512, true>), e.np, threads, 0, e);
+    else if ((size_t)n_tok * rows[0] <= GM_NORM_AHEAD) KS_LAUNCH(ctx, (gemm_finish_norm_split_kernel<512, true>), e.np, threads, 0, e);
     else KS_LAUNCH(ctx, (gemm_finish_norm_split_kernel<512, false>), e.np, threads, 0, e);
     return ks_after_launch(ctx, "gemm_finish_norm_split");
   }
