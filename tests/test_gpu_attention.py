@@ -25,9 +25,10 @@ def test_decode_attention_tile_edges(ctx, oracle, act, n_q, n_kv, hd):
 @pytest.mark.parametrize("n_q,n_kv,hd", [(8, 2, 256), (4, 4, 128)])
 def test_splits_dealt_by_length(ctx, oracle, act, n_q, n_kv, hd):
     """Slots of unequal contexts take splits by their lengths: sizes that fill the launch at once and sizes that need a spare chunk per
-    slot, contexts of one position, the most slots, launches on either side of the line to the plain layout, windows."""
+    slot, contexts of one position, the most slots, launches on either side of the two lines to the plain layout (contexts that average
+    four fifths of the longest: 2000 and 1200, 1000 and 2200 over three; 128 positions a split: 512 in four), windows."""
     for tlens, ns in (([3000, 5], 2), ([1, 700, 129, 2048], 4), ([5, 6, 7, 1500, 9, 10, 11, 12], 3), ([1100] + [1 + 7 * i for i in range(31)], 4),
-                      ([2000, 1600], 2), ([2000, 1599], 2), ([513, 1], 4), ([512, 1], 4), ([900, 16, 900, 100, 33], 5)):
+                      ([2000, 1600], 2), ([2000, 1599], 2), ([2000, 1200], 2), ([2000, 1199], 2), ([1000, 733, 733, 734], 4), ([1000, 733, 733, 733], 4), ([513, 1], 4), ([512, 1], 4), ([900, 16, 900, 100, 33], 5)):
         starts = [(11 * i) % 40 for i in range(len(tlens))]
         _attn_case(ctx, oracle, Eng(act), len(tlens), n_q, n_kv, hd, max(tlens) + 40, tlens, starts, hd ** -0.5, ns, act=act)
 

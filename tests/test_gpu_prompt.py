@@ -199,11 +199,12 @@ def test_mixed_passes_of_other_models(ctx, n_slots, n_kv, hd, act, window):
 
 
 @pytest.mark.parametrize("ffn", [2304, 3328, 16384])
-def test_gelu_of_four_rows_per_cluster(ctx, ffn):
+def test_gelu_of_four_rows_per_cluster(ctx, oracle, ffn):
     """From 128 rows and 2^18 values on four token rows share a cluster of blocks: row counts around a multiple of four, widths that
-    leave warps of a block and blocks of the cluster without work, the widest rows.  Against pieces of 100 rows, which have a cluster per row."""
+    leave warps of a block and blocks of the cluster without work, the widest rows.  Against pieces of 100 rows, which have a cluster per row,
+    and against the CPU decoder: the model's bounds."""
     cfg = ksm.ModelConfig(2, 256, ffn, 2, 1, 128, 1024, 256, 1, sigma_w=0.01, sigma_embd=1e-4)
-    model, _ = ksm.GemmaCudaModel.synthetic(ctx, cfg, seed=43, keep=True)
+    model, T = ksm.GemmaCudaModel.synthetic(ctx, cfg, seed=43, keep=True)
     model.slot_alloc()
     toks = [int(t) for t in synth.token_ids(43, "p", 200, cfg.vocab)]
     for n in (128, 129, 130, 131, 191):
@@ -211,6 +212,13 @@ def test_gelu_of_four_rows_per_cluster(ctx, ffn):
         got = _logits_after(model, ctx, [toks[:n]], toks[n])
         scale, err = np.abs(want).max(), np.abs(got - want)
         assert err.max() <= 1e-3 * scale and np.sqrt((err ** 2).mean()) <= 1e-4 * scale, n
+    cpu = oracle.CpuDecoder(oracle.decoder_cfg(cfg), T)
+    for t in toks[:n + 1]:
+        cpu.forward_token(t, True)
+    want = cpu.logits().astype(np.float64)
+    scale, err = np.abs(want).max(), np.abs(got - want)
+    assert err.max() <= 1e-3 * scale and np.sqrt((err ** 2).mean()) <= 1e-4 * scale
+    cpu.close()
     model.close()
 
 
@@ -243,7 +251,7 @@ def test_prompts_of_a_model_without_decoded_tiles(ctx, monkeypatch, window):
 
 
 def test_mixed_pass_with_more_context_than_its_decoded_tiles(ctx):
-    """Eight slots of 15 tiles of 64 positions and 32 KV heads are more than the 64 tiles such a model keeps decoded (256 MB): their short
+    """Eight slots of 15 tiles of 64 positions and 32 KV heads are more than the 63 tiles such a model keeps decoded (256 MB, 4 MB and a word per head each): their short
     pieces run in several passes.  Against the same pieces one by one, whose rows read the caches themselves: the model's bound."""
     cfg = ksm.ModelConfig(1, 256, 512, 32, 32, 256, 1024, 1024, 8, sigma_w=0.01, sigma_embd=1e-4)
     model, _ = ksm.GemmaCudaModel.synthetic(ctx, cfg, seed=53, keep=True)
