@@ -579,9 +579,12 @@ __global__ void __cluster_dims__(GM_GELU_CL, 1, 1) __launch_bounds__(GM_GELU_THR
 // (put_split8_rows4).  Bound by loads in flight: all first partials are requested before anything is waited for, and 64 registers
 // keep five blocks of 192 threads on an SM (with 94 and three: 60 us instead of 47; with the second partials requested early as well
 // it spills: 51).  The partial counts, half a dozen divisions each, are a lane's work each (31 to 24 million instructions).
-// 2047 rows of 6144 values, 111 MB read and 57 written: 78 us with a cluster of four per row, 47 here; 1530 rows of 10240: 107, 60.
+// 2047 rows of 6144 values, 113 MB read and 57 written: 84 us with a cluster of four per row, 45 here; 1530 rows of 10240: 121, 61.
 constexpr unsigned GM_R4_CL = 8, GM_R4_S = 2, GM_R4_WARPS = 16;  // blocks of a cluster, steps of a warp, warps at most
-constexpr int GM_R4_ROWS = 128;  // from so many rows and values on: 129 rows of 6144 values 7.8 and 6.6 us, of 1024 5.1 and 6.4; 1025 of 1024 15.9 and 8.7
+// From so many rows and more values than so many, a cluster per row / per four rows, each launch alone behind flushed caches: 129 rows of 6144
+// values 10.4 / 9.0 us, of 10240 15.9 / 10.7, of 3072 6.6 / 6.0, of 2048 6.1 / 5.5; 128 of 2048 6.1 / 7.7; 256 of 1024 6.3 / 7.7, 257 7.7 / 5.7.  (4096
+// values from 129 to 192 rows are on the wrong side: 7.2 / 7.9 to 7.7 / 8.5.)
+constexpr int GM_R4_ROWS = 128;
 constexpr size_t GM_R4_VALUES = 1u << 18;
 static_assert(GM_GELU_MOST <= GM_R4_CL * GM_R4_S * GM_R4_WARPS * 64, "the longest rows fit");
 __device__ __forceinline__ void ld8(const float* p, float (&v)[8]) {
@@ -1039,7 +1042,7 @@ int ks_launch_gemm_segs(ks_ctx* ctx, ks_dtype wdtype, int n_seg, const uint8_t* 
     return ks_after_launch(ctx, "gemm_finish_qkv");
   }
   if (mode == KS_GEMM_GELU_SPLIT) {
-    if (n_tok >= GM_R4_ROWS && (size_t)n_tok * rows[0] >= GM_R4_VALUES) {
+    if (n_tok >= GM_R4_ROWS && (size_t)n_tok * rows[0] > GM_R4_VALUES) {
       const unsigned per = ((unsigned)rows[0] / 64u + GM_R4_CL - 1u) / GM_R4_CL, warps = (per + GM_R4_S - 1u) / GM_R4_S;
       KS_LAUNCH(ctx, gemm_finish_gelu_rows_kernel, epi->next.np / 4u * GM_R4_CL, warps * 32u, 0, (const float*)out[0], (const float*)out[1], part_stride[0], map,
                 (unsigned)n_tok, epi->next.np, epi->next.tbn, (unsigned)rows[0], (__half*)epi->xt_out);
