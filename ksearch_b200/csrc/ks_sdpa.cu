@@ -259,11 +259,12 @@ sdpa_part_kernel(unsigned n_q, unsigned n_kv, float scale, const T* q, const uin
 }
 
 // Slots of unequal contexts share their launch's splits by length: every slot gets as many chunks of one size as its context has, or the
-// launch lasts as long as a share of its longest context (four slots of 1024, 4096, 16384 and 16384 positions in 32 splits each: 27.8
-// us, dealt 24; with 4 KV heads 41.4 and 30.9; eight of 50, 100, .. 6400 with one 20.3 and 14.8; figures before q was read in one trip).  Contexts that are short for the splits
-// (chunks of 128 positions) or average four fifths of the longest keep the plain layout (eight of 8192: 42.8 us either way); working the
-// rest out takes half a microsecond in each of the two launches (9000 and 30 positions: 16.4 and 16.8).  Chunk u of the launch leaves its
-// record at place u, one head behind the other.  A whole warp calls; lane s speaks for slot s.
+// launch lasts as long as a share of its longest context (four slots of 1024, 4096, 16384 and 16384 positions in 32 splits each: 24.2
+// us, dealt 20.9; with 4 KV heads 39.0 and 28.7; eight of 50, 100, .. 6400 with one 18.6 and 13.2).  Contexts that are short for the splits
+// (chunks of 128 positions) or average four fifths of the longest keep the plain layout; finding that out costs up to half a microsecond in
+// each of the two launches (eight of 8192 24.4 and 25.4, eight of 300 11.0 and 11.8, four of 16384 24.6 and 24.7).  Chunk u of the launch leaves
+// its record at place u, one head behind the other.  Steps of a model pass no max_t and keep the plain layout, the only one that the merge
+// into an operand image knows.  A whole warp calls; lane s speaks for slot s.
 constexpr unsigned kDealSlots = 32;
 constexpr unsigned kMinChunk = 128;  // positions of a split at least: a tile of 16 per warp
 struct Deal {

@@ -19,9 +19,9 @@
 //
 // Bound by the chain of a tile: scores (48 MMAs), probabilities, values (12 MMAs of 256 columns), 3.2 us for 128 x 64.  When eight warps
 // of every block decoded its tiles it was 5.7 us, 2.2 of them waiting for keys; one thread per row of scores: 3.7.  A block takes another
-// 8 us: q 3.6, records 2, setting up 2.  Launches with their image, back to back: 2047 rows of 8 heads (128 blocks of up to 32 tiles) 119
-// us, in two splits 78 (decoding in every block 205 and 118); 2000 rows behind 2000 positions, 2 KV heads (126 blocks of up to 63 tiles)
-// 218, in two splits 192 (387 and 343); 300 rows in three splits 23.6 (30).
+// 8 us: q 3.6, records 2, setting up 2.  Launches with their image, back to back: 2047 rows of 8 heads (128 blocks of up to 32 tiles) 118
+// us, in two splits 76 (decoding in every block 205 and 118); 2000 rows behind 2000 positions, 2 KV heads (126 blocks of up to 63 tiles)
+// 213, in two splits 188 (387 and 343); 300 rows in three splits 23.5 (30).
 #include "ks_gemm_common.cuh"
 
 namespace {
@@ -594,7 +594,8 @@ int launch_chunk(ks_ctx* ctx, dim3 grid, const ChunkParts& parts, size_t slot_st
 
 // Context splits of a chunk: enough blocks for every SM, at least two tiles each.  A nearly empty second wave costs more than fewer
 // splits, except against one: the later rows see most of the context, and half a chip waits for them (2047 rows of 8 heads, 128
-// blocks: 205 us, twice as many halves 118, three times as many thirds 151).  `ctx_len` may exceed what the rows see.
+// blocks: 118 us, twice as many halves 76, three times as many thirds 95; 64 blocks in halves 44, thirds 46; 19 blocks 31, 26 and 23.5; 126
+// blocks behind as many positions 213, 188 and 187).  `ctx_len` may exceed what the rows see.
 int ks_sdpa_chunk_splits(const ks_ctx* ctx, int n_tok, size_t n_q, size_t n_kv, size_t ctx_len, int most) {
   const size_t blocks = ((size_t)n_tok * (n_q / n_kv) + CH_BM - 1) / CH_BM * n_kv;
   size_t s = ((size_t)ctx->sm_count + blocks - 1) / blocks;
